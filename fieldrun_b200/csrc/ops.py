@@ -26,6 +26,8 @@ _SIGNATURES = {
     "frb_wait_probe": "lpp",
     "frb_add_rows": "ppl",
     "frb_attention_generic": "pppipipppiiiifiipippif" "iii",
+    "frb_attention_f32_tiles": "ppppi" "ppippppp" "iiiif" "ipippi" "fii",
+    "frb_attention_f32_token": "ppppi" "ppippip" "iiiif" "ipippi" "fii",
     "frb_layernorm": "ppppfppiii",
     "frb_unary_unit": "ppili",
     "frb_softcap": "plff",
@@ -100,6 +102,7 @@ _ENTRY_GROUPS = {
                "frb_latent_attention_mma", "frb_latent_attention_tc"),
     "attention": ("frb_attention_decode_mma", "frb_attention_prefill_mma", "frb_attention_decode_tma", "frb_attention_prefill_tc",
                   "frb_attention_pair_tc"),
+    "attention32": ("frb_attention_f32_tiles", "frb_attention_f32_token"),
     "streams": ("frb_weight_stream", "frb_expert_gemm_mma"),
     "experts": ("frb_router_topk", "frb_expert_plan", "frb_expert_combine", "frb_expert_gemm_generic", "frb_route_plan_small",
                 "frb_router_small", "frb_router_logits", "frb_scaled_rows"),
@@ -190,7 +193,7 @@ def _stream() -> int:
 
 
 _LAUNCHES = 0
-_KERNELS_PER_CALL = {"frb_gated_delta_rule": 2, "frb_gated_recurrence": 2, "frb_sample_floor": 3, "frb_argmax_rows": 2, "frb_expert_plan": 3, "frb_attention_decode_mma": 2, "frb_attention_decode_tma": 2}
+_KERNELS_PER_CALL = {"frb_gated_delta_rule": 2, "frb_gated_recurrence": 2, "frb_sample_floor": 3, "frb_argmax_rows": 2, "frb_expert_plan": 3, "frb_attention_decode_mma": 2, "frb_attention_decode_tma": 2, "frb_attention_f32_token": 2}
 
 
 def launches() -> int:
@@ -799,6 +802,67 @@ def attention_generic(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
           float(scale), int(window or 0), int(v_dim or head_dim), _ptr(slopes), int(chunk or 0), _ptr(sinks), _ptr(gate),
           gate.shape[1] if gate is not None else 0, float(softcap or 0.0), int(keep_first or 0), num_kv_heads // maps,
           int(out.dtype == torch.float32))
+
+
+def attention_f32_tiles_take(head_dim: int, v_dim: int) -> bool:
+    """Whether :func:`attention_f32_tiles` takes heads of these sizes: rows in 16-byte units, two blocks' tiles on an SM."""
+    return head_dim % 4 == 0 and 4 <= head_dim <= 128 and 1 <= v_dim <= 128
+
+
+def attention_f32_token_takes(head_dim: int, v_dim: int) -> bool:
+    """Whether :func:`attention_f32_token` takes heads of these sizes (it is compiled for the head sizes that models have)."""
+    return head_dim in (32, 64, 96, 128) and (v_dim == head_dim or (head_dim, v_dim) == (64, 128))
+
+
+def _attention_f32_options(q, k_pages, out, num_heads, num_kv_heads, head_dim, v_dim, scale, window, slopes, chunk, sinks, gate, softcap,
+                           keep_first, maps) -> tuple:
+    for t, what in ((q, "queries"), (k_pages, "keys"), (out, "the attention's output")):
+        _want(t, torch.float32, what)
+    _want_slopes(slopes, num_heads)
+    if sinks is not None:
+        _want(sinks, torch.float32, "softmax sinks")
+        if sinks.numel() != num_heads:
+            raise KernelError(f"{sinks.numel()} sinks for {num_heads} heads")
+    if gate is not None:
+        _want(gate, torch.float32, "head gates")
+        if gate.shape[0] != q.shape[0] or gate.shape[1] < num_heads:
+            raise KernelError(f"head gates of shape {list(gate.shape)} for {q.shape[0]} tokens of {num_heads} heads")
+    return (num_heads, num_kv_heads, head_dim, int(v_dim or head_dim), float(scale), int(window or 0), _ptr(slopes), int(chunk or 0),
+            _ptr(sinks), _ptr(gate), gate.shape[1] if gate is not None else 0, float(softcap or 0.0), int(keep_first or 0),
+            num_kv_heads // maps)
+
+
+def attention_f32_tiles(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, page_table: torch.Tensor, tile_seq: torch.Tensor,
+                        tile_q0: torch.Tensor, seq_slot: torch.Tensor, seq_start: torch.Tensor, seq_q_len: torch.Tensor,
+                        cu_q_len: torch.Tensor, out: torch.Tensor, *, num_heads: int, num_kv_heads: int, head_dim: int, scale: float,
+                        window: Optional[int], v_dim: Optional[int] = None, slopes: Optional[torch.Tensor] = None,
+                        chunk: Optional[int] = None, sinks: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None,
+                        softcap: Optional[float] = None, keep_first: int = 0, maps: int = 1) -> None:
+    """:func:`attention_generic` in float32 for a step of prompts, in tiles of queries (attention_f32.cu): ``tile_seq`` and
+    ``tile_q0`` are the step's tiles of 128 queries; head sizes as :func:`attention_f32_tiles_take` says."""
+    options = _attention_f32_options(q, k_pages, out, num_heads, num_kv_heads, head_dim, v_dim, scale, window, slopes, chunk, sinks, gate,
+                                     softcap, keep_first, maps)
+    _call("frb_attention_f32_tiles", _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(page_table), page_table.shape[1], _ptr(tile_seq),
+          _ptr(tile_q0), tile_seq.numel(), _ptr(seq_slot), _ptr(seq_start), _ptr(seq_q_len), _ptr(cu_q_len), _ptr(out), *options)
+
+
+def attention_f32_token(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, page_table: torch.Tensor, tok_pos: torch.Tensor,
+                        tok_slot: torch.Tensor, part_o: torch.Tensor, part_ml: torch.Tensor, out: torch.Tensor, *, max_chunks: int,
+                        num_heads: int, num_kv_heads: int, head_dim: int, scale: float, window: Optional[int],
+                        v_dim: Optional[int] = None, slopes: Optional[torch.Tensor] = None, chunk: Optional[int] = None,
+                        sinks: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, softcap: Optional[float] = None,
+                        keep_first: int = 0, maps: int = 1) -> None:
+    """:func:`attention_generic` in float32 for one token a sequence, in ``max_chunks`` chunks of ``ATTENTION_CHUNK`` keys
+    (attention_f32.cu); ``part_o`` [T, heads, max_chunks, v_dim] and ``part_ml`` [T, heads, max_chunks, 2] hold the chunks'
+    results; head sizes as :func:`attention_f32_token_takes` says."""
+    options = _attention_f32_options(q, k_pages, out, num_heads, num_kv_heads, head_dim, v_dim, scale, window, slopes, chunk, sinks, gate,
+                                     softcap, keep_first, maps)
+    for t, floats in ((part_o, int(v_dim or head_dim)), (part_ml, 2)):
+        _want(t, torch.float32, "the chunks' results")
+        if t.numel() < q.shape[0] * num_heads * max_chunks * floats:
+            raise KernelError(f"the results of {max_chunks} chunks do not fit {list(t.shape)}")
+    _call("frb_attention_f32_token", _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(page_table), page_table.shape[1], _ptr(tok_pos),
+          _ptr(tok_slot), q.shape[0], _ptr(part_o), _ptr(part_ml), max_chunks, _ptr(out), *options)
 
 
 ROUTE_SOFTMAX, ROUTE_FLOOR = 2, 4      # bits of the routing kernels' ``renormalize`` (bit 0: divide by the picked scores' sum)

@@ -1,0 +1,100 @@
+"""The float32 path's own kernels against the general ones, at the edges of their tiles and over all forms that they take."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+
+
+def ops():
+    from fieldrun_b200.csrc import ops as o
+    return o
+
+
+def i32(values):
+    return torch.tensor(np.asarray(values), dtype=torch.int32, device=DEV)
+
+
+def paged(starts, lengths, k_heads, v_heads, dim, vdim, seed):
+    """Pages in a scrambled order, filled with numbers to the end, for sequences that hold starts + lengths tokens."""
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    need = [(s + n + 63) // 64 for s, n in zip(starts, lengths)]
+    order = np.random.default_rng(seed).permutation(sum(need) + 3)
+    keys = torch.randn(len(order), k_heads, 64, dim, device=DEV, generator=gen)
+    values = torch.randn(len(order), v_heads, vdim, 64, device=DEV, generator=gen)
+    table = np.full((len(starts), max(need)), -1, dtype=np.int32)
+    at = 0
+    for row, count in enumerate(need):
+        table[row, :count] = order[at:at + count]
+        at += count
+    return keys, values, i32(table), gen
+
+
+FORMS = {
+    "plain": {},
+    "window": dict(window=70),
+    "window beside first tokens": dict(window=37, keep_first=5),
+    "chunks, sinks, gates": dict(chunk=48, sinks=True, gate=True),
+    "slopes": dict(slopes=True),
+    "cap": dict(softcap=3.0),
+}
+SHAPES = [(6, 2, 32, 32, 1), (8, 8, 64, 64, 1), (12, 2, 128, 128, 1), (9, 1, 96, 96, 1), (8, 4, 64, 128, 2), (6, 3, 12, 20, 1), (2, 1, 100, 7, 1)]
+
+
+def options(form, heads, tokens, gen):
+    made = dict(window=None)
+    made.update({k: v for k, v in FORMS[form].items() if v is not True})
+    if FORMS[form].get("sinks"):
+        made["sinks"] = torch.randn(heads, device=DEV, generator=gen)
+    if FORMS[form].get("slopes"):
+        made["slopes"] = torch.rand(heads, device=DEV, generator=gen) * 0.2
+    if FORMS[form].get("gate"):
+        made["gate"] = torch.randn(tokens, heads + 3, device=DEV, generator=gen)
+    return made
+
+
+def check(got, want, keys):
+    """Both sides are float32 sums of at most `keys` weighted values, whose weights carry the rounding of a product of at most
+    128 entries: the difference stays below (128 + keys / 8) roundings of the largest result."""
+    error = (got - want).abs().max().item() / want.abs().max().item()
+    assert torch.isfinite(got).all() and error < (128 + keys / 8) * 2.0 ** -24, error
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,maps", SHAPES)
+def test_prompts_in_tiles_equal_the_general_kernel(heads, kv_heads, dim, vdim, maps, form):
+    assert ops().attention_f32_tiles_take(dim, vdim)
+    starts, lengths = [0, 3, 0, 130, 64], [1, 64, 65, 200, 127]
+    keys, values, table, gen = paged(starts, lengths, kv_heads, kv_heads // maps, dim, vdim, 3)
+    tokens = sum(lengths)
+    q = torch.randn(tokens, heads * dim, device=DEV, generator=gen)
+    common = dict(num_heads=heads, num_kv_heads=kv_heads, head_dim=dim, v_dim=vdim, scale=dim ** -0.5, maps=maps,
+                  **options(form, heads, tokens, gen))
+    pos = np.concatenate([s + np.arange(n) for s, n in zip(starts, lengths)])
+    want, got = (torch.full((tokens, heads * vdim), float("nan"), device=DEV) for _ in range(2))
+    ops().attention_generic(q, keys, values, table, i32(pos), i32(np.repeat(np.arange(5), lengths)), want, **common)
+    tiles = [(b, q0) for b, n in enumerate(lengths) for q0 in range(0, n, 128)]
+    ops().attention_f32_tiles(q, keys, values, table, i32([t[0] for t in tiles]), i32([t[1] for t in tiles]), i32(range(5)), i32(starts),
+                              i32(lengths), i32(np.concatenate([[0], np.cumsum(lengths)])), got, **common)
+    check(got, want, 330)
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,maps", [s for s in SHAPES if s[2] % 32 == 0] + [(10, 1, 64, 64, 1), (20, 1, 32, 32, 1)])
+def test_single_tokens_in_chunks_equal_the_general_kernel(heads, kv_heads, dim, vdim, maps, form):
+    assert ops().attention_f32_token_takes(dim, vdim)
+    lengths = [1, 64, 65, 256, 257, 700]
+    keys, values, table, gen = paged([0] * 6, lengths, kv_heads, kv_heads // maps, dim, vdim, 4)
+    q = torch.randn(6, heads * dim, device=DEV, generator=gen)
+    common = dict(num_heads=heads, num_kv_heads=kv_heads, head_dim=dim, v_dim=vdim, scale=dim ** -0.5, maps=maps,
+                  **options(form, heads, 6, gen))
+    pos, slots = i32([n - 1 for n in lengths]), i32(range(6))
+    want, got = (torch.full((6, heads * vdim), float("nan"), device=DEV) for _ in range(2))
+    ops().attention_generic(q, keys, values, table, pos, slots, want, **common)
+    chunks = 4                                                    # more than the longest sequence needs
+    part_o = torch.full((6, heads, chunks, vdim), float("nan"), device=DEV)
+    part_ml = torch.full((6, heads, chunks, 2), float("nan"), device=DEV)
+    ops().attention_f32_token(q, keys, values, table, pos, slots, part_o, part_ml, got, max_chunks=chunks, **common)
+    check(got, want, 700)
