@@ -47,6 +47,7 @@ _SIGNATURES = {
     "frb_expert_plan": "piiiippppppp",
     "frb_expert_combine": "pppiiip",
     "frb_expert_gemm_generic": "ppipppppipiiiif",
+    "frb_rows_f32": "pppppppipiiif",
     "frb_sample_rows": "piipppp",
     "frb_argmax_rows": "piippp",
     "frb_sample_floor": "piippppppp",
@@ -103,7 +104,7 @@ _ENTRY_GROUPS = {
     "attention": ("frb_attention_decode_mma", "frb_attention_prefill_mma", "frb_attention_decode_tma", "frb_attention_prefill_tc",
                   "frb_attention_pair_tc"),
     "attention32": ("frb_attention_f32_tiles", "frb_attention_f32_token"),
-    "streams": ("frb_weight_stream", "frb_expert_gemm_mma"),
+    "streams": ("frb_weight_stream", "frb_expert_gemm_mma", "frb_rows_f32"),
     "experts": ("frb_router_topk", "frb_expert_plan", "frb_expert_combine", "frb_expert_gemm_generic", "frb_route_plan_small",
                 "frb_router_small", "frb_router_logits", "frb_scaled_rows"),
     "products": ("frb_expert_gemm_tc", "frb_gather_rows_bf16"),
@@ -920,6 +921,25 @@ def expert_gemm_generic(w: torch.Tensor, x: torch.Tensor, x_rows: Optional[torch
     feats = w.shape[1] // 2 if paired else w.shape[1]
     _call("frb_expert_gemm_generic", _ptr(w), _ptr(x), _code(w.dtype), _ptr(x_rows), _ptr(tile_expert), _ptr(tile_row0),
           _ptr(num_tiles), _ptr(offsets), max_tiles, _ptr(out), _code(out.dtype), feats, w.shape[2], int(paired), float(gate_limit))
+
+
+ROWS_F32_TILE = 8          # most rows of a tile that rows_f32 takes
+
+
+def rows_f32_takes(inner: int) -> bool:
+    """Whether :func:`rows_f32` takes weight rows of this size (16-byte loads)."""
+    return inner % 4 == 0
+
+
+def rows_f32(w: torch.Tensor, x: torch.Tensor, x_rows: Optional[torch.Tensor], tile_expert: torch.Tensor, tile_row0: torch.Tensor,
+             num_tiles: torch.Tensor, offsets: torch.Tensor, max_tiles: int, out: torch.Tensor, *, paired: bool, gate_limit: float = 0.0) -> None:
+    """:func:`expert_gemm_generic` in float32 for tiles of at most ``ROWS_F32_TILE`` rows, as a stream over the weights
+    (rows_f32.cu); inner sizes in steps of 4."""
+    for t, what in ((w, "expert weights"), (x, "their input"), (out, "their output")):
+        _want(t, torch.float32, what)
+    feats = w.shape[1] // 2 if paired else w.shape[1]
+    _call("frb_rows_f32", _ptr(w), _ptr(x), _ptr(x_rows), _ptr(tile_expert), _ptr(tile_row0), _ptr(num_tiles), _ptr(offsets), max_tiles,
+          _ptr(out), feats, w.shape[2], int(paired), float(gate_limit))
 
 
 def sample_rows(logits: torch.Tensor, temperature: Optional[torch.Tensor], uniform: Optional[torch.Tensor],

@@ -225,12 +225,20 @@ class RoutedExperts(FeedForward):
         return (self.dtype == torch.bfloat16 and self.hidden_size % 128 == 0 and self.expert_width % 128 == 0
                 and assignments > TENSOR_CORE_ROWS_PER_EXPERT["decode" if decode else "prompt"] * self.num_experts)
 
+    def streams_float32(self, assignments: int) -> bool:
+        """Whether the float32 stream over the weights takes the step: sizes in steps of 4 (16-byte loads), and lists of tiles
+        that fit its grid.  It is the faster kernel at any number of rows (rows_f32.cu); the general one keeps the rest."""
+        return (self.dtype == torch.float32 and ops.rows_f32_takes(self.hidden_size) and ops.rows_f32_takes(self.expert_width)
+                and assignments // ops.ROWS_F32_TILE + self.num_experts < 65535)
+
     def tile_rows(self, assignments: int, decode: bool = False) -> int:
         """Rows of one expert that one block takes: few when experts get few rows each, so that no block
         carries accumulators it does not need; enough that most experts fit one tile when they get many."""
         per_expert = assignments / self.num_experts
         if self.on_tensor_cores(assignments, decode):
             return next((t for t in (32, 64, 128, 256) if t >= 1.3 * per_expert), 256)
+        if self.streams_float32(assignments):
+            return ops.ROWS_F32_TILE
         if not self.streams():
             return TILE_ROWS
         return 8 if per_expert <= 4 else 16 if per_expert <= 12 else 32
@@ -293,10 +301,10 @@ class RoutedExperts(FeedForward):
                                 p["max_tiles"], p["tile_rows"], y, paired=False,
                                 **ops.stream_shape(tiles, self.hidden_size, self.expert_width, p["tile_rows"]))
             return y
-        ops.expert_gemm_generic(self.w13, act, sorted_token, p["tile_expert"], p["tile_row0"], p["num_tiles"],
-                                p["offsets"], p["max_tiles"], hidden, paired=True, gate_limit=limit)
-        ops.expert_gemm_generic(self.w2, hidden, None, p["tile_expert"], p["tile_row0"], p["num_tiles"], p["offsets"],
-                                p["max_tiles"], y, paired=False)
+        product = ops.rows_f32 if self.streams_float32(p["rows"]) else ops.expert_gemm_generic
+        product(self.w13, act, sorted_token, p["tile_expert"], p["tile_row0"], p["num_tiles"], p["offsets"], p["max_tiles"], hidden,
+                paired=True, gate_limit=limit)
+        product(self.w2, hidden, None, p["tile_expert"], p["tile_row0"], p["num_tiles"], p["offsets"], p["max_tiles"], y, paired=False)
         return y
 
     def route_and_plan(self, ctx, act32: torch.Tensor):

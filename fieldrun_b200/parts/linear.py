@@ -63,6 +63,12 @@ def linear(rows: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor]
     if rows.dtype == torch.float32:
         if torch.backends.cuda.matmul.allow_tf32 or torch.get_float32_matmul_precision() != "highest":
             raise RuntimeError("a float32 matrix product was asked for while TF32 is allowed")
+        if rows.shape[0] <= STREAM_ROWS and ops.rows_f32_takes(rows.shape[1]) and rows.is_contiguous() and weight.is_contiguous() \
+                and rows.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0 and (out is None or out.is_contiguous()) and len(rows):
+            tile_expert, tile_row0, num_tiles, offsets = one_tile(rows.device, rows.shape[0])
+            result = out if out is not None else torch.empty((rows.shape[0], weight.shape[0]), dtype=torch.float32, device=rows.device)
+            ops.rows_f32(weight.unsqueeze(0), rows, None, tile_expert, tile_row0, num_tiles, offsets, 1, result, paired=False)
+            return result
         with ops.timed(f"library_mm_f32[{weight.shape[0]}x{weight.shape[1]}]"):
             if out is None:
                 return torch.mm(rows, weight.t())

@@ -98,3 +98,24 @@ def test_single_tokens_in_chunks_equal_the_general_kernel(heads, kv_heads, dim, 
     part_ml = torch.full((6, heads, chunks, 2), float("nan"), device=DEV)
     ops().attention_f32_token(q, keys, values, table, pos, slots, part_o, part_ml, got, max_chunks=chunks, **common)
     check(got, want, 700)
+
+
+@pytest.mark.parametrize("paired,limit", [(True, 0.0), (True, 2.0), (False, 0.0)])
+@pytest.mark.parametrize("features,inner", [(1, 4), (7, 96), (16, 128), (17, 132), (48, 1024), (130, 3072)])
+def test_rows_equal_the_general_kernel(features, inner, paired, limit):
+    """Tiles of 1 to 8 rows, experts without rows, features and inner sizes that fill no warp or run.  Both sides round the
+    products of `inner` terms of size one: their sums differ by less than inner roundings of the largest."""
+    gen = torch.Generator(device=DEV).manual_seed(features + inner)
+    counts = [1, 0, 2, 3, 8, 5, 11]
+    offsets = np.concatenate([[0], np.cumsum(counts)])
+    total = int(offsets[-1])
+    w = torch.randn(len(counts), (2 if paired else 1) * features, inner, device=DEV, generator=gen) * inner ** -0.5
+    x = torch.randn(9, inner, device=DEV, generator=gen)
+    source = i32(np.random.default_rng(1).integers(0, 9, size=total))
+    tiles = [(e, offsets[e] + r) for e, n in enumerate(counts) for r in range(0, n, 8)]
+    lists = (i32([t[0] for t in tiles] + [0]), i32([t[1] for t in tiles] + [0]), i32([len(tiles)]), i32(offsets), len(tiles) + 1)
+    want, got = (torch.full((total, features), float("nan"), device=DEV) for _ in range(2))
+    ops().expert_gemm_generic(w, x, source, *lists, want, paired=paired, gate_limit=limit)
+    ops().rows_f32(w, x, source, *lists, got, paired=paired, gate_limit=limit)
+    assert torch.isfinite(got).all()
+    assert (got - want).abs().max() < 4 * max(inner, 16) * 2.0 ** -24 * max(want.abs().max().item(), 1.0)
