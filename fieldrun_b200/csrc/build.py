@@ -36,6 +36,7 @@ GROUPS: dict[str, tuple[str, ...]] = {
     "streams": ("experts_stream.cu", "experts_mma.cu", "rows_f32.cu"),
     "experts": ("routing.cu", "experts_generic.cu"),
     "products": ("experts_tc.cu",),
+    "products32": ("products_f32.cu",),
     "recurrent": ("gla.cu",),
     "scans": ("scans.cu",),
     "delta": ("delta_rule.cu",),

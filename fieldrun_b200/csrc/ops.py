@@ -48,6 +48,9 @@ _SIGNATURES = {
     "frb_expert_combine": "pppiiip",
     "frb_expert_gemm_generic": "ppipppppipiiiif",
     "frb_rows_f32": "pppppppipiiif",
+    "frb_weight_scales": "ppli",
+    "frb_split_rows": "pppplii" "f",
+    "frb_products_f32": "ppippl" "ppif" "ppppip" "iip",
     "frb_sample_rows": "piipppp",
     "frb_argmax_rows": "piippp",
     "frb_sample_floor": "piippppppp",
@@ -108,6 +111,7 @@ _ENTRY_GROUPS = {
     "experts": ("frb_router_topk", "frb_expert_plan", "frb_expert_combine", "frb_expert_gemm_generic", "frb_route_plan_small",
                 "frb_router_small", "frb_router_logits", "frb_scaled_rows"),
     "products": ("frb_expert_gemm_tc", "frb_gather_rows_bf16"),
+    "products32": ("frb_weight_scales", "frb_split_rows", "frb_products_f32"),
     "recurrent": ("frb_gla_scan",),
     "scans": ("frb_causal_conv", "frb_softplus_bias", "frb_selective_scan", "frb_gated_recurrence", "frb_state_space_scan", "frb_group_rms_norm",
               "frb_min_gru"),
@@ -942,6 +946,51 @@ def rows_f32(w: torch.Tensor, x: torch.Tensor, x_rows: Optional[torch.Tensor], t
           _ptr(out), feats, w.shape[2], int(paired), float(gate_limit))
 
 
+PRODUCTS_F32_TILE = 128    # rows of a tile of products_f32
+
+
+def products_f32_take(inner: int) -> bool:
+    """Whether :func:`products_f32` takes rows of this size (16-byte rows of float16; a row in shared memory)."""
+    return inner % 8 == 0 and 8 <= inner <= 32768
+
+
+def weight_scales(w: torch.Tensor) -> torch.Tensor:
+    """The power of two of every weight row (the last axis) that :func:`products_f32` splits it with, float32 [rows]."""
+    _want(w, torch.float32, "weights")
+    rows = w.numel() // w.shape[-1]
+    scale = torch.empty(rows, dtype=torch.float32, device=w.device)
+    _call("frb_weight_scales", _ptr(w), _ptr(scale), rows, w.shape[-1])
+    return scale
+
+
+def products_f32(w: torch.Tensor, w_scale: torch.Tensor, x: torch.Tensor, parts: torch.Tensor, x_scale: torch.Tensor, out: torch.Tensor, *,
+                 x_rows: Optional[torch.Tensor] = None, gated: bool = False, gate_limit: float = 0.0, lists: Optional[tuple] = None,
+                 max_tiles: int = 0) -> None:
+    """out[i] = W_e x[x_rows[i]] (x[i] without ``x_rows``) in float32 on the tensor cores (products_f32.cu).  ``w`` [E, F, K] with
+    its :func:`weight_scales`; ``parts`` (float16 [2, count, K]) and ``x_scale`` (float32 [count]) are scratch for the split rows;
+    ``gated``: the rows are silu(gate) * up of rows of x that hold K gates, then K ups (``gate_limit`` as in the other expert
+    products).  ``lists`` = (tile_expert, tile_row0, num_tiles, offsets) with tiles of ``PRODUCTS_F32_TILE`` rows, ``max_tiles``
+    at most; without lists ``w`` is one matrix for every row."""
+    for t, what in ((w, "weights"), (x, "their input"), (out, "their output"), (w_scale, "the weights' scales"), (x_scale, "the rows' scales")):
+        _want(t, torch.float32, what)
+    _want(parts, torch.float16, "the rows' parts")
+    if x_rows is not None:
+        _want(x_rows, torch.int32, "row indices")
+    experts, feats, inner = w.shape
+    count = parts.shape[1]
+    if (w_scale.numel() != experts * feats or x_scale.numel() != count or tuple(parts.shape) != (2, count, inner)
+            or x.shape[1] != inner * (2 if gated else 1) or (x_rows.numel() if x_rows is not None else x.shape[0]) != count
+            or out.numel() < count * feats):
+        raise KernelError(f"products of {list(w.shape)} weights with rows {list(x.shape)}, parts {list(parts.shape)} into {list(out.shape)}")
+    if lists is None:
+        if experts != 1:
+            raise KernelError("products without lists are of one weight matrix")
+        lists, max_tiles = (None, None, None, None), (count + PRODUCTS_F32_TILE - 1) // PRODUCTS_F32_TILE
+    _call("frb_split_rows", _ptr(x), _ptr(x_rows), _ptr(parts), _ptr(x_scale), count, inner, int(gated), float(gate_limit))
+    _call("frb_products_f32", _ptr(w), _ptr(w_scale), experts, _ptr(parts), _ptr(x_scale), count, _ptr(x), _ptr(x_rows), int(gated),
+          float(gate_limit), *(_ptr(t) for t in lists), max_tiles, _ptr(out), feats, inner, _ptr(tc_status(w.device)))
+
+
 def sample_rows(logits: torch.Tensor, temperature: Optional[torch.Tensor], uniform: Optional[torch.Tensor],
                 out: torch.Tensor, floor: Optional[torch.Tensor] = None) -> None:
     """out[r] = the largest logit of row r (the last index on ties), or where temperature[r] > 0 a sample of
@@ -1310,6 +1359,15 @@ _WAIT_CODES = {
     16: "prompt attention: the softmax waiting for the scores",
     18: "prompt attention: the correction waiting for the step before",
     19: "prompt attention: the epilogue waiting for the last steps",
+    41: "float32 products: the producer waiting for a free stage of weights",
+    42: "float32 products: the producer waiting for a free stage of rows",
+    43: "float32 products: the MMA thread waiting for the small sums to have been read",
+    44: "float32 products: the MMA thread waiting for the large sums to have been read",
+    45: "float32 products: the MMA thread waiting for the weights' parts",
+    46: "float32 products: the MMA thread waiting for a loaded stage of rows",
+    47: "float32 products: a worker waiting for finished sums",
+    48: "float32 products: a worker waiting for a loaded stage of weights",
+    49: "float32 products: a worker waiting for a free stage of parts",
     31: "attention of two maps: the producer waiting for a free key/value stage",
     32: "attention of two maps: the query tiles' copies",
     33: "attention of two maps: the MMA thread waiting for a loaded key/value stage",

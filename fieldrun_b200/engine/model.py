@@ -113,7 +113,7 @@ class DecoderModel:
         """The libraries of kernels that the model's parts launch from, each once."""
         groups: list[str] = []
         for part in self.all_parts():
-            for group in part.kernel_groups:
+            for group in part.kernel_groups + (("products32",) if self.dtype == torch.float32 else ()):      # their float32 products
                 if group not in groups:
                     groups.append(group)
         return groups

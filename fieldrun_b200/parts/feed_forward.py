@@ -41,6 +41,14 @@ TILE_ROWS = 32        # rows of one expert that a block of the expert kernels ta
 TENSOR_CORE_ROWS_PER_EXPERT = {"decode": 4.0, "prompt": 1.0}
 
 
+# Above this many rows per expert (on average) a float32 step's expert products run on the tensor cores as split products, in
+# tiles of 128 rows; up to it, and below SPLIT_WORK multiply-adds, where their two more launches cost more than they save, as a
+# stream over the weights in tiles of eight.  Measured on a B200, the whole part, microseconds, stream | split: MiniMax-M2's sizes
+# 8 rows per expert 3030 | 3155, 16 rows 4664 | 3310; 16 experts of 2048 x 2048 8 rows 224 | 243, 16 rows 335 | 255; of 1024 x
+# 1024 16 rows 153 | 149; 8 experts of 96 x 48 (2^25 multiply-adds) 384 rows 112 | 148.
+SPLIT_ROWS_PER_EXPERT = 8.0
+SPLIT_WORK = 1 << 28
+
 FUSED_ACTIVATION_ROWS = 64      # from this many rows of a prompt step on, a dense unit's first product carries its activation
 
 
@@ -122,6 +130,8 @@ class RoutedExperts(FeedForward):
         self.bias: Optional[torch.Tensor] = None
         self.w13: Optional[torch.Tensor] = None
         self.w2: Optional[torch.Tensor] = None
+        # float32: the powers of two that the split products multiply the rows of w13 and w2 with
+        self.split_scales: Optional[tuple[torch.Tensor, torch.Tensor]] = None
         self.on_route = None              # called with the picked ids [T, k] of every step (for measurements)
         # int32 [rows >= T, k] on the device, or None: when set, every step copies its picked ids into the first
         # T rows.  The copy is a device operation, so unlike ``on_route`` it also happens in a recorded step.
@@ -165,6 +175,8 @@ class RoutedExperts(FeedForward):
             self.w13[e, :i].copy_(gate)
             self.w13[e, i:].copy_(up)
             self.w2[e].copy_(down)
+        if self.dtype == torch.float32 and self.w13.is_cuda and ops.products_f32_take(d) and ops.products_f32_take(i):
+            self.split_scales = (ops.weight_scales(self.w13), ops.weight_scales(self.w2))
         if self.shared_width:
             fetched = [source.fetch(need) for need in self._shared_needs()]
             width = self.shared_width
@@ -205,7 +217,9 @@ class RoutedExperts(FeedForward):
             out = ctx.buffer("experts.logits", (tokens, self.num_experts), torch.float32)
             ops.router_logits(act32, self.router, out)
             return out
-        return linear(act32, self.router)
+        # a model in bfloat16 keeps the library's product: a router has few features, so the split product's tiles leave most of the
+        # device idle (2,048 rows of 256 features: 84 us, 76 split)
+        return linear(act32, self.router, split=self.dtype == torch.float32)
 
     def route(self, ctx, act32: torch.Tensor):
         tokens = act32.shape[0]
@@ -225,9 +239,15 @@ class RoutedExperts(FeedForward):
         return (self.dtype == torch.bfloat16 and self.hidden_size % 128 == 0 and self.expert_width % 128 == 0
                 and assignments > TENSOR_CORE_ROWS_PER_EXPERT["decode" if decode else "prompt"] * self.num_experts)
 
+    def on_split_products(self, assignments: int) -> bool:
+        """Whether a float32 step's experts run as split products on the tensor cores (products_f32.cu)."""
+        return (self.split_scales is not None and assignments > SPLIT_ROWS_PER_EXPERT * self.num_experts
+                and assignments * 3 * self.hidden_size * self.expert_width >= SPLIT_WORK and 2 * assignments < (1 << 31) - 1024)
+
     def streams_float32(self, assignments: int) -> bool:
         """Whether the float32 stream over the weights takes the step: sizes in steps of 4 (16-byte loads), and lists of tiles
-        that fit its grid.  It is the faster kernel at any number of rows (rows_f32.cu); the general one keeps the rest."""
+        that fit its grid.  It is faster than the general kernel at any number of rows (rows_f32.cu), which
+        keeps the rest."""
         return (self.dtype == torch.float32 and ops.rows_f32_takes(self.hidden_size) and ops.rows_f32_takes(self.expert_width)
                 and assignments // ops.ROWS_F32_TILE + self.num_experts < 65535)
 
@@ -237,6 +257,8 @@ class RoutedExperts(FeedForward):
         per_expert = assignments / self.num_experts
         if self.on_tensor_cores(assignments, decode):
             return next((t for t in (32, 64, 128, 256) if t >= 1.3 * per_expert), 256)
+        if self.on_split_products(assignments):
+            return ops.PRODUCTS_F32_TILE
         if self.streams_float32(assignments):
             return ops.ROWS_F32_TILE
         if not self.streams():
@@ -268,12 +290,20 @@ class RoutedExperts(FeedForward):
     def experts(self, ctx, act: torch.Tensor, p, scaled: Optional[torch.Tensor] = None) -> torch.Tensor:
         """y [N, d] float32: the output of its expert for every (token, rank), in expert-sorted order.  ``scaled``: the
         experts' input rows already in that order (each token's row times its expert's weight) instead of ``act``."""
-        hidden = ctx.buffer("experts.hidden", (p["rows"], self.expert_width), self.dtype)
         y = ctx.buffer("experts.y", (p["rows"], self.hidden_size), torch.float32)
         limit = self.gate_limit
         sorted_token = p["sorted_token"]
         if scaled is not None:
             act, sorted_token = scaled, None
+        if self.on_split_products(p["rows"]):
+            lists = dict(lists=(p["tile_expert"], p["tile_row0"], p["num_tiles"], p["offsets"]), max_tiles=p["max_tiles"])
+            both = ctx.buffer("experts.both", (p["rows"], 2 * self.expert_width), torch.float32)
+            parts = lambda width: ctx.buffer("experts.parts", (2, p["rows"], width), torch.float16)
+            scale = ctx.buffer("experts.row_scales", (p["rows"],), torch.float32)
+            ops.products_f32(self.w13, self.split_scales[0], act, parts(self.hidden_size), scale, both, x_rows=sorted_token, **lists)
+            ops.products_f32(self.w2, self.split_scales[1], both, parts(self.expert_width), scale, y, gated=True, gate_limit=limit, **lists)
+            return y
+        hidden = ctx.buffer("experts.hidden", (p["rows"], self.expert_width), self.dtype)
         if self.on_tensor_cores(p["rows"], ctx.is_decode):
             gathered = scaled
             if gathered is None:

@@ -22,6 +22,13 @@ STREAM_ROWS = 8           # up to this many rows a dense product is a stream ove
 STREAM_FEATURES = 65536   # beyond this many output features the library product is at the memory roofline anyway
 
 
+# A float32 product from this many multiply-adds on runs on the tensor cores, each operand as two float16 parts
+# (products_f32.cu).  Measured on a B200, microseconds, the library's float32 product | this one with its scales and parts:
+# 8192 x 3072 weights, 64 rows 101 | 82, 3,704 rows 3166 | 739; 3072 x 6144, 64 rows 153 | 112; 2048 x 2048,
+# 128 rows 43 | 57, 256 rows 59 | 57; 256 x 3072, 1,024 rows 62 | 73, 2,048 rows 84 | 76.
+SPLIT_PRODUCTS = 1 << 30
+
+
 def one_tile(device: torch.device, rows: int):
     key = (str(device), rows)
     if key not in _ONE_TILE:
@@ -48,8 +55,10 @@ def full_sums() -> None:
         torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = False
 
 
-def linear(rows: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None, rounded: bool = False) -> torch.Tensor:
-    """rows [T, in] @ weight[out, in]^T -> float32 [T, out]; with ``rounded`` (bfloat16 rows only) the float32 sums rounded once
+def linear(rows: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None, rounded: bool = False,
+           split: bool = True) -> torch.Tensor:
+    """rows [T, in] @ weight[out, in]^T -> float32 [T, out]; ``split``: whether a large float32 product may run as split products
+    on the tensor cores; with ``rounded`` (bfloat16 rows only) the float32 sums rounded once
     to bfloat16, for a reader that takes its operands in that type anyway."""
     if rounded:
         if rows.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or not rows.is_cuda or out is not None:
@@ -63,11 +72,18 @@ def linear(rows: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor]
     if rows.dtype == torch.float32:
         if torch.backends.cuda.matmul.allow_tf32 or torch.get_float32_matmul_precision() != "highest":
             raise RuntimeError("a float32 matrix product was asked for while TF32 is allowed")
-        if rows.shape[0] <= STREAM_ROWS and ops.rows_f32_takes(rows.shape[1]) and rows.is_contiguous() and weight.is_contiguous() \
-                and rows.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0 and (out is None or out.is_contiguous()) and len(rows):
+        plain = (rows.is_contiguous() and weight.is_contiguous() and rows.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
+                 and (out is None or out.is_contiguous()) and rows.numel() > 0)
+        if plain and rows.shape[0] <= STREAM_ROWS and ops.rows_f32_takes(rows.shape[1]):
             tile_expert, tile_row0, num_tiles, offsets = one_tile(rows.device, rows.shape[0])
             result = out if out is not None else torch.empty((rows.shape[0], weight.shape[0]), dtype=torch.float32, device=rows.device)
             ops.rows_f32(weight.unsqueeze(0), rows, None, tile_expert, tile_row0, num_tiles, offsets, 1, result, paired=False)
+            return result
+        if plain and split and rows.shape[0] * weight.numel() >= SPLIT_PRODUCTS and ops.products_f32_take(rows.shape[1]):
+            result = out if out is not None else torch.empty((rows.shape[0], weight.shape[0]), dtype=torch.float32, device=rows.device)
+            parts = torch.empty((2, *rows.shape), dtype=torch.float16, device=rows.device)
+            scale = torch.empty(rows.shape[0], dtype=torch.float32, device=rows.device)
+            ops.products_f32(weight.unsqueeze(0), ops.weight_scales(weight), rows, parts, scale, result)
             return result
         with ops.timed(f"library_mm_f32[{weight.shape[0]}x{weight.shape[1]}]"):
             if out is None:

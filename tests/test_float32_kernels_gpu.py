@@ -119,3 +119,80 @@ def test_rows_equal_the_general_kernel(features, inner, paired, limit):
     ops().rows_f32(w, x, source, *lists, got, paired=paired, gate_limit=limit)
     assert torch.isfinite(got).all()
     assert (got - want).abs().max() < 4 * max(inner, 16) * 2.0 ** -24 * max(want.abs().max().item(), 1.0)
+
+
+def split_product(w, x, lists=None, max_tiles=0, source=None, gated=False, limit=0.0):
+    """w [E, F, K] times the rows of x (of ``source``) by the tensor cores' float32 products."""
+    count = len(source) if source is not None else x.shape[0]
+    parts = torch.full((2, count, w.shape[2]), float("nan"), dtype=torch.float16, device=DEV)
+    scale, out = torch.full((count,), float("nan"), device=DEV), torch.full((count, w.shape[1]), float("nan"), device=DEV)
+    ops().products_f32(w, ops().weight_scales(w), x, parts, scale, out, x_rows=source, gated=gated, gate_limit=limit, lists=lists,
+                       max_tiles=max_tiles)
+    ops().tc_status_check(out.device)
+    return out
+
+
+def relative(got, want):
+    return ((got.double() - want).norm() / want.norm()).item()
+
+
+@pytest.mark.parametrize("rows,features,inner", [(1, 1, 8), (16, 128, 64), (17, 130, 72), (128, 256, 256), (129, 100, 264), (300, 384, 1000),
+                                                 (64, 512, 3072), (1000, 640, 6144)])
+def test_split_products_are_as_exact_as_float32(rows, features, inner):
+    """Tails of the rows, features and inner size, more items than blocks, chunks of 256 entries that end early.  The products
+    carry 22 bits, and the sums of 256 entries that are cut off are added rounded: errors of a few 2^-23 of the size that a sum of
+    entries of random signs has."""
+    gen = torch.Generator(device=DEV).manual_seed(rows + inner)
+    x = torch.randn(rows, inner, device=DEV, generator=gen) * torch.exp(3 * torch.randn(rows, 1, device=DEV, generator=gen))
+    w = torch.randn(1, features, inner, device=DEV, generator=gen) * torch.exp(3 * torch.randn(1, features, 1, device=DEV, generator=gen))
+    x[rows // 2] *= 0.0 if rows > 1 else 1.0
+    got, want = split_product(w, x), x.double() @ w[0].double().T
+    size = x.double().norm(dim=1, keepdim=True) * w[0].double().norm(dim=1)[None]
+    assert ((got.double() - want).abs() <= 8 * 2.0 ** -23 * size).all()
+
+
+@pytest.mark.parametrize("limit", [0.0, 1.5])
+def test_split_products_of_experts(limit):
+    """Expert lists: gathered rows, tiles of 1 to 128 rows, an expert without rows and one of several tiles, the gated second half."""
+    gen = torch.Generator(device=DEV).manual_seed(5)
+    counts, hidden, width = [1, 0, 130, 128, 15, 400], 96, 72
+    offsets = np.concatenate([[0], np.cumsum(counts)])
+    total = int(offsets[-1])
+    w13 = torch.randn(len(counts), 2 * width, hidden, device=DEV, generator=gen) * hidden ** -0.5
+    w2 = torch.randn(len(counts), hidden, width, device=DEV, generator=gen)
+    x = torch.randn(50, hidden, device=DEV, generator=gen)
+    source = i32(np.random.default_rng(1).integers(0, 50, size=total))
+    tiles = [(e, offsets[e] + r) for e, n in enumerate(counts) for r in range(0, n, 128)]
+    lists = (i32([t[0] for t in tiles] + [0]), i32([t[1] for t in tiles] + [0]), i32([len(tiles)]), i32(offsets))
+    both = split_product(w13, x, lists, len(tiles) + 1, source)
+    got = split_product(w2, both, lists, len(tiles) + 1, gated=True, limit=limit)
+    rows = x.double()[source.long()]
+    for e, n in enumerate(counts):
+        if n == 0:
+            continue
+        part = slice(int(offsets[e]), int(offsets[e + 1]))
+        assert relative(both[part], rows[part] @ w13[e].double().T) < 4 * 2.0 ** -23
+        gate, up = both[part].double().split(width, dim=1)
+        if limit:
+            gate = gate.clamp_max(limit)
+            unit = gate * torch.sigmoid(1.702 * gate) * (up.clamp(-limit, limit) + 1)
+        else:
+            unit = torch.nn.functional.silu(gate) * up
+        assert relative(got[part], unit @ w2[e].double().T) < 6 * 2.0 ** -23      # the unit's own rounding besides
+
+
+def test_split_products_keep_infinities_nans_and_far_exponents():
+    gen = torch.Generator(device=DEV).manual_seed(6)
+    x, w = torch.randn(140, 72, device=DEV, generator=gen), torch.randn(1, 130, 72, device=DEV, generator=gen)
+    x[3, 5], x[133, 0], x[7, 1] = float("inf"), float("nan"), 3e38
+    x[8] *= 1e-30
+    x[9] *= 1e-42
+    w[0, 129, 2], w[0, 1, 3] = -float("inf"), float("nan")
+    w[0, 4] *= 1e-20
+    w[0, 5] *= 1e30
+    got, want = split_product(w, x), torch.stack([(x[r][None] * w[0]).sum(1) for r in range(140)])
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    assert torch.equal(got[got.isinf()], want[want.isinf()])
+    fine = want.isfinite() & (want.abs() > 1e-36)                 # results that float32 holds to its full precision
+    size = x.double().abs() @ w[0].double().abs().T
+    assert ((got.double() - want.double()).abs() <= 1e-5 * size + 2e-43)[fine].all()
