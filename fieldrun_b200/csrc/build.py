@@ -37,7 +37,7 @@ GROUPS: dict[str, tuple[str, ...]] = {
     "experts": ("routing.cu", "experts_generic.cu"),
     "products": ("experts_tc.cu",),
     "products32": ("products_f32.cu",),
-    "recurrent": ("gla.cu",),
+    "recurrent": ("gla.cu", "gla_chunks.cu"),
     "scans": ("scans.cu",),
     "delta": ("delta_rule.cu",),
     "retention": ("retention.cu",),

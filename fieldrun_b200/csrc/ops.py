@@ -43,6 +43,7 @@ _SIGNATURES = {
     "frb_state_space_scan": "piiipiiipppppppllpiiiii",
     "frb_group_rms_norm": "pppiiiif",
     "frb_gla_scan": "piiiiiipipppppppiiiiiifffppppippi",
+    "frb_gla_chunks": "piiiiiipipppppppiiiiifffppppip",
     "frb_router_topk": "ppiiiifpp",
     "frb_expert_plan": "piiiippppppp",
     "frb_expert_combine": "pppiiip",
@@ -112,7 +113,7 @@ _ENTRY_GROUPS = {
                 "frb_router_small", "frb_router_logits", "frb_scaled_rows"),
     "products": ("frb_expert_gemm_tc", "frb_gather_rows_bf16"),
     "products32": ("frb_weight_scales", "frb_split_rows", "frb_products_f32"),
-    "recurrent": ("frb_gla_scan",),
+    "recurrent": ("frb_gla_scan", "frb_gla_chunks"),
     "scans": ("frb_causal_conv", "frb_softplus_bias", "frb_selective_scan", "frb_gated_recurrence", "frb_state_space_scan", "frb_group_rms_norm",
               "frb_min_gru"),
     "delta": ("frb_gated_delta_rule",),
@@ -198,7 +199,7 @@ def _stream() -> int:
 
 
 _LAUNCHES = 0
-_KERNELS_PER_CALL = {"frb_gated_delta_rule": 2, "frb_gated_recurrence": 2, "frb_sample_floor": 3, "frb_argmax_rows": 2, "frb_expert_plan": 3, "frb_attention_decode_mma": 2, "frb_attention_decode_tma": 2, "frb_attention_f32_token": 2}
+_KERNELS_PER_CALL = {"frb_gated_delta_rule": 2, "frb_gated_recurrence": 2, "frb_sample_floor": 3, "frb_argmax_rows": 2, "frb_expert_plan": 3, "frb_attention_decode_mma": 2, "frb_attention_decode_tma": 2, "frb_attention_f32_token": 2, "frb_gla_chunks": 3}
 
 
 def launches() -> int:
@@ -698,6 +699,42 @@ def gla_value_slices(dim: int, vdim: int) -> int:
 def gla_scratch_floats(items: int, heads: int, dim: int, vdim: int) -> int:
     """float32 elements of scratch that :func:`gla_scan` needs for ``items`` segments."""
     return 2 * items * heads * dim * vdim + items * heads * dim
+
+
+GLA_CHUNK_TOKENS = 64
+
+
+def gla_chunks_take(dim: int, vdim: int, rank: int, row: int, offsets: tuple) -> bool:
+    """Whether :func:`gla_chunks` takes heads of ``dim`` x ``vdim`` with a decay of ``rank`` in rows of ``row`` floats."""
+    return dim in (64, 128) and vdim in (64, 128) and rank % 4 == 0 and 4 <= rank <= 64 and not any(o % 4 for o in (row, *offsets))
+
+
+def gla_chunks_scratch_floats(chunks: int, tokens: int, heads: int, dim: int, vdim: int) -> int:
+    """float32 elements of scratch that :func:`gla_chunks` needs."""
+    return chunks * heads * dim * (vdim + 1) + tokens * heads * dim
+
+
+def gla_chunks(proj: torch.Tensor, offsets: tuple[int, int, int, int, int], a2: torch.Tensor, a2_bias: torch.Tensor,
+               norm_weight: torch.Tensor, state: torch.Tensor, seq_slot: torch.Tensor, seq_start: torch.Tensor,
+               cu_q_len: torch.Tensor, out: torch.Tensor, *, heads: int, dim: int, vdim: int, tau: float, q_scale: float,
+               eps: float, chunks: tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor], scratch: torch.Tensor) -> None:
+    """:func:`gla_scan` for prompts as matrix products (gla_chunks.cu).  ``chunks`` are segments as there, of at most
+    ``GLA_CHUNK_TOKENS`` tokens; ``scratch`` holds :func:`gla_chunks_scratch_floats` float32."""
+    for t, what in ((proj, "projected rows"), (state, "the recurrent state"), (a2_bias, "the decay's bias"),
+                    (norm_weight, "the output norm's weight"), (scratch, "scratch")):
+        _want(t, torch.float32, what)
+    if tuple(state.shape[1:]) != (2, heads, dim, vdim):
+        raise KernelError(f"the recurrent state is {list(state.shape)}, not [slots, 2, {heads}, {dim}, {vdim}]")
+    for t in chunks:
+        _want(t, torch.int32, "chunk tables")
+    count = chunks[0].numel()
+    if chunks[3].numel() != seq_slot.numel() + 1 or scratch.numel() < gla_chunks_scratch_floats(count, proj.shape[0], heads, dim, vdim):
+        raise KernelError("the chunk tables or the scratch of gated linear attention have the wrong size")
+    if a2.dtype != out.dtype:
+        raise KernelError("the decay's matrix and the outputs must have one type")
+    _call("frb_gla_chunks", _ptr(proj), proj.shape[1], *[int(o) for o in offsets], _ptr(a2), _code(a2.dtype), _ptr(a2_bias),
+          _ptr(norm_weight), _ptr(state), _ptr(seq_slot), _ptr(seq_start), _ptr(cu_q_len), _ptr(out), seq_slot.numel(), heads, dim, vdim,
+          a2.shape[1], float(tau), float(q_scale), float(eps), *(_ptr(t) for t in chunks), count, _ptr(scratch))
 
 
 NORM_MAX_SUMMED_ROWS = 32      # most weighted rows per token that the norm kernel sums itself (NORM_MAX_TOP_K)

@@ -1,0 +1,68 @@
+// Float32 products on mma.sync: each operand as two TF32 parts, hi = the entry cut to TF32 and lo = what is left, rounded to
+// TF32.  hi hi + hi lo + lo hi keeps 21 bits of every product; the sums are the tensor cores' float32 sums, which the callers
+// keep short (the adder cuts off instead of rounding: about 1e-9 of the sum with every entry).
+#pragma once
+
+#include "common.cuh"
+
+struct Tf32Parts {
+    uint32_t hi, lo;
+};
+
+// The tensor cores read the upper 19 bits of an operand.  Three full-rate instructions; with the conversion instruction (hi
+// rounded as well) the chunks of gla_chunks.cu took 525 us instead of 492.
+__device__ __forceinline__ Tf32Parts tf32_parts(float v) {
+    Tf32Parts p;
+    p.hi = __float_as_uint(v) & 0xffffe000u;
+    p.lo = __float_as_uint(v - __uint_as_float(p.hi)) + 0x1000u;         // rounded: half of the last place that is read
+    return p;
+}
+
+// C (16 x 8) += A (16 x 8) B (8 x 8).  With g = lane / 4 and t = lane % 4: a[0] = A(g, t), a[1] = A(g + 8, t), a[2] = A(g, t + 4),
+// a[3] = A(g + 8, t + 4), b[0] = B(t, g), b[1] = B(t + 4, g), c[0..1] = C(g, 2 t ..), c[2..3] = C(g + 8, 2 t ..).  The order of
+// the inner index is the caller's: here entries 2 t and 2 t + 1 of a run of eight take the places t and t + 4.
+__device__ __forceinline__ void mma_tf32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+__device__ __forceinline__ void mma_parts(float (&c)[4], const Tf32Parts (&a)[4], const Tf32Parts (&b)[2]) {
+    mma_tf32(c, a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi);
+    mma_tf32(c, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].lo, b[1].lo);
+    mma_tf32(c, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].hi, b[1].hi);
+}
+
+// Operands from shared memory.  `at` is the address of the fragment's first entry; rows of the inner index lie along the row
+// (stride = 8 modulo 32 floats: no bank conflicts) or down the column (stride = 4 modulo 16).
+__device__ __forceinline__ void a_along(Tf32Parts (&a)[4], const float* at, int stride, int lane) {
+    const float2 x = *(const float2*)(at + (lane >> 2) * stride + 2 * (lane & 3));
+    const float2 y = *(const float2*)(at + ((lane >> 2) + 8) * stride + 2 * (lane & 3));
+    a[0] = tf32_parts(x.x);
+    a[1] = tf32_parts(y.x);
+    a[2] = tf32_parts(x.y);
+    a[3] = tf32_parts(y.y);
+}
+__device__ __forceinline__ void a_down(Tf32Parts (&a)[4], const float* at, int stride, int lane) {
+    const float* x = at + 2 * (lane & 3) * stride + (lane >> 2);
+    a[0] = tf32_parts(x[0]);
+    a[1] = tf32_parts(x[8]);
+    a[2] = tf32_parts(x[stride]);
+    a[3] = tf32_parts(x[stride + 8]);
+}
+__device__ __forceinline__ void b_along(Tf32Parts (&b)[2], const float* at, int stride, int lane) {
+    const float2 x = *(const float2*)(at + (lane >> 2) * stride + 2 * (lane & 3));
+    b[0] = tf32_parts(x.x);
+    b[1] = tf32_parts(x.y);
+}
+__device__ __forceinline__ void b_down(Tf32Parts (&b)[2], const float* at, int stride, int lane) {
+    const float* x = at + 2 * (lane & 3) * stride + (lane >> 2);
+    b[0] = tf32_parts(x[0]);
+    b[1] = tf32_parts(x[stride]);
+}
+
+__device__ __forceinline__ void copy16_async(float* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }

@@ -10,8 +10,8 @@ shared by the heads, the heads side by side are multiplied by silu(G x_t), and t
 The state starts at zero (the cache zeroes a slot's state when it hands the slot out) and is carried from step
 to step in the cache line's state area, which holds two copies per slot so that a step of one token reads one
 and writes the other (see gla.cu).  q, k, v, the gate and A1 x come from one product; everything between that
-product and the output projection is one kernel in float32 (three launches of it for a long prompt, whose tokens
-are cut into segments that run side by side).
+product and the output projection is one kernel in float32 for single tokens, three for a prompt, whose tokens run in
+chunks as matrix products (gla_chunks.cu) or, at other sizes, are cut into segments that run side by side (gla.cu).
 """
 from __future__ import annotations
 
@@ -26,7 +26,11 @@ from .base import Mixer, register_part
 from .linear import linear
 
 
-SEGMENT_TOKENS = 128        # a long prompt's tokens run in segments of this many, side by side (see gla.cu)
+# From this many tokens of the longest prompt on a step runs in chunks as matrix products (gla_chunks.cu), where its sizes allow.
+# Measured on a B200, the whole part, microseconds, token by token | in chunks: one prompt of 32 tokens 70 | 90 (16 heads of
+# 128 x 128), 64 tokens 112 | 91, 1,024 tokens 371 | 140; 64 tokens with 32 heads 134 | 118, with 16 heads of 64 x 64 82 | 69.
+CHUNKED_TOKENS = 64
+SEGMENT_TOKENS = 128        # other sizes: a long prompt's tokens run in segments of this many, side by side (see gla.cu)
 
 
 class GatedLinearAttention(Mixer):
@@ -88,41 +92,45 @@ class GatedLinearAttention(Mixer):
     def cache_need(self) -> CacheNeed:
         return CacheNeed(state_shape=(2, self.num_heads, self.head_dim, self.value_dim), state_dtype="float32")
 
-    def segments(self, ctx):
-        """Tables that cut the step's prompts into segments of ``SEGMENT_TOKENS``, or None when the sequences as they
-        are give the device enough blocks (or are short).  Only a step of prompts comes here, and such a step is never
-        recorded, so the lengths may be read on the host."""
-        if ctx.is_decode or ctx.max_q_len < 2 * SEGMENT_TOKENS:
-            return None
-        if ctx.num_seqs * self.num_heads >= 2 * ops.sm_count(ctx.device):
-            return None
-        cached = getattr(ctx, "_token_segments", None)          # the same for every recurrent layer of the step
-        if cached is None:
+    def segments(self, ctx, size: int):
+        """Tables that cut the step's prompts into segments of ``size`` tokens: sequence, first token and end of each, and
+        every sequence's first segment.  Only a step of prompts comes here, and such a step is never recorded, so the lengths
+        may be read on the host."""
+        kept = ctx.__dict__.setdefault("_token_segments", {})   # the same for every recurrent layer of the step
+        if size not in kept:
             seqs, begins, ends, first = [], [], [], [0]
             for b, n in enumerate(ctx.seq_q_lens):
-                for lo in range(0, n, SEGMENT_TOKENS):
+                for lo in range(0, n, size):
                     seqs.append(b)
                     begins.append(lo)
-                    ends.append(min(lo + SEGMENT_TOKENS, n))
+                    ends.append(min(lo + size, n))
                 first.append(len(seqs))
             flat = torch.tensor(seqs + begins + ends + first, dtype=torch.int32).to(ctx.device)
             count = len(seqs)
-            cached = ctx._token_segments = (flat[:count], flat[count:2 * count], flat[2 * count:3 * count], flat[3 * count:])
-        return cached
+            kept[size] = (flat[:count], flat[count:2 * count], flat[2 * count:3 * count], flat[3 * count:])
+        return kept[size]
 
     def forward(self, ctx, act: torch.Tensor, line: LineView, writes_cache: bool) -> torch.Tensor:
         if not writes_cache:
             raise ValueError("a recurrent layer cannot read another layer's state: it has to write its own")
         proj = linear(act, self.w_in)                                       # float32 [T, 2 qk + 2 v + rank]
         out = ctx.buffer("linear_attention.out", (act.shape[0], self.v_width), self.dtype)
-        segments = self.segments(ctx)
-        scratch = None
-        if segments is not None:
+        sizes = dict(heads=self.num_heads, dim=self.head_dim, vdim=self.value_dim, tau=self.tau, q_scale=self.q_scale, eps=self.norm_eps)
+        args = (proj, self.offsets, self.w_decay, self.decay_bias, self.norm_weight, line.state, ctx.seq_slot, ctx.seq_start, ctx.cu_q_len, out)
+        if (not ctx.is_decode and ctx.max_q_len >= CHUNKED_TOKENS
+                and ops.gla_chunks_take(self.head_dim, self.value_dim, self.decay_rank, proj.shape[1], self.offsets)):
+            chunks = self.segments(ctx, ops.GLA_CHUNK_TOKENS)
+            floats = ops.gla_chunks_scratch_floats(chunks[0].numel(), act.shape[0], self.num_heads, self.head_dim, self.value_dim)
+            ops.gla_chunks(*args, chunks=chunks, scratch=ctx.buffer("linear_attention.segments", (floats,), torch.float32), **sizes)
+            return linear(out, self.w_o)
+        segments = scratch = None
+        # a long prompt whose heads give the device fewer than two blocks an SM
+        if (not ctx.is_decode and ctx.max_q_len >= 2 * SEGMENT_TOKENS
+                and ctx.num_seqs * self.num_heads < 2 * ops.sm_count(ctx.device)):
+            segments = self.segments(ctx, SEGMENT_TOKENS)
             floats = ops.gla_scratch_floats(segments[0].numel(), self.num_heads, self.head_dim, self.value_dim)
             scratch = ctx.buffer("linear_attention.segments", (floats,), torch.float32)
-        ops.gla_scan(proj, self.offsets, self.w_decay, self.decay_bias, self.norm_weight, line.state, ctx.seq_slot,
-                     ctx.seq_start, ctx.cu_q_len, out, heads=self.num_heads, dim=self.head_dim, vdim=self.value_dim,
-                     tau=self.tau, q_scale=self.q_scale, eps=self.norm_eps, segments=segments, scratch=scratch)
+        ops.gla_scan(*args, segments=segments, scratch=scratch, **sizes)
         return linear(out, self.w_o)
 
 

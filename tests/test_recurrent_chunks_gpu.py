@@ -1,0 +1,75 @@
+"""The recurrences of prompts in chunks of tokens against the same recurrences token by token."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+
+
+def ops():
+    from fieldrun_b200.csrc import ops as o
+    return o
+
+
+def i32(values):
+    return torch.tensor(np.asarray(values), dtype=torch.int32, device=DEV)
+
+
+def tables(lengths, size):
+    seqs, lo, hi, first = [], [], [], [0]
+    for b, n in enumerate(lengths):
+        for t in range(0, n, size):
+            seqs.append(b), lo.append(t), hi.append(min(t + size, n))
+        first.append(len(seqs))
+    return tuple(i32(x) for x in (seqs, lo, hi, first))
+
+
+def norm_error(got, want):
+    assert torch.isfinite(got).all()
+    return ((got.double() - want.double()).norm() / want.double().norm().clamp_min(1e-30)).item()
+
+
+# Both ways are float32 sums of the same terms; a state's decays are multiplied one after the other over the whole prompt
+# (about a rounding each: some hundred times 2^-24 for 300 tokens), or 16 and 64 at a time.
+LIMIT = 300 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("decay", ["mild", "strong", "extreme", "mixed"])
+@pytest.mark.parametrize("heads,dim,vdim,rank,dtype", [(3, 128, 128, 32, "float32"), (2, 64, 64, 16, "float32"), (2, 128, 64, 4, "float32"),
+                                                       (1, 64, 128, 64, "float32"), (3, 128, 128, 32, "bfloat16")])
+def test_gated_linear_attention_in_chunks(heads, dim, vdim, rank, dtype, decay):
+    """Chunks of 64, 16 k + r and one token, sequences that go on from a state at odd and even positions, decays of a chunk from
+    nearly one to exp(-10000)."""
+    gen = torch.Generator(device=DEV).manual_seed(dim + vdim)
+    lengths, starts, slots = [300, 64, 17, 1, 129], [0, 3, 10, 7, 64], [4, 0, 2, 1, 3]
+    tokens, width = sum(lengths), 2 * heads * (dim + vdim) + rank
+    offsets = (0, heads * dim, 2 * heads * dim, 2 * heads * dim + heads * vdim, 2 * heads * (dim + vdim))
+    kind = getattr(torch, dtype)
+    proj = torch.randn(tokens, width, device=DEV, generator=gen)
+    a2 = (torch.randn(heads * dim, rank, device=DEV, generator=gen) * 0.3).to(kind)
+    bias = torch.randn(heads * dim, device=DEV, generator=gen) + {"mild": 3.0, "strong": -20.0, "extreme": -150.0, "mixed": 0.0}[decay]
+    if decay == "mixed":
+        bias *= 20.0
+    norm = torch.randn(vdim, device=DEV, generator=gen)
+    state = torch.randn(5, 2, heads, dim, vdim, device=DEV, generator=gen)
+    sizes = dict(heads=heads, dim=dim, vdim=vdim, tau=1.0 if decay == "extreme" else 16.0, q_scale=dim ** -0.5, eps=1e-6)
+    cu = i32(np.concatenate([[0], np.cumsum(lengths)]))
+    results = []
+    for chunked in (False, True):
+        kept, out = state.clone(), torch.full((tokens, heads * vdim), float("nan"), device=DEV, dtype=kind)
+        args = (proj, offsets, a2, bias, norm, kept, i32(slots), i32(starts), cu, out)
+        if chunked:
+            assert ops().gla_chunks_take(dim, vdim, rank, width, offsets)
+            chunks = tables(lengths, 64)
+            scratch = torch.full((ops().gla_chunks_scratch_floats(chunks[0].numel(), tokens, heads, dim, vdim),), float("nan"), device=DEV)
+            ops().gla_chunks(*args, chunks=chunks, scratch=scratch, **sizes)
+        else:
+            ops().gla_scan(*args, **sizes)
+        results.append((out, kept))
+    assert norm_error(results[1][0].float(), results[0][0].float()) < (LIMIT if dtype == "float32" else 2.0 ** -9)
+    for n, start, slot in zip(lengths, starts, slots):
+        assert norm_error(results[1][1][slot, (start + n) & 1], results[0][1][slot, (start + n) & 1]) < LIMIT
+        if n % 2:
+            assert torch.equal(results[1][1][slot, start & 1], state[slot, start & 1])       # the copy it began from is left alone
