@@ -73,3 +73,35 @@ def test_gated_linear_attention_in_chunks(heads, dim, vdim, rank, dtype, decay):
         assert norm_error(results[1][1][slot, (start + n) & 1], results[0][1][slot, (start + n) & 1]) < LIMIT
         if n % 2:
             assert torch.equal(results[1][1][slot, start & 1], state[slot, start & 1])       # the copy it began from is left alone
+
+
+class Tables:
+    def __init__(self, lengths, starts, slots):
+        self.num_seqs, self.max_q_len = len(lengths), max(lengths)
+        self.seq_slot, self.seq_start = i32(slots), i32(starts)
+        self.cu_q_len = i32(np.concatenate([[0], np.cumsum(lengths)]))
+        self.tok_seq = i32(np.repeat(np.arange(len(lengths)), lengths))
+
+
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("channels,typed,biased", [(4, True, True), (520, False, True), (1028, True, False)])
+def test_convolution_of_four_channels_a_thread_equals_one_channel_a_thread(taps, channels, typed, biased):
+    """Sequences that end inside a run of eight rows, and shorter ones than the window; the same sums in the same order."""
+    gen = torch.Generator(device=DEV).manual_seed(channels)
+    lengths, starts, slots = [77, 1, 2, 3, 60, 8], [0, 5, 4, 7, 2, 0], [5, 3, 1, 0, 2, 4]
+    tokens = sum(lengths)
+    rows = torch.randn(tokens, channels, device=DEV, generator=gen)
+    weights, bias, in_bias = (torch.randn(*shape, device=DEV, generator=gen) for shape in ((channels, taps), (channels,), (channels,)))
+    results = []
+    for offset in (4, 3):                                        # 3: the rows do not begin on 16 bytes
+        shifted = torch.zeros(tokens, channels + 8, device=DEV)
+        shifted[:, offset:offset + channels] = rows
+        state = torch.ones(6, 2, (taps - 1) * channels, device=DEV)
+        out32 = torch.full((tokens, channels), float("nan"), device=DEV)
+        out = torch.zeros(tokens, channels, device=DEV, dtype=torch.bfloat16) if typed else None
+        ops().causal_conv(shifted, offset, channels, weights, bias if biased else None, Tables(lengths, starts, slots), state, 0, out32, out,
+                          in_bias=in_bias if biased else None, activation="silu")
+        results.append((out32, state, out))
+    assert torch.isfinite(results[0][0]).all()
+    for a, b in zip(*results):
+        assert a is None or torch.equal(a, b)
