@@ -38,7 +38,7 @@ GROUPS: dict[str, tuple[str, ...]] = {
     "products": ("experts_tc.cu",),
     "products32": ("products_f32.cu",),
     "recurrent": ("gla.cu", "gla_chunks.cu"),
-    "scans": ("scans.cu",),
+    "scans": ("scans.cu", "state_space_chunks.cu"),
     "delta": ("delta_rule.cu",),
     "retention": ("retention.cu",),
     "copies": ("stream_copies.cu",),

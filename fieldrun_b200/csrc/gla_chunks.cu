@@ -11,7 +11,7 @@
 // at most one each; within a block the 136 pairs run as the recurrence does, w k_j multiplied by one decay after the other.
 //
 // Everything is float32; the products run on tensor cores with each operand as two TF32 parts (tf32_parts.cuh), over inner
-// sizes of at most 192 entries.  Four prompts of 2,048 tokens, 16 heads of 128 x 128: 0.49 ms (0.19 + 0.04 + 0.27; gla.cu 1.66 ms
+// sizes of at most 192 entries.  Four prompts of 2,048 tokens, 16 heads of 128 x 128: 0.48 ms (0.19 + 0.04 + 0.26; gla.cu 1.66 ms
 // in segments of 128, whose 500 instructions a warp and token run one after the other).  What bounds them: the instructions around
 // the products (60 and 50 % of the issue slots; a decay's two exponentials and a logarithm, the parts, the block's own pairs),
 // with two blocks an SM to hide the rows' way in; with q, k and v loaded where they are used 0.68 ms.
@@ -129,15 +129,12 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_states_kernel(GlaChun
         float acc[2][4][4] = {};
 #pragma unroll 2
         for (int j = 0; j < GC_TOKENS; j += 8) {
-            Tf32Parts a[2][4], bb[2];
+            Tf32Parts a[2][4], bb[4][2];
 #pragma unroll
             for (int m = 0; m < 2; ++m) a_down(a[m], k_s + j * LK + c0 + 16 * m, LK, lane);
 #pragma unroll
-            for (int n = 0; n < 4; ++n) {
-                b_down(bb, v_s + j * LV + v0 + 8 * n, LV, lane);
-#pragma unroll
-                for (int m = 0; m < 2; ++m) mma_parts(acc[m][n], a[m], bb);
-            }
+            for (int n = 0; n < 4; ++n) b_down(bb[n], v_s + j * LV + v0 + 8 * n, LV, lane);
+            mma_tiles<2, 4, 4>(acc, 0, a, bb);
         }
 #pragma unroll
         for (int m = 0; m < 2; ++m)
@@ -159,18 +156,18 @@ gla_chunk_scan_kernel(GlaChunks p, int dim, int vdim) {
     const int start = p.seq_start[b], n = p.cu_q_len[b + 1] - p.cu_q_len[b];
     float* kept = p.state + ((size_t)p.seq_slot[b] * 2 * p.heads + h) * elements + e;
     float4 S = *(const float4*)(kept + (size_t)(start & 1) * p.heads * elements);
-    for (int s0 = first; s0 < last; s0 += 4) {
-        float4 u[4];
-        float decay[4];
+    for (int s0 = first; s0 < last; s0 += 8) {                  // eight chunks' loads on their way at once
+        float4 u[8];
+        float decay[8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 8; ++i)
             if (s0 + i < last) {
                 const size_t at = (size_t)(s0 + i) * p.heads + h;
                 u[i] = *(const float4*)(p.states + at * elements + e);
                 decay[i] = p.decays[at * dim + d];
             }
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 8; ++i)
             if (s0 + i < last) {
                 *(float4*)(p.states + ((size_t)(s0 + i) * p.heads + h) * elements + e) = S;
                 S.x = fmaf(decay[i], S.x, u[i].x);
@@ -319,15 +316,12 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_outputs_kernel(GlaChu
         if (works)
 #pragma unroll
             for (int k0 = 0; k0 < 32; k0 += 8) {
-                Tf32Parts a[2][4], bb[2];
+                Tf32Parts a[2][4], bb[4][2];
 #pragma unroll
                 for (int m = 0; m < 2; ++m) a_along(a[m], q_s + tiles[m] * 16 * LQ + c0 + k0, LQ, lane);
 #pragma unroll
-                for (int n = 0; n < 4; ++n) {
-                    b_down(bb, slab + k0 * LV + v0 + 8 * n, LV, lane);
-#pragma unroll
-                    for (int m = 0; m < 2; ++m) mma_parts(acc[m][n], a[m], bb);
-                }
+                for (int n = 0; n < 4; ++n) b_down(bb[n], slab + k0 * LV + v0 + 8 * n, LV, lane);
+                mma_tiles<2, 4, 4>(acc, 0, a, bb);
             }
     };
     copies_wait<2>();
@@ -368,13 +362,11 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_outputs_kernel(GlaChu
 #pragma unroll
         for (int m = 0; m < 2; ++m)
             for (int j = 0; j < (tiles[m] + 1) * GC_BLOCK; j += 8) {
-                Tf32Parts a[4], bb[2];
-                a_along(a, a_s + tiles[m] * 16 * LA + j, LA, lane);
+                Tf32Parts a[1][4], bb[4][2];
+                a_along(a[0], a_s + tiles[m] * 16 * LA + j, LA, lane);
 #pragma unroll
-                for (int n = 0; n < 4; ++n) {
-                    b_down(bb, v_s + j * LV + v0 + 8 * n, LV, lane);
-                    mma_parts(acc[m][n], a, bb);
-                }
+                for (int n = 0; n < 4; ++n) b_down(bb[n], v_s + j * LV + v0 + 8 * n, LV, lane);
+                mma_tiles<1, 4, 4>(reinterpret_cast<float (&)[1][4][4]>(acc[m]), 0, a, bb);
             }
 
     // the head's root mean square over the warps' columns, weight and gate

@@ -41,6 +41,7 @@ _SIGNATURES = {
     "frb_softplus_bias": "ppii",
     "frb_gated_recurrence": "piipppppppppppllpiiiiif",
     "frb_state_space_scan": "piiipiiipppppppllpiiiii",
+    "frb_state_space_chunks": "piiipiii" "ppp" "ppp" "pll" "piiiii" "ppppip",
     "frb_group_rms_norm": "pppiiiif",
     "frb_gla_scan": "piiiiiipipppppppiiiiiifffppppippi",
     "frb_gla_chunks": "piiiiiipipppppppiiiiifffppppip",
@@ -114,7 +115,7 @@ _ENTRY_GROUPS = {
     "products": ("frb_expert_gemm_tc", "frb_gather_rows_bf16"),
     "products32": ("frb_weight_scales", "frb_split_rows", "frb_products_f32"),
     "recurrent": ("frb_gla_scan", "frb_gla_chunks"),
-    "scans": ("frb_causal_conv", "frb_softplus_bias", "frb_selective_scan", "frb_gated_recurrence", "frb_state_space_scan", "frb_group_rms_norm",
+    "scans": ("frb_causal_conv", "frb_softplus_bias", "frb_selective_scan", "frb_gated_recurrence", "frb_state_space_scan", "frb_state_space_chunks", "frb_group_rms_norm",
               "frb_min_gru"),
     "delta": ("frb_gated_delta_rule",),
     "retention": ("frb_retention",),
@@ -199,7 +200,7 @@ def _stream() -> int:
 
 
 _LAUNCHES = 0
-_KERNELS_PER_CALL = {"frb_gated_delta_rule": 2, "frb_gated_recurrence": 2, "frb_sample_floor": 3, "frb_argmax_rows": 2, "frb_expert_plan": 3, "frb_attention_decode_mma": 2, "frb_attention_decode_tma": 2, "frb_attention_f32_token": 2, "frb_gla_chunks": 3}
+_KERNELS_PER_CALL = {"frb_gated_delta_rule": 2, "frb_gated_recurrence": 2, "frb_sample_floor": 3, "frb_argmax_rows": 2, "frb_expert_plan": 3, "frb_attention_decode_mma": 2, "frb_attention_decode_tma": 2, "frb_attention_f32_token": 2, "frb_gla_chunks": 3, "frb_state_space_chunks": 4}
 
 
 def launches() -> int:
@@ -675,6 +676,41 @@ def state_space_scan(proj: torch.Tensor, z_offset: int, dt_offset: int, xbc: tor
     _call("frb_state_space_scan", _ptr(proj), proj.shape[1], int(z_offset), int(dt_offset), _ptr(xbc), xbc.shape[1],
           int(b_offset), int(c_offset), _ptr(dt_bias), _ptr(a_log), _ptr(d), _ptr(ctx.seq_slot), _ptr(ctx.seq_start),
           _ptr(ctx.cu_q_len), *_state_place(state, state_offset), _ptr(out), ctx.num_seqs, heads, vdim, n, groups)
+
+
+STATE_SPACE_CHUNK_TOKENS = 128
+
+
+def state_space_chunks_take(heads: int, vdim: int, n: int, groups: int, z_offset: int, row: int, xbc_offsets: tuple, state: torch.Tensor,
+                            state_offset: int) -> bool:
+    """Whether :func:`state_space_chunks` takes ``heads`` of ``n`` x ``vdim`` in ``groups``: tiles of 128 columns inside a group, and
+    rows (``row`` floats of the projection, ``xbc_offsets`` and the state's place) that begin where its loads need them to."""
+    return (n in (64, 128) and vdim in (64, 128) and heads // groups * vdim % 128 == 0 and row % 2 == 0 and z_offset % 2 == 0
+            and not any(o % 4 for o in (*xbc_offsets, state.shape[2], state_offset)))
+
+
+def state_space_chunks_scratch_floats(chunks: int, heads: int, vdim: int, n: int, groups: int) -> int:
+    """float32 elements of scratch that :func:`state_space_chunks` needs."""
+    return chunks * (heads * n * vdim + groups * STATE_SPACE_CHUNK_TOKENS ** 2 + heads)
+
+
+def state_space_chunks(proj: torch.Tensor, z_offset: int, dt_offset: int, xbc: torch.Tensor, b_offset: int, c_offset: int,
+                       dt_bias: torch.Tensor, a_log: torch.Tensor, d: torch.Tensor, ctx, state: torch.Tensor, state_offset: int,
+                       out: torch.Tensor, *, heads: int, vdim: int, n: int, groups: int, chunks: tuple, scratch: torch.Tensor) -> None:
+    """:func:`state_space_scan` for prompts as matrix products (state_space_chunks.cu).  ``chunks`` = (sequence, first token, end
+    token of every chunk of at most ``STATE_SPACE_CHUNK_TOKENS``; first chunk of every sequence and, last, their number);
+    ``scratch`` holds :func:`state_space_chunks_scratch_floats` float32."""
+    for t in (proj, xbc, dt_bias, a_log, d, out, scratch):
+        _want(t, torch.float32, "state_space_chunks' operands")
+    for t in chunks:
+        _want(t, torch.int32, "chunk tables")
+    count = chunks[0].numel()
+    if chunks[3].numel() != ctx.num_seqs + 1 or scratch.numel() < state_space_chunks_scratch_floats(count, heads, vdim, n, groups):
+        raise KernelError("the chunk tables or the scratch of the state-space chunks have the wrong size")
+    _call("frb_state_space_chunks", _ptr(proj), proj.shape[1], int(z_offset), int(dt_offset), _ptr(xbc), xbc.shape[1], int(b_offset),
+          int(c_offset), _ptr(dt_bias), _ptr(a_log), _ptr(d), _ptr(ctx.seq_slot), _ptr(ctx.seq_start), _ptr(ctx.cu_q_len),
+          *_state_place(state, state_offset), _ptr(out), ctx.num_seqs, heads, vdim, n, groups, *(_ptr(t) for t in chunks), count,
+          _ptr(scratch))
 
 
 def group_rms_norm(rows_in: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, norm_groups: int, eps: float) -> None:

@@ -22,11 +22,27 @@ __device__ __forceinline__ Tf32Parts tf32_parts(float v) {
 // a[3] = A(g + 8, t + 4), b[0] = B(t, g), b[1] = B(t + 4, g), c[0..1] = C(g, 2 t ..), c[2..3] = C(g + 8, 2 t ..).  The order of
 // the inner index is the caller's: here entries 2 t and 2 t + 1 of a run of eight take the places t and t + 4.
 __device__ __forceinline__ void mma_tf32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// The products of M row tiles with NN column tiles.  The three products of a tile's parts depend on one another through its
+// accumulators: one part of all tiles after the other leaves every product M NN places to finish.
+template <int M, int NN, int NA>
+__device__ __forceinline__ void mma_tiles(float (&c)[M][NA][4], int n0, const Tf32Parts (&a)[M][4], const Tf32Parts (&b)[NN][2]) {
+#pragma unroll
+    for (int n = 0; n < NN; ++n)
+#pragma unroll
+        for (int m = 0; m < M; ++m) mma_tf32(c[m][n0 + n], a[m][0].lo, a[m][1].lo, a[m][2].lo, a[m][3].lo, b[n][0].hi, b[n][1].hi);
+#pragma unroll
+    for (int n = 0; n < NN; ++n)
+#pragma unroll
+        for (int m = 0; m < M; ++m) mma_tf32(c[m][n0 + n], a[m][0].hi, a[m][1].hi, a[m][2].hi, a[m][3].hi, b[n][0].lo, b[n][1].lo);
+#pragma unroll
+    for (int n = 0; n < NN; ++n)
+#pragma unroll
+        for (int m = 0; m < M; ++m) mma_tf32(c[m][n0 + n], a[m][0].hi, a[m][1].hi, a[m][2].hi, a[m][3].hi, b[n][0].hi, b[n][1].hi);
+}
 __device__ __forceinline__ void mma_parts(float (&c)[4], const Tf32Parts (&a)[4], const Tf32Parts (&b)[2]) {
     mma_tf32(c, a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi);
     mma_tf32(c, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].lo, b[1].lo);

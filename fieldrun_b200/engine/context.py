@@ -147,6 +147,24 @@ class StepContext:
     def buffer(self, name: str, shape: Sequence[int], dtype: torch.dtype) -> torch.Tensor:
         return self.workspace.buffer(name, shape, dtype)
 
+    def token_chunks(self, size: int) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
+        """The step's new tokens in chunks of at most ``size``: sequence, first token and end (among the sequence's new tokens) of
+        each, and every sequence's first chunk with, last, their number; int32 on the device.  For steps of prompts only: the
+        lengths are read on the host."""
+        kept = self.__dict__.setdefault("_token_chunks", {})
+        if size not in kept:
+            seqs, begins, ends, first = [], [], [], [0]
+            for b, n in enumerate(self.seq_q_lens):
+                for lo in range(0, n, size):
+                    seqs.append(b)
+                    begins.append(lo)
+                    ends.append(min(lo + size, n))
+                first.append(len(seqs))
+            flat = torch.tensor(seqs + begins + ends + first, dtype=torch.int32).to(self.device)
+            count = len(seqs)
+            kept[size] = (flat[:count], flat[count:2 * count], flat[2 * count:3 * count], flat[3 * count:])
+        return kept[size]
+
     def query_tiles(self, rows: int) -> tuple[torch.Tensor, torch.Tensor]:
         """Tiles of ``rows`` consecutive new tokens that never span two sequences: (sequence of each tile,
         first row of each tile among its sequence's new tokens), on the device."""

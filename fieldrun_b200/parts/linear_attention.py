@@ -92,24 +92,6 @@ class GatedLinearAttention(Mixer):
     def cache_need(self) -> CacheNeed:
         return CacheNeed(state_shape=(2, self.num_heads, self.head_dim, self.value_dim), state_dtype="float32")
 
-    def segments(self, ctx, size: int):
-        """Tables that cut the step's prompts into segments of ``size`` tokens: sequence, first token and end of each, and
-        every sequence's first segment.  Only a step of prompts comes here, and such a step is never recorded, so the lengths
-        may be read on the host."""
-        kept = ctx.__dict__.setdefault("_token_segments", {})   # the same for every recurrent layer of the step
-        if size not in kept:
-            seqs, begins, ends, first = [], [], [], [0]
-            for b, n in enumerate(ctx.seq_q_lens):
-                for lo in range(0, n, size):
-                    seqs.append(b)
-                    begins.append(lo)
-                    ends.append(min(lo + size, n))
-                first.append(len(seqs))
-            flat = torch.tensor(seqs + begins + ends + first, dtype=torch.int32).to(ctx.device)
-            count = len(seqs)
-            kept[size] = (flat[:count], flat[count:2 * count], flat[2 * count:3 * count], flat[3 * count:])
-        return kept[size]
-
     def forward(self, ctx, act: torch.Tensor, line: LineView, writes_cache: bool) -> torch.Tensor:
         if not writes_cache:
             raise ValueError("a recurrent layer cannot read another layer's state: it has to write its own")
@@ -119,7 +101,7 @@ class GatedLinearAttention(Mixer):
         args = (proj, self.offsets, self.w_decay, self.decay_bias, self.norm_weight, line.state, ctx.seq_slot, ctx.seq_start, ctx.cu_q_len, out)
         if (not ctx.is_decode and ctx.max_q_len >= CHUNKED_TOKENS
                 and ops.gla_chunks_take(self.head_dim, self.value_dim, self.decay_rank, proj.shape[1], self.offsets)):
-            chunks = self.segments(ctx, ops.GLA_CHUNK_TOKENS)
+            chunks = ctx.token_chunks(ops.GLA_CHUNK_TOKENS)
             floats = ops.gla_chunks_scratch_floats(chunks[0].numel(), act.shape[0], self.num_heads, self.head_dim, self.value_dim)
             ops.gla_chunks(*args, chunks=chunks, scratch=ctx.buffer("linear_attention.segments", (floats,), torch.float32), **sizes)
             return linear(out, self.w_o)
@@ -127,7 +109,7 @@ class GatedLinearAttention(Mixer):
         # a long prompt whose heads give the device fewer than two blocks an SM
         if (not ctx.is_decode and ctx.max_q_len >= 2 * SEGMENT_TOKENS
                 and ctx.num_seqs * self.num_heads < 2 * ops.sm_count(ctx.device)):
-            segments = self.segments(ctx, SEGMENT_TOKENS)
+            segments = ctx.token_chunks(SEGMENT_TOKENS)
             floats = ops.gla_scratch_floats(segments[0].numel(), self.num_heads, self.head_dim, self.value_dim)
             scratch = ctx.buffer("linear_attention.segments", (floats,), torch.float32)
         ops.gla_scan(*args, segments=segments, scratch=scratch, **sizes)

@@ -35,6 +35,12 @@ from .base import Mixer, register_part
 from .linear import linear
 
 
+# From this many tokens of the longest prompt on a step's recurrence runs in chunks as matrix products, where its sizes allow
+# (state_space_chunks.cu).  Measured on a B200, the whole part, microseconds, token by token | in chunks: one prompt of 96 tokens 106 |
+# 135 (64 heads of 128 x 64), 128 tokens 112 | 98, 1,024 tokens 702 | 216; 128 tokens with 32 heads 93 | 91, with 128 heads 159 | 146.
+STATE_SPACE_CHUNKED_TOKENS = 128
+
+
 class _StateMixer(Mixer):
     replayable = True
     kernel_groups = ("common", "streams", "scans")
@@ -210,8 +216,16 @@ class ScalarDecayStateSpace(_StateMixer):
         ops.causal_conv(proj, c, self.conv_channels, w["conv"], w["conv_bias"], ctx, line.state, self.state_floats, xbc,
                         activation="silu")
         y = ctx.buffer("state_space.y", (rows, c), torch.float32)
-        ops.state_space_scan(proj, 0, c + self.conv_channels, xbc, c, c + gn, w["dt_bias"], w["a_log"], w["d"], ctx, line.state,
-                             0, y, heads=self.num_heads, vdim=self.value_dim, n=self.state, groups=self.groups)
+        sizes = dict(heads=self.num_heads, vdim=self.value_dim, n=self.state, groups=self.groups)
+        args = (proj, 0, c + self.conv_channels, xbc, c, c + gn, w["dt_bias"], w["a_log"], w["d"], ctx, line.state, 0, y)
+        if (not ctx.is_decode and ctx.max_q_len >= STATE_SPACE_CHUNKED_TOKENS
+                and ops.state_space_chunks_take(z_offset=0, row=proj.shape[1], xbc_offsets=(self.conv_channels, c, c + gn), state=line.state,
+                                                state_offset=0, **sizes)):
+            chunks = ctx.token_chunks(ops.STATE_SPACE_CHUNK_TOKENS)
+            floats = ops.state_space_chunks_scratch_floats(chunks[0].numel(), **sizes)
+            ops.state_space_chunks(*args, chunks=chunks, scratch=ctx.buffer("state_space.chunks", (floats,), torch.float32), **sizes)
+        else:
+            ops.state_space_scan(*args, **sizes)
         out = ctx.buffer("state_space.out", (rows, c), self.dtype)
         ops.group_rms_norm(y, w["norm"], out, self.norm_groups, self.norm_eps)
         return linear(out, w["o_proj"])

@@ -105,3 +105,40 @@ def test_convolution_of_four_channels_a_thread_equals_one_channel_a_thread(taps,
     assert torch.isfinite(results[0][0]).all()
     for a, b in zip(*results):
         assert a is None or torch.equal(a, b)
+
+
+@pytest.mark.parametrize("decay", ["mild", "strong", "extreme", "mixed"])
+@pytest.mark.parametrize("heads,groups,n,vdim", [(4, 2, 128, 64), (2, 1, 64, 64), (2, 2, 128, 128), (3, 1, 64, 128)])
+def test_state_space_in_chunks(heads, groups, n, vdim, decay):
+    """Chunks of 128, 16 k + r and one token, sequences that go on from a state at odd and even positions, decays of a token from
+    nearly one to exp(-50)."""
+    gen = torch.Generator(device=DEV).manual_seed(n + vdim + heads)
+    lengths, starts, slots = [300, 128, 17, 1, 257], [0, 3, 10, 7, 64], [4, 0, 2, 1, 3]
+    tokens, inner = sum(lengths), heads * vdim
+    proj = torch.randn(tokens, inner + heads + heads % 2, device=DEV, generator=gen)
+    proj[:, inner:] += {"mild": -4.0, "strong": 2.0, "extreme": 8.0, "mixed": 0.0}[decay]
+    if decay == "mixed":
+        proj[:, inner:] *= 5.0
+    xbc = torch.randn(tokens, inner + 2 * groups * n, device=DEV, generator=gen) * 0.3
+    dt_bias, a_log, d = torch.randn(heads, device=DEV, generator=gen) * 0.2, torch.randn(heads, device=DEV, generator=gen) * 0.5, torch.ones(heads, device=DEV)
+    state = torch.randn(5, 2, 4 + heads * n * vdim + 8, device=DEV, generator=gen)
+    sizes = dict(heads=heads, vdim=vdim, n=n, groups=groups)
+    tabs = Tables(lengths, starts, slots)
+    results = []
+    for chunked in (False, True):
+        kept, out = state.clone(), torch.full((tokens, inner), float("nan"), device=DEV)
+        args = (proj, 0, inner, xbc, inner, inner + groups * n, dt_bias, a_log, d, tabs, kept, 4, out)
+        if chunked:
+            assert ops().state_space_chunks_take(z_offset=0, row=proj.shape[1], xbc_offsets=(xbc.shape[1], inner), state=kept, state_offset=4, **sizes)
+            chunks = tables(lengths, 128)
+            scratch = torch.full((ops().state_space_chunks_scratch_floats(chunks[0].numel(), **sizes),), float("nan"), device=DEV)
+            ops().state_space_chunks(*args, chunks=chunks, scratch=scratch, **sizes)
+        else:
+            ops().state_space_scan(*args, **sizes)
+        results.append((out, kept))
+    assert norm_error(results[1][0], results[0][0]) < LIMIT
+    for length, start, slot in zip(lengths, starts, slots):
+        copy = (start + length) & 1
+        assert norm_error(results[1][1][slot, copy, 4:-8], results[0][1][slot, copy, 4:-8]) < LIMIT
+        results[1][1][slot, copy, 4:-8] = state[slot, copy, 4:-8]
+    assert torch.equal(results[1][1], state)                     # nothing else was written
