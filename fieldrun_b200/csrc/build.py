@@ -39,7 +39,7 @@ GROUPS: dict[str, tuple[str, ...]] = {
     "products32": ("products_f32.cu",),
     "recurrent": ("gla.cu", "gla_chunks.cu"),
     "scans": ("scans.cu", "state_space_chunks.cu"),
-    "delta": ("delta_rule.cu",),
+    "delta": ("delta_rule.cu", "delta_chunks.cu"),
     "retention": ("retention.cu",),
     "copies": ("stream_copies.cu",),
     "latent": ("latent_attention.cu", "latent_attention_tc.cu"),

@@ -60,6 +60,7 @@ _SIGNATURES = {
     "frb_weighted_pair": "ppplff",
     "frb_sandwich_norm": "pppffpppippfpfiipipi",
     "frb_gated_delta_rule": "piiii" "piiii" "ppp" "ppp" "pll" "pi" "pii" "iiiii" "f",
+    "frb_delta_chunks": "piiii" "piiii" "ppp" "ppp" "pll" "pip" "iiiiiif" "ppppip",
     "frb_attention_decode_mma": "ppppipppppiiiifiippipf" "iiipff",
     "frb_attention_prefill_mma": "ppppippipppppiiifipipf" "iiii",
     "frb_attention_decode_tma": "pppipipppppiiiifiiippipf" "iiipff",
@@ -117,7 +118,7 @@ _ENTRY_GROUPS = {
     "recurrent": ("frb_gla_scan", "frb_gla_chunks"),
     "scans": ("frb_causal_conv", "frb_softplus_bias", "frb_selective_scan", "frb_gated_recurrence", "frb_state_space_scan", "frb_state_space_chunks", "frb_group_rms_norm",
               "frb_min_gru"),
-    "delta": ("frb_gated_delta_rule",),
+    "delta": ("frb_gated_delta_rule", "frb_delta_chunks"),
     "retention": ("frb_retention",),
     "copies": ("frb_stream_copies",),
     "extras": ("frb_wait_probe",),
@@ -200,7 +201,7 @@ def _stream() -> int:
 
 
 _LAUNCHES = 0
-_KERNELS_PER_CALL = {"frb_gated_delta_rule": 2, "frb_gated_recurrence": 2, "frb_sample_floor": 3, "frb_argmax_rows": 2, "frb_expert_plan": 3, "frb_attention_decode_mma": 2, "frb_attention_decode_tma": 2, "frb_attention_f32_token": 2, "frb_gla_chunks": 3, "frb_state_space_chunks": 4}
+_KERNELS_PER_CALL = {"frb_gated_delta_rule": 2, "frb_gated_recurrence": 2, "frb_sample_floor": 3, "frb_argmax_rows": 2, "frb_expert_plan": 3, "frb_attention_decode_mma": 2, "frb_attention_decode_tma": 2, "frb_attention_f32_token": 2, "frb_gla_chunks": 3, "frb_state_space_chunks": 4, "frb_delta_chunks": 3}
 
 
 def launches() -> int:
@@ -1199,6 +1200,41 @@ def gated_delta_rule(conv: torch.Tensor, q_off: int, k_off: int, v_off: int, pro
           int(b_off), int(a_off), int(g_off), _ptr(a_log), _ptr(dt_bias), _ptr(norm), _ptr(ctx.seq_slot), _ptr(ctx.seq_start),
           _ptr(ctx.cu_q_len), *_state_place(state, state_offset), _ptr(out), _code(out.dtype), _ptr(raw), conv.shape[0], int(slices or 0),
           ctx.num_seqs, int(heads), int(kv_heads), int(dim), int(vdim), float(eps))
+
+
+DELTA_CHUNK_TOKENS = 64
+
+
+def delta_chunks_take(dim: int, vdim: int, conv_offsets: tuple, state: torch.Tensor, state_offset: int) -> bool:
+    """Whether :func:`delta_chunks` takes heads of ``dim`` x ``vdim`` in rows that begin where its loads need them to."""
+    return (dim in (64, 128) and vdim in (64, 128) and not any(o % 4 for o in conv_offsets) and state.shape[2] % 2 == 0
+            and state_offset % 2 == 0)
+
+
+def delta_chunks_scratch_floats(chunks: int, heads: int, dim: int, vdim: int) -> int:
+    """float32 elements of scratch that :func:`delta_chunks` needs."""
+    return chunks * heads * (DELTA_CHUNK_TOKENS * (dim + vdim + DELTA_CHUNK_TOKENS + 2) + 4)
+
+
+def delta_chunks(conv: torch.Tensor, q_off: int, k_off: int, v_off: int, proj: torch.Tensor, b_off: int, a_off: int, g_off: int,
+                 a_log: torch.Tensor, dt_bias: torch.Tensor, norm: torch.Tensor, ctx, state: torch.Tensor, state_offset: int,
+                 out: torch.Tensor, *, heads: int, kv_heads: int, dim: int, vdim: int, eps: float, raw: torch.Tensor, chunks: tuple,
+                 scratch: torch.Tensor) -> None:
+    """:func:`gated_delta_rule` for prompts as matrix products (delta_chunks.cu).  ``chunks`` = (sequence, first token, end token of
+    every chunk of at most ``DELTA_CHUNK_TOKENS``; first chunk of every sequence and, last, their number); ``scratch`` holds
+    :func:`delta_chunks_scratch_floats` float32."""
+    for t in (conv, proj, a_log, dt_bias, norm, raw, scratch):
+        _want(t, torch.float32, "delta_chunks' operands")
+    for t in chunks:
+        _want(t, torch.int32, "chunk tables")
+    count = chunks[0].numel()
+    if (chunks[3].numel() != ctx.num_seqs + 1 or scratch.numel() < delta_chunks_scratch_floats(count, heads, dim, vdim)
+            or raw.numel() < out.numel()):
+        raise KernelError("the chunk tables, the scratch or the unnormed outputs of the delta rule's chunks have the wrong size")
+    _call("frb_delta_chunks", _ptr(conv), conv.shape[1], int(q_off), int(k_off), int(v_off), _ptr(proj), proj.shape[1], int(b_off),
+          int(a_off), int(g_off), _ptr(a_log), _ptr(dt_bias), _ptr(norm), _ptr(ctx.seq_slot), _ptr(ctx.seq_start), _ptr(ctx.cu_q_len),
+          *_state_place(state, state_offset), _ptr(out), _code(out.dtype), _ptr(raw), conv.shape[0], ctx.num_seqs, int(heads),
+          int(kv_heads), int(dim), int(vdim), float(eps), *(_ptr(t) for t in chunks), count, _ptr(scratch))
 
 
 MMA_HEAD_DIMS = (32, 64, 96, 128)

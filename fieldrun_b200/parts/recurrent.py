@@ -41,6 +41,11 @@ from .linear import linear
 STATE_SPACE_CHUNKED_TOKENS = 128
 
 
+# The same for the gated delta rule (delta_chunks.cu): 64 tokens 104 | 116 (16 heads of 128 x 128), 128 tokens 120 | 93, 1,024 tokens
+# 716 | 290; 96 tokens with 16 heads of 64 x 64 98 | 85, with 32 heads of 128 x 128 126 | 120.
+DELTA_CHUNKED_TOKENS = 96
+
+
 class _StateMixer(Mixer):
     replayable = True
     kernel_groups = ("common", "streams", "scans")
@@ -294,9 +299,16 @@ class GatedDeltaRule(_StateMixer):
         ops.causal_conv(proj, 0, self.conv_channels, w["conv"], None, ctx, line.state, self.state_floats, qkv, activation="silu")
         out = ctx.buffer("delta_rule.out", (rows, self.v_width), self.dtype)
         raw = ctx.buffer("delta_rule.raw", (rows, self.v_width), torch.float32)      # for steps that cut the heads over blocks
-        ops.gated_delta_rule(qkv, 0, self.qk_width, 2 * self.qk_width, proj, self.b_off, self.a_off, self.g_off, w["a_log"],
-                             w["dt_bias"], w["norm"], ctx, line.state, 0, out, heads=self.num_heads, kv_heads=self.num_kv_heads,
-                             dim=self.head_dim, vdim=self.value_dim, eps=self.norm_eps, raw=raw)
+        args = (qkv, 0, self.qk_width, 2 * self.qk_width, proj, self.b_off, self.a_off, self.g_off, w["a_log"], w["dt_bias"], w["norm"], ctx,
+                line.state, 0, out)
+        sizes = dict(heads=self.num_heads, kv_heads=self.num_kv_heads, dim=self.head_dim, vdim=self.value_dim, eps=self.norm_eps, raw=raw)
+        if (not ctx.is_decode and ctx.max_q_len >= DELTA_CHUNKED_TOKENS
+                and ops.delta_chunks_take(self.head_dim, self.value_dim, (self.conv_channels, self.qk_width), line.state, 0)):
+            chunks = ctx.token_chunks(ops.DELTA_CHUNK_TOKENS)
+            floats = ops.delta_chunks_scratch_floats(chunks[0].numel(), self.num_heads, self.head_dim, self.value_dim)
+            ops.delta_chunks(*args, chunks=chunks, scratch=ctx.buffer("delta_rule.chunks", (floats,), torch.float32), **sizes)
+        else:
+            ops.gated_delta_rule(*args, **sizes)
         return linear(out, w["o_proj"])
 
 

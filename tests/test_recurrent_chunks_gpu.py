@@ -142,3 +142,46 @@ def test_state_space_in_chunks(heads, groups, n, vdim, decay):
         assert norm_error(results[1][1][slot, copy, 4:-8], results[0][1][slot, copy, 4:-8]) < LIMIT
         results[1][1][slot, copy, 4:-8] = state[slot, copy, 4:-8]
     assert torch.equal(results[1][1], state)                     # nothing else was written
+
+
+@pytest.mark.parametrize("decay", ["mild", "strong", "extreme", "mixed"])
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,dtype", [(4, 2, 128, 128, "float32"), (2, 1, 64, 64, "float32"), (2, 2, 128, 64, "float32"),
+                                                           (1, 1, 64, 128, "float32"), (4, 1, 128, 128, "bfloat16")])
+def test_gated_delta_rule_in_chunks(heads, kv_heads, dim, vdim, dtype, decay):
+    """Chunks of 64, 16 k + r and one token, sequences that go on from a state at odd and even positions, decays of a token from
+    nearly one to exp(-50), keys that repeat one another (the substitution's hardest case) and a key of zeros."""
+    gen = torch.Generator(device=DEV).manual_seed(dim + vdim + heads)
+    lengths, starts, slots = [300, 64, 17, 1, 129], [0, 3, 10, 7, 64], [4, 0, 2, 1, 3]
+    tokens, qk, inner = sum(lengths), kv_heads * dim, heads * vdim
+    conv = torch.randn(tokens, 2 * qk + inner, device=DEV, generator=gen)
+    conv[70:100, qk:2 * qk] = conv[70, qk:2 * qk] * torch.where(torch.arange(30, device=DEV) % 3 == 1, -1.0, 2.0)[:, None]
+    conv[110, qk:2 * qk] = 0.0
+    proj = torch.randn(tokens, 2 * heads + inner, device=DEV, generator=gen)
+    proj[:, :heads] += 2.0                                       # beta close to one
+    proj[:, heads:2 * heads] += {"mild": -4.0, "strong": 2.0, "extreme": 8.0, "mixed": 0.0}[decay]
+    if decay == "mixed":
+        proj[:, heads:2 * heads] *= 5.0
+    a_log, dt_bias = torch.randn(heads, device=DEV, generator=gen) * 0.5, torch.randn(heads, device=DEV, generator=gen) * 0.2
+    norm = torch.randn(vdim, device=DEV, generator=gen)
+    state = torch.randn(5, 2, 2 + heads * dim * vdim + 6, device=DEV, generator=gen)
+    sizes = dict(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, eps=1e-6)
+    tabs = Tables(lengths, starts, slots)
+    results = []
+    for chunked in (False, True):
+        kept, out = state.clone(), torch.full((tokens, inner), float("nan"), device=DEV, dtype=getattr(torch, dtype))
+        raw = torch.full((tokens, inner), float("nan"), device=DEV)
+        args = (conv, 0, qk, 2 * qk, proj, 0, heads, 2 * heads, a_log, dt_bias, norm, tabs, kept, 2, out)
+        if chunked:
+            assert ops().delta_chunks_take(dim, vdim, (conv.shape[1], qk), kept, 2)
+            chunks = tables(lengths, 64)
+            scratch = torch.full((ops().delta_chunks_scratch_floats(chunks[0].numel(), heads, dim, vdim),), float("nan"), device=DEV)
+            ops().delta_chunks(*args, raw=raw, chunks=chunks, scratch=scratch, **sizes)
+        else:
+            ops().gated_delta_rule(*args, raw=raw, **sizes)
+        results.append((out, kept, raw))
+    assert norm_error(results[1][0].float(), results[0][0].float()) < (LIMIT if dtype == "float32" else 2.0 ** -9)
+    for n, start, slot in zip(lengths, starts, slots):
+        copy = (start + n) & 1
+        assert norm_error(results[1][1][slot, copy, 2:-6], results[0][1][slot, copy, 2:-6]) < LIMIT
+        results[1][1][slot, copy, 2:-6] = state[slot, copy, 2:-6]
+    assert torch.equal(results[1][1], state)                     # nothing else was written
