@@ -1,15 +1,16 @@
 // Attention over the paged cache in float32 for the head sizes that models have: the float32 path's prompts in tiles of 64
 // queries, and its single tokens in chunks of 256 keys that run side by side.  Same formulas and options as
 // attention_generic.cu (window, chunk, first tokens, slopes, sinks, cap, gates, a value head of another size, key heads that
-// share a value head), which keeps the sizes these kernels do not take.  Every product and sum is a float32 multiply-add.
+// share a value head), which keeps the sizes these kernels do not take.  Everything is float32; the tiles' products run on tensor
+// cores with each operand as two TF32 parts (tf32_parts.cuh).
 //
-// What bounds them.  Prompts: the float32 pipes (4 (head_dim + v_dim) operations a visible pair and head at 74 TFLOP/s);
-// attention_generic runs a block per token, which reads the token's keys and values for itself through scalar loads, and a
-// warp's 32 keys through one chain of multiply-adds: 15.2 ms for six prompts of 17 to 1,500 tokens (48 heads over 8 of 128,
-// 3.1 TFLOP/s); the whole layer went from 21.2 to 7.5 ms with the tiles, 5.9 of it the two dense products.  Single tokens: the
-// keys' and values' bytes; there a block per token and key head left 48 blocks on 148 SMs, each walking its whole sequence:
-// 1.20 ms for six sequences of 17 to 1,500 keys; the whole layer went from 1.33 to 0.15 ms, 0.14 of it the dense products.
-#include "common.cuh"
+// What bounds them.  Prompts: the instructions that split the operands and the tensor cores; attention_generic runs a block per
+// token, which reads the token's keys and values for itself through scalar loads, and a warp's 32 keys through one chain of
+// multiply-adds: 15.2 ms for six prompts of 17 to 1,500 tokens (48 heads over 8 of 128, 3.1 TFLOP/s).  Tiles of 64 queries with 8 x 4
+// scores and 8 x 8 sums a thread on the ordinary pipes took 1.59 ms (30 TFLOP/s), on the tensor cores 1.11 ms (43).  Single tokens: the
+// keys' and values' bytes; there a block per token and key head left 48 blocks on 148 SMs, each walking its whole sequence: 1.20 ms
+// for six sequences of 17 to 1,500 keys; the whole layer went from 1.33 to 0.08 ms, most of it the dense products.
+#include "tf32_parts.cuh"
 
 struct F32Attention {
     const float* q;           // [T, nh, hd]
@@ -23,12 +24,6 @@ struct F32Attention {
     float scale, softcap;
     int gate_stride, chunk, keep_first, window, max_pages, num_heads, num_kv_heads, v_heads, head_dim, v_dim;
 };
-
-__device__ __forceinline__ void f32_copy16(float* dst, const float* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void f32_copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int PENDING> __device__ __forceinline__ void f32_copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
 
 __device__ __forceinline__ float dot4(float4 a, float4 b, float c) {
     c = fmaf(a.x, b.x, c);
@@ -49,23 +44,24 @@ __device__ __forceinline__ float f32_score(const F32Attention& p, float raw, flo
 #define TILE_Q 64             // queries of one head a block takes
 #define TILE_THREADS 128
 
-// A block takes 64 neighbouring queries of one head and walks the pages of 64 keys that any of them sees.  A thread holds 8 x 4
-// scores and 8 x 16 VJ / 16 sums of the same 8 queries, so 12 (scores) and 8 + VJ (sums) 16-byte shared-memory loads serve 128
-// and 32 VJ multiply-adds.  Rows lie with their 16-byte units permuted by the row's low three bits: lanes of one load then meet
-// no bank twice and no row needs padding, which is what lets two blocks share an SM (112 KB each at head size 128).  The next
-// page's keys are on their way while this page's values are summed, its values while the next scores are computed.
-template <int VJ>
+// A block takes 64 neighbouring queries of one head and walks the pages of 64 keys that any of them sees; a warp has 16 of the
+// queries.  Both products run on tensor cores with each operand as two TF32 parts; the weights stay in the registers that the
+// scores are in, which are those that the second product wants them in.  A page's sums are added to the queries' in float32,
+// rounded (over thousands of keys the tensor cores' adder, which cuts off, would cost more than a rounding).  The next page's keys
+// are on their way while this page's values are summed, its values while the next scores are computed.  NT: column tiles of eight
+// value entries.
+template <int NT>
 __global__ void __launch_bounds__(TILE_THREADS, 2)
 attention_f32_tiles_kernel(F32Attention p, const int* __restrict__ tile_seq, const int* __restrict__ tile_q0,
                            const int* __restrict__ seq_slot, const int* __restrict__ seq_start, const int* __restrict__ seq_q_len,
                            const int* __restrict__ cu_q_len) {
+    constexpr int LV = FRB_PAGE + 8;
     extern __shared__ float4 f32_smem[];
     const int hd = p.head_dim, vd = p.v_dim;
-    const int hdp = (hd + 31) & ~31;                       // entries a row takes: whole groups of eight 16-byte units
-    float* q_s = (float*)f32_smem;                         // [TILE_Q][hdp]
-    float* k_s = q_s + TILE_Q * hdp;                       // [FRB_PAGE][hdp]
-    float* p_s = k_s + FRB_PAGE * hdp;                     // [TILE_Q][FRB_PAGE]
-    float* v_s = p_s + TILE_Q * FRB_PAGE;                  // [16 VJ][FRB_PAGE]
+    const int hd8 = (hd + 7) & ~7, ld = ((hd + 31) & ~31) + 8;           // entries of the inner size; a row's place
+    float* q_s = (float*)f32_smem;                         // [TILE_Q][ld]
+    float* k_s = q_s + TILE_Q * ld;                        // [FRB_PAGE][ld]
+    float* v_s = k_s + FRB_PAGE * ld;                      // [8 NT][LV]
     // the last tiles of the sequences see the most keys: they begin first.  A tile of the step's lists is 128 queries: two blocks
     const int unit = gridDim.y - 1 - blockIdx.y;
     const int head = blockIdx.x, seq = tile_seq[unit >> 1];
@@ -79,145 +75,144 @@ attention_f32_tiles_kernel(F32Attention p, const int* __restrict__ tile_seq, con
     const int kept = kept_runs(p.keep_first, FRB_PAGE, first_page);
     const int pages = kept + last / FRB_PAGE - first_page + 1;
     const int* table = p.page_table + (size_t)seq_slot[seq] * p.max_pages;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = tid & 15, ty = tid >> 4;
-    const int units = hd >> 2, units_p = hdp >> 2;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g8 = lane >> 2, t4 = lane & 3;
+    const int units = hd >> 2;
 
     // entries that no copy fills: the queries' and keys' padding, queries beyond the tile, value rows beyond v_dim
-    for (int i = tid; i < TILE_Q * units_p; i += TILE_THREADS) {
-        const int r = i / units_p, u = i - r * units_p;
-        float4* at = (float4*)(q_s + r * hdp) + (u ^ (r & 7));
-        if (u >= units || r >= rows) *at = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (u >= units) ((float4*)(k_s + r * hdp))[u ^ (r & 7)] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = tid; i < TILE_Q * (ld / 4); i += TILE_THREADS) {
+        const int r = i / (ld / 4), u = i - r * (ld / 4);
+        if (u >= units || r >= rows) *(float4*)(q_s + r * ld + 4 * u) = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (u >= units) *(float4*)(k_s + r * ld + 4 * u) = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    for (int i = vd * FRB_PAGE + tid; i < 16 * VJ * FRB_PAGE; i += TILE_THREADS) v_s[i] = 0.f;
+    for (int i = vd * LV + tid; i < 8 * NT * LV; i += TILE_THREADS) v_s[i] = 0.f;
 
     auto copy_keys = [&](int n) {
         const float* src = p.k_pages + ((size_t)table[run_at(n, kept, first_page)] * p.num_kv_heads + g) * FRB_PAGE * hd;
         for (int r = warp; r < FRB_PAGE; r += TILE_THREADS / 32)
-            for (int u = lane; u < units; u += 32) f32_copy16(k_s + r * hdp + 4 * (u ^ (r & 7)), src + r * hd + 4 * u);
+            for (int u = lane; u < units; u += 32) copy16_async(k_s + r * ld + 4 * u, src + r * hd + 4 * u);
     };
     auto copy_values = [&](int n) {
         const float* src = p.v_pages + ((size_t)table[run_at(n, kept, first_page)] * p.v_heads + vg) * FRB_PAGE * vd;
-        for (int d = ty; d < vd; d += TILE_THREADS / 16) f32_copy16(v_s + d * FRB_PAGE + 4 * (tx ^ (d & 7)), src + d * FRB_PAGE + 4 * tx);
+        for (int d = tid >> 4; d < vd; d += TILE_THREADS / 16) copy16_async(v_s + d * LV + 4 * (tid & 15), src + d * FRB_PAGE + 4 * (tid & 15));
     };
-
     for (int r = warp; r < rows; r += TILE_THREADS / 32)
-        for (int u = lane; u < units; u += 32)
-            f32_copy16(q_s + r * hdp + 4 * (u ^ (r & 7)), p.q + ((token0 + r) * p.num_heads + head) * hd + 4 * u);
+        for (int u = lane; u < units; u += 32) copy16_async(q_s + r * ld + 4 * u, p.q + ((token0 + r) * p.num_heads + head) * hd + 4 * u);
     copy_keys(0);
-    f32_copies_commit();
+    copies_commit();
     copy_values(0);
-    f32_copies_commit();
+    copies_commit();
 
     const float slope = p.slopes ? p.slopes[head] : 0.f;
-    float m[8], l[8], acc[8][VJ];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        m[i] = -INFINITY;
-        l[i] = 0.f;
-#pragma unroll
-        for (int j = 0; j < VJ; ++j) acc[i][j] = 0.f;
-    }
-    const int ksw = tx & 7;
+    const int pos[2] = {pos0 + warp * 16 + g8, pos0 + warp * 16 + g8 + 8};
+    const int lo[2] = {first_visible_key(pos[0], p.window, p.chunk), first_visible_key(pos[1], p.window, p.chunk)};
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, acc[NT][4] = {};
+    const float* q_rows = q_s + warp * 16 * ld;
 
     for (int n = 0; n < pages; ++n) {
         const int j0 = run_at(n, kept, first_page) * FRB_PAGE;
-        f32_copies_wait<1>();                              // this page's keys; its values may still be on their way
+        copies_wait<1>();                                  // this page's keys; its values may still be on their way
         __syncthreads();
-        float s[8][4];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+        float s[1][8][4] = {}, small[1][8][4] = {};
 #pragma unroll 2
-        for (int u = 0; u < units_p; ++u) {
-            float4 a[8], b[4];
+        for (int c = 0; c < hd8; c += 8) {
+            Tf32Parts a[1][4], b[8][2];
+            a_along(a[0], q_rows + c, ld, lane);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) a[i] = ((const float4*)(q_s + (ty + 8 * i) * hdp))[u ^ (ty & 7)];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = ((const float4*)(k_s + (tx + 16 * j) * hdp))[u ^ ksw];
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) s[i][j] = dot4(a[i], b[j], s[i][j]);
+            for (int j = 0; j < 8; ++j) b_along(b[j], k_s + 8 * j * ld + c, ld, lane);
+            mma_tiles_apart<1, 8>(s, small, a, b);
         }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[0][j][e] += small[0][j][e];
         const bool edge = j0 + FRB_PAGE - 1 > pos0 || p.window > 0 || p.chunk > 0;      // some query may not see some key
+        float corr[2];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int pos = pos0 + ty + 8 * i;
-            const int lo = first_visible_key(pos, p.window, p.chunk);
-            float top = m[i];
+        for (int half = 0; half < 2; ++half) {
+            float top = m[half];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int key = j0 + tx + 16 * j;
-                s[i][j] = f32_score(p, s[i][j], slope, pos, key, !edge || key_visible(key, lo, pos, p.keep_first));
-                top = fmaxf(top, s[i][j]);
-            }
+            for (int j = 0; j < 8; ++j)
 #pragma unroll
-            for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+                for (int e = 0; e < 2; ++e) {
+                    const int key = j0 + 8 * j + 2 * t4 + e;
+                    float& x = s[0][j][2 * half + e];
+                    x = f32_score(p, x, slope, pos[half], key, !edge || key_visible(key, lo[half], pos[half], p.keep_first));
+                    top = fmaxf(top, x);
+                }
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
             const float use = top == -INFINITY ? 0.f : top;           // a query that has seen no key yet
-            const float corr = expf(m[i] - use);
-            m[i] = top;
-            l[i] *= corr;
+            corr[half] = expf(m[half] - use);
+            m[half] = top;
+            l[half] *= corr[half];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int key = tx + 16 * j;
-                const float w = expf(s[i][j] - use);
-                l[i] += w;                                            // this thread's keys; the sixteen threads' sums meet at the end
-                p_s[(ty + 8 * i) * FRB_PAGE + 4 * ((key >> 2) ^ (ty & 7)) + (key & 3)] = w;
-            }
+            for (int j = 0; j < 8; ++j)
 #pragma unroll
-            for (int j = 0; j < VJ; ++j) acc[i][j] *= corr;
+                for (int e = 0; e < 2; ++e) {
+                    float& x = s[0][j][2 * half + e];
+                    x = expf(x - use);
+                    l[half] += x;                                     // this lane's keys; the four lanes' sums meet at the end
+                }
         }
-        __syncthreads();                                   // the weights are there, and nobody reads the keys any more
+        __syncthreads();                                   // nobody reads the keys any more
         if (n + 1 < pages) copy_keys(n + 1);
-        f32_copies_commit();
-        f32_copies_wait<1>();                              // this page's values
+        copies_commit();
+        copies_wait<1>();                                  // this page's values
         if (j0 + FRB_PAGE - 1 > last) {                    // keys behind the last one seen: whatever a page holds there counts for nothing
             __syncthreads();
-            for (int i = tid; i < vd * FRB_PAGE; i += TILE_THREADS) {
-                const int d = i / FRB_PAGE, k = i % FRB_PAGE;
-                if (j0 + k > last) v_s[d * FRB_PAGE + 4 * ((k >> 2) ^ (d & 7)) + (k & 3)] = 0.f;
-            }
+            for (int i = tid; i < vd * FRB_PAGE; i += TILE_THREADS)
+                if (j0 + i % FRB_PAGE > last) v_s[i / FRB_PAGE * LV + i % FRB_PAGE] = 0.f;
         }
         __syncthreads();
-#pragma unroll 2
-        for (int u = 0; u < FRB_PAGE / 4; ++u) {
-            float4 a[8], b[VJ];
+        constexpr int RUN = NT < 8 ? NT : 8;               // column tiles whose page's sums are in registers together
 #pragma unroll
-            for (int i = 0; i < 8; ++i) a[i] = ((const float4*)(p_s + (ty + 8 * i) * FRB_PAGE))[u ^ (ty & 7)];
+        for (int n0 = 0; n0 < NT; n0 += RUN) {
+            float page[1][RUN][4] = {};
 #pragma unroll
-            for (int j = 0; j < VJ; ++j) b[j] = ((const float4*)(v_s + (tx + 16 * j) * FRB_PAGE))[u ^ ksw];
+            for (int j = 0; j < 8; ++j) {                  // the scores' registers, keys 2 t and 2 t + 1 of a run of eight
+                const Tf32Parts a[1][4] = {{tf32_parts(s[0][j][0]), tf32_parts(s[0][j][2]), tf32_parts(s[0][j][1]), tf32_parts(s[0][j][3])}};
+                Tf32Parts b[RUN][2];
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+                for (int i = 0; i < RUN; ++i) b_along(b[i], v_s + 8 * (n0 + i) * LV + 8 * j, LV, lane);
+                mma_tiles<1, RUN, RUN>(page, 0, a, b);
+            }
 #pragma unroll
-                for (int j = 0; j < VJ; ++j) acc[i][j] = dot4(a[i], b[j], acc[i][j]);
+            for (int i = 0; i < RUN; ++i) {
+                float (&o)[4] = acc[n0 + i];
+                o[0] = fmaf(o[0], corr[0], page[0][i][0]);
+                o[1] = fmaf(o[1], corr[0], page[0][i][1]);
+                o[2] = fmaf(o[2], corr[1], page[0][i][2]);
+                o[3] = fmaf(o[3], corr[1], page[0][i][3]);
+            }
         }
         __syncthreads();
         if (n + 1 < pages) copy_values(n + 1);
-        f32_copies_commit();
+        copies_commit();
     }
-    f32_copies_wait<0>();
+    copies_wait<0>();
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int r = ty + 8 * i;
-        float total = l[i];
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+    for (int half = 0; half < 2; ++half) {
+        const int r = warp * 16 + 8 * half + g8;
+        float total = l[half];
+        total += __shfl_xor_sync(0xffffffffu, total, 1);
+        total += __shfl_xor_sync(0xffffffffu, total, 2);
         float factor = 1.f;
         if (p.sinks) {
-            const float sink = p.sinks[head], top = fmaxf(m[i], sink);
-            factor = expf(m[i] - top);
+            const float sink = p.sinks[head], top = fmaxf(m[half], sink);
+            factor = expf(m[half] - top);
             total = total * factor + expf(sink - top);
         }
         if (r >= rows) continue;
         float inv = factor / total;
         if (p.gate) inv *= 1.0f / (1.0f + expf(-p.gate[(token0 + r) * p.gate_stride + head]));
+        float* out = p.out + ((token0 + r) * p.num_heads + head) * vd;
 #pragma unroll
-        for (int j = 0; j < VJ; ++j) {
-            const int d = tx + 16 * j;
-            if (d < vd) p.out[((token0 + r) * p.num_heads + head) * vd + d] = acc[i][j] * inv;
-        }
+        for (int i = 0; i < NT; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int d = 8 * i + 2 * t4 + e;
+                if (d < vd) out[d] = acc[i][2 * half + e] * inv;
+            }
     }
 }
 
@@ -433,17 +428,17 @@ FRB_API int frb_attention_f32_tiles(const float* q, const float* k_pages, const 
     const int bad = f32_attention_params(&p, q, k_pages, v_pages, page_table, max_pages, out, num_heads, num_kv_heads, head_dim, v_dim, scale,
                                          window, slopes, chunk, sinks, gate, gate_stride, softcap, keep_first, num_v_heads);
     if (bad) return bad;
-    const int hdp = (head_dim + 31) & ~31;
-#define FRB_TILES(VJ)                                                                                                               \
+    const int ld = ((head_dim + 31) & ~31) + 8;
+#define FRB_TILES(NT)                                                                                                               \
     do {                                                                                                                            \
-        const size_t smem = ((size_t)(TILE_Q + FRB_PAGE) * hdp + (size_t)(TILE_Q + 16 * VJ) * FRB_PAGE) * sizeof(float);            \
-        cudaFuncSetAttribute(attention_f32_tiles_kernel<VJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);              \
-        attention_f32_tiles_kernel<VJ><<<dim3(num_heads, 2 * num_tiles), TILE_THREADS, smem, stream>>>(p, tile_seq, tile_q0,        \
+        const size_t smem = ((size_t)(TILE_Q + FRB_PAGE) * ld + (size_t)8 * NT * (FRB_PAGE + 8)) * sizeof(float);                   \
+        cudaFuncSetAttribute(attention_f32_tiles_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);              \
+        attention_f32_tiles_kernel<NT><<<dim3(num_heads, 2 * num_tiles), TILE_THREADS, smem, stream>>>(p, tile_seq, tile_q0,        \
                                                                                     seq_slot, seq_start, seq_q_len, cu_q_len);       \
     } while (0)
-    if (v_dim <= 32) FRB_TILES(2);
-    else if (v_dim <= 64) FRB_TILES(4);
-    else FRB_TILES(8);
+    if (v_dim <= 32) FRB_TILES(4);
+    else if (v_dim <= 64) FRB_TILES(8);
+    else FRB_TILES(16);
 #undef FRB_TILES
     FRB_RETURN_LAUNCH("attention_f32_tiles");
 }

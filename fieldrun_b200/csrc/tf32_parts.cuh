@@ -1,5 +1,6 @@
-// Float32 products on mma.sync: each operand as two TF32 parts, hi = the entry cut to TF32 and lo = what is left, rounded to
-// TF32.  hi hi + hi lo + lo hi keeps 21 bits of every product; the sums are the tensor cores' float32 sums, which the callers
+// Float32 products on mma.sync: each operand as two TF32 parts, hi = the entry rounded to TF32 and lo = what is left, of
+// either sign.  hi hi + hi lo + lo hi keeps 22 bits of every product (with hi cut instead of rounded, lo lo, which is left out, would
+// be four times as large and always of one sign); the sums are the tensor cores' float32 sums, which the callers
 // keep short (the adder cuts off instead of rounding: about 1e-9 of the sum with every entry).
 #pragma once
 
@@ -9,12 +10,12 @@ struct Tf32Parts {
     uint32_t hi, lo;
 };
 
-// The tensor cores read the upper 19 bits of an operand.  Three full-rate instructions; with the conversion instruction (hi
-// rounded as well) the chunks of gla_chunks.cu took 525 us instead of 492.
+// The tensor cores read the upper 19 bits of an operand.  Three full-rate instructions; with the conversion instruction (lo rounded as
+// well) the chunks of gla_chunks.cu took 525 us instead of 492.  A NaN stays one in lo.
 __device__ __forceinline__ Tf32Parts tf32_parts(float v) {
     Tf32Parts p;
-    p.hi = __float_as_uint(v) & 0xffffe000u;
-    p.lo = __float_as_uint(v - __uint_as_float(p.hi)) + 0x1000u;         // rounded: half of the last place that is read
+    p.hi = (__float_as_uint(v) + 0x1000u) & 0xffffe000u;                 // half of the last place that is kept, then cut
+    p.lo = __float_as_uint(v - __uint_as_float(p.hi));
     return p;
 }
 
@@ -42,6 +43,23 @@ __device__ __forceinline__ void mma_tiles(float (&c)[M][NA][4], int n0, const Tf
     for (int n = 0; n < NN; ++n)
 #pragma unroll
         for (int m = 0; m < M; ++m) mma_tf32(c[m][n0 + n], a[m][0].hi, a[m][1].hi, a[m][2].hi, a[m][3].hi, b[n][0].hi, b[n][1].hi);
+}
+// The same with the small products (hi lo and lo hi) in sums of their own: a third as many cuts of the large sums.
+template <int M, int NN>
+__device__ __forceinline__ void mma_tiles_apart(float (&large)[M][NN][4], float (&small)[M][NN][4], const Tf32Parts (&a)[M][4],
+                                                const Tf32Parts (&b)[NN][2]) {
+#pragma unroll
+    for (int n = 0; n < NN; ++n)
+#pragma unroll
+        for (int m = 0; m < M; ++m) mma_tf32(small[m][n], a[m][0].lo, a[m][1].lo, a[m][2].lo, a[m][3].lo, b[n][0].hi, b[n][1].hi);
+#pragma unroll
+    for (int n = 0; n < NN; ++n)
+#pragma unroll
+        for (int m = 0; m < M; ++m) mma_tf32(large[m][n], a[m][0].hi, a[m][1].hi, a[m][2].hi, a[m][3].hi, b[n][0].hi, b[n][1].hi);
+#pragma unroll
+    for (int n = 0; n < NN; ++n)
+#pragma unroll
+        for (int m = 0; m < M; ++m) mma_tf32(small[m][n], a[m][0].hi, a[m][1].hi, a[m][2].hi, a[m][3].hi, b[n][0].lo, b[n][1].lo);
 }
 __device__ __forceinline__ void mma_parts(float (&c)[4], const Tf32Parts (&a)[4], const Tf32Parts (&b)[2]) {
     mma_tf32(c, a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi);
