@@ -1,4 +1,5 @@
-"""Plain dense matrix products through the library (cuBLAS via torch.mm).
+"""Plain dense matrix products: few rows as a stream over the weight, large float32 products on the tensor cores with their
+operands in parts, the others through the library (cuBLAS via torch.mm).
 
 The reference's dense products (``Bundle::mm``, src/bundle.rs:644-683) are a
 library call as well: ndarray's ``dot`` over matrixmultiply or cblas.  Weights
