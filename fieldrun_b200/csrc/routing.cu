@@ -736,9 +736,43 @@ __global__ void combine_kernel(const float* __restrict__ y, const float* __restr
     out[(size_t)t * width + c] = acc;
 }
 
+// The same sums in the same order for widths in steps of four: 16 bytes a thread, four of the token's rows on their way at once.  Bound
+// by its bytes: 2,048 tokens of eight rows of 3,072, 226 MB, take 40 us (5.6 TB/s), one column a thread 54 us.
+__global__ void __launch_bounds__(256) combine4_kernel(const float4* __restrict__ y, const float* __restrict__ weights,
+                                                       const int* __restrict__ row_of_assign, int top_k, int units, float4* __restrict__ out) {
+    after_previous_kernel();
+    const int t = blockIdx.x, c = blockIdx.y * 256 + threadIdx.x;
+    if (c >= units) return;
+    weights += (size_t)t * top_k;
+    row_of_assign += (size_t)t * top_k;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int r0 = 0; r0 < top_k; r0 += 4) {
+        float4 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (r0 + i < top_k) v[i] = y[(size_t)row_of_assign[r0 + i] * units + c];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (r0 + i < top_k) {
+                const float w = weights[r0 + i];
+                acc.x += w * v[i].x;
+                acc.y += w * v[i].y;
+                acc.z += w * v[i].z;
+                acc.w += w * v[i].w;
+            }
+    }
+    out[(size_t)t * units + c] = acc;
+}
+
 FRB_API int frb_expert_combine(const float* y, const float* weights, const int* row_of_assign, int num_tokens, int top_k,
                                int width, float* out, cudaStream_t stream) {
     if (num_tokens == 0) return 0;
+    if (width % 4 == 0 && (((uintptr_t)y | (uintptr_t)out) & 15) == 0) {
+        const dim3 fours(num_tokens, (width / 4 + 255) / 256);
+        FRB_CHECK_ARG(fours.y <= 65535, "combine: a width of %d exceeds the grid", width);
+        launch_dependent(combine4_kernel, fours, dim3(256), 0, stream, (const float4*)y, weights, row_of_assign, top_k, width / 4, (float4*)out);
+        FRB_RETURN_LAUNCH("expert_combine");
+    }
     dim3 grid(num_tokens, (width + 255) / 256);
     FRB_CHECK_ARG(grid.y <= 65535, "combine: a width of %d exceeds the grid", width);
     launch_dependent(combine_kernel, dim3(grid), dim3(256), 0, stream, y, weights, row_of_assign, top_k, width, out);

@@ -196,3 +196,21 @@ def test_split_products_keep_infinities_nans_and_far_exponents():
     fine = want.isfinite() & (want.abs() > 1e-36)                 # results that float32 holds to its full precision
     size = x.double().abs() @ w[0].double().abs().T
     assert ((got.double() - want.double()).abs() <= 1e-5 * size + 2e-43)[fine].all()
+
+
+@pytest.mark.parametrize("top_k", [1, 3, 4, 8, 9])
+@pytest.mark.parametrize("width", [4, 96, 1028, 3072])
+def test_weighted_sums_of_four_columns_equal_those_of_one(width, top_k):
+    """The same sums in the same order: the bits of rows that lie one float off, which take a column a thread."""
+    gen = torch.Generator(device=DEV).manual_seed(width + top_k)
+    y, weights = torch.randn(7 * top_k, width, device=DEV, generator=gen), torch.rand(7, top_k, device=DEV, generator=gen)
+    rows = torch.randperm(7 * top_k, device=DEV, generator=gen).to(torch.int32)
+    results = []
+    for shift in (0, 1):
+        held = torch.zeros(y.numel() + 4, device=DEV)
+        shifted = held[shift:shift + y.numel()].view_as(y)
+        shifted.copy_(y)
+        out = torch.full((7, width), float("nan"), device=DEV)
+        ops().expert_combine(shifted, weights, rows, out)
+        results.append(out)
+    assert torch.isfinite(results[0]).all() and torch.equal(*results)
