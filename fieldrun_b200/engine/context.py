@@ -147,6 +147,10 @@ class StepContext:
     def buffer(self, name: str, shape: Sequence[int], dtype: torch.dtype) -> torch.Tensor:
         return self.workspace.buffer(name, shape, dtype)
 
+    def chunk_count(self, size: int) -> int:
+        """How many chunks :meth:`token_chunks` makes."""
+        return sum(-(-n // size) for n in self.seq_q_lens)
+
     def token_chunks(self, size: int) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
         """The step's new tokens in chunks of at most ``size``: sequence, first token and end (among the sequence's new tokens) of
         each, and every sequence's first chunk with, last, their number; int32 on the device.  For steps of prompts only: the

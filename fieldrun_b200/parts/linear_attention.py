@@ -26,9 +26,10 @@ from .base import Mixer, register_part
 from .linear import linear
 
 
-# From this many tokens of the longest prompt on a step runs in chunks as matrix products (gla_chunks.cu), where its sizes allow.
-# Measured on a B200, the whole part, microseconds, token by token | in chunks: one prompt of 32 tokens 70 | 90 (16 heads of
-# 128 x 128), 64 tokens 112 | 91, 1,024 tokens 371 | 140; 64 tokens with 32 heads 134 | 118, with 16 heads of 64 x 64 82 | 69.
+# From this many tokens of the longest prompt on a step may run in chunks as matrix products (gla_chunks.cu).  Measured on a B200,
+# the whole part, microseconds, token by token | in chunks (16 heads of 128 x 128): one prompt of 32 tokens 70 | 90, of 64 tokens
+# 112 | 91, of 1,024 tokens 371 | 140; 16 prompts of 65 tokens 171 | 183, of 130 tokens 332 | 272; 64 of 128 tokens 1235 | 764; one of
+# 256 tokens beside 31 of two 408 | 168.
 CHUNKED_TOKENS = 64
 SEGMENT_TOKENS = 128        # other sizes: a long prompt's tokens run in segments of this many, side by side (see gla.cu)
 
@@ -92,6 +93,15 @@ class GatedLinearAttention(Mixer):
     def cache_need(self) -> CacheNeed:
         return CacheNeed(state_shape=(2, self.num_heads, self.head_dim, self.value_dim), state_dtype="float32")
 
+    def chunks_pay(self, ctx) -> bool:
+        """Whether a step of prompts is faster in chunks.  Token by token it takes as long as its longest prompt, or, with more
+        than two heads an SM, as its tokens shared out; in chunks each (chunk, head) costs about an eighth of a token's time, and
+        the launches thirteen tokens' (fitted to the measurements above)."""
+        if ctx.is_decode or ctx.max_q_len < CHUNKED_TOKENS:
+            return False
+        serial = max(ctx.max_q_len, ctx.num_tokens * self.num_heads / (2 * ops.sm_count(ctx.device)))
+        return 0.13 * ctx.chunk_count(ops.GLA_CHUNK_TOKENS) * self.num_heads + 13 < serial
+
     def forward(self, ctx, act: torch.Tensor, line: LineView, writes_cache: bool) -> torch.Tensor:
         if not writes_cache:
             raise ValueError("a recurrent layer cannot read another layer's state: it has to write its own")
@@ -99,8 +109,7 @@ class GatedLinearAttention(Mixer):
         out = ctx.buffer("linear_attention.out", (act.shape[0], self.v_width), self.dtype)
         sizes = dict(heads=self.num_heads, dim=self.head_dim, vdim=self.value_dim, tau=self.tau, q_scale=self.q_scale, eps=self.norm_eps)
         args = (proj, self.offsets, self.w_decay, self.decay_bias, self.norm_weight, line.state, ctx.seq_slot, ctx.seq_start, ctx.cu_q_len, out)
-        if (not ctx.is_decode and ctx.max_q_len >= CHUNKED_TOKENS
-                and ops.gla_chunks_take(self.head_dim, self.value_dim, self.decay_rank, proj.shape[1], self.offsets)):
+        if self.chunks_pay(ctx) and ops.gla_chunks_take(self.head_dim, self.value_dim, self.decay_rank, proj.shape[1], self.offsets):
             chunks = ctx.token_chunks(ops.GLA_CHUNK_TOKENS)
             floats = ops.gla_chunks_scratch_floats(chunks[0].numel(), act.shape[0], self.num_heads, self.head_dim, self.value_dim)
             ops.gla_chunks(*args, chunks=chunks, scratch=ctx.buffer("linear_attention.segments", (floats,), torch.float32), **sizes)

@@ -35,15 +35,13 @@ from .base import Mixer, register_part
 from .linear import linear
 
 
-# From this many tokens of the longest prompt on a step's recurrence runs in chunks as matrix products, where its sizes allow
-# (state_space_chunks.cu).  Measured on a B200, the whole part, microseconds, token by token | in chunks: one prompt of 96 tokens 106 |
-# 135 (64 heads of 128 x 64), 128 tokens 112 | 98, 1,024 tokens 702 | 216; 128 tokens with 32 heads 93 | 91, with 128 heads 159 | 146.
-STATE_SPACE_CHUNKED_TOKENS = 128
-
-
-# The same for the gated delta rule (delta_chunks.cu): 64 tokens 104 | 116 (16 heads of 128 x 128), 128 tokens 120 | 93, 1,024 tokens
-# 716 | 290; 96 tokens with 16 heads of 64 x 64 98 | 85, with 32 heads of 128 x 128 126 | 120.
-DELTA_CHUNKED_TOKENS = 96
+# From this many tokens of the longest prompt on a step's recurrence may run in chunks as matrix products (state_space_chunks.cu,
+# delta_chunks.cu).  Measured on a B200, the whole part, microseconds, token by token | in chunks.  State space, 64 heads of 128 x 64:
+# one prompt of 128 tokens 112 | 98 (32 heads 77 | 103), of 1,024 tokens 702 | 216; 4 of 140 tokens 168 | 190; 16 of 130 tokens
+# 438 | 498, of 300 tokens 937 | 840; 64 of 128 tokens 1565 | 1406; one of 256 tokens beside 31 of two 243 | 421.  Delta rule, 16 heads
+# of 128 x 128: one prompt of 64 tokens 104 | 116, of 128 tokens 120 | 93, of 1,024 tokens 716 | 290; 16 of 65 tokens 267 | 222, 64 of 64
+# tokens 831 | 464; one of 128 tokens beside 63 of five 286 | 356; with 16 heads of 64 x 64 16 prompts of 130 tokens 155 | 163.
+STATE_SPACE_CHUNKED_TOKENS, DELTA_CHUNKED_TOKENS = 128, 64
 
 
 class _StateMixer(Mixer):
@@ -212,6 +210,15 @@ class ScalarDecayStateSpace(_StateMixer):
     def load(self, source: TensorSource) -> None:
         self.w = self._fetch(source)
 
+    def chunks_pay(self, ctx) -> bool:
+        """Whether a step of prompts is faster in chunks.  Token by token it takes as long as its longest prompt, or, with more
+        than two heads an SM, as its tokens shared out (0.7 us a token); in chunks each (chunk, head) costs 0.18 us and what
+        does not grow with them 85 (fitted to the measurements above, so that no step measured became slower)."""
+        if ctx.is_decode or ctx.max_q_len < STATE_SPACE_CHUNKED_TOKENS:
+            return False
+        serial = max(ctx.max_q_len, ctx.num_tokens * self.num_heads / (2 * ops.sm_count(ctx.device)))
+        return 0.18 * ctx.chunk_count(ops.STATE_SPACE_CHUNK_TOKENS) * self.num_heads + 85 < 0.7 * serial
+
     def forward(self, ctx, act: torch.Tensor, line: LineView, writes_cache: bool) -> torch.Tensor:
         self._check(writes_cache)
         w, rows, c = self.w, act.shape[0], self.inner
@@ -223,7 +230,7 @@ class ScalarDecayStateSpace(_StateMixer):
         y = ctx.buffer("state_space.y", (rows, c), torch.float32)
         sizes = dict(heads=self.num_heads, vdim=self.value_dim, n=self.state, groups=self.groups)
         args = (proj, 0, c + self.conv_channels, xbc, c, c + gn, w["dt_bias"], w["a_log"], w["d"], ctx, line.state, 0, y)
-        if (not ctx.is_decode and ctx.max_q_len >= STATE_SPACE_CHUNKED_TOKENS
+        if (self.chunks_pay(ctx)
                 and ops.state_space_chunks_take(z_offset=0, row=proj.shape[1], xbc_offsets=(self.conv_channels, c, c + gn), state=line.state,
                                                 state_offset=0, **sizes)):
             chunks = ctx.token_chunks(ops.STATE_SPACE_CHUNK_TOKENS)
@@ -291,6 +298,17 @@ class GatedDeltaRule(_StateMixer):
         w["conv"] = torch.cat([w.pop("q_conv"), w.pop("k_conv"), w.pop("v_conv")], dim=0).contiguous()
         self.w = w
 
+    def chunks_pay(self, ctx) -> bool:
+        """Whether a step of prompts is faster in chunks.  Token by token it takes 0.67 us a token of its longest prompt, or, shared
+        out, of one head of 128 x 128 in 64; in chunks each (chunk, head) of that size costs 0.09 us side by side, then 12 us a chunk
+        along the longest prompt, or 0.16 us a (chunk, head) shared out, and the launches 40 (fitted to the measurements above)."""
+        if ctx.is_decode or ctx.max_q_len < DELTA_CHUNKED_TOKENS:
+            return False
+        share = self.num_heads * self.head_dim * self.value_dim / 2 ** 14          # heads of 128 x 128 that these are as much as
+        items = ctx.chunk_count(ops.DELTA_CHUNK_TOKENS) * share
+        serial = max(ctx.max_q_len, ctx.num_tokens * share / 64)
+        return 40 + 0.09 * items + max(12.0 * ctx.max_q_len / ops.DELTA_CHUNK_TOKENS, 0.16 * items) < 0.67 * serial
+
     def forward(self, ctx, act: torch.Tensor, line: LineView, writes_cache: bool) -> torch.Tensor:
         self._check(writes_cache)
         w, rows = self.w, act.shape[0]
@@ -302,7 +320,7 @@ class GatedDeltaRule(_StateMixer):
         args = (qkv, 0, self.qk_width, 2 * self.qk_width, proj, self.b_off, self.a_off, self.g_off, w["a_log"], w["dt_bias"], w["norm"], ctx,
                 line.state, 0, out)
         sizes = dict(heads=self.num_heads, kv_heads=self.num_kv_heads, dim=self.head_dim, vdim=self.value_dim, eps=self.norm_eps, raw=raw)
-        if (not ctx.is_decode and ctx.max_q_len >= DELTA_CHUNKED_TOKENS
+        if (self.chunks_pay(ctx)
                 and ops.delta_chunks_take(self.head_dim, self.value_dim, (self.conv_channels, self.qk_width), line.state, 0)):
             chunks = ctx.token_chunks(ops.DELTA_CHUNK_TOKENS)
             floats = ops.delta_chunks_scratch_floats(chunks[0].numel(), self.num_heads, self.head_dim, self.value_dim)
