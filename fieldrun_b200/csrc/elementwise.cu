@@ -38,24 +38,6 @@ FRB_API int frb_embed_rows(const int* tokens, const void* table, int table_dtype
     FRB_RETURN_LAUNCH("embed_rows");
 }
 
-// Four neighbouring elements at once.
-template <typename T> __device__ __forceinline__ float4 load4(const T* p);
-template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
-template <> __device__ __forceinline__ float4 load4<bf16>(const bf16* p) {
-    const uint2 raw = *reinterpret_cast<const uint2*>(p);
-    const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&raw.x), hi = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
-    return make_float4(__low2float(lo), __high2float(lo), __low2float(hi), __high2float(hi));
-}
-template <typename T> __device__ __forceinline__ void store4(T* p, float4 v);
-template <> __device__ __forceinline__ void store4<float>(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-template <> __device__ __forceinline__ void store4<bf16>(bf16* p, float4 v) {
-    const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-    uint2 raw;
-    raw.x = *reinterpret_cast<const unsigned int*>(&lo);
-    raw.y = *reinterpret_cast<const unsigned int*>(&hi);
-    *reinterpret_cast<uint2*>(p) = raw;
-}
-
 // ----------------------------------------------------------------------------- RMSNorm (+ residual add)
 
 // Rows are one block each.  A step of few rows takes blocks of 1024 threads (the row's latency is the step's);

@@ -185,3 +185,25 @@ def test_gated_delta_rule_in_chunks(heads, kv_heads, dim, vdim, dtype, decay):
         assert norm_error(results[1][1][slot, copy, 2:-6], results[0][1][slot, copy, 2:-6]) < LIMIT
         results[1][1][slot, copy, 2:-6] = state[slot, copy, 2:-6]
     assert torch.equal(results[1][1], state)                     # nothing else was written
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("rows,width,groups", [(3, 4, 1), (2, 4096, 1), (5, 4100, 1), (2, 9000, 2), (5, 2304, 9), (3, 1024, 1), (1, 1028, 1),
+                                               (7, 780, 3)])
+def test_group_norm_of_four_columns_a_thread(rows, width, groups, dtype):
+    """Parts inside, at and beyond what a block keeps in registers, against 64 bits and against one column a thread."""
+    gen = torch.Generator(device=DEV).manual_seed(width)
+    store = torch.randn(rows * width + 1, device=DEV, generator=gen)
+    weight = torch.randn(width, device=DEV, generator=gen)
+    results = []
+    for place in (0, 1):                                         # 1: the rows do not begin on 16 bytes
+        x = store[place:place + rows * width].copy_(store[:rows * width].clone()).view(rows, width)
+        out = torch.full((rows, width), float("nan"), device=DEV, dtype=getattr(torch, dtype))
+        ops().group_rms_norm(x, weight, out, groups, 1e-6)
+        parts = x.double().view(rows, groups, -1)
+        want = (parts / (parts.square().mean(-1, keepdim=True) + 1e-6).sqrt()).view(rows, width) * weight.double()
+        # a rounding each of the root, the quotient and two products, and the sum's (a few: 128 threads each add up to 72 squares)
+        bound = want.abs() * (2.0 ** -20 if dtype == "float32" else 2.0 ** -8)
+        assert ((out.double() - want).abs() <= bound).all()
+        results.append(out)
+    assert norm_error(results[0].float(), results[1].float()) < (2.0 ** -20 if dtype == "float32" else 2.0 ** -8)
