@@ -126,29 +126,38 @@ __global__ void __launch_bounds__(128) causal_conv_rows_kernel(ConvParams p) {
 }
 
 // The same for prompts of the usual few taps: a thread takes CONV_ROWS rows of four neighbouring channels, 16 bytes at a time,
-// and has registers and multiply-adds for TAPS taps, not for the most there can be.  Bound by its bytes and by silu's
-// arithmetic: both kernels together, 8,192 rows of 3,072 channels 111 -> 70 us (2.9 TB/s), of 6,144 channels 210 -> 122, 1,024 rows
-// of 6,144 channels (where the kernel above has a thread a row) 117 -> 23.
+// and has registers and multiply-adds for TAPS taps, not for the most there can be.  The taps reach the threads through shared memory:
+// read in place, a warp's lanes lie a channel's taps apart and touch 16 lines a load, half of the kernel's time in the load unit.  Bound
+// by its bytes and by silu's arithmetic: both kernels together, 8,192 rows of 3,072 channels 70 -> 58 us (3.5 TB/s), of 6,144 channels
+// 123 -> 103 (3.9), 1,024 rows of 6,144 channels 22 -> 21 (the kernel above: 111, 210, 117).  Eight blocks an SM (64 registers): five
+// (94, as it comes) 64 and 116, seven 73 and 133, nine 63 and 109; four rows a thread 60 and 109, six 82 and 158.
 template <typename OutT, int TAPS>
-__global__ void __launch_bounds__(128) causal_conv_rows4_kernel(ConvParams p) {
+__global__ void __launch_bounds__(128, 8) causal_conv_rows4_kernel(ConvParams p) {
+    __shared__ __align__(16) float s_taps[TAPS][512 + 8];      // 8: a warp's lanes write four taps of eight channels to 32 banks
     after_previous_kernel();
-    const int c = 4 * (blockIdx.y * 128 + threadIdx.x);
-    if (c >= p.channels) return;
+    const int c0 = 512 * blockIdx.y, c = c0 + 4 * threadIdx.x;
+    const bool inside = c < p.channels;
     const int r_begin = blockIdx.x * CONV_ROWS, r_end = min(p.num_rows, r_begin + CONV_ROWS);
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 in_bias = p.in_bias ? *(const float4*)(p.in_bias + c) : zero, bias = p.bias ? *(const float4*)(p.bias + c) : zero;
+    const float4 in_bias = p.in_bias && inside ? *(const float4*)(p.in_bias + c) : zero, bias = p.bias && inside ? *(const float4*)(p.bias + c) : zero;
     const float* in = p.in + p.in_offset + c;
     float4 vals[CONV_ROWS + TAPS - 1];         // the input of row r_begin - (TAPS - 1) + m
 #pragma unroll
     for (int m = 0; m < CONV_ROWS + TAPS - 1; ++m) {
         const int r = r_begin - (TAPS - 1) + m;
-        vals[m] = r >= 0 && r < r_end ? *(const float4*)(in + (size_t)r * p.in_stride) : zero;
+        vals[m] = r >= 0 && r < r_end && inside ? *(const float4*)(in + (size_t)r * p.in_stride) : zero;
     }
-    float w[4][TAPS];
+    const int entries = min(512, p.channels - c0) * TAPS;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int u = 0; u < 4 * TAPS; ++u) {
+        const int e = u * 128 + threadIdx.x;
+        if (e < entries) s_taps[e % TAPS][e / TAPS] = p.taps[(size_t)c0 * TAPS + e];
+    }
+    __syncthreads();
+    if (!inside) return;
+    float4 w[TAPS];
 #pragma unroll
-        for (int k = 0; k < TAPS; ++k) w[i][k] = p.taps[(size_t)(c + i) * TAPS + k];
+    for (int k = 0; k < TAPS; ++k) w[k] = *(const float4*)&s_taps[k][4 * threadIdx.x];
     OutT* typed = (OutT*)p.out_typed;
     const int b_first = p.tok_seq[r_begin], b_last = p.tok_seq[r_end - 1];
     const int row0_first = p.seq.cu_q_len[b_first];
@@ -169,10 +178,10 @@ __global__ void __launch_bounds__(128) causal_conv_rows4_kernel(ConvParams p) {
         float4 acc = bias;
 #pragma unroll
         for (int k = 0; k < TAPS; ++k) {
-            acc.x = fmaf(w[0][k], vals[q + k].x, acc.x);
-            acc.y = fmaf(w[1][k], vals[q + k].y, acc.y);
-            acc.z = fmaf(w[2][k], vals[q + k].z, acc.z);
-            acc.w = fmaf(w[3][k], vals[q + k].w, acc.w);
+            acc.x = fmaf(w[k].x, vals[q + k].x, acc.x);
+            acc.y = fmaf(w[k].y, vals[q + k].y, acc.y);
+            acc.z = fmaf(w[k].z, vals[q + k].z, acc.z);
+            acc.w = fmaf(w[k].w, vals[q + k].w, acc.w);
         }
         acc = make_float4(conv_activation(acc.x, p.activation), conv_activation(acc.y, p.activation), conv_activation(acc.z, p.activation),
                           conv_activation(acc.w, p.activation));
