@@ -1016,6 +1016,8 @@ def rows_f32(w: torch.Tensor, x: torch.Tensor, x_rows: Optional[torch.Tensor], t
     for t, what in ((w, "expert weights"), (x, "their input"), (out, "their output")):
         _want(t, torch.float32, what)
     feats = w.shape[1] // 2 if paired else w.shape[1]
+    if x.dim() != 2 or x.shape[1] != w.shape[2] or out.dim() != 2 or out.shape[1] != feats or (x_rows is None and out.shape[0] < x.shape[0]):
+        raise KernelError(f"{list(w.shape)} weights with rows {list(x.shape)} into {list(out.shape)}")
     _call("frb_rows_f32", _ptr(w), _ptr(x), _ptr(x_rows), _ptr(tile_expert), _ptr(tile_row0), _ptr(num_tiles), _ptr(offsets), max_tiles,
           _ptr(out), feats, w.shape[2], int(paired), float(gate_limit))
 

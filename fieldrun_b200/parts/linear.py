@@ -56,6 +56,14 @@ def full_sums() -> None:
         torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = False
 
 
+def float32_kernels_read(rows: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor]) -> bool:
+    """Whether the float32 kernels may read these operands and write this result: matrices that fit together and lie in one piece
+    from a 16-byte boundary on.  The library takes the others, or refuses them."""
+    return (rows.dim() == 2 and weight.dim() == 2 and rows.shape[1] == weight.shape[1] and rows.numel() > 0
+            and (out is None or (out.shape == (rows.shape[0], weight.shape[0]) and out.dtype == torch.float32 and out.is_contiguous()))
+            and rows.is_contiguous() and weight.is_contiguous() and rows.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
+
+
 def linear(rows: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None, rounded: bool = False,
            split: bool = True) -> torch.Tensor:
     """rows [T, in] @ weight[out, in]^T -> float32 [T, out]; ``split``: whether a large float32 product may run as split products
@@ -73,18 +81,18 @@ def linear(rows: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor]
     if rows.dtype == torch.float32:
         if torch.backends.cuda.matmul.allow_tf32 or torch.get_float32_matmul_precision() != "highest":
             raise RuntimeError("a float32 matrix product was asked for while TF32 is allowed")
-        plain = (rows.is_contiguous() and weight.is_contiguous() and rows.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0
-                 and (out is None or out.is_contiguous()) and rows.numel() > 0)
-        if plain and rows.shape[0] <= STREAM_ROWS and ops.rows_f32_takes(rows.shape[1]):
-            tile_expert, tile_row0, num_tiles, offsets = one_tile(rows.device, rows.shape[0])
+        few = rows.shape[0] <= STREAM_ROWS
+        many = not few and split and rows.shape[0] * weight.numel() >= SPLIT_PRODUCTS
+        if (few or many) and float32_kernels_read(rows, weight, out) \
+                and (ops.rows_f32_takes(rows.shape[1]) if few else ops.products_f32_take(rows.shape[1])):
             result = out if out is not None else torch.empty((rows.shape[0], weight.shape[0]), dtype=torch.float32, device=rows.device)
-            ops.rows_f32(weight.unsqueeze(0), rows, None, tile_expert, tile_row0, num_tiles, offsets, 1, result, paired=False)
-            return result
-        if plain and split and rows.shape[0] * weight.numel() >= SPLIT_PRODUCTS and ops.products_f32_take(rows.shape[1]):
-            result = out if out is not None else torch.empty((rows.shape[0], weight.shape[0]), dtype=torch.float32, device=rows.device)
-            parts = torch.empty((2, *rows.shape), dtype=torch.float16, device=rows.device)
-            scale = torch.empty(rows.shape[0], dtype=torch.float32, device=rows.device)
-            ops.products_f32(weight.unsqueeze(0), ops.weight_scales(weight), rows, parts, scale, result)
+            if few:
+                tile_expert, tile_row0, num_tiles, offsets = one_tile(rows.device, rows.shape[0])
+                ops.rows_f32(weight.unsqueeze(0), rows, None, tile_expert, tile_row0, num_tiles, offsets, 1, result, paired=False)
+            else:
+                parts = torch.empty((2, *rows.shape), dtype=torch.float16, device=rows.device)
+                scale = torch.empty(rows.shape[0], dtype=torch.float32, device=rows.device)
+                ops.products_f32(weight.unsqueeze(0), ops.weight_scales(weight), rows, parts, scale, result)
             return result
         with ops.timed(f"library_mm_f32[{weight.shape[0]}x{weight.shape[1]}]"):
             if out is None:

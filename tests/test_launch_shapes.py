@@ -39,3 +39,27 @@ def test_experts_get_tiles_by_the_rows_an_expert_sees(assignments, decode, tenso
     part = build_part("feed_forward", spec, torch.bfloat16)
     assert part.on_tensor_cores(assignments, decode) == tensor_cores
     assert part.tile_rows(assignments, decode) == expected
+
+
+def test_float32_products_of_operands_that_do_not_fit_are_left_to_the_library():
+    """The kernels take their sizes from the weight: rows of another length, a result of another shape or type and operands in
+    pieces must not reach them (the library refuses the first two, and takes the last)."""
+    import torch
+    from fieldrun_b200.parts.linear import float32_kernels_read
+    rows, weight = torch.zeros(6, 96), torch.zeros(32, 96)
+    assert float32_kernels_read(rows, weight, None) and float32_kernels_read(rows, weight, torch.zeros(6, 32))
+    for other_rows, other_weight, out in ((torch.zeros(6, 64), weight, None), (rows, torch.zeros(32, 128), None), (rows[0], weight, None),
+                                          (rows, weight, torch.zeros(5, 32)), (rows, weight, torch.zeros(6, 31)), (rows, weight, torch.zeros(6 * 32)),
+                                          (rows, weight, torch.zeros(6, 32, dtype=torch.float64)), (rows, weight, torch.zeros(32, 6).t()),
+                                          (torch.zeros(96, 6).t(), weight, None), (rows, torch.zeros(96, 32).t(), None), (rows[:0], weight, None),
+                                          (torch.zeros(6 * 96 + 1)[1:].view(6, 96), weight, None)):
+        assert not float32_kernels_read(other_rows, other_weight, out)
+
+
+def test_float32_rows_are_checked_against_the_weights_before_a_launch():
+    import torch
+    from fieldrun_b200.csrc import ops
+    lists, tile = (torch.zeros(1, dtype=torch.int32),) * 4, 1
+    for x, out in ((torch.zeros(2, 8), torch.zeros(2, 16)), (torch.zeros(2, 12), torch.zeros(2, 8)), (torch.zeros(3, 12), torch.zeros(2, 16))):
+        with pytest.raises(ops.KernelError, match="with rows"):
+            ops.rows_f32(torch.zeros(1, 16, 12), x, None, *lists, tile, out, paired=False)
