@@ -15,7 +15,7 @@ import torch
 from ..cache import CacheNeed, SequenceCache
 from ..config.plan import ModelPlan
 from ..parts import build_block, build_part
-from ..parts.linear import full_sums, require_true_float32
+from ..parts.linear import full_sums, require_true_float32, split_products_reach
 from ..weights.loader import TensorNeed, TensorSource
 from .context import StepContext
 
@@ -113,7 +113,8 @@ class DecoderModel:
         """The libraries of kernels that the model's parts launch from, each once."""
         groups: list[str] = []
         for part in self.all_parts():
-            for group in part.kernel_groups + (("products32",) if self.dtype == torch.float32 else ()):      # their float32 products
+            splits = self.dtype == torch.float32 and split_products_reach(part.dense_needs())
+            for group in part.kernel_groups + (("products32",) if splits else ()):
                 if group not in groups:
                     groups.append(group)
         return groups

@@ -124,7 +124,9 @@ class GQAAttention(Mixer):
             raise ValueError(f"rotary_dim {self.position.rotary_dim} exceeds head_dim {self.head_dim}")
         self.tensor_cores = dtype == torch.bfloat16 and (self.head_dim, self.value_dim) in ops.MMA_HEAD_SIZES
         if not self.tensor_cores:                                # the tensor-core kernels take none of this part's steps
-            self.kernel_groups = ("common", "streams", "attention32") if dtype == torch.float32 else ("common", "streams")
+            float32 = dtype == torch.float32 and (ops.attention_f32_tiles_take(self.head_dim, self.value_dim)
+                                                  or ops.attention_f32_token_takes(self.head_dim, self.value_dim))
+            self.kernel_groups = ("common", "streams", "attention32") if float32 else ("common", "streams")
         # heads as the kernels see them: with two maps per head, two query heads and two key heads
         self.q_heads, self.k_heads = self.maps * self.num_heads, self.maps * self.num_kv_heads
         self.q_width = self.q_heads * self.head_dim

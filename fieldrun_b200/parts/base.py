@@ -65,6 +65,10 @@ class Part:
     def tensor_needs(self) -> list[TensorNeed]:
         return []
 
+    def dense_needs(self) -> list[TensorNeed]:
+        """The tensors whose matrices are multiplied with a step's rows as dense products."""
+        return self.tensor_needs()
+
     def load(self, source: TensorSource) -> None:
         pass
 

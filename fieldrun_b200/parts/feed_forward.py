@@ -126,6 +126,9 @@ class RoutedExperts(FeedForward):
         self.tiles = OneExpertTiles()
         if not self.shared_tc and not (dtype == torch.bfloat16 and self.hidden_size % 128 == 0 and self.expert_width % 128 == 0):
             self.kernel_groups = ("common", "streams", "experts")      # sizes the tcgen05 products never take
+        self.may_split = dtype == torch.float32 and ops.products_f32_take(self.hidden_size) and ops.products_f32_take(self.expert_width)
+        if self.may_split:
+            self.kernel_groups += ("products32",)
         self.router: Optional[torch.Tensor] = None
         self.bias: Optional[torch.Tensor] = None
         self.w13: Optional[torch.Tensor] = None
@@ -162,6 +165,9 @@ class RoutedExperts(FeedForward):
             needs.extend(self._expert_needs(e))
         return needs + self._shared_needs()
 
+    def dense_needs(self):
+        return [TensorNeed(self.name_of("router"), (self.num_experts, self.hidden_size), VECTOR, "normal")] + self._shared_needs()
+
     def load(self, source: TensorSource) -> None:
         d, i, n = self.hidden_size, self.expert_width, self.num_experts
         self.router = source.fetch(TensorNeed(self.name_of("router"), (n, d), VECTOR, "normal"))
@@ -175,7 +181,7 @@ class RoutedExperts(FeedForward):
             self.w13[e, :i].copy_(gate)
             self.w13[e, i:].copy_(up)
             self.w2[e].copy_(down)
-        if self.dtype == torch.float32 and self.w13.is_cuda and ops.products_f32_take(d) and ops.products_f32_take(i):
+        if self.may_split and self.w13.is_cuda:
             self.split_scales = (ops.weight_scales(self.w13), ops.weight_scales(self.w2))
         if self.shared_width:
             fetched = [source.fetch(need) for need in self._shared_needs()]

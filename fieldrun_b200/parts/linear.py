@@ -28,6 +28,14 @@ STREAM_FEATURES = 65536   # beyond this many output features the library product
 # 8192 x 3072 weights, 64 rows 101 | 82, 3,704 rows 3166 | 739; 3072 x 6144, 64 rows 153 | 112; 2048 x 2048,
 # 128 rows 43 | 57, 256 rows 59 | 57; 256 x 3072, 1,024 rows 62 | 73, 2,048 rows 84 | 76.
 SPLIT_PRODUCTS = 1 << 30
+LONG_STEP = 16384         # tokens of the longest step that the generation loop runs
+
+
+def split_products_reach(needs) -> bool:
+    """Whether a step of up to LONG_STEP tokens may run a float32 product with one of these matrices (or with all of them as one weight)
+    as split products: a part whose products stay below that does not ask for their kernels."""
+    sizes = [need.shape[0] * need.shape[1] for need in needs if len(need.shape) == 2 and ops.products_f32_take(need.shape[1])]
+    return sum(sizes) * LONG_STEP >= SPLIT_PRODUCTS
 
 
 def one_tile(device: torch.device, rows: int):

@@ -63,3 +63,23 @@ def test_float32_rows_are_checked_against_the_weights_before_a_launch():
     for x, out in ((torch.zeros(2, 8), torch.zeros(2, 16)), (torch.zeros(2, 12), torch.zeros(2, 8)), (torch.zeros(3, 12), torch.zeros(2, 16))):
         with pytest.raises(ops.KernelError, match="with rows"):
             ops.rows_f32(torch.zeros(1, 16, 12), x, None, *lists, tile, out, paired=False)
+
+
+@pytest.mark.parametrize("hidden,heads,dim,experts,width,vocab,expected", [
+    (3072, 48, 128, 256, 1536, 200064, {"attention32", "products32"}),       # MiniMax-M2's layer
+    (96, 8, 12, 8, 48, 384, {"attention32", "products32"}),                  # small: attention in tiles; experts on the tensor cores
+    (100, 4, 10, 4, 36, 384, set()),                                         # sizes that neither kernel takes
+    (96, 8, 12, 8, 36, 384, {"attention32"}),                                # dense products too small at any step's rows
+    (1024, 4, 130, 4, 36, 2000, {"products32"}),                             # heads beyond both attention kernels, a large head matrix
+])
+def test_a_float32_model_asks_for_the_kernels_its_sizes_use(hidden, heads, dim, experts, width, vocab, expected):
+    import torch
+    from fieldrun_b200.api import build_model
+    from fieldrun_b200.config.registry import architecture_for
+    config = dict(architectures=["MiniMaxM2ForCausalLM"], model_type="minimax_m2", num_hidden_layers=1, hidden_size=hidden,
+                  num_attention_heads=heads, num_key_value_heads=2, head_dim=dim, rotary_dim=2, rope_theta=1e6, use_qk_norm=False,
+                  num_local_experts=experts, num_experts_per_tok=2, intermediate_size=width, vocab_size=vocab, rms_norm_eps=1e-5,
+                  tie_word_embeddings=False)
+    arch = architecture_for(config, "config")
+    model = build_model(arch, arch.config_from_dict(config, "config"), torch.float32)
+    assert set(model.kernel_groups()) == {"common", "streams", "experts"} | expected
