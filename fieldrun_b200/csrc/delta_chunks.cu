@@ -12,7 +12,9 @@
 //   2. along the chunks of a sequence, a block a (sequence, head, 64 value columns) that keeps the state in registers: u = U' - W S,
 //      o, and the new state.
 //   3. the head's root mean square, weight and gate.
-// Weights are exponentials of sums of logarithms over 16 tokens at most, and products of such factors, never a quotient.
+// A weight is the exponential of a sum of logarithms that has its tokens' alone, or a product of such factors: never a quotient, and no
+// difference of two sums either, which behind one strong decay would have lost the digits of the mild ones.  The sums run over up to 16
+// tokens inside a block and up to 48 between blocks: a rounding of their logarithms, which are large only where the weight is small.
 //
 // Everything is float32; the products run on tensor cores with each operand as two TF32 parts (tf32_parts.cuh), over inner sizes of
 // at most 128 entries; a chunk's new state is added to the decayed old one in float32 registers, rounded.  Four prompts of 2,048
@@ -66,6 +68,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
     extern __shared__ float4 dc_smem[];
     __shared__ float beta_s[DC_TOKENS], log_s[DC_TOKENS], to_s[DC_TOKENS], from_s[DC_TOKENS], start_s[DC_TOKENS], q_inv[DC_TOKENS], k_inv[DC_TOKENS];
     __shared__ float block_log[DC_BLOCKS], between[DC_BLOCKS][DC_BLOCKS];
+    __shared__ __align__(16) float own[DC_TOKENS][DC_BLOCK + 4];         // w(j, i) of the tokens j of i's block; zero for later ones
     float* q_s = (float*)dc_smem;                   // [DC_TOKENS][LQ]
     float* k_s = q_s + DC_TOKENS * LQ;              // [DC_TOKENS][LQ]
     float* m_s = k_s + DC_TOKENS * LQ;              // [DC_TOKENS][LS]: M, column by column
@@ -92,7 +95,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
         }
         float tail = __shfl_down_sync(0xffffffffu, behind, 1, DC_BLOCK);
         if (tid % DC_BLOCK == DC_BLOCK - 1) { tail = 0.f; block_log[tid / DC_BLOCK] = before; }
-        log_s[tid] = before;
+        log_s[tid] = la;
         to_s[tid] = expf(before);
         from_s[tid] = expf(tail);
     }
@@ -118,6 +121,16 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
         float sum = 0.f;
         for (int m = j + 1; m < i; ++m) sum += block_log[m];
         between[i][j] = expf(sum);
+    } else if (tid >= 64 && tid < 64 + DC_TOKENS) {  // a token's weights in its block: the sums begin anew for each, at the token itself
+        const int t = tid - 64, i = t % DC_BLOCK;
+        float sum = 0.f, row[DC_BLOCK];
+#pragma unroll
+        for (int j = DC_BLOCK - 1; j >= 0; --j) {
+            row[j] = j <= i ? expf(sum) : 0.f;
+            if (j <= i) sum += log_s[t - i + j];
+        }
+#pragma unroll
+        for (int j = 0; j < DC_BLOCK; j += 4) *(float4*)&own[t][j] = make_float4(row[j], row[j + 1], row[j + 2], row[j + 3]);
     } else if (tid >= 128 && tid < 128 + DC_TOKENS) {
         const int t = tid - 128;
         float sum = 0.f;
@@ -163,7 +176,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
                 for (int e = 0; e < 4; ++e) {
                     const int i = tiles[m] * DC_BLOCK + (lane >> 2) + 8 * (e >> 1), j = n * DC_BLOCK + 8 * odd + 2 * (lane & 3) + (e & 1);
                     const bool seen = keys ? j < i : j <= i;
-                    const float w = !seen ? 0.f : n < tiles[m] ? to_s[i] * between[tiles[m]][n] * from_s[j] : expf(log_s[i] - log_s[j]);
+                    const float w = n < tiles[m] ? to_s[i] * between[tiles[m]][n] * from_s[j] : own[i][j % DC_BLOCK];
                     const float value = seen ? acc[m][n][e] * w * k_inv[j] * (keys ? beta_s[i] * k_inv[i] : q_inv[i]) : 0.f;
                     if (keys) m_s[j * LS + i] = value;
                     else pairs[i * DC_TOKENS + j] = value;

@@ -8,8 +8,10 @@
 //   2. per chunk, 128 columns of the group's heads at a time: the chunk's own contribution U = sum_j B_j (w(j, end) dt_j x_j)^T;
 //   3. along the chunks: the state at each chunk's start over U's place, and the sequence's new state;
 //   4. per chunk and head: y_i = w(start, i) (S^T C_i) + sum_(j <= i) w(j, i) (C_i . B_j) (dt_j x_j), then D x and the gate.
-// Weights are exponentials of sums of logarithms over 16 tokens at most, and products of such factors, never a quotient: the sums
-// stay short, so their rounding stays below that of the decays multiplied one after the other.
+// A weight is the exponential of a sum of logarithms that has its tokens' alone, or a product of such factors: never a quotient, and no
+// difference of two sums either, which behind one strong decay would have lost the digits of the mild ones.  The sums run over up to 16
+// tokens inside a block, 112 between blocks and 127 to the chunk's end: a rounding of their logarithms, which are large only where the
+// weight is small.
 //
 // Everything is float32; the products run on tensor cores with each operand as two TF32 parts (tf32_parts.cuh), over inner sizes
 // of at most 256 entries.  Four prompts of 2,048 tokens, 64 heads of 128 x 64 in 8 groups: 0.65 ms (0.04 + 0.17
@@ -218,12 +220,19 @@ __global__ void __launch_bounds__(256) state_space_chain_kernel(StateSpaceChunks
     *(float4*)(kept + ((start + n) & 1) * p.copy_floats) = S;
 }
 
+// w(j, i) of a chunk's pairs.
+struct ChunkWeights {
+    float to[SC_TOKENS], from[SC_TOKENS], start[SC_TOKENS];              // from its block's start, to its block's end, from the chunk's start
+    float between[SC_BLOCKS][SC_BLOCKS];                                 // the whole blocks between two
+    __align__(16) float own[SC_TOKENS][SC_BLOCK + 8];                    // with the tokens of its block; zero for later ones
+};
+
 // Launch 4.  grid (chunk, head, slice of 64 value columns).  A warp takes row tiles a and 7 - a by 32 columns.
 __global__ void __launch_bounds__(SC_THREADS, 2) state_space_outputs_kernel(StateSpaceChunks p) {
     constexpr int LV = SC_SLICE + 4;
     extern __shared__ float4 sc_smem[];
-    __shared__ float step_s[SC_TOKENS], to_s[SC_TOKENS], from_s[SC_TOKENS], log_s[SC_TOKENS], start_s[SC_TOKENS];
-    __shared__ float block_log[SC_BLOCKS], between[SC_BLOCKS][SC_BLOCKS];
+    __shared__ float step_s[SC_TOKENS], log_s[SC_TOKENS], block_log[SC_BLOCKS];
+    __shared__ ChunkWeights weights;
     constexpr int PART = 32, LP = PART + 8;         // state rows of a part; two parts in turn
     float* parts = (float*)sc_smem;                 // [2]: C [SC_TOKENS][LP], S [PART][LV]
     float* x_s = parts + 2 * (SC_TOKENS * LP + PART * LV);               // [SC_TOKENS][LV]
@@ -242,8 +251,9 @@ __global__ void __launch_bounds__(SC_THREADS, 2) state_space_outputs_kernel(Stat
 
     // a token a thread: its step; the logarithms of the decays from its block's start (with its own) and to its block's end
     if (tid < SC_TOKENS) {
-        const float step = tid < count ? sc_softplus(p.proj[(row0 + tid) * p.proj_stride + p.dt_offset + h] + p.dt_bias[h]) : 0.f;
-        const float la = -expf(p.a_log[h]) * step;
+        const bool in = tid < count;
+        const float step = in ? sc_softplus(p.proj[(row0 + tid) * p.proj_stride + p.dt_offset + h] + p.dt_bias[h]) : 0.f;
+        const float la = in ? -expf(p.a_log[h]) * step : 0.f;
         float before = la, behind = la;
 #pragma unroll
         for (int o = 1; o < SC_BLOCK; o <<= 1) {
@@ -254,21 +264,32 @@ __global__ void __launch_bounds__(SC_THREADS, 2) state_space_outputs_kernel(Stat
         float tail = __shfl_down_sync(0xffffffffu, behind, 1, SC_BLOCK);
         if (tid % SC_BLOCK == SC_BLOCK - 1) { tail = 0.f; block_log[tid / SC_BLOCK] = before; }
         step_s[tid] = step;
-        log_s[tid] = before;
-        to_s[tid] = expf(before);
-        from_s[tid] = expf(tail);
+        log_s[tid] = la;
+        weights.to[tid] = expf(before);
+        weights.from[tid] = expf(tail);
     }
     __syncthreads();
-    if (tid < SC_BLOCKS * SC_BLOCKS) {               // the whole blocks between two
-        const int i = tid / SC_BLOCKS, j = tid % SC_BLOCKS;
-        float sum = 0.f;
-        for (int m = j + 1; m < i; ++m) sum += block_log[m];
-        between[i][j] = expf(sum);
-    } else if (tid >= 128) {
-        const int t = tid - 128;
+    if (tid < SC_TOKENS) {                           // a token's weights in its block: the sums begin anew for each, at the token itself
+        const int i = tid % SC_BLOCK;
+        float sum = 0.f, row[SC_BLOCK];
+#pragma unroll
+        for (int j = SC_BLOCK - 1; j >= 0; --j) {
+            row[j] = j <= i ? expf(sum) : 0.f;
+            if (j <= i) sum += log_s[tid - i + j];
+        }
+#pragma unroll
+        for (int j = 0; j < SC_BLOCK; j += 4) *(float4*)&weights.own[tid][j] = make_float4(row[j], row[j + 1], row[j + 2], row[j + 3]);
+    } else {
+        const int t = tid - SC_TOKENS;
         float sum = 0.f;
         for (int m = 0; m < t / SC_BLOCK; ++m) sum += block_log[m];
-        start_s[t] = expf(sum) * to_s[t];
+        weights.start[t] = expf(sum) * weights.to[t];
+        if (t < SC_BLOCKS * SC_BLOCKS) {
+            const int i = t / SC_BLOCKS, j = t % SC_BLOCKS;
+            sum = 0.f;
+            for (int m = j + 1; m < i; ++m) sum += block_log[m];
+            weights.between[i][j] = expf(sum);
+        }
     }
 
     const int tiles[2] = {warp & 3, 7 - (warp & 3)}, v0 = (warp >> 2) * 32;
@@ -310,7 +331,7 @@ __global__ void __launch_bounds__(SC_THREADS, 2) state_space_outputs_kernel(Stat
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
         const int bi = tiles[m], i0 = bi * SC_BLOCK + (lane >> 2), i1 = i0 + 8;
-        const float e0 = start_s[i0], e1 = start_s[i1];
+        const float e0 = weights.start[i0], e1 = weights.start[i1];
 #pragma unroll
         for (int n = 0; n < 4; ++n) {
             acc[m][n][0] *= e0;
@@ -319,7 +340,7 @@ __global__ void __launch_bounds__(SC_THREADS, 2) state_space_outputs_kernel(Stat
             acc[m][n][3] *= e1;
         }
         const float* at = pairs + i0 * SC_TOKENS + 2 * (lane & 3);
-        const float f0 = to_s[i0], f1 = to_s[i1], l0 = log_s[i0], l1 = log_s[i1];
+        const float f0 = weights.to[i0], f1 = weights.to[i1];
         const int end = (bi + 1) * SC_BLOCK;
         float2 x_next[2], y_next[2];                 // the pairs of a block's 16 columns, asked for a block ahead
 #pragma unroll
@@ -338,13 +359,11 @@ __global__ void __launch_bounds__(SC_THREADS, 2) state_space_outputs_kernel(Stat
             const float2 x = xs[q], y = ys[q];
             float w00, w01, w10, w11;
             if (bj < bi) {
-                const float both = between[bi][bj], u = both * from_s[j], v = both * from_s[j + 1];
+                const float both = weights.between[bi][bj], u = both * weights.from[j], v = both * weights.from[j + 1];
                 w00 = f0 * u; w01 = f0 * v; w10 = f1 * u; w11 = f1 * v;
             } else {
-                w00 = j <= i0 ? expf(l0 - log_s[j]) : 0.f;
-                w01 = j + 1 <= i0 ? expf(l0 - log_s[j + 1]) : 0.f;
-                w10 = j <= i1 ? expf(l1 - log_s[j]) : 0.f;
-                w11 = j + 1 <= i1 ? expf(l1 - log_s[j + 1]) : 0.f;
+                const float2 wx = *(const float2*)&weights.own[i0][j - block0], wy = *(const float2*)&weights.own[i1][j - block0];
+                w00 = wx.x; w01 = wx.y; w10 = wy.x; w11 = wy.y;
             }
             const Tf32Parts a[1][4] = {{tf32_parts(x.x * w00), tf32_parts(y.x * w10), tf32_parts(x.y * w01), tf32_parts(y.y * w11)}};
             Tf32Parts bb[4][2];

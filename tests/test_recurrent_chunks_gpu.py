@@ -207,3 +207,113 @@ def test_group_norm_of_four_columns_a_thread(rows, width, groups, dtype):
         assert ((out.double() - want).abs() <= bound).all()
         results.append(out)
     assert norm_error(results[0].float(), results[1].float()) < (2.0 ** -20 if dtype == "float32" else 2.0 ** -8)
+
+
+# ------------------------------------------------------------------------------- numbers that are not finite, one strong decay
+
+INF, NAN = float("inf"), float("nan")
+LENGTHS, STARTS, SLOTS = [300, 64, 17, 1, 129], [0, 3, 10, 7, 64], [4, 0, 2, 1, 3]
+AT = [int(c) for c in np.concatenate([[0], np.cumsum(LENGTHS)])]
+
+
+def state_space_case():
+    heads, groups, n, vdim = 4, 2, 64, 64
+    gen = torch.Generator(device=DEV).manual_seed(2)
+    tokens, inner = AT[-1], heads * vdim
+    proj, xbc = torch.randn(tokens, inner + heads, device=DEV, generator=gen), torch.randn(tokens, inner + 2 * groups * n, device=DEV, generator=gen) * 0.3
+    proj[:, inner:] -= 3.0
+    dt_bias, a_log, d = (torch.randn(heads, device=DEV, generator=gen) * 0.2 + c for c in (0.0, 0.0, 1.0))
+    state = torch.randn(5, 2, heads * n * vdim, device=DEV, generator=gen)
+    views = {"x": xbc[:, :inner], "b": xbc[:, inner:inner + groups * n], "c": xbc[:, inner + groups * n:], "gate": proj[:, :inner], "decay": proj[:, inner:]}
+    sizes, tabs = dict(heads=heads, vdim=vdim, n=n, groups=groups), Tables(LENGTHS, STARTS, SLOTS)
+
+    def run(chunked):
+        kept, out = state.clone(), torch.full((tokens, inner), NAN, device=DEV)
+        args = (proj, 0, inner, xbc, inner, inner + groups * n, dt_bias, a_log, d, tabs, kept, 0, out)
+        if chunked:
+            chunks = tables(LENGTHS, 128)
+            scratch = torch.full((ops().state_space_chunks_scratch_floats(chunks[0].numel(), **sizes),), NAN, device=DEV)
+            ops().state_space_chunks(*args, chunks=chunks, scratch=scratch, **sizes)
+        else:
+            ops().state_space_scan(*args, **sizes)
+        return out, kept
+
+    def exact():
+        step = torch.nn.functional.softplus(views["decay"].double() + dt_bias.double())
+        decay, x = torch.exp(-a_log.double().exp() * step), views["x"].double().view(tokens, heads, vdim)
+        b, c = (views[m].double().view(tokens, groups, n).repeat_interleave(heads // groups, 1) for m in "bc")
+        outs, states = [], []
+        for row, length in enumerate(LENGTHS):
+            kept = state[SLOTS[row], STARTS[row] & 1].double().view(heads, n, vdim)
+            for t in range(AT[row], AT[row] + length):
+                kept = kept * decay[t][:, None, None] + b[t][:, :, None] * (step[t][:, None] * x[t])[:, None]
+                outs.append((kept * c[t][:, :, None]).sum(1) + d.double()[:, None] * x[t])
+            states.append(kept)
+        return (torch.stack(outs).view(tokens, inner) * torch.nn.functional.silu(views["gate"].double())).view(tokens, heads, vdim), states
+    return views, run, exact
+
+
+def delta_case():
+    heads, kv_heads, dim, vdim = 4, 2, 64, 64
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    tokens, qk, inner = AT[-1], kv_heads * dim, heads * vdim
+    conv, proj = torch.randn(tokens, 2 * qk + inner, device=DEV, generator=gen), torch.randn(tokens, 2 * heads + inner, device=DEV, generator=gen)
+    proj[:, heads:2 * heads] -= 3.0
+    a_log, dt_bias, norm = (torch.randn(*shape, device=DEV, generator=gen) * 0.2 + c for shape, c in (((heads,), 0.0), ((heads,), 0.0), ((vdim,), 1.0)))
+    state = torch.randn(5, 2, heads * dim * vdim, device=DEV, generator=gen)
+    views = {"q": conv[:, :qk], "k": conv[:, qk:2 * qk], "v": conv[:, 2 * qk:], "beta": proj[:, :heads], "decay": proj[:, heads:2 * heads],
+             "gate": proj[:, 2 * heads:]}
+    sizes, tabs = dict(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, eps=1e-6), Tables(LENGTHS, STARTS, SLOTS)
+
+    def run(chunked):
+        kept, out = state.clone(), torch.full((tokens, inner), NAN, device=DEV)
+        raw = torch.full((tokens, inner), NAN, device=DEV)
+        args = (conv, 0, qk, 2 * qk, proj, 0, heads, 2 * heads, a_log, dt_bias, norm, tabs, kept, 0, out)
+        if chunked:
+            chunks = tables(LENGTHS, 64)
+            scratch = torch.full((ops().delta_chunks_scratch_floats(chunks[0].numel(), heads, dim, vdim),), NAN, device=DEV)
+            ops().delta_chunks(*args, raw=raw, chunks=chunks, scratch=scratch, **sizes)
+        else:
+            ops().gated_delta_rule(*args, raw=raw, **sizes)
+        return out, kept
+
+    def exact():
+        q, k = (views[m].double().view(tokens, kv_heads, dim) for m in "qk")
+        q, k = ((z * torch.rsqrt((z * z).sum(-1, keepdim=True) + 1e-6)).repeat_interleave(heads // kv_heads, 1) for z in (q, k))
+        v, beta = views["v"].double().view(tokens, heads, vdim), torch.sigmoid(views["beta"].double())
+        decay = torch.exp(-a_log.double().exp() * torch.nn.functional.softplus(views["decay"].double() + dt_bias.double()))
+        outs, states = [], []
+        for row, length in enumerate(LENGTHS):
+            kept = state[SLOTS[row], STARTS[row] & 1].double().view(heads, dim, vdim)
+            for t in range(AT[row], AT[row] + length):
+                kept = kept * decay[t][:, None, None]
+                u = beta[t][:, None] * (v[t] - (kept * k[t][:, :, None]).sum(1))
+                kept = kept + k[t][:, :, None] * u[:, None]
+                outs.append((kept * q[t][:, :, None]).sum(1) * dim ** -0.5)
+            states.append(kept)
+        o = torch.stack(outs)
+        o = o * torch.rsqrt((o * o).mean(-1, keepdim=True) + 1e-6) * norm.double()
+        return o * torch.nn.functional.silu(views["gate"].double()).view(tokens, heads, vdim), states
+    return views, run, exact
+
+
+CASES = {"state space": state_space_case, "delta": delta_case}
+
+
+@pytest.mark.parametrize("case,strong", [(c, s) for c in ("state space", "delta") for s in (-20.0, -200.0, -2000.0)] + [("delta", -INF)])
+def test_one_strong_decay_among_mild_ones(case, strong):
+    """Tokens that all but clear the state (logarithm of the decay down to about -2,000, and a decay of zero), one in each of some blocks,
+    at the starts of chunks and blocks among them, the others mild: against 64 bits, every token's head by itself.  A weight between
+    tokens behind such a one that is made from sums reaching across it has lost 2,000 2^-24 of its size.  The limit: 128 entries of
+    a sum over the states and 64 of a sum over tokens, a rounding each, on results that are at least an eighth of what they are sums of."""
+    views, run, exact = CASES[case]()
+    for t in (3, 64, 80, 127, 128, 145, 200, 299):
+        views["decay"][t] = -strong
+    want, states = exact()
+    got, kept = run(True)
+    error = (got.double().view_as(want) - want).norm(dim=-1) / want.norm(dim=-1)
+    print(case, strong, "outputs", error.max().item(), "token by token", ((run(False)[0].double().view_as(want) - want).norm(dim=-1) / want.norm(dim=-1)).max().item())
+    assert error.max() < 8 * 192 * 2.0 ** -24
+    for row, slot in enumerate(SLOTS):
+        state = kept[slot, (STARTS[row] + LENGTHS[row]) & 1].double().view_as(states[row])
+        assert ((state - states[row]).norm(dim=(1, 2)) / states[row].norm(dim=(1, 2))).max() < 300 * 2.0 ** -24
