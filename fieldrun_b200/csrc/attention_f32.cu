@@ -119,7 +119,7 @@ attention_f32_tiles_kernel(F32Attention p, const int* __restrict__ tile_seq, con
             a_along(a[0], q_rows + c, ld, lane);
 #pragma unroll
             for (int j = 0; j < 8; ++j) b_along(b[j], k_s + 8 * j * ld + c, ld, lane);
-            mma_tiles_apart<1, 8>(s, small, a, b);
+            mma_tiles_apart(s, small, a, b);
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j)
@@ -174,7 +174,7 @@ attention_f32_tiles_kernel(F32Attention p, const int* __restrict__ tile_seq, con
                 Tf32Parts b[RUN][2];
 #pragma unroll
                 for (int i = 0; i < RUN; ++i) b_along(b[i], v_s + 8 * (n0 + i) * LV + 8 * j, LV, lane);
-                mma_tiles<1, RUN, RUN>(page, 0, a, b);
+                mma_tiles(page, a, b);
             }
 #pragma unroll
             for (int i = 0; i < RUN; ++i) {

@@ -17,8 +17,8 @@
 // tokens inside a block and up to 48 between blocks: a rounding of their logarithms, which are large only where the weight is small.
 //
 // Everything is float32; the products run on tensor cores with each operand as two TF32 parts (tf32_parts.cuh), over inner sizes of
-// at most 128 entries; a chunk's new state is added to the decayed old one in float32 registers, rounded.  Four prompts of 2,048
-// tokens, 16 heads of 128 x 128 over 4 key heads: 0.60 ms (0.19 + 0.37 + 0.04 for the launches in turn; delta_rule.cu token by
+// at most 128 entries, added in float32 registers every 16; so is a chunk's new state to the decayed old one.  Four prompts of 2,048
+// tokens, 16 heads of 128 x 128 over 4 key heads: 0.59 ms (0.19 + 0.36 + 0.04 for the launches in turn; delta_rule.cu token by
 // token 1.38 ms).  Launch 1 issues on 57 % of the cycles (with the values' loads each waited for in turn: 0.37 ms).  Launch 2 is bound
 // by the tensor cores and by the barriers of its three phases: a chunk takes 11.7 us where its products alone take 5.
 #include "tf32_parts.cuh"
@@ -153,17 +153,25 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
     const int tiles[2] = {warp & 1, 3 - (warp & 1)}, odd = warp >> 1 & 1;
     const float* left = keys ? k_s : q_s;
     float acc[2][DC_BLOCKS][4] = {};
-#pragma unroll 2
-    for (int c = 0; c < DIM; c += 8) {
-        Tf32Parts a[2][4], bb[2];
+#pragma unroll 1
+    for (int c = 0; c < DIM; c += 16) {
+        Tf32Parts a[2][2][1][4], bb[2][1][2];
 #pragma unroll
-        for (int m = 0; m < 2; ++m) a_along(a[m], left + tiles[m] * DC_BLOCK * LQ + c, LQ, lane);
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) a_along(a[m][r][0], left + tiles[m] * DC_BLOCK * LQ + c + 8 * r, LQ, lane);
 #pragma unroll
         for (int n = 0; n < DC_BLOCKS; ++n) {
-            b_along(bb, k_s + (n * DC_BLOCK + 8 * odd) * LQ + c, LQ, lane);
+#pragma unroll
+            for (int r = 0; r < 2; ++r) b_along(bb[r][0], k_s + (n * DC_BLOCK + 8 * odd) * LQ + c + 8 * r, LQ, lane);
 #pragma unroll
             for (int m = 0; m < 2; ++m)
-                if (n <= tiles[m]) mma_parts(acc[m][n], a[m], bb);
+                if (n <= tiles[m]) {
+                    float t[1][1][4];
+                    mma_runs(t, a[m], bb);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[m][n][e] += t[0][0][e];
+                }
         }
     }
     float* pairs = p.pairs + at * DC_TOKENS * DC_TOKENS;
@@ -290,12 +298,11 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_chain_kernel(DeltaChunks p
         __syncthreads();                             // W and q are there, and so is the state
         const float* left = (makes_u ? w_s : q_s) + tile * 16 * LQ;
 #pragma unroll 2
-        for (int c = 0; c < DIM; c += 8) {
-            Tf32Parts a[1][4], bb[4][2];
-            a_along(a[0], left + c, LQ, lane);
+        for (int c = 0; c < DIM; c += 16) {
+            Tf32Parts a[2][1][4];
 #pragma unroll
-            for (int n = 0; n < 4; ++n) b_down(bb[n], s_s + c * LV + v0 + 8 * n, LV, lane);
-            mma_tiles<1, 4, 4>(acc, 0, a, bb);
+            for (int r = 0; r < 2; ++r) a_along(a[r][0], left + c + 8 * r, LQ, lane);
+            add_runs<4>(acc, a, [&](Tf32Parts (&b)[2], int r, int n) { b_down(b, s_s + (c + 8 * r) * LV + v0 + 8 * n, LV, lane); });
         }
         if (makes_u) {
 #pragma unroll
@@ -318,12 +325,11 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_chain_kernel(DeltaChunks p
         __syncthreads();                             // u, the pairs' weights and the keys are there; nobody reads W, q and the state any more
         if (item + 1 < last) copy_first(item + 1);
         if (!makes_u) {
-            for (int j = 0; j < (tile + 1) * DC_BLOCK; j += 8) {
-                Tf32Parts a[1][4], bb[4][2];
-                a_along(a[0], a_s + tile * 16 * DC_LM + j, DC_LM, lane);
+            for (int j = 0; j < (tile + 1) * DC_BLOCK; j += 16) {
+                Tf32Parts a[2][1][4];
 #pragma unroll
-                for (int n = 0; n < 4; ++n) b_down(bb[n], u_s + j * LV + v0 + 8 * n, LV, lane);
-                mma_tiles<1, 4, 4>(acc, 0, a, bb);
+                for (int r = 0; r < 2; ++r) a_along(a[r][0], a_s + tile * 16 * DC_LM + j + 8 * r, DC_LM, lane);
+                add_runs<4>(acc, a, [&](Tf32Parts (&b)[2], int r, int n) { b_down(b, u_s + (j + 8 * r) * LV + v0 + 8 * n, LV, lane); });
             }
             const int begin = p.chunk_begin[item], count = p.chunk_end[item] - begin;
 #pragma unroll
@@ -336,21 +342,22 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_chain_kernel(DeltaChunks p
             }
         }
         float fresh[MT][2][4] = {};
-#pragma unroll 2
-        for (int j = 0; j < DC_TOKENS; j += 8) {
-            const float2 f = *(const float2*)&k_factor[item & 1][j + 2 * t4];
-            Tf32Parts a[MT][4], bb[2][2];
+#pragma unroll 1
+        for (int j = 0; j < DC_TOKENS; j += 16) {
+            Tf32Parts a[2][MT][4];
 #pragma unroll
-            for (int m = 0; m < MT; ++m) {
-                const float* x = k_s + (j + 2 * t4) * LK + c0 + 16 * m + g8;
-                a[m][0] = tf32_parts(x[0] * f.x);
-                a[m][1] = tf32_parts(x[8] * f.x);
-                a[m][2] = tf32_parts(x[LK] * f.y);
-                a[m][3] = tf32_parts(x[LK + 8] * f.y);
+            for (int r = 0; r < 2; ++r) {
+                const float2 f = *(const float2*)&k_factor[item & 1][j + 8 * r + 2 * t4];
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    const float* x = k_s + (j + 8 * r + 2 * t4) * LK + c0 + 16 * m + g8;
+                    a[r][m][0] = tf32_parts(x[0] * f.x);
+                    a[r][m][1] = tf32_parts(x[8] * f.x);
+                    a[r][m][2] = tf32_parts(x[LK] * f.y);
+                    a[r][m][3] = tf32_parts(x[LK + 8] * f.y);
+                }
             }
-#pragma unroll
-            for (int n = 0; n < 2; ++n) b_down(bb[n], u_s + j * LV + s0 + 8 * n, LV, lane);
-            mma_tiles<MT, 2, 2>(fresh, 0, a, bb);
+            add_runs<2>(fresh, a, [&](Tf32Parts (&b)[2], int r, int n) { b_down(b, u_s + (j + 8 * r) * LV + s0 + 8 * n, LV, lane); });
         }
 #pragma unroll
         for (int m = 0; m < MT; ++m)

@@ -11,8 +11,8 @@
 // at most one each; within a block the 136 pairs run as the recurrence does, w k_j multiplied by one decay after the other.
 //
 // Everything is float32; the products run on tensor cores with each operand as two TF32 parts (tf32_parts.cuh), over inner
-// sizes of at most 192 entries.  Four prompts of 2,048 tokens, 16 heads of 128 x 128: 0.48 ms (0.19 + 0.04 + 0.26; gla.cu 1.66 ms
-// in segments of 128, whose 500 instructions a warp and token run one after the other).  What bounds them: the instructions around
+// sizes of at most 192 entries, added in float32 registers every 16.  Four prompts of 2,048 tokens, 16 heads of 128 x 128: 0.50 ms
+// (gla.cu 1.66 ms in segments of 128, whose 500 instructions a warp and token run one after the other).  What bounds them: the instructions around
 // the products (60 and 50 % of the issue slots; a decay's two exponentials and a logarithm, the parts, the block's own pairs),
 // with two blocks an SM to hide the rows' way in; with q, k and v loaded where they are used 0.68 ms.
 #include "tf32_parts.cuh"
@@ -127,14 +127,14 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_states_kernel(GlaChun
     for (int tile = warp; tile < TILES; tile += GC_THREADS / 32) {
         const int c0 = tile / (VDIM / 32) * 32, v0 = tile % (VDIM / 32) * 32;
         float acc[2][4][4] = {};
-#pragma unroll 2
-        for (int j = 0; j < GC_TOKENS; j += 8) {
-            Tf32Parts a[2][4], bb[4][2];
+#pragma unroll 1
+        for (int j = 0; j < GC_TOKENS; j += 16) {
+            Tf32Parts a[2][2][4];
 #pragma unroll
-            for (int m = 0; m < 2; ++m) a_down(a[m], k_s + j * LK + c0 + 16 * m, LK, lane);
+            for (int r = 0; r < 2; ++r)
 #pragma unroll
-            for (int n = 0; n < 4; ++n) b_down(bb[n], v_s + j * LV + v0 + 8 * n, LV, lane);
-            mma_tiles<2, 4, 4>(acc, 0, a, bb);
+                for (int m = 0; m < 2; ++m) a_down(a[r][m], k_s + (j + 8 * r) * LK + c0 + 16 * m, LK, lane);
+            add_runs<2>(acc, a, [&](Tf32Parts (&b)[2], int r, int n) { b_down(b, v_s + (j + 8 * r) * LV + v0 + 8 * n, LV, lane); });
         }
 #pragma unroll
         for (int m = 0; m < 2; ++m)
@@ -284,10 +284,13 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_outputs_kernel(GlaChu
                 const float2 w = *(const float2*)&block_decay[m][k0 + 2 * (lane & 3)];
                 x.x *= w.x; x.y *= w.y; y.x *= w.x; y.y *= w.y;
             }
-            const Tf32Parts a[4] = {tf32_parts(x.x), tf32_parts(y.x), tf32_parts(x.y), tf32_parts(y.y)};
-            Tf32Parts bb[2];
-            b_along(bb, k_s + (bj * GC_BLOCK + 8 * (unit & 1)) * LQ + k0, LQ, lane);
-            mma_parts(across[u], a, bb);
+            const Tf32Parts a[1][1][4] = {{{tf32_parts(x.x), tf32_parts(y.x), tf32_parts(x.y), tf32_parts(y.y)}}};
+            Tf32Parts bb[1][1][2];
+            b_along(bb[0][0], k_s + (bj * GC_BLOCK + 8 * (unit & 1)) * LQ + k0, LQ, lane);
+            float t[1][1][4];
+            mma_runs(t, a, bb);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) across[u][e] += t[0][0][e];
         }
     }
     __syncthreads();                                                     // the keys are read
@@ -314,14 +317,14 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_outputs_kernel(GlaChu
     float acc[2][4][4] = {};
     auto with_state = [&](const float* slab, int c0) {
         if (works)
+#pragma unroll 1
+            for (int k0 = 0; k0 < 32; k0 += 16) {
+                Tf32Parts a[2][2][4];
 #pragma unroll
-            for (int k0 = 0; k0 < 32; k0 += 8) {
-                Tf32Parts a[2][4], bb[4][2];
+                for (int r = 0; r < 2; ++r)
 #pragma unroll
-                for (int m = 0; m < 2; ++m) a_along(a[m], q_s + tiles[m] * 16 * LQ + c0 + k0, LQ, lane);
-#pragma unroll
-                for (int n = 0; n < 4; ++n) b_down(bb[n], slab + k0 * LV + v0 + 8 * n, LV, lane);
-                mma_tiles<2, 4, 4>(acc, 0, a, bb);
+                    for (int m = 0; m < 2; ++m) a_along(a[r][m], q_s + tiles[m] * 16 * LQ + c0 + k0 + 8 * r, LQ, lane);
+                add_runs<2>(acc, a, [&](Tf32Parts (&b)[2], int r, int n) { b_down(b, slab + (k0 + 8 * r) * LV + v0 + 8 * n, LV, lane); });
             }
     };
     copies_wait<2>();
@@ -361,12 +364,12 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_outputs_kernel(GlaChu
     if (works)
 #pragma unroll
         for (int m = 0; m < 2; ++m)
-            for (int j = 0; j < (tiles[m] + 1) * GC_BLOCK; j += 8) {
-                Tf32Parts a[1][4], bb[4][2];
-                a_along(a[0], a_s + tiles[m] * 16 * LA + j, LA, lane);
+            for (int j = 0; j < (tiles[m] + 1) * GC_BLOCK; j += 16) {
+                Tf32Parts a[2][1][4];
 #pragma unroll
-                for (int n = 0; n < 4; ++n) b_down(bb[n], v_s + j * LV + v0 + 8 * n, LV, lane);
-                mma_tiles<1, 4, 4>(reinterpret_cast<float (&)[1][4][4]>(acc[m]), 0, a, bb);
+                for (int r = 0; r < 2; ++r) a_along(a[r][0], a_s + tiles[m] * 16 * LA + j + 8 * r, LA, lane);
+                add_runs<4>(reinterpret_cast<float (&)[1][4][4]>(acc[m]), a,
+                                        [&](Tf32Parts (&b)[2], int r, int n) { b_down(b, v_s + (j + 8 * r) * LV + v0 + 8 * n, LV, lane); });
             }
 
     // the head's root mean square over the warps' columns, weight and gate

@@ -14,8 +14,9 @@
 // weight is small.
 //
 // Everything is float32; the products run on tensor cores with each operand as two TF32 parts (tf32_parts.cuh), over inner sizes
-// of at most 256 entries.  Four prompts of 2,048 tokens, 64 heads of 128 x 64 in 8 groups: 0.65 ms (0.04 + 0.17
-// + 0.07 + 0.40 for the launches in turn; scans.cu token by token 1.21 ms).  What bounds them: launch 4 issues on half of the
+// of at most 256 entries, added in float32 registers every 16 (launches 1 and 2: every 8).  Four prompts of 2,048 tokens, 64 heads of
+// 128 x 64 in 8 groups: 0.68 ms (scans.cu token by token 1.21 ms; its four launches took 0.04 + 0.17 + 0.07 + 0.40 of 0.65 with all
+// sums on the tensor cores).  What bounds them: launch 4 issues on half of the
 // cycles, a third of its instructions the operands' parts, and keeps the tensor cores busy for 39 %.
 #include "tf32_parts.cuh"
 
@@ -72,18 +73,23 @@ __global__ void __launch_bounds__(SC_THREADS, 2) state_space_pairs_kernel(StateS
         copies_commit();
         copies_wait<0>();
         __syncthreads();
-#pragma unroll
+#pragma unroll 2
         for (int k = 0; k < 64; k += 8) {
-            Tf32Parts a[2][4], bb[2];
+            Tf32Parts a[2][1][1][4], bb[1][1][2];
 #pragma unroll
-            for (int m = 0; m < 2; ++m) a_along(a[m], c_s + tiles[m] * SC_BLOCK * SC_LC + k, SC_LC, lane);
+            for (int m = 0; m < 2; ++m) a_along(a[m][0][0], c_s + tiles[m] * SC_BLOCK * SC_LC + k, SC_LC, lane);
 #pragma unroll
             for (int n = 0; n < SC_BLOCKS; ++n) {                        // n: the 16 columns of block n, this warp's half of them
                 if (n > tiles[0] && n > tiles[1]) break;
-                b_along(bb, b_s + (n * SC_BLOCK + 8 * odd) * SC_LC + k, SC_LC, lane);
+                b_along(bb[0][0], b_s + (n * SC_BLOCK + 8 * odd) * SC_LC + k, SC_LC, lane);
 #pragma unroll
                 for (int m = 0; m < 2; ++m)
-                    if (n <= tiles[m]) mma_parts(acc[m][n], a[m], bb);
+                    if (n <= tiles[m]) {
+                        float t[1][1][4];
+                        mma_runs(t, a[m], bb);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) acc[m][n][e] += t[0][0][e];
+                    }
             }
         }
     }
@@ -166,15 +172,10 @@ __global__ void __launch_bounds__(SC_THREADS, 2) state_space_states_kernel(State
         __syncthreads();
 #pragma unroll 2
         for (int j = 0; j < PART; j += 8) {
-            Tf32Parts a[2][4], bb[4][2];
+            Tf32Parts a[1][2][4];
 #pragma unroll
-            for (int m = 0; m < 2; ++m) a_down(a[m], b_s + j * LB + c0 + 16 * m, LB, lane);
-#pragma unroll
-            for (int n0 = 0; n0 < NT; n0 += 4) {
-#pragma unroll
-                for (int n = 0; n < 4; ++n) b_down(bb[n], x_s + j * LX + v0 + 8 * (n0 + n), LX, lane);
-                mma_tiles<2, 4, NT>(acc, n0, a, bb);
-            }
+            for (int m = 0; m < 2; ++m) a_down(a[0][m], b_s + j * LB + c0 + 16 * m, LB, lane);
+            add_runs<2>(acc, a, [&](Tf32Parts (&b)[2], int, int n) { b_down(b, x_s + j * LX + v0 + 8 * n, LX, lane); });
         }
     }
 #pragma unroll
@@ -306,14 +307,14 @@ __global__ void __launch_bounds__(SC_THREADS, 2) state_space_outputs_kernel(Stat
         }
         const float* c_s = parts + (part & 1) * (SC_TOKENS * LP + PART * LV);
         const float* s_s = c_s + SC_TOKENS * LP;
-#pragma unroll 2
-        for (int k = 0; k < PART; k += 8) {
-            Tf32Parts a[2][4], bb[4][2];
+#pragma unroll 1
+        for (int k = 0; k < PART; k += 16) {
+            Tf32Parts a[2][2][4];
 #pragma unroll
-            for (int m = 0; m < 2; ++m) a_along(a[m], c_s + tiles[m] * SC_BLOCK * LP + k, LP, lane);
+            for (int r = 0; r < 2; ++r)
 #pragma unroll
-            for (int n = 0; n < 4; ++n) b_down(bb[n], s_s + k * LV + v0 + 8 * n, LV, lane);
-            mma_tiles<2, 4, 4>(acc, 0, a, bb);
+                for (int m = 0; m < 2; ++m) a_along(a[r][m], c_s + tiles[m] * SC_BLOCK * LP + k + 8 * r, LP, lane);
+            add_runs<2>(acc, a, [&](Tf32Parts (&b)[2], int r, int n) { b_down(b, s_s + (k + 8 * r) * LV + v0 + 8 * n, LV, lane); });
         }
     }
     copies_wait<0>();
@@ -353,24 +354,26 @@ __global__ void __launch_bounds__(SC_THREADS, 2) state_space_outputs_kernel(Stat
                 x_next[q] = *(const float2*)(at + block0 + SC_BLOCK + 8 * q);
                 y_next[q] = *(const float2*)(at + 8 * SC_TOKENS + block0 + SC_BLOCK + 8 * q);
             }
+          Tf32Parts a[2][1][4];
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
-            const int j0 = block0 + 8 * q, j = j0 + 2 * (lane & 3), bj = block0 / SC_BLOCK;
+            const int j = block0 + 8 * q + 2 * (lane & 3), bj = block0 / SC_BLOCK;
             const float2 x = xs[q], y = ys[q];
-            float w00, w01, w10, w11;
+            float x0, x1, y0, y1;
             if (bj < bi) {
                 const float both = weights.between[bi][bj], u = both * weights.from[j], v = both * weights.from[j + 1];
-                w00 = f0 * u; w01 = f0 * v; w10 = f1 * u; w11 = f1 * v;
+                x0 = x.x * (f0 * u); x1 = x.y * (f0 * v); y0 = y.x * (f1 * u); y1 = y.y * (f1 * v);
             } else {
                 const float2 wx = *(const float2*)&weights.own[i0][j - block0], wy = *(const float2*)&weights.own[i1][j - block0];
-                w00 = wx.x; w01 = wx.y; w10 = wy.x; w11 = wy.y;
+                x0 = x.x * wx.x; x1 = x.y * wx.y; y0 = y.x * wy.x; y1 = y.y * wy.y;
             }
-            const Tf32Parts a[1][4] = {{tf32_parts(x.x * w00), tf32_parts(y.x * w10), tf32_parts(x.y * w01), tf32_parts(y.y * w11)}};
-            Tf32Parts bb[4][2];
-#pragma unroll
-            for (int n = 0; n < 4; ++n) b_down(bb[n], x_s + j0 * LV + v0 + 8 * n, LV, lane);
-            mma_tiles<1, 4, 4>(reinterpret_cast<float (&)[1][4][4]>(acc[m]), 0, a, bb);
+            a[q][0][0] = tf32_parts(x0);
+            a[q][0][1] = tf32_parts(y0);
+            a[q][0][2] = tf32_parts(x1);
+            a[q][0][3] = tf32_parts(y1);
           }
+          add_runs<4>(reinterpret_cast<float (&)[1][4][4]>(acc[m]), a,
+                                  [&](Tf32Parts (&b)[2], int q, int n) { b_down(b, x_s + (block0 + 8 * q) * LV + v0 + 8 * n, LV, lane); });
         }
     }
     const float dskip = p.d[h];
