@@ -136,6 +136,18 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_states_kernel(GlaChun
                 for (int m = 0; m < 2; ++m) a_down(a[r][m], k_s + (j + 8 * r) * LK + c0 + 16 * m, LK, lane);
             add_runs<2>(acc, a, [&](Tf32Parts (&b)[2], int r, int n) { b_down(b, v_s + (j + 8 * r) * LV + v0 + 8 * n, LV, lane); });
         }
+        if (!all_finite(acc)) {
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int n = 0; n < 4; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (!is_finite(acc[m][n][e]))
+                            acc[m][n][e] = sum_entry_by_entry(k_s + c0 + 16 * m + (lane >> 2) + 8 * (e >> 1), LK,
+                                                              v_s + v0 + 8 * n + 2 * (lane & 3) + (e & 1), LV, nullptr, GC_TOKENS);
+        }
+        __syncwarp();
 #pragma unroll
         for (int m = 0; m < 2; ++m)
 #pragma unroll
@@ -292,6 +304,21 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_outputs_kernel(GlaChu
 #pragma unroll
             for (int e = 0; e < 4; ++e) across[u][e] += t[0][0][e];
         }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (!is_finite(across[u][e])) {
+                const float* q = q_s + (bi * GC_BLOCK + (lane >> 2) + 8 * (e >> 1)) * LQ;
+                const float* k = k_s + (bj * GC_BLOCK + 8 * (unit & 1) + 2 * (lane & 3) + (e & 1)) * LQ;
+                float sum = 0.f;
+#pragma unroll 1
+                for (int c = 0; c < DIM; ++c) {
+                    float x = q[c];
+                    for (int m = bj + 1; m < bi; ++m) x *= block_decay[m][c];
+                    sum = fmaf(x, k[c], sum);
+                }
+                across[u][e] = sum;
+            }
+        __syncwarp();
     }
     __syncthreads();                                                     // the keys are read
     if (SLABS > 2) copy_slab(k_s, 2);
@@ -371,6 +398,21 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_outputs_kernel(GlaChu
                 add_runs<4>(reinterpret_cast<float (&)[1][4][4]>(acc[m]), a,
                                         [&](Tf32Parts (&b)[2], int r, int n) { b_down(b, v_s + (j + 8 * r) * LV + v0 + 8 * n, LV, lane); });
             }
+
+    // a token's output has the tokens up to it alone: where an infinity or a NaN of the block behind it came in with a weight of zero, the
+    // output is added again
+    if (works && !all_finite(acc))
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (!is_finite(acc[m][n][e])) {
+                        const int t = tiles[m] * 16 + 8 * (e >> 1) + (lane >> 2), v = v0 + 8 * n + 2 * (lane & 3) + (e & 1);
+                        acc[m][n][e] = sum_entry_by_entry(q_s + t * LQ, 1, state + v, VDIM, nullptr, DIM) +
+                                       sum_entry_by_entry(a_s + t * LA, 1, v_s + v, LV, nullptr, t + 1);
+                    }
 
     // the head's root mean square over the warps' columns, weight and gate
     if (works)

@@ -141,6 +141,29 @@ __device__ __forceinline__ void b_down(Tf32Parts (&b)[2], const float* at, int s
     b[1] = tf32_parts(x[stride]);
 }
 
+// An infinity has no parts: its lo is a NaN, and so is every product it meets; entries next to the largest float32 round to one.
+// A caller looks at its finished sums and adds those that are not finite again, entry by entry from the operands themselves.
+__device__ __forceinline__ bool is_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+
+template <int M, int NN>
+__device__ __forceinline__ bool all_finite(const float (&c)[M][NN][4]) {
+    float sum = 0.f;                                                     // becomes a NaN at the first that is not
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+#pragma unroll
+        for (int n = 0; n < NN; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sum = fmaf(c[m][n][e], 0.f, sum);
+    return sum == 0.f;
+}
+
+// sum_k a[k] b[k] f[k] (without `f`: all one), the entries of a and b so far apart.
+static __device__ __noinline__ float sum_entry_by_entry(const float* a, size_t a_stride, const float* b, size_t b_stride, const float* f, int count) {
+    float sum = 0.f;
+    for (int k = 0; k < count; ++k) sum = fmaf(f ? a[k * a_stride] * f[k] : a[k * a_stride], b[k * b_stride], sum);
+    return sum;
+}
+
 __device__ __forceinline__ void copy16_async(float* dst, const float* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }

@@ -216,6 +216,31 @@ LENGTHS, STARTS, SLOTS = [300, 64, 17, 1, 129], [0, 3, 10, 7, 64], [4, 0, 2, 1, 
 AT = [int(c) for c in np.concatenate([[0], np.cumsum(LENGTHS)])]
 
 
+def gla_case():
+    """heads x dim x vdim 2 x 64 x 64, decay rank 8: the inputs by name (views of the projection's rows), and run(chunked)."""
+    heads, dim, vdim, rank = 2, 64, 64, 8
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    tokens, width = AT[-1], 2 * heads * (dim + vdim) + rank
+    offsets = (0, heads * dim, 2 * heads * dim, 2 * heads * dim + heads * vdim, 2 * heads * (dim + vdim))
+    proj = torch.randn(tokens, width, device=DEV, generator=gen)
+    a2, bias = torch.randn(heads * dim, rank, device=DEV, generator=gen) * 0.3, torch.randn(heads * dim, device=DEV, generator=gen) + 2.0
+    norm, state = torch.randn(vdim, device=DEV, generator=gen), torch.randn(5, 2, heads, dim, vdim, device=DEV, generator=gen)
+    views = {n: proj[:, a:b] for n, a, b in zip(("q", "k", "v", "gate", "decay"), offsets, (*offsets[1:], width))}
+    sizes = dict(heads=heads, dim=dim, vdim=vdim, tau=16.0, q_scale=dim ** -0.5, eps=1e-6)
+
+    def run(chunked):
+        kept, out = state.clone(), torch.full((tokens, heads * vdim), NAN, device=DEV)
+        args = (proj, offsets, a2, bias, norm, kept, i32(SLOTS), i32(STARTS), i32(AT), out)
+        if chunked:
+            chunks = tables(LENGTHS, 64)
+            scratch = torch.full((ops().gla_chunks_scratch_floats(chunks[0].numel(), tokens, heads, dim, vdim),), NAN, device=DEV)
+            ops().gla_chunks(*args, chunks=chunks, scratch=scratch, **sizes)
+        else:
+            ops().gla_scan(*args, **sizes)
+        return out, kept.view(5, 2, -1)
+    return views, run
+
+
 def state_space_case():
     heads, groups, n, vdim = 4, 2, 64, 64
     gen = torch.Generator(device=DEV).manual_seed(2)
@@ -297,7 +322,38 @@ def delta_case():
     return views, run, exact
 
 
-CASES = {"state space": state_space_case, "delta": delta_case}
+CASES = {"gla": gla_case, "state space": state_space_case, "delta": delta_case}
+
+
+NAMES = [("gla", n) for n in ("q", "k", "v", "decay")]
+
+
+@pytest.mark.parametrize("case,name,number", [(*c, n) for c in NAMES for n in (INF, NAN)])
+def test_a_token_that_is_not_finite_reaches_no_token_before_it(case, name, number):
+    """One entry of a token in the middle of a chunk, of a chunk's last block and of a short sequence: the heads of the outputs and the
+    entries of the states that it makes infinities or NaNs of are those that it does token by token, and the tokens before it keep
+    theirs.  (The largest float32 rounds to an infinity when it is cut in parts; here no product with it is one.)"""
+    views, run = CASES[case]()[:2]
+    hit = [AT[0] + 70, AT[0] + 170, AT[1] + 5, AT[2] + 15]
+    for t in hit:
+        views[name][t, 1] = number
+    want, got = run(False), run(True)
+    clean = torch.ones(AT[-1], dtype=torch.bool, device=DEV)                 # rows that no such number has come into
+    for row, begin in enumerate(AT[:-1]):
+        first = min((t for t in hit if begin <= t < AT[row + 1]), default=AT[row + 1])
+        clean[first:AT[row + 1]] = False
+    assert want[0][clean].isfinite().all() and norm_error(got[0][clean], want[0][clean]) < LIMIT
+    heads = [out.view(AT[-1], -1, 64).isfinite().all(2) for out in (want[0], got[0])]
+    assert torch.equal(*heads)
+    pairs = [(got[0].view(AT[-1], -1, 64)[heads[0]], want[0].view(AT[-1], -1, 64)[heads[0]])]
+    for row, slot in enumerate(SLOTS):
+        copy = (STARTS[row] + LENGTHS[row]) & 1
+        a, b = got[1][slot, copy], want[1][slot, copy]
+        assert torch.equal(a.isfinite(), b.isfinite())
+        pairs.append((a[b.isfinite()], b[b.isfinite()]))
+    for a, b in pairs:
+        if b.numel():
+            assert norm_error(a, b) < LIMIT
 
 
 @pytest.mark.parametrize("case,strong", [(c, s) for c in ("state space", "delta") for s in (-20.0, -200.0, -2000.0)] + [("delta", -INF)])
