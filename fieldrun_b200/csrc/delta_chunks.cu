@@ -185,6 +185,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
                     const int i = tiles[m] * DC_BLOCK + (lane >> 2) + 8 * (e >> 1), j = n * DC_BLOCK + 8 * odd + 2 * (lane & 3) + (e & 1);
                     const bool seen = keys ? j < i : j <= i;
                     const float w = n < tiles[m] ? to_s[i] * between[tiles[m]][n] * from_s[j] : own[i][j % DC_BLOCK];
+                    if (seen && !is_finite(acc[m][n][e])) acc[m][n][e] = sum_entry_by_entry(left + i * LQ, 1, k_s + j * LQ, 1, nullptr, DIM);
                     const float value = seen ? acc[m][n][e] * w * k_inv[j] * (keys ? beta_s[i] * k_inv[i] : q_inv[i]) : 0.f;
                     if (keys) m_s[j * LS + i] = value;
                     else pairs[i * DC_TOKENS + j] = value;
@@ -304,6 +305,14 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_chain_kernel(DeltaChunks p
             for (int r = 0; r < 2; ++r) a_along(a[r][0], left + c + 8 * r, LQ, lane);
             add_runs<4>(acc, a, [&](Tf32Parts (&b)[2], int r, int n) { b_down(b, s_s + (c + 8 * r) * LV + v0 + 8 * n, LV, lane); });
         }
+        if (!all_finite(acc)) {
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (!is_finite(acc[0][n][e]))
+                        acc[0][n][e] = sum_entry_by_entry(left + (g8 + 8 * (e >> 1)) * LQ, 1, s_s + v0 + 8 * n + 2 * t4 + (e & 1), LV, nullptr, DIM);
+        }
         if (makes_u) {
 #pragma unroll
             for (int n = 0; n < 4; ++n) {
@@ -325,12 +334,30 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_chain_kernel(DeltaChunks p
         __syncthreads();                             // u, the pairs' weights and the keys are there; nobody reads W, q and the state any more
         if (item + 1 < last) copy_first(item + 1);
         if (!makes_u) {
+            float with_pairs[1][4][4];
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) with_pairs[0][n][e] = acc[0][n][e];
             for (int j = 0; j < (tile + 1) * DC_BLOCK; j += 16) {
                 Tf32Parts a[2][1][4];
 #pragma unroll
                 for (int r = 0; r < 2; ++r) a_along(a[r][0], a_s + tile * 16 * DC_LM + j + 8 * r, DC_LM, lane);
-                add_runs<4>(acc, a, [&](Tf32Parts (&b)[2], int r, int n) { b_down(b, u_s + (j + 8 * r) * LV + v0 + 8 * n, LV, lane); });
+                add_runs<4>(with_pairs, a, [&](Tf32Parts (&b)[2], int r, int n) { b_down(b, u_s + (j + 8 * r) * LV + v0 + 8 * n, LV, lane); });
             }
+            // a token's output has the tokens up to it alone: where an infinity or a NaN of the block behind it came in with a weight of
+            // zero, the output is added again
+            if (!all_finite(with_pairs)) {
+#pragma unroll
+                for (int n = 0; n < 4; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (!is_finite(with_pairs[0][n][e])) {
+                            const int t = tile * 16 + g8 + 8 * (e >> 1);
+                            with_pairs[0][n][e] = acc[0][n][e] + sum_entry_by_entry(a_s + t * DC_LM, 1, u_s + v0 + 8 * n + 2 * t4 + (e & 1), LV, nullptr, t + 1);
+                        }
+            }
+            __syncwarp();
             const int begin = p.chunk_begin[item], count = p.chunk_end[item] - begin;
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
@@ -338,7 +365,7 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_chain_kernel(DeltaChunks p
                 if (t >= count) continue;
                 float* to = p.raw + ((seq_row0 + begin + t) * p.heads + h) * vdim + column0 + v0 + 2 * t4;
 #pragma unroll
-                for (int n = 0; n < 4; ++n) *(float2*)(to + 8 * n) = make_float2(acc[0][n][2 * half], acc[0][n][2 * half + 1]);
+                for (int n = 0; n < 4; ++n) *(float2*)(to + 8 * n) = make_float2(with_pairs[0][n][2 * half], with_pairs[0][n][2 * half + 1]);
             }
         }
         float fresh[MT][2][4] = {};
@@ -358,6 +385,17 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_chain_kernel(DeltaChunks p
                 }
             }
             add_runs<2>(fresh, a, [&](Tf32Parts (&b)[2], int r, int n) { b_down(b, u_s + (j + 8 * r) * LV + s0 + 8 * n, LV, lane); });
+        }
+        if (!all_finite(fresh)) {
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (!is_finite(fresh[m][n][e]))
+                            fresh[m][n][e] = sum_entry_by_entry(k_s + c0 + 16 * m + g8 + 8 * (e >> 1), LK, u_s + s0 + 8 * n + 2 * t4 + (e & 1), LV,
+                                                                k_factor[item & 1], DC_TOKENS);
         }
 #pragma unroll
         for (int m = 0; m < MT; ++m)
