@@ -93,6 +93,19 @@ __global__ void __launch_bounds__(SC_THREADS, 2) state_space_pairs_kernel(StateS
             }
         }
     }
+    if (!all_finite(acc)) {
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int n = 0; n < SC_BLOCKS; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int i = tiles[m] * SC_BLOCK + (lane >> 2) + 8 * (e >> 1), j = n * SC_BLOCK + 8 * odd + 2 * (lane & 3) + (e & 1);
+                    if (j <= i && i < count && !is_finite(acc[m][n][e]))
+                        acc[m][n][e] = sum_entry_by_entry(rows + (size_t)i * p.xbc_stride + p.c_offset + g * p.N, 1,
+                                                          rows + (size_t)j * p.xbc_stride + p.b_offset + g * p.N, 1, nullptr, p.N);
+                }
+    }
     float* out = p.pairs + ((size_t)item * p.groups + g) * SC_TOKENS * SC_TOKENS;
 #pragma unroll
     for (int m = 0; m < 2; ++m)
@@ -178,6 +191,20 @@ __global__ void __launch_bounds__(SC_THREADS, 2) state_space_states_kernel(State
             add_runs<2>(acc, a, [&](Tf32Parts (&b)[2], int, int n) { b_down(b, x_s + j * LX + v0 + 8 * n, LX, lane); });
         }
     }
+    if (!all_finite(acc)) {
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (!is_finite(acc[m][n][e])) {
+                        const int column = v0 + 8 * n + 2 * (lane & 3) + (e & 1);
+                        acc[m][n][e] = sum_entry_by_entry(rows + p.b_offset + g * N + c0 + 16 * m + (lane >> 2) + 8 * (e >> 1), p.xbc_stride,
+                                                          rows + column0 + column, p.xbc_stride, factor[heads_here == 2 ? column / SC_SLICE : 0],
+                                                          count);
+                    }
+    }
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
         const int column = column0 + v0 + 8 * n, h = column / p.vdim;
@@ -226,7 +253,20 @@ struct ChunkWeights {
     float to[SC_TOKENS], from[SC_TOKENS], start[SC_TOKENS];              // from its block's start, to its block's end, from the chunk's start
     float between[SC_BLOCKS][SC_BLOCKS];                                 // the whole blocks between two
     __align__(16) float own[SC_TOKENS][SC_BLOCK + 8];                    // with the tokens of its block; zero for later ones
+
+    __device__ __forceinline__ float of(int j, int i) const {
+        const int bi = i / SC_BLOCK, bj = j / SC_BLOCK;
+        return bj < bi ? to[i] * (between[bi][bj] * from[j]) : own[i][j % SC_BLOCK];
+    }
 };
+
+// A token's output from the state at the chunk's start and the tokens up to it: sum_n C_n S_n w(start, i) + sum_(j <= i) w(j, i) pair_j x_j.
+static __device__ __noinline__ float output_entry_by_entry(const ChunkWeights& w, int i, const float* c, const float* state, int vdim, int N,
+                                                           const float* pairs, const float* x, int ld) {
+    float sum = sum_entry_by_entry(c, 1, state, vdim, nullptr, N) * w.start[i];
+    for (int j = 0; j <= i; ++j) sum = fmaf(pairs[j] * w.of(j, i), x[j * ld], sum);
+    return sum;
+}
 
 // Launch 4.  grid (chunk, head, slice of 64 value columns).  A warp takes row tiles a and 7 - a by 32 columns.
 __global__ void __launch_bounds__(SC_THREADS, 2) state_space_outputs_kernel(StateSpaceChunks p) {
@@ -365,7 +405,10 @@ __global__ void __launch_bounds__(SC_THREADS, 2) state_space_outputs_kernel(Stat
                 x0 = x.x * (f0 * u); x1 = x.y * (f0 * v); y0 = y.x * (f1 * u); y1 = y.y * (f1 * v);
             } else {
                 const float2 wx = *(const float2*)&weights.own[i0][j - block0], wy = *(const float2*)&weights.own[i1][j - block0];
-                x0 = x.x * wx.x; x1 = x.y * wx.y; y0 = y.x * wy.x; y1 = y.y * wy.y;
+                x0 = j <= i0 ? x.x * wx.x : 0.f;
+                x1 = j + 1 <= i0 ? x.y * wx.y : 0.f;
+                y0 = j <= i1 ? y.x * wy.x : 0.f;
+                y1 = j + 1 <= i1 ? y.y * wy.y : 0.f;
             }
             a[q][0][0] = tf32_parts(x0);
             a[q][0][1] = tf32_parts(y0);
@@ -375,6 +418,21 @@ __global__ void __launch_bounds__(SC_THREADS, 2) state_space_outputs_kernel(Stat
           add_runs<4>(reinterpret_cast<float (&)[1][4][4]>(acc[m]), a,
                                   [&](Tf32Parts (&b)[2], int q, int n) { b_down(b, x_s + (block0 + 8 * q) * LV + v0 + 8 * n, LV, lane); });
         }
+    }
+    // a token's output has the tokens up to it alone: where an infinity or a NaN of the block behind it came in with a weight of zero, the
+    // output is added again
+    if (!all_finite(acc)) {
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int t = tiles[m] * SC_BLOCK + 8 * (e >> 1) + (lane >> 2), v = v0 + 8 * n + 2 * (lane & 3) + (e & 1);
+                    if (t < count && !is_finite(acc[m][n][e]))
+                        acc[m][n][e] = output_entry_by_entry(weights, t, rows + (size_t)t * p.xbc_stride + p.c_offset + g * p.N, state + v, p.vdim,
+                                                             p.N, pairs + t * SC_TOKENS, x_s + v, LV);
+                }
     }
     const float dskip = p.d[h];
 #pragma unroll

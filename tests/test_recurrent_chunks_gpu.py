@@ -325,11 +325,12 @@ def delta_case():
 CASES = {"gla": gla_case, "state space": state_space_case, "delta": delta_case}
 
 
-NAMES = [("gla", n) for n in ("q", "k", "v", "decay")] + [
+NAMES = [("gla", n) for n in ("q", "k", "v", "decay")] + [("state space", n) for n in ("x", "b", "c", "decay")] + [
     ("delta", n) for n in ("q", "k", "v", "beta", "decay")]
 
 
-@pytest.mark.parametrize("case,name,number", [(*c, n) for c in NAMES for n in (INF, NAN)] + [("delta", "v", 3.4028234e38)])
+@pytest.mark.parametrize("case,name,number", [(*c, n) for c in NAMES for n in (INF, NAN)] + [("state space", "x", 3.4028234e38),
+                                                                                             ("delta", "v", 3.4028234e38)])
 def test_a_token_that_is_not_finite_reaches_no_token_before_it(case, name, number):
     """One entry of a token in the middle of a chunk, of a chunk's last block and of a short sequence: the heads of the outputs and the
     entries of the states that it makes infinities or NaNs of are those that it does token by token, and the tokens before it keep
