@@ -324,6 +324,15 @@ attention_f32_token_kernel(F32Attention p, const int* __restrict__ tok_pos, cons
                 float4 v[VR];
 #pragma unroll
                 for (int j = 0; j < VR; ++j) v[j] = *(const float4*)(values + (size_t)(d0 + 2 * j) * FRB_PAGE);
+                const int key = run_at(begin + n, kept, first_page) * FRB_PAGE;
+                if (key < lo || key + FRB_PAGE - 1 > pos) {          // values that the token does not see are left out, whatever they are
+                    const int k0 = key + 4 * l16;
+                    const bool seen[4] = {key_visible(k0, lo, pos, p.keep_first), key_visible(k0 + 1, lo, pos, p.keep_first),
+                                          key_visible(k0 + 2, lo, pos, p.keep_first), key_visible(k0 + 3, lo, pos, p.keep_first)};
+#pragma unroll
+                    for (int j = 0; j < VR; ++j)
+                        v[j] = make_float4(seen[0] ? v[j].x : 0.f, seen[1] ? v[j].y : 0.f, seen[2] ? v[j].z : 0.f, seen[3] ? v[j].w : 0.f);
+                }
 #pragma unroll
                 for (int h = 0; h < GB; ++h) {
                     const float4 w = weights[h][n * (FRB_PAGE / 4) + l16];

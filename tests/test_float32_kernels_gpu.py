@@ -214,3 +214,50 @@ def test_weighted_sums_of_four_columns_equal_those_of_one(width, top_k):
         ops().expert_combine(shifted, weights, rows, out)
         results.append(out)
     assert torch.isfinite(results[0]).all() and torch.equal(*results)
+
+
+def plant(keys, values, table, row, position, key=None, value=None):
+    """A number in one entry of the key, or in one or every entry of the value, of a sequence's token."""
+    page, at = int(table[row, position // 64]), position % 64
+    if key is not None:
+        keys[page, :, at, 1] = key
+    if value is not None:
+        values[page, :, :3, at] = value
+
+
+def same_but_for_rounding(got, want, keys):
+    """NaNs and infinities in the same places, and everything else as close as ever."""
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got.isinf(), want.isinf()) and torch.equal(got[got.isinf()], want[want.isinf()])
+    fine = want.isfinite()
+    assert fine.any() and not fine.all()
+    check(got[fine], want[fine], keys)
+
+
+INF, NAN = float("inf"), float("nan")
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,maps", [SHAPES[0], SHAPES[2], SHAPES[3], SHAPES[4]])
+def test_values_that_a_token_does_not_see_do_not_reach_it(heads, kv_heads, dim, vdim, maps, form):
+    """Single tokens: numbers that are not finite behind a sequence's last token (what an earlier sequence left in the page), and,
+    where a window or a chunk ends, before the first key seen.  One that is seen reaches the result as in the general kernel."""
+    lengths = [1, 64, 65, 256, 257, 700, 130]
+    count = len(lengths)
+    keys, values, table, gen = paged([0] * count, lengths, kv_heads, kv_heads // maps, dim, vdim, 8)
+    for row, n in enumerate(lengths):
+        for at in range(n, (n + 63) // 64 * 64):
+            plant(keys, values, table, row, at, NAN, NAN if at % 2 else INF)
+    for row in (4, 5):
+        plant(keys, values, table, row, lengths[row] - 72, NAN, INF)     # hidden by the windows and the chunks, seen without
+    plant(keys, values, table, 6, 129, value=INF)                        # seen by all
+    plant(keys, values, table, 6, 128, key=3.4e38)
+    q = torch.randn(count, heads * dim, device=DEV, generator=gen)
+    common = dict(num_heads=heads, num_kv_heads=kv_heads, head_dim=dim, v_dim=vdim, scale=dim ** -0.5, maps=maps,
+                  **options(form, heads, count, gen))
+    pos, slots = i32([n - 1 for n in lengths]), i32(range(count))
+    want, got = (torch.full((count, heads * vdim), NAN, device=DEV) for _ in range(2))
+    ops().attention_generic(q, keys, values, table, pos, slots, want, **common)
+    part_o, part_ml = torch.full((count, heads, 3, vdim), NAN, device=DEV), torch.full((count, heads, 3, 2), NAN, device=DEV)
+    ops().attention_f32_token(q, keys, values, table, pos, slots, part_o, part_ml, got, max_chunks=3, **common)
+    same_but_for_rounding(got, want, 700)
