@@ -7,7 +7,7 @@
 // What bounds them.  Prompts: the instructions that split the operands and the tensor cores; attention_generic runs a block per
 // token, which reads the token's keys and values for itself through scalar loads, and a warp's 32 keys through one chain of
 // multiply-adds: 15.2 ms for six prompts of 17 to 1,500 tokens (48 heads over 8 of 128, 3.1 TFLOP/s).  Tiles of 64 queries with 8 x 4
-// scores and 8 x 8 sums a thread on the ordinary pipes took 1.59 ms (30 TFLOP/s), on the tensor cores 1.11 ms (43).  Single tokens: the
+// scores and 8 x 8 sums a thread on the ordinary pipes took 1.59 ms (30 TFLOP/s), on the tensor cores 1.12 ms (43).  Single tokens: the
 // keys' and values' bytes; there a block per token and key head left 48 blocks on 148 SMs, each walking its whole sequence: 1.20 ms
 // for six sequences of 17 to 1,500 keys; the whole layer went from 1.33 to 0.08 ms, most of it the dense products.
 #include "tf32_parts.cuh"
@@ -44,12 +44,57 @@ __device__ __forceinline__ float f32_score(const F32Attention& p, float raw, flo
 #define TILE_Q 64             // queries of one head a block takes
 #define TILE_THREADS 128
 
+// One query of one head key by key in float32, a warp a query: the sums of attention_generic.
+static __device__ __forceinline__ void f32_query_key_by_key(const F32Attention& p, const int* table, int head, int g, int vg, int pos, size_t token) {
+    const int lane = threadIdx.x & 31, hd = p.head_dim, vd = p.v_dim, lo = first_visible_key(pos, p.window, p.chunk);
+    const int first = lo / 32, kept = kept_runs(p.keep_first, 32, first), blocks = kept + pos / 32 - first + 1;
+    const float* q = p.q + (token * p.num_heads + head) * hd;
+    const float slope = p.slopes ? p.slopes[head] : 0.f;
+    float m = -INFINITY, l = 0.f, acc[4] = {};
+    for (int n = 0; n < blocks; ++n) {
+        const int j0 = run_at(n, kept, first) * 32, j = j0 + lane, page = table[j0 / FRB_PAGE], in_page = j0 % FRB_PAGE;
+        const bool visible = key_visible(j, lo, pos, p.keep_first);
+        const float* k = p.k_pages + (((size_t)page * p.num_kv_heads + g) * FRB_PAGE + in_page + lane) * hd;
+        const float* v = p.v_pages + ((size_t)page * p.v_heads + vg) * FRB_PAGE * vd + in_page;
+        float s = 0.f;
+        if (visible)
+            for (int d = 0; d < hd; ++d) s = fmaf(q[d], k[d], s);
+        s = f32_score(p, s, slope, pos, j, visible);
+        const float top = fmaxf(m, warp_max(s)), corr = expf(m - top), w = visible ? expf(s - top) : 0.f;
+        l = l * corr + warp_sum(w);
+        m = top;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i] *= corr;
+        for (int kk = 0; kk < 32; ++kk) {
+            const float wk = __shfl_sync(0xffffffffu, w, kk);
+            if (key_visible(j0 + kk, lo, pos, p.keep_first))
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (lane + 32 * i < vd) acc[i] = fmaf(wk, v[(size_t)(lane + 32 * i) * FRB_PAGE + kk], acc[i]);
+        }
+    }
+    if (p.sinks) {
+        const float sink = p.sinks[head], top = fmaxf(m, sink), corr = expf(m - top);
+        l = l * corr + expf(sink - top);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i] *= corr;
+    }
+    float inv = 1.0f / l;
+    if (p.gate) inv *= 1.0f / (1.0f + expf(-p.gate[token * p.gate_stride + head]));
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (lane + 32 * i < vd) p.out[(token * p.num_heads + head) * vd + lane + 32 * i] = acc[i] * inv;
+}
+
 // A block takes 64 neighbouring queries of one head and walks the pages of 64 keys that any of them sees; a warp has 16 of the
 // queries.  Both products run on tensor cores with each operand as two TF32 parts; the weights stay in the registers that the
 // scores are in, which are those that the second product wants them in.  A page's sums are added to the queries' in float32,
 // rounded (over thousands of keys the tensor cores' adder, which cuts off, would cost more than a rounding).  The next page's keys
 // are on their way while this page's values are summed, its values while the next scores are computed.  NT: column tiles of eight
 // value entries.
+//
+// A query whose results are not all finite is taken again by its warp, key by key and with the hidden ones left out: an infinity has no
+// parts, and a hidden value counts here with a weight of zero, which an infinity or a NaN does not bear.
 template <int NT>
 __global__ void __launch_bounds__(TILE_THREADS, 2)
 attention_f32_tiles_kernel(F32Attention p, const int* __restrict__ tile_seq, const int* __restrict__ tile_q0,
@@ -202,17 +247,26 @@ attention_f32_tiles_kernel(F32Attention p, const int* __restrict__ tile_seq, con
             factor = expf(m[half] - top);
             total = total * factor + expf(sink - top);
         }
-        if (r >= rows) continue;
-        float inv = factor / total;
-        if (p.gate) inv *= 1.0f / (1.0f + expf(-p.gate[(token0 + r) * p.gate_stride + head]));
-        float* out = p.out + ((token0 + r) * p.num_heads + head) * vd;
+        float inv = factor / total, sum = 0.f;                           // sum: becomes a NaN at the first result that is not finite
+        if (r < rows) {
+            if (p.gate) inv *= 1.0f / (1.0f + expf(-p.gate[(token0 + r) * p.gate_stride + head]));
+            float* out = p.out + ((token0 + r) * p.num_heads + head) * vd;
 #pragma unroll
-        for (int i = 0; i < NT; ++i)
+            for (int i = 0; i < NT; ++i)
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int d = 8 * i + 2 * t4 + e;
-                if (d < vd) out[d] = acc[i][2 * half + e] * inv;
-            }
+                for (int e = 0; e < 2; ++e) {
+                    const int d = 8 * i + 2 * t4 + e;
+                    if (d < vd) {
+                        const float x = acc[i][2 * half + e] * inv;
+                        out[d] = x;
+                        sum = fmaf(x, 0.f, sum);
+                    }
+                }
+        }
+        uint32_t again = __ballot_sync(0xffffffffu, sum != 0.f);         // four lanes a query
+        __syncwarp();                                                    // the results above are written before they are written again
+        for (int i = 0; again; ++i, again >>= 4)
+            if (again & 15) f32_query_key_by_key(p, table, head, g, vg, pos0 + warp * 16 + 8 * half + i, token0 + warp * 16 + 8 * half + i);
     }
 }
 

@@ -261,3 +261,33 @@ def test_values_that_a_token_does_not_see_do_not_reach_it(heads, kv_heads, dim, 
     part_o, part_ml = torch.full((count, heads, 3, vdim), NAN, device=DEV), torch.full((count, heads, 3, 2), NAN, device=DEV)
     ops().attention_f32_token(q, keys, values, table, pos, slots, part_o, part_ml, got, max_chunks=3, **common)
     same_but_for_rounding(got, want, 700)
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,maps", [SHAPES[0], SHAPES[2], SHAPES[4], SHAPES[5], SHAPES[6]])
+def test_infinities_and_nans_reach_the_queries_that_see_them(heads, kv_heads, dim, vdim, maps, form):
+    """Prompts: a token's value, key or query that is not finite, or so large that a part of it is not, changes the results of the
+    queries that see it and of no others; what lies behind a sequence's last token changes none."""
+    starts, lengths = [0, 3, 0, 130, 64], [1, 64, 65, 200, 127]
+    keys, values, table, gen = paged(starts, lengths, kv_heads, kv_heads // maps, dim, vdim, 9)
+    tokens, ends = sum(lengths), [s + n for s, n in zip(starts, lengths)]
+    for row, n in enumerate(ends):
+        for at in range(n, (n + 63) // 64 * 64):
+            plant(keys, values, table, row, at, NAN, NAN if at % 2 else INF)
+    plant(keys, values, table, 1, 40, value=INF)
+    plant(keys, values, table, 2, 63, value=NAN)
+    plant(keys, values, table, 2, 64, value=-3.4028234e38)               # rounds to an infinity as a part
+    plant(keys, values, table, 3, 100, key=INF, value=-INF)
+    plant(keys, values, table, 3, 300, key=NAN)
+    plant(keys, values, table, 4, 100, key=3.4028234e38)
+    q = torch.randn(tokens, heads * dim, device=DEV, generator=gen)
+    q[tokens - 10, 2], q[tokens - 5, 1] = INF, NAN
+    common = dict(num_heads=heads, num_kv_heads=kv_heads, head_dim=dim, v_dim=vdim, scale=dim ** -0.5, maps=maps,
+                  **options(form, heads, tokens, gen))
+    pos = np.concatenate([s + np.arange(n) for s, n in zip(starts, lengths)])
+    want, got = (torch.full((tokens, heads * vdim), NAN, device=DEV) for _ in range(2))
+    ops().attention_generic(q, keys, values, table, i32(pos), i32(np.repeat(np.arange(5), lengths)), want, **common)
+    tiles = [(b, q0) for b, n in enumerate(lengths) for q0 in range(0, n, 128)]
+    ops().attention_f32_tiles(q, keys, values, table, i32([t[0] for t in tiles]), i32([t[1] for t in tiles]), i32(range(5)), i32(starts),
+                              i32(lengths), i32(np.concatenate([[0], np.cumsum(lengths)])), got, **common)
+    same_but_for_rounding(got, want, 330)
