@@ -301,6 +301,8 @@ class RoutedExperts(FeedForward):
         sorted_token = p["sorted_token"]
         if scaled is not None:
             act, sorted_token = scaled, None
+        if act.data_ptr() % 16 and (self.on_split_products(p["rows"]) or self.streams_float32(p["rows"])):
+            act = ctx.buffer("experts.aligned", act.shape, torch.float32).copy_(act)      # rows at an odd offset: 16-byte loads
         if self.on_split_products(p["rows"]):
             lists = dict(lists=(p["tile_expert"], p["tile_row0"], p["num_tiles"], p["offsets"]), max_tiles=p["max_tiles"])
             both = ctx.buffer("experts.both", (p["rows"], 2 * self.expert_width), torch.float32)

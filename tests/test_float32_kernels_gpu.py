@@ -291,3 +291,27 @@ def test_infinities_and_nans_reach_the_queries_that_see_them(heads, kv_heads, di
     ops().attention_f32_tiles(q, keys, values, table, i32([t[0] for t in tiles]), i32([t[1] for t in tiles]), i32(range(5)), i32(starts),
                               i32(lengths), i32(np.concatenate([[0], np.cumsum(lengths)])), got, **common)
     same_but_for_rounding(got, want, 330)
+
+
+@pytest.mark.parametrize("tokens", [3, 700])
+def test_experts_take_rows_at_any_offset(tokens):
+    """Rows that do not begin on 16 bytes, few of them (the stream over the weights) and many (the split products)."""
+    from fieldrun_b200.config.plan import PartSpec
+    from fieldrun_b200.engine.context import StepContext, Workspace
+    from fieldrun_b200.parts import build_part
+
+    class Source:
+        def fetch(self, need):
+            gen = torch.Generator(device=DEV).manual_seed(sum(need.name.encode()))
+            return torch.randn(need.shape, device=DEV, generator=gen) * need.shape[-1] ** -0.5
+
+    hidden = 512
+    part = build_part("feed_forward", PartSpec("routed_experts", {"hidden_size": hidden, "num_experts": 4, "top_k": 2, "expert_width": 256,
+                                                                  "renormalize": True},
+                                               {"router": "r", "w_gate": "{e}g", "w_up": "{e}u", "w_down": "{e}d"}), torch.float32)
+    part.load(Source())
+    assert part.on_split_products(2 * tokens) == (tokens == 700)
+    ctx = StepContext(Workspace(DEV), torch.float32, [0], [0], [tokens])
+    rows = torch.randn(tokens, hidden, device=DEV)
+    shifted = torch.zeros(rows.numel() + 1, device=DEV)[1:].view_as(rows).copy_(rows)
+    assert torch.equal(part.forward(ctx, shifted, rows).clone(), part.forward(ctx, rows, rows))
