@@ -224,7 +224,7 @@ class RoutedExperts(FeedForward):
             ops.router_logits(act32, self.router, out)
             return out
         # a model in bfloat16 keeps the library's product: a router has few features, so the split product's tiles leave most of the
-        # device idle (2,048 rows of 256 features: 84 us, 76 split)
+        # device idle (2,048 rows of 256 features: 94 us, 110 split)
         return linear(act32, self.router, split=self.dtype == torch.float32)
 
     def route(self, ctx, act32: torch.Tensor):

@@ -23,11 +23,16 @@ STREAM_ROWS = 8           # up to this many rows a dense product is a stream ove
 STREAM_FEATURES = 65536   # beyond this many output features the library product is at the memory roofline anyway
 
 
-# A float32 product from this many multiply-adds on runs on the tensor cores, each operand as two float16 parts
-# (products_f32.cu).  Measured on a B200, microseconds, the library's float32 product | this one with its scales and parts:
-# 8192 x 3072 weights, 64 rows 101 | 82, 3,704 rows 3166 | 739; 3072 x 6144, 64 rows 153 | 112; 2048 x 2048,
-# 128 rows 43 | 57, 256 rows 59 | 57; 256 x 3072, 1,024 rows 62 | 73, 2,048 rows 84 | 76.
-SPLIT_PRODUCTS = 1 << 30
+# A float32 product runs on the tensor cores, each operand as two float16 parts (products_f32.cu), from SPLIT_PRODUCTS multiply-adds,
+# SPLIT_ROWS rows and SPLIT_TILES tiles of 128 x 128 results on.  Below, the pass over the weight for its scales (half of the bytes of
+# a product of few rows), the launches or the idle SMs cost more than the products save.  Measured on a B200 with weights that are not in
+# L2, microseconds, the library's float32 product | this one with its scales and parts: 200064 x 3072 weights, 9 rows 868 | 1040, 32 rows
+# 901 | 1006, 48 rows 1354 | 1075; 32768 x 4096, 32 rows 224 | 280, 48 rows 347 | 290; 8192 x 3072, 64 rows (2^30) 109 | 120, 96 rows
+# 135 | 126, 2,048 rows 1827 | 609; 3072 x 6144, 128 rows (24 tiles) 178 | 189, 256 rows 254 | 187; 2048 x 2048, 256 rows (2^30) 63 | 87, 512
+# rows 94 | 87; 1024 x 1024, 1,024 rows (2^30) 51 | 71, 2,048 rows 92 | 75; 256 x 3072, 2,048 rows 94 | 110.
+SPLIT_ROWS = 48
+SPLIT_TILES = 32
+SPLIT_PRODUCTS = 1 << 31
 LONG_STEP = 16384         # tokens of the longest step that the generation loop runs
 
 
@@ -64,6 +69,12 @@ def full_sums() -> None:
         torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = False
 
 
+def split_products_pay(rows: int, weight: torch.Tensor) -> bool:
+    tile = ops.PRODUCTS_F32_TILE
+    return (rows * weight.numel() >= SPLIT_PRODUCTS and rows >= SPLIT_ROWS
+            and -(-rows // tile) * -(-weight.shape[0] // tile) >= SPLIT_TILES)
+
+
 def float32_kernels_read(rows: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor]) -> bool:
     """Whether the float32 kernels may read these operands and write this result: matrices that fit together and lie in one piece
     from a 16-byte boundary on.  The library takes the others, or refuses them."""
@@ -90,7 +101,7 @@ def linear(rows: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor]
         if torch.backends.cuda.matmul.allow_tf32 or torch.get_float32_matmul_precision() != "highest":
             raise RuntimeError("a float32 matrix product was asked for while TF32 is allowed")
         few = rows.shape[0] <= STREAM_ROWS
-        many = not few and split and rows.shape[0] * weight.numel() >= SPLIT_PRODUCTS
+        many = split and rows.shape[0] >= SPLIT_ROWS and split_products_pay(rows.shape[0], weight)
         if (few or many) and float32_kernels_read(rows, weight, out) \
                 and (ops.rows_f32_takes(rows.shape[1]) if few else ops.products_f32_take(rows.shape[1])):
             result = out if out is not None else torch.empty((rows.shape[0], weight.shape[0]), dtype=torch.float32, device=rows.device)

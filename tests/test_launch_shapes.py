@@ -83,3 +83,13 @@ def test_a_float32_model_asks_for_the_kernels_its_sizes_use(hidden, heads, dim, 
     arch = architecture_for(config, "config")
     model = build_model(arch, arch.config_from_dict(config, "config"), torch.float32)
     assert set(model.kernel_groups()) == {"common", "streams", "experts"} | expected
+
+
+@pytest.mark.parametrize("rows,features,inner,pays", [
+    (9, 200064, 3072, False), (32, 200064, 3072, False), (48, 200064, 3072, True), (32, 32768, 4096, False), (48, 32768, 4096, True),
+    (64, 8192, 3072, False), (96, 8192, 3072, True), (3704, 8192, 3072, True), (128, 3072, 6144, False), (256, 3072, 6144, True),
+    (256, 2048, 2048, False), (512, 2048, 2048, True), (1024, 1024, 1024, False), (2048, 1024, 1024, True), (2048, 256, 3072, False)])
+def test_float32_products_are_split_where_that_was_measured_to_be_faster(rows, features, inner, pays):
+    import torch
+    from fieldrun_b200.parts.linear import split_products_pay
+    assert split_products_pay(rows, torch.empty(features, inner, device="meta")) == pays
