@@ -883,14 +883,19 @@ def attention_generic(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
           int(out.dtype == torch.float32))
 
 
-def attention_f32_tiles_take(head_dim: int, v_dim: int) -> bool:
-    """Whether :func:`attention_f32_tiles` takes heads of these sizes: rows in 16-byte units, two blocks' tiles on an SM."""
-    return head_dim % 4 == 0 and 4 <= head_dim <= 128 and 1 <= v_dim <= 128
+MAX_GRID_YZ = 65535        # blocks of a grid along y and z
 
 
-def attention_f32_token_takes(head_dim: int, v_dim: int) -> bool:
-    """Whether :func:`attention_f32_token` takes heads of these sizes (it is compiled for the head sizes that models have)."""
-    return head_dim in (32, 64, 96, 128) and (v_dim == head_dim or (head_dim, v_dim) == (64, 128))
+def attention_f32_tiles_take(head_dim: int, v_dim: int, tiles: int = 1) -> bool:
+    """Whether :func:`attention_f32_tiles` takes heads of these sizes (rows in 16-byte units, two blocks' tiles on an SM) and so many
+    tiles of 128 queries (two blocks along y each)."""
+    return head_dim % 4 == 0 and 4 <= head_dim <= 128 and 1 <= v_dim <= 128 and 2 * tiles <= MAX_GRID_YZ
+
+
+def attention_f32_token_takes(head_dim: int, v_dim: int, tokens: int = 1) -> bool:
+    """Whether :func:`attention_f32_token` takes heads of these sizes (it is compiled for the head sizes that models have) and so many
+    tokens (along z)."""
+    return head_dim in (32, 64, 96, 128) and (v_dim == head_dim or (head_dim, v_dim) == (64, 128)) and tokens <= MAX_GRID_YZ
 
 
 def _attention_f32_options(q, k_pages, out, num_heads, num_kv_heads, head_dim, v_dim, scale, window, slopes, chunk, sinks, gate, softcap,

@@ -287,7 +287,7 @@ class GQAAttention(Mixer):
                                           ctx.seq_start, ctx.seq_q_len, ctx.cu_q_len, maps_out, **common)
             if gate is not None:
                 ops.head_gate(out, gate, self.num_heads, self.value_dim)
-        elif self.dtype == torch.float32 and ctx.is_decode and ops.attention_f32_token_takes(self.head_dim, self.value_dim):
+        elif self.dtype == torch.float32 and ctx.is_decode and ops.attention_f32_token_takes(self.head_dim, self.value_dim, ctx.num_seqs):
             # float32: one token a sequence in chunks of keys side by side, prompts in tiles of queries; the general kernel, a
             # block per token, keeps the head sizes neither takes
             chunks = (ctx.max_kv_len + ops.ATTENTION_CHUNK - 1) // ops.ATTENTION_CHUNK
@@ -295,7 +295,8 @@ class GQAAttention(Mixer):
             part_ml = ctx.buffer("attention.part_ml", (ctx.num_seqs, self.q_heads, chunks, 2), torch.float32)
             ops.attention_f32_token(q, line.keys, line.values, line.page_table, ctx.tok_pos, ctx.tok_slot, part_o, part_ml, maps_out,
                                     max_chunks=chunks, gate=gate, **common)
-        elif self.dtype == torch.float32 and not ctx.is_decode and ops.attention_f32_tiles_take(self.head_dim, self.value_dim):
+        elif (self.dtype == torch.float32 and not ctx.is_decode
+              and ops.attention_f32_tiles_take(self.head_dim, self.value_dim, ctx.chunk_count(ops.TC_ATTENTION_QUERIES))):
             tile_seq, tile_q0 = ctx.query_tiles(ops.TC_ATTENTION_QUERIES)
             ops.attention_f32_tiles(q, line.keys, line.values, line.page_table, tile_seq, tile_q0, ctx.seq_slot, ctx.seq_start,
                                     ctx.seq_q_len, ctx.cu_q_len, maps_out, gate=gate, **common)

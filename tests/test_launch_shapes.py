@@ -93,3 +93,9 @@ def test_float32_products_are_split_where_that_was_measured_to_be_faster(rows, f
     import torch
     from fieldrun_b200.parts.linear import split_products_pay
     assert split_products_pay(rows, torch.empty(features, inner, device="meta")) == pays
+
+
+def test_float32_attention_leaves_steps_beyond_its_grid_to_the_general_kernel():
+    from fieldrun_b200.csrc import ops
+    assert ops.attention_f32_tiles_take(128, 128, 32767) and not ops.attention_f32_tiles_take(128, 128, 32768)
+    assert ops.attention_f32_token_takes(128, 128, 65535) and not ops.attention_f32_token_takes(128, 128, 65536)
