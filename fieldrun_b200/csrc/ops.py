@@ -682,6 +682,12 @@ def state_space_scan(proj: torch.Tensor, z_offset: int, dt_offset: int, xbc: tor
 STATE_SPACE_CHUNK_TOKENS = 128
 
 
+def chunks_pay(chunks_us: float, tokens_us: float) -> bool:
+    """Whether a step's recurrence runs in chunks: 5 % for what the two estimates are off by, and 12 us for the chunks' tables, which a
+    step makes and sends once."""
+    return 1.05 * chunks_us + 12.0 < tokens_us
+
+
 def state_space_chunks_take(heads: int, vdim: int, n: int, groups: int, z_offset: int, row: int, xbc_offsets: tuple, state: torch.Tensor,
                             state_offset: int) -> bool:
     """Whether :func:`state_space_chunks` takes ``heads`` of ``n`` x ``vdim`` in ``groups``: tiles of 128 columns inside a group, and

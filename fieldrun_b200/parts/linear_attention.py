@@ -26,10 +26,11 @@ from .base import Mixer, register_part
 from .linear import linear
 
 
-# From this many tokens of the longest prompt on a step may run in chunks as matrix products (gla_chunks.cu).  Measured on a B200,
-# the whole part, microseconds, token by token | in chunks (16 heads of 128 x 128): one prompt of 32 tokens 70 | 90, of 64 tokens
-# 112 | 91, of 1,024 tokens 371 | 140; 16 prompts of 65 tokens 171 | 183, of 130 tokens 332 | 272; 64 of 128 tokens 1235 | 764; one of
-# 256 tokens beside 31 of two 408 | 168.
+# From this many tokens of the longest prompt on a step may run in chunks as matrix products (gla_chunks.cu).  Measured on a B200, the
+# kernels alone, microseconds, token by token | in chunks: 16 heads of 128 x 128, one prompt of 64 tokens 103 | 62, of 1,024 tokens
+# 329 | 87, 16 prompts of 65 tokens 128 | 143, of 130 tokens 257 | 213, one of 128 tokens beside 63 of five 273 | 265; 16 heads of 64 x 64,
+# 16 of 65 tokens 90 | 79, of 130 tokens 162 | 114; 64 heads of 64 x 64, one of 128 beside 63 of five 329 | 436; 64 heads of 128 x 64, 64 of 128
+# tokens 2841 | 1490.
 CHUNKED_TOKENS = 64
 SEGMENT_TOKENS = 128        # other sizes: a long prompt's tokens run in segments of this many, side by side (see gla.cu)
 
@@ -94,13 +95,15 @@ class GatedLinearAttention(Mixer):
         return CacheNeed(state_shape=(2, self.num_heads, self.head_dim, self.value_dim), state_dtype="float32")
 
     def chunks_pay(self, ctx) -> bool:
-        """Whether a step of prompts is faster in chunks.  Token by token it takes as long as its longest prompt, or, with more
-        than two heads an SM, as its tokens shared out; in chunks each (chunk, head) costs about an eighth of a token's time, and
-        the launches thirteen tokens' (fitted to the measurements above)."""
+        """Whether a step of prompts is faster in chunks: microseconds of both ways, fitted to 144 steps of eight head counts and sizes
+        (the measurements above among them; no step of them is slower this way than token by token)."""
         if ctx.is_decode or ctx.max_q_len < CHUNKED_TOKENS:
             return False
-        serial = max(ctx.max_q_len, ctx.num_tokens * self.num_heads / (2 * ops.sm_count(ctx.device)))
-        return 0.13 * ctx.chunk_count(ops.GLA_CHUNK_TOKENS) * self.num_heads + 13 < serial
+        size = self.head_dim * self.value_dim / 2 ** 14                     # as a share of 128 x 128
+        tokens = ctx.num_tokens * self.num_heads
+        serial = max((1.26 + 0.35 * size) * ctx.max_q_len, (0.0042 + 0.0036 * size) * tokens)
+        items = ctx.chunk_count(ops.GLA_CHUNK_TOKENS) * self.num_heads
+        return ops.chunks_pay(max(39 + 24 * size, 23 + (0.05 + 0.19 * size) * items + 0.00056 * tokens), serial)
 
     def forward(self, ctx, act: torch.Tensor, line: LineView, writes_cache: bool) -> torch.Tensor:
         if not writes_cache:

@@ -36,11 +36,11 @@ from .linear import linear
 
 
 # From this many tokens of the longest prompt on a step's recurrence may run in chunks as matrix products (state_space_chunks.cu,
-# delta_chunks.cu).  Measured on a B200, the whole part, microseconds, token by token | in chunks.  State space, 64 heads of 128 x 64:
-# one prompt of 128 tokens 112 | 98 (32 heads 77 | 103), of 1,024 tokens 702 | 216; 4 of 140 tokens 168 | 190; 16 of 130 tokens
-# 438 | 498, of 300 tokens 937 | 840; 64 of 128 tokens 1565 | 1406; one of 256 tokens beside 31 of two 243 | 421.  Delta rule, 16 heads
-# of 128 x 128: one prompt of 64 tokens 104 | 116, of 128 tokens 120 | 93, of 1,024 tokens 716 | 290; 16 of 65 tokens 267 | 222, 64 of 64
-# tokens 831 | 464; one of 128 tokens beside 63 of five 286 | 356; with 16 heads of 64 x 64 16 prompts of 130 tokens 155 | 163.
+# delta_chunks.cu).  Measured on a B200, the kernels alone, microseconds, token by token | in chunks.  State space: 64 heads of 128 x 64, one
+# prompt of 128 tokens 55 | 70, of 1,024 tokens 350 | 119, 16 of 130 tokens 279 | 353, of 256 tokens 525 | 390, one of 256 beside 31 of two
+# 188 | 374; 16 heads of 64 x 64, 64 of 128 tokens 159 | 185; of 128 x 128, 4 of 300 tokens 166 | 119.  Delta rule: 16 heads of 128 x 128, one
+# prompt of 64 tokens 63 | 52, of 1,024 tokens 670 | 231, 16 of 65 tokens 213 | 178, 64 of 64 tokens 687 | 339; 64 heads of 64 x 64, 16 of 65 tokens
+# 205 | 271; 64 heads of 128 x 64, one of 256 beside 31 of two 330 | 449.
 STATE_SPACE_CHUNKED_TOKENS, DELTA_CHUNKED_TOKENS = 128, 64
 
 
@@ -211,13 +211,17 @@ class ScalarDecayStateSpace(_StateMixer):
         self.w = self._fetch(source)
 
     def chunks_pay(self, ctx) -> bool:
-        """Whether a step of prompts is faster in chunks.  Token by token it takes as long as its longest prompt, or, with more
-        than two heads an SM, as its tokens shared out (0.7 us a token); in chunks each (chunk, head) costs 0.18 us and what
-        does not grow with them 85 (fitted to the measurements above, so that no step measured became slower)."""
+        """Whether a step of prompts is faster in chunks: microseconds of both ways, fitted to 144 steps of eight head counts and sizes
+        (the measurements above among them; the worst choice against token by token costs 5 %)."""
         if ctx.is_decode or ctx.max_q_len < STATE_SPACE_CHUNKED_TOKENS:
             return False
-        serial = max(ctx.max_q_len, ctx.num_tokens * self.num_heads / (2 * ops.sm_count(ctx.device)))
-        return 0.18 * ctx.chunk_count(ops.STATE_SPACE_CHUNK_TOKENS) * self.num_heads + 85 < 0.7 * serial
+        rows, columns = self.state / 128, self.value_dim / 128
+        size, blocks, tokens = rows * columns, ctx.num_seqs * self.num_heads, ctx.num_tokens * self.num_heads
+        longest = (0.02 + 0.18 * rows + 0.32 * columns) * ctx.max_q_len
+        crowded = 0.01 * size * self.num_heads * ctx.max_q_len if blocks > 4 * ops.sm_count(ctx.device) else 0.0      # long ones side by side
+        serial = 11 + max(longest + crowded + 0.027 * blocks, 0.29 * longest + (0.00026 + 0.0034 * size) * tokens)
+        items = ctx.chunk_count(ops.STATE_SPACE_CHUNK_TOKENS) * self.num_heads
+        return ops.chunks_pay(max(35 + 32 * rows, 39 + 0.32 * size * items + (0.0009 * columns - 0.00045 * size) * tokens), serial)
 
     def forward(self, ctx, act: torch.Tensor, line: LineView, writes_cache: bool) -> torch.Tensor:
         self._check(writes_cache)
@@ -299,15 +303,16 @@ class GatedDeltaRule(_StateMixer):
         self.w = w
 
     def chunks_pay(self, ctx) -> bool:
-        """Whether a step of prompts is faster in chunks.  Token by token it takes 0.67 us a token of its longest prompt, or, shared
-        out, of one head of 128 x 128 in 64; in chunks each (chunk, head) of that size costs 0.09 us side by side, then 12 us a chunk
-        along the longest prompt, or 0.16 us a (chunk, head) shared out, and the launches 40 (fitted to the measurements above)."""
+        """Whether a step of prompts is faster in chunks: microseconds of both ways, fitted to 144 steps of eight head counts and sizes
+        (the measurements above among them; no step of them is slower this way than token by token)."""
         if ctx.is_decode or ctx.max_q_len < DELTA_CHUNKED_TOKENS:
             return False
-        share = self.num_heads * self.head_dim * self.value_dim / 2 ** 14          # heads of 128 x 128 that these are as much as
-        items = ctx.chunk_count(ops.DELTA_CHUNK_TOKENS) * share
-        serial = max(ctx.max_q_len, ctx.num_tokens * share / 64)
-        return 40 + 0.09 * items + max(12.0 * ctx.max_q_len / ops.DELTA_CHUNK_TOKENS, 0.16 * items) < 0.67 * serial
+        size = self.head_dim * self.value_dim / 2 ** 14                     # as a share of 128 x 128
+        tokens, chunk = ctx.num_tokens * self.num_heads, ops.DELTA_CHUNK_TOKENS
+        serial = 15 + max((0.6 + 0.2 * size) * ctx.max_q_len, (0.0002 + 0.0105 * size) * tokens)
+        items = ctx.chunk_count(chunk) * self.num_heads
+        along = max((6 + 6 * size) * -(-ctx.max_q_len // chunk), (0.026 + 0.13 * size) * items)
+        return ops.chunks_pay(max(42 + 10 * size, 31 + (0.046 + 0.096 * size) * items + along), serial)
 
     def forward(self, ctx, act: torch.Tensor, line: LineView, writes_cache: bool) -> torch.Tensor:
         self._check(writes_cache)

@@ -99,3 +99,28 @@ def test_float32_attention_leaves_steps_beyond_its_grid_to_the_general_kernel():
     from fieldrun_b200.csrc import ops
     assert ops.attention_f32_tiles_take(128, 128, 32767) and not ops.attention_f32_tiles_take(128, 128, 32768)
     assert ops.attention_f32_token_takes(128, 128, 65535) and not ops.attention_f32_token_takes(128, 128, 65536)
+
+
+@pytest.mark.parametrize("kind,heads,dim,vdim,lengths,chunks", [
+    ("gated_linear_attention", 16, 128, 128, [63] * 16, False), ("gated_linear_attention", 16, 128, 128, [64], True),
+    ("gated_linear_attention", 16, 128, 128, [65] * 16, False), ("gated_linear_attention", 16, 128, 128, [130] * 16, True),
+    ("gated_linear_attention", 64, 64, 64, [128] + [5] * 63, False), ("gated_linear_attention", 64, 64, 64, [65] * 16, True),
+    ("scalar_decay_state_space", 64, 128, 64, [128], False), ("scalar_decay_state_space", 64, 128, 64, [256], True),
+    ("scalar_decay_state_space", 64, 128, 64, [130] * 16, False), ("scalar_decay_state_space", 64, 128, 64, [256] * 16, True),
+    ("scalar_decay_state_space", 64, 128, 64, [256] + [2] * 31, False), ("scalar_decay_state_space", 64, 128, 64, [1024] + [16] * 31, True),
+    ("scalar_decay_state_space", 16, 64, 64, [128] * 64, False), ("scalar_decay_state_space", 16, 64, 64, [1024] * 4, True),
+    ("gated_delta_rule", 16, 128, 128, [64], False), ("gated_delta_rule", 16, 128, 128, [128], True),
+    ("gated_delta_rule", 16, 64, 64, [130] * 16, False), ("gated_delta_rule", 64, 64, 64, [65] * 16, False),
+    ("gated_delta_rule", 64, 128, 64, [256] + [2] * 31, False), ("gated_delta_rule", 16, 128, 128, [64] * 64, True)])
+def test_recurrences_run_in_chunks_where_that_was_measured_to_be_faster(kind, heads, dim, vdim, lengths, chunks, monkeypatch):
+    from types import SimpleNamespace
+    import torch
+    from fieldrun_b200.csrc import ops
+    from fieldrun_b200.engine.context import StepContext
+    from test_recurrent_chunks_gpu import mixer_spec
+    from fieldrun_b200.parts import build_part
+    monkeypatch.setattr(ops, "sm_count", lambda device: 148)
+    part = build_part("mixer", mixer_spec(kind, heads, dim, vdim), torch.bfloat16)
+    ctx = SimpleNamespace(seq_q_lens=lengths, num_seqs=len(lengths), num_tokens=sum(lengths), max_q_len=max(lengths), is_decode=False, device=None)
+    ctx.chunk_count = lambda size: StepContext.chunk_count(ctx, size)
+    assert part.chunks_pay(ctx) == chunks

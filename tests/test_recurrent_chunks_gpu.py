@@ -390,3 +390,72 @@ def test_chunks_are_as_near_to_64_bits_as_tokens(case):
         errors.append([norm_error(out.view_as(want), want)] + [norm_error(kept[slot, (start + n) & 1].view_as(state), state)
                                                                for slot, start, n, state in zip(SLOTS, STARTS, LENGTHS, states)])
     assert all(b < 2 * a + 2.0 ** -25 for a, b in zip(*errors)), errors
+
+
+# ------------------------------------------------------------------------------------------- the choice, through the parts
+
+def mixer_spec(kind, heads, dim, vdim):
+    from fieldrun_b200.config.plan import PartSpec
+    args = {"hidden_size": 256, "num_heads": heads, "norm_eps": 1e-6}
+    if kind == "gated_linear_attention":
+        args.update(head_dim=dim, value_dim=vdim, decay_rank=8, tau=16.0)
+        names = ("q_proj", "k_proj", "v_proj", "gate_proj", "decay_in", "decay_out", "decay_bias", "out_norm", "o_proj")
+    elif kind == "gated_delta_rule":
+        args.update(num_kv_heads=heads // 2, head_dim=dim, value_dim=vdim, conv=4)
+        names = ("q_proj", "k_proj", "v_proj", "beta_proj", "decay_proj", "gate_proj", "q_conv", "k_conv", "v_conv", "a_log", "dt_bias", "norm", "o_proj")
+    else:
+        args.update(value_dim=vdim, state=dim, groups=2, norm_groups=1, conv=4)
+        names = ("in_proj", "conv", "conv_bias", "dt_bias", "a_log", "d", "norm", "o_proj")
+    return PartSpec(kind, args, {n: "r/" + n for n in names})
+
+
+def mixer(kind, heads, dim, vdim, dtype):
+    from fieldrun_b200.parts import build_part
+
+    class Source:
+        def fetch(self, need):
+            gen = torch.Generator(device=DEV).manual_seed(sum(need.name.encode()))
+            value = torch.randn(need.shape, device=DEV, generator=gen) * (need.shape[-1] ** -0.5 if need.role == "matrix" else 0.3)
+            return value.to(getattr(torch, dtype)) if need.role == "matrix" else value
+
+    part = build_part("mixer", mixer_spec(kind, heads, dim, vdim), getattr(torch, dtype))
+    part.load(Source())
+    return part
+
+
+@pytest.mark.parametrize("lengths", [[63], [64], [127, 5], [128], [129, 300], [2] * 7 + [256], [1500]])
+@pytest.mark.parametrize("kind", ["gated_linear_attention", "gated_delta_rule", "scalar_decay_state_space"])
+def test_a_prompt_has_the_same_results_on_either_side_of_the_choice(kind, lengths, monkeypatch):
+    """Steps below, at and beyond the lengths where the chunks begin to pay: what the part picks, chunks and token by token."""
+    from fieldrun_b200.cache import SequenceCache
+    from fieldrun_b200.engine.context import StepContext, Workspace
+    part = mixer(kind, 8, 64, 64, "float32")
+    act = torch.randn(sum(lengths), 256, device=DEV, generator=torch.Generator(device=DEV).manual_seed(4))
+
+    def run(chunks):
+        if chunks is not None:
+            monkeypatch.setattr(type(part), "chunks_pay", lambda self, ctx: chunks)
+        cache = SequenceCache([part.cache_need()], max_tokens=64 * len(lengths) + sum(lengths), num_slots=len(lengths), dtype=torch.float32, device=DEV)
+        part.prepare(cache.max_tokens, DEV)
+        slots = [cache.alloc() for _ in lengths]
+        cache.begin_step(slots, lengths)
+        ctx = StepContext(Workspace(DEV), torch.float32, slots, [0] * len(lengths), lengths)
+        update = part.forward(ctx, act, cache.line(0), True)
+        states = cache.line(0).state.view(len(lengths), 2, -1)
+        return update.clone(), [states[b, n & 1].clone() for b, n in enumerate(lengths)], part.chunks_pay(ctx)
+
+    picked, chunked, plain = run(None), run(True), run(False)
+    same = chunked if picked[2] else plain
+    assert torch.equal(picked[0], same[0]) and all(torch.equal(a, b) for a, b in zip(picked[1], same[1]))
+    assert norm_error(chunked[0], plain[0]) < LIMIT
+    for a, b in zip(chunked[1], plain[1]):
+        assert norm_error(a, b) < LIMIT
+
+
+def test_short_steps_and_decode_steps_go_token_by_token_and_long_prompts_in_chunks():
+    from fieldrun_b200.engine.context import StepContext, Workspace
+    for kind in ("gated_linear_attention", "gated_delta_rule", "scalar_decay_state_space"):
+        part, space = mixer(kind, 16, 64, 64, "bfloat16"), Workspace(DEV)
+        pays = lambda lengths: part.chunks_pay(StepContext(space, torch.bfloat16, range(len(lengths)), [0] * len(lengths), lengths))
+        assert not any(pays(lengths) for lengths in ([1], [1] * 64, [30], [63] * 8, [5] * 63 + [64]))
+        assert all(pays(lengths) for lengths in ([2048], [2048] * 4, [1024] + [16] * 4))
