@@ -447,9 +447,9 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_outputs_kernel(GlaChu
 #pragma unroll
                 for (int n = 0; n < 4; ++n) {
                     const int v = v0 + 8 * n + 2 * (lane & 3);
-                    const float2 g = *(const float2*)(gate + v), nw = *(const float2*)(p.norm_w + v);
-                    out[v] = from_f32<OutT>(acc[m][n][2 * half] * rinv * nw.x * (g.x / (1.0f + expf(-g.x))));
-                    out[v + 1] = from_f32<OutT>(acc[m][n][2 * half + 1] * rinv * nw.y * (g.y / (1.0f + expf(-g.y))));
+                    const float2 g = *(const float2*)(gate + v);
+                    out[v] = from_f32<OutT>(acc[m][n][2 * half] * rinv * p.norm_w[v] * (g.x / (1.0f + expf(-g.x))));
+                    out[v + 1] = from_f32<OutT>(acc[m][n][2 * half + 1] * rinv * p.norm_w[v + 1] * (g.y / (1.0f + expf(-g.y))));
                 }
             }
 }

@@ -459,3 +459,21 @@ def test_short_steps_and_decode_steps_go_token_by_token_and_long_prompts_in_chun
         pays = lambda lengths: part.chunks_pay(StepContext(space, torch.bfloat16, range(len(lengths)), [0] * len(lengths), lengths))
         assert not any(pays(lengths) for lengths in ([1], [1] * 64, [30], [63] * 8, [5] * 63 + [64]))
         assert all(pays(lengths) for lengths in ([2048], [2048] * 4, [1024] + [16] * 4))
+
+
+def test_gated_linear_attention_takes_a_norm_weight_at_any_offset():
+    """The output norm's weight as a view that does not begin on eight bytes: the results of the same weight at a boundary."""
+    heads, dim, vdim, rank, tokens = 2, 64, 64, 8, 130
+    gen = torch.Generator(device=DEV).manual_seed(5)
+    offsets = (0, heads * dim, 2 * heads * dim, 3 * heads * dim, 4 * heads * dim)
+    proj = torch.randn(tokens, offsets[4] + rank, device=DEV, generator=gen)
+    a2, bias = torch.randn(heads * dim, rank, device=DEV, generator=gen), torch.randn(heads * dim, device=DEV, generator=gen)
+    store, results = torch.randn(vdim + 1, device=DEV, generator=gen), []
+    for norm in (store[1:], store[1:].clone()):
+        state, out = torch.zeros(1, 2, heads, dim, vdim, device=DEV), torch.empty(tokens, heads * vdim, device=DEV)
+        chunks = tables([tokens], 64)
+        ops().gla_chunks(proj, offsets, a2, bias, norm, state, i32([0]), i32([0]), i32([0, tokens]), out, heads=heads, dim=dim, vdim=vdim, tau=16.0,
+                         q_scale=0.125, eps=1e-6, chunks=chunks,
+                         scratch=torch.empty(ops().gla_chunks_scratch_floats(chunks[0].numel(), tokens, heads, dim, vdim), device=DEV))
+        results.append(out)
+    assert torch.equal(*results)
