@@ -52,7 +52,7 @@ _SIGNATURES = {
     "frb_rows_f32": "pppppppipiiif",
     "frb_weight_scales": "ppli",
     "frb_split_rows": "pppplii" "f",
-    "frb_products_f32": "ppippl" "ppif" "ppppip" "iip",
+    "frb_products_f32": "ppippl" "ppif" "ppppip" "iipp",
     "frb_sample_rows": "piipppp",
     "frb_argmax_rows": "piippp",
     "frb_sample_floor": "piippppppp",
@@ -201,7 +201,7 @@ def _stream() -> int:
 
 
 _LAUNCHES = 0
-_KERNELS_PER_CALL = {"frb_gated_delta_rule": 2, "frb_gated_recurrence": 2, "frb_sample_floor": 3, "frb_argmax_rows": 2, "frb_expert_plan": 3, "frb_attention_decode_mma": 2, "frb_attention_decode_tma": 2, "frb_attention_f32_token": 2, "frb_gla_chunks": 3, "frb_state_space_chunks": 4, "frb_delta_chunks": 3}
+_KERNELS_PER_CALL = {"frb_gated_delta_rule": 2, "frb_gated_recurrence": 2, "frb_sample_floor": 3, "frb_argmax_rows": 2, "frb_expert_plan": 3, "frb_attention_decode_mma": 2, "frb_attention_decode_tma": 2, "frb_attention_f32_token": 2, "frb_gla_chunks": 3, "frb_state_space_chunks": 4, "frb_delta_chunks": 3, "frb_products_f32": 2}
 
 
 def launches() -> int:
@@ -1034,6 +1034,7 @@ def rows_f32(w: torch.Tensor, x: torch.Tensor, x_rows: Optional[torch.Tensor], t
 
 
 PRODUCTS_F32_TILE = 128    # rows of a tile of products_f32
+PRODUCTS_F32_AGAIN = 8 * (32 * 8 + 1)      # bytes of scratch for a tile and 128 features (FRB_PRODUCTS_AGAIN)
 
 
 def products_f32_take(inner: int) -> bool:
@@ -1073,9 +1074,10 @@ def products_f32(w: torch.Tensor, w_scale: torch.Tensor, x: torch.Tensor, parts:
         if experts != 1:
             raise KernelError("products without lists are of one weight matrix")
         lists, max_tiles = (None, None, None, None), (count + PRODUCTS_F32_TILE - 1) // PRODUCTS_F32_TILE
+    again = torch.empty(PRODUCTS_F32_AGAIN * max_tiles * -(-feats // 128), dtype=torch.uint8, device=w.device)
     _call("frb_split_rows", _ptr(x), _ptr(x_rows), _ptr(parts), _ptr(x_scale), count, inner, int(gated), float(gate_limit))
     _call("frb_products_f32", _ptr(w), _ptr(w_scale), experts, _ptr(parts), _ptr(x_scale), count, _ptr(x), _ptr(x_rows), int(gated),
-          float(gate_limit), *(_ptr(t) for t in lists), max_tiles, _ptr(out), feats, inner, _ptr(tc_status(w.device)))
+          float(gate_limit), *(_ptr(t) for t in lists), max_tiles, _ptr(out), feats, inner, _ptr(again), _ptr(tc_status(w.device)))
 
 
 def sample_rows(logits: torch.Tensor, temperature: Optional[torch.Tensor], uniform: Optional[torch.Tensor],

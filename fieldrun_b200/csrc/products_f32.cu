@@ -1,8 +1,8 @@
 // Products of many float32 rows with float32 weights on the tensor cores (tcgen05), each operand as two float16 parts.
 //
 // y[row, f] = sum_k x[row, k] W_e[f, k].  Every row of x and every weight row is multiplied by a power of two that brings its
-// largest entry to [2^14, 2^15), then split into hi = float16(v) and lo = float16(v - hi).  Entries down to 2^-17 of the row's
-// largest keep 22 bits or more, smaller ones an absolute error of 2^-40 of that largest; the product is hi hi + (hi lo + lo hi),
+// largest entry to [2^14, 2^15), then split into hi = float16(v) and lo = float16(2^11 (v - hi)).  Entries down to 2^-29 of the row's
+// largest keep 22 bits or more, smaller ones an absolute error of 2^-51 of that largest; the product is hi hi + 2^-11 (hi lo + lo hi),
 // whose terms are exact in float32, and lo lo is below 2^-22 of it.  What would cost precision is the tensor cores' adder: it
 // cuts the sum off instead of rounding it, so an error grows by about 1e-9 of the sum with every entry of the inner size
 // (measured: 2.3e-7 of the result after 256 entries, 3.2e-6 after 3,072).  So the large products (hi hi) are summed in tensor
@@ -10,8 +10,10 @@
 // that, have accumulators of their own.  Against 64-bit sums the result is off by 3.6e-7 at any inner size from 2,048 to 6,144;
 // the library's float32 product by 2e-7 to 1.4e-6, the kernel for any sizes (experts_generic.cu) by 1.7e-6.
 //
-// Rows with an infinity or a NaN or without an entry of 2^-112 (of x or of the weights) have no such scale: it is set to 0, and
-// the outputs that such a row meets are summed again entry by entry in float32.
+// Some outputs are summed again entry by entry in float32: those of rows without a scale (rows with an infinity or a NaN or without an
+// entry of 2^-112); and those so small that entries below 2^-29 of their rows' largest may have had a part in them.  In units of the scaled rows each such entry is off by at most 2^-36 and meets entries below 2^15, so a sum
+// of K is off by less than K 2^-20, both sides together: 2^-25 of any sum from 32 K on, where the largest product is 2^30.  Of rows
+// of normally distributed numbers one output in 40,000 is below that.
 //
 // What bounds it: 3,704 tokens on MiniMax-M2's 256 experts have to read 14.5 GB of weights (2.2 ms) and take 2.5 PFLOP of
 // float16 products (1.6 ms at the tensor cores' peak).  The two products of those sizes take 4.6 ms (in tiles of eight rows on
@@ -61,6 +63,9 @@ struct ProductsParams {
     float gate_limit;
     const int *tile_expert, *tile_row0, *num_tiles, *offsets;
     float* out;                // [rows, F]
+    // outputs to be summed again: for every item and worker whether there are any, and, if so, a lane's columns
+    uint8_t* again;            // [items * PF_WORKERS]
+    unsigned long long* columns;               // [items * PF_WORKERS][32]
     int* status;
     int F, K, tiles;           // tiles: without lists
     long long rows_total;
@@ -71,26 +76,18 @@ struct ProductsParams {
     __device__ __forceinline__ int end_row(int e) const { return offsets ? offsets[e + 1] : (int)rows_total; }
 };
 
-// An output that a row without a scale meets, summed entry by entry.
-__device__ __noinline__ float product_entry_by_entry(const ProductsParams& p, long long w_row, long long row) {
-    const float* w = p.W + w_row * p.K;
-    const float* x = p.x + (p.x_rows ? p.x_rows[row] : row) * (p.gated ? 2ll * p.K : (long long)p.K);
-    float sum = 0.f;
-    for (int k = 0; k < p.K; ++k) sum = fmaf(p.gated ? paired_gate(x[k], x[p.K + k], p.gate_limit) : x[k], w[k], sum);
-    return sum;
-}
-
 __device__ __forceinline__ uint32_t half2_bits(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
 
-// The parts of four entries times their row's scale.
+// The parts of four entries times their row's scale; lo is 2^11 times what hi leaves, so that it is no smaller than hi.
+#define PF_LO 2048.f
 __device__ __forceinline__ void split_four(float4 v, float scale, uint32_t& hi0, uint32_t& hi1, uint32_t& lo0, uint32_t& lo1) {
     const float a = v.x * scale, b = v.y * scale, c = v.z * scale, d = v.w * scale;
     const __half2 h0 = __floats2half2_rn(a, b), h1 = __floats2half2_rn(c, d);
     const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
     hi0 = half2_bits(h0);
     hi1 = half2_bits(h1);
-    lo0 = half2_bits(__floats2half2_rn(a - f0.x, b - f0.y));
-    lo1 = half2_bits(__floats2half2_rn(c - f1.x, d - f1.y));
+    lo0 = half2_bits(__floats2half2_rn((a - f0.x) * PF_LO, (b - f0.y) * PF_LO));
+    lo1 = half2_bits(__floats2half2_rn((c - f1.x) * PF_LO, (d - f1.y) * PF_LO));
 }
 
 // A wait of a whole warp: either all of its lanes go on or none.
@@ -98,8 +95,13 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volati
     return __all_sync(0xffffffffu, bar_wait(bar, parity, failed));
 }
 
-// The exponent of a scale, a power of two.
-__device__ __forceinline__ int scale_exponent(float scale) { return (int)(__float_as_uint(scale) >> 23) - 127; }
+// The exponent of a scale, a power of two, whatever its sign: -1 marks a row of zeros.
+__device__ __forceinline__ int scale_exponent(float scale) { return (int)(__float_as_uint(scale) >> 23 & 255) - 127; }
+
+// Whether an output is zero for its row's or its weight row's zeros (the other being finite, and the sum zero still).
+__device__ __forceinline__ bool is_of_zeros(float sum, float w_scale, float x_scale) {
+    return sum == 0.f && (x_scale < 0.f ? w_scale != 0.f : w_scale < 0.f && x_scale != 0.f);
+}
 
 __global__ void __launch_bounds__(PF_THREADS, 1)
 products_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
@@ -217,8 +219,7 @@ products_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 #pragma unroll
         for (int i = 0; i < PF_COLS; ++i) sums[i] = 0.f;
         // of the item in hand, and of the chunk that is finished but not taken yet (0: none, 1: one, 2: its item's last)
-        int row0 = 0, rows = 0, f = 0, taken_row0 = 0, taken_rows = 0, taken_f = 0, pending = 0;
-        long long w_row = 0, taken_w_row = 0;
+        int row0 = 0, rows = 0, f = 0, taken_row0 = 0, taken_rows = 0, taken_f = 0, taken_item = 0, pending = 0;
         float taken_scale = 0.f;
 
         // Each turn splits one step's weights, then takes the chunk that the turn before it finished: the tensor cores have this
@@ -231,8 +232,7 @@ products_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     row0 = p.first_row(tile) + part * PF_COLS;
                     rows = min(PF_COLS, p.end_row(e) - row0);            // of this part's columns; 0 or less: none
                     f = (item - tile * feature_blocks) * PF_FEATS + r;
-                    w_row = (long long)e * p.F + min(f, p.F - 1);
-                    scale = p.w_scale[w_row];
+                    scale = p.w_scale[(long long)e * p.F + min(f, p.F - 1)];
                 }
                 if (!warp_wait(&w_full[ws], w_parity, &failed)) { if (lane == 0) atomicExch(p.status, 48); break; }
                 // 32 entries of a row are 128 bytes of a box; 16-byte chunk c of row r lies at chunk c ^ (r & 7)
@@ -282,28 +282,37 @@ products_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                         if (c + 1 < PF_COLS / 16 && 16 * (c + 1) < taken_rows) tmem_ld16(small + 16 * (c + 1), v[(c + 1) & 1]);
                         if (16 * c < taken_rows)
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) sums[16 * c + j] += __uint_as_float(v[c & 1][j]);
+                            for (int j = 0; j < 16; ++j) sums[16 * c + j] = fmaf(__uint_as_float(v[c & 1][j]), 1.0f / PF_LO, sums[16 * c + j]);
                     }
                     fence_before_sync();
                     __syncwarp();
                     if (lane == 0) bar_arrive(&item_read);
                     const int w_exponent = scale_exponent(taken_scale);
+                    const float least = 32.f * (float)p.K;
+                    uint32_t bad[2] = {0, 0};
+                    const float own_x_scales[2] = {lane < taken_rows ? p.x_scale[taken_row0 + lane] : 0.f,
+                                                   lane + 32 < taken_rows ? p.x_scale[taken_row0 + lane + 32] : 0.f};
 #pragma unroll
                     for (int n = 0; n < PF_COLS; ++n) {
+                        const float x_scale = __shfl_sync(0xffffffffu, own_x_scales[n / 32], n % 32);
                         if (n < taken_rows && taken_f < p.F) {
                             const long long row = (long long)taken_row0 + n;
-                            const float x_scale = p.x_scale[row];
-                            p.out[row * p.F + taken_f] = taken_scale != 0.f && x_scale != 0.f
-                                                             ? ldexpf(sums[n], -(w_exponent + scale_exponent(x_scale)))
-                                                             : product_entry_by_entry(p, taken_w_row, row);
+                            const float size = fabsf(sums[n]);
+                            if (!(size >= least && taken_scale > 0.f && x_scale > 0.f) &&
+                                !is_of_zeros(sums[n], taken_scale, x_scale)) bad[n / 32] |= 1u << n % 32;
+                            p.out[row * p.F + taken_f] = ldexpf(sums[n], -(w_exponent + scale_exponent(x_scale)));
                         }
                         sums[n] = 0.f;
                     }
+                    const bool any = __any_sync(0xffffffffu, (bad[0] | bad[1]) != 0);
+                    const long long unit = (long long)taken_item * PF_WORKERS + warp - 2;
+                    if (any) p.columns[unit * 32 + lane] = (unsigned long long)bad[1] << 32 | bad[0];
+                    if (lane == 0) p.again[unit] = any;
                 }
             }
             if (!more) break;
             pending = step == steps - 1 ? 2 : step % PF_CHUNK == PF_CHUNK - 1 ? 1 : 0;
-            if (pending) { taken_row0 = row0; taken_rows = rows; taken_f = f; taken_w_row = w_row; taken_scale = scale; }
+            if (pending) { taken_row0 = row0; taken_rows = rows; taken_f = f; taken_item = item; taken_scale = scale; }
             if (++step == steps) { step = 0; item += gridDim.x; }
         }
     }
@@ -318,13 +327,61 @@ products_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     if (warp == 1) tmem_free(tmem, 512);
 }
 
+// The outputs to be summed again, a warp each: a warp takes the workers' outputs of an item that have some, and their columns in turn.  A
+// kernel of its own: called from the workers' loop the same cost that a quarter of its speed.  3,704 rows with 8192 x 3072 and 3072 x 6144
+// weights, on average: 626 us with this kernel, 28 of them its own; 800 the other way; 606 with no output summed again but those of rows
+// without a scale.
+__global__ void __launch_bounds__(256, 4) products_f32_again_kernel(const __grid_constant__ ProductsParams p) {
+    const int lane = threadIdx.x & 31, feature_blocks = (p.F + PF_FEATS - 1) / PF_FEATS;
+    const long long units = (long long)p.count() * feature_blocks * PF_WORKERS, warps = (long long)gridDim.x * 8;
+    for (long long first = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); first < units; first += 32 * warps) {
+        const long long mine = first + lane * warps;
+        for (uint32_t left = __ballot_sync(0xffffffffu, mine < units && p.again[mine]); left; left &= left - 1) {
+            const long long unit = first + (__ffs(left) - 1) * warps;
+            const int item = (int)(unit / PF_WORKERS), worker = (int)(unit % PF_WORKERS), tile = item / feature_blocks, e = p.expert(tile);
+            // the worker of warp w: weight rows 32 (w & 3) on, columns of part (w - 2) / 4
+            const int f = (item - tile * feature_blocks) * PF_FEATS + ((worker + 2) & 3) * 32 + lane;
+            const long long row0 = p.first_row(tile) + (worker >> 2) * PF_COLS, w_row = (long long)e * p.F + min(f, p.F - 1);
+            const unsigned long long columns = p.columns[unit * 32 + lane];
+            unsigned long long all = (unsigned long long)__reduce_or_sync(0xffffffffu, (uint32_t)(columns >> 32)) << 32 |
+                                     __reduce_or_sync(0xffffffffu, (uint32_t)columns);
+            for (; all; all &= all - 1) {
+                const int n = __ffsll((long long)all) - 1;
+                const long long row = row0 + n;
+                const float* x = p.x + (p.x_rows ? p.x_rows[row] : row) * (p.gated ? 2ll * p.K : (long long)p.K);
+                for (uint32_t mask = __ballot_sync(0xffffffffu, (columns >> n & 1) != 0); mask; mask &= mask - 1) {
+                    const int of = __ffs(mask) - 1;
+                    const float* w = p.W + __shfl_sync(0xffffffffu, w_row, of) * p.K;
+                    float sum = 0.f;
+#pragma unroll 8
+                    for (int k = 4 * lane; k < p.K; k += 128) {
+                        const float4 a = *(const float4*)(w + k);
+                        float4 b = *(const float4*)(x + k);
+                        if (p.gated) {
+                            const float4 up = *(const float4*)(x + p.K + k);
+                            b = make_float4(paired_gate(b.x, up.x, p.gate_limit), paired_gate(b.y, up.y, p.gate_limit),
+                                            paired_gate(b.z, up.z, p.gate_limit), paired_gate(b.w, up.w, p.gate_limit));
+                        }
+                        sum = fmaf(a.x, b.x, sum);
+                        sum = fmaf(a.y, b.y, sum);
+                        sum = fmaf(a.z, b.z, sum);
+                        sum = fmaf(a.w, b.w, sum);
+                    }
+                    sum = warp_sum(sum);
+                    if (lane == of) p.out[row * p.F + f] = sum;
+                }
+            }
+        }
+    }
+}
+
 // ----------------------------------------------------------------------------- scales and parts
 
-// The power of two that brings `top` to [2^14, 2^15); 1 for a row of zeros, 0 for one with an infinity or a NaN or whose scale
+// The power of two that brings `top` to [2^14, 2^15); -1 for a row of zeros, 0 for one with an infinity or a NaN or whose scale
 // would leave float32.
 __device__ __forceinline__ float row_scale(float top) {
     if (!(top <= 3.402823466e38f)) return 0.f;
-    if (top == 0.f) return 1.f;
+    if (top == 0.f) return -1.f;
     const int exponent = 14 - ilogbf(top);
     return exponent <= 126 ? __uint_as_float((uint32_t)(exponent + 127) << 23) : 0.f;
 }
@@ -434,13 +491,17 @@ FRB_API int frb_split_rows(const float* x, const int* rows, void* parts, float* 
 
 // W float32 [E][F][K] with w_scale [E * F]; parts float16 [2][rows_total][K] with x_scale [rows_total], made from x (with x_rows,
 // gated, gate_limit as for frb_split_rows), the rows of each expert together; tiles of at most 128 rows (null lists: the tiles of
-// one weight matrix); out float32 [rows_total, F].  status: one int on the device, zero before the call.
+// one weight matrix); out float32 [rows_total, F].  again: scratch, FRB_PRODUCTS_AGAIN bytes for every tile and 128 features.  status:
+// one int on the device, zero before the call.
+#define FRB_PRODUCTS_AGAIN (PF_WORKERS * (32 * 8 + 1))
 FRB_API int frb_products_f32(const float* W, const float* w_scale, int num_experts, const void* parts, const float* x_scale, long long rows_total,
                              const float* x, const int* x_rows, int gated, float gate_limit, const int* tile_expert, const int* tile_row0,
-                             const int* num_tiles, const int* offsets, int max_tiles, float* out, int F, int K, int* status, cudaStream_t stream) {
+                             const int* num_tiles, const int* offsets, int max_tiles, float* out, int F, int K, void* again, int* status,
+                             cudaStream_t stream) {
     if (max_tiles == 0 || F == 0) return 0;
     FRB_CHECK_ARG(K > 0 && K % 8 == 0, "float32 products: an inner size of %d is not a multiple of 8", K);
-    FRB_CHECK_ARG((((uintptr_t)W | (uintptr_t)parts) & 15) == 0, "float32 products: operands must be 16-byte aligned");
+    FRB_CHECK_ARG((((uintptr_t)W | (uintptr_t)parts | (uintptr_t)x) & 15) == 0 && ((uintptr_t)again & 7) == 0,
+                  "float32 products: operands must be 16-byte aligned");
     FRB_CHECK_ARG(2 * rows_total + PF_ROWS < (1ll << 31) && (long long)num_experts * F < (1ll << 31) - PF_FEATS,
                   "float32 products: %lld rows or %d experts of %d features exceed a coordinate", rows_total, num_experts, F);
     const long long items = (long long)max_tiles * ((F + PF_FEATS - 1) / PF_FEATS);
@@ -449,13 +510,14 @@ FRB_API int frb_products_f32(const float* W, const float* w_scale, int num_exper
     FRB_CHECK_ARG(map_rows_of_128_bytes(&map_w, W, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)num_experts * F, K, PF_FEATS) &&
                       map_rows_of_128_bytes(&map_x, parts, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, 2 * rows_total, K, PF_ROWS),
                   "float32 products: cuTensorMapEncodeTiled failed or is not available");
-    const ProductsParams p = {W, w_scale, x_scale, x, x_rows, gated, gate_limit, tile_expert, tile_row0, num_tiles, offsets, out, status, F, K,
-                              max_tiles, rows_total};
+    const ProductsParams p = {W, w_scale, x_scale, x, x_rows, gated, gate_limit, tile_expert, tile_row0, num_tiles, offsets, out,
+                              (uint8_t*)again + items * PF_WORKERS * 32 * 8, (unsigned long long*)again, status, F, K, max_tiles, rows_total};
     int device = 0, sms = 0;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const size_t smem = PF_WSTAGES * PF_WBYTES + PF_XSTAGES * PF_XBYTES + 1024;
     cudaFuncSetAttribute(products_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     products_f32_kernel<<<(unsigned)(items < sms ? items : sms), PF_THREADS, smem, stream>>>(map_w, map_x, p);
+    products_f32_again_kernel<<<4 * sms, 256, 0, stream>>>(p);
     FRB_RETURN_LAUNCH("products_f32");
 }

@@ -293,6 +293,27 @@ def test_infinities_and_nans_reach_the_queries_that_see_them(heads, kv_heads, di
     same_but_for_rounding(got, want, 330)
 
 
+@pytest.mark.parametrize("inner", [8, 256, 3072])
+@pytest.mark.parametrize("spread", [0, 20, 60])
+def test_split_products_of_rows_whose_entries_lie_far_apart(inner, spread):
+    """Entries over 2^spread either way in every row of both operands, rows and weight rows with a single entry that is not zero, and an
+    entry 2^40 above the rest that the weights leave out: every output within 2^-21 (two operands of 22 bits, and the product of their
+    small parts) and a float32 sum's roundings of the sum of its terms' sizes, which no norm of a row hides."""
+    gen = torch.Generator(device=DEV).manual_seed(inner + spread)
+    x, w = torch.randn(40, inner, device=DEV, generator=gen), torch.randn(1, 150, inner, device=DEV, generator=gen)
+    x, w = (t * torch.exp2((torch.rand(t.shape, device=DEV, generator=gen) * 2 - 1) * spread) for t in (x, w))
+    for r in range(8):
+        x[r], x[r, r] = 0.0, 1.7 * 2.0 ** -r
+    for f in range(64):
+        w[0, f], w[0, f, f % inner] = 0.0, 1.3
+    x[20:30, 0], w[0, 100:, 0] = 2.0 ** 40, 0.0
+    x[31], w[0, 99] = 0.0, 0.0
+    got, want = split_product(w, x).double(), x.double() @ w[0].double().T
+    size = x.double().abs() @ w[0].double().abs().T
+    assert ((got - want).abs() <= (2.0 ** -21 + inner ** 0.5 * 2.0 ** -24) * size).all()
+    assert (got[31] == 0).all() and (got[:, 99] == 0).all()
+
+
 @pytest.mark.parametrize("tokens", [3, 700])
 def test_experts_take_rows_at_any_offset(tokens):
     """Rows that do not begin on 16 bytes, few of them (the stream over the weights) and many (the split products)."""
