@@ -11,9 +11,11 @@
 // the library's float32 product by 2e-7 to 1.4e-6, the kernel for any sizes (experts_generic.cu) by 1.7e-6.
 //
 // Some outputs are summed again entry by entry in float32: those of rows without a scale (rows with an infinity or a NaN or without an
-// entry of 2^-112); and those so small that entries below 2^-29 of their rows' largest may have had a part in them.  In units of the scaled rows each such entry is off by at most 2^-36 and meets entries below 2^15, so a sum
+// entry of 2^-112); those that came out as an infinity or a NaN; and those so small that entries below 2^-29 of their rows' largest may
+// have had a part in them.  In units of the scaled rows each such entry is off by at most 2^-36 and meets entries below 2^15, so a sum
 // of K is off by less than K 2^-20, both sides together: 2^-25 of any sum from 32 K on, where the largest product is 2^30.  Of rows
-// of normally distributed numbers one output in 40,000 is below that.
+// of normally distributed numbers one output in 40,000 is below that.  The last two also hold where weights were written after
+// the scales were made of them, and no longer suit them.
 //
 // What bounds it: 3,704 tokens on MiniMax-M2's 256 experts have to read 14.5 GB of weights (2.2 ms) and take 2.5 PFLOP of
 // float16 products (1.6 ms at the tensor cores' peak).  The two products of those sizes take 4.6 ms (in tiles of eight rows on
@@ -298,7 +300,7 @@ products_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                         if (n < taken_rows && taken_f < p.F) {
                             const long long row = (long long)taken_row0 + n;
                             const float size = fabsf(sums[n]);
-                            if (!(size >= least && taken_scale > 0.f && x_scale > 0.f) &&
+                            if (!(size >= least && size <= 3.402823466e38f && taken_scale > 0.f && x_scale > 0.f) &&
                                 !is_of_zeros(sums[n], taken_scale, x_scale)) bad[n / 32] |= 1u << n % 32;
                             p.out[row * p.F + taken_f] = ldexpf(sums[n], -(w_exponent + scale_exponent(x_scale)));
                         }

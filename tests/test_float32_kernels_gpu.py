@@ -314,6 +314,25 @@ def test_split_products_of_rows_whose_entries_lie_far_apart(inner, spread):
     assert (got[31] == 0).all() and (got[:, 99] == 0).all()
 
 
+@pytest.mark.parametrize("factor", [1e9, 1e-9, 0.0])
+def test_split_products_of_weights_written_after_their_scales(factor):
+    """Scales are made when weights are loaded; weights of another size written in their place later give the products of the new ones."""
+    gen = torch.Generator(device=DEV).manual_seed(7)
+    x, w = torch.randn(30, 264, device=DEV, generator=gen), torch.randn(1, 140, 264, device=DEV, generator=gen)
+    w[0, 0] = 0.0
+    scales = ops().weight_scales(w)
+    w.mul_(factor)
+    w[0, 0, 3] = 1.0
+    w[0, 1, 1] = INF
+    parts, scale = torch.empty(2, 30, 264, dtype=torch.float16, device=DEV), torch.empty(30, device=DEV)
+    out = torch.empty(30, 140, device=DEV)
+    ops().products_f32(w, scales, x, parts, scale, out)
+    ops().tc_status_check(out.device)
+    want, fine = x.double() @ w[0].double().T, w[0].isfinite().all(1)
+    assert torch.equal(out[:, 1].double(), want[:, 1])                       # an infinity, as the entries of x give it its sign
+    assert ((out.double() - want).abs()[:, fine] <= 2.0 ** -20 * (x.double().abs() @ w[0].double().abs().T)[:, fine]).all()
+
+
 @pytest.mark.parametrize("tokens", [3, 700])
 def test_experts_take_rows_at_any_offset(tokens):
     """Rows that do not begin on 16 bytes, few of them (the stream over the weights) and many (the split products)."""
