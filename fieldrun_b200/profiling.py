@@ -366,10 +366,20 @@ def step_timeline(launches: int, batch: int = 8) -> dict:
             "middle_layer": rows}
 
 
+def _chunk_tables(lengths, size: int):
+    """Every sequence's tokens in chunks: sequence, first and end token of each; first chunk of each sequence and, last, their number."""
+    seqs, lo, hi, first = [], [], [], [0]
+    for b, n in enumerate(lengths):
+        for t in range(0, n, size):
+            seqs.append(b), lo.append(t), hi.append(min(t + size, n))
+        first.append(len(seqs))
+    return tuple(torch.tensor(x, dtype=torch.int32, device=DEV) for x in (seqs, lo, hi, first))
+
+
 def linear_attention(kind: str, launches: int) -> dict:
-    """The gated linear attention scan alone, 16 heads of 128 x 128 with a decay of rank 32: ``prefill`` four prompts of
-    2,048 tokens in segments of 128 (three launches a call), ``prefill_whole`` the same without segments, ``decode`` 64
-    sequences of one token.  FLOPs are those of the recurrence: four per state element and token."""
+    """The gated linear attention scan alone, 16 heads of 128 x 128 with a decay of rank 32: ``chunks`` four prompts of 2,048
+    tokens as matrix products, ``prefill`` token by token in segments of 128 (three launches a call), ``prefill_whole`` the same
+    without segments, ``decode`` 64 sequences of one token.  FLOPs are those of the recurrence: four per state element and token."""
     heads, dim, vdim, rank = 16, 128, 128, 32
     if kind == "decode":
         lengths = [1] * 64
@@ -388,18 +398,18 @@ def linear_attention(kind: str, launches: int) -> dict:
     cu = torch.tensor([0] + list(np.cumsum(lengths)), dtype=torch.int32, device=DEV)
     segments = scratch = None
     if kind == "prefill":
-        size, seqs, lo, hi, first = 128, [], [], [], [0]
-        for b, n in enumerate(lengths):
-            for t in range(0, n, size):
-                seqs.append(b), lo.append(t), hi.append(min(t + size, n))
-            first.append(len(seqs))
-        segments = tuple(torch.tensor(x, dtype=torch.int32, device=DEV) for x in (seqs, lo, hi, first))
-        scratch = torch.empty(ops.gla_scratch_floats(len(seqs), heads, dim, vdim), device=DEV)
+        segments = _chunk_tables(lengths, 128)
+        scratch = torch.empty(ops.gla_scratch_floats(segments[0].numel(), heads, dim, vdim), device=DEV)
+    elif kind == "chunks":
+        segments = _chunk_tables(lengths, ops.GLA_CHUNK_TOKENS)
+        scratch = torch.empty(ops.gla_chunks_scratch_floats(segments[0].numel(), tokens, heads, dim, vdim), device=DEV)
     offsets = (0, heads * dim, 2 * heads * dim, 2 * heads * dim + heads * vdim, 2 * heads * dim + 2 * heads * vdim)
 
     def launch():
-        ops.gla_scan(proj, offsets, a2, bias, norm, state, slots, starts, cu, out, heads=heads, dim=dim, vdim=vdim, tau=16.0,
-                     q_scale=dim ** -0.5, eps=1e-6, segments=segments, scratch=scratch)
+        how = dict(chunks=segments) if kind == "chunks" else dict(segments=segments)
+        (ops.gla_chunks if kind == "chunks" else ops.gla_scan)(
+            proj, offsets, a2, bias, norm, state, slots, starts, cu, out, heads=heads, dim=dim, vdim=vdim, tau=16.0,
+            q_scale=dim ** -0.5, eps=1e-6, scratch=scratch, **how)
 
     ms = _time(launch, launches)
     flops = 4.0 * tokens * heads * dim * vdim
@@ -422,7 +432,8 @@ class _Tables:
 
 def scans(kind: str, launches: int) -> dict:
     """The recurrences of scans.cu alone, at the sizes of a model of width 2048, over four prompts of 2,048 tokens:
-    ``selective`` 4,096 channels with 16 state elements each, ``state_space`` 64 heads of 128 x 64, ``gated`` 2,048
+    ``selective`` 4,096 channels with 16 state elements each, ``state_space`` 64 heads of 128 x 64 (``state_space_chunks``: as
+    matrix products), ``gated`` 2,048
     channels, ``conv`` 4,096 channels with four taps.  Updates: state elements times tokens."""
     lengths = [2048] * 4
     tokens = sum(lengths)
@@ -441,7 +452,7 @@ def scans(kind: str, launches: int) -> dict:
         def launch():
             ops.selective_scan(xz, inner, x, low, rank, rank + n, dt, zero, a_log, d, tables, state, 0, out)
         updates, moved = tokens * inner * n, (xz.numel() // 2 + x.numel() + 2 * dt.numel() + low.numel()) * 4 + out.numel() * 2
-    elif kind == "state_space":
+    elif kind in ("state_space", "state_space_chunks"):
         heads, vdim, n, groups = 64, 64, 128, 8
         inner = heads * vdim
         proj = torch.randn(tokens, inner + heads, device=DEV)
@@ -451,9 +462,16 @@ def scans(kind: str, launches: int) -> dict:
         state = torch.zeros(4, 2, heads * n * vdim, device=DEV)
         out = torch.empty(tokens, inner, device=DEV)
 
+        sizes = dict(heads=heads, vdim=vdim, n=n, groups=groups)
+        chunks = _chunk_tables(lengths, ops.STATE_SPACE_CHUNK_TOKENS)
+        how = dict(chunks=chunks, scratch=torch.empty(ops.state_space_chunks_scratch_floats(chunks[0].numel(), **sizes), device=DEV))
+
         def launch():
-            ops.state_space_scan(proj, 0, inner, xbc, inner, inner + groups * n, dt_bias, a_log, d, tables, state, 0, out,
-                                 heads=heads, vdim=vdim, n=n, groups=groups)
+            args = (proj, 0, inner, xbc, inner, inner + groups * n, dt_bias, a_log, d, tables, state, 0, out)
+            if kind == "state_space":
+                ops.state_space_scan(*args, **sizes)
+            else:
+                ops.state_space_chunks(*args, **how, **sizes)
         updates, moved = tokens * heads * n * vdim, (proj.numel() + xbc.numel() + out.numel()) * 4
     elif kind == "gated":
         width, blocks = 2048, 16
@@ -486,10 +504,11 @@ def scans(kind: str, launches: int) -> dict:
 
 
 def delta_rule(kind: str, launches: int) -> dict:
-    """The gated delta rule of delta_rule.cu alone, 16 heads of 128 x 128 over 4 key heads: ``prefill`` four prompts of
-    2,048 tokens (``prefill_whole``: every head's value columns in one block), ``decode`` 64 sequences of one token.  Updates: state elements times tokens (four multiply-adds each)."""
+    """The gated delta rule alone, 16 heads of 128 x 128 over 4 key heads: ``chunks`` four prompts of 2,048 tokens as matrix
+    products, ``prefill`` token by token (``prefill_whole``: every head's value columns in one block), ``decode`` 64 sequences of one
+    token.  Updates: state elements times tokens (four multiply-adds each)."""
     heads, kv_heads, dim, vdim = 16, 4, 128, 128
-    lengths = [2048] * 4 if kind.startswith("prefill") else [1] * 64
+    lengths = [1] * 64 if kind == "decode" else [2048] * 4
     tokens = sum(lengths)
     tables = _Tables(lengths)
     channels = 2 * kv_heads * dim + heads * vdim
@@ -501,14 +520,85 @@ def delta_rule(kind: str, launches: int) -> dict:
     raw = torch.empty(tokens, heads * vdim, device=DEV)
     slices = None if kind != "prefill_whole" else 1
 
+    args = (conv, 0, kv_heads * dim, 2 * kv_heads * dim, proj, 0, heads, 2 * heads, a_log, dt_bias, norm, tables, state, 0, out)
+    sizes = dict(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, eps=1e-6, raw=raw)
+    chunks = _chunk_tables(lengths, ops.DELTA_CHUNK_TOKENS)
+    scratch = torch.empty(ops.delta_chunks_scratch_floats(chunks[0].numel(), heads, dim, vdim), device=DEV) if kind == "chunks" else None
+
     def launch():
-        ops.gated_delta_rule(conv, 0, kv_heads * dim, 2 * kv_heads * dim, proj, 0, heads, 2 * heads, a_log, dt_bias, norm, tables,
-                             state, 0, out, heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, eps=1e-6, raw=raw, slices=slices)
+        if kind == "chunks":
+            ops.delta_chunks(*args, chunks=chunks, scratch=scratch, **sizes)
+        else:
+            ops.gated_delta_rule(*args, slices=slices, **sizes)
     ms = _time(launch, launches)
     updates = tokens * heads * dim * vdim
     moved = (conv.numel() + proj.numel()) * 4 + out.numel() * 2 + (2 * state[:, 0].numel() * 4 if kind == "decode" else 0)
     return {"case": f"delta_rule_{kind}", "tokens": tokens, "ms": round(ms, 4), "updates_per_ns": round(updates / ms / 1e6, 1),
             "tflops_float32": round(8.0 * updates / ms / 1e9, 2), "gbs": round(moved / ms / 1e6, 1)}
+
+
+def group_norm(launches: int) -> dict:
+    """The root-mean-square norm in parts (scans.cu), 8,192 rows of 4,096 as one part each, to bfloat16."""
+    rows, width = 8192, 4096
+    x, weight = torch.randn(rows, width, device=DEV), torch.ones(width, device=DEV)
+    out = torch.empty(rows, width, dtype=torch.bfloat16, device=DEV)
+    ms = _time(lambda: ops.group_rms_norm(x, weight, out, 1, 1e-6), launches)
+    return {"case": "scan_group_norm", "tokens": rows, "ms": round(ms, 4), "gbs": round(rows * width * 6 / ms / 1e6, 1)}
+
+
+def float32_products(kind: str, launches: int) -> dict:
+    """The float32 products: ``experts`` 16 experts of 3,072 x 1,536 with 128 rows each on the tensor cores (both products), ``dense``
+    3,704 rows with 8192 x 3072 weights with their scales and parts, ``rows`` six rows with 8192 x 3072 weights as a stream over them."""
+    if kind == "experts":
+        experts_n, rows = 16, 128
+        n = experts_n * rows
+        w13, w2 = torch.randn(experts_n, 2 * WIDTH, HIDDEN, device=DEV) * 0.02, torch.randn(experts_n, HIDDEN, WIDTH, device=DEV) * 0.02
+        x, both, y = torch.randn(n, HIDDEN, device=DEV), torch.empty(n, 2 * WIDTH, device=DEV), torch.empty(n, HIDDEN, device=DEV)
+        *lists, tiles = _expert_lists([rows] * experts_n, ops.PRODUCTS_F32_TILE, DEV)
+        scales, parts = (ops.weight_scales(w13), ops.weight_scales(w2)), torch.empty(2 * n * HIDDEN, dtype=torch.float16, device=DEV)
+        scale, how = torch.empty(n, device=DEV), dict(lists=tuple(lists), max_tiles=tiles)
+
+        def launch():
+            ops.products_f32(w13, scales[0], x, parts.view(2, n, HIDDEN), scale, both, **how)
+            ops.products_f32(w2, scales[1], both, parts[:2 * n * WIDTH].view(2, n, WIDTH), scale, y, gated=True, **how)
+        flops, weights = 6.0 * n * HIDDEN * WIDTH, (w13.numel() + w2.numel()) * 4
+    else:
+        from .parts.linear import linear, require_true_float32
+        require_true_float32()
+        w, x = torch.randn(8192, HIDDEN, device=DEV) * 0.02, torch.randn(6 if kind == "rows" else 3704, HIDDEN, device=DEV)
+
+        def launch():
+            linear(x, w)
+        flops, weights = 2.0 * x.shape[0] * w.numel(), w.numel() * 4
+    ms = _time(launch, launches)
+    ops.tc_status_check(torch.device(DEV))
+    return {"case": f"float32_{kind}", "ms": round(ms, 4), "tflops": round(flops / ms / 1e9, 2), "weight_gb_per_s": round(weights / ms / 1e6, 1)}
+
+
+def float32_attention(kind: str, launches: int) -> dict:
+    """Float32 attention, 48 heads over 8 of 128: ``prompts`` a prompt of 1,500 tokens in tiles, ``tokens`` one token each of sixteen
+    sequences of 4,096 keys in chunks."""
+    batch, context = (16, 4096) if kind == "tokens" else (1, 1500)
+    pages_per = (context + 63) // 64
+    keys, values = (torch.randn(batch * pages_per, KV_HEADS, *shape, device=DEV) for shape in ((64, HEAD_DIM), (HEAD_DIM, 64)))
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    table = torch.arange(batch * pages_per, dtype=torch.int32, device=DEV).view(batch, pages_per)
+    tokens = batch if kind == "tokens" else context
+    q, out = torch.randn(tokens, HEADS * HEAD_DIM, device=DEV), torch.empty(tokens, HEADS * HEAD_DIM, device=DEV)
+    common = dict(num_heads=HEADS, num_kv_heads=KV_HEADS, head_dim=HEAD_DIM, scale=HEAD_DIM ** -0.5, window=None)
+    if kind == "tokens":
+        pos, slots, chunks = i32([context - 1] * batch), i32(list(range(batch))), context // ops.ATTENTION_CHUNK
+        part_o, part_ml = torch.empty(batch, HEADS, chunks, HEAD_DIM, device=DEV), torch.empty(batch, HEADS, chunks, 2, device=DEV)
+        launch = lambda: ops.attention_f32_token(q, keys, values, table, pos, slots, part_o, part_ml, out, max_chunks=chunks, **common)
+        flops = 4.0 * batch * context * HEADS * HEAD_DIM
+    else:
+        firsts = list(range(0, context, 128))
+        tables = (i32([0] * len(firsts)), i32(firsts), i32([0]), i32([0]), i32([context]), i32([0, context]))
+        launch = lambda: ops.attention_f32_tiles(q, keys, values, table, *tables, out, **common)
+        flops = 2.0 * context * (context + 1) * HEADS * HEAD_DIM
+    ms = _time(launch, launches)
+    return {"case": f"float32_attention_{kind}", "ms": round(ms, 4), "tflops": round(flops / ms / 1e9, 2),
+            "kv_gb_per_s": round((keys.numel() + values.numel()) * 4 / ms / 1e6, 1)}
 
 
 def output_norm(launches: int, tokens: int) -> dict:
@@ -646,6 +736,9 @@ CASES = {
     **{f"duzinex_{kind}": (lambda n, kind=kind: duzinex(kind, n))
        for kind in ("retention_prefill", "retention_decode", "gru_prefill", "gru_decode", "shift_prefill", "shift_decode",
                     "powers_prefill", "powers_decode")},
+    **{f"float32_{kind}": (lambda n, kind=kind: float32_products(kind, n)) for kind in ("experts", "dense", "rows")},
+    **{f"float32_attention_{kind}": (lambda n, kind=kind: float32_attention(kind, n)) for kind in ("prompts", "tokens")},
+    "delta_rule_chunks": lambda n: delta_rule("chunks", n),
     "delta_rule_prefill": lambda n: delta_rule("prefill", n),
     "delta_rule_prefill_whole": lambda n: delta_rule("prefill_whole", n),
     "delta_rule_decode": lambda n: delta_rule("decode", n),
@@ -653,8 +746,11 @@ CASES = {
     "output_norm_decode": lambda n: output_norm(n, 8),
     "scan_selective": lambda n: scans("selective", n),
     "scan_state_space": lambda n: scans("state_space", n),
+    "scan_state_space_chunks": lambda n: scans("state_space_chunks", n),
     "scan_gated": lambda n: scans("gated", n),
     "scan_conv": lambda n: scans("conv", n),
+    "scan_group_norm": group_norm,
+    "linear_attention_chunks": lambda n: linear_attention("chunks", n),
     "linear_attention_prefill": lambda n: linear_attention("prefill", n),
     "linear_attention_prefill_whole": lambda n: linear_attention("prefill_whole", n),
     "linear_attention_decode": lambda n: linear_attention("decode", n),
