@@ -1,6 +1,6 @@
 // Attention over the paged cache, any head size up to 256 and any group size, float32 arithmetic.
-// It is the whole attention of the float32 path and the fallback of the bfloat16 path for shapes that
-// the tensor-core kernels refuse.
+// It takes what the other kernels do not: float32 heads and steps outside attention_f32.cu, and the shapes that
+// the tensor-core kernels of the bfloat16 path refuse.
 //
 // Per query head h with kv = h / (nh / nkv): s_j = (q . K_j) * scale for the keys the query may see
 // (j <= its position, and j > position - window when a window is set), p = exp(s - max) / sum,

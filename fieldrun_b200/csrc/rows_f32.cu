@@ -7,8 +7,9 @@
 // Eight tokens of MiniMax-M2's experts (57 used, 3.2 GB of weights) took 4.59 ms there, 0.7 TB/s.  Here a warp reads eight
 // weight rows side by side through a ring of its own in shared memory (asynchronous copies; a lane reads back only what it
 // copied, so the ring needs no barrier), and every weight meets all rows of its tile in registers; the rows come through L1,
-// which the weights bypass: 0.23 ms a product (7 TB/s).  Prompts run here too: 3,704 tokens, tiles of eight rows that read an
-// expert's weights again from L2, 14.4 ms a product against 36.1 there.
+// which the weights bypass: 0.23 ms a product (7 TB/s).  Steps of up to eight rows an expert, and of sizes or so little work that the
+// products on the tensor cores (products_f32.cu) do not take them, run here in tiles of eight rows that read an expert's weights
+// again from L2.
 #include "common.cuh"
 
 #define RF_WARPS 4
@@ -154,8 +155,9 @@ FRB_API int frb_rows_f32(const float* W, const float* X, const int* x_rows, cons
     const RowsParams p = {W, X, x_rows, tile_expert, tile_row0, num_tiles, offsets, out, F, K, gate_limit};
     const int outs = paired ? RF_FEATS / 2 : RF_FEATS, groups = (F + outs - 1) / outs;      // runs of eight weight rows of a tile
     // A single tile's blocks of four runs are one or two a SM and end unevenly: there four warps share a run of weight rows.
-    // (Six rows with 8192 x 3072 and 3072 x 6144 weights, timed with an event pair around each launch: 34 us on average, 52 and
-    // 57 with other splits of the same sizes into blocks of four and two runs.)  With many tiles a warp to a run has the fewer joins.
+    // (Six rows with 8192 x 3072 and 3072 x 6144 weights, an event pair around each launch, which itself is about 6 us: 33 us on
+    // average, 52 and 57 with other splits of the same sizes into blocks of four and two runs.)  With many tiles a warp to a run has
+    // the fewer joins.
     const bool parts = (long long)groups * max_tiles < 16384;
     const dim3 grid(parts ? groups : (groups + RF_WARPS - 1) / RF_WARPS, max_tiles);
     const size_t smem = (size_t)RF_WARPS * RF_STAGES * RF_FEATS * 32 * sizeof(float4);

@@ -249,9 +249,10 @@ class GQAAttention(Mixer):
 
     def attend(self, ctx, q: torch.Tensor, line: LineView, out: torch.Tensor, gate: Optional[torch.Tensor] = None) -> None:
         """Tensor-core kernels for bfloat16 and the head sizes of ``ops.MMA_HEAD_SIZES`` (tcgen05 for prompts with key
-        heads of 64 and 128, mma.sync otherwise); the general kernel for everything else.  All of them take the distance
-        slopes, chunks, sinks and first tokens; the general kernel applies the head gates itself, after the others a small
-        kernel does.  With two maps per head the one-token kernels take the maps' difference where they join their partial
+        heads of 64 and 128, mma.sync otherwise); for float32 tiles of queries or, for one token a sequence, chunks of keys, at the
+        head sizes that ``ops.attention_f32_tiles_take`` and ``attention_f32_token_takes`` name; the general kernel for everything
+        else.  All of them take the distance slopes, chunks, sinks and first tokens; the float32 and the general kernels apply the
+        head gates themselves, after the others a small kernel does.  With two maps per head the one-token kernels take the maps' difference where they join their partial
         results, after the others a small kernel does."""
         common = dict(num_heads=self.q_heads, num_kv_heads=self.k_heads, head_dim=self.head_dim, v_dim=self.value_dim,
                       scale=self.softmax_scale, window=self.window, slopes=self.slopes, chunk=self.chunk, sinks=self.sinks,

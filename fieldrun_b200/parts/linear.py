@@ -4,9 +4,9 @@ operands in parts, the others through the library (cuBLAS via torch.mm).
 The reference's dense products (``Bundle::mm``, src/bundle.rs:644-683) are a
 library call as well: ndarray's ``dot`` over matrixmultiply or cblas.  Weights
 stay in the checkpoint's ``(out, in)`` layout; the product is ``rows @ W^T``
-with float32 accumulation and a float32 result.  In float32 mode the reduced
-precision matrix modes (TF32, bf16 reductions) are switched off and that is
-checked at every call.
+with float32 accumulation and a float32 result.  In float32 mode the library's
+reduced precision matrix modes (TF32, bf16 reductions) are switched off and that
+is checked at every call.
 """
 from __future__ import annotations
 
@@ -53,7 +53,8 @@ def one_tile(device: torch.device, rows: int):
 
 
 def require_true_float32() -> None:
-    """Switch off every reduced-precision mode of float32 matrix products."""
+    """Switch off every reduced-precision mode of the library's float32 matrix products.  (This library's own products split their
+    operands where they run on tensor cores, and are held to 64-bit sums: products_f32.cu, tf32_parts.cuh.)"""
     torch.backends.cuda.matmul.allow_tf32 = False
     torch.backends.cudnn.allow_tf32 = False
     torch.set_float32_matmul_precision("highest")
