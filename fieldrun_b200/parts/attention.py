@@ -123,10 +123,11 @@ class GQAAttention(Mixer):
         if self.position is not None and self.position.rotary_dim > self.head_dim:
             raise ValueError(f"rotary_dim {self.position.rotary_dim} exceeds head_dim {self.head_dim}")
         self.tensor_cores = dtype == torch.bfloat16 and (self.head_dim, self.value_dim) in ops.MMA_HEAD_SIZES
+        # float32: head sizes that the tiles of queries (prompts) and the chunks of keys (one token a sequence) take
+        self.float32_tiles = dtype == torch.float32 and ops.attention_f32_tiles_take(self.head_dim, self.value_dim)
+        self.float32_token = dtype == torch.float32 and ops.attention_f32_token_takes(self.head_dim, self.value_dim)
         if not self.tensor_cores:                                # the tensor-core kernels take none of this part's steps
-            float32 = dtype == torch.float32 and (ops.attention_f32_tiles_take(self.head_dim, self.value_dim)
-                                                  or ops.attention_f32_token_takes(self.head_dim, self.value_dim))
-            self.kernel_groups = ("common", "streams", "attention32") if float32 else ("common", "streams")
+            self.kernel_groups = ("common", "streams", "attention32") if self.float32_tiles or self.float32_token else ("common", "streams")
         # heads as the kernels see them: with two maps per head, two query heads and two key heads
         self.q_heads, self.k_heads = self.maps * self.num_heads, self.maps * self.num_kv_heads
         self.q_width = self.q_heads * self.head_dim
@@ -288,7 +289,7 @@ class GQAAttention(Mixer):
                                           ctx.seq_start, ctx.seq_q_len, ctx.cu_q_len, maps_out, **common)
             if gate is not None:
                 ops.head_gate(out, gate, self.num_heads, self.value_dim)
-        elif self.dtype == torch.float32 and ctx.is_decode and ops.attention_f32_token_takes(self.head_dim, self.value_dim, ctx.num_seqs):
+        elif self.float32_token and ctx.is_decode and ops.attention_f32_token_takes(self.head_dim, self.value_dim, ctx.num_seqs):
             # float32: one token a sequence in chunks of keys side by side, prompts in tiles of queries; the general kernel, a
             # block per token, keeps the head sizes neither takes
             chunks = (ctx.max_kv_len + ops.ATTENTION_CHUNK - 1) // ops.ATTENTION_CHUNK
@@ -296,8 +297,8 @@ class GQAAttention(Mixer):
             part_ml = ctx.buffer("attention.part_ml", (ctx.num_seqs, self.q_heads, chunks, 2), torch.float32)
             ops.attention_f32_token(q, line.keys, line.values, line.page_table, ctx.tok_pos, ctx.tok_slot, part_o, part_ml, maps_out,
                                     max_chunks=chunks, gate=gate, **common)
-        elif (self.dtype == torch.float32 and not ctx.is_decode
-              and ops.attention_f32_tiles_take(self.head_dim, self.value_dim, ctx.chunk_count(ops.TC_ATTENTION_QUERIES))):
+        elif (self.float32_tiles and not ctx.is_decode
+              and ops.attention_f32_tiles_take(self.head_dim, self.value_dim, ctx.query_tiles(ops.TC_ATTENTION_QUERIES)[0].numel())):
             tile_seq, tile_q0 = ctx.query_tiles(ops.TC_ATTENTION_QUERIES)
             ops.attention_f32_tiles(q, line.keys, line.values, line.page_table, tile_seq, tile_q0, ctx.seq_slot, ctx.seq_start,
                                     ctx.seq_q_len, ctx.cu_q_len, maps_out, gate=gate, **common)
