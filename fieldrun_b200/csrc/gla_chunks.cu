@@ -12,8 +12,9 @@
 //
 // Everything is float32; the products run on tensor cores with each operand as two TF32 parts (tf32_parts.cuh), over inner
 // sizes of at most 192 entries, added in float32 registers every 16.  Four prompts of 2,048 tokens, 16 heads of 128 x 128: 0.50 ms
-// (gla.cu 1.66 ms in segments of 128, whose 500 instructions a warp and token run one after the other).  What bounds them: the instructions around
-// the products (60 and 50 % of the issue slots; a decay's two exponentials and a logarithm, the parts, the block's own pairs),
+// (about 0.20 + 0.04 + 0.26 for the launches in turn; gla.cu 1.66 ms in segments of 128, whose 500 instructions a warp and token run
+// one after the other).  What bounds them: the instructions around
+// the products (58 and 48 % of the issue slots; a decay's two exponentials and a logarithm, the parts, the block's own pairs),
 // with two blocks an SM to hide the rows' way in; with q, k and v loaded where they are used 0.68 ms.
 #include "tf32_parts.cuh"
 

@@ -18,10 +18,11 @@
 // the scales were made of them, and no longer suit them.
 //
 // What bounds it: 3,704 tokens on MiniMax-M2's 256 experts have to read 14.5 GB of weights (2.2 ms) and take 2.5 PFLOP of
-// float16 products (1.6 ms at the tensor cores' peak).  The two products of those sizes take 4.6 ms (in tiles of eight rows on
-// the ordinary pipes, rows_f32.cu: 28.8 ms); 3,704 rows with 8192 x 3072 weights 0.71 ms, 790 TFLOP/s of float16 products (the library's float32 product 3.17 ms).  What
-// holds it is the way from L2 to shared memory: a step of 6.3 MFLOP takes 64 KB a SM, and with the copies and barriers alone it
-// takes 1,430 cycles of the 2,210 (without the products 1,800, without the split 1,990; 16 workers instead of eight: 2,400).
+// float16 products (1.6 ms at the tensor cores' peak).  The two products of those sizes take 4.9 ms (in tiles of eight rows on
+// the ordinary pipes, rows_f32.cu: 28.8 ms); 3,704 rows with 8192 x 3072 weights 0.78 ms with their scales and parts, 720 TFLOP/s of
+// float16 products (the library's float32 product 3.17 ms).  What holds it is the way from L2 to shared memory: a step of 6.3 MFLOP
+// takes 64 KB a SM, and with the copies and barriers alone it takes 1,430 cycles of the 2,210 (without the products 1,800, without the
+// split 1,990; 16 workers instead of eight: 2,400).
 //
 // A block (one per SM, for the whole launch) takes items of 128 features x 128 rows in turn.  Two producer threads fill a ring each
 // by TMA: weights as float32 [128][64], rows as their two parts [2][128][64].  Eight warps read a weight tile, a row and half

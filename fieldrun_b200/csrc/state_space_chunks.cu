@@ -15,9 +15,9 @@
 //
 // Everything is float32; the products run on tensor cores with each operand as two TF32 parts (tf32_parts.cuh), over inner sizes
 // of at most 256 entries, added in float32 registers every 16 (launches 1 and 2: every 8).  Four prompts of 2,048 tokens, 64 heads of
-// 128 x 64 in 8 groups: 0.68 ms (scans.cu token by token 1.21 ms; its four launches took 0.04 + 0.17 + 0.07 + 0.40 of 0.65 with all
-// sums on the tensor cores).  What bounds them: launch 4 issues on half of the
-// cycles, a third of its instructions the operands' parts, and keeps the tensor cores busy for 39 %.
+// 128 x 64 in 8 groups: 0.68 ms (about 0.05 + 0.19 + 0.06 + 0.38 for the launches in turn; scans.cu token by token 1.21 ms).  What bounds
+// them: launch 4 issues on half of the cycles, a third of its instructions the operands' parts, and keeps the tensor cores busy for
+// 39 %.
 #include "tf32_parts.cuh"
 
 #define SC_TOKENS 128
