@@ -345,7 +345,9 @@ __global__ void __launch_bounds__(256, 4) products_f32_again_kernel(const __grid
             // the worker of warp w: weight rows 32 (w & 3) on, columns of part (w - 2) / 4
             const int f = (item - tile * feature_blocks) * PF_FEATS + ((worker + 2) & 3) * 32 + lane;
             const long long row0 = p.first_row(tile) + (worker >> 2) * PF_COLS, w_row = (long long)e * p.F + min(f, p.F - 1);
-            const unsigned long long columns = p.columns[unit * 32 + lane];
+            const long long rows_here = p.end_row(e) - row0;             // whatever a launch that gave up has left in `again`: no row beyond
+            const unsigned long long there = rows_here >= 64 ? ~0ull : rows_here > 0 ? (1ull << rows_here) - 1 : 0;
+            const unsigned long long columns = f < p.F ? p.columns[unit * 32 + lane] & there : 0;
             unsigned long long all = (unsigned long long)__reduce_or_sync(0xffffffffu, (uint32_t)(columns >> 32)) << 32 |
                                      __reduce_or_sync(0xffffffffu, (uint32_t)columns);
             for (; all; all &= all - 1) {
