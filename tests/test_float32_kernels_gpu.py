@@ -355,3 +355,37 @@ def test_experts_take_rows_at_any_offset(tokens):
     rows = torch.randn(tokens, hidden, device=DEV)
     shifted = torch.zeros(rows.numel() + 1, device=DEV)[1:].view_as(rows).copy_(rows)
     assert torch.equal(part.forward(ctx, shifted, rows).clone(), part.forward(ctx, rows, rows))
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim", [(6, 2, 32), (8, 8, 64), (12, 2, 128), (6, 3, 12)])
+def test_float32_attention_is_as_near_to_64_bits_as_the_general_kernel(heads, kv_heads, dim):
+    """Prompts in tiles and single tokens in chunks against a softmax in 64 bits: off by no more than twice what the general kernel's
+    roundings come to on the same inputs."""
+    starts, lengths = [0, 130], [300, 129]
+    keys, values, table, gen = paged(starts, lengths, kv_heads, kv_heads, dim, dim, 11)
+    tokens = sum(lengths)
+    q = torch.randn(tokens, heads * dim, device=DEV, generator=gen)
+    pos = np.concatenate([s + np.arange(n) for s, n in zip(starts, lengths)])
+    slots, common = np.repeat(np.arange(2), lengths), dict(num_heads=heads, num_kv_heads=kv_heads, head_dim=dim, scale=dim ** -0.5, window=None)
+    exact = torch.empty(tokens, heads, dim, dtype=torch.float64, device=DEV)
+    for row in range(2):
+        held, mine = starts[row] + lengths[row], slice(*(int(c) for c in np.searchsorted(slots, [row, row + 1])))
+        pages = table[row, :(held + 63) // 64].long()
+        k = keys[pages].double().permute(1, 0, 2, 3).reshape(kv_heads, -1, dim)[:, :held].repeat_interleave(heads // kv_heads, 0)
+        v = values[pages].double().permute(1, 0, 3, 2).reshape(kv_heads, -1, dim)[:, :held].repeat_interleave(heads // kv_heads, 0)
+        scores = q[mine].double().view(-1, heads, dim).transpose(0, 1) @ k.transpose(1, 2) * dim ** -0.5
+        hidden = torch.arange(held, device=DEV)[None] > torch.as_tensor(pos[mine], device=DEV)[:, None]
+        exact[mine] = (scores.masked_fill(hidden, -INF).softmax(-1) @ v).transpose(0, 1)
+    exact = exact.view(tokens, heads * dim)
+    general, tiles = (torch.full((tokens, heads * dim), NAN, device=DEV) for _ in range(2))
+    ops().attention_generic(q, keys, values, table, i32(pos), i32(slots), general, **common)
+    cut = [(b, q0) for b, n in enumerate(lengths) for q0 in range(0, n, 128)]
+    ops().attention_f32_tiles(q, keys, values, table, i32([t[0] for t in cut]), i32([t[1] for t in cut]), i32(range(2)), i32(starts), i32(lengths),
+                              i32(np.concatenate([[0], np.cumsum(lengths)])), tiles, **common)
+    limit = 2 * relative(general, exact)
+    assert relative(tiles, exact) < limit
+    if ops().attention_f32_token_takes(dim, dim):
+        last = [lengths[0] - 1, tokens - 1]
+        token, part_o, part_ml = (torch.full(shape, NAN, device=DEV) for shape in ((2, heads * dim), (2, heads, 2, dim), (2, heads, 2, 2)))
+        ops().attention_f32_token(q[last], keys, values, table, i32(pos[last]), i32(range(2)), part_o, part_ml, token, max_chunks=2, **common)
+        assert relative(token, exact[last]) < limit

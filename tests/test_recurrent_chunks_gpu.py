@@ -238,7 +238,22 @@ def gla_case():
         else:
             ops().gla_scan(*args, **sizes)
         return out, kept.view(5, 2, -1)
-    return views, run
+
+    def exact():
+        q, k, v, gate, inside = (views[m].double() for m in ("q", "k", "v", "gate", "decay"))
+        alpha = torch.exp(torch.nn.functional.logsigmoid(inside @ a2.double().T + bias.double()) / 16.0).view(tokens, heads, dim, 1)
+        q, k, v = (z.view(tokens, heads, *shape) for z, shape in ((q, (dim, 1)), (k, (dim, 1)), (v, (1, vdim))))
+        outs, states = [], []
+        for row, length in enumerate(LENGTHS):
+            kept = state[SLOTS[row], STARTS[row] & 1].double()
+            for t in range(AT[row], AT[row] + length):
+                kept = kept * alpha[t] + k[t] * v[t]
+                outs.append((kept * q[t]).sum(1) * dim ** -0.5)
+            states.append(kept)
+        o = torch.stack(outs)
+        o = o * torch.rsqrt((o * o).mean(-1, keepdim=True) + 1e-6) * norm.double()
+        return o * torch.nn.functional.silu(gate).view(tokens, heads, vdim), states
+    return views, run, exact
 
 
 def state_space_case():
@@ -377,7 +392,7 @@ def test_one_strong_decay_among_mild_ones(case, strong):
         assert ((state - states[row]).norm(dim=(1, 2)) / states[row].norm(dim=(1, 2))).max() < 300 * 2.0 ** -24
 
 
-@pytest.mark.parametrize("case", ["state space", "delta"])
+@pytest.mark.parametrize("case", CASES)
 def test_chunks_are_as_near_to_64_bits_as_tokens(case):
     """Outputs and states against a recurrence in 64 bits: a chunk's sums, of operands of 22 bits, are off by less than twice what the
     roundings of the decays and sums token by token come to.  (Left on the tensor cores, whose adder cuts off, they were off by up to
