@@ -1033,8 +1033,8 @@ def rows_f32(w: torch.Tensor, x: torch.Tensor, x_rows: Optional[torch.Tensor], t
           _ptr(out), feats, w.shape[2], int(paired), float(gate_limit))
 
 
-PRODUCTS_F32_TILE = 128    # rows of a tile of products_f32
-PRODUCTS_F32_AGAIN = 8 * (32 * 8 + 1)      # bytes of scratch for a tile and 128 features (FRB_PRODUCTS_AGAIN)
+PRODUCTS_F32_TILE = 160    # rows of a tile of products_f32
+PRODUCTS_F32_AGAIN = 8 * (32 * 12 + 1)     # bytes of scratch for a tile and 128 features (FRB_PRODUCTS_AGAIN)
 
 
 def products_f32_take(inner: int) -> bool:

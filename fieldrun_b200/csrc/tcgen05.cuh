@@ -40,6 +40,23 @@ __device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a_tmem, uint64_t b, 
         ::"r"(d), "r"(a_tmem), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
 }
 
+// D[tmem] = D 2^-SHIFT + A[tmem] * B[smem]^T (SHIFT up to 15)
+template <int SHIFT>
+__device__ __forceinline__ void mma_ts_scaled(uint32_t d, uint32_t a_tmem, uint64_t b, uint32_t idesc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, 1, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p, %4;\n\t}"
+        ::"r"(d), "r"(a_tmem), "l"(b), "r"(idesc), "n"(SHIFT) : "memory");
+}
+
+// True in one lane of a converged warp.  A loop that issues MMAs is run by a whole warp, and only the instructions themselves by this
+// lane: their operands are then in uniform registers, where a loop of one lane would have to move each of them there every time.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t mine;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(mine));
+    return mine != 0;
+}
+
 // The barrier gets one arrival when every MMA that this thread has issued so far has finished.
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");

@@ -26,10 +26,9 @@ STREAM_FEATURES = 65536   # beyond this many output features the library product
 # A float32 product runs on the tensor cores, each operand as two float16 parts (products_f32.cu), from SPLIT_PRODUCTS multiply-adds,
 # SPLIT_ROWS rows and SPLIT_TILES tiles of 128 x 128 results on.  Below, the pass over the weight for its scales (half of the bytes of
 # a product of few rows), the launches or the idle SMs cost more than the products save.  Measured on a B200 with weights that are not in
-# L2, microseconds, the library's float32 product | this one with its scales and parts: 200064 x 3072 weights, 9 rows 868 | 1040, 32 rows
-# 901 | 1006, 48 rows 1354 | 1075; 32768 x 4096, 32 rows 224 | 280, 48 rows 347 | 290; 8192 x 3072, 64 rows (2^30) 109 | 120, 96 rows
-# 135 | 126, 2,048 rows 1827 | 609; 3072 x 6144, 128 rows (24 tiles) 178 | 189, 256 rows 254 | 187; 2048 x 2048, 256 rows (2^30) 63 | 87, 512
-# rows 94 | 87; 1024 x 1024, 1,024 rows (2^30) 51 | 71, 2,048 rows 92 | 75; 256 x 3072, 2,048 rows 94 | 110.
+# L2, microseconds, the library's float32 product | this one with its scales and parts: 200064 x 3072 weights, 9 rows 868 | 1040 (not
+# faster since: the pass over the weight alone), 150 rows 4440 | 926; 32768 x 4096, 48 rows 332 | 209; 8192 x 3072, 96 rows 129 | 77, 700
+# rows 613 | 160; 3072 x 6144, 256 rows 250 | 113; 2048 x 2048, 512 rows 89 | 55; 1024 x 1024, 2,048 rows 87 | 46.
 SPLIT_ROWS = 48
 SPLIT_TILES = 32
 SPLIT_PRODUCTS = 1 << 31
@@ -71,9 +70,8 @@ def full_sums() -> None:
 
 
 def split_products_pay(rows: int, weight: torch.Tensor) -> bool:
-    tile = ops.PRODUCTS_F32_TILE
     return (rows * weight.numel() >= SPLIT_PRODUCTS and rows >= SPLIT_ROWS
-            and -(-rows // tile) * -(-weight.shape[0] // tile) >= SPLIT_TILES)
+            and -(-rows // 128) * -(-weight.shape[0] // 128) >= SPLIT_TILES)
 
 
 def float32_kernels_read(rows: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor]) -> bool:

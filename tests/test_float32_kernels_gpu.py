@@ -151,6 +151,18 @@ def test_split_products_are_as_exact_as_float32(rows, features, inner):
     assert ((got.double() - want).abs() <= 8 * 2.0 ** -23 * size).all()
 
 
+@pytest.mark.parametrize("rows,features,inner", [(1500, 6144, 2048), (1930, 4100, 200), (161, 21000, 320), (40, 40000, 64)])
+def test_split_products_of_several_items_a_block(rows, features, inner):
+    """A block goes on from item to item with its rings and accumulators at any place, while
+    the item before is written: the same bounds as for a single item."""
+    gen = torch.Generator(device=DEV).manual_seed(rows)
+    x, w = torch.randn(rows, inner, device=DEV, generator=gen), torch.randn(1, features, inner, device=DEV, generator=gen)
+    for _ in range(3):
+        got, want = split_product(w, x), x.double() @ w[0].double().T
+        size = x.double().norm(dim=1, keepdim=True) * w[0].double().norm(dim=1)[None]
+        assert ((got.double() - want).abs() <= 8 * 2.0 ** -23 * size).all()
+
+
 @pytest.mark.parametrize("limit", [0.0, 1.5])
 def test_split_products_of_experts(limit):
     """Expert lists: gathered rows, tiles of 1 to 128 rows, an expert without rows and one of several tiles, the gated second half."""
