@@ -42,12 +42,12 @@ TENSOR_CORE_ROWS_PER_EXPERT = {"decode": 4.0, "prompt": 1.0}
 
 
 # Above this many rows per expert (on average) a float32 step's expert products run on the tensor cores as split products, in
-# tiles of 128 rows; up to it, and below SPLIT_WORK multiply-adds, where their two more launches cost more than they save, as a
+# tiles of 160 rows; up to it, and below SPLIT_WORK multiply-adds, where their two more launches cost more than they save, as a
 # stream over the weights in tiles of eight.  Measured on a B200, the whole part, microseconds, stream | split: MiniMax-M2's sizes
-# 8 rows per expert 3030 | 3155, 16 rows 4664 | 3310; 16 experts of 2048 x 2048 8 rows 224 | 243, 16 rows 335 | 255; of 1024 x
-# 1024 16 rows 153 | 149; 8 experts of 96 x 48 (2^25 multiply-adds) 384 rows 112 | 148.
-SPLIT_ROWS_PER_EXPERT = 8.0
-SPLIT_WORK = 1 << 28
+# 3 rows per expert 2294 | 2303, 5 rows 2747 | 2466, 8 rows 3178 | 2497, 16 rows 4791 | 2600; 16 experts of 2048 x 2048 4 rows 231 | 249,
+# 6 rows 244 | 238, 16 rows 355 | 264; of 1024 x 1024 12 rows 166 | 221, 16 rows (3 x 2^28 multiply-adds) 157 | 151, 20 rows 190 | 152.
+SPLIT_ROWS_PER_EXPERT = 4.0
+SPLIT_WORK = 3 << 28
 
 FUSED_ACTIVATION_ROWS = 64      # from this many rows of a prompt step on, a dense unit's first product carries its activation
 
