@@ -64,7 +64,7 @@ attention_pair_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
 
     let_next_kernel_start();
     const int tile = gridDim.x - 1 - blockIdx.x, head = blockIdx.y;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int group = p.heads / p.v_heads, vh = head / group;
     const int b = p.tile_seq[tile], q0 = p.tile_q0[tile];
     const int q_len = p.seq_q_len[b], start = p.seq_start[b], tok0 = p.cu_q_len[b] + q0;
@@ -93,7 +93,7 @@ attention_pair_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
-    const uint32_t tmem = tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
     wait_for_previous_kernel();
 
     if (warp == 0) {
@@ -116,42 +116,49 @@ attention_pair_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc_o = instr_desc_bf16(AT_QUERIES, VD);
-            bool ok = bar_wait(&q_full, 0, failed);
-            if (!ok) atomicExch(p.status, 32);
-            auto issue_scores = [&](int m, int j) -> bool {
-                const int s = j % AP_STAGES;
-                if (!bar_wait(&kv_full[s], (j / AP_STAGES) & 1, failed)) { atomicExch(p.status, 33); return false; }
-                fence_after_sync();
-                const int pages = min(AP_STEP_PAGES, num_pages - AP_STEP_PAGES * j);
-                const uint32_t idesc_s = instr_desc_bf16(AT_QUERIES, pages * FRB_PAGE);
-                const uint64_t q_desc = tile_desc(smem_addr(q_tiles + m * Q_BYTES));
-                const uint64_t k_desc = tile_desc(smem_addr(stage0 + (size_t)s * STAGE_BYTES + m * K_STEP));
+        // the whole warp goes through the loop (elect_one, tcgen05.cuh)
+        const uint32_t idesc_o = instr_desc_bf16(AT_QUERIES, VD);
+        const uint32_t q_at = smem_addr(q_tiles), stages_at = smem_addr(stage0);
+        const int all_pages = __shfl_sync(0xffffffffu, num_pages, 0), steps = __shfl_sync(0xffffffffu, num_steps, 0);
+        bool ok = warp_wait(&q_full, 0, failed);
+        if (!ok && lane == 0) atomicExch(p.status, 32);
+        auto issue_scores = [&](int m, int j) -> bool {
+            const int s = j % AP_STAGES;
+            if (!warp_wait(&kv_full[s], (j / AP_STAGES) & 1, failed)) { if (lane == 0) atomicExch(p.status, 33); return false; }
+            fence_after_sync();
+            const int pages = min(AP_STEP_PAGES, all_pages - AP_STEP_PAGES * j);
+            const uint32_t idesc_s = instr_desc_bf16(AT_QUERIES, pages * FRB_PAGE);
+            const uint64_t q_desc = tile_desc(q_at + m * Q_BYTES), k_desc = tile_desc(stages_at + s * STAGE_BYTES + m * K_STEP);
+            if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < HD / 16; ++k)
                     mma_ss(tmem + SP_COL0 + AP_STEP_KEYS * m, q_desc + 2 * k, k_desc + 2 * k, idesc_s, k != 0);
                 mma_commit(&s_full[m]);
-                return true;
-            };
-            if (ok) ok = issue_scores(0, 0) && issue_scores(1, 0);
-            for (int j = 0; j < num_steps && ok; ++j) {
-                const int s = j % AP_STAGES;
-                const int pages = min(AP_STEP_PAGES, num_pages - AP_STEP_PAGES * j);
-                const uint64_t v_desc = tile_desc(smem_addr(stage0 + (size_t)s * STAGE_BYTES + 2 * K_STEP));
-                for (int m = 0; m < 2 && ok; ++m) {
-                    for (int h = 0; h < pages && ok; ++h) {
-                        if (!bar_wait(&p_full[m][h], j & 1, failed)) { atomicExch(p.status, 35); ok = false; break; }
-                        fence_after_sync();
+            }
+            __syncwarp();
+            return true;
+        };
+        if (ok) ok = issue_scores(0, 0) && issue_scores(1, 0);
+        for (int j = 0; j < steps && ok; ++j) {
+            const int s = j % AP_STAGES;
+            const int pages = min(AP_STEP_PAGES, all_pages - AP_STEP_PAGES * j);
+            const uint64_t v_desc = tile_desc(stages_at + s * STAGE_BYTES + 2 * K_STEP);
+            for (int m = 0; m < 2 && ok; ++m) {
+                for (int h = 0; h < pages && ok; ++h) {
+                    if (!warp_wait(&p_full[m][h], j & 1, failed)) { if (lane == 0) atomicExch(p.status, 35); ok = false; break; }
+                    fence_after_sync();
+                    if (elect_one()) {
 #pragma unroll
                         for (int k = 0; k < 4; ++k)            // 16 keys per MMA: 8 columns of packed P, 32 bytes of a V^T row
                             mma_ts(tmem + O_COL0 + 128 * m, tmem + SP_COL0 + AP_STEP_KEYS * m + 64 * h + 8 * k,
                                    v_desc + ((h * V_BYTES + k * 32) >> 4), idesc_o, (j | h | k) != 0);
+                        // every product of the step has been issued: its stage, once they end
+                        if (m == 1 && h == pages - 1) mma_commit(&kv_empty[s]);
                     }
-                    if (!ok) break;
-                    if (m == 1) mma_commit(&kv_empty[s]);      // every product of the step has been issued: its stage, once they end
-                    if (j + 1 < num_steps) ok = issue_scores(m, j + 1);
+                    __syncwarp();
                 }
+                if (!ok) break;
+                if (j + 1 < steps) ok = issue_scores(m, j + 1);
             }
         }
     } else {

@@ -83,7 +83,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     // are read, and barriers and tensor memory set up, while that kernel still runs.
     let_next_kernel_start();
     const int tile = gridDim.x - 1 - blockIdx.x, head = blockIdx.y;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int group = p.num_heads / p.num_kv_heads, kvh = head / group;
     const int b = p.tile_seq[tile], q0 = p.tile_q0[tile];
     const int q_len = p.seq_q_len[b], start = p.seq_start[b], tok0 = p.cu_q_len[b] + q0;
@@ -116,7 +116,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
-    const uint32_t tmem = tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
     wait_for_previous_kernel();
 
     if (warp == 0) {
@@ -142,22 +142,26 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // float32 accumulate, bf16 operands, K-major; S: M 128 x N 128 (64 for a step of one page); O_h: M 128 x N VD.
-            // The MMAs of this thread run in the order of their issue.  So S of step j + 2 may be asked for into the
-            // buffer of step j without a wait: P V of step j, which reads that buffer, was issued before, and was issued
-            // only when the softmax of step j had read its S and written its P.
-            const uint32_t idesc_o = instr_desc_bf16(AT_QUERIES, VD);
-            const uint64_t q_desc = tile_desc(smem_addr(q_tile));
-            bool ok = bar_wait(&q_full, 0, failed);
-            if (!ok) atomicExch(p.status, 12);
-            auto issue_scores = [&](int j) -> bool {
-                const int s = j % AT_STAGES;
-                if (!bar_wait(&kv_full[s], (j / AT_STAGES) & 1, failed)) { atomicExch(p.status, 13); return false; }
-                fence_after_sync();
-                const int pages = min(AT_STEP_PAGES, num_pages - AT_STEP_PAGES * j);
-                const uint32_t idesc_s = instr_desc_bf16(AT_QUERIES, pages * FRB_PAGE);
-                const uint64_t k_desc = tile_desc(smem_addr(stage0 + (size_t)s * STAGE_BYTES));
+        // The whole warp goes through the loop (elect_one, tcgen05.cuh): a prompt of 2,048 tokens in 48 heads of 128 takes 92 us, with a
+        // loop of one lane 99.
+        // float32 accumulate, bf16 operands, K-major; S: M 128 x N 128 (64 for a step of one page); O_h: M 128 x N VD.
+        // The MMAs of this warp run in the order of their issue.  So S of step j + 2 may be asked for into the
+        // buffer of step j without a wait: P V of step j, which reads that buffer, was issued before, and was issued
+        // only when the softmax of step j had read its S and written its P.
+        const uint32_t idesc_o = instr_desc_bf16(AT_QUERIES, VD);
+        const uint32_t stages_at = smem_addr(stage0);
+        const uint64_t q_desc = tile_desc(smem_addr(q_tile));
+        const int all_pages = __shfl_sync(0xffffffffu, num_pages, 0), steps = __shfl_sync(0xffffffffu, num_steps, 0);
+        bool ok = warp_wait(&q_full, 0, failed);
+        if (!ok && lane == 0) atomicExch(p.status, 12);
+        auto issue_scores = [&](int j) -> bool {
+            const int s = j % AT_STAGES;
+            if (!warp_wait(&kv_full[s], (j / AT_STAGES) & 1, failed)) { if (lane == 0) atomicExch(p.status, 13); return false; }
+            fence_after_sync();
+            const int pages = min(AT_STEP_PAGES, all_pages - AT_STEP_PAGES * j);
+            const uint32_t idesc_s = instr_desc_bf16(AT_QUERIES, pages * FRB_PAGE);
+            const uint64_t k_desc = tile_desc(stages_at + s * STAGE_BYTES);
+            if (elect_one()) {
 #pragma unroll
                 for (int kb = 0; kb < KBLOCKS; ++kb)
 #pragma unroll
@@ -165,27 +169,29 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                         mma_ss(tmem + SP_COL0 + AT_STEP_KEYS * (j & 1), q_desc + ((kb * (AT_QUERIES * 128) + k * 32) >> 4),
                                k_desc + ((kb * K_BLOCK_BYTES + k * 32) >> 4), idesc_s, (kb | k) != 0);
                 mma_commit(&s_full[j & 1]);
-                return true;
-            };
-            if (ok) ok = issue_scores(0);
-            bool begun[AT_STEP_PAGES] = {false, false};        // whether O_h holds anything yet
-            for (int j = 0; j < num_steps && ok; ++j) {
-                if (j + 1 < num_steps) ok = issue_scores(j + 1);
-                if (!ok) break;
-                const int s = j % AT_STAGES;
-                const int pages = min(AT_STEP_PAGES, num_pages - AT_STEP_PAGES * j);
-                const uint64_t v_desc = tile_desc(smem_addr(stage0 + (size_t)s * STAGE_BYTES + AT_STEP_PAGES * K_BYTES));
-                for (int h = 0; h < pages && ok; ++h) {
-                    if (!bar_wait(&p_full[j & 1][h], (j >> 1) & 1, failed)) { atomicExch(p.status, 15); ok = false; break; }
-                    fence_after_sync();
+            }
+            __syncwarp();
+            return true;
+        };
+        if (ok) ok = issue_scores(0);
+        for (int j = 0; j < steps && ok; ++j) {
+            if (j + 1 < steps) ok = issue_scores(j + 1);
+            if (!ok) break;
+            const int s = j % AT_STAGES;
+            const int pages = min(AT_STEP_PAGES, all_pages - AT_STEP_PAGES * j);
+            const uint64_t v_desc = tile_desc(stages_at + s * STAGE_BYTES + AT_STEP_PAGES * K_BYTES);
+            for (int h = 0; h < pages && ok; ++h) {
+                if (!warp_wait(&p_full[j & 1][h], (j >> 1) & 1, failed)) { if (lane == 0) atomicExch(p.status, 15); ok = false; break; }
+                fence_after_sync();
+                if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < 4; ++k)                // 16 keys per MMA: 8 columns of packed P, 32 bytes of a V^T row
                         mma_ts(tmem + O_COL0 + 128 * h, tmem + SP_COL0 + AT_STEP_KEYS * (j & 1) + 64 * h + 8 * k,
-                               v_desc + ((h * V_BYTES + k * 32) >> 4), idesc_o, begun[h] || k != 0);
-                    begun[h] = true;
+                               v_desc + ((h * V_BYTES + k * 32) >> 4), idesc_o, (j | k) != 0);     // step 0 begins O_h
+                    // the step's P V has ended: its stage is free, its O may be read
+                    if (h == pages - 1) mma_commit(&kv_empty[s]);
                 }
-                if (!ok) break;
-                mma_commit(&kv_empty[s]);              // the step's P V has ended: its stage is free, its O may be read
+                __syncwarp();
             }
         }
     } else {

@@ -135,11 +135,6 @@ __device__ __forceinline__ void split_four(float4 v, float scale, uint32_t& hi0,
     split_two(mul_pairs(pair_of(v.z, v.w), s), hi1, lo1);
 }
 
-// A wait of a whole warp: either all of its lanes go on or none.
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* failed) {
-    return __all_sync(0xffffffffu, bar_wait(bar, parity, failed));
-}
-
 // The exponent of a scale, a power of two, whatever its sign: -1 marks a row of zeros.
 __device__ __forceinline__ int scale_exponent(float scale) { return (int)(__float_as_uint(scale) >> 23 & 255) - 127; }
 

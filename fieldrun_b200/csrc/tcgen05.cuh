@@ -1,6 +1,6 @@
 // The fifth-generation tensor core: operand descriptors, MMA issue, completion, tensor-memory loads and stores.
 //
-// One thread of a block issues the MMAs; the accumulators (and, for `mma_ts`, the A operand) live in tensor
+// One warp of a block issues the MMAs, each by one of its lanes; the accumulators (and, for `mma_ts`, the A operand) live in tensor
 // memory, which one warp of the block allocates and frees.  Operands in shared memory are K-major tiles of
 // rows of 128 bytes under the 128-byte swizzle that TMA writes (tma.cuh).
 #pragma once
@@ -55,6 +55,11 @@ __device__ __forceinline__ bool elect_one() {
     uint32_t mine;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(mine));
     return mine != 0;
+}
+
+// A wait of a whole warp: either all of its lanes go on or none.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* failed) {
+    return __all_sync(0xffffffffu, frb_tma::bar_wait(bar, parity, failed));
 }
 
 // The barrier gets one arrival when every MMA that this thread has issued so far has finished.
