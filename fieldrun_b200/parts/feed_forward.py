@@ -41,13 +41,12 @@ TILE_ROWS = 32        # rows of one expert that a block of the expert kernels ta
 TENSOR_CORE_ROWS_PER_EXPERT = {"decode": 4.0, "prompt": 1.0}
 
 
-# Above this many rows per expert (on average) a float32 step's expert products run on the tensor cores as split products, in
-# tiles of 160 rows; up to it, and below SPLIT_WORK multiply-adds, where their two more launches cost more than they save, as a
+# A float32 step's expert products run on the tensor cores as split products, in tiles of 160 rows, where experts get more than so many
+# rows (on average) and the step has at least so many multiply-adds; elsewhere, where their two more launches cost more than they save, as a
 # stream over the weights in tiles of eight.  Measured on a B200, the whole part, microseconds, stream | split: MiniMax-M2's sizes
 # 3 rows per expert 2294 | 2303, 5 rows 2747 | 2466, 8 rows 3178 | 2497, 16 rows 4791 | 2600; 16 experts of 2048 x 2048 4 rows 231 | 249,
-# 6 rows 244 | 238, 16 rows 355 | 264; of 1024 x 1024 12 rows 166 | 221, 16 rows (3 x 2^28 multiply-adds) 157 | 151, 20 rows 190 | 152.
-SPLIT_ROWS_PER_EXPERT = 4.0
-SPLIT_WORK = 3 << 28
+# 6 rows 244 | 238, 16 rows 355 | 264; of 1024 x 1024 8 rows 108 | 187, 16 rows 157 | 151, 20 rows 190 | 152.
+SPLIT_ROWS_PER_EXPERT = ((4.0, 1 << 30), (8.0, 1 << 28))
 
 FUSED_ACTIVATION_ROWS = 64      # from this many rows of a prompt step on, a dense unit's first product carries its activation
 
@@ -247,8 +246,9 @@ class RoutedExperts(FeedForward):
 
     def on_split_products(self, assignments: int) -> bool:
         """Whether a float32 step's experts run as split products on the tensor cores (products_f32.cu)."""
-        return (self.split_scales is not None and assignments > SPLIT_ROWS_PER_EXPERT * self.num_experts
-                and assignments * 3 * self.hidden_size * self.expert_width >= SPLIT_WORK and 2 * assignments < (1 << 31) - 1024)
+        work = assignments * 3 * self.hidden_size * self.expert_width
+        return (self.split_scales is not None and any(assignments > rows * self.num_experts and work >= least for rows, least in SPLIT_ROWS_PER_EXPERT)
+                and 2 * assignments < (1 << 31) - 1024)
 
     def streams_float32(self, assignments: int) -> bool:
         """Whether the float32 stream over the weights takes the step: sizes in steps of 4 (16-byte loads), and lists of tiles
