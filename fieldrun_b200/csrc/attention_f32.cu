@@ -1,7 +1,8 @@
 // Attention over the paged cache in float32 for the head sizes that models have: the float32 path's prompts in tiles of 64
 // queries, and its single tokens in chunks of 256 keys that run side by side.  Same formulas and options as
 // attention_generic.cu (window, chunk, first tokens, slopes, sinks, cap, gates, a value head of another size, key heads that
-// share a value head), which keeps the sizes these kernels do not take.  Everything is float32; the tiles' products run on tensor
+// share a value head), which keeps the sizes these kernels do not take; attention_f32_tc.cu takes all but the smallest steps of prompts with
+// heads of 64 and 128.  Everything is float32; the tiles' products run on tensor
 // cores with each operand as two TF32 parts (tf32_parts.cuh).
 //
 // What bounds them.  Prompts: the instructions that split the operands and the tensor cores; attention_generic runs a block per
@@ -10,20 +11,8 @@
 // scores and 8 x 8 sums a thread on the ordinary pipes took 1.59 ms (30 TFLOP/s), on the tensor cores 1.12 ms (43).  Single tokens: the
 // keys' and values' bytes; there a block per token and key head left 48 blocks on 148 SMs, each walking its whole sequence: 1.20 ms
 // for six sequences of 17 to 1,500 keys; the whole layer went from 1.33 to 0.08 ms, most of it the dense products.
+#include "attention_f32.cuh"
 #include "tf32_parts.cuh"
-
-struct F32Attention {
-    const float* q;           // [T, nh, hd]
-    const float* k_pages;     // [pages, nkv, PAGE, hd]
-    const float* v_pages;     // [pages, v_heads, vd, PAGE]
-    const float* slopes;      // [nh] or null
-    const float* sinks;       // [nh] or null
-    const float* gate;        // [T, gate_stride] or null
-    const int* page_table;    // [slots, max_pages]
-    float* out;               // [T, nh * vd]
-    float scale, softcap;
-    int gate_stride, chunk, keep_first, window, max_pages, num_heads, num_kv_heads, v_heads, head_dim, v_dim;
-};
 
 __device__ __forceinline__ float dot4(float4 a, float4 b, float c) {
     c = fmaf(a.x, b.x, c);
@@ -32,59 +21,10 @@ __device__ __forceinline__ float dot4(float4 a, float4 b, float c) {
     return fmaf(a.w, b.w, c);
 }
 
-// The score of key j for the query at `pos` from the raw product, or -infinity where the key is hidden.
-__device__ __forceinline__ float f32_score(const F32Attention& p, float raw, float slope, int pos, int j, bool visible) {
-    float s = raw * p.scale;
-    if (p.softcap > 0.f) s = p.softcap * tanhf(s / p.softcap);
-    return visible ? s - slope * (float)(pos - j) : -INFINITY;
-}
-
 // ----------------------------------------------------------------------------- prompts
 
 #define TILE_Q 64             // queries of one head a block takes
 #define TILE_THREADS 128
-
-// One query of one head key by key in float32, a warp a query: the sums of attention_generic.
-static __device__ __forceinline__ void f32_query_key_by_key(const F32Attention& p, const int* table, int head, int g, int vg, int pos, size_t token) {
-    const int lane = threadIdx.x & 31, hd = p.head_dim, vd = p.v_dim, lo = first_visible_key(pos, p.window, p.chunk);
-    const int first = lo / 32, kept = kept_runs(p.keep_first, 32, first), blocks = kept + pos / 32 - first + 1;
-    const float* q = p.q + (token * p.num_heads + head) * hd;
-    const float slope = p.slopes ? p.slopes[head] : 0.f;
-    float m = -INFINITY, l = 0.f, acc[4] = {};
-    for (int n = 0; n < blocks; ++n) {
-        const int j0 = run_at(n, kept, first) * 32, j = j0 + lane, page = table[j0 / FRB_PAGE], in_page = j0 % FRB_PAGE;
-        const bool visible = key_visible(j, lo, pos, p.keep_first);
-        const float* k = p.k_pages + (((size_t)page * p.num_kv_heads + g) * FRB_PAGE + in_page + lane) * hd;
-        const float* v = p.v_pages + ((size_t)page * p.v_heads + vg) * FRB_PAGE * vd + in_page;
-        float s = 0.f;
-        if (visible)
-            for (int d = 0; d < hd; ++d) s = fmaf(q[d], k[d], s);
-        s = f32_score(p, s, slope, pos, j, visible);
-        const float top = fmaxf(m, warp_max(s)), corr = expf(m - top), w = visible ? expf(s - top) : 0.f;
-        l = l * corr + warp_sum(w);
-        m = top;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[i] *= corr;
-        for (int kk = 0; kk < 32; ++kk) {
-            const float wk = __shfl_sync(0xffffffffu, w, kk);
-            if (key_visible(j0 + kk, lo, pos, p.keep_first))
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (lane + 32 * i < vd) acc[i] = fmaf(wk, v[(size_t)(lane + 32 * i) * FRB_PAGE + kk], acc[i]);
-        }
-    }
-    if (p.sinks) {
-        const float sink = p.sinks[head], top = fmaxf(m, sink), corr = expf(m - top);
-        l = l * corr + expf(sink - top);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[i] *= corr;
-    }
-    float inv = 1.0f / l;
-    if (p.gate) inv *= 1.0f / (1.0f + expf(-p.gate[token * p.gate_stride + head]));
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-        if (lane + 32 * i < vd) p.out[(token * p.num_heads + head) * vd + lane + 32 * i] = acc[i] * inv;
-}
 
 // A block takes 64 neighbouring queries of one head and walks the pages of 64 keys that any of them sees; a warp has 16 of the
 // queries.  Both products run on tensor cores with each operand as two TF32 parts; the weights stay in the registers that the
@@ -460,22 +400,6 @@ attention_f32_merge_kernel(F32Attention p, const int* __restrict__ tok_pos, cons
 }
 
 // ----------------------------------------------------------------------------- host side
-
-static int f32_attention_params(F32Attention* p, const float* q, const float* k_pages, const float* v_pages, const int* page_table,
-                                int max_pages, float* out, int num_heads, int num_kv_heads, int head_dim, int v_dim, float scale, int window,
-                                const float* slopes, int chunk, const float* sinks, const float* gate, int gate_stride, float softcap,
-                                int keep_first, int num_v_heads) {
-    FRB_CHECK_ARG(num_kv_heads >= 1 && num_heads % num_kv_heads == 0, "attention: %d heads are not a multiple of %d kv heads", num_heads,
-                  num_kv_heads);
-    FRB_CHECK_ARG(num_v_heads >= 1 && num_kv_heads % num_v_heads == 0, "attention: %d key heads over %d value heads", num_kv_heads, num_v_heads);
-    FRB_CHECK_ARG(keep_first >= 0 && !(keep_first > 0 && chunk > 0), "attention: %d first tokens together with chunks", keep_first);
-    FRB_CHECK_ARG((((uintptr_t)q | (uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0, "attention: queries and pages must be 16-byte aligned");
-    p->q = q; p->k_pages = k_pages; p->v_pages = v_pages; p->slopes = slopes; p->sinks = sinks; p->gate = gate; p->page_table = page_table;
-    p->out = out; p->scale = scale; p->softcap = softcap; p->gate_stride = gate_stride; p->chunk = chunk;
-    p->keep_first = window > 0 ? keep_first : 0; p->window = window; p->max_pages = max_pages; p->num_heads = num_heads;
-    p->num_kv_heads = num_kv_heads; p->v_heads = num_v_heads; p->head_dim = head_dim; p->v_dim = v_dim;
-    return 0;
-}
 
 // Prompts.  tile_seq/tile_q0: the step's tiles of 128 queries (sequence, first query among its new tokens).
 FRB_API int frb_attention_f32_tiles(const float* q, const float* k_pages, const float* v_pages, const int* page_table, int max_pages,

@@ -13,9 +13,8 @@
 //                  accumulator of its own (all 512 columns: S/P twice, O twice).
 //   the end        out = (O_0 a_0 + O_1 a_1) / (l_0 a_0 + l_1 a_1) with a_h = 2^(m_h - max(m_0, m_1)).
 // One warp per scheduler (four in all) could not hide its own latencies: measured with clock stamps, a step's
-// softmax then took 1,790 cycles beside 1,600 cycles of MMA issue (8 + 8 MMAs of about 100 cycles each, the
-// least that one tcgen05.mma of M 128 takes here whatever N up to 128), and each side waited a quarter of its
-// time for the other.
+// softmax then took 1,790 cycles beside 1,600 cycles of MMA issue (8 + 8 MMAs of about 100 cycles each when one
+// lane ran the loop that issues them), and each side waited a quarter of its time for the other.
 // The running maximum of a row is only raised when the step's maximum exceeds it by more than 8 (in units of
 // log2): the weights are then at most 2^8, the result is the same after the division by the row's sum, and
 // O has to be rescaled (read, multiplied, written back) only on those rare pages.

@@ -32,7 +32,7 @@ GROUPS: dict[str, tuple[str, ...]] = {
     "common": ("elementwise.cu", "layernorm.cu", "attention_generic.cu", "sampling.cu", "stream_ops.cu", "token_inputs.cu",
                "sandwich_norm.cu", "poly_norm.cu"),
     "attention": ("attention_mma.cu", "attention_decode_tma.cu", "attention_tc.cu", "attention_pair_tc.cu"),
-    "attention32": ("attention_f32.cu",),
+    "attention32": ("attention_f32.cu", "attention_f32_tc.cu"),
     "streams": ("experts_stream.cu", "experts_mma.cu", "rows_f32.cu"),
     "experts": ("routing.cu", "experts_generic.cu"),
     "products": ("experts_tc.cu",),

@@ -27,6 +27,7 @@ _SIGNATURES = {
     "frb_add_rows": "ppl",
     "frb_attention_generic": "pppipipppiiiifiipippif" "iii",
     "frb_attention_f32_tiles": "ppppi" "ppippppp" "iiiif" "ipippi" "fii",
+    "frb_attention_f32_tc": "ppppi" "ppippppii" "pp" "piiiif" "ipippi" "fii",
     "frb_attention_f32_token": "ppppi" "ppippip" "iiiif" "ipippi" "fii",
     "frb_layernorm": "ppppfppiii",
     "frb_unary_unit": "ppili",
@@ -109,7 +110,7 @@ _ENTRY_GROUPS = {
                "frb_latent_attention_mma", "frb_latent_attention_tc"),
     "attention": ("frb_attention_decode_mma", "frb_attention_prefill_mma", "frb_attention_decode_tma", "frb_attention_prefill_tc",
                   "frb_attention_pair_tc"),
-    "attention32": ("frb_attention_f32_tiles", "frb_attention_f32_token"),
+    "attention32": ("frb_attention_f32_tiles", "frb_attention_f32_tc", "frb_attention_f32_token"),
     "streams": ("frb_weight_stream", "frb_expert_gemm_mma", "frb_rows_f32"),
     "experts": ("frb_router_topk", "frb_expert_plan", "frb_expert_combine", "frb_expert_gemm_generic", "frb_route_plan_small",
                 "frb_router_small", "frb_router_logits", "frb_scaled_rows"),
@@ -201,7 +202,7 @@ def _stream() -> int:
 
 
 _LAUNCHES = 0
-_KERNELS_PER_CALL = {"frb_gated_delta_rule": 2, "frb_gated_recurrence": 2, "frb_sample_floor": 3, "frb_argmax_rows": 2, "frb_expert_plan": 3, "frb_attention_decode_mma": 2, "frb_attention_decode_tma": 2, "frb_attention_f32_token": 2, "frb_gla_chunks": 3, "frb_state_space_chunks": 4, "frb_delta_chunks": 3, "frb_products_f32": 2}
+_KERNELS_PER_CALL = {"frb_gated_delta_rule": 2, "frb_gated_recurrence": 2, "frb_sample_floor": 3, "frb_argmax_rows": 2, "frb_expert_plan": 3, "frb_attention_decode_mma": 2, "frb_attention_decode_tma": 2, "frb_attention_f32_token": 2, "frb_gla_chunks": 3, "frb_state_space_chunks": 4, "frb_delta_chunks": 3, "frb_products_f32": 2, "frb_attention_f32_tc": 2}
 
 
 def launches() -> int:
@@ -892,10 +893,24 @@ def attention_generic(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
 MAX_GRID_YZ = 65535        # blocks of a grid along y and z
 
 
+PAGE = 64                  # tokens of a cache page (FRB_PAGE)
+
+
 def attention_f32_tiles_take(head_dim: int, v_dim: int, tiles: int = 1) -> bool:
     """Whether :func:`attention_f32_tiles` takes heads of these sizes (rows in 16-byte units, two blocks' tiles on an SM) and so many
     tiles of 128 queries (two blocks along y each)."""
     return head_dim % 4 == 0 and 4 <= head_dim <= 128 and 1 <= v_dim <= 128 and 2 * tiles <= MAX_GRID_YZ
+
+
+def attention_f32_tc_takes(head_dim: int, v_dim: int, scale: float, tiles: int = 1) -> bool:
+    """Whether :func:`attention_f32_tc` takes heads of these sizes, this softmax scale and so many tiles of 128 queries (along y)."""
+    return (head_dim, v_dim) in ((64, 64), (64, 128), (128, 128)) and scale > 0 and tiles <= MAX_GRID_YZ
+
+
+def attention_f32_tc_scratch(pages: int, num_kv_heads: int, head_dim: int, v_dim: int, maps: int = 1) -> int:
+    """Floats of scratch that :func:`attention_f32_tc` needs for so many pages: the parts of the keys and values, and their scales."""
+    v_heads = num_kv_heads // maps
+    return pages * (num_kv_heads * PAGE * head_dim + v_heads * PAGE * v_dim + num_kv_heads + v_heads)
 
 
 def attention_f32_token_takes(head_dim: int, v_dim: int, tokens: int = 1) -> bool:
@@ -934,6 +949,25 @@ def attention_f32_tiles(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.T
                                      softcap, keep_first, maps)
     _call("frb_attention_f32_tiles", _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(page_table), page_table.shape[1], _ptr(tile_seq),
           _ptr(tile_q0), tile_seq.numel(), _ptr(seq_slot), _ptr(seq_start), _ptr(seq_q_len), _ptr(cu_q_len), _ptr(out), *options)
+
+
+def attention_f32_tc(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, page_table: torch.Tensor, tile_seq: torch.Tensor,
+                     tile_q0: torch.Tensor, seq_slot: torch.Tensor, seq_start: torch.Tensor, seq_q_len: torch.Tensor,
+                     cu_q_len: torch.Tensor, scratch: torch.Tensor, total_pages: int,
+                     out: torch.Tensor, *, num_heads: int, num_kv_heads: int, head_dim: int, scale: float,
+                     window: Optional[int], v_dim: Optional[int] = None, slopes: Optional[torch.Tensor] = None,
+                     chunk: Optional[int] = None, sinks: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None,
+                     softcap: Optional[float] = None, keep_first: int = 0, maps: int = 1) -> None:
+    """:func:`attention_f32_tiles` on tcgen05 (attention_f32_tc.cu).  ``total_pages``: the pages that the step's sequences may see
+    (``StepContext.visible_pages``); ``scratch``: :func:`attention_f32_tc_scratch` floats; sizes as :func:`attention_f32_tc_takes` says."""
+    options = _attention_f32_options(q, k_pages, out, num_heads, num_kv_heads, head_dim, v_dim, scale, window, slopes, chunk, sinks, gate,
+                                     softcap, keep_first, maps)
+    _want(scratch, torch.float32, "the pages' parts")
+    if scratch.numel() < attention_f32_tc_scratch(total_pages, num_kv_heads, head_dim, options[3], maps):
+        raise KernelError(f"the parts of {total_pages} pages do not fit {list(scratch.shape)}")
+    _call("frb_attention_f32_tc", _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(page_table), page_table.shape[1], _ptr(tile_seq),
+          _ptr(tile_q0), tile_seq.numel(), _ptr(seq_slot), _ptr(seq_start), _ptr(seq_q_len), _ptr(cu_q_len), seq_q_len.numel(), total_pages,
+          _ptr(scratch), _ptr(tc_status(q.device)), _ptr(out), *options)
 
 
 def attention_f32_token(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, page_table: torch.Tensor, tok_pos: torch.Tensor,
@@ -1485,13 +1519,17 @@ _WAIT_CODES = {
     19: "prompt attention: the epilogue waiting for the last steps",
     41: "float32 products: the producer waiting for a free stage of weights",
     42: "float32 products: the producer waiting for a free stage of rows",
-    43: "float32 products: the MMA thread waiting for the small sums to have been read",
-    44: "float32 products: the MMA thread waiting for the large sums to have been read",
-    45: "float32 products: the MMA thread waiting for the weights' parts",
-    46: "float32 products: the MMA thread waiting for a loaded stage of rows",
-    47: "float32 products: a worker waiting for finished sums",
-    48: "float32 products: a worker waiting for a loaded stage of weights",
-    49: "float32 products: a worker waiting for a free stage of parts",
+    43: "float32 products: the MMA warp waiting for a step's operands or for its sums to have been read",
+    44: "float32 products: a splitter waiting for a loaded stage of weights",
+    45: "float32 products: a splitter waiting for a free stage of parts",
+    46: "float32 products: a collector waiting for finished sums",
+    51: "float32 prompt attention: the producer waiting for a free stage of keys",
+    52: "float32 prompt attention: the producer waiting for a free stage of values",
+    53: "float32 prompt attention: the MMA warp waiting for a page's keys",
+    54: "float32 prompt attention: waiting for the queries' parts",
+    55: "float32 prompt attention: the MMA warp waiting for a page's weights or values",
+    58: "float32 prompt attention: the rows waiting for a page's sums",
+    59: "float32 prompt attention: the rows waiting for a page's scores",
     31: "attention of two maps: the producer waiting for a free key/value stage",
     32: "attention of two maps: the query tiles' copies",
     33: "attention of two maps: the MMA thread waiting for a loaded key/value stage",

@@ -34,10 +34,7 @@
 // of the entries a lane, split it and store the parts to tensor memory, where they are the first operand of
 // tcgen05.mma: shared memory then carries the weights twice and the rows of x three times a step instead of the split weights
 // three times more.  Eight more warps take the sums of one step out of tensor memory while the tensor cores make the next one's.
-#include <cuda_fp16.h>
-
-#include "attention_tc.cuh"
-#include "tcgen05.cuh"
+#include "f16_parts.cuh"
 
 #define PF_FEATS 128
 #define PF_ROWS 160
@@ -67,7 +64,6 @@ static_assert(PF_PARTS(PF_STAGES) <= 512, "columns of tensor memory");
 
 using namespace frb_tma;
 using namespace frb_tc;
-using namespace frb_at;
 
 // An item: a tile's rows, and 128 features from f0 on.
 struct Item {
@@ -113,41 +109,12 @@ struct ProductsParams {
     }
 };
 
-__device__ __forceinline__ uint32_t half2_bits(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
-
-// The parts of four entries times their row's scale; lo is 2^11 times what hi leaves, so that it is no smaller than hi.
-#define PF_LO 2048.f
-__device__ __forceinline__ void split_two(uint64_t v, uint32_t& hi, uint32_t& lo) {
-    float a, b;
-    halves_of(v, a, b);
-    const __half2 h = __floats2half2_rn(a, b);
-    hi = half2_bits(h);
-    // 2^11 v - 2^11 hi: both exact, and so is what is left
-    halves_of(mul_pairs(v, pair_of(PF_LO, PF_LO)), a, b);
-    asm("{\n\t.reg .f16 l, h, m;\n\tmov.b32 {l, h}, %2;\n\tmov.b16 m, 0xE800;\n\t"
-        "fma.rn.f32.f16 %0, l, m, %0;\n\tfma.rn.f32.f16 %1, h, m, %1;\n\t}" : "+f"(a), "+f"(b) : "r"(hi));
-    lo = half2_bits(__floats2half2_rn(a, b));
-}
-
-__device__ __forceinline__ void split_four(float4 v, float scale, uint32_t& hi0, uint32_t& hi1, uint32_t& lo0, uint32_t& lo1) {
-    const uint64_t s = pair_of(scale, scale);
-    split_two(mul_pairs(pair_of(v.x, v.y), s), hi0, lo0);
-    split_two(mul_pairs(pair_of(v.z, v.w), s), hi1, lo1);
-}
-
 // The exponent of a scale, a power of two, whatever its sign: -1 marks a row of zeros.
 __device__ __forceinline__ int scale_exponent(float scale) { return (int)(__float_as_uint(scale) >> 23 & 255) - 127; }
 
 // Whether an output is zero for its row's or its weight row's zeros (the other being finite, and the sum zero still).
 __device__ __forceinline__ bool is_of_zeros(float sum, float w_scale, float x_scale) {
     return sum == 0.f && (x_scale < 0.f ? w_scale != 0.f : w_scale < 0.f && x_scale != 0.f);
-}
-
-// The waits of a warp for two barriers, both looked at before either is waited for.
-__device__ __forceinline__ bool warp_wait_both(uint64_t* bar0, uint32_t parity0, uint64_t* bar1, uint32_t parity1, volatile int* failed) {
-    const bool first = bar_try(smem_addr(bar0), parity0), second = bar_try(smem_addr(bar1), parity1);
-    if (__all_sync(0xffffffffu, first && second)) return true;
-    return warp_wait(bar0, parity0, failed) && warp_wait(bar1, parity1, failed);
 }
 
 // A collector's columns of an item: the sums in units of the scales, to out [rows, features]; which of them are to be summed again.

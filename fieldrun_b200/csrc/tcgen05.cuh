@@ -62,6 +62,13 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volati
     return __all_sync(0xffffffffu, frb_tma::bar_wait(bar, parity, failed));
 }
 
+// The waits of a warp for two barriers, both looked at before either is waited for.
+__device__ __forceinline__ bool warp_wait_both(uint64_t* bar0, uint32_t parity0, uint64_t* bar1, uint32_t parity1, volatile int* failed) {
+    const bool first = frb_tma::bar_try(smem_addr(bar0), parity0), second = frb_tma::bar_try(smem_addr(bar1), parity1);
+    if (__all_sync(0xffffffffu, first && second)) return true;
+    return warp_wait(bar0, parity0, failed) && warp_wait(bar1, parity1, failed);
+}
+
 // The barrier gets one arrival when every MMA that this thread has issued so far has finished.
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");

@@ -8,10 +8,12 @@ the host (for decisions) and on the device (for the kernels).
 """
 from __future__ import annotations
 
-from typing import Sequence
+from typing import Optional, Sequence
 
 import numpy as np
 import torch
+
+from ..cache.sequence_cache import PAGE_TOKENS
 
 
 class Workspace:
@@ -168,6 +170,24 @@ class StepContext:
             count = len(seqs)
             kept[size] = (flat[:count], flat[count:2 * count], flat[2 * count:3 * count], flat[3 * count:])
         return kept[size]
+
+    def visible_pages(self, window: Optional[int], chunk: Optional[int], keep_first: int) -> int:
+        """How many cache pages the new tokens may see, each sequence's own: from its first token's window (or chunk) on, and the pages
+        of the first tokens that stay visible beside the window.  For steps of prompts only, as :meth:`token_chunks`."""
+        kept = self.__dict__.setdefault("_visible_pages", {})
+        key = (window, chunk, keep_first)
+        if key not in kept:
+            total = 0
+            for start, n in zip(self.seq_starts, self.seq_q_lens):
+                if n == 0:
+                    continue
+                low = max(0, start - int(window) + 1) if window else 0
+                if chunk:
+                    low = max(low, start // chunk * chunk)
+                first = low // PAGE_TOKENS
+                total += min(-(-(keep_first if window else 0) // PAGE_TOKENS), first) + (start + n - 1) // PAGE_TOKENS - first + 1
+            kept[key] = total
+        return kept[key]
 
     def query_tiles(self, rows: int) -> tuple[torch.Tensor, torch.Tensor]:
         """Tiles of ``rows`` consecutive new tokens that never span two sequences: (sequence of each tile,

@@ -50,6 +50,12 @@ from .linear import linear
 
 
 TC_ATTENTION_MIN_QUERIES = 64       # a step whose longest run of new tokens is shorter uses tiles of 16 queries
+# A float32 prompt's attention runs on tcgen05 (attention_f32_tc.cu) where query heads times the longest sequence's keys come to this, else
+# in tiles on mma.sync.  Measured on a B200, microseconds of the kernels, tiles | tcgen05: 48 heads over 8 of 128, prompts of 64 tokens 25 | 17, 300
+# tokens 66 | 22, 527 tokens 116 | 38, 64 tokens behind 20,000 2925 | 465; 16 heads over 4 of 64, 64 tokens 13 | 11, 200 tokens 32 | 14.  Its second
+# launch is 12 us of the host's time more, which a small layer's step of a few dozen tokens waits for.
+F32_TC_KEYS = 3072
+F32_TC_SCRATCH = 1 << 28           # floats that the parts of the pages in sight may take (a gigabyte: 128,000 tokens of MiniMax-M2's layer)
 
 
 class GQAAttention(Mixer):
@@ -300,8 +306,17 @@ class GQAAttention(Mixer):
         elif (self.float32_tiles and not ctx.is_decode
               and ops.attention_f32_tiles_take(self.head_dim, self.value_dim, ctx.query_tiles(ops.TC_ATTENTION_QUERIES)[0].numel())):
             tile_seq, tile_q0 = ctx.query_tiles(ops.TC_ATTENTION_QUERIES)
-            ops.attention_f32_tiles(q, line.keys, line.values, line.page_table, tile_seq, tile_q0, ctx.seq_slot, ctx.seq_start,
-                                    ctx.seq_q_len, ctx.cu_q_len, maps_out, gate=gate, **common)
+            pages = floats = 0
+            if self.q_heads * ctx.max_kv_len >= F32_TC_KEYS and ops.attention_f32_tc_takes(self.head_dim, self.value_dim, self.softmax_scale, tile_seq.numel()):
+                pages = ctx.visible_pages(self.window, self.chunk, self.keep_first)
+                floats = ops.attention_f32_tc_scratch(pages, self.k_heads, self.head_dim, self.value_dim, self.maps)
+            if 0 < floats <= F32_TC_SCRATCH:
+                ops.attention_f32_tc(q, line.keys, line.values, line.page_table, tile_seq, tile_q0, ctx.seq_slot, ctx.seq_start,
+                                     ctx.seq_q_len, ctx.cu_q_len, ctx.buffer("attention.parts", (floats,), torch.float32), pages, maps_out,
+                                     gate=gate, **common)
+            else:
+                ops.attention_f32_tiles(q, line.keys, line.values, line.page_table, tile_seq, tile_q0, ctx.seq_slot, ctx.seq_start,
+                                        ctx.seq_q_len, ctx.cu_q_len, maps_out, gate=gate, **common)
         else:
             ops.attention_generic(q, line.keys, line.values, line.page_table, ctx.tok_pos, ctx.tok_slot, maps_out, gate=gate, **common)
         if maps_out is not out:

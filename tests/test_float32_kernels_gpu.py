@@ -3,6 +3,8 @@ import numpy as np
 import pytest
 import torch
 
+from fieldrun_b200.engine.context import StepContext, Workspace
+
 pytestmark = pytest.mark.gpu
 
 DEV = "cuda"
@@ -401,3 +403,105 @@ def test_float32_attention_is_as_near_to_64_bits_as_the_general_kernel(heads, kv
         token, part_o, part_ml = (torch.full(shape, NAN, device=DEV) for shape in ((2, heads * dim), (2, heads, 2, dim), (2, heads, 2, 2)))
         ops().attention_f32_token(q[last], keys, values, table, i32(pos[last]), i32(range(2)), part_o, part_ml, token, max_chunks=2, **common)
         assert relative(token, exact[last]) < limit
+
+
+TC_SHAPES = [(8, 8, 64, 64, 1), (12, 2, 128, 128, 1), (8, 4, 64, 128, 2), (3, 1, 128, 128, 1)]
+
+
+def attention_on_tcgen05(q, keys, values, table, starts, lengths, out, **common):
+    """Prompts by the tcgen05 kernel, its scratch full of NaNs before."""
+    kv_heads, maps, dim, vdim = common["num_kv_heads"], common.get("maps", 1), common["head_dim"], common.get("v_dim") or common["head_dim"]
+    assert ops().attention_f32_tc_takes(dim, vdim, common["scale"])
+    pages = StepContext(Workspace(DEV), torch.float32, range(len(starts)), starts, lengths).visible_pages(
+        common.get("window"), common.get("chunk"), common.get("keep_first", 0))
+    scratch = torch.full((ops().attention_f32_tc_scratch(pages, kv_heads, dim, vdim, maps) + 64,), NAN, device=DEV)
+    tiles = [(b, q0) for b, n in enumerate(lengths) for q0 in range(0, n, 128)]
+    ops().attention_f32_tc(q, keys, values, table, i32([t[0] for t in tiles]), i32([t[1] for t in tiles]), i32(range(len(lengths))), i32(starts),
+                           i32(lengths), i32(np.concatenate([[0], np.cumsum(lengths)])), scratch[:-64], pages, out, **common)
+    ops().tc_status_check(out.device)
+    assert scratch[-64:].isnan().all() and not scratch[:-64].isnan().all()
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,maps", TC_SHAPES)
+@pytest.mark.parametrize("starts,lengths", [([0, 3, 0, 130, 64], [1, 64, 65, 200, 127]), ([0, 700, 64], [620, 150, 1]), ([0] * 70, [1, 2, 64, 65, 129] * 14)])
+def test_prompts_on_tcgen05_equal_the_general_kernel(heads, kv_heads, dim, vdim, maps, form, starts, lengths):
+    """One page to a dozen, tiles of 1 to 128 queries, more sequences than a warp has lanes; the bounds of the tiles on mma.sync."""
+    keys, values, table, gen = paged(starts, lengths, kv_heads, kv_heads // maps, dim, vdim, 3)
+    tokens = sum(lengths)
+    q = torch.randn(tokens, heads * dim, device=DEV, generator=gen)
+    common = dict(num_heads=heads, num_kv_heads=kv_heads, head_dim=dim, v_dim=vdim, scale=dim ** -0.5, maps=maps,
+                  **options(form, heads, tokens, gen))
+    pos = np.concatenate([s + np.arange(n) for s, n in zip(starts, lengths)])
+    want, got = (torch.full((tokens, heads * vdim), NAN, device=DEV) for _ in range(2))
+    ops().attention_generic(q, keys, values, table, i32(pos), i32(np.repeat(np.arange(len(starts)), lengths)), want, **common)
+    attention_on_tcgen05(q, keys, values, table, starts, lengths, got, **common)
+    check(got, want, 850)
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,maps", TC_SHAPES[:3])
+def test_infinities_and_nans_on_tcgen05_reach_the_queries_that_see_them(heads, kv_heads, dim, vdim, maps, form):
+    """As for the tiles on mma.sync; and queries and keys too large for parts, and pages far apart in size."""
+    starts, lengths = [0, 3, 0, 130, 64], [1, 64, 65, 200, 127]
+    keys, values, table, gen = paged(starts, lengths, kv_heads, kv_heads // maps, dim, vdim, 9)
+    tokens, ends = sum(lengths), [s + n for s, n in zip(starts, lengths)]
+    values[int(table[3, 0])] *= 1e-30
+    values[int(table[3, 1])] *= 1e25
+    keys[int(table[2, 0])] *= 1e-25
+    for row, n in enumerate(ends):
+        for at in range(n, (n + 63) // 64 * 64):
+            plant(keys, values, table, row, at, NAN, NAN if at % 2 else INF)
+    plant(keys, values, table, 1, 40, value=INF)
+    plant(keys, values, table, 2, 63, value=NAN)
+    plant(keys, values, table, 2, 64, value=-3.4028234e38)
+    plant(keys, values, table, 3, 100, key=INF, value=-INF)
+    plant(keys, values, table, 3, 300, key=NAN)
+    plant(keys, values, table, 4, 100, key=3.4028234e38)
+    q = torch.randn(tokens, heads * dim, device=DEV, generator=gen)
+    q[tokens - 10, 2], q[tokens - 5, 1], q[tokens - 20] = INF, NAN, q[tokens - 20] * 1e-30
+    common = dict(num_heads=heads, num_kv_heads=kv_heads, head_dim=dim, v_dim=vdim, scale=dim ** -0.5, maps=maps,
+                  **options(form, heads, tokens, gen))
+    pos = np.concatenate([s + np.arange(n) for s, n in zip(starts, lengths)])
+    want, got = (torch.full((tokens, heads * vdim), NAN, device=DEV) for _ in range(2))
+    ops().attention_generic(q, keys, values, table, i32(pos), i32(np.repeat(np.arange(5), lengths)), want, **common)
+    attention_on_tcgen05(q, keys, values, table, starts, lengths, got, **common)
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got.isinf(), want.isinf()) and torch.equal(got[got.isinf()], want[want.isinf()])
+    for row in range(5):                                  # a sequence at a time: their values are of very different sizes
+        mine = slice(sum(lengths[:row]), sum(lengths[:row + 1]))
+        fine = want[mine].isfinite()
+        if fine.any():
+            check(got[mine][fine], want[mine][fine], 330)
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim", [(8, 8, 64), (12, 2, 128)])
+@pytest.mark.parametrize("spread", [1.0, 6.0])
+def test_attention_on_tcgen05_is_as_near_to_64_bits_as_the_general_kernel(heads, kv_heads, dim, spread):
+    """Against a softmax in 64 bits, with scores of a few units and of dozens: no further off than the tiles on mma.sync, or than the general
+    kernel by a fifth."""
+    starts, lengths = [0, 130, 1500], [300, 129, 100]
+    keys, values, table, gen = paged(starts, lengths, kv_heads, kv_heads, dim, dim, 11)
+    tokens = sum(lengths)
+    q = torch.randn(tokens, heads * dim, device=DEV, generator=gen) * spread
+    pos = np.concatenate([s + np.arange(n) for s, n in zip(starts, lengths)])
+    slots, common = np.repeat(np.arange(3), lengths), dict(num_heads=heads, num_kv_heads=kv_heads, head_dim=dim, scale=dim ** -0.5, window=None)
+    exact = torch.empty(tokens, heads, dim, dtype=torch.float64, device=DEV)
+    for row in range(3):
+        held, mine = starts[row] + lengths[row], slice(*(int(c) for c in np.searchsorted(slots, [row, row + 1])))
+        pages = table[row, :(held + 63) // 64].long()
+        k = keys[pages].double().permute(1, 0, 2, 3).reshape(kv_heads, -1, dim)[:, :held].repeat_interleave(heads // kv_heads, 0)
+        v = values[pages].double().permute(1, 0, 3, 2).reshape(kv_heads, -1, dim)[:, :held].repeat_interleave(heads // kv_heads, 0)
+        scores = q[mine].double().view(-1, heads, dim).transpose(0, 1) @ k.transpose(1, 2) * dim ** -0.5
+        hidden = torch.arange(held, device=DEV)[None] > torch.as_tensor(pos[mine], device=DEV)[:, None]
+        exact[mine] = (scores.masked_fill(hidden, -INF).softmax(-1) @ v).transpose(0, 1)
+    exact = exact.view(tokens, heads * dim)
+    general, tiles, got = (torch.full((tokens, heads * dim), NAN, device=DEV) for _ in range(3))
+    ops().attention_generic(q, keys, values, table, i32(pos), i32(slots), general, **common)
+    cut = [(b, q0) for b, n in enumerate(lengths) for q0 in range(0, n, 128)]
+    ops().attention_f32_tiles(q, keys, values, table, i32([t[0] for t in cut]), i32([t[1] for t in cut]), i32(range(3)), i32(starts), i32(lengths),
+                              i32(np.concatenate([[0], np.cumsum(lengths)])), tiles, **common)
+    attention_on_tcgen05(q, keys, values, table, starts, lengths, got, **common)
+    errors = [relative(t, exact) for t in (general, tiles, got)]
+    print("errors: general %.2e, tiles on mma.sync %.2e, tcgen05 %.2e" % tuple(errors))
+    assert errors[2] < max(errors[1], 1.2 * errors[0])
