@@ -153,19 +153,6 @@ __device__ __forceinline__ void copy_bulk(void* dst, const void* src, uint32_t b
                  ::"r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(bar)) : "memory");
 }
 
-// `sums` = the products of an operand in tensor memory (its parts at a_hi and a_lo) with one in shared memory, KSTEPS runs of sixteen
-// entries; b_at(k): the place of run k from the second operand's start, in units of 16 bytes.  One lane.
-template <int KSTEPS, typename At>
-__device__ __forceinline__ void products_of_parts(uint32_t sums, uint32_t a_hi, uint32_t a_lo, uint64_t b_hi, uint64_t b_lo, uint32_t idesc, At b_at) {
-#pragma unroll
-    for (int k = 0; k < KSTEPS; ++k) mma_ts(sums, a_lo + 8 * k, b_hi + b_at(k), idesc, k != 0);
-#pragma unroll
-    for (int k = 0; k < KSTEPS; ++k) mma_ts(sums, a_hi + 8 * k, b_lo + b_at(k), idesc, 1);
-    mma_ts_scaled<11>(sums, a_hi, b_hi, idesc);
-#pragma unroll
-    for (int k = 1; k < KSTEPS; ++k) mma_ts(sums, a_hi + 8 * k, b_hi + b_at(k), idesc, 1);
-}
-
 // grid (head, tile of 128 queries).  MODIFIED: capped scores or slopes.
 template <int HD, int VD, bool MODIFIED>
 __global__ void __launch_bounds__(FT_THREADS, 1)

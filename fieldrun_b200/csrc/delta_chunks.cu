@@ -6,21 +6,23 @@
 // With S the state at a chunk's start and w(j, i) the product of the decays of its tokens j + 1 .. i (w(i): from the chunk's start):
 //     (I + M) u = beta v - beta w k^T S,   M_ij = beta_i w(j, i) (k_i . k_j) for j < i,
 //     o_i = w(i) S^T q_i + sum_(j <= i) w(j, i) (q_i . k_j) u_j,   S <- w(end) S + sum_j w(j, end) k_j u_j^T.
-//   1. every chunk and head side by side: M and the pairs' weights for o; then (I + M) X = [beta w k | beta v] by substitution, a
-//      thread a column, in float32: W and U' with u = U' - W S.  (The entries of (I + M)^(-1) are at most one: each is what is left
-//      of a unit of v_j under steps that shorten, times beta k_i.)
-//   2. along the chunks of a sequence, a block a (sequence, head, 64 value columns) that keeps the state in registers: u = U' - W S,
-//      o, and the new state.
-//   3. the head's root mean square, weight and gate.
+//   1. every chunk and key head side by side: the products of the unit keys with one another and with the unit queries;
+//   2. every chunk and head side by side: the weights, M and the pairs' weights for o; then (I + M) X = [beta w k | beta v] by
+//      substitution, a thread a column, in float32: W and U' with u = U' - W S.  (The entries of (I + M)^(-1) are at most one: each is
+//      what is left of a unit of v_j under steps that shorten, times beta k_i.)
+//   3. along the chunks of a sequence, a block that keeps the state in registers: u = U' - W S, o, and the new state.  Heads of 128 value
+//      columns: on tcgen05, a block a (sequence, head); of 64: on mma.sync.
+//   4. the head's root mean square, weight and gate.
 // A weight is the exponential of a sum of logarithms that has its tokens' alone, or a product of such factors: never a quotient, and no
 // difference of two sums either, which behind one strong decay would have lost the digits of the mild ones.  The sums run over up to 16
 // tokens inside a block and up to 48 between blocks: a rounding of their logarithms, which are large only where the weight is small.
 //
-// Everything is float32; the products run on tensor cores with each operand as two TF32 parts (tf32_parts.cuh), over inner sizes of
-// at most 128 entries, added in float32 registers every 16; so is a chunk's new state to the decayed old one.  Four prompts of 2,048
-// tokens, 16 heads of 128 x 128 over 4 key heads: 0.59 ms (0.19 + 0.36 + 0.04 for the launches in turn; delta_rule.cu token by
-// token 1.38 ms).  Launch 1 issues on 57 % of the cycles (with the values' loads each waited for in turn: 0.37 ms).  Launch 2 is bound
-// by the tensor cores and by the barriers of its three phases: a chunk takes 11.7 us where its products alone take 5.
+// Everything is float32; the products run on tensor cores with each operand as two parts (tf32_parts.cuh: sums of 16 entries, added in
+// float32 registers; f16_parts.cuh: of at most 128).  Four prompts of 2,048 tokens, 16 heads of 128 x 128 over 4 key heads: 340 us (34 +
+// 151 + 118 + 34 for the launches in turn; delta_rule.cu token by token 1,387).  With launch 1's products made by launch 2 for every head, and
+// launch 3 on mma.sync, 589 (189 + 368 + 34).  Launch 2 is bound by the instructions of its substitution, two entries each (one
+// each: 168 us), and by the latencies before it, two blocks an SM; launch 3 by the chain of its phases.
+#include "f16_parts.cuh"
 #include "tf32_parts.cuh"
 
 #define DC_TOKENS 64
@@ -28,6 +30,10 @@
 #define DC_BLOCKS (DC_TOKENS / DC_BLOCK)
 #define DC_SLICE 64           // value columns a block of launch 2 keeps
 #define DC_LM (DC_TOKENS + 8)
+#define DC_FACTORS (3 * DC_TOKENS + 4)
+#define DC_W_SCALE 8          // exponents of the parts' scales
+#define DC_Q_SCALE 17
+#define DC_K_SCALE 14
 
 struct DeltaChunks {
     const float* conv;       // [T, conv_stride]: q at q_off (kv_heads * dim), k at k_off, v at v_off (heads * vdim)
@@ -44,6 +50,13 @@ struct DeltaChunks {
     float* q_factor;         // [chunks][heads][DC_TOKENS]: w(i) and the query's norm
     float* k_factor;         // [chunks][heads][DC_TOKENS]: w(j, end) and the key's norm
     float* decays;           // [chunks][heads]: w(end)
+    // for the chain on tcgen05, in place of w and pairs: their parts, and the unit keys' and queries'
+    uint16_t* w_parts;       // [chunks][heads][part][dim / 64][DC_TOKENS][64], the row times 2^8 / (a power of two about w(i))
+    uint16_t* pair_parts;    // [chunks][heads][part][DC_TOKENS][DC_TOKENS], times 2^17
+    uint16_t *q_parts, *k_parts;     // [chunks][kv_heads][part][dim / 64][DC_TOKENS][64], times 2^17 and 2^14
+    float* raw_pairs;        // [chunks][kv_heads][2][DC_TOKENS][DC_TOKENS]: the unit keys' products [j][i], the queries' with them [i][j], j <= i
+    float* norms;            // [chunks][kv_heads][2][DC_TOKENS]: what makes the queries (with dim^(-1/2)) and keys unit vectors
+    float* factors;          // [chunks][heads][DC_FACTORS]: what takes w's scale off; w(i) 2^-17; w(j, end); w(end)
     int conv_stride, q_off, k_off, v_off, proj_stride, b_off, a_off, g_off, heads, kv_heads;
     float eps;
 };
@@ -61,44 +74,31 @@ __device__ __forceinline__ void dc_copy_rows(float* to, int ld, const float* fro
     }
 }
 
-// Launch 1.  grid (chunk, head).
-template <int DIM, int VDIM>
-__global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p) {
-    constexpr int LQ = DIM + 8, LS = DC_TOKENS + 4;
+__device__ __forceinline__ float dc_power(int exponent) { return __uint_as_float((uint32_t)(exponent + 127) << 23); }
+
+// The place of entry `c` (even) of row `r` in pieces [64 rows][64 entries] of rows of 128 bytes, 128-byte swizzle, in float16 entries.
+__device__ __forceinline__ int dc_place(int r, int c) { return (c >> 6) * (DC_TOKENS * 64) + r * 64 + (((c >> 3 & 7) ^ (r & 7)) << 3) + (c & 7); }
+
+// The exponent that brings entries of W's row i, at most 2^6 w(i), below 2^14.
+__device__ __forceinline__ int dc_w_exponent(float start) { return DC_W_SCALE - max(ilogbf(fmaxf(start, 1e-30f)), -100); }
+
+// Launch 1.  grid (chunk, key head): the products of the unit keys with one another and with the unit queries, once for all heads over
+// them.  PARTS: also those rows as float16 parts, for the chain on tcgen05.
+template <int DIM, bool PARTS>
+__global__ void __launch_bounds__(256, 2) delta_chunk_pairs_kernel(DeltaChunks p) {
+    constexpr int LQ = DIM + 8;
     extern __shared__ float4 dc_smem[];
-    __shared__ float beta_s[DC_TOKENS], log_s[DC_TOKENS], to_s[DC_TOKENS], from_s[DC_TOKENS], start_s[DC_TOKENS], q_inv[DC_TOKENS], k_inv[DC_TOKENS];
-    __shared__ float block_log[DC_BLOCKS], between[DC_BLOCKS][DC_BLOCKS];
-    __shared__ __align__(16) float own[DC_TOKENS][DC_BLOCK + 4];         // w(j, i) of the tokens j of i's block; zero for later ones
+    __shared__ float q_inv[DC_TOKENS], k_inv[DC_TOKENS];
     float* q_s = (float*)dc_smem;                   // [DC_TOKENS][LQ]
     float* k_s = q_s + DC_TOKENS * LQ;              // [DC_TOKENS][LQ]
-    float* m_s = k_s + DC_TOKENS * LQ;              // [DC_TOKENS][LS]: M, column by column
-    const int item = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int b = p.chunk_seq[item], count = p.chunk_end[item] - p.chunk_begin[item], kvh = h / (p.heads / p.kv_heads);
-    const size_t row0 = (size_t)p.cu_q_len[b] + p.chunk_begin[item], at = (size_t)item * p.heads + h;
+    const int item = blockIdx.x, kvh = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    let_next_kernel_start();
+    const int b = p.chunk_seq[item], count = p.chunk_end[item] - p.chunk_begin[item];
+    const size_t row0 = (size_t)p.cu_q_len[b] + p.chunk_begin[item], at = (size_t)item * p.kv_heads + kvh;
     const float* rows = p.conv + row0 * p.conv_stride;
     dc_copy_rows<DIM, 256>(q_s, LQ, rows + p.q_off + kvh * DIM, p.conv_stride, count);
     dc_copy_rows<DIM, 256>(k_s, LQ, rows + p.k_off + kvh * DIM, p.conv_stride, count);
     copies_commit();
-
-    // a token a thread: beta; the logarithms of the decays from its block's start (with its own) and to its block's end
-    if (tid < DC_TOKENS) {
-        const float* logits = p.proj + (row0 + min(tid, count - 1)) * p.proj_stride + h;
-        const bool in = tid < count;
-        beta_s[tid] = in ? 1.0f / (1.0f + expf(-logits[p.b_off])) : 0.f;
-        const float la = in ? -expf(p.a_log[h]) * dc_softplus(logits[p.a_off] + p.dt_bias[h]) : 0.f;
-        float before = la, behind = la;
-#pragma unroll
-        for (int o = 1; o < DC_BLOCK; o <<= 1) {
-            const float up = __shfl_up_sync(0xffffffffu, before, o, DC_BLOCK), down = __shfl_down_sync(0xffffffffu, behind, o, DC_BLOCK);
-            if (tid % DC_BLOCK >= o) before += up;
-            if (tid % DC_BLOCK + o < DC_BLOCK) behind += down;
-        }
-        float tail = __shfl_down_sync(0xffffffffu, behind, 1, DC_BLOCK);
-        if (tid % DC_BLOCK == DC_BLOCK - 1) { tail = 0.f; block_log[tid / DC_BLOCK] = before; }
-        log_s[tid] = la;
-        to_s[tid] = expf(before);
-        from_s[tid] = expf(tail);
-    }
     copies_wait<0>();
     __syncthreads();
     for (int t = warp; t < DC_TOKENS; t += 8) {
@@ -112,40 +112,29 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
         qq = warp_sum(qq);
         kk = warp_sum(kk);
         if (lane == 0) {
-            q_inv[t] = 1.0f / sqrtf((float)DIM) / sqrtf(qq + 1e-6f);
-            k_inv[t] = 1.0f / sqrtf(kk + 1e-6f);
+            const float q = 1.0f / sqrtf((float)DIM) / sqrtf(qq + 1e-6f), k = 1.0f / sqrtf(kk + 1e-6f);
+            q_inv[t] = q;
+            k_inv[t] = k;
+            p.norms[at * 2 * DC_TOKENS + t] = q;
+            p.norms[at * 2 * DC_TOKENS + DC_TOKENS + t] = k;
         }
     }
-    if (tid < DC_BLOCKS * DC_BLOCKS) {               // the whole blocks between two
-        const int i = tid / DC_BLOCKS, j = tid % DC_BLOCKS;
-        float sum = 0.f;
-        for (int m = j + 1; m < i; ++m) sum += block_log[m];
-        between[i][j] = expf(sum);
-    } else if (tid >= 64 && tid < 64 + DC_TOKENS) {  // a token's weights in its block: the sums begin anew for each, at the token itself
-        const int t = tid - 64, i = t % DC_BLOCK;
-        float sum = 0.f, row[DC_BLOCK];
-#pragma unroll
-        for (int j = DC_BLOCK - 1; j >= 0; --j) {
-            row[j] = j <= i ? expf(sum) : 0.f;
-            if (j <= i) sum += log_s[t - i + j];
-        }
-#pragma unroll
-        for (int j = 0; j < DC_BLOCK; j += 4) *(float4*)&own[t][j] = make_float4(row[j], row[j + 1], row[j + 2], row[j + 3]);
-    } else if (tid >= 128 && tid < 128 + DC_TOKENS) {
-        const int t = tid - 128;
-        float sum = 0.f;
-        for (int m = 0; m < t / DC_BLOCK; ++m) sum += block_log[m];
-        start_s[t] = expf(sum) * to_s[t];
-    }
-    // the chunk's factors for launch 2: a token's decays to the chunk's end
-    float rest = 0.f;
-    if (tid < DC_TOKENS)
-        for (int m = tid / DC_BLOCK + 1; m < DC_BLOCKS; ++m) rest += block_log[m];
     __syncthreads();
-    if (tid < DC_TOKENS) {
-        p.q_factor[at * DC_TOKENS + tid] = start_s[tid] * q_inv[tid];
-        p.k_factor[at * DC_TOKENS + tid] = from_s[tid] * expf(rest) * k_inv[tid];
-        if (tid == DC_TOKENS - 1) p.decays[at] = start_s[tid];
+    if (PARTS) {
+        constexpr int UNITS = DC_TOKENS * DIM / 8;
+        const size_t to = at * 2 * DC_TOKENS * DIM;
+        for (int u = tid; u < 2 * UNITS; u += 256) {
+            const bool key = u >= UNITS;
+            const int r = u % UNITS / (DIM / 8), c = u % (DIM / 8) * 8;
+            const float* from = (key ? k_s : q_s) + r * LQ + c;
+            const float scale = (key ? k_inv[r] : q_inv[r]) * dc_power(key ? DC_K_SCALE : DC_Q_SCALE);
+            uint4 hi, lo;
+            split_four(*(const float4*)from, scale, hi.x, hi.y, lo.x, lo.y);
+            split_four(*(const float4*)(from + 4), scale, hi.z, hi.w, lo.z, lo.w);
+            uint16_t* parts = (key ? p.k_parts : p.q_parts) + to + dc_place(r, c);
+            *(uint4*)parts = hi;
+            *(uint4*)(parts + DC_TOKENS * DIM) = lo;
+        }
     }
 
     // warps 0 .. 3 the products of keys with keys, 4 .. 7 of queries with keys: row tiles a and 3 - a, every other eight columns
@@ -174,7 +163,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
                 }
         }
     }
-    float* pairs = p.pairs + at * DC_TOKENS * DC_TOKENS;
+    float* kk = p.raw_pairs + at * 2 * DC_TOKENS * DC_TOKENS;            // [j][i], then q k [i][j]
 #pragma unroll
     for (int m = 0; m < 2; ++m)
 #pragma unroll
@@ -183,50 +172,187 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int i = tiles[m] * DC_BLOCK + (lane >> 2) + 8 * (e >> 1), j = n * DC_BLOCK + 8 * odd + 2 * (lane & 3) + (e & 1);
-                    const bool seen = keys ? j < i : j <= i;
-                    const float w = n < tiles[m] ? to_s[i] * between[tiles[m]][n] * from_s[j] : own[i][j % DC_BLOCK];
-                    if (seen && !is_finite(acc[m][n][e])) acc[m][n][e] = sum_entry_by_entry(left + i * LQ, 1, k_s + j * LQ, 1, nullptr, DIM);
-                    const float value = seen ? acc[m][n][e] * w * k_inv[j] * (keys ? beta_s[i] * k_inv[i] : q_inv[i]) : 0.f;
-                    if (keys) m_s[j * LS + i] = value;
-                    else pairs[i * DC_TOKENS + j] = value;
+                    if (j <= i && !is_finite(acc[m][n][e])) acc[m][n][e] = sum_entry_by_entry(left + i * LQ, 1, k_s + j * LQ, 1, nullptr, DIM);
+                    const float value = acc[m][n][e] * k_inv[j] * (keys ? k_inv[i] : q_inv[i]);
+                    if (keys) kk[j * DC_TOKENS + i] = value;
+                    else kk[DC_TOKENS * DC_TOKENS + i * DC_TOKENS + j] = value;
                 }
+}
+
+// Launch 2.  grid (chunk, head): the weights, M and the pairs' weights for o, and the substitution.  PARTS: what it leaves for launch 3 as
+// float16 parts (the chain on tcgen05).
+template <int DIM, int VDIM, bool PARTS>
+__global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p) {
+    constexpr int LS = DC_TOKENS + 4;
+    __shared__ float beta_s[DC_TOKENS], log_s[DC_TOKENS], to_s[DC_TOKENS], from_s[DC_TOKENS], start_s[DC_TOKENS], q_inv[DC_TOKENS], k_inv[DC_TOKENS], w_scale[DC_TOKENS];
+    __shared__ float block_log[DC_BLOCKS], between[DC_BLOCKS][DC_BLOCKS];
+    __shared__ __align__(16) float own[DC_TOKENS][DC_BLOCK + 4];         // w(j, i) of the tokens j of i's block; zero for later ones
+    __shared__ __align__(16) float m_s[DC_TOKENS * LS];                  // M, column by column
+    const int item = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
+    const int b = p.chunk_seq[item], count = p.chunk_end[item] - p.chunk_begin[item], kvh = h / (p.heads / p.kv_heads);
+    const size_t row0 = (size_t)p.cu_q_len[b] + p.chunk_begin[item], at = (size_t)item * p.heads + h, kv_at = (size_t)item * p.kv_heads + kvh;
+    const float* rows = p.conv + row0 * p.conv_stride;
+
+    // the substitution's right-hand side, a column of [k | v] a thread, on its way meanwhile
+    float x[DC_TOKENS];
+    const bool key = tid < DIM;
+    if (tid < DIM + VDIM) {
+        const float* column = rows + (key ? p.k_off + kvh * DIM + tid : p.v_off + h * VDIM + tid - DIM);
+#pragma unroll
+        for (int i = 0; i < DC_TOKENS; ++i) x[i] = column[(size_t)min(i, count - 1) * p.conv_stride];
+    }
+    // a token a thread: beta; the logarithms of the decays from its block's start (with its own) and to its block's end
+    if (tid < DC_TOKENS) {
+        const float* logits = p.proj + (row0 + min(tid, count - 1)) * p.proj_stride + h;
+        const bool in = tid < count;
+        beta_s[tid] = in ? 1.0f / (1.0f + expf(-logits[p.b_off])) : 0.f;
+        const float la = in ? -expf(p.a_log[h]) * dc_softplus(logits[p.a_off] + p.dt_bias[h]) : 0.f;
+        float before = la, behind = la;
+#pragma unroll
+        for (int o = 1; o < DC_BLOCK; o <<= 1) {
+            const float up = __shfl_up_sync(0xffffffffu, before, o, DC_BLOCK), down = __shfl_down_sync(0xffffffffu, behind, o, DC_BLOCK);
+            if (tid % DC_BLOCK >= o) before += up;
+            if (tid % DC_BLOCK + o < DC_BLOCK) behind += down;
+        }
+        float tail = __shfl_down_sync(0xffffffffu, behind, 1, DC_BLOCK);
+        if (tid % DC_BLOCK == DC_BLOCK - 1) { tail = 0.f; block_log[tid / DC_BLOCK] = before; }
+        log_s[tid] = la;
+        to_s[tid] = expf(before);
+        from_s[tid] = expf(tail);
+    }
+    __syncthreads();
+    if (tid < DC_BLOCKS * DC_BLOCKS) {               // the whole blocks between two
+        const int i = tid / DC_BLOCKS, j = tid % DC_BLOCKS;
+        float sum = 0.f;
+        for (int m = j + 1; m < i; ++m) sum += block_log[m];
+        between[i][j] = expf(sum);
+    } else if (tid >= 64 && tid < 64 + DC_TOKENS) {  // a token's weights in its block: the sums begin anew for each, at the token itself
+        const int t = tid - 64, i = t % DC_BLOCK;
+        float sum = 0.f, row[DC_BLOCK];
+#pragma unroll
+        for (int j = DC_BLOCK - 1; j >= 0; --j) {
+            row[j] = j <= i ? expf(sum) : 0.f;
+            if (j <= i) sum += log_s[t - i + j];
+        }
+#pragma unroll
+        for (int j = 0; j < DC_BLOCK; j += 4) *(float4*)&own[t][j] = make_float4(row[j], row[j + 1], row[j + 2], row[j + 3]);
+    } else if (tid >= 128 && tid < 128 + DC_TOKENS) {
+        const int t = tid - 128;
+        float sum = 0.f;
+        for (int m = 0; m < t / DC_BLOCK; ++m) sum += block_log[m];
+        start_s[t] = expf(sum) * to_s[t];
+    }
+    // the chunk's factors for launch 3: a token's decays to the chunk's end
+    float rest = 0.f;
+    if (tid < DC_TOKENS)
+        for (int m = tid / DC_BLOCK + 1; m < DC_BLOCKS; ++m) rest += block_log[m];
+    after_previous_kernel();                         // launch 1, whose products come from here on; it began when the rows were there
+    if (tid < 2 * DC_TOKENS) (tid < DC_TOKENS ? q_inv : k_inv)[tid % DC_TOKENS] = p.norms[kv_at * 2 * DC_TOKENS + tid];
+    __syncthreads();
+    if (tid < DC_TOKENS) {
+        const float to_end = from_s[tid] * expf(rest);
+        if (PARTS) {
+            float* factors = p.factors + at * DC_FACTORS;
+            const int exponent = dc_w_exponent(start_s[tid]);
+            w_scale[tid] = dc_power(exponent);
+            factors[tid] = dc_power(-exponent);
+            factors[DC_TOKENS + tid] = start_s[tid] * dc_power(-DC_Q_SCALE);
+            factors[2 * DC_TOKENS + tid] = to_end;
+            if (tid == DC_TOKENS - 1) factors[3 * DC_TOKENS] = start_s[tid];
+        } else {
+            p.q_factor[at * DC_TOKENS + tid] = start_s[tid] * q_inv[tid];
+            p.k_factor[at * DC_TOKENS + tid] = to_end * k_inv[tid];
+            if (tid == DC_TOKENS - 1) p.decays[at] = start_s[tid];
+        }
+    }
+
+    // four entries of M's columns at a time, then eight of the pairs' rows
+    const float* kk = p.raw_pairs + kv_at * 2 * DC_TOKENS * DC_TOKENS;
+    auto weight = [&](int i, int j) {
+        const int ib = i / DC_BLOCK, jb = j / DC_BLOCK;
+        return jb < ib ? to_s[i] * between[ib][jb] * from_s[j] : own[i][j % DC_BLOCK];
+    };
+#pragma unroll
+    for (int u = tid; u < DC_TOKENS * DC_TOKENS / 4; u += 256) {
+        const int j = u / (DC_TOKENS / 4), i0 = u % (DC_TOKENS / 4) * 4;
+        float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i0 + 3 > j) {
+            const float4 raw = *(const float4*)(kk + j * DC_TOKENS + i0);
+            const float r[4] = {raw.x, raw.y, raw.z, raw.w};
+            float* to = (float*)&m;
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (i0 + e > j) to[e] = r[e] * weight(i0 + e, j) * beta_s[i0 + e];
+        }
+        *(float4*)(m_s + j * LS + i0) = m;
+    }
+    for (int u = tid; u < DC_TOKENS * DC_TOKENS / 8; u += 256) {
+        const int i = u / (DC_TOKENS / 8), j0 = u % (DC_TOKENS / 8) * 8;
+        float y[8] = {};
+        if (j0 <= i) {
+            const float* from = kk + DC_TOKENS * DC_TOKENS + i * DC_TOKENS + j0;
+            const float4 a = *(const float4*)from, c = *(const float4*)(from + 4);
+            const float r[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                if (j0 + e <= i) y[e] = r[e] * weight(i, j0 + e);
+        }
+        if (PARTS) {
+            uint4 hi, lo;
+            split_four(make_float4(y[0], y[1], y[2], y[3]), dc_power(DC_Q_SCALE), hi.x, hi.y, lo.x, lo.y);
+            split_four(make_float4(y[4], y[5], y[6], y[7]), dc_power(DC_Q_SCALE), hi.z, hi.w, lo.z, lo.w);
+            uint16_t* to = p.pair_parts + at * 2 * DC_TOKENS * DC_TOKENS + dc_place(i, j0);
+            *(uint4*)to = hi;
+            *(uint4*)(to + DC_TOKENS * DC_TOKENS) = lo;
+        } else {
+            float4* to = (float4*)(p.pairs + at * DC_TOKENS * DC_TOKENS + i * DC_TOKENS + j0);
+            to[0] = make_float4(y[0], y[1], y[2], y[3]);
+            to[1] = make_float4(y[4], y[5], y[6], y[7]);
+        }
+    }
     __syncthreads();
 
     // substitution: a thread a column of [beta w k | beta v], its 64 entries in registers
     if (tid < DIM + VDIM) {
-        const bool key = tid < DIM;
-        const float* v = rows + p.v_off + h * VDIM + tid - DIM;
-        float x[DC_TOKENS];
         if (key) {
 #pragma unroll
-            for (int i = 0; i < DC_TOKENS; ++i) x[i] = beta_s[i] * start_s[i] * k_inv[i] * k_s[i * LQ + tid];
-        } else {                                     // all of the column's loads on their way before the first is used
-#pragma unroll
-            for (int i = 0; i < DC_TOKENS; ++i) x[i] = v[(size_t)min(i, count - 1) * p.conv_stride];
+            for (int i = 0; i < DC_TOKENS; ++i) x[i] = i < count ? beta_s[i] * start_s[i] * k_inv[i] * x[i] : 0.f;
+        } else {
 #pragma unroll
             for (int i = 0; i < DC_TOKENS; ++i) x[i] = i < count ? x[i] * beta_s[i] : 0.f;
         }
         float* to = key ? p.w + at * DC_TOKENS * DIM + tid : p.u + at * DC_TOKENS * VDIM + tid - DIM;
+        uint16_t* w_parts = p.w_parts + at * 2 * DC_TOKENS * DIM;
         const int width = key ? DIM : VDIM;
         // an entry once it is final leaves every later one: those do not depend on one another
 #pragma unroll
         for (int i = 0; i < DC_TOKENS; ++i) {
             const float* m = m_s + i * LS;
             const float done = x[i];
-            to[(size_t)i * width] = done;
+            if (!PARTS || !key) to[(size_t)i * width] = done;
+            else if (i & 1) {                        // two columns' entries of two rows: a lane of the two has one row's
+                const bool odd_column = tid & 1;
+                const float theirs = __shfl_xor_sync(0xffffffffu, odd_column ? x[i - 1] : done, 1);
+                const int r = odd_column ? i : i - 1;
+                const float scale = w_scale[r];
+                uint32_t hi, lo;
+                split_two(mul_pairs(odd_column ? pair_of(theirs, done) : pair_of(x[i - 1], theirs), pair_of(scale, scale)), hi, lo);
+                uint16_t* parts = w_parts + dc_place(r, tid & ~1);
+                *(uint32_t*)parts = hi;
+                *(uint32_t*)(parts + DC_TOKENS * DIM) = lo;
+            }
+            const uint64_t leaves = pair_of(-done, -done);
 #pragma unroll
-            for (int j = (i + 1) & ~3; j < DC_TOKENS; j += 4) {
-                const float4 w = *(const float4*)(m + j);
-                if (j > i) x[j] = fmaf(-w.x, done, x[j]);
-                if (j + 1 > i) x[j + 1] = fmaf(-w.y, done, x[j + 1]);
-                if (j + 2 > i) x[j + 2] = fmaf(-w.z, done, x[j + 2]);
-                if (j + 3 > i) x[j + 3] = fmaf(-w.w, done, x[j + 3]);
+            for (int j = (i + 1) & ~3; j < DC_TOKENS; j += 4) {      // two entries at a time; M is zero up to its diagonal
+                const ulonglong2 w = *(const ulonglong2*)(m + j);
+                if (j + 1 > i) halves_of(fma_pairs(w.x, leaves, pair_of(x[j], x[j + 1])), x[j], x[j + 1]);
+                halves_of(fma_pairs(w.y, leaves, pair_of(x[j + 2], x[j + 3])), x[j + 2], x[j + 3]);
             }
         }
     }
 }
 
-// Launch 2.  grid (sequence, head, slice of 64 value columns), 16 warps.  W and the queries are free once u is there, the pairs' weights
+// Launch 3.  grid (sequence, head, slice of 64 value columns), 16 warps.  W and the queries are free once u is there, the pairs' weights
 // and the keys once the new state is: each time the next chunk's are asked for.
 template <int DIM>
 __global__ void __launch_bounds__(512, 1) delta_chunk_chain_kernel(DeltaChunks p, int vdim) {
@@ -261,6 +387,7 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_chain_kernel(DeltaChunks p
         if (tid < DC_TOKENS / 4) copy16_async(k_factor[item & 1] + 4 * tid, p.k_factor + at * DC_TOKENS + 4 * tid);
         copies_commit();
     };
+    after_previous_kernel();
     if (first < last) {
         copy_first(first);
         copy_second(first);
@@ -421,10 +548,388 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_chain_kernel(DeltaChunks p
         }
 }
 
-// Launch 3.  A warp a (token, head): bound by reading o and the gate once.
+// Launch 3 on tcgen05, for heads of 128 value columns.  grid (sequence, head): a block keeps the head's state, transposed: a lane of tensor
+// memory is a value column, and two threads have half of its DIM entries each, in float32.  With every operand as two float16 parts (the
+// small products first, 2^11 times too large, taken down by the first large one), for every chunk
+//     D1 = S^T [W; Q]^T        128 x 64 x DIM, W first: the state's parts in tensor memory, W's and the queries' rows in shared memory;
+//     u^T = U'^T - D1          two threads a column, 32 tokens each; its parts, and those of u w(j, end), go to tensor memory;
+//     DS = (u w(j, end))^T K   128 x DIM x 64, the keys N-major;   DO = u^T pairs^T   128 x 64 x 64;
+//     S <- w(end) S + DS^T, o = w(i) D1 + DO in float32 registers.
+// The columns' parts have a power of two of their own each, from the largest entry of the state or of u.  What bounds it: the chain of a
+// chunk's phases, 6,300 cycles (11.5 us on mma.sync): the first product 1,150, the third 1,250, the state's split 1,250, u and its two
+// splits 2,000, the new state 560; the SMs that have a sequence's head, 64 of them for four prompts in sixteen heads, issue an
+// instruction on nearly every cycle of the splits.  A column with a number that is not finite, or with a token 2^28 times larger than the first of its chunk, makes the block
+// take the sequence's head again, token by token.
+#define DT_SHARES 2            // threads a column: each half of its entries and of a chunk's tokens (four: 127 us instead of 118)
+#define DT_WARPS (4 * DT_SHARES)
+#define DT_ROWS (32 * DT_WARPS)
+#define DT_THREADS (DT_ROWS + 96)        // the columns' warps (w & 3: lanes; w >> 2: share), then one each for copies, products, outputs
+#define DT_TOKENS (DC_TOKENS / DT_SHARES)
+
+using namespace frb_tma;
+using namespace frb_tc;
+
+__device__ __forceinline__ void dt_copy(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(bar)) : "memory");
+}
+
+// An N-major operand of pieces [64 of the inner size][64 entries] (rows of 128 bytes, 128-byte swizzle), a piece DC_TOKENS * 128 bytes.
+__device__ __forceinline__ uint64_t dt_desc_n_major(uint32_t addr) {
+    return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)(DC_TOKENS * 128 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
+           ((uint64_t)2 << 61);
+}
+
+// N entries of a column times its scale, as parts, to N / 2 columns of tensor memory each.
+template <int N>
+__device__ __forceinline__ void dt_store_parts(const float (&x)[N], float scale, uint32_t to_hi, uint32_t to_lo) {
+    static_assert(N % 32 == 0, "entries of a store");
+#pragma unroll
+    for (int n = 0; n < N; n += 32) {
+        uint32_t hi[16], lo[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) split_two(mul_pairs(pair_of(x[n + 2 * i], x[n + 2 * i + 1]), pair_of(scale, scale)), hi[i], lo[i]);
+        tmem_st16(to_hi + n / 2, hi);
+        tmem_st16(to_lo + n / 2, lo);
+    }
+}
+
+// N columns of tensor memory, there after tmem_wait_ld().
+template <int N>
+__device__ __forceinline__ void dt_load(uint32_t from, uint32_t (&v)[N / 16][16]) {
+#pragma unroll
+    for (int i = 0; i < N / 16; ++i) tmem_ld16(from + 16 * i, v[i]);
+}
+
+// A sequence's head token by token (delta_rule.cu's formula): 128 threads of a block, one a value column; `rows_s`: 2 DIM + 3 floats.
+template <int DIM>
+static __device__ __noinline__ void dt_token_by_token(const DeltaChunks& p, int b, int h, float* rows_s) {
+    constexpr int VDIM = 128;
+    float *q_s = rows_s, *k_s = rows_s + DIM, *norms = rows_s + 2 * DIM;
+    const int tid = threadIdx.x, kvh = h / (p.heads / p.kv_heads);
+    const int start = p.seq_start[b], n_tok = p.cu_q_len[b + 1] - p.cu_q_len[b];
+    float* kept = p.state + (size_t)p.seq_slot[b] * 2 * p.copy_floats + p.state_offset + (size_t)h * DIM * VDIM + tid;
+    auto meet = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };
+    float S[DIM];
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) S[d] = (kept + (start & 1) * p.copy_floats)[(size_t)d * VDIM];
+    for (int t = 0; t < n_tok; ++t) {
+        const size_t row = (size_t)p.cu_q_len[b] + t;
+        const float* rows = p.conv + row * p.conv_stride;
+        const float* logits = p.proj + row * p.proj_stride + h;
+        meet();
+        if (tid < DIM) {
+            q_s[tid] = rows[p.q_off + kvh * DIM + tid];
+            k_s[tid] = rows[p.k_off + kvh * DIM + tid];
+        }
+        meet();
+        if (tid < 96) {                              // a warp the query's norm, one the key's, one their product
+            const float *x = tid < 32 ? q_s : k_s, *y = tid < 64 ? x : q_s;
+            float ss = 0.f;
+            for (int d = tid & 31; d < DIM; d += 32) ss = fmaf(x[d], y[d], ss);
+            ss = warp_sum(ss);
+            if ((tid & 31) == 0) norms[tid >> 5] = tid >= 64 ? ss : (tid < 32 ? 1.0f / sqrtf((float)DIM) : 1.0f) / sqrtf(ss + 1e-6f);
+        }
+        meet();
+        const float beta = 1.0f / (1.0f + expf(-logits[p.b_off]));
+        const float decay = expf(-expf(p.a_log[h]) * dc_softplus(logits[p.a_off] + p.dt_bias[h]));
+        float seen = 0.f, o = 0.f;
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+            S[d] *= decay;
+            seen = fmaf(S[d], k_s[d] * norms[1], seen);
+            o = fmaf(S[d], q_s[d] * norms[0], o);
+        }
+        const float u = beta * (rows[p.v_off + h * VDIM + tid] - seen);
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) S[d] = fmaf(k_s[d] * norms[1], u, S[d]);
+        p.raw[(row * p.heads + h) * VDIM + tid] = fmaf(u, norms[2] * norms[0] * norms[1], o);
+    }
+    float* to = kept + ((start + n_tok) & 1) * p.copy_floats;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) to[(size_t)d * VDIM] = S[d];
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(DeltaChunks p, int* __restrict__ status) {
+    constexpr int VDIM = 128, SHARE = DIM / DT_SHARES;
+    constexpr uint32_t ROWS_PART = DC_TOKENS * DIM * 2, PAIR_PART = DC_TOKENS * DC_TOKENS * 2;       // bytes of one part
+    // tensor memory: the state's parts; D1 of W, later u's parts; D1 of Q; the parts of u w(j, end); DO; DS
+    constexpr int S_HI = 0, S_LO = DIM / 2, D1_W = 128, D1_Q = 192, UK = 256, D_O = 320, D_S = 384;
+    extern __shared__ uint8_t dt_smem[];
+    __shared__ uint64_t w_full, q_full, k_full, pairs_full, u_full, s_ready, u_ready, d1w_done, d1q_done, ds_done, do_done, o_stored, o_free;
+    __shared__ float tops[4][DT_SHARES][VDIM];
+    __shared__ __align__(16) float factors[2][DC_FACTORS];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int failed_flag, odd_numbers;
+    volatile int* failed = &failed_flag;
+    uint8_t* w_s = (uint8_t*)(((uintptr_t)dt_smem + 1023) & ~(uintptr_t)1023);
+    uint8_t* q_s = w_s + 2 * ROWS_PART;
+    uint8_t* k_s = q_s + 2 * ROWS_PART;
+    uint8_t* pairs_s = k_s + 2 * ROWS_PART;
+    float* u_s = (float*)(pairs_s + 2 * PAIR_PART);                      // [DC_TOKENS][VDIM]: U'
+    float* o_s = u_s + DC_TOKENS * VDIM;                                 // the same of the outputs
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int b = blockIdx.x, h = blockIdx.y, kvh = h / (p.heads / p.kv_heads);
+    const int first = p.seq_chunk0[b], last = __shfl_sync(0xffffffffu, p.seq_chunk0[b + 1], 0), start = p.seq_start[b];
+    const int n_tok = p.cu_q_len[b + 1] - p.cu_q_len[b], chunks = __shfl_sync(0xffffffffu, last - first, 0);
+    const size_t seq_row0 = p.cu_q_len[b];
+
+    if (threadIdx.x == 0) {
+        bar_init(&w_full, 1); bar_init(&q_full, 1); bar_init(&k_full, 1); bar_init(&pairs_full, 1);
+        bar_init(&u_full, 1); bar_init(&o_stored, DT_ROWS / 32); bar_init(&o_free, 1);
+        bar_init(&s_ready, DT_ROWS / 32); bar_init(&u_ready, DT_ROWS / 32);
+        bar_init(&d1w_done, 1); bar_init(&d1q_done, 1); bar_init(&ds_done, 1); bar_init(&do_done, 1);
+        failed_flag = 0;
+        odd_numbers = 0;
+        bar_init_fence();
+    }
+    if (warp == DT_WARPS + 1) tmem_alloc(&tmem_slot, 512);
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
+    after_previous_kernel();                         // barriers and tensor memory were set up while it still ran
+
+    if (warp == DT_WARPS) {
+        if (lane == 0) {
+            for (int c = 0; c < chunks; ++c) {
+                const size_t at = (size_t)(first + c) * p.heads + h, kv_at = (size_t)(first + c) * p.kv_heads + kvh;
+                const uint32_t before = (c & 1) ^ 1;                     // of the phase that the chunk before has ended
+                if (c && !bar_wait(&d1w_done, before, failed)) { atomicExch(status, 61); break; }
+                bar_expect(&w_full, 2 * ROWS_PART + DC_FACTORS * 4);
+                dt_copy(w_s, p.w_parts + at * 2 * DC_TOKENS * DIM, 2 * ROWS_PART, &w_full);
+                dt_copy(factors[c & 1], p.factors + at * DC_FACTORS, DC_FACTORS * 4, &w_full);
+                if (c && !bar_wait(&u_ready, before, failed)) { atomicExch(status, 73); break; }
+                bar_expect(&u_full, DC_TOKENS * VDIM * 4);
+                dt_copy(u_s, p.u + at * DC_TOKENS * VDIM, DC_TOKENS * VDIM * 4, &u_full);
+                if (c && !bar_wait(&d1q_done, before, failed)) { atomicExch(status, 62); break; }
+                bar_expect(&q_full, 2 * ROWS_PART);
+                dt_copy(q_s, p.q_parts + kv_at * 2 * DC_TOKENS * DIM, 2 * ROWS_PART, &q_full);
+                if (c && !bar_wait(&ds_done, before, failed)) { atomicExch(status, 63); break; }
+                bar_expect(&k_full, 2 * ROWS_PART);
+                dt_copy(k_s, p.k_parts + kv_at * 2 * DC_TOKENS * DIM, 2 * ROWS_PART, &k_full);
+                if (c && !bar_wait(&do_done, before, failed)) { atomicExch(status, 64); break; }
+                bar_expect(&pairs_full, 2 * PAIR_PART);
+                dt_copy(pairs_s, p.pair_parts + at * 2 * DC_TOKENS * DC_TOKENS, 2 * PAIR_PART, &pairs_full);
+            }
+        }
+    } else if (warp == DT_WARPS + 1) {
+        // the whole warp goes through the loop (elect_one, tcgen05.cuh); its products run in the order of their issue
+        constexpr uint32_t idesc64 = (1u << 4) | ((uint32_t)(64 >> 3) << 17) | ((uint32_t)(VDIM >> 4) << 24);
+        constexpr uint32_t idesc_k = (1u << 4) | (1u << 16) | ((uint32_t)(DIM >> 3) << 17) | ((uint32_t)(VDIM >> 4) << 24);
+        const uint64_t w_at = tile_desc(smem_addr(w_s)), q_at = tile_desc(smem_addr(q_s)), pairs_at = tile_desc(smem_addr(pairs_s));
+        const uint64_t k_at = dt_desc_n_major(smem_addr(k_s));
+        auto along = [](int k) { return (k / 4) * (DC_TOKENS * 128 >> 4) + (k % 4) * 2; };
+        auto down = [](int k) { return k * (16 * 128 >> 4); };
+        for (int c = 0; c < chunks; ++c) {
+            const uint32_t phase = c & 1;
+            if (!warp_wait_both(&w_full, phase, &s_ready, phase, failed)) { if (lane == 0) atomicExch(status, 65); break; }
+            fence_after_sync();
+            if (elect_one()) {
+                products_of_parts<DIM / 16>(tmem + D1_W, tmem + S_HI, tmem + S_LO, w_at, w_at + (ROWS_PART >> 4), idesc64, along);
+                mma_commit(&d1w_done);
+            }
+            __syncwarp();
+            if (!warp_wait(&q_full, phase, failed)) { if (lane == 0) atomicExch(status, 66); break; }
+            fence_after_sync();
+            if (elect_one()) {
+                products_of_parts<DIM / 16>(tmem + D1_Q, tmem + S_HI, tmem + S_LO, q_at, q_at + (ROWS_PART >> 4), idesc64, along);
+                mma_commit(&d1q_done);
+            }
+            __syncwarp();
+            if (!warp_wait_both(&k_full, phase, &u_ready, phase, failed)) { if (lane == 0) atomicExch(status, 67); break; }
+            fence_after_sync();
+            if (elect_one()) {
+                products_of_parts<DC_TOKENS / 16>(tmem + D_S, tmem + UK, tmem + UK + 32, k_at, k_at + (ROWS_PART >> 4), idesc_k, down);
+                mma_commit(&ds_done);
+            }
+            __syncwarp();
+            if (!warp_wait(&pairs_full, phase, failed)) { if (lane == 0) atomicExch(status, 68); break; }
+            fence_after_sync();
+            if (elect_one()) {
+                products_of_parts<DC_TOKENS / 16>(tmem + D_O, tmem + D1_W, tmem + D1_W + 32, pairs_at, pairs_at + (PAIR_PART >> 4), idesc64,
+                                                  [](int k) { return k * 2; });
+                mma_commit(&do_done);
+            }
+            __syncwarp();
+        }
+    } else if (warp == DT_WARPS + 2) {
+        for (int c = 0; c < chunks; ++c) {           // a chunk's outputs, a token's 512 bytes a copy
+            if (!warp_wait(&o_stored, c & 1, failed)) { if (lane == 0) atomicExch(status, 74); break; }
+            const int begin = p.chunk_begin[first + c], count = p.chunk_end[first + c] - begin;
+            for (int t = lane; t < count; t += 32)
+                asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+                             ::"l"(p.raw + ((seq_row0 + begin + t) * p.heads + h) * VDIM), "r"(smem_addr(o_s + t * VDIM)), "r"(VDIM * 4) : "memory");
+            asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group.read 0;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) bar_arrive(&o_free);
+        }
+        asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    } else {
+        // A wait that gives up does not end the loop: the block's later waits then return at once, and every thread reaches the barriers.
+        const int share = warp >> 2, quarter = warp & 3, column = quarter * 32 + lane, t0 = DT_TOKENS * share;
+        const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16);
+        float* kept = p.state + (size_t)p.seq_slot[b] * 2 * p.copy_floats + p.state_offset + (size_t)h * DIM * VDIM + (size_t)share * SHARE * VDIM + column;
+        bool ok = true;
+        auto wait = [&](uint64_t* bar, uint32_t phase, int code) {
+            if (!bar_wait(bar, phase, failed)) { if (ok && lane == 0) atomicExch(status, code); ok = false; }
+            __syncwarp();
+            fence_after_sync();
+        };
+        auto meet = [] { asm volatile("bar.sync 1, %0;" ::"n"(DT_ROWS) : "memory"); };
+        auto largest = [&](int slot) {               // of what the column's threads have put there
+            float top = tops[slot][0][column];
+#pragma unroll
+            for (int i = 1; i < DT_SHARES; ++i) top = fmaxf(top, tops[slot][i][column]);
+            return top;
+        };
+        auto scale_exponent = [](float top) { return 14 - ilogbf(fminf(fmaxf(top, 7.888609052210118e-31f), 3.402823466e38f)); };     // from 2^-100
+        float S[SHARE], o[DT_TOKENS];
+        uint64_t finite = 0ull;                      // becomes NaNs at the first number that is not finite
+#pragma unroll
+        for (int d = 0; d < SHARE; ++d) S[d] = (kept + (start & 1) * p.copy_floats)[(size_t)d * VDIM];
+        float u_inv = 0.f;
+        auto write_outputs = [&](int c) {            // what u gives the outputs of chunk c, behind what its state gave
+            wait(&do_done, c & 1, 72);
+            uint32_t v[DT_TOKENS / 16][16];
+            dt_load<DT_TOKENS>(lanes + D_O + t0, v);
+            tmem_wait_ld();
+            if (c > 0) wait(&o_free, (c & 1) ^ 1, 75);           // the copies of the chunk before have read its outputs
+#pragma unroll
+            for (int t = 0; t < DT_TOKENS; ++t) {
+                o[t] = fmaf(__uint_as_float(v[t / 16][t % 16]), u_inv, o[t]);
+                o_s[(t0 + t) * VDIM + column] = o[t];
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) bar_arrive(&o_stored);
+#pragma unroll
+            for (int t = 0; t < DT_TOKENS; t += 2) finite = fma_pairs(pair_of(o[t], o[t + 1]), 0ull, finite);
+        };
+        for (int c = 0; c < chunks; ++c) {
+            const uint32_t phase = c & 1;
+            const float4* f4 = (const float4*)factors[c & 1];            // W's, the queries' and the keys' factors, sixteen of four each
+            float top[2] = {0.f, 0.f};
+#pragma unroll
+            for (int d = 0; d < SHARE; d += 2) top[d / 2 & 1] = max3(top[d / 2 & 1], fabsf(S[d]), fabsf(S[d + 1]));
+            tops[0][share][column] = fmaxf(top[0], top[1]);
+            meet();
+            const int s_exponent = scale_exponent(largest(0));
+            dt_store_parts(S, dc_power(s_exponent), lanes + S_HI + share * (SHARE / 2), lanes + S_LO + share * (SHARE / 2));
+            tmem_wait_st();
+            // the factors came with W: waited for before s_ready, behind which the next chunk's may come and end the barrier's next phase
+            if (!bar_wait(&w_full, phase, failed)) ok = false;
+            fence_before_sync();
+            __syncwarp();
+            if (lane == 0) bar_arrive(&s_ready);
+            if (c > 0) write_outputs(c - 1);         // while W S is made
+
+            // u of this thread's tokens
+            wait(&d1w_done, phase, 69);
+            const float s_inv = dc_power(-s_exponent);
+            uint32_t v[DT_TOKENS / 16][16];
+            dt_load<DT_TOKENS>(lanes + D1_W + t0, v);
+            float u[DT_TOKENS], uk[DT_TOKENS], u_top = 0.f, uk_top = 0.f;
+            if (!bar_wait(&u_full, phase, failed)) ok = false;           // U'; the next chunk's comes behind u_ready
+            __syncwarp();
+#pragma unroll
+            for (int t = 0; t < DT_TOKENS; ++t) u[t] = u_s[(t0 + t) * VDIM + column];
+            tmem_wait_ld();
+#pragma unroll
+            for (int t = 0; t < DT_TOKENS; t += 4) {
+                const float4 fw = f4[(t0 + t) / 4], fk = f4[(2 * DC_TOKENS + t0 + t) / 4];
+                const float ws[4] = {fw.x, fw.y, fw.z, fw.w}, ks[4] = {fk.x, fk.y, fk.z, fk.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    u[t + i] = fmaf(-__uint_as_float(v[(t + i) / 16][(t + i) % 16]), s_inv * ws[i], u[t + i]);
+                    uk[t + i] = u[t + i] * ks[i];
+                }
+                u_top = max3(u_top, fmaxf(fabsf(u[t]), fabsf(u[t + 1])), fmaxf(fabsf(u[t + 2]), fabsf(u[t + 3])));
+                uk_top = max3(uk_top, fmaxf(fabsf(uk[t]), fabsf(uk[t + 1])), fmaxf(fabsf(uk[t + 2]), fabsf(uk[t + 3])));
+            }
+#pragma unroll
+            for (int t = 0; t < DT_TOKENS; t += 2) finite = fma_pairs(pair_of(u[t], u[t + 1]), 0ull, finite);
+            fence_before_sync();                                         // D1's columns are read before another share's parts go over them
+            float begins = fabsf(u[0]);                                  // the first of u that is not zero
+            if (begins == 0.f) {
+#pragma unroll
+                for (int t = DT_TOKENS - 1; t > 0; --t) begins = u[t] != 0.f ? fabsf(u[t]) : begins;
+            }
+            tops[1][share][column] = u_top;
+            tops[2][share][column] = uk_top;
+            tops[3][share][column] = begins;
+            meet();
+            u_top = largest(1);
+            // parts of one scale: a token so much larger than those before it would cost them their digits
+#pragma unroll
+            for (int i = DT_SHARES - 1; i >= 0; --i) begins = tops[3][i][column] != 0.f ? tops[3][i][column] : i == DT_SHARES - 1 ? 0.f : begins;
+            if (begins != 0.f && begins < u_top * 3.725290298461914e-09f) finite = pair_of(NAN, NAN);       // 2^-28
+            const int u_exponent = scale_exponent(u_top), uk_exponent = scale_exponent(largest(2));
+            fence_after_sync();
+            dt_store_parts(uk, dc_power(uk_exponent), lanes + UK + t0 / 2, lanes + UK + 32 + t0 / 2);
+            dt_store_parts(u, dc_power(u_exponent), lanes + D1_W + t0 / 2, lanes + D1_W + 32 + t0 / 2);
+            tmem_wait_st();
+            fence_before_sync();
+            __syncwarp();
+            if (lane == 0) bar_arrive(&u_ready);
+            u_inv = dc_power(-u_exponent) * dc_power(-DC_Q_SCALE);
+
+            // what the state gives the outputs, then the new state
+            wait(&d1q_done, phase, 70);
+            dt_load<DT_TOKENS>(lanes + D1_Q + t0, v);
+            tmem_wait_ld();
+#pragma unroll
+            for (int t = 0; t < DT_TOKENS; t += 4) {
+                const float4 fq = f4[(DC_TOKENS + t0 + t) / 4];
+                const float qs[4] = {fq.x, fq.y, fq.z, fq.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) o[t + i] = __uint_as_float(v[(t + i) / 16][(t + i) % 16]) * (s_inv * qs[i]);
+            }
+            const float decay = factors[c & 1][3 * DC_TOKENS], uk_inv = dc_power(-uk_exponent) * dc_power(-DC_K_SCALE);
+            wait(&ds_done, phase, 71);
+            uint32_t fresh[SHARE / 16][16];
+            dt_load<SHARE>(lanes + D_S + share * SHARE, fresh);
+            tmem_wait_ld();
+#pragma unroll
+            for (int d = 0; d < SHARE; d += 2) {
+                const uint64_t now = fma_pairs(pair_of(S[d], S[d + 1]), pair_of(decay, decay),
+                                               mul_pairs(pair_of(__uint_as_float(fresh[d / 16][d % 16]), __uint_as_float(fresh[d / 16][d % 16 + 1])), pair_of(uk_inv, uk_inv)));
+                finite = fma_pairs(now, 0ull, finite);
+                halves_of(now, S[d], S[d + 1]);
+            }
+        }
+        if (chunks > 0) write_outputs(chunks - 1);
+        float even, odd;
+        halves_of(finite, even, odd);
+        if (even != 0.f || odd != 0.f) odd_numbers = 1;
+        meet();
+        if (chunks > 0) {
+            if (!odd_numbers && ok && !*failed) {
+                float* to = kept + ((start + n_tok) & 1) * p.copy_floats;
+#pragma unroll
+                for (int d = 0; d < SHARE; ++d) to[(size_t)d * VDIM] = S[d];
+            }
+        }
+    }
+    fence_before_sync();
+    __syncthreads();
+    if (failed_flag && warp == 0 && lane == 0) {
+        // copies may still be on their way into this block's shared memory: give them a bounded time to land
+        uint64_t* bars[5] = {&w_full, &q_full, &k_full, &pairs_full, &u_full};
+        for (int i = 0; i < 5; ++i)
+            for (uint32_t parity = 0; parity < 2; ++parity) { int zero = 0; bar_wait(bars[i], parity, &zero, 2000000); }
+    }
+    __syncthreads();
+    if (warp == DT_WARPS + 1) tmem_free(tmem, 512);
+    if (odd_numbers && !failed_flag && warp < 4) dt_token_by_token<DIM>(p, b, h, (float*)w_s);       // over the outputs written, whose copies have ended
+}
+
+// The last launch.  A warp a (token, head): bound by reading o and the gate once.
 template <int VDIM, typename OutT>
 __global__ void __launch_bounds__(256) delta_chunk_finish_kernel(DeltaChunks p, int items) {
     constexpr int EACH = VDIM / 32;
+    after_previous_kernel();
     const int lane = threadIdx.x & 31, item = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (item >= items) return;
     const size_t row = item / p.heads;
@@ -445,13 +950,14 @@ __global__ void __launch_bounds__(256) delta_chunk_finish_kernel(DeltaChunks p, 
 // ----------------------------------------------------------------------------- host side
 
 // Chunks of at most 64 tokens: chunk_seq/begin/end and, per sequence, its first chunk (one entry more at the end).  raw: num_rows *
-// heads * vdim floats; scratch: num_chunks * heads * (64 (dim + vdim + 64 + 2) + 4) floats.
+// heads * vdim floats; scratch: num_chunks * (heads * (64 (dim + vdim + 64 + 3) + 4) + 128 kv_heads (dim + 65)) floats.  status: one int on
+// the device, zero before the call.
 FRB_API int frb_delta_chunks(const float* conv, int conv_stride, int q_off, int k_off, int v_off, const float* proj, int proj_stride, int b_off,
                              int a_off, int g_off, const float* a_log, const float* dt_bias, const float* norm, const int* seq_slot,
                              const int* seq_start, const int* cu_q_len, float* state, long long copy_floats, long long state_offset, void* out,
                              int out_dtype, float* raw, int num_rows, int num_seqs, int heads, int kv_heads, int dim, int vdim, float eps,
                              const int* chunk_seq, const int* chunk_begin, const int* chunk_end, const int* seq_chunk0, int num_chunks,
-                             float* scratch, cudaStream_t stream) {
+                             float* scratch, int* status, cudaStream_t stream) {
     if (num_seqs == 0 || num_chunks == 0) return 0;
     FRB_CHECK_ARG((dim == 64 || dim == 128) && (vdim == 64 || vdim == 128) && kv_heads >= 1 && heads % kv_heads == 0 && heads <= 65535,
                   "delta chunks: %d heads of %d x %d over %d key heads", heads, dim, vdim, kv_heads);
@@ -470,20 +976,35 @@ FRB_API int frb_delta_chunks(const float* conv, int conv_stride, int q_off, int 
     p.q_factor = p.pairs + items * DC_TOKENS * DC_TOKENS;
     p.k_factor = p.q_factor + items * DC_TOKENS;
     p.decays = p.k_factor + items * DC_TOKENS;
+    p.w_parts = (uint16_t*)p.w;
+    p.pair_parts = (uint16_t*)p.pairs;
+    p.factors = p.q_factor;
+    p.q_parts = (uint16_t*)(p.factors + items * DC_FACTORS);
+    p.k_parts = p.q_parts + (size_t)num_chunks * kv_heads * 2 * DC_TOKENS * dim;
+    p.raw_pairs = (float*)(p.k_parts + (size_t)num_chunks * kv_heads * 2 * DC_TOKENS * dim);
+    p.norms = p.raw_pairs + (size_t)num_chunks * kv_heads * 2 * DC_TOKENS * DC_TOKENS;
     p.conv_stride = conv_stride; p.q_off = q_off; p.k_off = k_off; p.v_off = v_off; p.proj_stride = proj_stride; p.b_off = b_off; p.a_off = a_off;
     p.g_off = g_off; p.heads = heads; p.kv_heads = kv_heads; p.eps = eps;
-    const size_t one = (size_t)(2 * DC_TOKENS * (dim + 8) + DC_TOKENS * (DC_TOKENS + 4)) * sizeof(float);
+    const size_t one = (size_t)2 * DC_TOKENS * (dim + 8) * sizeof(float);
     const size_t two = (size_t)(2 * DC_TOKENS * (dim + 8) + DC_TOKENS * (dim + 4) + DC_TOKENS * DC_LM + (dim + DC_TOKENS) * (DC_SLICE + 4)) * sizeof(float);
     const dim3 chains(num_seqs, heads, vdim / DC_SLICE);
     const int rows_heads = num_rows * heads;
 #define FRB_DELTA_CHUNKS(DIM, VDIM)                                                                                                  \
     do {                                                                                                                             \
-        cudaFuncSetAttribute(delta_chunk_solve_kernel<DIM, VDIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)one);            \
-        cudaFuncSetAttribute(delta_chunk_chain_kernel<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)two);                  \
-        delta_chunk_solve_kernel<DIM, VDIM><<<dim3(num_chunks, heads), 256, one, stream>>>(p);                                       \
-        delta_chunk_chain_kernel<DIM><<<chains, 512, two, stream>>>(p, vdim);                                                        \
+        constexpr bool PARTS = VDIM == 128;                                                                                          \
+        cudaFuncSetAttribute(delta_chunk_pairs_kernel<DIM, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)one);           \
+        delta_chunk_pairs_kernel<DIM, PARTS><<<dim3(num_chunks, kv_heads), 256, one, stream>>>(p);                                   \
+        launch_dependent_resident(2, delta_chunk_solve_kernel<DIM, VDIM, PARTS>, dim3(num_chunks, heads), dim3(256), 0, stream, p);  \
+        if constexpr (PARTS) {                                                                                                       \
+            const size_t tc = (size_t)(6 * DIM + 2 * DC_TOKENS + 4 * VDIM) * DC_TOKENS * 2 + 1024;                                   \
+            cudaFuncSetAttribute(delta_chunk_chain_tc_kernel<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc);            \
+            launch_dependent(delta_chunk_chain_tc_kernel<DIM>, dim3(num_seqs, heads), dim3(DT_THREADS), tc, stream, p, status);      \
+        } else {                                                                                                                     \
+            cudaFuncSetAttribute(delta_chunk_chain_kernel<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)two);              \
+            launch_dependent(delta_chunk_chain_kernel<DIM>, chains, dim3(512), two, stream, p, vdim);                                \
+        }                                                                                                                            \
         FRB_DISPATCH_DTYPE(out_dtype, OutT, {                                                                                        \
-            delta_chunk_finish_kernel<VDIM, OutT><<<(rows_heads + 7) / 8, 256, 0, stream>>>(p, rows_heads);                          \
+            launch_dependent_resident(8, delta_chunk_finish_kernel<VDIM, OutT>, dim3((rows_heads + 7) / 8), dim3(256), 0, stream, p, rows_heads); \
         });                                                                                                                          \
     } while (0)
     if (dim == 128 && vdim == 128) FRB_DELTA_CHUNKS(128, 128);

@@ -29,3 +29,16 @@ __device__ __forceinline__ void split_four(float4 v, float scale, uint32_t& hi0,
     split_two(mul_pairs(pair_of(v.x, v.y), s), hi0, lo0);
     split_two(mul_pairs(pair_of(v.z, v.w), s), hi1, lo1);
 }
+
+// `sums` = the products of an operand in tensor memory (its parts at a_hi and a_lo) with one in shared memory, KSTEPS runs of sixteen
+// entries; b_at(k): the place of run k from the second operand's start, in units of 16 bytes.  One lane.
+template <int KSTEPS, typename At>
+__device__ __forceinline__ void products_of_parts(uint32_t sums, uint32_t a_hi, uint32_t a_lo, uint64_t b_hi, uint64_t b_lo, uint32_t idesc, At b_at) {
+#pragma unroll
+    for (int k = 0; k < KSTEPS; ++k) frb_tc::mma_ts(sums, a_lo + 8 * k, b_hi + b_at(k), idesc, k != 0);
+#pragma unroll
+    for (int k = 0; k < KSTEPS; ++k) frb_tc::mma_ts(sums, a_hi + 8 * k, b_lo + b_at(k), idesc, 1);
+    frb_tc::mma_ts_scaled<11>(sums, a_hi, b_hi, idesc);
+#pragma unroll
+    for (int k = 1; k < KSTEPS; ++k) frb_tc::mma_ts(sums, a_hi + 8 * k, b_hi + b_at(k), idesc, 1);
+}

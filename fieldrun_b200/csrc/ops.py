@@ -61,7 +61,7 @@ _SIGNATURES = {
     "frb_weighted_pair": "ppplff",
     "frb_sandwich_norm": "pppffpppippfpfiipipi",
     "frb_gated_delta_rule": "piiii" "piiii" "ppp" "ppp" "pll" "pi" "pii" "iiiii" "f",
-    "frb_delta_chunks": "piiii" "piiii" "ppp" "ppp" "pll" "pip" "iiiiiif" "ppppip",
+    "frb_delta_chunks": "piiii" "piiii" "ppp" "ppp" "pll" "pip" "iiiiiif" "ppppipp",
     "frb_attention_decode_mma": "ppppipppppiiiifiippipf" "iiipff",
     "frb_attention_prefill_mma": "ppppippipppppiiifipipf" "iiii",
     "frb_attention_decode_tma": "pppipipppppiiiifiiippipf" "iiipff",
@@ -202,7 +202,7 @@ def _stream() -> int:
 
 
 _LAUNCHES = 0
-_KERNELS_PER_CALL = {"frb_gated_delta_rule": 2, "frb_gated_recurrence": 2, "frb_sample_floor": 3, "frb_argmax_rows": 2, "frb_expert_plan": 3, "frb_attention_decode_mma": 2, "frb_attention_decode_tma": 2, "frb_attention_f32_token": 2, "frb_gla_chunks": 3, "frb_state_space_chunks": 4, "frb_delta_chunks": 3, "frb_products_f32": 2, "frb_attention_f32_tc": 2}
+_KERNELS_PER_CALL = {"frb_gated_delta_rule": 2, "frb_gated_recurrence": 2, "frb_sample_floor": 3, "frb_argmax_rows": 2, "frb_expert_plan": 3, "frb_attention_decode_mma": 2, "frb_attention_decode_tma": 2, "frb_attention_f32_token": 2, "frb_gla_chunks": 3, "frb_state_space_chunks": 4, "frb_delta_chunks": 4, "frb_products_f32": 2, "frb_attention_f32_tc": 2}
 
 
 def launches() -> int:
@@ -1260,9 +1260,10 @@ def delta_chunks_take(dim: int, vdim: int, conv_offsets: tuple, state: torch.Ten
             and state_offset % 2 == 0)
 
 
-def delta_chunks_scratch_floats(chunks: int, heads: int, dim: int, vdim: int) -> int:
+def delta_chunks_scratch_floats(chunks: int, heads: int, dim: int, vdim: int, kv_heads: Optional[int] = None) -> int:
     """float32 elements of scratch that :func:`delta_chunks` needs."""
-    return chunks * heads * (DELTA_CHUNK_TOKENS * (dim + vdim + DELTA_CHUNK_TOKENS + 2) + 4)
+    return chunks * (heads * (DELTA_CHUNK_TOKENS * (dim + vdim + DELTA_CHUNK_TOKENS + 3) + 4)
+                     + 2 * (heads if kv_heads is None else kv_heads) * DELTA_CHUNK_TOKENS * (dim + DELTA_CHUNK_TOKENS + 1))
 
 
 def delta_chunks(conv: torch.Tensor, q_off: int, k_off: int, v_off: int, proj: torch.Tensor, b_off: int, a_off: int, g_off: int,
@@ -1277,13 +1278,13 @@ def delta_chunks(conv: torch.Tensor, q_off: int, k_off: int, v_off: int, proj: t
     for t in chunks:
         _want(t, torch.int32, "chunk tables")
     count = chunks[0].numel()
-    if (chunks[3].numel() != ctx.num_seqs + 1 or scratch.numel() < delta_chunks_scratch_floats(count, heads, dim, vdim)
+    if (chunks[3].numel() != ctx.num_seqs + 1 or scratch.numel() < delta_chunks_scratch_floats(count, heads, dim, vdim, kv_heads)
             or raw.numel() < out.numel()):
         raise KernelError("the chunk tables, the scratch or the unnormed outputs of the delta rule's chunks have the wrong size")
     _call("frb_delta_chunks", _ptr(conv), conv.shape[1], int(q_off), int(k_off), int(v_off), _ptr(proj), proj.shape[1], int(b_off),
           int(a_off), int(g_off), _ptr(a_log), _ptr(dt_bias), _ptr(norm), _ptr(ctx.seq_slot), _ptr(ctx.seq_start), _ptr(ctx.cu_q_len),
           *_state_place(state, state_offset), _ptr(out), _code(out.dtype), _ptr(raw), conv.shape[0], ctx.num_seqs, int(heads),
-          int(kv_heads), int(dim), int(vdim), float(eps), *(_ptr(t) for t in chunks), count, _ptr(scratch))
+          int(kv_heads), int(dim), int(vdim), float(eps), *(_ptr(t) for t in chunks), count, _ptr(scratch), _ptr(tc_status(conv.device)))
 
 
 MMA_HEAD_DIMS = (32, 64, 96, 128)
@@ -1523,6 +1524,21 @@ _WAIT_CODES = {
     44: "float32 products: a splitter waiting for a loaded stage of weights",
     45: "float32 products: a splitter waiting for a free stage of parts",
     46: "float32 products: a collector waiting for finished sums",
+    61: "delta rule in chunks: the producer waiting for W to have been read",
+    62: "delta rule in chunks: the producer waiting for the queries to have been read",
+    63: "delta rule in chunks: the producer waiting for the keys to have been read",
+    64: "delta rule in chunks: the producer waiting for the pairs' weights to have been read",
+    65: "delta rule in chunks: the MMA warp waiting for W or the state's parts",
+    66: "delta rule in chunks: the MMA warp waiting for the queries",
+    67: "delta rule in chunks: the MMA warp waiting for the keys or u's parts",
+    68: "delta rule in chunks: the MMA warp waiting for the pairs' weights",
+    69: "delta rule in chunks: the columns waiting for W S",
+    70: "delta rule in chunks: the columns waiting for Q S",
+    71: "delta rule in chunks: the columns waiting for the new state",
+    72: "delta rule in chunks: the columns waiting for the outputs",
+    73: "delta rule in chunks: the producer waiting for U' to have been read",
+    74: "delta rule in chunks: the outputs' copies waiting for the outputs",
+    75: "delta rule in chunks: the columns waiting for the outputs' copies",
     51: "float32 prompt attention: the producer waiting for a free stage of keys",
     52: "float32 prompt attention: the producer waiting for a free stage of values",
     53: "float32 prompt attention: the MMA warp waiting for a page's keys",

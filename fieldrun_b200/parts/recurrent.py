@@ -39,8 +39,8 @@ from .linear import linear
 # delta_chunks.cu).  Measured on a B200, the kernels alone, microseconds, token by token | in chunks.  State space: 64 heads of 128 x 64, one
 # prompt of 128 tokens 55 | 70, of 1,024 tokens 350 | 119, 16 of 130 tokens 279 | 353, of 256 tokens 525 | 390, one of 256 beside 31 of two
 # 188 | 374; 16 heads of 64 x 64, 64 of 128 tokens 159 | 185; of 128 x 128, 4 of 300 tokens 166 | 119.  Delta rule: 16 heads of 128 x 128, one
-# prompt of 64 tokens 63 | 52, of 1,024 tokens 670 | 231, 16 of 65 tokens 213 | 178, 64 of 64 tokens 687 | 339; 64 heads of 64 x 64, 16 of 65 tokens
-# 205 | 271; 64 heads of 128 x 64, one of 256 beside 31 of two 330 | 449.
+# prompt of 64 tokens 51 | 42, of 1,024 tokens 671 | 104, 16 of 65 tokens 208 | 95, 100 of 17 beside one of 64 460 | 273; 64 heads of 64 x 64, 16 of
+# 65 tokens 205 | 271; 64 heads of 128 x 64, one of 256 beside 31 of two 330 | 449.
 STATE_SPACE_CHUNKED_TOKENS, DELTA_CHUNKED_TOKENS = 128, 64
 
 
@@ -310,9 +310,12 @@ class GatedDeltaRule(_StateMixer):
         size = self.head_dim * self.value_dim / 2 ** 14                     # as a share of 128 x 128
         tokens, chunk = ctx.num_tokens * self.num_heads, ops.DELTA_CHUNK_TOKENS
         serial = 15 + max((0.6 + 0.2 * size) * ctx.max_q_len, (0.0002 + 0.0105 * size) * tokens)
-        items = ctx.chunk_count(chunk) * self.num_heads
-        along = max((6 + 6 * size) * -(-ctx.max_q_len // chunk), (0.026 + 0.13 * size) * items)
-        return ops.chunks_pay(max(42 + 10 * size, 31 + (0.046 + 0.096 * size) * items + along), serial)
+        items, longest = ctx.chunk_count(chunk) * self.num_heads, -(-ctx.max_q_len // chunk)
+        if self.value_dim == 128:                                           # the chain along the chunks on tcgen05
+            along = max((3.2 + 0.6 * size) * longest, 0.06 * items)
+            return ops.chunks_pay(max(48 + 4 * size, 30 + (0.045 + 0.045 * size) * items + along), serial)
+        along = max((6 + 6 * size) * longest, (0.026 + 0.13 * size) * items)
+        return ops.chunks_pay(max(44 + 10 * size, 33 + (0.046 + 0.096 * size) * items + along), serial)
 
     def forward(self, ctx, act: torch.Tensor, line: LineView, writes_cache: bool) -> torch.Tensor:
         self._check(writes_cache)
@@ -328,7 +331,7 @@ class GatedDeltaRule(_StateMixer):
         if (self.chunks_pay(ctx)
                 and ops.delta_chunks_take(self.head_dim, self.value_dim, (self.conv_channels, self.qk_width), line.state, 0)):
             chunks = ctx.token_chunks(ops.DELTA_CHUNK_TOKENS)
-            floats = ops.delta_chunks_scratch_floats(chunks[0].numel(), self.num_heads, self.head_dim, self.value_dim)
+            floats = ops.delta_chunks_scratch_floats(chunks[0].numel(), self.num_heads, self.head_dim, self.value_dim, self.num_kv_heads)
             ops.delta_chunks(*args, chunks=chunks, scratch=ctx.buffer("delta_rule.chunks", (floats,), torch.float32), **sizes)
         else:
             ops.gated_delta_rule(*args, **sizes)

@@ -293,8 +293,8 @@ def state_space_case():
     return views, run, exact
 
 
-def delta_case():
-    heads, kv_heads, dim, vdim = 4, 2, 64, 64
+def delta_case(vdim=64):
+    heads, kv_heads, dim = 4, 2, 64
     gen = torch.Generator(device=DEV).manual_seed(3)
     tokens, qk, inner = AT[-1], kv_heads * dim, heads * vdim
     conv, proj = torch.randn(tokens, 2 * qk + inner, device=DEV, generator=gen), torch.randn(tokens, 2 * heads + inner, device=DEV, generator=gen)
@@ -337,15 +337,17 @@ def delta_case():
     return views, run, exact
 
 
-CASES = {"gla": gla_case, "state space": state_space_case, "delta": delta_case}
+# with 128 value columns the chain along the chunks runs on tcgen05
+CASES = {"gla": gla_case, "state space": state_space_case, "delta": delta_case, "delta 128": lambda: delta_case(128)}
 
 
 NAMES = [("gla", n) for n in ("q", "k", "v", "decay")] + [("state space", n) for n in ("x", "b", "c", "decay")] + [
-    ("delta", n) for n in ("q", "k", "v", "beta", "decay")]
+    (c, n) for c in ("delta", "delta 128") for n in ("q", "k", "v", "beta", "decay")]
 
 
 @pytest.mark.parametrize("case,name,number", [(*c, n) for c in NAMES for n in (INF, NAN)] + [("state space", "x", 3.4028234e38),
-                                                                                             ("delta", "v", 3.4028234e38)])
+                                                                                             ("delta", "v", 3.4028234e38),
+                                                                                             ("delta 128", "v", 3.4028234e38)])
 def test_a_token_that_is_not_finite_reaches_no_token_before_it(case, name, number):
     """One entry of a token in the middle of a chunk, of a chunk's last block and of a short sequence: the heads of the outputs and the
     entries of the states that it makes infinities or NaNs of are those that it does token by token, and the tokens before it keep
@@ -373,7 +375,8 @@ def test_a_token_that_is_not_finite_reaches_no_token_before_it(case, name, numbe
             assert norm_error(a, b) < LIMIT
 
 
-@pytest.mark.parametrize("case,strong", [(c, s) for c in ("state space", "delta") for s in (-20.0, -200.0, -2000.0)] + [("delta", -INF)])
+@pytest.mark.parametrize("case,strong", [(c, s) for c in ("state space", "delta", "delta 128") for s in (-20.0, -200.0, -2000.0)] +
+                         [("delta", -INF), ("delta 128", -INF)])
 def test_one_strong_decay_among_mild_ones(case, strong):
     """Tokens that all but clear the state (logarithm of the decay down to about -2,000, and a decay of zero), one in each of some blocks,
     at the starts of chunks and blocks among them, the others mild: against 64 bits, every token's head by itself.  A weight between
