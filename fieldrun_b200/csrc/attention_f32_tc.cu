@@ -54,8 +54,6 @@ __device__ __forceinline__ PageRun pages_of(const F32Attention& p, int start, in
     return r;
 }
 
-__device__ __forceinline__ float power_of_two(int exponent) { return __uint_as_float((uint32_t)(exponent + 127) << 23); }
-
 // ----------------------------------------------------------------------------- the pages' parts
 
 // A block a page of one key head (blockIdx.z 0) or value head (1).  Scratch: keys [page][key head][part][HD / 64][64 keys][64 entries],
@@ -147,11 +145,6 @@ attention_f32_split_kernel(F32Attention p, const int* __restrict__ seq_slot, con
 }
 
 // ----------------------------------------------------------------------------- the tiles
-
-__device__ __forceinline__ void copy_bulk(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(bar)) : "memory");
-}
 
 // grid (head, tile of 128 queries).  MODIFIED: capped scores or slopes.
 template <int HD, int VD, bool MODIFIED>

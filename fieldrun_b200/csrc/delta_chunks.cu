@@ -74,11 +74,6 @@ __device__ __forceinline__ void dc_copy_rows(float* to, int ld, const float* fro
     }
 }
 
-__device__ __forceinline__ float dc_power(int exponent) { return __uint_as_float((uint32_t)(exponent + 127) << 23); }
-
-// The place of entry `c` (even) of row `r` in pieces [64 rows][64 entries] of rows of 128 bytes, 128-byte swizzle, in float16 entries.
-__device__ __forceinline__ int dc_place(int r, int c) { return (c >> 6) * (DC_TOKENS * 64) + r * 64 + (((c >> 3 & 7) ^ (r & 7)) << 3) + (c & 7); }
-
 // The exponent that brings entries of W's row i, at most 2^6 w(i), below 2^14.
 __device__ __forceinline__ int dc_w_exponent(float start) { return DC_W_SCALE - max(ilogbf(fmaxf(start, 1e-30f)), -100); }
 
@@ -127,11 +122,11 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_pairs_kernel(DeltaChunks p
             const bool key = u >= UNITS;
             const int r = u % UNITS / (DIM / 8), c = u % (DIM / 8) * 8;
             const float* from = (key ? k_s : q_s) + r * LQ + c;
-            const float scale = (key ? k_inv[r] : q_inv[r]) * dc_power(key ? DC_K_SCALE : DC_Q_SCALE);
+            const float scale = (key ? k_inv[r] : q_inv[r]) * power_of_two(key ? DC_K_SCALE : DC_Q_SCALE);
             uint4 hi, lo;
             split_four(*(const float4*)from, scale, hi.x, hi.y, lo.x, lo.y);
             split_four(*(const float4*)(from + 4), scale, hi.z, hi.w, lo.z, lo.w);
-            uint16_t* parts = (key ? p.k_parts : p.q_parts) + to + dc_place(r, c);
+            uint16_t* parts = (key ? p.k_parts : p.q_parts) + to + piece_place(r, c);
             *(uint4*)parts = hi;
             *(uint4*)(parts + DC_TOKENS * DIM) = lo;
         }
@@ -254,9 +249,9 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
         if (PARTS) {
             float* factors = p.factors + at * DC_FACTORS;
             const int exponent = dc_w_exponent(start_s[tid]);
-            w_scale[tid] = dc_power(exponent);
-            factors[tid] = dc_power(-exponent);
-            factors[DC_TOKENS + tid] = start_s[tid] * dc_power(-DC_Q_SCALE);
+            w_scale[tid] = power_of_two(exponent);
+            factors[tid] = power_of_two(-exponent);
+            factors[DC_TOKENS + tid] = start_s[tid] * power_of_two(-DC_Q_SCALE);
             factors[2 * DC_TOKENS + tid] = to_end;
             if (tid == DC_TOKENS - 1) factors[3 * DC_TOKENS] = start_s[tid];
         } else {
@@ -299,9 +294,9 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
         }
         if (PARTS) {
             uint4 hi, lo;
-            split_four(make_float4(y[0], y[1], y[2], y[3]), dc_power(DC_Q_SCALE), hi.x, hi.y, lo.x, lo.y);
-            split_four(make_float4(y[4], y[5], y[6], y[7]), dc_power(DC_Q_SCALE), hi.z, hi.w, lo.z, lo.w);
-            uint16_t* to = p.pair_parts + at * 2 * DC_TOKENS * DC_TOKENS + dc_place(i, j0);
+            split_four(make_float4(y[0], y[1], y[2], y[3]), power_of_two(DC_Q_SCALE), hi.x, hi.y, lo.x, lo.y);
+            split_four(make_float4(y[4], y[5], y[6], y[7]), power_of_two(DC_Q_SCALE), hi.z, hi.w, lo.z, lo.w);
+            uint16_t* to = p.pair_parts + at * 2 * DC_TOKENS * DC_TOKENS + piece_place(i, j0);
             *(uint4*)to = hi;
             *(uint4*)(to + DC_TOKENS * DC_TOKENS) = lo;
         } else {
@@ -337,7 +332,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
                 const float scale = w_scale[r];
                 uint32_t hi, lo;
                 split_two(mul_pairs(odd_column ? pair_of(theirs, done) : pair_of(x[i - 1], theirs), pair_of(scale, scale)), hi, lo);
-                uint16_t* parts = w_parts + dc_place(r, tid & ~1);
+                uint16_t* parts = w_parts + piece_place(r, tid & ~1);
                 *(uint32_t*)parts = hi;
                 *(uint32_t*)(parts + DC_TOKENS * DIM) = lo;
             }
@@ -569,38 +564,6 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_chain_kernel(DeltaChunks p
 using namespace frb_tma;
 using namespace frb_tc;
 
-__device__ __forceinline__ void dt_copy(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(bar)) : "memory");
-}
-
-// An N-major operand of pieces [64 of the inner size][64 entries] (rows of 128 bytes, 128-byte swizzle), a piece DC_TOKENS * 128 bytes.
-__device__ __forceinline__ uint64_t dt_desc_n_major(uint32_t addr) {
-    return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)(DC_TOKENS * 128 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
-           ((uint64_t)2 << 61);
-}
-
-// N entries of a column times its scale, as parts, to N / 2 columns of tensor memory each.
-template <int N>
-__device__ __forceinline__ void dt_store_parts(const float (&x)[N], float scale, uint32_t to_hi, uint32_t to_lo) {
-    static_assert(N % 32 == 0, "entries of a store");
-#pragma unroll
-    for (int n = 0; n < N; n += 32) {
-        uint32_t hi[16], lo[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) split_two(mul_pairs(pair_of(x[n + 2 * i], x[n + 2 * i + 1]), pair_of(scale, scale)), hi[i], lo[i]);
-        tmem_st16(to_hi + n / 2, hi);
-        tmem_st16(to_lo + n / 2, lo);
-    }
-}
-
-// N columns of tensor memory, there after tmem_wait_ld().
-template <int N>
-__device__ __forceinline__ void dt_load(uint32_t from, uint32_t (&v)[N / 16][16]) {
-#pragma unroll
-    for (int i = 0; i < N / 16; ++i) tmem_ld16(from + 16 * i, v[i]);
-}
-
 // A sequence's head token by token (delta_rule.cu's formula): 128 threads of a block, one a value column; `rows_s`: 2 DIM + 3 floats.
 template <int DIM>
 static __device__ __noinline__ void dt_token_by_token(const DeltaChunks& p, int b, int h, float* rows_s) {
@@ -698,20 +661,20 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(Del
                 const uint32_t before = (c & 1) ^ 1;                     // of the phase that the chunk before has ended
                 if (c && !bar_wait(&d1w_done, before, failed)) { atomicExch(status, 61); break; }
                 bar_expect(&w_full, 2 * ROWS_PART + DC_FACTORS * 4);
-                dt_copy(w_s, p.w_parts + at * 2 * DC_TOKENS * DIM, 2 * ROWS_PART, &w_full);
-                dt_copy(factors[c & 1], p.factors + at * DC_FACTORS, DC_FACTORS * 4, &w_full);
+                copy_bulk(w_s, p.w_parts + at * 2 * DC_TOKENS * DIM, 2 * ROWS_PART, &w_full);
+                copy_bulk(factors[c & 1], p.factors + at * DC_FACTORS, DC_FACTORS * 4, &w_full);
                 if (c && !bar_wait(&u_ready, before, failed)) { atomicExch(status, 73); break; }
                 bar_expect(&u_full, DC_TOKENS * VDIM * 4);
-                dt_copy(u_s, p.u + at * DC_TOKENS * VDIM, DC_TOKENS * VDIM * 4, &u_full);
+                copy_bulk(u_s, p.u + at * DC_TOKENS * VDIM, DC_TOKENS * VDIM * 4, &u_full);
                 if (c && !bar_wait(&d1q_done, before, failed)) { atomicExch(status, 62); break; }
                 bar_expect(&q_full, 2 * ROWS_PART);
-                dt_copy(q_s, p.q_parts + kv_at * 2 * DC_TOKENS * DIM, 2 * ROWS_PART, &q_full);
+                copy_bulk(q_s, p.q_parts + kv_at * 2 * DC_TOKENS * DIM, 2 * ROWS_PART, &q_full);
                 if (c && !bar_wait(&ds_done, before, failed)) { atomicExch(status, 63); break; }
                 bar_expect(&k_full, 2 * ROWS_PART);
-                dt_copy(k_s, p.k_parts + kv_at * 2 * DC_TOKENS * DIM, 2 * ROWS_PART, &k_full);
+                copy_bulk(k_s, p.k_parts + kv_at * 2 * DC_TOKENS * DIM, 2 * ROWS_PART, &k_full);
                 if (c && !bar_wait(&do_done, before, failed)) { atomicExch(status, 64); break; }
                 bar_expect(&pairs_full, 2 * PAIR_PART);
-                dt_copy(pairs_s, p.pair_parts + at * 2 * DC_TOKENS * DC_TOKENS, 2 * PAIR_PART, &pairs_full);
+                copy_bulk(pairs_s, p.pair_parts + at * 2 * DC_TOKENS * DC_TOKENS, 2 * PAIR_PART, &pairs_full);
             }
         }
     } else if (warp == DT_WARPS + 1) {
@@ -719,7 +682,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(Del
         constexpr uint32_t idesc64 = (1u << 4) | ((uint32_t)(64 >> 3) << 17) | ((uint32_t)(VDIM >> 4) << 24);
         constexpr uint32_t idesc_k = (1u << 4) | (1u << 16) | ((uint32_t)(DIM >> 3) << 17) | ((uint32_t)(VDIM >> 4) << 24);
         const uint64_t w_at = tile_desc(smem_addr(w_s)), q_at = tile_desc(smem_addr(q_s)), pairs_at = tile_desc(smem_addr(pairs_s));
-        const uint64_t k_at = dt_desc_n_major(smem_addr(k_s));
+        const uint64_t k_at = desc_n_major(smem_addr(k_s));
         auto along = [](int k) { return (k / 4) * (DC_TOKENS * 128 >> 4) + (k % 4) * 2; };
         auto down = [](int k) { return k * (16 * 128 >> 4); };
         for (int c = 0; c < chunks; ++c) {
@@ -784,7 +747,6 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(Del
             for (int i = 1; i < DT_SHARES; ++i) top = fmaxf(top, tops[slot][i][column]);
             return top;
         };
-        auto scale_exponent = [](float top) { return 14 - ilogbf(fminf(fmaxf(top, 7.888609052210118e-31f), 3.402823466e38f)); };     // from 2^-100
         float S[SHARE], o[DT_TOKENS];
         uint64_t finite = 0ull;                      // becomes NaNs at the first number that is not finite
 #pragma unroll
@@ -793,7 +755,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(Del
         auto write_outputs = [&](int c) {            // what u gives the outputs of chunk c, behind what its state gave
             wait(&do_done, c & 1, 72);
             uint32_t v[DT_TOKENS / 16][16];
-            dt_load<DT_TOKENS>(lanes + D_O + t0, v);
+            load_columns<DT_TOKENS>(lanes + D_O + t0, v);
             tmem_wait_ld();
             if (c > 0) wait(&o_free, (c & 1) ^ 1, 75);           // the copies of the chunk before have read its outputs
 #pragma unroll
@@ -815,8 +777,8 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(Del
             for (int d = 0; d < SHARE; d += 2) top[d / 2 & 1] = max3(top[d / 2 & 1], fabsf(S[d]), fabsf(S[d + 1]));
             tops[0][share][column] = fmaxf(top[0], top[1]);
             meet();
-            const int s_exponent = scale_exponent(largest(0));
-            dt_store_parts(S, dc_power(s_exponent), lanes + S_HI + share * (SHARE / 2), lanes + S_LO + share * (SHARE / 2));
+            const int s_exponent = parts_exponent(largest(0));
+            store_parts(S, power_of_two(s_exponent), lanes + S_HI + share * (SHARE / 2), lanes + S_LO + share * (SHARE / 2));
             tmem_wait_st();
             // the factors came with W: waited for before s_ready, behind which the next chunk's may come and end the barrier's next phase
             if (!bar_wait(&w_full, phase, failed)) ok = false;
@@ -827,9 +789,9 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(Del
 
             // u of this thread's tokens
             wait(&d1w_done, phase, 69);
-            const float s_inv = dc_power(-s_exponent);
+            const float s_inv = power_of_two(-s_exponent);
             uint32_t v[DT_TOKENS / 16][16];
-            dt_load<DT_TOKENS>(lanes + D1_W + t0, v);
+            load_columns<DT_TOKENS>(lanes + D1_W + t0, v);
             float u[DT_TOKENS], uk[DT_TOKENS], u_top = 0.f, uk_top = 0.f;
             if (!bar_wait(&u_full, phase, failed)) ok = false;           // U'; the next chunk's comes behind u_ready
             __syncwarp();
@@ -851,33 +813,27 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(Del
 #pragma unroll
             for (int t = 0; t < DT_TOKENS; t += 2) finite = fma_pairs(pair_of(u[t], u[t + 1]), 0ull, finite);
             fence_before_sync();                                         // D1's columns are read before another share's parts go over them
-            float begins = fabsf(u[0]);                                  // the first of u that is not zero
-            if (begins == 0.f) {
-#pragma unroll
-                for (int t = DT_TOKENS - 1; t > 0; --t) begins = u[t] != 0.f ? fabsf(u[t]) : begins;
-            }
             tops[1][share][column] = u_top;
             tops[2][share][column] = uk_top;
-            tops[3][share][column] = begins;
+            if (share == 0) tops[3][0][column] = first_row_top(u);
             meet();
             u_top = largest(1);
             // parts of one scale: a token so much larger than those before it would cost them their digits
-#pragma unroll
-            for (int i = DT_SHARES - 1; i >= 0; --i) begins = tops[3][i][column] != 0.f ? tops[3][i][column] : i == DT_SHARES - 1 ? 0.f : begins;
-            if (begins != 0.f && begins < u_top * 3.725290298461914e-09f) finite = pair_of(NAN, NAN);       // 2^-28
-            const int u_exponent = scale_exponent(u_top), uk_exponent = scale_exponent(largest(2));
+            const float first_top = tops[3][0][column];
+            if (first_top != 0.f && first_top < u_top * 3.725290298461914e-09f) finite = pair_of(NAN, NAN);       // 2^-28
+            const int u_exponent = parts_exponent(u_top), uk_exponent = parts_exponent(largest(2));
             fence_after_sync();
-            dt_store_parts(uk, dc_power(uk_exponent), lanes + UK + t0 / 2, lanes + UK + 32 + t0 / 2);
-            dt_store_parts(u, dc_power(u_exponent), lanes + D1_W + t0 / 2, lanes + D1_W + 32 + t0 / 2);
+            store_parts(uk, power_of_two(uk_exponent), lanes + UK + t0 / 2, lanes + UK + 32 + t0 / 2);
+            store_parts(u, power_of_two(u_exponent), lanes + D1_W + t0 / 2, lanes + D1_W + 32 + t0 / 2);
             tmem_wait_st();
             fence_before_sync();
             __syncwarp();
             if (lane == 0) bar_arrive(&u_ready);
-            u_inv = dc_power(-u_exponent) * dc_power(-DC_Q_SCALE);
+            u_inv = power_of_two(-u_exponent) * power_of_two(-DC_Q_SCALE);
 
             // what the state gives the outputs, then the new state
             wait(&d1q_done, phase, 70);
-            dt_load<DT_TOKENS>(lanes + D1_Q + t0, v);
+            load_columns<DT_TOKENS>(lanes + D1_Q + t0, v);
             tmem_wait_ld();
 #pragma unroll
             for (int t = 0; t < DT_TOKENS; t += 4) {
@@ -886,10 +842,10 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(Del
 #pragma unroll
                 for (int i = 0; i < 4; ++i) o[t + i] = __uint_as_float(v[(t + i) / 16][(t + i) % 16]) * (s_inv * qs[i]);
             }
-            const float decay = factors[c & 1][3 * DC_TOKENS], uk_inv = dc_power(-uk_exponent) * dc_power(-DC_K_SCALE);
+            const float decay = factors[c & 1][3 * DC_TOKENS], uk_inv = power_of_two(-uk_exponent) * power_of_two(-DC_K_SCALE);
             wait(&ds_done, phase, 71);
             uint32_t fresh[SHARE / 16][16];
-            dt_load<SHARE>(lanes + D_S + share * SHARE, fresh);
+            load_columns<SHARE>(lanes + D_S + share * SHARE, fresh);
             tmem_wait_ld();
 #pragma unroll
             for (int d = 0; d < SHARE; d += 2) {

@@ -42,3 +42,56 @@ __device__ __forceinline__ void products_of_parts(uint32_t sums, uint32_t a_hi, 
 #pragma unroll
     for (int k = 1; k < KSTEPS; ++k) frb_tc::mma_ts(sums, a_hi + 8 * k, b_hi + b_at(k), idesc, 1);
 }
+
+__device__ __forceinline__ float power_of_two(int exponent) { return __uint_as_float((uint32_t)(exponent + 127) << 23); }
+
+__device__ __forceinline__ void copy_bulk(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(frb_tma::smem_addr(dst)), "l"(src), "r"(bytes), "r"(frb_tma::smem_addr(bar)) : "memory");
+}
+
+// The place of entry `c` of row `r` in pieces [64 rows][64 entries] of rows of 128 bytes, 128-byte swizzle, in float16 entries.
+__device__ __forceinline__ int piece_place(int r, int c) { return (c >> 6) * (64 * 64) + r * 64 + (((c >> 3 & 7) ^ (r & 7)) << 3) + (c & 7); }
+
+// An N-major operand of such pieces, the rows along the inner size: a run of sixteen of it is 128 on in units of 16 bytes.
+__device__ __forceinline__ uint64_t desc_n_major(uint32_t addr) {
+    return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)(64 * 128 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
+           ((uint64_t)2 << 61);
+}
+
+// N entries of a lane times its scale, as parts, to N / 2 columns of tensor memory each.
+template <int N>
+__device__ __forceinline__ void store_parts(const float (&x)[N], float scale, uint32_t to_hi, uint32_t to_lo) {
+    static_assert(N % 32 == 0, "entries of a store");
+#pragma unroll
+    for (int n = 0; n < N; n += 32) {
+        uint32_t hi[16], lo[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) split_two(mul_pairs(pair_of(x[n + 2 * i], x[n + 2 * i + 1]), pair_of(scale, scale)), hi[i], lo[i]);
+        frb_tc::tmem_st16(to_hi + n / 2, hi);
+        frb_tc::tmem_st16(to_lo + n / 2, lo);
+    }
+}
+
+// N columns of tensor memory, there after tmem_wait_ld().
+template <int N>
+__device__ __forceinline__ void load_columns(uint32_t from, uint32_t (&v)[N / 16][16]) {
+#pragma unroll
+    for (int i = 0; i < N / 16; ++i) frb_tc::tmem_ld16(from + 16 * i, v[i]);
+}
+
+// The exponent of the power of two that brings `top` to [2^14, 2^15); of a smaller one than 2^-100 as if it were that, of a NaN too.
+__device__ __forceinline__ int parts_exponent(float top) { return 14 - ilogbf(fminf(fmaxf(top, 7.888609052210118e-31f), 3.402823466e38f)); }
+
+// The largest entry over the warp's columns of the first of eight tokens that has one; zero: none has.  (A single column's may be as
+// small as chance has it.)
+template <int N>
+__device__ __forceinline__ float first_row_top(const float (&u)[N]) {
+    uint32_t top = 0;
+#pragma unroll
+    for (int t = 7; t >= 0; --t) {
+        const uint32_t row = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(u[t])));
+        if (row != 0) top = row;
+    }
+    return __uint_as_float(top);
+}

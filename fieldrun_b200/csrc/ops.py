@@ -42,7 +42,7 @@ _SIGNATURES = {
     "frb_softplus_bias": "ppii",
     "frb_gated_recurrence": "piipppppppppppllpiiiiif",
     "frb_state_space_scan": "piiipiiipppppppllpiiiii",
-    "frb_state_space_chunks": "piiipiii" "ppp" "ppp" "pll" "piiiii" "ppppip",
+    "frb_state_space_chunks": "piiipiii" "ppp" "ppp" "pll" "piiiii" "ppppiipp",
     "frb_group_rms_norm": "pppiiiif",
     "frb_gla_scan": "piiiiiipipppppppiiiiiifffppppippi",
     "frb_gla_chunks": "piiiiiipipppppppiiiiifffppppip",
@@ -202,7 +202,7 @@ def _stream() -> int:
 
 
 _LAUNCHES = 0
-_KERNELS_PER_CALL = {"frb_gated_delta_rule": 2, "frb_gated_recurrence": 2, "frb_sample_floor": 3, "frb_argmax_rows": 2, "frb_expert_plan": 3, "frb_attention_decode_mma": 2, "frb_attention_decode_tma": 2, "frb_attention_f32_token": 2, "frb_gla_chunks": 3, "frb_state_space_chunks": 4, "frb_delta_chunks": 4, "frb_products_f32": 2, "frb_attention_f32_tc": 2}
+_KERNELS_PER_CALL = {"frb_gated_delta_rule": 2, "frb_gated_recurrence": 2, "frb_sample_floor": 3, "frb_argmax_rows": 2, "frb_expert_plan": 3, "frb_attention_decode_mma": 2, "frb_attention_decode_tma": 2, "frb_attention_f32_token": 2, "frb_gla_chunks": 3, "frb_state_space_chunks": 3, "frb_delta_chunks": 4, "frb_products_f32": 2, "frb_attention_f32_tc": 2}
 
 
 def launches() -> int:
@@ -699,7 +699,8 @@ def state_space_chunks_take(heads: int, vdim: int, n: int, groups: int, z_offset
 
 def state_space_chunks_scratch_floats(chunks: int, heads: int, vdim: int, n: int, groups: int) -> int:
     """float32 elements of scratch that :func:`state_space_chunks` needs."""
-    return chunks * (heads * n * vdim + groups * STATE_SPACE_CHUNK_TOKENS ** 2 + heads)
+    half = STATE_SPACE_CHUNK_TOKENS // 2
+    return 2 * chunks * (groups * (half * (half + 2 * n + 1) + 4) + heads * (half * half + 4 * half + 4))
 
 
 def state_space_chunks(proj: torch.Tensor, z_offset: int, dt_offset: int, xbc: torch.Tensor, b_offset: int, c_offset: int,
@@ -718,7 +719,7 @@ def state_space_chunks(proj: torch.Tensor, z_offset: int, dt_offset: int, xbc: t
     _call("frb_state_space_chunks", _ptr(proj), proj.shape[1], int(z_offset), int(dt_offset), _ptr(xbc), xbc.shape[1], int(b_offset),
           int(c_offset), _ptr(dt_bias), _ptr(a_log), _ptr(d), _ptr(ctx.seq_slot), _ptr(ctx.seq_start), _ptr(ctx.cu_q_len),
           *_state_place(state, state_offset), _ptr(out), ctx.num_seqs, heads, vdim, n, groups, *(_ptr(t) for t in chunks), count,
-          _ptr(scratch))
+          xbc.shape[0], _ptr(scratch), _ptr(tc_status(xbc.device)))
 
 
 def group_rms_norm(rows_in: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, norm_groups: int, eps: float) -> None:
@@ -1539,6 +1540,19 @@ _WAIT_CODES = {
     73: "delta rule in chunks: the producer waiting for U' to have been read",
     74: "delta rule in chunks: the outputs' copies waiting for the outputs",
     75: "delta rule in chunks: the columns waiting for the outputs' copies",
+    81: "state space in chunks: the producer waiting for the values to have been read",
+    82: "state space in chunks: the producer waiting for B to have been read",
+    83: "state space in chunks: the producer waiting for C to have been read",
+    84: "state space in chunks: the producer waiting for the pairs' weights to have been read",
+    85: "state space in chunks: the MMA warp waiting for the columns' parts or B",
+    86: "state space in chunks: the MMA warp waiting for C",
+    87: "state space in chunks: the MMA warp waiting for the pairs' weights",
+    88: "state space in chunks: the columns waiting for the values",
+    89: "state space in chunks: the columns waiting for the new state",
+    90: "state space in chunks: the columns waiting for C S",
+    91: "state space in chunks: the columns waiting for the pairs' sums",
+    92: "state space in chunks: the producer or the columns waiting for the outputs to have been read",
+    93: "state space in chunks: the outputs waiting for the columns",
     51: "float32 prompt attention: the producer waiting for a free stage of keys",
     52: "float32 prompt attention: the producer waiting for a free stage of values",
     53: "float32 prompt attention: the MMA warp waiting for a page's keys",

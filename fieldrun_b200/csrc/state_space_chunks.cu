@@ -1,32 +1,33 @@
-// The state-space scan of scans.cu for prompts, in chunks of 128 tokens that run side by side.  Per head, with one decay a token
-// and B, C shared by the heads of a group:
+// The state-space scan of scans.cu for prompts, in chunks of 64 tokens.  Per head, with one decay a token and B, C shared by the heads of
+// a group:
 //
 //     S <- a_t S + B_t (dt_t x_t)^T,   y_t = S^T C_t + D x_t,   a_t = exp(-exp(A_log) dt_t)          (S is [N, vdim])
 //
-// With w(j, i) the product of the decays of tokens j + 1 .. i of a chunk:
-//   1. per chunk and group the products C_i . B_j of its pairs j <= i, for all heads of the group;
-//   2. per chunk, 128 columns of the group's heads at a time: the chunk's own contribution U = sum_j B_j (w(j, end) dt_j x_j)^T;
-//   3. along the chunks: the state at each chunk's start over U's place, and the sequence's new state;
-//   4. per chunk and head: y_i = w(start, i) (S^T C_i) + sum_(j <= i) w(j, i) (C_i . B_j) (dt_j x_j), then D x and the gate.
+// With w(j, i) the product of the decays of tokens j + 1 .. i of a chunk and u_j = dt_j x_j:
+//   1. per chunk and group: the products C_i . B_j of its pairs j <= i, for all heads of the group, and the rows of B and C as parts;
+//   2. per chunk and head: the decays, the pairs' weights P_ij = w(j, i) (C_i . B_j) as parts, the tokens' factors;
+//   3. along the chunks, a block a (sequence, 128 columns of a group's values: two heads of 64 or one of 128): the state stays in
+//      registers; y_i = w(start, i) (S^T C_i) + sum_(j <= i) P_ij u_j, S <- w(end) S + sum_j B_j (w(j, end) u_j)^T; then D x and the gate.
 // A weight is the exponential of a sum of logarithms that has its tokens' alone, or a product of such factors: never a quotient, and no
 // difference of two sums either, which behind one strong decay would have lost the digits of the mild ones.  The sums run over up to 16
-// tokens inside a block, 112 between blocks and 127 to the chunk's end: a rounding of their logarithms, which are large only where the
-// weight is small.
+// tokens inside a block and 48 between blocks: a rounding of their logarithms, which are large only where the weight is small.
 //
-// Everything is float32; the products run on tensor cores with each operand as two TF32 parts (tf32_parts.cuh), over inner sizes
-// of at most 256 entries, added in float32 registers every 16 (launches 1 and 2: every 8).  Four prompts of 2,048 tokens, 64 heads of
-// 128 x 64 in 8 groups: 0.68 ms (about 0.05 + 0.19 + 0.06 + 0.38 for the launches in turn; scans.cu token by token 1.21 ms).  What bounds
-// them: launch 4 issues on half of the cycles, a third of its instructions the operands' parts, and keeps the tensor cores busy for
-// 39 %.
+// Everything is float32; launch 1's products run on mma.sync in TF32 parts (tf32_parts.cuh), sums of 16 entries, added in float32
+// registers; launch 3's on tcgen05 in float16 parts (f16_parts.cuh), over at most 128 entries.
+// Four prompts of 2,048 tokens, 64 heads of 128 x 64 in 8 groups: 44 + 45 + 179 us, against 676 us of four launches on mma.sync with a
+// state written and read for every chunk of 128 tokens (states 189, chain 65, outputs 382, pairs 40), and 1,210 token by token.
+#include "f16_parts.cuh"
 #include "tf32_parts.cuh"
 
-#define SC_TOKENS 128
+#define SC_CHUNK 128          // tokens of the callers' chunks: two of this file's
+#define SC_TOKENS 64
 #define SC_BLOCK 16
 #define SC_BLOCKS (SC_TOKENS / SC_BLOCK)
-#define SC_THREADS 256
-#define SC_COLUMNS 128        // columns of U a block of launch 2 takes
-#define SC_LC (64 + 8)        // rows of 64 entries of the inner size, read along
-#define SC_SLICE 64           // value columns a block of launch 4 takes
+#define SC_COLUMNS 128        // value columns of a block of launch 3
+#define SC_FACTORS (4 * SC_TOKENS + 4)
+
+using namespace frb_tma;
+using namespace frb_tc;
 
 struct StateSpaceChunks {
     const float* proj;       // [T, proj_stride]: z of channel j at z_offset + j, dt of head h at dt_offset + h
@@ -36,260 +37,131 @@ struct StateSpaceChunks {
     float* state;            // [slots][2][copy_floats], this part's [heads][N][vdim] at state_offset
     long long copy_floats, state_offset;
     float* out;              // [T, heads * vdim]
-    float* states;           // [chunks][heads][N][vdim]
-    float* decays;           // [chunks][heads]
-    float* pairs;            // [chunks][groups][SC_TOKENS][SC_TOKENS]
+    // of every half of a caller's chunk (a chunk here)
+    uint16_t *c_parts, *b_parts;     // [chunk][group][part][N / 64][SC_TOKENS][64]: C's rows with a scale each, B's with one for the chunk
+    uint16_t* pair_parts;    // [chunk][columns / 128][part][head of the columns][SC_TOKENS][SC_TOKENS]: P's rows with a scale each
+    float* raw_pairs;        // [chunk][group][SC_TOKENS][SC_TOKENS]: C_i . B_j, j <= i
+    float* scales;           // [chunk][group][SC_TOKENS + 4]: what takes the scales of C's rows off, and that of B (a NaN: no parts serve)
+    float* factors;          // [chunk][head][SC_FACTORS]: w(start, i) and C's scale off; P's scales off; w(j, end); dt_j; w(end), B's scale off
     int proj_stride, z_offset, dt_offset, xbc_stride, b_offset, c_offset, heads, vdim, N, groups;
+
+    __device__ __forceinline__ int tokens_of(int chunk) const {          // 0 or less: none
+        const int item = chunk >> 1;
+        return min(SC_TOKENS, chunk_end[item] - chunk_begin[item] - (chunk & 1) * SC_TOKENS);
+    }
+    __device__ __forceinline__ size_t row_of(int chunk) const {
+        const int item = chunk >> 1;
+        return (size_t)cu_q_len[chunk_seq[item]] + chunk_begin[item] + (chunk & 1) * SC_TOKENS;
+    }
 };
 
 __device__ __forceinline__ float sc_softplus(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
 
-// `count` rows of WIDTH floats on their way into rows `ld` apart; zeros in the rows up to `most`.
-template <int WIDTH>
-__device__ __forceinline__ void sc_copy_rows(float* to, int ld, const float* from, int stride, int count, int most) {
-#pragma unroll 4
-    for (int i = threadIdx.x; i < most * (WIDTH / 4); i += SC_THREADS) {
-        const int t = i / (WIDTH / 4), u = i % (WIDTH / 4);
-        if (t < count) copy16_async(to + t * ld + 4 * u, from + (size_t)t * stride + 4 * u);
-        else *(float4*)(to + t * ld + 4 * u) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-}
-
-// Launch 1.  grid (chunk, group).  A warp takes row tiles a and 7 - a (the same number of earlier tokens for every a) and every
-// other eight columns.
-__global__ void __launch_bounds__(SC_THREADS, 2) state_space_pairs_kernel(StateSpaceChunks p) {
-    extern __shared__ float4 sc_smem[];
-    float* c_s = (float*)sc_smem;                   // [SC_TOKENS][SC_LC]
-    float* b_s = c_s + SC_TOKENS * SC_LC;           // [SC_TOKENS][SC_LC]
-    const int item = blockIdx.x, g = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int b = p.chunk_seq[item], count = p.chunk_end[item] - p.chunk_begin[item];
-    const float* rows = p.xbc + ((size_t)p.cu_q_len[b] + p.chunk_begin[item]) * p.xbc_stride;
-    const int tiles[2] = {warp & 3, 7 - (warp & 3)}, odd = warp >> 2;
-    float acc[2][SC_BLOCKS][4] = {};
-    for (int n0 = 0; n0 < p.N; n0 += 64) {
-        __syncthreads();
-        sc_copy_rows<64>(c_s, SC_LC, rows + p.c_offset + g * p.N + n0, p.xbc_stride, count, SC_TOKENS);
-        sc_copy_rows<64>(b_s, SC_LC, rows + p.b_offset + g * p.N + n0, p.xbc_stride, count, SC_TOKENS);
-        copies_commit();
-        copies_wait<0>();
-        __syncthreads();
-#pragma unroll 2
-        for (int k = 0; k < 64; k += 8) {
-            Tf32Parts a[2][1][1][4], bb[1][1][2];
+// z / (1 + exp(-z)), of sixteen z.  Below 80 the divisor and its reciprocal are far from the ends of float32: there an approximate reciprocal
+// serves, and the quotient's residual, which fma() has exactly, corrects it (Markstein, IBM Journal of Research and Development 34,
+// 1990): the bits of the division at 4 x 10^6 places of each of nine ranges up to 80.  A division's own branch lets no other work in between: with one for each z launch 3 was bound by these, at 196 us.
+__device__ __forceinline__ void sc_silu(float (&z)[16]) {
+    float top = 0.f;
 #pragma unroll
-            for (int m = 0; m < 2; ++m) a_along(a[m][0][0], c_s + tiles[m] * SC_BLOCK * SC_LC + k, SC_LC, lane);
+    for (int i = 0; i < 16; ++i) top = fmaxf(top, fabsf(z[i]));
+    if (top < 80.f) {
 #pragma unroll
-            for (int n = 0; n < SC_BLOCKS; ++n) {                        // n: the 16 columns of block n, this warp's half of them
-                if (n > tiles[0] && n > tiles[1]) break;
-                b_along(bb[0][0], b_s + (n * SC_BLOCK + 8 * odd) * SC_LC + k, SC_LC, lane);
-#pragma unroll
-                for (int m = 0; m < 2; ++m)
-                    if (n <= tiles[m]) {
-                        float t[1][1][4];
-                        mma_runs(t, a[m], bb);
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) acc[m][n][e] += t[0][0][e];
-                    }
-            }
+        for (int i = 0; i < 16; ++i) {
+            const float d = 1.0f + expf(-z[i]);
+            float r;
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+            const float q = z[i] * r;
+            z[i] = fmaf(fmaf(-q, d, z[i]), r, q);
         }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) z[i] = z[i] / (1.0f + expf(-z[i]));
     }
-    if (!all_finite(acc)) {
-#pragma unroll
-        for (int m = 0; m < 2; ++m)
-#pragma unroll
-            for (int n = 0; n < SC_BLOCKS; ++n)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int i = tiles[m] * SC_BLOCK + (lane >> 2) + 8 * (e >> 1), j = n * SC_BLOCK + 8 * odd + 2 * (lane & 3) + (e & 1);
-                    if (j <= i && i < count && !is_finite(acc[m][n][e]))
-                        acc[m][n][e] = sum_entry_by_entry(rows + (size_t)i * p.xbc_stride + p.c_offset + g * p.N, 1,
-                                                          rows + (size_t)j * p.xbc_stride + p.b_offset + g * p.N, 1, nullptr, p.N);
-                }
-    }
-    float* out = p.pairs + ((size_t)item * p.groups + g) * SC_TOKENS * SC_TOKENS;
-#pragma unroll
-    for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int n = 0; n < SC_BLOCKS; ++n)
-            if (n <= tiles[m]) {
-                float* to = out + (tiles[m] * SC_BLOCK + (lane >> 2)) * SC_TOKENS + n * SC_BLOCK + 8 * odd + 2 * (lane & 3);
-                *(float2*)to = make_float2(acc[m][n][0], acc[m][n][1]);
-                *(float2*)(to + 8 * SC_TOKENS) = make_float2(acc[m][n][2], acc[m][n][3]);
-            }
 }
 
-// Launch 2.  grid (chunk, tile of 128 columns of the heads' values).  A warp takes 32 rows (64 with N = 64: two warps a row tile
-// less) by 64 columns of U.
+// Launch 1.  grid (chunk, group).  A warp takes a row tile of 16 and every other eight columns of the blocks up to it.
 template <int N>
-__global__ void __launch_bounds__(SC_THREADS, 2) state_space_states_kernel(StateSpaceChunks p) {
-    constexpr int LB = N + 4, LX = SC_COLUMNS + 4, PART = 32;            // tokens of a part; two parts in turn
+__global__ void __launch_bounds__(256, 2) state_space_pairs_kernel(StateSpaceChunks p) {
+    constexpr int LC = N + 8, UNITS = SC_TOKENS * N / 8;
     extern __shared__ float4 sc_smem[];
-    __shared__ float factor[2][SC_TOKENS], warp_sums[2][SC_TOKENS / 32];
-    float* parts = (float*)sc_smem;                 // [2]: B [PART][LB], x [PART][LX]
-    const int item = blockIdx.x, column0 = blockIdx.y * SC_COLUMNS, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int b = p.chunk_seq[item], count = p.chunk_end[item] - p.chunk_begin[item];
-    const size_t row0 = (size_t)p.cu_q_len[b] + p.chunk_begin[item];
-    const float* rows = p.xbc + row0 * p.xbc_stride;
-    const int heads_here = p.vdim >= SC_COLUMNS ? 1 : 2, head0 = column0 / p.vdim, g = head0 / (p.heads / p.groups);
-
-    auto copy_part = [&](int part) {
-        float* b_s = parts + (part & 1) * PART * (LB + LX);
-        const float* at = rows + (size_t)(part * PART) * p.xbc_stride;
-        const int left = count - part * PART;
-        sc_copy_rows<N>(b_s, LB, at + p.b_offset + g * N, p.xbc_stride, left, PART);
-        sc_copy_rows<SC_COLUMNS>(b_s + PART * LB, LX, at + column0, p.xbc_stride, left, PART);
-        copies_commit();
-    };
-    copy_part(0);
-
-    // a thread a (head, token): the step times the decays behind it, to the chunk's end
-    {
-        const int hh = tid / SC_TOKENS, t = tid % SC_TOKENS, h = head0 + hh;
-        const bool in = hh < heads_here && t < count;
-        const float step = in ? sc_softplus(p.proj[(row0 + t) * p.proj_stride + p.dt_offset + h] + p.dt_bias[h]) : 0.f;
-        const float la = in ? -expf(p.a_log[h]) * step : 0.f;
-        float sum = la;                              // of this token and those behind it in the warp
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const float other = __shfl_down_sync(0xffffffffu, sum, o);
-            if (lane + o < 32) sum += other;
-        }
-        float tail = __shfl_down_sync(0xffffffffu, sum, 1);
-        if (lane == 31) tail = 0.f;
-        if (lane == 0) warp_sums[hh][warp % (SC_TOKENS / 32)] = sum;
-        __syncthreads();
-        for (int w = t / 32 + 1; w < SC_TOKENS / 32; ++w) tail += warp_sums[hh][w];
-        factor[hh][t] = step * expf(tail);
-        if (t == 0 && hh < heads_here && column0 % p.vdim == 0) p.decays[(size_t)item * p.heads + h] = expf(la + tail);
+    __shared__ float c_top[SC_TOKENS], b_top[SC_TOKENS];
+    float* c_s = (float*)sc_smem;                   // [SC_TOKENS][LC]
+    float* b_s = c_s + SC_TOKENS * LC;              // [SC_TOKENS][LC]
+    const int chunk = blockIdx.x, g = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, count = p.tokens_of(chunk);
+    const float* rows = p.xbc + p.row_of(chunk) * p.xbc_stride;
+    const size_t at = (size_t)chunk * p.groups + g;
+    for (int i = tid; i < 2 * SC_TOKENS * (N / 4); i += 256) {
+        const int t = i / (N / 4) % SC_TOKENS, u = i % (N / 4);
+        const bool is_b = i >= SC_TOKENS * (N / 4);
+        float* to = (is_b ? b_s : c_s) + t * LC + 4 * u;
+        if (t < count) copy16_async(to, rows + (size_t)t * p.xbc_stride + (is_b ? p.b_offset : p.c_offset) + g * N + 4 * u);
+        else *(float4*)to = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-
-    constexpr int ROW_TILES = N / 32;                // 4 or 2 runs of 32 rows
-    const int c0 = warp % ROW_TILES * 32, wide = SC_COLUMNS / (SC_THREADS / 32 / ROW_TILES), v0 = warp / ROW_TILES * wide;
-    constexpr int NT = SC_COLUMNS / (SC_THREADS / 32 / ROW_TILES) / 8;
-    float acc[2][NT][4] = {};
-    for (int part = 0; part * PART < count; ++part) {
-        const float* b_s = parts + (part & 1) * PART * (LB + LX);
-        float* x_s = parts + (part & 1) * PART * (LB + LX) + PART * LB;
-        copies_wait<0>();
-        __syncthreads();                             // this part is there, and nobody reads the other one any more
-        if ((part + 1) * PART < count) copy_part(part + 1);
+    copies_commit();
+    copies_wait<0>();
+    __syncthreads();
+    for (int t = warp; t < 2 * SC_TOKENS; t += 8) {
+        const float* row = (t < SC_TOKENS ? c_s : b_s) + t % SC_TOKENS * LC;
+        float top = 0.f;
 #pragma unroll
-        for (int i = tid; i < PART * SC_COLUMNS / 4; i += SC_THREADS) {
-            const int t = i / (SC_COLUMNS / 4), u = i % (SC_COLUMNS / 4);
-            const float f = factor[heads_here == 2 ? 4 * u / SC_SLICE : 0][part * PART + t];
-            float4* at = (float4*)(x_s + t * LX + 4 * u);
-            float4 x = *at;
-            x.x *= f; x.y *= f; x.z *= f; x.w *= f;
-            *at = x;
-        }
-        __syncthreads();
+        for (int n = 0; n < N; n += 32) top = fmaxf(top, fabsf(row[n + lane]));
+        top = warp_max(top);
+        if (lane == 0) (t < SC_TOKENS ? c_top : b_top)[t % SC_TOKENS] = top;
+    }
+    __syncthreads();
+    // one scale for B: a row far larger than another would cost that one its digits
+    const float b0 = b_top[lane], b1 = b_top[lane + 32], large = warp_max(fmaxf(b0, b1));
+    const float least = -warp_max(-fminf(b0 > 0.f ? b0 : INFINITY, b1 > 0.f ? b1 : INFINITY));
+    const int b_exponent = parts_exponent(large);
+    if (tid < SC_TOKENS) p.scales[at * (SC_TOKENS + 4) + tid] = power_of_two(-parts_exponent(c_top[tid]));
+    if (tid == 0) p.scales[at * (SC_TOKENS + 4) + SC_TOKENS] = least * 67108864.f < large ? NAN : power_of_two(-b_exponent);          // 2^26
+    for (int u = tid; u < 2 * UNITS; u += 256) {
+        const bool is_b = u >= UNITS;
+        const int r = u % UNITS / (N / 8), c = u % (N / 8) * 8;
+        const float* from = (is_b ? b_s : c_s) + r * LC + c;
+        const float scale = power_of_two(is_b ? b_exponent : parts_exponent(c_top[r]));
+        uint4 hi, lo;
+        split_four(*(const float4*)from, scale, hi.x, hi.y, lo.x, lo.y);
+        split_four(*(const float4*)(from + 4), scale, hi.z, hi.w, lo.z, lo.w);
+        uint16_t* parts = (is_b ? p.b_parts : p.c_parts) + at * 2 * SC_TOKENS * N + piece_place(r, c);
+        *(uint4*)parts = hi;
+        *(uint4*)(parts + SC_TOKENS * N) = lo;
+    }
+    const int tile = warp & 3, odd = warp >> 2;
+    float acc[SC_BLOCKS][4] = {};
 #pragma unroll 2
-        for (int j = 0; j < PART; j += 8) {
-            Tf32Parts a[1][2][4];
+    for (int k = 0; k < N; k += 16) {
+        Tf32Parts a[2][1][4], bb[2][1][2];
 #pragma unroll
-            for (int m = 0; m < 2; ++m) a_down(a[0][m], b_s + j * LB + c0 + 16 * m, LB, lane);
-            add_runs<2>(acc, a, [&](Tf32Parts (&b)[2], int, int n) { b_down(b, x_s + j * LX + v0 + 8 * n, LX, lane); });
+        for (int r = 0; r < 2; ++r) a_along(a[r][0], c_s + tile * SC_BLOCK * LC + k + 8 * r, LC, lane);
+#pragma unroll
+        for (int n = 0; n < SC_BLOCKS; ++n) {
+            if (n > tile) break;
+#pragma unroll
+            for (int r = 0; r < 2; ++r) b_along(bb[r][0], b_s + (n * SC_BLOCK + 8 * odd) * LC + k + 8 * r, LC, lane);
+            float t[1][1][4];
+            mma_runs(t, a, bb);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[n][e] += t[0][0][e];
         }
     }
-    if (!all_finite(acc)) {
+    float* out = p.raw_pairs + at * SC_TOKENS * SC_TOKENS + (tile * SC_BLOCK + (lane >> 2)) * SC_TOKENS + 8 * odd + 2 * (lane & 3);
 #pragma unroll
-        for (int n = 0; n < NT; ++n)
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (!is_finite(acc[m][n][e])) {
-                        const int column = v0 + 8 * n + 2 * (lane & 3) + (e & 1);
-                        acc[m][n][e] = sum_entry_by_entry(rows + p.b_offset + g * N + c0 + 16 * m + (lane >> 2) + 8 * (e >> 1), p.xbc_stride,
-                                                          rows + column0 + column, p.xbc_stride, factor[heads_here == 2 ? column / SC_SLICE : 0],
-                                                          count);
-                    }
-    }
-#pragma unroll
-    for (int n = 0; n < NT; ++n) {
-        const int column = column0 + v0 + 8 * n, h = column / p.vdim;
-        float* out = p.states + ((size_t)item * p.heads + h) * N * p.vdim + column - h * p.vdim + 2 * (lane & 3);
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            float* to = out + (size_t)(c0 + 16 * m + (lane >> 2)) * p.vdim;
-            *(float2*)to = make_float2(acc[m][n][0], acc[m][n][1]);
-            *(float2*)(to + 8 * (size_t)p.vdim) = make_float2(acc[m][n][2], acc[m][n][3]);
+    for (int n = 0; n < SC_BLOCKS; ++n)
+        if (n <= tile) {
+            *(float2*)(out + n * SC_BLOCK) = make_float2(acc[n][0], acc[n][1]);
+            *(float2*)(out + n * SC_BLOCK + 8 * SC_TOKENS) = make_float2(acc[n][2], acc[n][3]);
         }
-    }
 }
 
-// Launch 3.  grid (sequence, head, runs of 1,024 state elements): bound by reading and writing U's place once.
-__global__ void __launch_bounds__(256) state_space_chain_kernel(StateSpaceChunks p) {
-    const int b = blockIdx.x, h = blockIdx.y, e = (blockIdx.z * 256 + threadIdx.x) * 4, elements = p.N * p.vdim;
-    if (e >= elements) return;
-    const int first = p.seq_chunk0[b], last = p.seq_chunk0[b + 1], start = p.seq_start[b], n = p.cu_q_len[b + 1] - p.cu_q_len[b];
-    float* kept = p.state + (size_t)p.seq_slot[b] * 2 * p.copy_floats + p.state_offset + (size_t)h * elements + e;
-    float4 S = *(const float4*)(kept + (start & 1) * p.copy_floats);
-    for (int s0 = first; s0 < last; s0 += 8) {                  // eight chunks' loads on their way at once
-        float4 u[8];
-        float decay[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            if (s0 + i < last) {
-                const size_t at = (size_t)(s0 + i) * p.heads + h;
-                u[i] = *(const float4*)(p.states + at * elements + e);
-                decay[i] = p.decays[at];
-            }
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            if (s0 + i < last) {
-                *(float4*)(p.states + ((size_t)(s0 + i) * p.heads + h) * elements + e) = S;
-                S.x = fmaf(decay[i], S.x, u[i].x);
-                S.y = fmaf(decay[i], S.y, u[i].y);
-                S.z = fmaf(decay[i], S.z, u[i].z);
-                S.w = fmaf(decay[i], S.w, u[i].w);
-            }
-    }
-    *(float4*)(kept + ((start + n) & 1) * p.copy_floats) = S;
-}
-
-// w(j, i) of a chunk's pairs.
-struct ChunkWeights {
-    float to[SC_TOKENS], from[SC_TOKENS], start[SC_TOKENS];              // from its block's start, to its block's end, from the chunk's start
-    float between[SC_BLOCKS][SC_BLOCKS];                                 // the whole blocks between two
-    __align__(16) float own[SC_TOKENS][SC_BLOCK + 8];                    // with the tokens of its block; zero for later ones
-
-    __device__ __forceinline__ float of(int j, int i) const {
-        const int bi = i / SC_BLOCK, bj = j / SC_BLOCK;
-        return bj < bi ? to[i] * (between[bi][bj] * from[j]) : own[i][j % SC_BLOCK];
-    }
-};
-
-// A token's output from the state at the chunk's start and the tokens up to it: sum_n C_n S_n w(start, i) + sum_(j <= i) w(j, i) pair_j x_j.
-static __device__ __noinline__ float output_entry_by_entry(const ChunkWeights& w, int i, const float* c, const float* state, int vdim, int N,
-                                                           const float* pairs, const float* x, int ld) {
-    float sum = sum_entry_by_entry(c, 1, state, vdim, nullptr, N) * w.start[i];
-    for (int j = 0; j <= i; ++j) sum = fmaf(pairs[j] * w.of(j, i), x[j * ld], sum);
-    return sum;
-}
-
-// Launch 4.  grid (chunk, head, slice of 64 value columns).  A warp takes row tiles a and 7 - a by 32 columns.
-__global__ void __launch_bounds__(SC_THREADS, 2) state_space_outputs_kernel(StateSpaceChunks p) {
-    constexpr int LV = SC_SLICE + 4;
-    extern __shared__ float4 sc_smem[];
-    __shared__ float step_s[SC_TOKENS], log_s[SC_TOKENS], block_log[SC_BLOCKS];
-    __shared__ ChunkWeights weights;
-    constexpr int PART = 32, LP = PART + 8;         // state rows of a part; two parts in turn
-    float* parts = (float*)sc_smem;                 // [2]: C [SC_TOKENS][LP], S [PART][LV]
-    float* x_s = parts + 2 * (SC_TOKENS * LP + PART * LV);               // [SC_TOKENS][LV]
-    const int item = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, column0 = blockIdx.z * SC_SLICE;
-    const int b = p.chunk_seq[item], count = p.chunk_end[item] - p.chunk_begin[item], g = h / (p.heads / p.groups);
-    const size_t row0 = (size_t)p.cu_q_len[b] + p.chunk_begin[item];
-    const float* rows = p.xbc + row0 * p.xbc_stride;
-    const float* state = p.states + ((size_t)item * p.heads + h) * p.N * p.vdim + column0;
-    auto copy_part = [&](int part) {
-        float* c_s = parts + (part & 1) * (SC_TOKENS * LP + PART * LV);
-        sc_copy_rows<PART>(c_s, LP, rows + p.c_offset + g * p.N + part * PART, p.xbc_stride, count, SC_TOKENS);
-        sc_copy_rows<SC_SLICE>(c_s + SC_TOKENS * LP, LV, state + (size_t)(part * PART) * p.vdim, p.vdim, PART, PART);
-        copies_commit();
-    };
-    copy_part(0);
-
+// Launch 2.  grid (chunk, head), 128 threads: bound by reading the group's pairs and writing the head's parts once.
+__global__ void __launch_bounds__(128) state_space_weights_kernel(StateSpaceChunks p) {
+    __shared__ float log_s[SC_TOKENS], to_s[SC_TOKENS], from_s[SC_TOKENS], step_s[SC_TOKENS];
+    __shared__ float block_log[SC_BLOCKS], between[SC_BLOCKS][SC_BLOCKS];
+    __shared__ __align__(16) float own[SC_TOKENS][SC_BLOCK + 4];         // w(j, i) of the tokens j of i's block; zero for later ones
+    const int chunk = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, g = h / (p.heads / p.groups), count = p.tokens_of(chunk);
+    const size_t row0 = p.row_of(chunk);
+    float* factors = p.factors + ((size_t)chunk * p.heads + h) * SC_FACTORS;
     // a token a thread: its step; the logarithms of the decays from its block's start (with its own) and to its block's end
     if (tid < SC_TOKENS) {
         const bool in = tid < count;
@@ -306,8 +178,8 @@ __global__ void __launch_bounds__(SC_THREADS, 2) state_space_outputs_kernel(Stat
         if (tid % SC_BLOCK == SC_BLOCK - 1) { tail = 0.f; block_log[tid / SC_BLOCK] = before; }
         step_s[tid] = step;
         log_s[tid] = la;
-        weights.to[tid] = expf(before);
-        weights.from[tid] = expf(tail);
+        to_s[tid] = expf(before);
+        from_s[tid] = expf(tail);
     }
     __syncthreads();
     if (tid < SC_TOKENS) {                           // a token's weights in its block: the sums begin anew for each, at the token itself
@@ -319,182 +191,473 @@ __global__ void __launch_bounds__(SC_THREADS, 2) state_space_outputs_kernel(Stat
             if (j <= i) sum += log_s[tid - i + j];
         }
 #pragma unroll
-        for (int j = 0; j < SC_BLOCK; j += 4) *(float4*)&weights.own[tid][j] = make_float4(row[j], row[j + 1], row[j + 2], row[j + 3]);
+        for (int j = 0; j < SC_BLOCK; j += 4) *(float4*)&own[tid][j] = make_float4(row[j], row[j + 1], row[j + 2], row[j + 3]);
     } else {
         const int t = tid - SC_TOKENS;
-        float sum = 0.f;
-        for (int m = 0; m < t / SC_BLOCK; ++m) sum += block_log[m];
-        weights.start[t] = expf(sum) * weights.to[t];
-        if (t < SC_BLOCKS * SC_BLOCKS) {
+        if (t < SC_BLOCKS * SC_BLOCKS) {             // the whole blocks between two
             const int i = t / SC_BLOCKS, j = t % SC_BLOCKS;
-            sum = 0.f;
+            float sum = 0.f;
             for (int m = j + 1; m < i; ++m) sum += block_log[m];
-            weights.between[i][j] = expf(sum);
+            between[i][j] = expf(sum);
         }
-    }
-
-    const int tiles[2] = {warp & 3, 7 - (warp & 3)}, v0 = (warp >> 2) * 32;
-    float acc[2][4][4] = {};
-    const int last = p.N / PART - 1;
-    for (int part = 0; part <= last; ++part) {
-        copies_wait<0>();
-        __syncthreads();                             // this part is there, and nobody reads the other one any more
-        if (part < last) {
-            copy_part(part + 1);
-        } else {                                     // behind the last part: the values
-            sc_copy_rows<SC_SLICE>(x_s, LV, rows + h * p.vdim + column0, p.xbc_stride, count, SC_TOKENS);
-            copies_commit();
+        float sum = 0.f, rest = 0.f;
+        for (int m = 0; m < t / SC_BLOCK; ++m) sum += block_log[m];
+        for (int m = t / SC_BLOCK + 1; m < SC_BLOCKS; ++m) rest += block_log[m];
+        const float* scales = p.scales + ((size_t)chunk * p.groups + g) * (SC_TOKENS + 4);
+        const float start = expf(sum) * to_s[t];
+        factors[t] = start * scales[t];
+        factors[2 * SC_TOKENS + t] = from_s[t] * expf(rest);
+        factors[3 * SC_TOKENS + t] = step_s[t];
+        if (t == SC_TOKENS - 1) {
+            factors[4 * SC_TOKENS] = start;
+            factors[4 * SC_TOKENS + 1] = scales[SC_TOKENS];
         }
-        const float* c_s = parts + (part & 1) * (SC_TOKENS * LP + PART * LV);
-        const float* s_s = c_s + SC_TOKENS * LP;
-#pragma unroll 1
-        for (int k = 0; k < PART; k += 16) {
-            Tf32Parts a[2][2][4];
-#pragma unroll
-            for (int r = 0; r < 2; ++r)
-#pragma unroll
-                for (int m = 0; m < 2; ++m) a_along(a[r][m], c_s + tiles[m] * SC_BLOCK * LP + k + 8 * r, LP, lane);
-            add_runs<2>(acc, a, [&](Tf32Parts (&b)[2], int r, int n) { b_down(b, s_s + (k + 8 * r) * LV + v0 + 8 * n, LV, lane); });
-        }
-    }
-    copies_wait<0>();
-    __syncthreads();
-    for (int i = tid; i < SC_TOKENS * SC_SLICE / 4; i += SC_THREADS) {
-        const int t = i / (SC_SLICE / 4), u = i % (SC_SLICE / 4);
-        const float f = step_s[t];
-        float4* at = (float4*)(x_s + t * LV + 4 * u);
-        float4 x = *at;
-        x.x *= f; x.y *= f; x.z *= f; x.w *= f;
-        *at = x;
     }
     __syncthreads();
-    const float* pairs = p.pairs + ((size_t)item * p.groups + g) * SC_TOKENS * SC_TOKENS;
+    // eight entries of a row of P at a time; eight neighbouring threads have a row
+    const int heads_here = SC_COLUMNS / p.vdim;
+    const float* raw = p.raw_pairs + ((size_t)chunk * p.groups + g) * SC_TOKENS * SC_TOKENS;
+    uint16_t* parts = p.pair_parts + ((size_t)chunk * (p.heads / heads_here) + h / heads_here) * 2 * heads_here * SC_TOKENS * SC_TOKENS
+                      + (h % heads_here) * SC_TOKENS * SC_TOKENS;
 #pragma unroll
-    for (int m = 0; m < 2; ++m) {
-        const int bi = tiles[m], i0 = bi * SC_BLOCK + (lane >> 2), i1 = i0 + 8;
-        const float e0 = weights.start[i0], e1 = weights.start[i1];
+    for (int u = tid; u < SC_TOKENS * SC_TOKENS / 8; u += 128) {
+        const int i = u / (SC_TOKENS / 8), j0 = u % (SC_TOKENS / 8) * 8, ib = i / SC_BLOCK, jb = j0 / SC_BLOCK;
+        float y[8] = {}, top = 0.f;
+        if (j0 <= i) {
+            const float4 a = *(const float4*)(raw + i * SC_TOKENS + j0), c = *(const float4*)(raw + i * SC_TOKENS + j0 + 4);
+            const float r[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
 #pragma unroll
-        for (int n = 0; n < 4; ++n) {
-            acc[m][n][0] *= e0;
-            acc[m][n][1] *= e0;
-            acc[m][n][2] *= e1;
-            acc[m][n][3] *= e1;
-        }
-        const float* at = pairs + i0 * SC_TOKENS + 2 * (lane & 3);
-        const float f0 = weights.to[i0], f1 = weights.to[i1];
-        const int end = (bi + 1) * SC_BLOCK;
-        float2 x_next[2], y_next[2];                 // the pairs of a block's 16 columns, asked for a block ahead
-#pragma unroll
-        for (int q = 0; q < 2; ++q) { x_next[q] = *(const float2*)(at + 8 * q); y_next[q] = *(const float2*)(at + 8 * SC_TOKENS + 8 * q); }
-        for (int block0 = 0; block0 < end; block0 += SC_BLOCK) {
-          const float2 xs[2] = {x_next[0], x_next[1]}, ys[2] = {y_next[0], y_next[1]};
-          if (block0 + SC_BLOCK < end)
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                x_next[q] = *(const float2*)(at + block0 + SC_BLOCK + 8 * q);
-                y_next[q] = *(const float2*)(at + 8 * SC_TOKENS + block0 + SC_BLOCK + 8 * q);
-            }
-          Tf32Parts a[2][1][4];
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const int j = block0 + 8 * q + 2 * (lane & 3), bj = block0 / SC_BLOCK;
-            const float2 x = xs[q], y = ys[q];
-            float x0, x1, y0, y1;
-            if (bj < bi) {
-                const float both = weights.between[bi][bj], u = both * weights.from[j], v = both * weights.from[j + 1];
-                x0 = x.x * (f0 * u); x1 = x.y * (f0 * v); y0 = y.x * (f1 * u); y1 = y.y * (f1 * v);
-            } else {
-                const float2 wx = *(const float2*)&weights.own[i0][j - block0], wy = *(const float2*)&weights.own[i1][j - block0];
-                x0 = j <= i0 ? x.x * wx.x : 0.f;
-                x1 = j + 1 <= i0 ? x.y * wx.y : 0.f;
-                y0 = j <= i1 ? y.x * wy.x : 0.f;
-                y1 = j + 1 <= i1 ? y.y * wy.y : 0.f;
-            }
-            a[q][0][0] = tf32_parts(x0);
-            a[q][0][1] = tf32_parts(y0);
-            a[q][0][2] = tf32_parts(x1);
-            a[q][0][3] = tf32_parts(y1);
-          }
-          add_runs<4>(reinterpret_cast<float (&)[1][4][4]>(acc[m]), a,
-                                  [&](Tf32Parts (&b)[2], int q, int n) { b_down(b, x_s + (block0 + 8 * q) * LV + v0 + 8 * n, LV, lane); });
-        }
-    }
-    // a token's output has the tokens up to it alone: where an infinity or a NaN of the block behind it came in with a weight of zero, the
-    // output is added again
-    if (!all_finite(acc)) {
-#pragma unroll
-        for (int m = 0; m < 2; ++m)
-#pragma unroll
-            for (int n = 0; n < 4; ++n)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int t = tiles[m] * SC_BLOCK + 8 * (e >> 1) + (lane >> 2), v = v0 + 8 * n + 2 * (lane & 3) + (e & 1);
-                    if (t < count && !is_finite(acc[m][n][e]))
-                        acc[m][n][e] = output_entry_by_entry(weights, t, rows + (size_t)t * p.xbc_stride + p.c_offset + g * p.N, state + v, p.vdim,
-                                                             p.N, pairs + t * SC_TOKENS, x_s + v, LV);
+            for (int e = 0; e < 8; ++e)
+                if (j0 + e <= i) {
+                    y[e] = r[e] * (jb < ib ? to_s[i] * (between[ib][jb] * from_s[j0 + e]) : own[i][(j0 + e) % SC_BLOCK]);
+                    top = fmaxf(top, fabsf(y[e]));
                 }
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        const int exponent = parts_exponent(top);
+        if (j0 == 0) factors[SC_TOKENS + i] = power_of_two(-exponent);
+        uint4 hi, lo;
+        split_four(make_float4(y[0], y[1], y[2], y[3]), power_of_two(exponent), hi.x, hi.y, lo.x, lo.y);
+        split_four(make_float4(y[4], y[5], y[6], y[7]), power_of_two(exponent), hi.z, hi.w, lo.z, lo.w);
+        uint16_t* to = parts + piece_place(i, j0);
+        *(uint4*)to = hi;
+        *(uint4*)(to + heads_here * SC_TOKENS * SC_TOKENS) = lo;
     }
-    const float dskip = p.d[h];
+}
+
+// Launch 3.  grid (sequence, columns / 128): a lane of tensor memory is a value column; two threads have half of its N state entries
+// each, in float32, and half of a chunk's tokens.  The products of parts of a chunk:
+//     DS = (u w(j, end))^T B   128 x N x 64, B's rows N-major;    D1 = S^T C^T   128 x 64 x N;    DO = u^T P^T   128 x 64 x 64, with two heads
+//     128 x 64 x 128: a head's columns have u in their half of the inner size and zeros in the other's.
+// The columns' parts have a power of two of their own each, from the largest entry of the state or of u.  Eight more warps take the
+// outputs through D x and the gate while the next chunk is made: with these in the columns' warps a chunk took 4,000 cycles more.  A chunk is
+// bound by the instructions of both, 9,000 to 10,000 cycles: the columns' splits 1,900, u 1,300, the waits for the products 1,900, the outputs' gates 4,000.  A column with a number that is not finite, or with a token 2^28 times
+// larger than the first of its chunk, or a chunk whose rows of B lie 2^26 apart, makes the block take its columns of the sequence
+// again, token by token.
+#define ST_THREADS 640         // warps 0 copies, 1 products; 4-11 the columns' two halves (w & 3: lanes), 12-19 the outputs
+#define ST_ROWS 256
+#define ST_SHARE_TOKENS (SC_TOKENS / 2)
+// registers a thread: at launch, and of each group of warps after it (their sum over the threads is below the launch's)
+#define ST_REGS_LAUNCH 96
+#define ST_REGS_ISSUE 40
+#define ST_REGS_ROWS 152
+#define ST_REGS_OUTPUTS 64
+static_assert(128 * ST_REGS_ISSUE + ST_ROWS * (ST_REGS_ROWS + ST_REGS_OUTPUTS) <= ST_THREADS * ST_REGS_LAUNCH, "registers of the groups");
+
+// A sequence's columns token by token: 128 threads, one a column; `rows_s`: 2 N floats.
+template <int N>
+static __device__ __noinline__ void st_token_by_token(const StateSpaceChunks& p, int b, int column, int tid, float* rows_s) {
+    float *b_s = rows_s, *c_s = rows_s + N;
+    const int h = column / p.vdim, g = h / (p.heads / p.groups), start = p.seq_start[b], n_tok = p.cu_q_len[b + 1] - p.cu_q_len[b];
+    float* kept = p.state + (size_t)p.seq_slot[b] * 2 * p.copy_floats + p.state_offset + (size_t)h * N * p.vdim + column % p.vdim;
+    auto meet = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };
+    const float rate = expf(p.a_log[h]);
+    float S[N];
 #pragma unroll
-    for (int m = 0; m < 2; ++m)
+    for (int n = 0; n < N; ++n) S[n] = (kept + (start & 1) * p.copy_floats)[(size_t)n * p.vdim];
+    for (int t = 0; t < n_tok; ++t) {
+        const size_t row = (size_t)p.cu_q_len[b] + t;
+        const float *rows = p.xbc + row * p.xbc_stride, *proj = p.proj + row * p.proj_stride;
+        meet();
+        if (tid < N) {
+            b_s[tid] = rows[p.b_offset + g * N + tid];
+            c_s[tid] = rows[p.c_offset + g * N + tid];
+        }
+        meet();
+        const float step = sc_softplus(proj[p.dt_offset + h] + p.dt_bias[h]), less_one = expm1f(-rate * step), x = rows[column], u = step * x;
+        float y = 0.f;
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int t = tiles[m] * SC_BLOCK + 8 * half + (lane >> 2);
-            if (t >= count) continue;
-            const int v = h * p.vdim + column0 + v0 + 2 * (lane & 3);
-            const float* x = rows + (size_t)t * p.xbc_stride + v;
-            const float* z = p.proj + (row0 + t) * p.proj_stride + p.z_offset + v;
-            float* out = p.out + (row0 + t) * ((size_t)p.heads * p.vdim) + v;
+        for (int n = 0; n < N; ++n) {
+            S[n] = fmaf(less_one, S[n], S[n]) + b_s[n] * u;
+            y = fmaf(S[n], c_s[n], y);
+        }
+        const float z = proj[p.z_offset + column];
+        p.out[row * ((size_t)p.heads * p.vdim) + column] = fmaf(p.d[h], x, y) * (z / (1.0f + expf(-z)));
+    }
+    float* to = kept + ((start + n_tok) & 1) * p.copy_floats;
 #pragma unroll
-            for (int n = 0; n < 4; ++n) {
-                const float2 xv = *(const float2*)(x + 8 * n), zv = *(const float2*)(z + 8 * n);
-                const float y0 = fmaf(dskip, xv.x, acc[m][n][2 * half]), y1 = fmaf(dskip, xv.y, acc[m][n][2 * half + 1]);
-                *(float2*)(out + 8 * n) = make_float2(y0 * (zv.x / (1.0f + expf(-zv.x))), y1 * (zv.y / (1.0f + expf(-zv.y))));
+    for (int n = 0; n < N; ++n) to[(size_t)n * p.vdim] = S[n];
+}
+
+template <int N, bool TWO>
+__global__ void __launch_bounds__(ST_THREADS, 1) state_space_chain_kernel(const __grid_constant__ CUtensorMap map_x, StateSpaceChunks p, int* __restrict__ status) {
+    constexpr int SHARE = N / 2, HEADS = TWO ? 2 : 1, UK = HEADS * SC_TOKENS;        // UK: columns of u's parts
+    constexpr uint32_t ROWS_PART = SC_TOKENS * N * 2, PAIR_PART = HEADS * SC_TOKENS * SC_TOKENS * 2, X_BYTES = SC_TOKENS * SC_COLUMNS * 4;
+    // tensor memory: the state's parts, later DO over their first columns; D1; u's parts; those of u w(j, end); DS
+    constexpr int S_HI = 0, S_LO = N / 2, D_O = 0, D_1 = 128, U_HI = 192, U_LO = U_HI + UK / 2, UE_HI = 320, UE_LO = 352, D_S = 384;
+    extern __shared__ uint8_t st_smem[];
+    __shared__ uint64_t x_full, b_full, c_full, pairs_full, ready, d1_done, ds_done, do_done, o_stored, o_free[2];
+    __shared__ float tops[3][2][SC_COLUMNS];
+    __shared__ __align__(16) float factors[2][HEADS][SC_FACTORS];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int failed_flag, odd_numbers;
+    volatile int* failed = &failed_flag;
+    uint8_t* c_s = (uint8_t*)(((uintptr_t)st_smem + 1023) & ~(uintptr_t)1023);
+    uint8_t* b_s = c_s + 2 * ROWS_PART;
+    uint8_t* pairs_s = b_s + 2 * ROWS_PART;
+    float* x_s = (float*)(pairs_s + 2 * PAIR_PART);                      // [chunk & 1][SC_TOKENS][SC_COLUMNS]
+    float* o_s = x_s + 2 * SC_TOKENS * SC_COLUMNS;                       // of S^T C + sum P u
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int b = blockIdx.x, block = blockIdx.y, column0 = block * SC_COLUMNS, h0 = column0 / p.vdim, g = h0 / (p.heads / p.groups);
+    const int first = 2 * p.seq_chunk0[b], last = p.seq_chunk0[b + 1], start = p.seq_start[b], n_tok = p.cu_q_len[b + 1] - p.cu_q_len[b];
+    int chunks = 2 * last - first;
+    if (chunks > 0 && p.tokens_of(first + chunks - 1) <= 0) --chunks;
+    chunks = __shfl_sync(0xffffffffu, chunks, 0);
+
+    if (threadIdx.x == 0) {
+        bar_init(&x_full, 1); bar_init(&b_full, 1); bar_init(&c_full, 1); bar_init(&pairs_full, 1); bar_init(&ready, ST_ROWS / 32);
+        bar_init(&d1_done, 1); bar_init(&ds_done, 1); bar_init(&do_done, 1); bar_init(&o_stored, ST_ROWS / 32); bar_init(&o_free[0], ST_ROWS / 32); bar_init(&o_free[1], ST_ROWS / 32);
+        failed_flag = 0;
+        odd_numbers = 0;
+        bar_init_fence();
+    }
+    if (warp == 1) tmem_alloc(&tmem_slot, 512);
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
+    after_previous_kernel();                         // barriers and tensor memory were set up while it still ran
+
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ST_REGS_ISSUE));
+        if (warp == 0) {
+            for (int c = 0; c < chunks; ++c) {
+                const int chunk = first + c;
+                const uint32_t before = (c & 1) ^ 1;                     // of the phase that the chunk before has ended
+                const size_t group_at = (size_t)chunk * p.groups + g, factor_bytes = HEADS * SC_FACTORS * 4;
+                if (c && !warp_wait(&ready, before, failed)) { if (lane == 0) atomicExch(status, 81); break; }
+                if (c > 1 && !warp_wait(&o_free[c & 1], (c >> 1 & 1) ^ 1, failed)) { if (lane == 0) atomicExch(status, 92); break; }
+                if (lane == 0) {
+                    bar_expect(&x_full, X_BYTES + factor_bytes);
+                    load_2d(x_s + (c & 1) * SC_TOKENS * SC_COLUMNS, &map_x, column0, (int)p.row_of(chunk), &x_full);
+                    copy_bulk(factors[c & 1], p.factors + ((size_t)chunk * p.heads + h0) * SC_FACTORS, factor_bytes, &x_full);
+                }
+                if (c && !warp_wait(&ds_done, before, failed)) { if (lane == 0) atomicExch(status, 82); break; }
+                if (lane == 0) {
+                    bar_expect(&b_full, 2 * ROWS_PART);
+                    copy_bulk(b_s, p.b_parts + group_at * 2 * SC_TOKENS * N, 2 * ROWS_PART, &b_full);
+                }
+                if (c && !warp_wait(&d1_done, before, failed)) { if (lane == 0) atomicExch(status, 83); break; }
+                if (lane == 0) {
+                    bar_expect(&c_full, 2 * ROWS_PART);
+                    copy_bulk(c_s, p.c_parts + group_at * 2 * SC_TOKENS * N, 2 * ROWS_PART, &c_full);
+                }
+                if (c && !warp_wait(&do_done, before, failed)) { if (lane == 0) atomicExch(status, 84); break; }
+                if (lane == 0) {
+                    bar_expect(&pairs_full, 2 * PAIR_PART);
+                    copy_bulk(pairs_s, p.pair_parts + ((size_t)chunk * gridDim.y + block) * 2 * HEADS * SC_TOKENS * SC_TOKENS, 2 * PAIR_PART, &pairs_full);
+                }
+                __syncwarp();
+            }
+        } else if (warp == 1) {
+            // the whole warp goes through the loop (elect_one, tcgen05.cuh); its products run in the order of their issue, so DO may be
+            // asked for over the state's parts, which D1 has read
+            constexpr uint32_t idesc64 = (1u << 4) | ((uint32_t)(64 >> 3) << 17) | ((uint32_t)(SC_COLUMNS >> 4) << 24);
+            constexpr uint32_t idesc_b = (1u << 4) | (1u << 16) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(SC_COLUMNS >> 4) << 24);
+            const uint64_t c_at = tile_desc(smem_addr(c_s)), pairs_at = tile_desc(smem_addr(pairs_s)), b_at = desc_n_major(smem_addr(b_s));
+            auto along = [](int k) { return (k / 4) * (SC_TOKENS * 128 >> 4) + (k % 4) * 2; };
+            for (int c = 0; c < chunks; ++c) {
+                const uint32_t phase = c & 1;
+                if (!warp_wait_both(&ready, phase, &b_full, phase, failed)) { if (lane == 0) atomicExch(status, 85); break; }
+                fence_after_sync();
+                if (elect_one()) {
+                    products_of_parts<SC_TOKENS / 16>(tmem + D_S, tmem + UE_HI, tmem + UE_LO, b_at, b_at + (ROWS_PART >> 4), idesc_b,
+                                                      [](int k) { return k * (16 * 128 >> 4); });
+                    mma_commit(&ds_done);
+                }
+                __syncwarp();
+                if (!warp_wait(&c_full, phase, failed)) { if (lane == 0) atomicExch(status, 86); break; }
+                fence_after_sync();
+                if (elect_one()) {
+                    products_of_parts<N / 16>(tmem + D_1, tmem + S_HI, tmem + S_LO, c_at, c_at + (ROWS_PART >> 4), idesc64, along);
+                    mma_commit(&d1_done);
+                }
+                __syncwarp();
+                if (!warp_wait(&pairs_full, phase, failed)) { if (lane == 0) atomicExch(status, 87); break; }
+                fence_after_sync();
+                if (elect_one()) {
+                    products_of_parts<UK / 16>(tmem + D_O, tmem + U_HI, tmem + U_LO, pairs_at, pairs_at + (PAIR_PART >> 4), idesc64, along);
+                    mma_commit(&do_done);
+                }
+                __syncwarp();
             }
         }
+    } else if (warp < 12) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(ST_REGS_ROWS));
+        // A wait that gives up does not end the loop: the block's later waits then return at once, and every thread reaches the barriers.
+        const int share = (warp - 4) >> 2, quarter = warp & 3, column = quarter * 32 + lane, t0 = ST_SHARE_TOKENS * share;
+        const int hh = TWO ? quarter >> 1 : 0;       // the column's head among the block's
+        const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16);
+        const size_t state_at = p.state_offset + ((size_t)(h0 + hh) * N + share * SHARE) * p.vdim + column % p.vdim;
+        float* kept = p.state + (size_t)p.seq_slot[b] * 2 * p.copy_floats + state_at;
+        bool ok = true;
+        auto wait = [&](uint64_t* bar, uint32_t phase, int code) {
+            if (!bar_wait(bar, phase, failed)) { if (ok && lane == 0) atomicExch(status, code); ok = false; }
+            __syncwarp();
+            fence_after_sync();
+        };
+        auto meet = [] { asm volatile("bar.sync 1, %0;" ::"n"(ST_ROWS) : "memory"); };
+        float S[SHARE];
+        uint64_t finite = 0ull;                      // becomes NaNs at the first number that is not finite
+#pragma unroll
+        for (int n = 0; n < SHARE; ++n) S[n] = (kept + (start & 1) * p.copy_floats)[(size_t)n * p.vdim];
+        if (TWO) {                                   // the other head's half of the inner size: zeros for good
+            const uint32_t zeros[16] = {};
+            tmem_st16(lanes + U_HI + (hh ^ 1) * 32 + 16 * share, zeros);
+            tmem_st16(lanes + U_LO + (hh ^ 1) * 32 + 16 * share, zeros);
+        }
+        for (int c = 0; c < chunks; ++c) {
+            const uint32_t phase = c & 1;
+            const float4* f4 = (const float4*)factors[c & 1][hh];        // sixteen of four each: D1's, DO's, w(j, end), dt
+            const int count = p.tokens_of(first + c);
+            wait(&x_full, phase, 88);                // and the factors; what they overwrite was used before the chunk before was ready
+            float u[ST_SHARE_TOKENS], u_top = 0.f, s_top = 0.f;
+#pragma unroll
+            for (int t = 0; t < ST_SHARE_TOKENS; ++t) u[t] = x_s[((c & 1) * SC_TOKENS + t0 + t) * SC_COLUMNS + column];
+#pragma unroll
+            for (int t = 0; t < ST_SHARE_TOKENS; t += 4) {
+                const float4 f = f4[(3 * SC_TOKENS + t0 + t) / 4];
+                halves_of(mul_pairs(pair_of(u[t], u[t + 1]), pair_of(f.x, f.y)), u[t], u[t + 1]);
+                halves_of(mul_pairs(pair_of(u[t + 2], u[t + 3]), pair_of(f.z, f.w)), u[t + 2], u[t + 3]);
+            }
+            if (t0 + ST_SHARE_TOKENS > count) {      // behind the last token are other rows
+#pragma unroll
+                for (int t = 0; t < ST_SHARE_TOKENS; ++t)
+                    if (t0 + t >= count) u[t] = 0.f;
+            }
+#pragma unroll
+            for (int t = 0; t < ST_SHARE_TOKENS; t += 2) u_top = max3(u_top, fabsf(u[t]), fabsf(u[t + 1]));
+#pragma unroll
+            for (int n = 0; n < SHARE; n += 2) s_top = max3(s_top, fabsf(S[n]), fabsf(S[n + 1]));
+            tops[0][share][column] = s_top;
+            tops[1][share][column] = u_top;
+            if (share == 0) tops[2][0][column] = first_row_top(u);
+            fence_before_sync();                     // DO's columns are read before the state's parts go over them
+            meet();
+            fence_after_sync();
+            u_top = fmaxf(tops[1][0][column], tops[1][1][column]);
+            const float first_top = tops[2][0][column];
+            if (first_top != 0.f && first_top < u_top * 3.725290298461914e-09f) finite = pair_of(NAN, NAN);         // 2^-28
+            const int s_exponent = parts_exponent(fmaxf(tops[0][0][column], tops[0][1][column])), u_exponent = parts_exponent(u_top);
+            store_parts(S, power_of_two(s_exponent), lanes + S_HI + share * (SHARE / 2), lanes + S_LO + share * (SHARE / 2));
+            store_parts(u, power_of_two(u_exponent), lanes + U_HI + hh * 32 + t0 / 2, lanes + U_LO + hh * 32 + t0 / 2);
+#pragma unroll
+            for (int t = 0; t < ST_SHARE_TOKENS; t += 4) {
+                const float4 fe = f4[(2 * SC_TOKENS + t0 + t) / 4];
+                halves_of(mul_pairs(pair_of(u[t], u[t + 1]), pair_of(fe.x, fe.y)), u[t], u[t + 1]);
+                halves_of(mul_pairs(pair_of(u[t + 2], u[t + 3]), pair_of(fe.z, fe.w)), u[t + 2], u[t + 3]);
+            }
+            store_parts(u, power_of_two(u_exponent), lanes + UE_HI + t0 / 2, lanes + UE_LO + t0 / 2);
+            tmem_wait_st();
+            fence_before_sync();
+            __syncwarp();
+            if (lane == 0) bar_arrive(&ready);
+
+            // the new state, then the outputs
+            const float decay = factors[c & 1][hh][4 * SC_TOKENS], s_inv = power_of_two(-s_exponent), u_inv = power_of_two(-u_exponent);
+            const float ue_inv = u_inv * factors[c & 1][hh][4 * SC_TOKENS + 1];
+            wait(&ds_done, phase, 89);
+#pragma unroll
+            for (int n0 = 0; n0 < SHARE; n0 += 32) {
+                uint32_t v[2][16];
+                load_columns<32>(lanes + D_S + share * SHARE + n0, v);
+                tmem_wait_ld();
+#pragma unroll
+                for (int n = 0; n < 32; n += 2) {
+                    const uint64_t now = fma_pairs(pair_of(S[n0 + n], S[n0 + n + 1]), pair_of(decay, decay),
+                                                   mul_pairs(pair_of(__uint_as_float(v[n / 16][n % 16]), __uint_as_float(v[n / 16][n % 16 + 1])), pair_of(ue_inv, ue_inv)));
+                    halves_of(now, S[n0 + n], S[n0 + n + 1]);
+                }
+            }
+            uint32_t v[2][16];
+            uint64_t o[ST_SHARE_TOKENS / 2];
+            auto sums_at = [&](int t) { return pair_of(__uint_as_float(v[t / 16][t % 16]), __uint_as_float(v[t / 16][t % 16 + 1])); };
+            wait(&d1_done, phase, 90);
+            load_columns<32>(lanes + D_1 + t0, v);
+            tmem_wait_ld();
+#pragma unroll
+            for (int t = 0; t < ST_SHARE_TOKENS; t += 4) {
+                const float4 f = f4[(t0 + t) / 4];
+                const uint64_t fs[2] = {pair_of(f.x, f.y), pair_of(f.z, f.w)};
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    o[t / 2 + i] = mul_pairs(sums_at(t + 2 * i), mul_pairs(pair_of(s_inv, s_inv), fs[i]));
+            }
+            wait(&do_done, phase, 91);
+            load_columns<32>(lanes + D_O + t0, v);
+            tmem_wait_ld();
+            if (c > 0) wait(&o_free[phase ^ 1], (c - 1) >> 1 & 1, 92);       // the chunk before has been read
+#pragma unroll
+            for (int t = 0; t < ST_SHARE_TOKENS; t += 4) {
+                const float4 f = f4[(SC_TOKENS + t0 + t) / 4];
+                const uint64_t fs[2] = {pair_of(f.x, f.y), pair_of(f.z, f.w)};
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const uint64_t y = fma_pairs(sums_at(t + 2 * i), mul_pairs(pair_of(u_inv, u_inv), fs[i]), o[t / 2 + i]);
+                    finite = fma_pairs(y, 0ull, finite);
+                    float y0, y1;
+                    halves_of(y, y0, y1);
+                    o_s[(t0 + t + 2 * i) * SC_COLUMNS + column] = y0;
+                    o_s[(t0 + t + 2 * i + 1) * SC_COLUMNS + column] = y1;
+                }
+            }
+            __syncwarp();
+            if (lane == 0) bar_arrive(&o_stored);
+        }
+#pragma unroll
+        for (int n = 0; n < SHARE; n += 2) finite = fma_pairs(pair_of(S[n], S[n + 1]), 0ull, finite);        // an earlier one reached the outputs
+        float even, odd;
+        halves_of(finite, even, odd);
+        if (even != 0.f || odd != 0.f) odd_numbers = 1;
+        meet();
+        if (chunks > 0 && !odd_numbers && ok && !*failed) {
+            float* to = kept + ((start + n_tok) & 1) * p.copy_floats;
+#pragma unroll
+            for (int n = 0; n < SHARE; ++n) to[(size_t)n * p.vdim] = S[n];
+        }
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ST_REGS_OUTPUTS));
+        // a thread two columns of every fourth token; z is asked for into L2 a chunk ahead
+        const int tid = threadIdx.x - 384, column = column0 + 2 * (tid & 63), t0 = tid >> 6;
+        const float dskip = p.d[column / p.vdim];
+        auto z_of = [&](int chunk, int t) { return p.proj + (p.row_of(chunk) + t) * p.proj_stride + p.z_offset; };
+        float gates[2][16];
+        auto load = [&](int c, int half) {
+            const int count = p.tokens_of(first + c);
+            const float* z = z_of(first + c, t0) + column;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int t = half * (SC_TOKENS / 2) + 4 * k;
+                float2 v = make_float2(0.f, 0.f);
+                if (t0 + t < count) v = *(const float2*)(z + (size_t)t * p.proj_stride);
+                gates[half][2 * k] = v.x;
+                gates[half][2 * k + 1] = v.y;
+            }
+        };
+        if (chunks > 0) load(0, 0);
+        for (int c = 0; c < chunks; ++c) {
+            const int count = p.tokens_of(first + c);
+            float* out = p.out + (p.row_of(first + c) + t0) * ((size_t)p.heads * p.vdim) + column;
+            const float* sums = o_s + t0 * SC_COLUMNS + 2 * (tid & 63);
+            const float* x = x_s + ((c & 1) * SC_TOKENS + t0) * SC_COLUMNS + 2 * (tid & 63);
+            if (c + 1 < chunks && (tid >> 2) < p.tokens_of(first + c + 1))
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(z_of(first + c + 1, tid >> 2) + column0 + 32 * (tid & 3)));
+            auto write = [&](int half) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const int t = half * (SC_TOKENS / 2) + 4 * k;
+                    const float2 o = *(const float2*)(sums + t * SC_COLUMNS), xs = *(const float2*)(x + t * SC_COLUMNS);
+                    const float2 y = make_float2(fmaf(dskip, xs.x, o.x) * gates[half][2 * k], fmaf(dskip, xs.y, o.y) * gates[half][2 * k + 1]);
+                    if (t0 + t < count) *(float2*)(out + (size_t)t * p.heads * p.vdim) = y;
+                }
+            };
+            sc_silu(gates[0]);
+            load(c, 1);
+            if (!bar_wait(&o_stored, c & 1, failed)) { if (lane == 0) atomicExch(status, 93); }
+            __syncwarp();
+            write(0);
+            if (c + 1 < chunks) load(c + 1, 0);
+            sc_silu(gates[1]);
+            write(1);
+            __syncwarp();
+            if (lane == 0) bar_arrive(&o_free[c & 1]);
+        }
+    }
+    fence_before_sync();
+    __syncthreads();
+    if (failed_flag && warp == 0 && lane == 0) {
+        // copies may still be on their way into this block's shared memory: give them a bounded time to land
+        uint64_t* bars[4] = {&x_full, &b_full, &c_full, &pairs_full};
+        for (int i = 0; i < 4; ++i)
+            for (uint32_t parity = 0; parity < 2; ++parity) { int zero = 0; bar_wait(bars[i], parity, &zero, 2000000); }
+    }
+    __syncthreads();
+    if (warp == 1) tmem_free(tmem, 512);
+    if (odd_numbers && !failed_flag && warp >= 4 && warp < 8)
+        st_token_by_token<N>(p, b, column0 + threadIdx.x - 128, threadIdx.x - 128, (float*)c_s);         // over the outputs written
 }
 
 // ----------------------------------------------------------------------------- host side
 
 // Chunks of at most 128 tokens: chunk_seq/begin/end and, per sequence, its first chunk (one entry more at the end).  scratch:
-// num_chunks * (heads * N * vdim + groups * 128 * 128 + heads) floats.
+// 2 * num_chunks * (groups * (64 (64 + 2 N + 1) + 4) + heads * (64 * 64 + 260)) floats.  status: one int on the device, zero before
+// the call.  num_rows: the rows of xbc.
 FRB_API int frb_state_space_chunks(const float* proj, int proj_stride, int z_offset, int dt_offset, const float* xbc, int xbc_stride,
                                    int b_offset, int c_offset, const float* dt_bias, const float* a_log, const float* d, const int* seq_slot,
                                    const int* seq_start, const int* cu_q_len, float* state, long long copy_floats, long long state_offset,
                                    float* out, int num_seqs, int heads, int vdim, int N, int groups, const int* chunk_seq,
-                                   const int* chunk_begin, const int* chunk_end, const int* seq_chunk0, int num_chunks, float* scratch,
-                                   cudaStream_t stream) {
+                                   const int* chunk_begin, const int* chunk_end, const int* seq_chunk0, int num_chunks, int num_rows,
+                                   float* scratch, int* status, cudaStream_t stream) {
     if (num_seqs == 0 || num_chunks == 0) return 0;
     FRB_CHECK_ARG((N == 64 || N == 128) && (vdim == 64 || vdim == 128) && groups >= 1 && heads % groups == 0 &&
                       heads / groups * vdim % SC_COLUMNS == 0 && heads <= 65535, "state-space chunks: %d heads of %d x %d in %d groups", heads, N,
                   vdim, groups);
-    FRB_CHECK_ARG(((xbc_stride | b_offset | c_offset) & 3) == 0 && ((proj_stride | z_offset) & 1) == 0 && ((copy_floats | state_offset) & 3) == 0 &&
-                      (((uintptr_t)xbc | (uintptr_t)state | (uintptr_t)scratch | (uintptr_t)out) & 15) == 0 && ((uintptr_t)proj & 7) == 0,
+    FRB_CHECK_ARG(((xbc_stride | b_offset | c_offset) & 3) == 0 && ((proj_stride | z_offset) & 1) == 0 &&
+                      (((uintptr_t)xbc | (uintptr_t)scratch | (uintptr_t)out) & 15) == 0 && ((uintptr_t)proj & 7) == 0,
                   "state-space chunks: rows of %d entries are not in steps of 16 bytes", xbc_stride);
     StateSpaceChunks p;
     p.proj = proj; p.xbc = xbc; p.dt_bias = dt_bias; p.a_log = a_log; p.d = d; p.seq_slot = seq_slot; p.seq_start = seq_start;
     p.cu_q_len = cu_q_len; p.chunk_seq = chunk_seq; p.chunk_begin = chunk_begin; p.chunk_end = chunk_end; p.seq_chunk0 = seq_chunk0;
     p.state = state; p.copy_floats = copy_floats; p.state_offset = state_offset; p.out = out;
-    p.states = scratch;
-    p.pairs = scratch + (size_t)num_chunks * heads * N * vdim;
-    p.decays = p.pairs + (size_t)num_chunks * groups * SC_TOKENS * SC_TOKENS;
+    const size_t chunks = 2 * (size_t)num_chunks, rows = chunks * groups * SC_TOKENS * N;
+    p.c_parts = (uint16_t*)scratch;
+    p.b_parts = (uint16_t*)(scratch + rows);
+    p.pair_parts = (uint16_t*)(scratch + 2 * rows);
+    p.raw_pairs = scratch + 2 * rows + chunks * heads * SC_TOKENS * SC_TOKENS;
+    p.scales = p.raw_pairs + chunks * groups * SC_TOKENS * SC_TOKENS;
+    p.factors = p.scales + chunks * groups * (SC_TOKENS + 4);
     p.proj_stride = proj_stride; p.z_offset = z_offset; p.dt_offset = dt_offset; p.xbc_stride = xbc_stride; p.b_offset = b_offset;
     p.c_offset = c_offset; p.heads = heads; p.vdim = vdim; p.N = N; p.groups = groups;
-    const size_t pairs_smem = 2 * SC_TOKENS * SC_LC * sizeof(float);
-    const size_t states_smem = 2 * 32 * (N + 4 + SC_COLUMNS + 4) * sizeof(float);
-    const size_t outputs_smem = (2 * (SC_TOKENS * (32 + 8) + 32 * (SC_SLICE + 4)) + SC_TOKENS * (SC_SLICE + 4)) * sizeof(float);
-    cudaFuncSetAttribute(state_space_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pairs_smem);
-    cudaFuncSetAttribute(state_space_outputs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)outputs_smem);
-    state_space_pairs_kernel<<<dim3(num_chunks, groups), SC_THREADS, pairs_smem, stream>>>(p);
-    const dim3 states_grid(num_chunks, heads * vdim / SC_COLUMNS);
-    if (N == 128) {
-        cudaFuncSetAttribute(state_space_states_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)states_smem);
-        state_space_states_kernel<128><<<states_grid, SC_THREADS, states_smem, stream>>>(p);
-    } else {
-        cudaFuncSetAttribute(state_space_states_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)states_smem);
-        state_space_states_kernel<64><<<states_grid, SC_THREADS, states_smem, stream>>>(p);
-    }
-    state_space_chain_kernel<<<dim3(num_seqs, heads, (N * vdim + 1023) / 1024), 256, 0, stream>>>(p);
-    state_space_outputs_kernel<<<dim3(num_chunks, heads, vdim / SC_SLICE), SC_THREADS, outputs_smem, stream>>>(p);
+    const int two = vdim == 64 ? 2 : 1;
+    const size_t pairs_smem = 2 * (size_t)SC_TOKENS * (N + 8) * sizeof(float);
+    const size_t chain_smem = (size_t)SC_TOKENS * 2 * (4 * N + 2 * two * SC_TOKENS + 6 * SC_COLUMNS) + 1024;
+    CUtensorMap map_x;
+    EncodeFn encode = encoder();
+    cuuint64_t dims[2] = {(cuuint64_t)xbc_stride, (cuuint64_t)num_rows}, strides[1] = {(cuuint64_t)xbc_stride * 4};
+    cuuint32_t box[2] = {SC_COLUMNS, SC_TOKENS}, steps[2] = {1, 1};
+    FRB_CHECK_ARG(encode && encode(&map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(xbc), dims, strides, box, steps,
+                                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS,
+                  "state-space chunks: cuTensorMapEncodeTiled failed or is not available");
+    const dim3 chains(num_seqs, heads * vdim / SC_COLUMNS);
+#define FRB_STATE_SPACE(NN, TWO)                                                                                                      \
+    do {                                                                                                                              \
+        auto chain = state_space_chain_kernel<NN, TWO>;                                                                               \
+        /* the groups of warps share out the registers that the block is launched with: fewer, and they would wait for ever */        \
+        static const int registers = [&] {                                                                                            \
+            cudaFuncAttributes attributes;                                                                                            \
+            return cudaFuncGetAttributes(&attributes, chain) == cudaSuccess ? attributes.numRegs : 0;                                 \
+        }();                                                                                                                          \
+        FRB_CHECK_ARG(registers >= ST_REGS_LAUNCH, "state-space chunks: the kernel was compiled to %d registers", registers);         \
+        cudaFuncSetAttribute(state_space_pairs_kernel<NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pairs_smem);             \
+        cudaFuncSetAttribute(chain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chain_smem);                                    \
+        state_space_pairs_kernel<NN><<<dim3((unsigned)chunks, groups), 256, pairs_smem, stream>>>(p);                                 \
+        state_space_weights_kernel<<<dim3((unsigned)chunks, heads), 128, 0, stream>>>(p);                                             \
+        launch_dependent(chain, chains, dim3(ST_THREADS), chain_smem, stream, map_x, p, status);                                             \
+    } while (0)
+    if (N == 128) { if (two == 2) FRB_STATE_SPACE(128, true); else FRB_STATE_SPACE(128, false); }
+    else { if (two == 2) FRB_STATE_SPACE(64, true); else FRB_STATE_SPACE(64, false); }
+#undef FRB_STATE_SPACE
     FRB_RETURN_LAUNCH("state_space_chunks");
 }

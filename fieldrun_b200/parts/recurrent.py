@@ -37,11 +37,11 @@ from .linear import linear
 
 # From this many tokens of the longest prompt on a step's recurrence may run in chunks as matrix products (state_space_chunks.cu,
 # delta_chunks.cu).  Measured on a B200, the kernels alone, microseconds, token by token | in chunks.  State space: 64 heads of 128 x 64, one
-# prompt of 128 tokens 55 | 70, of 1,024 tokens 350 | 119, 16 of 130 tokens 279 | 353, of 256 tokens 525 | 390, one of 256 beside 31 of two
-# 188 | 374; 16 heads of 64 x 64, 64 of 128 tokens 159 | 185; of 128 x 128, 4 of 300 tokens 166 | 119.  Delta rule: 16 heads of 128 x 128, one
+# prompt of 64 tokens 28 | 34, of 128 tokens 53 | 39, of 1,024 tokens 341 | 111, 16 of 64 tokens 143 | 98, 8 of 130 tokens 159 | 89, one of 256
+# beside 31 of two 178 | 173, 100 of 17 beside one of 64 319 | 432; 8 heads of 64 x 64, 16 of 64 tokens 22 | 29; 16 of 128 x 128, 4 of 300 tokens 160 | 51.  Delta rule: 16 heads of 128 x 128, one
 # prompt of 64 tokens 51 | 42, of 1,024 tokens 671 | 104, 16 of 65 tokens 208 | 95, 100 of 17 beside one of 64 460 | 273; 64 heads of 64 x 64, 16 of
 # 65 tokens 205 | 271; 64 heads of 128 x 64, one of 256 beside 31 of two 330 | 449.
-STATE_SPACE_CHUNKED_TOKENS, DELTA_CHUNKED_TOKENS = 128, 64
+STATE_SPACE_CHUNKED_TOKENS, DELTA_CHUNKED_TOKENS = 64, 64
 
 
 class _StateMixer(Mixer):
@@ -211,17 +211,19 @@ class ScalarDecayStateSpace(_StateMixer):
         self.w = self._fetch(source)
 
     def chunks_pay(self, ctx) -> bool:
-        """Whether a step of prompts is faster in chunks: microseconds of both ways, fitted to 144 steps of eight head counts and sizes
-        (the measurements above among them; the worst choice against token by token costs 5 %)."""
+        """Whether a step of prompts is faster in chunks: microseconds of both ways, fitted to 141 steps of eight head counts and sizes
+        (the measurements above among them; no step of them is more than 3 % slower this way than token by token)."""
         if ctx.is_decode or ctx.max_q_len < STATE_SPACE_CHUNKED_TOKENS:
             return False
         rows, columns = self.state / 128, self.value_dim / 128
         size, blocks, tokens = rows * columns, ctx.num_seqs * self.num_heads, ctx.num_tokens * self.num_heads
         longest = (0.02 + 0.18 * rows + 0.32 * columns) * ctx.max_q_len
-        crowded = 0.01 * size * self.num_heads * ctx.max_q_len if blocks > 4 * ops.sm_count(ctx.device) else 0.0      # long ones side by side
+        crowded = 0.005 * size * self.num_heads * ctx.max_q_len if blocks > 4 * ops.sm_count(ctx.device) else 0.0     # long ones side by side
         serial = 11 + max(longest + crowded + 0.027 * blocks, 0.29 * longest + (0.00026 + 0.0034 * size) * tokens)
+        # the chain along the longest prompt's chunks of 64, or of all when they fill the device; a block has 128 columns
         items = ctx.chunk_count(ops.STATE_SPACE_CHUNK_TOKENS) * self.num_heads
-        return ops.chunks_pay(max(35 + 32 * rows, 39 + 0.32 * size * items + (0.0009 * columns - 0.00045 * size) * tokens), serial)
+        along = max(-(-ctx.max_q_len // 64), 2.6 * items * columns / ops.sm_count(ctx.device))
+        return ops.chunks_pay(23 + 3 * rows + (3.2 + 1.3 * rows) * along + (0.015 + 0.01 * rows) * items, serial)
 
     def forward(self, ctx, act: torch.Tensor, line: LineView, writes_cache: bool) -> torch.Tensor:
         self._check(writes_cache)

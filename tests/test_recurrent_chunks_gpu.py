@@ -256,8 +256,8 @@ def gla_case():
     return views, run, exact
 
 
-def state_space_case():
-    heads, groups, n, vdim = 4, 2, 64, 64
+def state_space_case(n=64, vdim=64):
+    heads, groups = 4, 2
     gen = torch.Generator(device=DEV).manual_seed(2)
     tokens, inner = AT[-1], heads * vdim
     proj, xbc = torch.randn(tokens, inner + heads, device=DEV, generator=gen), torch.randn(tokens, inner + 2 * groups * n, device=DEV, generator=gen) * 0.3
@@ -338,14 +338,15 @@ def delta_case(vdim=64):
 
 
 # with 128 value columns the chain along the chunks runs on tcgen05
-CASES = {"gla": gla_case, "state space": state_space_case, "delta": delta_case, "delta 128": lambda: delta_case(128)}
+CASES = {"gla": gla_case, "state space": state_space_case, "state space 128": lambda: state_space_case(128, 128), "delta": delta_case, "delta 128": lambda: delta_case(128)}
 
 
-NAMES = [("gla", n) for n in ("q", "k", "v", "decay")] + [("state space", n) for n in ("x", "b", "c", "decay")] + [
+NAMES = [("gla", n) for n in ("q", "k", "v", "decay")] + [(c, n) for c in ("state space", "state space 128") for n in ("x", "b", "c", "decay")] + [
     (c, n) for c in ("delta", "delta 128") for n in ("q", "k", "v", "beta", "decay")]
 
 
 @pytest.mark.parametrize("case,name,number", [(*c, n) for c in NAMES for n in (INF, NAN)] + [("state space", "x", 3.4028234e38),
+                                                                                             ("state space 128", "x", 3.4028234e38),
                                                                                              ("delta", "v", 3.4028234e38),
                                                                                              ("delta 128", "v", 3.4028234e38)])
 def test_a_token_that_is_not_finite_reaches_no_token_before_it(case, name, number):
@@ -375,7 +376,7 @@ def test_a_token_that_is_not_finite_reaches_no_token_before_it(case, name, numbe
             assert norm_error(a, b) < LIMIT
 
 
-@pytest.mark.parametrize("case,strong", [(c, s) for c in ("state space", "delta", "delta 128") for s in (-20.0, -200.0, -2000.0)] +
+@pytest.mark.parametrize("case,strong", [(c, s) for c in ("state space", "state space 128", "delta", "delta 128") for s in (-20.0, -200.0, -2000.0)] +
                          [("delta", -INF), ("delta 128", -INF)])
 def test_one_strong_decay_among_mild_ones(case, strong):
     """Tokens that all but clear the state (logarithm of the decay down to about -2,000, and a decay of zero), one in each of some blocks,
