@@ -40,8 +40,9 @@ from .linear import linear
 # prompt of 64 tokens 28 | 34, of 128 tokens 53 | 39, of 1,024 tokens 341 | 111, 16 of 64 tokens 143 | 98, 8 of 130 tokens 159 | 89, one of 256
 # beside 31 of two 178 | 173, 100 of 17 beside one of 64 319 | 432; 8 heads of 64 x 64, 16 of 64 tokens 22 | 29; 16 of 128 x 128, 4 of 300 tokens 160 | 51.  Delta rule: 16 heads of 128 x 128, one
 # prompt of 64 tokens 51 | 42, of 1,024 tokens 671 | 104, 16 of 65 tokens 208 | 95, 100 of 17 beside one of 64 460 | 273; 64 heads of 64 x 64, 16 of
-# 65 tokens 205 | 271; 64 heads of 128 x 64, one of 256 beside 31 of two 330 | 449.
-STATE_SPACE_CHUNKED_TOKENS, DELTA_CHUNKED_TOKENS = 64, 64
+# 65 tokens 205 | 271; 64 heads of 128 x 64, one of 256 beside 31 of two 330 | 449.  State space: steps of shorter
+# prompts than 192 tokens keep the results that they had token by token; chunks would save 14 us (one of 128) to 70 (8 of 130).
+STATE_SPACE_CHUNKED_TOKENS, DELTA_CHUNKED_TOKENS = 192, 64
 
 
 class _StateMixer(Mixer):
@@ -212,13 +213,13 @@ class ScalarDecayStateSpace(_StateMixer):
 
     def chunks_pay(self, ctx) -> bool:
         """Whether a step of prompts is faster in chunks: microseconds of both ways, fitted to 141 steps of eight head counts and sizes
-        (the measurements above among them; no step of them is more than 3 % slower this way than token by token)."""
+        (the measurements above among them; from 192 tokens on no step of them is more than 3 % slower this way than token by token)."""
         if ctx.is_decode or ctx.max_q_len < STATE_SPACE_CHUNKED_TOKENS:
             return False
         rows, columns = self.state / 128, self.value_dim / 128
         size, blocks, tokens = rows * columns, ctx.num_seqs * self.num_heads, ctx.num_tokens * self.num_heads
         longest = (0.02 + 0.18 * rows + 0.32 * columns) * ctx.max_q_len
-        crowded = 0.005 * size * self.num_heads * ctx.max_q_len if blocks > 4 * ops.sm_count(ctx.device) else 0.0     # long ones side by side
+        crowded = 0.002 * size * self.num_heads * ctx.max_q_len if blocks > 4 * ops.sm_count(ctx.device) else 0.0     # long ones side by side
         serial = 11 + max(longest + crowded + 0.027 * blocks, 0.29 * longest + (0.00026 + 0.0034 * size) * tokens)
         # the chain along the longest prompt's chunks of 64, or of all when they fill the device; a block has 128 columns
         items = ctx.chunk_count(ops.STATE_SPACE_CHUNK_TOKENS) * self.num_heads
