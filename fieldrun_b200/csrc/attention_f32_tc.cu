@@ -11,8 +11,11 @@
 //   P V            128 x VD x 64 in the same order of parts, from zero for every page: the tensor cores' adder cuts off instead of rounding, so
 //                  a page's sum is added to the query's in float32 registers, rounded, when the next page's weights are on their way;
 //   the end        the two threads of a query join their sums.
-// A query with a result that is not finite is taken again key by key: an infinity or a NaN makes its page's (its query's) parts NaNs, and
-// with them all results that the page has a part in.
+// A query is taken again key by key where a result is not finite (an infinity or a NaN makes its page's, or its query's, parts NaNs, and
+// with them all results that the page has a part in), and where parts of one scale may not hold its digits: entries 2^29 times smaller
+// than the largest of their query or page, which may be a token's that the query does not see, are off by 2^-51 of that largest.  So a
+// query keeps the largest scales of the pages that it sees, and looks at the end whether its scores could be off by what they say
+// (FT_SCORE_UNIT) and whether its result is small beside it (FT_VALUE_UNITS): a result that passes is as exact as one without such an entry.
 //
 // What bounds it: six prompts of 17 to 1,500 tokens (48 heads over 8 of 128) are 48 GFLOP, 144 of parts: 90 us at the tensor cores' rate.
 // They take 220 us and 13 for the pages' parts (tiles on mma.sync 1,115).  A page of a tile is 36 products, 1,600 cycles, and takes 1,900: a
@@ -35,6 +38,12 @@ static_assert(128 * FT_REGS_ISSUE + FT_ROW_THREADS * FT_REGS_ROWS <= FT_THREADS 
 #define FT_LARGEST 1099511627776.f         // 2^40: queries and keys beyond it have no parts; those of a query or page below
 #define FT_SMALLEST 8.6736173798840355e-19f      // 2^-60 are split with that one's scale (their products are below 2^-20 of any score)
 #define FT_NO_SHIFT 1e30f      // a query's shift before its first visible key
+// An entry that its scale leaves below 2^-13 is off by at most 2^-36.  Scores: HD products with parts of the other operand below 2^15, times
+// this unit at most: off by less than 2^-21 (2^-29 for errors of random signs), far less than the rounding of scores that large.
+#define FT_SCORE_UNIT 0.00390625f          // 2^-8
+// Results: a key's weight off by 2^-36 meets values below 2^15, beside a result of at least 2^11 of the same units: 2^-32 of it a key.  The
+// largest weight being 2^14, only values 2^18 times larger than the result make it smaller than that.
+#define FT_VALUE_UNITS 2048.f
 
 using namespace frb_tma;
 using namespace frb_tc;
@@ -125,7 +134,7 @@ attention_f32_split_kernel(F32Attention p, const int* __restrict__ seq_slot, con
     whole = top <= (values ? 3.402823466e38f : FT_LARGEST);
     const int exponent = whole ? min(14 - ilogbf(fmaxf(top, values ? 1.1754943508222875e-38f : FT_SMALLEST)), 126) : 0;
     const float scale = power_of_two(exponent);
-    if (threadIdx.x == 0) inv[(values ? (size_t)total_pages * p.num_kv_heads : 0) + (size_t)blockIdx.x * heads + head] = power_of_two(-exponent);
+    if (threadIdx.x == 0) inv[(values ? (size_t)total_pages * p.num_kv_heads : 0) + (size_t)blockIdx.x * heads + head] = top > 0.f ? power_of_two(-exponent) : 0.f;
     uint4* dst = (values ? value_parts : key_parts) + ((size_t)blockIdx.x * heads + head) * 2 * units;
 #pragma unroll
     for (int i = 0; i < MOST; ++i) {
@@ -156,8 +165,8 @@ attention_f32_tc_kernel(F32Attention p, const int* __restrict__ tile_seq, const 
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t q_full, k_full[FT_STAGES], k_empty[FT_STAGES], v_full[FT_STAGES], v_empty[FT_STAGES];
     __shared__ uint64_t s_full[2], p_full[2], o_full[2];          // of even and odd pages
-    __shared__ float q_top[2][FT_QUERIES], told[2][2][FT_QUERIES];
-    __shared__ int again[FT_QUERIES], base_slot, failed_flag;
+    __shared__ float q_top[2][FT_QUERIES], told[2][4][FT_QUERIES];
+    __shared__ int again[FT_QUERIES], held[FT_QUERIES], base_slot, failed_flag;
     __shared__ uint32_t tmem_slot;
     volatile int* failed = &failed_flag;
     constexpr uint32_t K_PART = FRB_PAGE * HD * 2, V_PART = VD * FRB_PAGE * 2;     // bytes of one part of a page
@@ -200,7 +209,7 @@ attention_f32_tc_kernel(F32Attention p, const int* __restrict__ tile_seq, const 
         failed_flag = 0;
         bar_init_fence();
     }
-    if (threadIdx.x < FT_QUERIES) again[threadIdx.x] = 0;
+    if (threadIdx.x < FT_QUERIES) again[threadIdx.x] = held[threadIdx.x] = 0;
     if (warp == 1) tmem_alloc(&tmem_slot, 512);
     if (warp == 2) {                                       // the scratch's pages before this sequence's
         int before = 0;
@@ -331,6 +340,7 @@ attention_f32_tc_kernel(F32Attention p, const int* __restrict__ tile_seq, const 
 #pragma unroll
         for (int i = 0; i < VD; ++i) o[i] = 0.f;
         float corr_before = 1.f, value_before = 0.f;       // of the page whose sums are still to be added
+        float key_largest = 0.f, value_largest = 0.f;      // of the pages that the query sees: what takes their scales off
         auto add_page = [&](int n) {
             if (!bar_wait(&o_full[e], (n >> 1) & 1, failed)) { if (ok && lane == 0) atomicExch(status, 58); ok = false; }
             __syncwarp();
@@ -401,6 +411,10 @@ attention_f32_tc_kernel(F32Attention p, const int* __restrict__ tile_seq, const 
             const float c_hi = __fmul_rd(scale, LOG2E), c_lo = fmaf(scale, LOG2E_LO, fmaf(scale, LOG2E, -c_hi));
             const float page_top = max3(fmaxf(top[0], top[1]), top[2], top[3]);
             const float shift_now = page_top == -INFINITY ? shift : fminf(shift, 14.f - page_top * c_hi);
+            if (page_top != -INFINITY) {
+                key_largest = fmaxf(key_largest, key_factor);
+                value_largest = fmaxf(value_largest, value_factor);
+            }
             const float corr = exp2_fast(shift_now - shift);
             shift = shift_now;
             const uint64_t hi_pair = pair_of(c_hi, c_hi), lo_pair = pair_of(c_lo, c_lo), shift_pair = pair_of(shift, shift);
@@ -438,6 +452,8 @@ attention_f32_tc_kernel(F32Attention p, const int* __restrict__ tile_seq, const 
         // when both groups have come here: every product has ended), chunk c of row r at chunk c ^ (r & 7).
         told[e][0][row] = shift;
         told[e][1][row] = sum;
+        told[e][2][row] = q_factor * key_largest;
+        told[e][3][row] = value_largest;
         asm volatile("bar.sync 1, %0;" ::"n"(FT_ROW_THREADS) : "memory");
         float4* mine4 = (float4*)(base + e * (FT_QUERIES * VD * 4)) + row * (VD / 4);
 #pragma unroll
@@ -456,6 +472,8 @@ attention_f32_tc_kernel(F32Attention p, const int* __restrict__ tile_seq, const 
             if (p.gate && valid) factor *= 1.0f / (1.0f + expf(-p.gate[(token0 + row) * p.gate_stride + head]));
             q_top[0][row] = w0 * factor;
             q_top[1][row] = w1 * factor;
+            if (fmaxf(told[0][2][row], told[1][2][row]) > FT_SCORE_UNIT) again[row] = 1;
+            told[0][0][row] = FT_VALUE_UNITS * fmaxf(told[0][3][row], told[1][3][row]) * (fmaxf(w0, w1) * factor);      // the least that holds its digits
         }
         asm volatile("bar.sync 1, %0;" ::"n"(FT_ROW_THREADS) : "memory");
         for (int u = threadIdx.x - 128; u < rows * (VD / 4); u += FT_ROW_THREADS) {
@@ -464,12 +482,14 @@ attention_f32_tc_kernel(F32Attention p, const int* __restrict__ tile_seq, const 
             const float wa = q_top[0][r], wb = q_top[1][r];
             const float4 y = make_float4(fmaf(a.x, wa, b.x * wb), fmaf(a.y, wa, b.y * wb), fmaf(a.z, wa, b.z * wb), fmaf(a.w, wa, b.w * wb));
             ((float4*)(p.out + ((token0 + r) * p.num_heads + head) * VD))[chunk] = y;
-            if (!(fabsf(y.x) <= 3.402823466e38f && fabsf(y.y) <= 3.402823466e38f && fabsf(y.z) <= 3.402823466e38f && fabsf(y.w) <= 3.402823466e38f) &&
-                ok && !*failed) again[r] = 1;
+            const float largest = fmaxf(fmaxf(fabsf(y.x), fabsf(y.y)), fmaxf(fabsf(y.z), fabsf(y.w)));
+            if (!(fabsf(y.x) <= 3.402823466e38f && fabsf(y.y) <= 3.402823466e38f && fabsf(y.z) <= 3.402823466e38f && fabsf(y.w) <= 3.402823466e38f)) again[r] = 1;
+            if (largest >= told[0][0][r]) held[r] = 1;
         }
         asm volatile("bar.sync 1, %0;" ::"n"(FT_ROW_THREADS) : "memory");
         const int* table = p.page_table + (size_t)seq_slot[seq] * p.max_pages;
-        for (uint32_t left = __ballot_sync(0xffffffffu, again[row] != 0 && (lane & 1) == e); left; left &= left - 1) {
+        const bool whole = ok && !*failed;
+        for (uint32_t left = __ballot_sync(0xffffffffu, valid && (again[row] != 0 || held[row] == 0) && whole && (lane & 1) == e); left; left &= left - 1) {
             const int r = quarter * 32 + __ffs(left) - 1;
             f32_query_key_by_key(p, table, head, g, vg, pos0 + r, token0 + r);
         }

@@ -505,3 +505,41 @@ def test_attention_on_tcgen05_is_as_near_to_64_bits_as_the_general_kernel(heads,
     errors = [relative(t, exact) for t in (general, tiles, got)]
     print("errors: general %.2e, tiles on mma.sync %.2e, tcgen05 %.2e" % tuple(errors))
     assert errors[2] < max(errors[1], 1.2 * errors[0])
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,maps", TC_SHAPES[:3])
+@pytest.mark.parametrize("number", [1e8, 1e12, 1e15, 1e20])
+def test_large_finite_numbers_on_tcgen05_cost_no_other_token_its_digits(heads, kv_heads, dim, vdim, maps, form, number):
+    """One large entry of a value or a key in the middle of a page, in a page of the first tokens, and in one that the windows leave out; an
+    entry of the queries that meets only zeros; a large value seen with a weight of e^-40.  Every query's head by itself: its
+    distance from the general kernel's, in units of the sum of its weights times its values' sizes, has the bounds of `check`."""
+    starts, lengths = [0, 30, 0, 100, 0, 0], [100, 90, 200, 90, 70, 90]
+    keys, values, table, gen = paged(starts, lengths, kv_heads, kv_heads // maps, dim, vdim, 13)
+    tokens, cu = sum(lengths), [0, *(int(c) for c in np.cumsum(lengths))]
+    q = torch.randn(tokens, heads * dim, device=DEV, generator=gen)
+    plant(keys, values, table, 0, 40, value=number)
+    plant(keys, values, table, 1, 40, key=number)
+    plant(keys, values, table, 2, 2, value=number)
+    plant(keys, values, table, 2, 150, key=-number, value=-number)
+    plant(keys, values, table, 3, 60, value=number)
+    plant(keys, values, table, 3, 61, key=number)
+    for page in table[4, :2].tolist():
+        keys[page, :, :, 0] = 0.0
+    q.view(tokens, heads, dim)[cu[4]:cu[5], :, 0] = number
+    one = torch.randn(dim, device=DEV, generator=gen)
+    q.view(tokens, heads, dim)[cu[5]:] = one + 0.01 * torch.randn(90, heads, dim, device=DEV, generator=gen)
+    keys[int(table[5, 0]), :, 20] = one * (-40.0 * dim ** 0.5 / (one * one).sum())
+    plant(keys, values, table, 5, 20, value=1e17)
+    common = dict(num_heads=heads, num_kv_heads=kv_heads, head_dim=dim, v_dim=vdim, scale=dim ** -0.5, maps=maps,
+                  **options(form, heads, tokens, gen))
+    pos = i32(np.concatenate([s + np.arange(n) for s, n in zip(starts, lengths)]))
+    slots = i32(np.repeat(np.arange(6), lengths))
+    want, size, got = (torch.full((tokens, heads * vdim), NAN, device=DEV) for _ in range(3))
+    ops().attention_generic(q, keys, values, table, pos, slots, want, **common)
+    ops().attention_generic(q, keys, values.abs(), table, pos, slots, size, **common)
+    attention_on_tcgen05(q, keys, values, table, starts, lengths, got, **common)
+    assert got.isfinite().all()
+    error = (got - want).abs().view(tokens, heads, vdim).amax(2) / size.view(tokens, heads, vdim).amax(2)
+    print("largest error of each sequence:", [error[a:b].max().item() for a, b in zip(cu, cu[1:])])
+    assert error.max() < (128 + 200 / 8) * 2.0 ** -24
