@@ -18,8 +18,9 @@
 // tokens inside a block and up to 48 between blocks: a rounding of their logarithms, which are large only where the weight is small.
 //
 // Everything is float32; the products run on tensor cores with each operand as two parts (tf32_parts.cuh: sums of 16 entries, added in
-// float32 registers; f16_parts.cuh: of at most 128).  Four prompts of 2,048 tokens, 16 heads of 128 x 128 over 4 key heads: 340 us (34 +
-// 151 + 118 + 34 for the launches in turn; delta_rule.cu token by token 1,387).  With launch 1's products made by launch 2 for every head, and
+// float32 registers; f16_parts.cuh: of at most 128).  Four prompts of 2,048 tokens, 16 heads of 128 x 128 over 4 key heads: 350 us (35 +
+// 154 + 134 + 35 for the launches in turn; 34 + 151 + 130 + 34 without the scales of single rows and the look at the outputs that they are
+// for; delta_rule.cu token by token 1,367).  With launch 1's products made by launch 2 for every head, and
 // launch 3 on mma.sync, 589 (189 + 368 + 34).  Launch 2 is bound by the instructions of its substitution, two entries each (one
 // each: 168 us), and by the latencies before it, two blocks an SM; launch 3 by the chain of its phases.
 #include "f16_parts.cuh"
@@ -30,9 +31,8 @@
 #define DC_BLOCKS (DC_TOKENS / DC_BLOCK)
 #define DC_SLICE 64           // value columns a block of launch 2 keeps
 #define DC_LM (DC_TOKENS + 8)
-#define DC_FACTORS (3 * DC_TOKENS + 4)
+#define DC_FACTORS (4 * DC_TOKENS + 4)
 #define DC_W_SCALE 8          // exponents of the parts' scales
-#define DC_Q_SCALE 17
 #define DC_K_SCALE 14
 
 struct DeltaChunks {
@@ -52,11 +52,11 @@ struct DeltaChunks {
     float* decays;           // [chunks][heads]: w(end)
     // for the chain on tcgen05, in place of w and pairs: their parts, and the unit keys' and queries'
     uint16_t* w_parts;       // [chunks][heads][part][dim / 64][DC_TOKENS][64], the row times 2^8 / (a power of two about w(i))
-    uint16_t* pair_parts;    // [chunks][heads][part][DC_TOKENS][DC_TOKENS], times 2^17
-    uint16_t *q_parts, *k_parts;     // [chunks][kv_heads][part][dim / 64][DC_TOKENS][64], times 2^17 and 2^14
+    uint16_t* pair_parts;    // [chunks][heads][part][DC_TOKENS][DC_TOKENS], rows with a scale each
+    uint16_t *q_parts, *k_parts;     // [chunks][kv_heads][part][dim / 64][DC_TOKENS][64], queries with a scale each, keys times 2^14
     float* raw_pairs;        // [chunks][kv_heads][2][DC_TOKENS][DC_TOKENS]: the unit keys' products [j][i], the queries' with them [i][j], j <= i
-    float* norms;            // [chunks][kv_heads][2][DC_TOKENS]: what makes the queries (with dim^(-1/2)) and keys unit vectors
-    float* factors;          // [chunks][heads][DC_FACTORS]: what takes w's scale off; w(i) 2^-17; w(j, end); w(end)
+    float* norms;            // [chunks][kv_heads][3][DC_TOKENS]: what makes the queries (with dim^(-1/2)) and keys unit vectors; the queries' scales off
+    float* factors;          // [chunks][heads][DC_FACTORS]: w's scale off; w(i), the query's scale off; w(j, end); the pairs' scales off; w(end)
     int conv_stride, q_off, k_off, v_off, proj_stride, b_off, a_off, g_off, heads, kv_heads;
     float eps;
 };
@@ -83,7 +83,7 @@ template <int DIM, bool PARTS>
 __global__ void __launch_bounds__(256, 2) delta_chunk_pairs_kernel(DeltaChunks p) {
     constexpr int LQ = DIM + 8;
     extern __shared__ float4 dc_smem[];
-    __shared__ float q_inv[DC_TOKENS], k_inv[DC_TOKENS];
+    __shared__ float q_inv[DC_TOKENS], k_inv[DC_TOKENS], q_scale[DC_TOKENS];
     float* q_s = (float*)dc_smem;                   // [DC_TOKENS][LQ]
     float* k_s = q_s + DC_TOKENS * LQ;              // [DC_TOKENS][LQ]
     const int item = blockIdx.x, kvh = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -97,21 +97,28 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_pairs_kernel(DeltaChunks p
     copies_wait<0>();
     __syncthreads();
     for (int t = warp; t < DC_TOKENS; t += 8) {
-        float qq = 0.f, kk = 0.f;
+        float qq = 0.f, kk = 0.f, q_top = 0.f;
 #pragma unroll
         for (int d = 0; d < DIM; d += 32) {
             const float x = q_s[t * LQ + d + lane], y = k_s[t * LQ + d + lane];
             qq = fmaf(x, x, qq);
             kk = fmaf(y, y, kk);
+            q_top = fmaxf(q_top, fabsf(x));
         }
         qq = warp_sum(qq);
         kk = warp_sum(kk);
+        if (PARTS) q_top = warp_max(q_top);
         if (lane == 0) {
             const float q = 1.0f / sqrtf((float)DIM) / sqrtf(qq + 1e-6f), k = 1.0f / sqrtf(kk + 1e-6f);
             q_inv[t] = q;
             k_inv[t] = k;
-            p.norms[at * 2 * DC_TOKENS + t] = q;
-            p.norms[at * 2 * DC_TOKENS + DC_TOKENS + t] = k;
+            p.norms[at * 3 * DC_TOKENS + t] = q;
+            p.norms[at * 3 * DC_TOKENS + DC_TOKENS + t] = k;
+            if (PARTS) {
+                const int exponent = parts_exponent(q_top * q);
+                q_scale[t] = q * power_of_two(exponent);
+                p.norms[at * 3 * DC_TOKENS + 2 * DC_TOKENS + t] = q_top > 0.f ? power_of_two(-exponent) : 0.f;
+            }
         }
     }
     __syncthreads();
@@ -122,7 +129,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_pairs_kernel(DeltaChunks p
             const bool key = u >= UNITS;
             const int r = u % UNITS / (DIM / 8), c = u % (DIM / 8) * 8;
             const float* from = (key ? k_s : q_s) + r * LQ + c;
-            const float scale = (key ? k_inv[r] : q_inv[r]) * power_of_two(key ? DC_K_SCALE : DC_Q_SCALE);
+            const float scale = key ? k_inv[r] * power_of_two(DC_K_SCALE) : q_scale[r];
             uint4 hi, lo;
             split_four(*(const float4*)from, scale, hi.x, hi.y, lo.x, lo.y);
             split_four(*(const float4*)(from + 4), scale, hi.z, hi.w, lo.z, lo.w);
@@ -242,7 +249,8 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
     if (tid < DC_TOKENS)
         for (int m = tid / DC_BLOCK + 1; m < DC_BLOCKS; ++m) rest += block_log[m];
     after_previous_kernel();                         // launch 1, whose products come from here on; it began when the rows were there
-    if (tid < 2 * DC_TOKENS) (tid < DC_TOKENS ? q_inv : k_inv)[tid % DC_TOKENS] = p.norms[kv_at * 2 * DC_TOKENS + tid];
+    // (with PARTS what takes the queries' scales off in the place of their norms, which are in their parts)
+    if (tid < 2 * DC_TOKENS) (tid < DC_TOKENS ? q_inv : k_inv)[tid % DC_TOKENS] = p.norms[kv_at * 3 * DC_TOKENS + (PARTS && tid < DC_TOKENS ? 2 * DC_TOKENS : 0) + tid];
     __syncthreads();
     if (tid < DC_TOKENS) {
         const float to_end = from_s[tid] * expf(rest);
@@ -251,9 +259,9 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
             const int exponent = dc_w_exponent(start_s[tid]);
             w_scale[tid] = power_of_two(exponent);
             factors[tid] = power_of_two(-exponent);
-            factors[DC_TOKENS + tid] = start_s[tid] * power_of_two(-DC_Q_SCALE);
+            factors[DC_TOKENS + tid] = start_s[tid] * q_inv[tid];
             factors[2 * DC_TOKENS + tid] = to_end;
-            if (tid == DC_TOKENS - 1) factors[3 * DC_TOKENS] = start_s[tid];
+            if (tid == DC_TOKENS - 1) factors[4 * DC_TOKENS] = start_s[tid];
         } else {
             p.q_factor[at * DC_TOKENS + tid] = start_s[tid] * q_inv[tid];
             p.k_factor[at * DC_TOKENS + tid] = to_end * k_inv[tid];
@@ -292,10 +300,17 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
             for (int e = 0; e < 8; ++e)
                 if (j0 + e <= i) y[e] = r[e] * weight(i, j0 + e);
         }
-        if (PARTS) {
+        if (PARTS) {                                 // eight neighbouring threads have a row
+            float top = 0.f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) top = fmaxf(top, fabsf(y[e]));
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+            const int exponent = parts_exponent(top);
+            if (j0 == 0) p.factors[at * DC_FACTORS + 3 * DC_TOKENS + i] = top > 0.f ? power_of_two(-exponent) : 0.f;
             uint4 hi, lo;
-            split_four(make_float4(y[0], y[1], y[2], y[3]), power_of_two(DC_Q_SCALE), hi.x, hi.y, lo.x, lo.y);
-            split_four(make_float4(y[4], y[5], y[6], y[7]), power_of_two(DC_Q_SCALE), hi.z, hi.w, lo.z, lo.w);
+            split_four(make_float4(y[0], y[1], y[2], y[3]), power_of_two(exponent), hi.x, hi.y, lo.x, lo.y);
+            split_four(make_float4(y[4], y[5], y[6], y[7]), power_of_two(exponent), hi.z, hi.w, lo.z, lo.w);
             uint16_t* to = p.pair_parts + at * 2 * DC_TOKENS * DC_TOKENS + piece_place(i, j0);
             *(uint4*)to = hi;
             *(uint4*)(to + DC_TOKENS * DC_TOKENS) = lo;
@@ -553,8 +568,8 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_chain_kernel(DeltaChunks p
 // The columns' parts have a power of two of their own each, from the largest entry of the state or of u.  What bounds it: the chain of a
 // chunk's phases, 6,300 cycles (11.5 us on mma.sync): the first product 1,150, the third 1,250, the state's split 1,250, u and its two
 // splits 2,000, the new state 560; the SMs that have a sequence's head, 64 of them for four prompts in sixteen heads, issue an
-// instruction on nearly every cycle of the splits.  A column with a number that is not finite, or with a token 2^28 times larger than the first of its chunk, makes the block
-// take the sequence's head again, token by token.
+// instruction on nearly every cycle of the splits.  A number that is not finite, or a token whose outputs may have lost digits (PARTS_LEAST),
+// makes the block take the sequence's head again, token by token.
 #define DT_SHARES 2            // threads a column: each half of its entries and of a chunk's tokens (four: 127 us instead of 118)
 #define DT_WARPS (4 * DT_SHARES)
 #define DT_ROWS (32 * DT_WARPS)
@@ -621,8 +636,9 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(Del
     constexpr int S_HI = 0, S_LO = DIM / 2, D1_W = 128, D1_Q = 192, UK = 256, D_O = 320, D_S = 384;
     extern __shared__ uint8_t dt_smem[];
     __shared__ uint64_t w_full, q_full, k_full, pairs_full, u_full, s_ready, u_ready, d1w_done, d1q_done, ds_done, do_done, o_stored, o_free;
-    __shared__ float tops[4][DT_SHARES][VDIM];
-    __shared__ __align__(16) float factors[2][DC_FACTORS];
+    __shared__ float tops[3][DT_SHARES][VDIM];
+    __shared__ int first_rows[DT_SHARES][4];
+    __shared__ __align__(16) float factors[3][DC_FACTORS];               // of chunk c at c % 3: a chunk's are read until the next one's state is split
     __shared__ uint32_t tmem_slot;
     __shared__ int failed_flag, odd_numbers;
     volatile int* failed = &failed_flag;
@@ -662,7 +678,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(Del
                 if (c && !bar_wait(&d1w_done, before, failed)) { atomicExch(status, 61); break; }
                 bar_expect(&w_full, 2 * ROWS_PART + DC_FACTORS * 4);
                 copy_bulk(w_s, p.w_parts + at * 2 * DC_TOKENS * DIM, 2 * ROWS_PART, &w_full);
-                copy_bulk(factors[c & 1], p.factors + at * DC_FACTORS, DC_FACTORS * 4, &w_full);
+                copy_bulk(factors[c % 3], p.factors + at * DC_FACTORS, DC_FACTORS * 4, &w_full);
                 if (c && !bar_wait(&u_ready, before, failed)) { atomicExch(status, 73); break; }
                 bar_expect(&u_full, DC_TOKENS * VDIM * 4);
                 copy_bulk(u_s, p.u + at * DC_TOKENS * VDIM, DC_TOKENS * VDIM * 4, &u_full);
@@ -751,33 +767,55 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(Del
         uint64_t finite = 0ull;                      // becomes NaNs at the first number that is not finite
 #pragma unroll
         for (int d = 0; d < SHARE; ++d) S[d] = (kept + (start & 1) * p.copy_floats)[(size_t)d * VDIM];
-        float u_inv = 0.f;
+        float u_inv = 0.f, s_least = 0.f, u_least = 0.f;
+        int first_token = 0;
         auto write_outputs = [&](int c) {            // what u gives the outputs of chunk c, behind what its state gave
+            const float4* f4 = (const float4*)factors[c % 3];
             wait(&do_done, c & 1, 72);
             uint32_t v[DT_TOKENS / 16][16];
             load_columns<DT_TOKENS>(lanes + D_O + t0, v);
             tmem_wait_ld();
             if (c > 0) wait(&o_free, (c & 1) ^ 1, 75);           // the copies of the chunk before have read its outputs
+            float smallest = INFINITY;               // of the column's outputs
 #pragma unroll
-            for (int t = 0; t < DT_TOKENS; ++t) {
-                o[t] = fmaf(__uint_as_float(v[t / 16][t % 16]), u_inv, o[t]);
-                o_s[(t0 + t) * VDIM + column] = o[t];
+            for (int t = 0; t < DT_TOKENS; t += 4) {
+                const float4 fp = f4[(3 * DC_TOKENS + t0 + t) / 4];
+                const uint64_t ps[2] = {pair_of(fp.x, fp.y), pair_of(fp.z, fp.w)};
+#pragma unroll
+                for (int i = 0; i < 4; i += 2) {
+                    const uint64_t sums = pair_of(__uint_as_float(v[(t + i) / 16][(t + i) % 16]), __uint_as_float(v[(t + i) / 16][(t + i) % 16 + 1]));
+                    const uint64_t y = fma_pairs(sums, mul_pairs(pair_of(u_inv, u_inv), ps[i / 2]), pair_of(o[t + i], o[t + i + 1]));
+                    float y0, y1;
+                    halves_of(y, y0, y1);
+                    smallest = min3(smallest, fabsf(y0), fabsf(y1));
+                    finite = fma_pairs(y, 0ull, finite);
+                    o_s[(t0 + t + i) * VDIM + column] = y0;
+                    o_s[(t0 + t + i + 1) * VDIM + column] = y1;
+                }
+            }
+            // Queries and pairs' weights are at most dim^(-1/2), so that what takes their scales off is at most 2^-17.  Where no column has
+            // outputs that are all large enough by that: a token's row at a time; one before the first that is not zero may be of zeros.
+            if (!__any_sync(0xffffffffu, smallest >= (s_least + u_least) * power_of_two(-17))) {
+                for (int t = t0; t < t0 + DT_TOKENS; ++t) {
+                    const float from_state = s_least * factors[c % 3][DC_TOKENS + t];
+                    const float least = t < first_token ? from_state : fmaf(u_least, factors[c % 3][3 * DC_TOKENS + t], from_state);
+                    if (!__any_sync(0xffffffffu, fabsf(o_s[t * VDIM + column]) >= least)) finite = pair_of(NAN, NAN);
+                }
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) bar_arrive(&o_stored);
-#pragma unroll
-            for (int t = 0; t < DT_TOKENS; t += 2) finite = fma_pairs(pair_of(o[t], o[t + 1]), 0ull, finite);
         };
         for (int c = 0; c < chunks; ++c) {
             const uint32_t phase = c & 1;
-            const float4* f4 = (const float4*)factors[c & 1];            // W's, the queries' and the keys' factors, sixteen of four each
+            const float4* f4 = (const float4*)factors[c % 3];            // W's, the queries' and the keys' factors, sixteen of four each
             float top[2] = {0.f, 0.f};
 #pragma unroll
             for (int d = 0; d < SHARE; d += 2) top[d / 2 & 1] = max3(top[d / 2 & 1], fabsf(S[d]), fabsf(S[d + 1]));
             tops[0][share][column] = fmaxf(top[0], top[1]);
             meet();
-            const int s_exponent = parts_exponent(largest(0));
+            const float s_top = largest(0);
+            const int s_exponent = parts_exponent(s_top);
             store_parts(S, power_of_two(s_exponent), lanes + S_HI + share * (SHARE / 2), lanes + S_LO + share * (SHARE / 2));
             tmem_wait_st();
             // the factors came with W: waited for before s_ready, behind which the next chunk's may come and end the barrier's next phase
@@ -815,12 +853,10 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(Del
             fence_before_sync();                                         // D1's columns are read before another share's parts go over them
             tops[1][share][column] = u_top;
             tops[2][share][column] = uk_top;
-            if (share == 0) tops[3][0][column] = first_row_top(u);
+            const int first_here = first_row(u);
+            if (lane == 0) first_rows[share][quarter] = first_here;
             meet();
             u_top = largest(1);
-            // parts of one scale: a token so much larger than those before it would cost them their digits
-            const float first_top = tops[3][0][column];
-            if (first_top != 0.f && first_top < u_top * 3.725290298461914e-09f) finite = pair_of(NAN, NAN);       // 2^-28
             const int u_exponent = parts_exponent(u_top), uk_exponent = parts_exponent(largest(2));
             fence_after_sync();
             store_parts(uk, power_of_two(uk_exponent), lanes + UK + t0 / 2, lanes + UK + 32 + t0 / 2);
@@ -829,7 +865,10 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(Del
             fence_before_sync();
             __syncwarp();
             if (lane == 0) bar_arrive(&u_ready);
-            u_inv = power_of_two(-u_exponent) * power_of_two(-DC_Q_SCALE);
+            u_inv = power_of_two(-u_exponent);
+            s_least = PARTS_LEAST * warp_unit(s_top, s_exponent);
+            u_least = PARTS_LEAST * warp_unit(u_top, u_exponent);
+            first_token = first_rows[0][quarter] < DT_TOKENS ? first_rows[0][quarter] : DT_TOKENS + first_rows[1][quarter];
 
             // what the state gives the outputs, then the new state
             wait(&d1q_done, phase, 70);
@@ -842,7 +881,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(Del
 #pragma unroll
                 for (int i = 0; i < 4; ++i) o[t + i] = __uint_as_float(v[(t + i) / 16][(t + i) % 16]) * (s_inv * qs[i]);
             }
-            const float decay = factors[c & 1][3 * DC_TOKENS], uk_inv = power_of_two(-uk_exponent) * power_of_two(-DC_K_SCALE);
+            const float decay = factors[c % 3][4 * DC_TOKENS], uk_inv = power_of_two(-uk_exponent) * power_of_two(-DC_K_SCALE);
             wait(&ds_done, phase, 71);
             uint32_t fresh[SHARE / 16][16];
             load_columns<SHARE>(lanes + D_S + share * SHARE, fresh);
@@ -851,11 +890,12 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(Del
             for (int d = 0; d < SHARE; d += 2) {
                 const uint64_t now = fma_pairs(pair_of(S[d], S[d + 1]), pair_of(decay, decay),
                                                mul_pairs(pair_of(__uint_as_float(fresh[d / 16][d % 16]), __uint_as_float(fresh[d / 16][d % 16 + 1])), pair_of(uk_inv, uk_inv)));
-                finite = fma_pairs(now, 0ull, finite);
                 halves_of(now, S[d], S[d + 1]);
             }
         }
         if (chunks > 0) write_outputs(chunks - 1);
+#pragma unroll
+        for (int d = 0; d < SHARE; d += 2) finite = fma_pairs(pair_of(S[d], S[d + 1]), 0ull, finite);        // an earlier one reached the outputs
         float even, odd;
         halves_of(finite, even, odd);
         if (even != 0.f || odd != 0.f) odd_numbers = 1;
@@ -906,7 +946,7 @@ __global__ void __launch_bounds__(256) delta_chunk_finish_kernel(DeltaChunks p, 
 // ----------------------------------------------------------------------------- host side
 
 // Chunks of at most 64 tokens: chunk_seq/begin/end and, per sequence, its first chunk (one entry more at the end).  raw: num_rows *
-// heads * vdim floats; scratch: num_chunks * (heads * (64 (dim + vdim + 64 + 3) + 4) + 128 kv_heads (dim + 65)) floats.  status: one int on
+// heads * vdim floats; scratch: num_chunks * (heads * (64 (dim + vdim + 64 + 4) + 4) + 64 kv_heads (2 dim + 131)) floats.  status: one int on
 // the device, zero before the call.
 FRB_API int frb_delta_chunks(const float* conv, int conv_stride, int q_off, int k_off, int v_off, const float* proj, int proj_stride, int b_off,
                              int a_off, int g_off, const float* a_log, const float* dt_bias, const float* norm, const int* seq_slot,

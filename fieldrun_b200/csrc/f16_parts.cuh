@@ -83,15 +83,29 @@ __device__ __forceinline__ void load_columns(uint32_t from, uint32_t (&v)[N / 16
 // The exponent of the power of two that brings `top` to [2^14, 2^15); of a smaller one than 2^-100 as if it were that, of a NaN too.
 __device__ __forceinline__ int parts_exponent(float top) { return 14 - ilogbf(fminf(fmaxf(top, 7.888609052210118e-31f), 3.402823466e38f)); }
 
-// The largest entry over the warp's columns of the first of eight tokens that has one; zero: none has.  (A single column's may be as
-// small as chance has it.)
+// Parts of one scale hold the digits of entries down to 2^-29 of the largest; smaller ones are off by up to 2^-51 of it, and with them the
+// sums that they alone make.  Whether that counts is seen at the sums: in units of the scales, products of parts below 2^15 whose errors
+// are up to 2^-21 each.  A warp's row of 32 sums with one of PARTS_LEAST units or more is off by 2^-31 of it a product, at most 2^-24 with 128.
+#define PARTS_LEAST 1024.f
+
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float d;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
+// The unit of the warp's columns: the largest of what takes their scales off, a column of zeros aside.
+__device__ __forceinline__ float warp_unit(float top, int exponent) {
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, top > 0.f ? __float_as_uint(power_of_two(-exponent)) : 0u));
+}
+
+// The first of the warp's rows with an entry that is not zero; N: none.
 template <int N>
-__device__ __forceinline__ float first_row_top(const float (&u)[N]) {
-    uint32_t top = 0;
+__device__ __forceinline__ int first_row(const float (&u)[N]) {
+    if (__any_sync(0xffffffffu, u[0] != 0.f)) return 0;
+    int first = N;
 #pragma unroll
-    for (int t = 7; t >= 0; --t) {
-        const uint32_t row = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(u[t])));
-        if (row != 0) top = row;
-    }
-    return __uint_as_float(top);
+    for (int t = N - 1; t > 0; --t)
+        if (__any_sync(0xffffffffu, u[t] != 0.f)) first = t;
+    return first;
 }

@@ -1263,8 +1263,8 @@ def delta_chunks_take(dim: int, vdim: int, conv_offsets: tuple, state: torch.Ten
 
 def delta_chunks_scratch_floats(chunks: int, heads: int, dim: int, vdim: int, kv_heads: Optional[int] = None) -> int:
     """float32 elements of scratch that :func:`delta_chunks` needs."""
-    return chunks * (heads * (DELTA_CHUNK_TOKENS * (dim + vdim + DELTA_CHUNK_TOKENS + 3) + 4)
-                     + 2 * (heads if kv_heads is None else kv_heads) * DELTA_CHUNK_TOKENS * (dim + DELTA_CHUNK_TOKENS + 1))
+    return chunks * (heads * (DELTA_CHUNK_TOKENS * (dim + vdim + DELTA_CHUNK_TOKENS + 4) + 4)
+                     + (heads if kv_heads is None else kv_heads) * DELTA_CHUNK_TOKENS * (2 * (dim + DELTA_CHUNK_TOKENS) + 3))
 
 
 def delta_chunks(conv: torch.Tensor, q_off: int, k_off: int, v_off: int, proj: torch.Tensor, b_off: int, a_off: int, g_off: int,

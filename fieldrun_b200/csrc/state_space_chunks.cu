@@ -14,8 +14,9 @@
 //
 // Everything is float32; launch 1's products run on mma.sync in TF32 parts (tf32_parts.cuh), sums of 16 entries, added in float32
 // registers; launch 3's on tcgen05 in float16 parts (f16_parts.cuh), over at most 128 entries.
-// Four prompts of 2,048 tokens, 64 heads of 128 x 64 in 8 groups: 44 + 45 + 179 us, against 676 us of four launches on mma.sync with a
-// state written and read for every chunk of 128 tokens (states 189, chain 65, outputs 382, pairs 40), and 1,210 token by token.
+// Four prompts of 2,048 tokens, 64 heads of 128 x 64 in 8 groups: 45 + 45 + 184 us (181 without the look for outputs that may have lost
+// digits), against 676 us of four launches on mma.sync with a state written and read for every chunk of 128 tokens (states 189, chain
+// 65, outputs 382, pairs 40), and 1,210 token by token.
 #include "f16_parts.cuh"
 #include "tf32_parts.cuh"
 
@@ -25,6 +26,7 @@
 #define SC_BLOCKS (SC_TOKENS / SC_BLOCK)
 #define SC_COLUMNS 128        // value columns of a block of launch 3
 #define SC_FACTORS (4 * SC_TOKENS + 4)
+#define SC_B_FAR 1048576.f    // 2^20: a new state is then off by less than 2^-24 of its columns' largest (64 products, 2^-50 each)
 
 using namespace frb_tma;
 using namespace frb_tc;
@@ -113,8 +115,8 @@ __global__ void __launch_bounds__(256, 2) state_space_pairs_kernel(StateSpaceChu
     const float b0 = b_top[lane], b1 = b_top[lane + 32], large = warp_max(fmaxf(b0, b1));
     const float least = -warp_max(-fminf(b0 > 0.f ? b0 : INFINITY, b1 > 0.f ? b1 : INFINITY));
     const int b_exponent = parts_exponent(large);
-    if (tid < SC_TOKENS) p.scales[at * (SC_TOKENS + 4) + tid] = power_of_two(-parts_exponent(c_top[tid]));
-    if (tid == 0) p.scales[at * (SC_TOKENS + 4) + SC_TOKENS] = least * 67108864.f < large ? NAN : power_of_two(-b_exponent);          // 2^26
+    if (tid < SC_TOKENS) p.scales[at * (SC_TOKENS + 4) + tid] = c_top[tid] > 0.f ? power_of_two(-parts_exponent(c_top[tid])) : 0.f;
+    if (tid == 0) p.scales[at * (SC_TOKENS + 4) + SC_TOKENS] = least * SC_B_FAR < large ? NAN : power_of_two(-b_exponent);
     for (int u = tid; u < 2 * UNITS; u += 256) {
         const bool is_b = u >= UNITS;
         const int r = u % UNITS / (N / 8), c = u % (N / 8) * 8;
@@ -236,7 +238,7 @@ __global__ void __launch_bounds__(128) state_space_weights_kernel(StateSpaceChun
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
         const int exponent = parts_exponent(top);
-        if (j0 == 0) factors[SC_TOKENS + i] = power_of_two(-exponent);
+        if (j0 == 0) factors[SC_TOKENS + i] = top > 0.f ? power_of_two(-exponent) : 0.f;
         uint4 hi, lo;
         split_four(make_float4(y[0], y[1], y[2], y[3]), power_of_two(exponent), hi.x, hi.y, lo.x, lo.y);
         split_four(make_float4(y[4], y[5], y[6], y[7]), power_of_two(exponent), hi.z, hi.w, lo.z, lo.w);
@@ -250,11 +252,11 @@ __global__ void __launch_bounds__(128) state_space_weights_kernel(StateSpaceChun
 // each, in float32, and half of a chunk's tokens.  The products of parts of a chunk:
 //     DS = (u w(j, end))^T B   128 x N x 64, B's rows N-major;    D1 = S^T C^T   128 x 64 x N;    DO = u^T P^T   128 x 64 x 64, with two heads
 //     128 x 64 x 128: a head's columns have u in their half of the inner size and zeros in the other's.
-// The columns' parts have a power of two of their own each, from the largest entry of the state or of u.  Eight more warps take the
+// The columns' parts have a power of two of their own each, from the largest entry of the state, of u or of u w(j, end).  Eight more warps take the
 // outputs through D x and the gate while the next chunk is made: with these in the columns' warps a chunk took 4,000 cycles more.  A chunk is
-// bound by the instructions of both, 9,000 to 10,000 cycles: the columns' splits 1,900, u 1,300, the waits for the products 1,900, the outputs' gates 4,000.  A column with a number that is not finite, or with a token 2^28 times
-// larger than the first of its chunk, or a chunk whose rows of B lie 2^26 apart, makes the block take its columns of the sequence
-// again, token by token.
+// bound by the instructions of both, 9,000 to 10,000 cycles: the columns' splits 1,900, u 1,300, the waits for the products 1,900, the
+// outputs' gates 4,000.  A number that is not finite, a token whose sums may have lost digits (PARTS_LEAST), or a chunk whose rows of B lie 2^20 apart makes the block take its
+// columns of the sequence again, token by token.
 #define ST_THREADS 640         // warps 0 copies, 1 products; 4-11 the columns' two halves (w & 3: lanes), 12-19 the outputs
 #define ST_ROWS 256
 #define ST_SHARE_TOKENS (SC_TOKENS / 2)
@@ -309,6 +311,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) state_space_chain_kernel(const 
     extern __shared__ uint8_t st_smem[];
     __shared__ uint64_t x_full, b_full, c_full, pairs_full, ready, d1_done, ds_done, do_done, o_stored, o_free[2];
     __shared__ float tops[3][2][SC_COLUMNS];
+    __shared__ int first_rows[2][4];
     __shared__ __align__(16) float factors[2][HEADS][SC_FACTORS];
     __shared__ uint32_t tmem_slot;
     __shared__ int failed_flag, odd_numbers;
@@ -432,7 +435,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) state_space_chain_kernel(const 
             const float4* f4 = (const float4*)factors[c & 1][hh];        // sixteen of four each: D1's, DO's, w(j, end), dt
             const int count = p.tokens_of(first + c);
             wait(&x_full, phase, 88);                // and the factors; what they overwrite was used before the chunk before was ready
-            float u[ST_SHARE_TOKENS], u_top = 0.f, s_top = 0.f;
+            float u[ST_SHARE_TOKENS], u_top = 0.f, ue_top = 0.f, s_top = 0.f;
 #pragma unroll
             for (int t = 0; t < ST_SHARE_TOKENS; ++t) u[t] = x_s[((c & 1) * SC_TOKENS + t0 + t) * SC_COLUMNS + column];
 #pragma unroll
@@ -447,19 +450,30 @@ __global__ void __launch_bounds__(ST_THREADS, 1) state_space_chain_kernel(const 
                     if (t0 + t >= count) u[t] = 0.f;
             }
 #pragma unroll
-            for (int t = 0; t < ST_SHARE_TOKENS; t += 2) u_top = max3(u_top, fabsf(u[t]), fabsf(u[t + 1]));
+            for (int t = 0; t < ST_SHARE_TOKENS; t += 4) {
+                const float4 fe = f4[(2 * SC_TOKENS + t0 + t) / 4];
+                u_top = max3(max3(u_top, fabsf(u[t]), fabsf(u[t + 1])), fabsf(u[t + 2]), fabsf(u[t + 3]));
+                float e[4];
+                halves_of(mul_pairs(pair_of(u[t], u[t + 1]), pair_of(fe.x, fe.y)), e[0], e[1]);
+                halves_of(mul_pairs(pair_of(u[t + 2], u[t + 3]), pair_of(fe.z, fe.w)), e[2], e[3]);
+                ue_top = max3(max3(ue_top, fabsf(e[0]), fabsf(e[1])), fabsf(e[2]), fabsf(e[3]));
+            }
 #pragma unroll
             for (int n = 0; n < SHARE; n += 2) s_top = max3(s_top, fabsf(S[n]), fabsf(S[n + 1]));
             tops[0][share][column] = s_top;
             tops[1][share][column] = u_top;
-            if (share == 0) tops[2][0][column] = first_row_top(u);
+            tops[2][share][column] = ue_top;
+            const int first_here = first_row(u);
+            if (lane == 0) first_rows[share][quarter] = first_here;
             fence_before_sync();                     // DO's columns are read before the state's parts go over them
             meet();
             fence_after_sync();
+            s_top = fmaxf(tops[0][0][column], tops[0][1][column]);
             u_top = fmaxf(tops[1][0][column], tops[1][1][column]);
-            const float first_top = tops[2][0][column];
-            if (first_top != 0.f && first_top < u_top * 3.725290298461914e-09f) finite = pair_of(NAN, NAN);         // 2^-28
-            const int s_exponent = parts_exponent(fmaxf(tops[0][0][column], tops[0][1][column])), u_exponent = parts_exponent(u_top);
+            const int s_exponent = parts_exponent(s_top), u_exponent = parts_exponent(u_top);
+            const int ue_exponent = parts_exponent(fmaxf(tops[2][0][column], tops[2][1][column]));
+            const float s_least = PARTS_LEAST * warp_unit(s_top, s_exponent), u_least = PARTS_LEAST * warp_unit(u_top, u_exponent);
+            const int first_token = first_rows[0][quarter] < ST_SHARE_TOKENS ? first_rows[0][quarter] : ST_SHARE_TOKENS + first_rows[1][quarter];
             store_parts(S, power_of_two(s_exponent), lanes + S_HI + share * (SHARE / 2), lanes + S_LO + share * (SHARE / 2));
             store_parts(u, power_of_two(u_exponent), lanes + U_HI + hh * 32 + t0 / 2, lanes + U_LO + hh * 32 + t0 / 2);
 #pragma unroll
@@ -468,7 +482,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) state_space_chain_kernel(const 
                 halves_of(mul_pairs(pair_of(u[t], u[t + 1]), pair_of(fe.x, fe.y)), u[t], u[t + 1]);
                 halves_of(mul_pairs(pair_of(u[t + 2], u[t + 3]), pair_of(fe.z, fe.w)), u[t + 2], u[t + 3]);
             }
-            store_parts(u, power_of_two(u_exponent), lanes + UE_HI + t0 / 2, lanes + UE_LO + t0 / 2);
+            store_parts(u, power_of_two(ue_exponent), lanes + UE_HI + t0 / 2, lanes + UE_LO + t0 / 2);
             tmem_wait_st();
             fence_before_sync();
             __syncwarp();
@@ -476,7 +490,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) state_space_chain_kernel(const 
 
             // the new state, then the outputs
             const float decay = factors[c & 1][hh][4 * SC_TOKENS], s_inv = power_of_two(-s_exponent), u_inv = power_of_two(-u_exponent);
-            const float ue_inv = u_inv * factors[c & 1][hh][4 * SC_TOKENS + 1];
+            const float ue_inv = power_of_two(-ue_exponent) * factors[c & 1][hh][4 * SC_TOKENS + 1];
             wait(&ds_done, phase, 89);
 #pragma unroll
             for (int n0 = 0; n0 < SHARE; n0 += 32) {
@@ -508,18 +522,29 @@ __global__ void __launch_bounds__(ST_THREADS, 1) state_space_chain_kernel(const 
             load_columns<32>(lanes + D_O + t0, v);
             tmem_wait_ld();
             if (c > 0) wait(&o_free[phase ^ 1], (c - 1) >> 1 & 1, 92);       // the chunk before has been read
+            float spare = INFINITY;                  // by how much the column's sums exceed the least that holds its digits
 #pragma unroll
             for (int t = 0; t < ST_SHARE_TOKENS; t += 4) {
-                const float4 f = f4[(SC_TOKENS + t0 + t) / 4];
-                const uint64_t fs[2] = {pair_of(f.x, f.y), pair_of(f.z, f.w)};
+                const float4 f = f4[(SC_TOKENS + t0 + t) / 4], g4 = f4[(t0 + t) / 4];
+                const uint64_t fs[2] = {pair_of(f.x, f.y), pair_of(f.z, f.w)}, gs[2] = {pair_of(g4.x, g4.y), pair_of(g4.z, g4.w)};
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
                     const uint64_t y = fma_pairs(sums_at(t + 2 * i), mul_pairs(pair_of(u_inv, u_inv), fs[i]), o[t / 2 + i]);
                     finite = fma_pairs(y, 0ull, finite);
-                    float y0, y1;
+                    float y0, y1, least0, least1;
                     halves_of(y, y0, y1);
+                    halves_of(fma_pairs(pair_of(s_least, s_least), gs[i], mul_pairs(pair_of(u_least, u_least), fs[i])), least0, least1);
+                    spare = min3(spare, fabsf(y0) - least0, fabsf(y1) - least1);
                     o_s[(t0 + t + 2 * i) * SC_COLUMNS + column] = y0;
                     o_s[(t0 + t + 2 * i + 1) * SC_COLUMNS + column] = y1;
+                }
+            }
+            // no column whose sums all do: a token's row at a time; one before the first that is not zero may be of zeros
+            if (!__any_sync(0xffffffffu, spare >= 0.f)) {
+                for (int t = 0; t < ST_SHARE_TOKENS; ++t) {
+                    const float y = fabsf(o_s[(t0 + t) * SC_COLUMNS + column]), from_state = s_least * factors[c & 1][hh][t0 + t];
+                    const float least = t0 + t < first_token ? from_state : fmaf(u_least, factors[c & 1][hh][SC_TOKENS + t0 + t], from_state);
+                    if (!__any_sync(0xffffffffu, y >= least)) finite = pair_of(NAN, NAN);
                 }
             }
             __syncwarp();

@@ -396,6 +396,48 @@ def test_one_strong_decay_among_mild_ones(case, strong):
         assert ((state - states[row]).norm(dim=(1, 2)) / states[row].norm(dim=(1, 2))).max() < 300 * 2.0 ** -24
 
 
+# by name: the tokens made large, those whose decay clears the state, and the rows of zeros in front
+SETTINGS = {
+    "a large token, cleared by a decay": ({20: 1.0}, (30, 80), 0),
+    "a large first token, cleared by a decay": ({0: 1.0, 64: 1.0}, (8, 70), 0),
+    "a large token behind zeros": ({20: 1.0}, (), 9),
+    "a large token behind small ones": ({50: 1.0, 140: 1.0}, (), 0),
+    "a large last token": ({63: 1.0, 127: 1.0}, (64, 128), 0),
+}
+
+
+@pytest.mark.parametrize("setting", SETTINGS)
+@pytest.mark.parametrize("case,name", [(c, n) for c in ("state space", "state space 128") for n in "xb"] + [("delta", "v"), ("delta 128", "v")])
+@pytest.mark.parametrize("power", [8, 16, 19, 22, 26, 30, 36, 50, 66])
+def test_a_large_token_costs_no_other_token_its_digits(case, name, setting, power):
+    """Tokens 2^power larger than the others, with a decay of e^-200 behind them, or behind eight rows of zeros and none, or behind small ones:
+    against 64 bits, every token's head by itself, as in the test before; the states' columns too, behind the last token."""
+    views, run, exact = CASES[case]()
+    large, cleared, zeros = SETTINGS[setting]
+    for begin in AT[:-1]:
+        end = AT[AT.index(begin) + 1]
+        for t in large:
+            if begin + t < end:
+                views[name][begin + t] *= 2.0 ** power
+        for t in cleared:
+            if begin + t < end:
+                views["decay"][begin + t] = 200.0
+        views[name][begin:min(begin + zeros, end)] = 0.0
+    want, states = exact()
+    plain, kept_plain = run(False)
+    got, kept = run(True)
+    size = want.norm(dim=-1)
+    error, least = (((t.double().view_as(want) - want).norm(dim=-1) / size)[size > 0] for t in (got, plain))
+    assert torch.equal(got.view_as(want)[size == 0], plain.view_as(want)[size == 0])
+    print(case, name, setting, power, "outputs", error.max().item(), "token by token", least.max().item())
+    assert (error <= 8 * 192 * 2.0 ** -24 + 4 * least).all()
+    for row, slot in enumerate(SLOTS):
+        copy = (STARTS[row] + LENGTHS[row]) & 1
+        a, b, c = (z.double().view_as(states[row]) for z in (kept[slot, copy], kept_plain[slot, copy], states[row]))
+        off, least = ((z - c).norm(dim=1) / c.norm(dim=1) for z in (a, b))         # a column each
+        assert (off <= 8 * 192 * 2.0 ** -24 + 4 * least).all(), (off.max(), least.max())
+
+
 @pytest.mark.parametrize("case", CASES)
 def test_chunks_are_as_near_to_64_bits_as_tokens(case):
     """Outputs and states against a recurrence in 64 bits: a chunk's sums, of operands of 22 bits, are off by less than twice what the
