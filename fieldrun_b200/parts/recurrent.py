@@ -37,12 +37,14 @@ from .linear import linear
 
 # From this many tokens of the longest prompt on a step's recurrence may run in chunks as matrix products (state_space_chunks.cu,
 # delta_chunks.cu).  Measured on a B200, the kernels alone, microseconds, token by token | in chunks.  State space: 64 heads of 128 x 64, one
-# prompt of 64 tokens 28 | 34, of 128 tokens 53 | 39, of 1,024 tokens 341 | 111, 16 of 64 tokens 143 | 98, 8 of 130 tokens 159 | 89, one of 256
-# beside 31 of two 178 | 173, 100 of 17 beside one of 64 319 | 432; 8 heads of 64 x 64, 16 of 64 tokens 22 | 29; 16 of 128 x 128, 4 of 300 tokens 160 | 51.  Delta rule: 16 heads of 128 x 128, one
-# prompt of 64 tokens 51 | 42, of 1,024 tokens 671 | 104, 16 of 65 tokens 208 | 95, 100 of 17 beside one of 64 460 | 273; 64 heads of 64 x 64, 16 of
-# 65 tokens 205 | 271; 64 heads of 128 x 64, one of 256 beside 31 of two 330 | 449.  State space: steps of shorter
-# prompts than 192 tokens keep the results that they had token by token; chunks would save 14 us (one of 128) to 70 (8 of 130).
-STATE_SPACE_CHUNKED_TOKENS, DELTA_CHUNKED_TOKENS = 192, 64
+# prompt of 64 tokens 36 | 33, of 128 tokens 69 | 38, of 191 tokens 98 | 43, 16 of 64 tokens 142 | 97, of 128 tokens 269 | 119, of 191 tokens
+# 394 | 163, 32 of 64 tokens 279 | 164, one of 256 beside 31 of two 178 | 173, 100 of 17 beside one of 64 319 | 432; 16 of 128 x 128, one
+# prompt of 64 tokens 38 | 33, 16 of 64 tokens 77 | 60, of 128 tokens 142 | 74, 4 of 300 tokens 160 | 51; 8 heads of 64 x 64, one prompt of 64
+# tokens 20 | 27, 16 of 64 tokens 35 | 28, 32 of 191 tokens 74 | 47.  (Chunks would pay from 8 prompts of 48 tokens on, 64 | 53; what they
+# cost below 64 tokens is not in the estimate.)  Delta rule: 16 heads of 128 x 128, one prompt of 64 tokens 51 | 42, of 1,024 tokens 671 |
+# 104, 16 of 65 tokens 208 | 95, 100 of 17 beside one of 64 460 | 273; 64 heads of 64 x 64, 16 of 65 tokens 205 | 271; 64 heads of 128 x 64,
+# one of 256 beside 31 of two 330 | 449.
+STATE_SPACE_CHUNKED_TOKENS, DELTA_CHUNKED_TOKENS = 64, 64
 
 
 class _StateMixer(Mixer):
@@ -213,7 +215,7 @@ class ScalarDecayStateSpace(_StateMixer):
 
     def chunks_pay(self, ctx) -> bool:
         """Whether a step of prompts is faster in chunks: microseconds of both ways, fitted to 141 steps of eight head counts and sizes
-        (the measurements above among them; from 192 tokens on no step of them is more than 3 % slower this way than token by token)."""
+        (the measurements above among them; no step of them is more than 3 % slower this way than token by token)."""
         if ctx.is_decode or ctx.max_q_len < STATE_SPACE_CHUNKED_TOKENS:
             return False
         rows, columns = self.state / 128, self.value_dim / 128

@@ -484,7 +484,7 @@ def mixer(kind, heads, dim, vdim, dtype):
     return part
 
 
-@pytest.mark.parametrize("lengths", [[63], [64], [127, 5], [128], [129, 300], [2] * 7 + [256], [1500]])
+@pytest.mark.parametrize("lengths", [[63], [64], [127, 5], [128], [191], [192, 5], [129, 300], [2] * 7 + [256], [1500]])
 @pytest.mark.parametrize("kind", ["gated_linear_attention", "gated_delta_rule", "scalar_decay_state_space"])
 def test_a_prompt_has_the_same_results_on_either_side_of_the_choice(kind, lengths, monkeypatch):
     """Steps below, at and beyond the lengths where the chunks begin to pay: what the part picks, chunks and token by token."""
@@ -538,3 +538,14 @@ def test_gated_linear_attention_takes_a_norm_weight_at_any_offset():
                          scratch=torch.empty(ops().gla_chunks_scratch_floats(chunks[0].numel(), tokens, heads, dim, vdim), device=DEV))
         results.append(out)
     assert torch.equal(*results)
+
+
+def test_state_space_steps_on_either_side_of_the_line():
+    """Heads for which chunks pay from the line on: there, and not one token below, and nowhere where their tables cost more than they save."""
+    from fieldrun_b200.engine.context import StepContext, Workspace
+    space = Workspace(DEV)
+    for heads, n, vdim, some, none in ((64, 128, 64, ([64] * 8, [128], [130] * 8, [191], [192]), ([63] * 64, [64], [17] * 100 + [64])),
+                                       (16, 128, 128, ([64] * 16, [128] * 4, [191]), ([63] * 64, [30])), (8, 64, 64, ([191], [192]), ([64] * 8, [128]))):
+        part = mixer("scalar_decay_state_space", heads, n, vdim, "bfloat16")
+        pays = lambda lengths: part.chunks_pay(StepContext(space, torch.bfloat16, range(len(lengths)), [0] * len(lengths), lengths))
+        assert [pays(lengths) for lengths in some] == [True] * len(some) and [pays(lengths) for lengths in none] == [False] * len(none)
