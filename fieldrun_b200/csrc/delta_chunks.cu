@@ -18,9 +18,9 @@
 // tokens inside a block and up to 48 between blocks: a rounding of their logarithms, which are large only where the weight is small.
 //
 // Everything is float32; the products run on tensor cores with each operand as two parts (tf32_parts.cuh: sums of 16 entries, added in
-// float32 registers; f16_parts.cuh: of at most 128).  Four prompts of 2,048 tokens, 16 heads of 128 x 128 over 4 key heads: 350 us (35 +
-// 154 + 134 + 35 for the launches in turn; 34 + 151 + 130 + 34 without the scales of single rows and the look at the outputs that they are
-// for; delta_rule.cu token by token 1,367).  With launch 1's products made by launch 2 for every head, and
+// float32 registers; f16_parts.cuh: of at most 128).  Four prompts of 2,048 tokens, 16 heads of 128 x 128 over 4 key heads: 350 us (34 +
+// 153 + 133 + 35 for the launches in turn; 34 + 151 + 130 + 35 without the pairs' scales of single rows and the look at the outputs that
+// they are for; delta_rule.cu token by token 1,367).  With launch 1's products made by launch 2 for every head, and
 // launch 3 on mma.sync, 589 (189 + 368 + 34).  Launch 2 is bound by the instructions of its substitution, two entries each (one
 // each: 168 us), and by the latencies before it, two blocks an SM; launch 3 by the chain of its phases.
 #include "f16_parts.cuh"
@@ -33,6 +33,7 @@
 #define DC_LM (DC_TOKENS + 8)
 #define DC_FACTORS (4 * DC_TOKENS + 4)
 #define DC_W_SCALE 8          // exponents of the parts' scales
+#define DC_Q_SCALE 17
 #define DC_K_SCALE 14
 
 struct DeltaChunks {
@@ -53,9 +54,9 @@ struct DeltaChunks {
     // for the chain on tcgen05, in place of w and pairs: their parts, and the unit keys' and queries'
     uint16_t* w_parts;       // [chunks][heads][part][dim / 64][DC_TOKENS][64], the row times 2^8 / (a power of two about w(i))
     uint16_t* pair_parts;    // [chunks][heads][part][DC_TOKENS][DC_TOKENS], rows with a scale each
-    uint16_t *q_parts, *k_parts;     // [chunks][kv_heads][part][dim / 64][DC_TOKENS][64], queries with a scale each, keys times 2^14
+    uint16_t *q_parts, *k_parts;     // [chunks][kv_heads][part][dim / 64][DC_TOKENS][64], times 2^17 and 2^14
     float* raw_pairs;        // [chunks][kv_heads][2][DC_TOKENS][DC_TOKENS]: the unit keys' products [j][i], the queries' with them [i][j], j <= i
-    float* norms;            // [chunks][kv_heads][3][DC_TOKENS]: what makes the queries (with dim^(-1/2)) and keys unit vectors; the queries' scales off
+    float* norms;            // [chunks][kv_heads][3][DC_TOKENS]: what makes the queries (with dim^(-1/2)) and keys unit vectors; the queries' scale off (0: zeros)
     float* factors;          // [chunks][heads][DC_FACTORS]: w's scale off; w(i), the query's scale off; w(j, end); the pairs' scales off; w(end)
     int conv_stride, q_off, k_off, v_off, proj_stride, b_off, a_off, g_off, heads, kv_heads;
     float eps;
@@ -83,7 +84,7 @@ template <int DIM, bool PARTS>
 __global__ void __launch_bounds__(256, 2) delta_chunk_pairs_kernel(DeltaChunks p) {
     constexpr int LQ = DIM + 8;
     extern __shared__ float4 dc_smem[];
-    __shared__ float q_inv[DC_TOKENS], k_inv[DC_TOKENS], q_scale[DC_TOKENS];
+    __shared__ float q_inv[DC_TOKENS], k_inv[DC_TOKENS];
     float* q_s = (float*)dc_smem;                   // [DC_TOKENS][LQ]
     float* k_s = q_s + DC_TOKENS * LQ;              // [DC_TOKENS][LQ]
     const int item = blockIdx.x, kvh = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -97,28 +98,25 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_pairs_kernel(DeltaChunks p
     copies_wait<0>();
     __syncthreads();
     for (int t = warp; t < DC_TOKENS; t += 8) {
-        float qq = 0.f, kk = 0.f, q_top = 0.f;
+        float qq = 0.f, kk = 0.f;
+        bool some = false;                           // an entry of the query that is not zero
 #pragma unroll
         for (int d = 0; d < DIM; d += 32) {
             const float x = q_s[t * LQ + d + lane], y = k_s[t * LQ + d + lane];
             qq = fmaf(x, x, qq);
             kk = fmaf(y, y, kk);
-            q_top = fmaxf(q_top, fabsf(x));
+            some = some || x != 0.f;
         }
         qq = warp_sum(qq);
         kk = warp_sum(kk);
-        if (PARTS) q_top = warp_max(q_top);
+        if (PARTS) some = __any_sync(0xffffffffu, some);
         if (lane == 0) {
             const float q = 1.0f / sqrtf((float)DIM) / sqrtf(qq + 1e-6f), k = 1.0f / sqrtf(kk + 1e-6f);
             q_inv[t] = q;
             k_inv[t] = k;
             p.norms[at * 3 * DC_TOKENS + t] = q;
             p.norms[at * 3 * DC_TOKENS + DC_TOKENS + t] = k;
-            if (PARTS) {
-                const int exponent = parts_exponent(q_top * q);
-                q_scale[t] = q * power_of_two(exponent);
-                p.norms[at * 3 * DC_TOKENS + 2 * DC_TOKENS + t] = q_top > 0.f ? power_of_two(-exponent) : 0.f;
-            }
+            if (PARTS) p.norms[at * 3 * DC_TOKENS + 2 * DC_TOKENS + t] = some ? power_of_two(-DC_Q_SCALE) : 0.f;
         }
     }
     __syncthreads();
@@ -129,7 +127,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_pairs_kernel(DeltaChunks p
             const bool key = u >= UNITS;
             const int r = u % UNITS / (DIM / 8), c = u % (DIM / 8) * 8;
             const float* from = (key ? k_s : q_s) + r * LQ + c;
-            const float scale = key ? k_inv[r] * power_of_two(DC_K_SCALE) : q_scale[r];
+            const float scale = (key ? k_inv[r] : q_inv[r]) * power_of_two(key ? DC_K_SCALE : DC_Q_SCALE);
             uint4 hi, lo;
             split_four(*(const float4*)from, scale, hi.x, hi.y, lo.x, lo.y);
             split_four(*(const float4*)(from + 4), scale, hi.z, hi.w, lo.z, lo.w);
@@ -249,7 +247,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
     if (tid < DC_TOKENS)
         for (int m = tid / DC_BLOCK + 1; m < DC_BLOCKS; ++m) rest += block_log[m];
     after_previous_kernel();                         // launch 1, whose products come from here on; it began when the rows were there
-    // (with PARTS what takes the queries' scales off in the place of their norms, which are in their parts)
+    // (with PARTS what takes the queries' scale off in the place of their norms, which are in their parts)
     if (tid < 2 * DC_TOKENS) (tid < DC_TOKENS ? q_inv : k_inv)[tid % DC_TOKENS] = p.norms[kv_at * 3 * DC_TOKENS + (PARTS && tid < DC_TOKENS ? 2 * DC_TOKENS : 0) + tid];
     __syncthreads();
     if (tid < DC_TOKENS) {
@@ -579,57 +577,99 @@ __global__ void __launch_bounds__(512, 1) delta_chunk_chain_kernel(DeltaChunks p
 using namespace frb_tma;
 using namespace frb_tc;
 
-// A sequence's head token by token (delta_rule.cu's formula): 128 threads of a block, one a value column; `rows_s`: 2 DIM + 3 floats.
+// A sequence's head token by token (delta_rule.cu's formula) by the columns' threads, DT_SHARES a column, each with its entries of the state.
+// room: shared memory for the rows of 32 tokens and the threads' sums.  Bound by the reads of q and k from there: a token takes
+// 1.4 us (one thread a column, its state spilled, the rows fetched token by token: 7.5 us).
 template <int DIM>
-static __device__ __noinline__ void dt_token_by_token(const DeltaChunks& p, int b, int h, float* rows_s) {
-    constexpr int VDIM = 128;
-    float *q_s = rows_s, *k_s = rows_s + DIM, *norms = rows_s + 2 * DIM;
-    const int tid = threadIdx.x, kvh = h / (p.heads / p.kv_heads);
-    const int start = p.seq_start[b], n_tok = p.cu_q_len[b + 1] - p.cu_q_len[b];
-    float* kept = p.state + (size_t)p.seq_slot[b] * 2 * p.copy_floats + p.state_offset + (size_t)h * DIM * VDIM + tid;
-    auto meet = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };
-    float S[DIM];
+static __device__ __noinline__ void dt_token_by_token(const DeltaChunks& p, int b, int h, float* room) {
+    constexpr int VDIM = 128, SHARE = DIM / DT_SHARES, BATCH = 32;
+    float *q_s = room, *k_s = q_s + BATCH * DIM, *v_s = k_s + BATCH * DIM;
+    float4* scalars = (float4*)(v_s + BATCH * VDIM);                     // beta, decay, the query's product with the key
+    float2* sums = (float2*)(scalars + BATCH);                           // [token & 1][share][column]
+    const int tid = threadIdx.x, lane = tid & 31, share = tid / VDIM, column = tid % VDIM, kvh = h / (p.heads / p.kv_heads);
+    auto meet = [] { asm volatile("bar.sync 1, %0;" ::"n"(DT_ROWS) : "memory"); };
+    const int start = p.seq_start[b], count = p.cu_q_len[b + 1] - p.cu_q_len[b];
+    const size_t row0 = p.cu_q_len[b];
+    float* state = p.state + (size_t)p.seq_slot[b] * 2 * p.copy_floats + p.state_offset + ((size_t)h * DIM + share * SHARE) * VDIM + column;
+    const float* from = state + (start & 1) * p.copy_floats;
+    float* to = state + ((start + count) & 1) * p.copy_floats;
+    const float rate = expf(p.a_log[h]), bias = p.dt_bias[h];
+    uint64_t S[SHARE / 2];
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) S[d] = (kept + (start & 1) * p.copy_floats)[(size_t)d * VDIM];
-    for (int t = 0; t < n_tok; ++t) {
-        const size_t row = (size_t)p.cu_q_len[b] + t;
-        const float* rows = p.conv + row * p.conv_stride;
-        const float* logits = p.proj + row * p.proj_stride + h;
-        meet();
-        if (tid < DIM) {
-            q_s[tid] = rows[p.q_off + kvh * DIM + tid];
-            k_s[tid] = rows[p.k_off + kvh * DIM + tid];
+    for (int d = 0; d < SHARE / 2; ++d) S[d] = pair_of(from[(size_t)(2 * d) * VDIM], from[(size_t)(2 * d + 1) * VDIM]);
+    for (int t0 = 0; t0 < count; t0 += BATCH) {
+        const int here = min(BATCH, count - t0);
+        meet();                                      // nobody reads the rows before any more
+        for (int t = share; t < here; t += DT_SHARES) v_s[t * VDIM + column] = p.conv[(row0 + t0 + t) * p.conv_stride + p.v_off + h * VDIM + column];
+        for (int t = tid >> 5; t < here; t += DT_WARPS) {
+            const float* rows = p.conv + (row0 + t0 + t) * p.conv_stride;
+            const float* logits = p.proj + (row0 + t0 + t) * p.proj_stride + h;
+            float x[DIM / 32], y[DIM / 32], qq = 0.f, kk = 0.f, qk = 0.f;
+#pragma unroll
+            for (int d = 0; d < DIM / 32; ++d) {
+                x[d] = rows[p.q_off + kvh * DIM + 32 * d + lane];
+                y[d] = rows[p.k_off + kvh * DIM + 32 * d + lane];
+                qq = fmaf(x[d], x[d], qq);
+                kk = fmaf(y[d], y[d], kk);
+                qk = fmaf(x[d], y[d], qk);
+            }
+            const float q = 1.0f / sqrtf((float)DIM) / sqrtf(warp_sum(qq) + 1e-6f), k = 1.0f / sqrtf(warp_sum(kk) + 1e-6f);
+            qk = warp_sum(qk) * q * k;
+#pragma unroll
+            for (int d = 0; d < DIM / 32; ++d) {
+                q_s[t * DIM + 32 * d + lane] = x[d] * q;
+                k_s[t * DIM + 32 * d + lane] = y[d] * k;
+            }
+            if (lane == 0)
+                scalars[t] = make_float4(1.0f / (1.0f + expf(-logits[p.b_off])), expf(-rate * dc_softplus(logits[p.a_off] + bias)), qk, 0.f);
         }
         meet();
-        if (tid < 96) {                              // a warp the query's norm, one the key's, one their product
-            const float *x = tid < 32 ? q_s : k_s, *y = tid < 64 ? x : q_s;
-            float ss = 0.f;
-            for (int d = tid & 31; d < DIM; d += 32) ss = fmaf(x[d], y[d], ss);
-            ss = warp_sum(ss);
-            if ((tid & 31) == 0) norms[tid >> 5] = tid >= 64 ? ss : (tid < 32 ? 1.0f / sqrtf((float)DIM) : 1.0f) / sqrtf(ss + 1e-6f);
-        }
-        meet();
-        const float beta = 1.0f / (1.0f + expf(-logits[p.b_off]));
-        const float decay = expf(-expf(p.a_log[h]) * dc_softplus(logits[p.a_off] + p.dt_bias[h]));
-        float seen = 0.f, o = 0.f;
+        for (int t = 0; t < here; ++t) {
+            const float4 f = scalars[t];
+            const ulonglong2 *k2 = (const ulonglong2*)(k_s + t * DIM + share * SHARE), *q2 = (const ulonglong2*)(q_s + t * DIM + share * SHARE);
+            const uint64_t decay = pair_of(f.y, f.y);
+            uint64_t seen[2] = {0ull, 0ull}, from_state[2] = {0ull, 0ull};
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) {
-            S[d] *= decay;
-            seen = fmaf(S[d], k_s[d] * norms[1], seen);
-            o = fmaf(S[d], q_s[d] * norms[0], o);
-        }
-        const float u = beta * (rows[p.v_off + h * VDIM + tid] - seen);
+            for (int d = 0; d < SHARE / 4; ++d) {
+                const ulonglong2 k = k2[d], q = q2[d];
+                S[2 * d] = mul_pairs(S[2 * d], decay);
+                S[2 * d + 1] = mul_pairs(S[2 * d + 1], decay);
+                seen[0] = fma_pairs(S[2 * d], k.x, seen[0]);
+                seen[1] = fma_pairs(S[2 * d + 1], k.y, seen[1]);
+                from_state[0] = fma_pairs(S[2 * d], q.x, from_state[0]);
+                from_state[1] = fma_pairs(S[2 * d + 1], q.y, from_state[1]);
+            }
+            float a, b, c, e;
+            halves_of(add_pairs(seen[0], seen[1]), a, b);
+            halves_of(add_pairs(from_state[0], from_state[1]), c, e);
+            float2* told = sums + (t & 1) * DT_SHARES * VDIM + column;
+            told[share * VDIM] = make_float2(a + b, c + e);
+            meet();
+            float2 all = told[0];
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) S[d] = fmaf(k_s[d] * norms[1], u, S[d]);
-        p.raw[(row * p.heads + h) * VDIM + tid] = fmaf(u, norms[2] * norms[0] * norms[1], o);
+            for (int i = 1; i < DT_SHARES; ++i) { all.x += told[i * VDIM].x; all.y += told[i * VDIM].y; }
+            const float u = f.x * (v_s[t * VDIM + column] - all.x);
+            const uint64_t us = pair_of(u, u);
+#pragma unroll
+            for (int d = 0; d < SHARE / 4; ++d) {
+                const ulonglong2 k = k2[d];
+                S[2 * d] = fma_pairs(k.x, us, S[2 * d]);
+                S[2 * d + 1] = fma_pairs(k.y, us, S[2 * d + 1]);
+            }
+            if (share == 0) p.raw[((row0 + t0 + t) * p.heads + h) * VDIM + column] = fmaf(u, f.z, all.y);
+        }
     }
-    float* to = kept + ((start + n_tok) & 1) * p.copy_floats;
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) to[(size_t)d * VDIM] = S[d];
+    for (int d = 0; d < SHARE / 2; ++d) {
+        float even, odd;
+        halves_of(S[d], even, odd);
+        to[(size_t)(2 * d) * VDIM] = even;
+        to[(size_t)(2 * d + 1) * VDIM] = odd;
+    }
 }
 
 template <int DIM>
-__global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(DeltaChunks p, int* __restrict__ status) {
+__global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(const __grid_constant__ DeltaChunks p, int* __restrict__ status) {
     constexpr int VDIM = 128, SHARE = DIM / DT_SHARES;
     constexpr uint32_t ROWS_PART = DC_TOKENS * DIM * 2, PAIR_PART = DC_TOKENS * DC_TOKENS * 2;       // bytes of one part
     // tensor memory: the state's parts; D1 of W, later u's parts; D1 of Q; the parts of u w(j, end); DO; DS
@@ -918,7 +958,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(Del
     }
     __syncthreads();
     if (warp == DT_WARPS + 1) tmem_free(tmem, 512);
-    if (odd_numbers && !failed_flag && warp < 4) dt_token_by_token<DIM>(p, b, h, (float*)w_s);       // over the outputs written, whose copies have ended
+    if (odd_numbers && !failed_flag && warp < DT_WARPS) dt_token_by_token<DIM>(p, b, h, (float*)w_s);       // over the outputs written, whose copies have ended
 }
 
 // The last launch.  A warp a (token, head): bound by reading o and the gate once.

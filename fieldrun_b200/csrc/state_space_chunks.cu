@@ -14,7 +14,7 @@
 //
 // Everything is float32; launch 1's products run on mma.sync in TF32 parts (tf32_parts.cuh), sums of 16 entries, added in float32
 // registers; launch 3's on tcgen05 in float16 parts (f16_parts.cuh), over at most 128 entries.
-// Four prompts of 2,048 tokens, 64 heads of 128 x 64 in 8 groups: 45 + 45 + 184 us (181 without the look for outputs that may have lost
+// Four prompts of 2,048 tokens, 64 heads of 128 x 64 in 8 groups: 45 + 45 + 182 us (178 without the look for outputs that may have lost
 // digits), against 676 us of four launches on mma.sync with a state written and read for every chunk of 128 tokens (states 189, chain
 // 65, outputs 382, pairs 40), and 1,210 token by token.
 #include "f16_parts.cuh"
@@ -267,43 +267,83 @@ __global__ void __launch_bounds__(128) state_space_weights_kernel(StateSpaceChun
 #define ST_REGS_OUTPUTS 64
 static_assert(128 * ST_REGS_ISSUE + ST_ROWS * (ST_REGS_ROWS + ST_REGS_OUTPUTS) <= ST_THREADS * ST_REGS_LAUNCH, "registers of the groups");
 
-// A sequence's columns token by token: 128 threads, one a column; `rows_s`: 2 N floats.
+// A sequence's columns token by token, by the columns' threads, two a column, each with half of its state.  tid: among those threads;
+// column0: the block's first; room: shared memory for the rows of 32 tokens and the threads' sums.  Bound by
+// the reads of B and C from there: a token takes 1.3 us (one thread a column, its state spilled, the rows fetched token by token: 6.9 us).
 template <int N>
-static __device__ __noinline__ void st_token_by_token(const StateSpaceChunks& p, int b, int column, int tid, float* rows_s) {
-    float *b_s = rows_s, *c_s = rows_s + N;
-    const int h = column / p.vdim, g = h / (p.heads / p.groups), start = p.seq_start[b], n_tok = p.cu_q_len[b + 1] - p.cu_q_len[b];
-    float* kept = p.state + (size_t)p.seq_slot[b] * 2 * p.copy_floats + p.state_offset + (size_t)h * N * p.vdim + column % p.vdim;
-    auto meet = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };
-    const float rate = expf(p.a_log[h]);
-    float S[N];
+static __device__ __forceinline__ void st_token_by_token(const StateSpaceChunks& p, int b, int column0, int tid, float* room, volatile int* failed) {
+    constexpr int SHARE = N / 2, BATCH = 32;
+    float *b_s = room, *c_s = b_s + BATCH * N, *x_s = c_s + BATCH * N, *z_s = x_s + BATCH * SC_COLUMNS;
+    float2* steps = (float2*)(z_s + BATCH * SC_COLUMNS);                          // [token][head of the block]: the step, the decay less one
+    float* sums = (float*)(steps + 2 * BATCH);                           // [token & 1][share][column]
+    const int share = tid / SC_COLUMNS, column = column0 + tid % SC_COLUMNS, h0 = column0 / p.vdim, h = column / p.vdim;
+    const int g = h / (p.heads / p.groups), heads_here = SC_COLUMNS / p.vdim;
+    auto meet = [] { asm volatile("bar.sync 1, %0;" ::"n"(ST_ROWS) : "memory"); };
+    const int start = p.seq_start[b], count = p.cu_q_len[b + 1] - p.cu_q_len[b], at = tid % SC_COLUMNS;
+    const size_t row0 = p.cu_q_len[b];
+    float* state = p.state + (size_t)p.seq_slot[b] * 2 * p.copy_floats + p.state_offset + ((size_t)h * N + share * SHARE) * p.vdim + column % p.vdim;
+    const float* from = state + (start & 1) * p.copy_floats;
+    float* to = state + ((start + count) & 1) * p.copy_floats;
+    const float dskip = p.d[h];
+    uint64_t S[SHARE / 2];
 #pragma unroll
-    for (int n = 0; n < N; ++n) S[n] = (kept + (start & 1) * p.copy_floats)[(size_t)n * p.vdim];
-    for (int t = 0; t < n_tok; ++t) {
-        const size_t row = (size_t)p.cu_q_len[b] + t;
-        const float *rows = p.xbc + row * p.xbc_stride, *proj = p.proj + row * p.proj_stride;
-        meet();
-        if (tid < N) {
-            b_s[tid] = rows[p.b_offset + g * N + tid];
-            c_s[tid] = rows[p.c_offset + g * N + tid];
+    for (int n = 0; n < SHARE / 2; ++n) S[n] = pair_of(from[(size_t)(2 * n) * p.vdim], from[(size_t)(2 * n + 1) * p.vdim]);
+    for (int t0 = 0; t0 < count; t0 += BATCH) {
+        const int here = min(BATCH, count - t0);
+        meet();                                      // nobody reads the rows before any more
+        for (int t = share; t < here; t += 2) {
+            x_s[t * SC_COLUMNS + at] = p.xbc[(row0 + t0 + t) * p.xbc_stride + column];
+            z_s[t * SC_COLUMNS + at] = p.proj[(row0 + t0 + t) * p.proj_stride + p.z_offset + column];
+        }
+        for (int i = tid; i < here * (2 * N / 4); i += ST_ROWS) {
+            const int t = i / (2 * N / 4), u = i % (2 * N / 4);
+            const bool is_b = u < N / 4;
+            const float* row = p.xbc + (row0 + t0 + t) * p.xbc_stride + (is_b ? p.b_offset : p.c_offset) + g * N + 4 * (u % (N / 4));
+            *(float4*)((is_b ? b_s : c_s) + t * N + 4 * (u % (N / 4))) = *(const float4*)row;
+        }
+        if (tid < 2 * BATCH && tid / 2 < here && tid % 2 < heads_here) {
+            const int hh = h0 + tid % 2;
+            const float step = sc_softplus(p.proj[(row0 + t0 + tid / 2) * p.proj_stride + p.dt_offset + hh] + p.dt_bias[hh]);
+            steps[tid] = make_float2(step, expm1f(-expf(p.a_log[hh]) * step));
         }
         meet();
-        const float step = sc_softplus(proj[p.dt_offset + h] + p.dt_bias[h]), less_one = expm1f(-rate * step), x = rows[column], u = step * x;
-        float y = 0.f;
+        for (int t = 0; t < here; ++t) {
+            const float2 f = steps[2 * t + h - h0];
+            const ulonglong2 *b2 = (const ulonglong2*)(b_s + t * N + share * SHARE), *c2 = (const ulonglong2*)(c_s + t * N + share * SHARE);
+            const float x = x_s[t * SC_COLUMNS + at];
+            const uint64_t less_one = pair_of(f.y, f.y), u = pair_of(f.x * x, f.x * x);
+            uint64_t y[2] = {0ull, 0ull};
 #pragma unroll
-        for (int n = 0; n < N; ++n) {
-            S[n] = fmaf(less_one, S[n], S[n]) + b_s[n] * u;
-            y = fmaf(S[n], c_s[n], y);
+            for (int n = 0; n < SHARE / 4; ++n) {
+                const ulonglong2 b = b2[n], c = c2[n];
+                S[2 * n] = fma_pairs(b.x, u, fma_pairs(less_one, S[2 * n], S[2 * n]));
+                S[2 * n + 1] = fma_pairs(b.y, u, fma_pairs(less_one, S[2 * n + 1], S[2 * n + 1]));
+                y[0] = fma_pairs(S[2 * n], c.x, y[0]);
+                y[1] = fma_pairs(S[2 * n + 1], c.y, y[1]);
+            }
+            float even, odd;
+            halves_of(add_pairs(y[0], y[1]), even, odd);
+            float* told = sums + (t & 1) * 2 * SC_COLUMNS + at;
+            told[share * SC_COLUMNS] = even + odd;
+            meet();
+            if (share == 0) {
+                const float z = z_s[t * SC_COLUMNS + at];
+                p.out[(row0 + t0 + t) * ((size_t)p.heads * p.vdim) + column] = fmaf(dskip, x, told[0] + told[SC_COLUMNS]) * (z / (1.0f + expf(-z)));
+            }
         }
-        const float z = proj[p.z_offset + column];
-        p.out[row * ((size_t)p.heads * p.vdim) + column] = fmaf(p.d[h], x, y) * (z / (1.0f + expf(-z)));
     }
-    float* to = kept + ((start + n_tok) & 1) * p.copy_floats;
+    if (*failed) return;
 #pragma unroll
-    for (int n = 0; n < N; ++n) to[(size_t)n * p.vdim] = S[n];
+    for (int n = 0; n < SHARE / 2; ++n) {
+        float even, odd;
+        halves_of(S[n], even, odd);
+        to[(size_t)(2 * n) * p.vdim] = even;
+        to[(size_t)(2 * n + 1) * p.vdim] = odd;
+    }
 }
 
 template <int N, bool TWO>
-__global__ void __launch_bounds__(ST_THREADS, 1) state_space_chain_kernel(const __grid_constant__ CUtensorMap map_x, StateSpaceChunks p, int* __restrict__ status) {
+__global__ void __launch_bounds__(ST_THREADS, 1) state_space_chain_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ StateSpaceChunks p, int* __restrict__ status) {
     constexpr int SHARE = N / 2, HEADS = TWO ? 2 : 1, UK = HEADS * SC_TOKENS;        // UK: columns of u's parts
     constexpr uint32_t ROWS_PART = SC_TOKENS * N * 2, PAIR_PART = HEADS * SC_TOKENS * SC_TOKENS * 2, X_BYTES = SC_TOKENS * SC_COLUMNS * 4;
     // tensor memory: the state's parts, later DO over their first columns; D1; u's parts; those of u w(j, end); DS
@@ -556,7 +596,12 @@ __global__ void __launch_bounds__(ST_THREADS, 1) state_space_chain_kernel(const 
         halves_of(finite, even, odd);
         if (even != 0.f || odd != 0.f) odd_numbers = 1;
         meet();
-        if (chunks > 0 && !odd_numbers && ok && !*failed) {
+        if (chunks > 0 && odd_numbers) {
+            // over the outputs written, of which the last have been by then; in the place of the last chunk's operands (inlined: these warps'
+            // registers hold the state)
+            wait(&o_free[(chunks - 1) & 1], (chunks - 1) >> 1 & 1, 92);
+            st_token_by_token<N>(p, b, column0, threadIdx.x - 128, (float*)c_s, failed);
+        } else if (chunks > 0 && ok && !*failed) {
             float* to = kept + ((start + n_tok) & 1) * p.copy_floats;
 #pragma unroll
             for (int n = 0; n < SHARE; ++n) to[(size_t)n * p.vdim] = S[n];
@@ -619,8 +664,6 @@ __global__ void __launch_bounds__(ST_THREADS, 1) state_space_chain_kernel(const 
     }
     __syncthreads();
     if (warp == 1) tmem_free(tmem, 512);
-    if (odd_numbers && !failed_flag && warp >= 4 && warp < 8)
-        st_token_by_token<N>(p, b, column0 + threadIdx.x - 128, threadIdx.x - 128, (float*)c_s);         // over the outputs written
 }
 
 // ----------------------------------------------------------------------------- host side
