@@ -14,7 +14,7 @@
 //
 // Everything is float32; launch 1's products run on mma.sync in TF32 parts (tf32_parts.cuh), sums of 16 entries, added in float32
 // registers; launch 3's on tcgen05 in float16 parts (f16_parts.cuh), over at most 128 entries.
-// Four prompts of 2,048 tokens, 64 heads of 128 x 64 in 8 groups: 45 + 45 + 182 us (178 without the look for outputs that may have lost
+// Four prompts of 2,048 tokens, 64 heads of 128 x 64 in 8 groups: 45 + 45 + 183 us (180 without the look for outputs that may have lost
 // digits), against 676 us of four launches on mma.sync with a state written and read for every chunk of 128 tokens (states 189, chain
 // 65, outputs 382, pairs 40), and 1,210 token by token.
 #include "f16_parts.cuh"
@@ -61,7 +61,9 @@ __device__ __forceinline__ float sc_softplus(float v) { return fmaxf(v, 0.f) + l
 
 // z / (1 + exp(-z)), of sixteen z.  Below 80 the divisor and its reciprocal are far from the ends of float32: there an approximate reciprocal
 // serves, and the quotient's residual, which fma() has exactly, corrects it (Markstein, IBM Journal of Research and Development 34,
-// 1990): the bits of the division at 4 x 10^6 places of each of nine ranges up to 80.  A division's own branch lets no other work in between: with one for each z launch 3 was bound by these, at 196 us.
+// 1990).  That alone does not promise the division's bits; a test has them at a million z of each of nine sizes and both signs.  (The
+// residual's sign is that way round so that minus zero stays what it is.)  A division's own branch lets no other work in between: with one
+// for each z launch 3 was bound by these, at 196 us.
 __device__ __forceinline__ void sc_silu(float (&z)[16]) {
     float top = 0.f;
 #pragma unroll
@@ -73,7 +75,7 @@ __device__ __forceinline__ void sc_silu(float (&z)[16]) {
             float r;
             asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
             const float q = z[i] * r;
-            z[i] = fmaf(fmaf(-q, d, z[i]), r, q);
+            z[i] = fmaf(-fmaf(q, d, -z[i]), r, q);
         }
     } else {
 #pragma unroll
@@ -255,8 +257,8 @@ __global__ void __launch_bounds__(128) state_space_weights_kernel(StateSpaceChun
 // The columns' parts have a power of two of their own each, from the largest entry of the state, of u or of u w(j, end).  Eight more warps take the
 // outputs through D x and the gate while the next chunk is made: with these in the columns' warps a chunk took 4,000 cycles more.  A chunk is
 // bound by the instructions of both, 9,000 to 10,000 cycles: the columns' splits 1,900, u 1,300, the waits for the products 1,900, the
-// outputs' gates 4,000.  A number that is not finite, a token whose sums may have lost digits (PARTS_LEAST), or a chunk whose rows of B lie 2^20 apart makes the block take its
-// columns of the sequence again, token by token.
+// outputs' gates 4,000.  A number that is not finite, a token whose sums may have lost digits (PARTS_LEAST), or a chunk whose rows of B
+// lie 2^20 apart makes the block take its columns of the sequence again, token by token.
 #define ST_THREADS 640         // warps 0 copies, 1 products; 4-11 the columns' two halves (w & 3: lanes), 12-19 the outputs
 #define ST_ROWS 256
 #define ST_SHARE_TOKENS (SC_TOKENS / 2)

@@ -617,3 +617,39 @@ def test_one_number_that_is_not_finite_does_not_make_a_prompt_slow(case, name, m
     views[name][1000, 1] = INF
     assert shortest() < 12 * clean
 
+
+GATES = {"subnormal": (1e-45, 1e-38), "tiny": (1e-38, 1e-8), "small": (1e-8, 0.1), "about one": (0.1, 4.0), "some": (4.0, 20.0), "large": (20.0, 60.0),
+         "up to 80": (60.0, 79.9999), "around 80": (79.5, 80.5), "beyond": (80.0, 200.0)}
+
+
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+@pytest.mark.parametrize("size", GATES)
+def test_gates_have_the_bits_of_the_division(size, sign):
+    """x and D of one and a B of zeros: the outputs are z / (1 + exp(-z)), in chunks by a reciprocal and one correction below 80, token by
+    token by a division.  A million z of every size, and zeros, infinities and NaNs among them."""
+    heads, groups, n, vdim, tokens = 4, 1, 64, 64, 4096
+    inner, gen = heads * vdim, torch.Generator(device=DEV).manual_seed(7)
+    low, high = GATES[size]
+    proj = torch.zeros(tokens, inner + heads, device=DEV)
+    spread = torch.rand(tokens, inner, device=DEV, generator=gen, dtype=torch.float64)
+    proj[:, :inner] = (sign * torch.exp(spread * np.log(high / low)) * low).float()
+    for row, odd in ((70, INF), (200, -INF), (330, NAN), (460, 0.0), (590, -0.0), (720, 500.0), (850, -500.0)):
+        proj[row, ::7] = odd
+    xbc = torch.ones(tokens, inner + 2 * groups * n, device=DEV)
+    xbc[:, inner:] = 0.0
+    zeros, ones = torch.zeros(heads, device=DEV), torch.ones(heads, device=DEV)
+    sizes, tabs, results = dict(heads=heads, vdim=vdim, n=n, groups=groups), Tables([tokens], [0], [0]), []
+    for chunked in (False, True):
+        state, out = torch.zeros(1, 2, heads * n * vdim, device=DEV), torch.full((tokens, inner), NAN, device=DEV)
+        args = (proj, 0, inner, xbc, inner, inner + groups * n, zeros, zeros, ones, tabs, state, 0, out)
+        if chunked:
+            chunks = tables([tokens], 128)
+            scratch = torch.full((ops().state_space_chunks_scratch_floats(chunks[0].numel(), **sizes),), NAN, device=DEV)
+            ops().state_space_chunks(*args, chunks=chunks, scratch=scratch, **sizes)
+        else:
+            ops().state_space_scan(*args, **sizes)
+        results.append(out)
+    plain, got = results
+    assert torch.equal(plain.isnan(), got.isnan()) and plain.isnan().any()
+    differ = (plain.view(torch.int32) != got.view(torch.int32)) & ~plain.isnan()
+    assert not differ.any(), (differ.sum().item(), proj[:, :inner][differ][:5].tolist(), plain[differ][:5].tolist(), got[differ][:5].tolist())
