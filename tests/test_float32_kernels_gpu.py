@@ -167,16 +167,17 @@ def test_split_products_of_several_items_a_block(rows, features, inner):
 
 @pytest.mark.parametrize("limit", [0.0, 1.5])
 def test_split_products_of_experts(limit):
-    """Expert lists: gathered rows, tiles of 1 to 128 rows, an expert without rows and one of several tiles, the gated second half."""
+    """Expert lists: gathered rows, tiles of 1 to 160 rows, each output of one tile alone, an expert without rows and some of several tiles,
+    the gated second half."""
     gen = torch.Generator(device=DEV).manual_seed(5)
-    counts, hidden, width = [1, 0, 130, 128, 15, 400], 96, 72
+    counts, hidden, width = [1, 0, 130, 128, 15, 400, 159, 160, 161, 320], 96, 72
     offsets = np.concatenate([[0], np.cumsum(counts)])
     total = int(offsets[-1])
     w13 = torch.randn(len(counts), 2 * width, hidden, device=DEV, generator=gen) * hidden ** -0.5
     w2 = torch.randn(len(counts), hidden, width, device=DEV, generator=gen)
     x = torch.randn(50, hidden, device=DEV, generator=gen)
     source = i32(np.random.default_rng(1).integers(0, 50, size=total))
-    tiles = [(e, offsets[e] + r) for e, n in enumerate(counts) for r in range(0, n, 128)]
+    tiles = [(e, offsets[e] + r) for e, n in enumerate(counts) for r in range(0, n, ops().PRODUCTS_F32_TILE)]
     lists = (i32([t[0] for t in tiles] + [0]), i32([t[1] for t in tiles] + [0]), i32([len(tiles)]), i32(offsets))
     both = split_product(w13, x, lists, len(tiles) + 1, source)
     got = split_product(w2, both, lists, len(tiles) + 1, gated=True, limit=limit)
