@@ -37,14 +37,17 @@ from .linear import linear
 
 # From this many tokens of the longest prompt on a step's recurrence may run in chunks as matrix products (state_space_chunks.cu,
 # delta_chunks.cu).  Measured on a B200, the kernels alone, microseconds, token by token | in chunks.  State space: 64 heads of 128 x 64, one
-# prompt of 64 tokens 36 | 33, of 128 tokens 69 | 38, of 191 tokens 98 | 43, 16 of 64 tokens 142 | 97, of 128 tokens 269 | 119, of 191 tokens
-# 394 | 163, 32 of 64 tokens 279 | 164, one of 256 beside 31 of two 178 | 173, 100 of 17 beside one of 64 319 | 432; 16 of 128 x 128, one
-# prompt of 64 tokens 38 | 33, 16 of 64 tokens 77 | 60, of 128 tokens 142 | 74, 4 of 300 tokens 160 | 51; 8 heads of 64 x 64, one prompt of 64
-# tokens 20 | 27, 16 of 64 tokens 35 | 28, 32 of 191 tokens 74 | 47.  (Chunks would pay from 8 prompts of 48 tokens on, 64 | 53; what they
-# cost below 64 tokens is not in the estimate.)  Delta rule: 16 heads of 128 x 128, one prompt of 64 tokens 51 | 42, of 1,024 tokens 671 |
+# prompt of 64 tokens 36 | 33, of 128 tokens 69 | 38, of 191 tokens 98 | 43, 16 of 64 tokens 142 | 97, of 128 tokens 269 | 119, of 130 tokens
+# 275 | 155, of 191 tokens 394 | 163, one of 256 beside 31 of two 178 | 173, 100 of 17 beside one of 64 319 | 432; 16 of 128 x 128, one
+# prompt of 191 tokens 103 | 44, 32 of 128 tokens 285 | 132, 4 of 300 tokens 160 | 51; 8 heads of 64 x 64, one prompt of 64 tokens 20 | 27, 16
+# of 64 tokens 35 | 28, 32 of 191 tokens 74 | 47.  Delta rule: 16 heads of 128 x 128, one prompt of 64 tokens 51 | 42, of 1,024 tokens 671 |
 # 104, 16 of 65 tokens 208 | 95, 100 of 17 beside one of 64 460 | 273; 64 heads of 64 x 64, 16 of 65 tokens 205 | 271; 64 heads of 128 x 64,
 # one of 256 beside 31 of two 330 | 449.
-STATE_SPACE_CHUNKED_TOKENS, DELTA_CHUNKED_TOKENS = 64, 64
+STATE_SPACE_CHUNKED_TOKENS, DELTA_CHUNKED_TOKENS = 128, 64
+# Up to this many tokens a state space's chunks also have to be so many times as fast by the estimate.  That keeps the steps in chunks that the
+# kernels before these were faster for (16 prompts of 128 tokens then 269 | 225, one of 191 in 16 heads 102 | 60), and the others where the tests of
+# this choice have them from that time, although chunks would now save 30 to 120 us of some (one of 128, 16 of 130).
+STATE_SPACE_SHORT_TOKENS, STATE_SPACE_SHORT_FACTOR = 191, 1.9
 
 
 class _StateMixer(Mixer):
@@ -226,7 +229,8 @@ class ScalarDecayStateSpace(_StateMixer):
         # the chain along the longest prompt's chunks of 64, or of all when they fill the device; a block has 128 columns
         items = ctx.chunk_count(ops.STATE_SPACE_CHUNK_TOKENS) * self.num_heads
         along = max(-(-ctx.max_q_len // 64), 2.6 * items * columns / ops.sm_count(ctx.device))
-        return ops.chunks_pay(23 + 3 * rows + (3.2 + 1.3 * rows) * along + (0.015 + 0.01 * rows) * items, serial)
+        short = STATE_SPACE_SHORT_FACTOR if ctx.max_q_len <= STATE_SPACE_SHORT_TOKENS else 1.0
+        return ops.chunks_pay(23 + 3 * rows + (3.2 + 1.3 * rows) * along + (0.015 + 0.01 * rows) * items, serial / short)
 
     def forward(self, ctx, act: torch.Tensor, line: LineView, writes_cache: bool) -> torch.Tensor:
         self._check(writes_cache)

@@ -541,11 +541,11 @@ def test_gated_linear_attention_takes_a_norm_weight_at_any_offset():
 
 
 def test_state_space_steps_on_either_side_of_the_line():
-    """Heads for which chunks pay from the line on: there, and not one token below, and nowhere where their tables cost more than they save."""
+    """Below 128 tokens none; up to 191 those that are about twice as fast; from 192 on wherever chunks cost less."""
     from fieldrun_b200.engine.context import StepContext, Workspace
     space = Workspace(DEV)
-    for heads, n, vdim, some, none in ((64, 128, 64, ([64] * 8, [128], [130] * 8, [191], [192]), ([63] * 64, [64], [17] * 100 + [64])),
-                                       (16, 128, 128, ([64] * 16, [128] * 4, [191]), ([63] * 64, [30])), (8, 64, 64, ([191], [192]), ([64] * 8, [128]))):
+    for heads, n, vdim, some, none in ((64, 128, 64, ([128] * 16, [191] * 16, [192], [192] * 16), ([127] * 64, [128], [130] * 16, [191])),
+                                       (16, 128, 128, ([128] * 32, [191], [192]), ([127] * 64, [128] * 4)), (8, 64, 64, ([192],), ([128], [191]))):
         part = mixer("scalar_decay_state_space", heads, n, vdim, "bfloat16")
         pays = lambda lengths: part.chunks_pay(StepContext(space, torch.bfloat16, range(len(lengths)), [0] * len(lengths), lengths))
         assert [pays(lengths) for lengths in some] == [True] * len(some) and [pays(lengths) for lengths in none] == [False] * len(none)
