@@ -511,8 +511,9 @@ attention_f32_tc_kernel(F32Attention p, const int* __restrict__ tile_seq, const 
 // total_pages * (kv heads + value heads) floats.  status: one int on the device, zero before the call.
 FRB_API int frb_attention_f32_tc(const float* q, const float* k_pages, const float* v_pages, const int* page_table, int max_pages,
                                  const int* tile_seq, const int* tile_q0, int num_tiles, const int* seq_slot, const int* seq_start,
-                                 const int* seq_q_len, const int* cu_q_len, int num_seqs, int total_pages, float* scratch, int* status, float* out, int num_heads, int num_kv_heads, int head_dim, int v_dim, float scale,
-                                 int window, const float* slopes, int chunk, const float* sinks, const float* gate, int gate_stride, float softcap,
+                                 const int* seq_q_len, const int* cu_q_len, int num_seqs, int total_pages, float* scratch, int* status,
+                                 float* out, int num_heads, int num_kv_heads, int head_dim, int v_dim, float scale, int window,
+                                 const float* slopes, int chunk, const float* sinks, const float* gate, int gate_stride, float softcap,
                                  int keep_first, int num_v_heads, cudaStream_t stream) {
     if (num_tiles == 0) return 0;
     FRB_CHECK_ARG((head_dim == 64 && (v_dim == 64 || v_dim == 128)) || (head_dim == 128 && v_dim == 128),

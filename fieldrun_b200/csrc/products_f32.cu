@@ -371,9 +371,9 @@ products_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 }
 
 // The outputs to be summed again, a warp each: a warp takes a collector's outputs of an item that have some, and their columns in turn.  A
-// kernel of its own: called from the workers' loop the same cost that a quarter of its speed.  3,704 rows with 8192 x 3072 and 3072 x 6144
-// weights, on average: 626 us with this kernel, 28 of them its own; 800 the other way; 606 with no output summed again but those of rows
-// without a scale.
+// kernel of its own: called from the workers' loop the same cost that a quarter of its speed (with tiles of 128 rows, 3,704 rows with 8192 x
+// 3072 and 3072 x 6144 weights, on average: 626 us with a kernel of its own, 800 without).  With those weights it takes 25 and 35 us beside
+// 450 and 314 of the products.
 __global__ void __launch_bounds__(256, 4) products_f32_again_kernel(const __grid_constant__ ProductsParams p) {
     const int lane = threadIdx.x & 31, tiles = p.count();
     const long long units = (long long)tiles * p.feature_blocks() * PF_WORKERS, warps = (long long)gridDim.x * 8;

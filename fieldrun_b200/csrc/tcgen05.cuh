@@ -1,6 +1,6 @@
 // The fifth-generation tensor core: operand descriptors, MMA issue, completion, tensor-memory loads and stores.
 //
-// One warp of a block issues the MMAs, each by one of its lanes; the accumulators (and, for `mma_ts`, the A operand) live in tensor
+// One warp of a block issues the MMAs, by one of its lanes (in latent_attention_tc.cu that lane runs the loop, elsewhere the warp); the accumulators (and, for `mma_ts`, the A operand) live in tensor
 // memory, which one warp of the block allocates and frees.  Operands in shared memory are K-major tiles of
 // rows of 128 bytes under the 128-byte swizzle that TMA writes (tma.cuh).
 #pragma once

@@ -44,8 +44,10 @@ TENSOR_CORE_ROWS_PER_EXPERT = {"decode": 4.0, "prompt": 1.0}
 # A float32 step's expert products run on the tensor cores as split products, in tiles of 160 rows, where experts get more than so many
 # rows (on average) and the step has at least so many multiply-adds; elsewhere, where their two more launches cost more than they save, as a
 # stream over the weights in tiles of eight.  Measured on a B200, the whole part, microseconds, stream | split: MiniMax-M2's sizes
-# 3 rows per expert 2294 | 2303, 5 rows 2747 | 2466, 8 rows 3178 | 2497, 16 rows 4791 | 2600; 16 experts of 2048 x 2048 4 rows 231 | 249,
-# 6 rows 244 | 238, 16 rows 355 | 264; of 1024 x 1024 8 rows 108 | 187, 16 rows 157 | 151, 20 rows 190 | 152.
+# 3 rows per expert 2294 | 2303, 5 rows 2747 | 2466, 8 rows 3178 | 2497, 16 rows 4791 | 2600; 16 experts of 2048 x 2048 4 rows 190 | 217,
+# 5 rows 203 | 218, 6 rows 222 | 218, 8 rows 223 | 219, 12 rows 278 | 223; of 1024 x 1024 8 rows 101 | 145, 9 rows 106 | 146, 12 rows 127 | 147,
+# 15 rows 146 | 145, 20 rows 179 | 148.  (Where the work is below 2^30 the second line lies where it was with the kernel before; by
+# these figures it would lie at 14 rows.)
 SPLIT_ROWS_PER_EXPERT = ((4.0, 1 << 30), (8.0, 1 << 28))
 
 FUSED_ACTIVATION_ROWS = 64      # from this many rows of a prompt step on, a dense unit's first product carries its activation

@@ -26,9 +26,11 @@ STREAM_FEATURES = 65536   # beyond this many output features the library product
 # A float32 product runs on the tensor cores, each operand as two float16 parts (products_f32.cu), from SPLIT_PRODUCTS multiply-adds,
 # SPLIT_ROWS rows and SPLIT_TILES tiles of 128 x 128 results on.  Below, the pass over the weight for its scales (half of the bytes of
 # a product of few rows), the launches or the idle SMs cost more than the products save.  Measured on a B200 with weights that are not in
-# L2, microseconds, the library's float32 product | this one with its scales and parts: 200064 x 3072 weights, 9 rows 868 | 1040 (not
-# faster since: the pass over the weight alone), 150 rows 4440 | 926; 32768 x 4096, 48 rows 332 | 209; 8192 x 3072, 96 rows 129 | 77, 700
-# rows 613 | 160; 3072 x 6144, 256 rows 250 | 113; 2048 x 2048, 512 rows 89 | 55; 1024 x 1024, 2,048 rows 87 | 46.
+# L2, microseconds, the library's float32 product | this one with its scales and parts: 200064 x 3072 weights, 9 rows 853 | 1218, 32 rows
+# 896 | 772, 48 rows 1397 | 820; 32768 x 4096, 32 rows 265 | 229, 64 rows 341 | 209; 8192 x 3072, 48 rows (2^30.2) 97 | 71, 64 rows 97 | 72,
+# 96 rows 128 | 76, 700 rows 613 | 160; 3072 x 6144, 64 rows 151 | 94, 128 rows (24 tiles) 169 | 103, 256 rows 250 | 112; 2048 x 2048, 128 rows
+# (2^29) 52 | 47, 256 rows 58 | 49, 512 rows 88 | 53; 1024 x 1024, 1,024 rows (2^30) 48 | 39, 2,048 rows 86 | 40; 256 x 3072, 2,048 rows 82 | 67.
+# (The lines lie where they were with the kernel before; by these figures they would lie at 2^30, 32 rows and 16 tiles.)
 SPLIT_ROWS = 48
 SPLIT_TILES = 32
 SPLIT_PRODUCTS = 1 << 31

@@ -576,8 +576,8 @@ def float32_products(kind: str, launches: int) -> dict:
 
 
 def float32_attention(kind: str, launches: int) -> dict:
-    """Float32 attention, 48 heads over 8 of 128: ``prompts`` a prompt of 1,500 tokens in tiles, ``tokens`` one token each of sixteen
-    sequences of 4,096 keys in chunks."""
+    """Float32 attention, 48 heads over 8 of 128: ``prompts`` a prompt of 1,500 tokens on tcgen05 (``prompts_mma``: in tiles on
+    mma.sync), ``tokens`` one token each of sixteen sequences of 4,096 keys in chunks."""
     batch, context = (16, 4096) if kind == "tokens" else (1, 1500)
     pages_per = (context + 63) // 64
     keys, values = (torch.randn(batch * pages_per, KV_HEADS, *shape, device=DEV) for shape in ((64, HEAD_DIM), (HEAD_DIM, 64)))
@@ -594,7 +594,11 @@ def float32_attention(kind: str, launches: int) -> dict:
     else:
         firsts = list(range(0, context, 128))
         tables = (i32([0] * len(firsts)), i32(firsts), i32([0]), i32([0]), i32([context]), i32([0, context]))
-        launch = lambda: ops.attention_f32_tiles(q, keys, values, table, *tables, out, **common)
+        scratch = torch.empty(ops.attention_f32_tc_scratch(pages_per, KV_HEADS, HEAD_DIM, HEAD_DIM), device=DEV)
+        if kind == "prompts":
+            launch = lambda: ops.attention_f32_tc(q, keys, values, table, *tables, scratch, pages_per, out, **common)
+        else:
+            launch = lambda: ops.attention_f32_tiles(q, keys, values, table, *tables, out, **common)
         flops = 2.0 * context * (context + 1) * HEADS * HEAD_DIM
     ms = _time(launch, launches)
     return {"case": f"float32_attention_{kind}", "ms": round(ms, 4), "tflops": round(flops / ms / 1e9, 2),
@@ -737,7 +741,7 @@ CASES = {
        for kind in ("retention_prefill", "retention_decode", "gru_prefill", "gru_decode", "shift_prefill", "shift_decode",
                     "powers_prefill", "powers_decode")},
     **{f"float32_{kind}": (lambda n, kind=kind: float32_products(kind, n)) for kind in ("experts", "dense", "rows")},
-    **{f"float32_attention_{kind}": (lambda n, kind=kind: float32_attention(kind, n)) for kind in ("prompts", "tokens")},
+    **{f"float32_attention_{kind}": (lambda n, kind=kind: float32_attention(kind, n)) for kind in ("prompts", "prompts_mma", "tokens")},
     "delta_rule_chunks": lambda n: delta_rule("chunks", n),
     "delta_rule_prefill": lambda n: delta_rule("prefill", n),
     "delta_rule_prefill_whole": lambda n: delta_rule("prefill_whole", n),
