@@ -18,8 +18,8 @@
 // tokens inside a block and up to 48 between blocks: a rounding of their logarithms, which are large only where the weight is small.
 //
 // Everything is float32; the products run on tensor cores with each operand as two parts (tf32_parts.cuh: sums of 16 entries, added in
-// float32 registers; f16_parts.cuh: of at most 128).  Four prompts of 2,048 tokens, 16 heads of 128 x 128 over 4 key heads: 350 us (34 +
-// 153 + 133 + 35 for the launches in turn; 34 + 151 + 130 + 35 without the pairs' scales of single rows and the look at the outputs that
+// float32 registers; f16_parts.cuh: of at most 128).  Four prompts of 2,048 tokens, 16 heads of 128 x 128 over 4 key heads: 345 us (34 +
+// 153 + 129 + 35 for the launches in turn; 34 + 151 + 129 + 35 without the pairs' scales of single rows and the look at the outputs that
 // they are for; delta_rule.cu token by token 1,367).  With launch 1's products made by launch 2 for every head, and
 // launch 3 on mma.sync, 589 (189 + 368 + 34).  Launch 2 is bound by the instructions of its substitution, two entries each (one
 // each: 168 us), and by the latencies before it, two blocks an SM; launch 3 by the chain of its phases.
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
         if (PARTS) {                                 // eight neighbouring threads have a row
             float top = 0.f;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) top = fmaxf(top, fabsf(y[e]));
+            for (int e = 0; e < 8; e += 2) top = max3(top, fabsf(y[e]), fabsf(y[e + 1]));
 #pragma unroll
             for (int o = 1; o < 8; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
             const int exponent = parts_exponent(top);
@@ -808,7 +808,6 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(con
 #pragma unroll
         for (int d = 0; d < SHARE; ++d) S[d] = (kept + (start & 1) * p.copy_floats)[(size_t)d * VDIM];
         float u_inv = 0.f, s_least = 0.f, u_least = 0.f;
-        int first_token = 0;
         auto write_outputs = [&](int c) {            // what u gives the outputs of chunk c, behind what its state gave
             const float4* f4 = (const float4*)factors[c % 3];
             wait(&do_done, c & 1, 72);
@@ -836,6 +835,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(con
             // Queries and pairs' weights are at most dim^(-1/2), so that what takes their scales off is at most 2^-17.  Where no column has
             // outputs that are all large enough by that: a token's row at a time; one before the first that is not zero may be of zeros.
             if (!__any_sync(0xffffffffu, smallest >= (s_least + u_least) * power_of_two(-17))) {
+                const int first_token = first_rows[0][quarter] < DT_TOKENS ? first_rows[0][quarter] : DT_TOKENS + first_rows[1][quarter];
                 for (int t = t0; t < t0 + DT_TOKENS; ++t) {
                     const float from_state = s_least * factors[c % 3][DC_TOKENS + t];
                     const float least = t < first_token ? from_state : fmaf(u_least, factors[c % 3][3 * DC_TOKENS + t], from_state);
@@ -893,8 +893,6 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(con
             fence_before_sync();                                         // D1's columns are read before another share's parts go over them
             tops[1][share][column] = u_top;
             tops[2][share][column] = uk_top;
-            const int first_here = first_row(u);
-            if (lane == 0) first_rows[share][quarter] = first_here;
             meet();
             u_top = largest(1);
             const int u_exponent = parts_exponent(u_top), uk_exponent = parts_exponent(largest(2));
@@ -908,7 +906,8 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(con
             u_inv = power_of_two(-u_exponent);
             s_least = PARTS_LEAST * warp_unit(s_top, s_exponent);
             u_least = PARTS_LEAST * warp_unit(u_top, u_exponent);
-            first_token = first_rows[0][quarter] < DT_TOKENS ? first_rows[0][quarter] : DT_TOKENS + first_rows[1][quarter];
+            const int first_here = first_row(u);
+            if (lane == 0) first_rows[share][quarter] = first_here;              // read behind the next meeting, with the outputs
 
             // what the state gives the outputs, then the new state
             wait(&d1q_done, phase, 70);
@@ -933,7 +932,10 @@ __global__ void __launch_bounds__(DT_THREADS, 1) delta_chunk_chain_tc_kernel(con
                 halves_of(now, S[d], S[d + 1]);
             }
         }
-        if (chunks > 0) write_outputs(chunks - 1);
+        if (chunks > 0) {
+            meet();
+            write_outputs(chunks - 1);
+        }
 #pragma unroll
         for (int d = 0; d < SHARE; d += 2) finite = fma_pairs(pair_of(S[d], S[d + 1]), 0ull, finite);        // an earlier one reached the outputs
         float even, odd;

@@ -81,7 +81,9 @@ __device__ __forceinline__ void load_columns(uint32_t from, uint32_t (&v)[N / 16
 }
 
 // The exponent of the power of two that brings `top` to [2^14, 2^15); of a smaller one than 2^-100 as if it were that, of a NaN too.
-__device__ __forceinline__ int parts_exponent(float top) { return 14 - ilogbf(fminf(fmaxf(top, 7.888609052210118e-31f), 3.402823466e38f)); }
+__device__ __forceinline__ int parts_exponent(float top) {
+    return 14 + 127 - (int)(__float_as_uint(fminf(fmaxf(top, 7.888609052210118e-31f), 3.402823466e38f)) >> 23);
+}
 
 // Parts of one scale hold the digits of entries down to 2^-29 of the largest; smaller ones are off by up to 2^-51 of it, and with them the
 // sums that they alone make.  Whether that counts is seen at the sums: in units of the scales, products of parts below 2^15 whose errors

@@ -14,7 +14,7 @@
 //
 // Everything is float32; launch 1's products run on mma.sync in TF32 parts (tf32_parts.cuh), sums of 16 entries, added in float32
 // registers; launch 3's on tcgen05 in float16 parts (f16_parts.cuh), over at most 128 entries.
-// Four prompts of 2,048 tokens, 64 heads of 128 x 64 in 8 groups: 45 + 45 + 183 us (180 without the look for outputs that may have lost
+// Four prompts of 2,048 tokens, 64 heads of 128 x 64 in 8 groups: 45 + 44 + 180 us (45 + 45 + 178 without the look for outputs that may have lost
 // digits), against 676 us of four launches on mma.sync with a state written and read for every chunk of 128 tokens (states 189, chain
 // 65, outputs 382, pairs 40), and 1,210 token by token.
 #include "f16_parts.cuh"
