@@ -18,7 +18,7 @@
 // A decay a = exp(l) with l close to 0 is kept as a - 1 = expm1(l) and applied as S + (a - 1) S: rounded to float32, a
 // itself would lose its distance from 1, by the same amount at every step, and over a thousand tokens that bias adds
 // up to 1e-4 of the state; the rounding of S + (a - 1) S has no preferred direction.
-#include "common.cuh"
+#include "silu.cuh"
 
 #define SCAN_TOKENS 8        // tokens whose rows are asked for together
 
@@ -77,6 +77,7 @@ struct ConvParams {
 __device__ __forceinline__ float conv_activation(float v, int activation) { return activation == 1 ? silu_f(v) : v; }
 
 #define CONV_ROWS 8          // rows of the step that one thread takes, one after the other, for its channel
+#define CONV_FOURS_BATCH 4   // rows that such a thread has on their way at a time
 #define CONV_FOURS_ROWS 128  // from this many rows on a thread takes four channels: it is the faster from one thread an SM on
 
 // The rows that see only inputs of their own step (row i >= K-1 of its sequence).  A thread takes CONV_ROWS rows of the
@@ -125,28 +126,58 @@ __global__ void __launch_bounds__(128) causal_conv_rows_kernel(ConvParams p) {
     }
 }
 
-// The same for prompts of the usual few taps: a thread takes CONV_ROWS rows of four neighbouring channels, 16 bytes at a time,
-// and has registers and multiply-adds for TAPS taps, not for the most there can be.  The taps reach the threads through shared memory:
-// read in place, a warp's lanes lie a channel's taps apart and touch 16 lines a load, half of the kernel's time in the load unit.  Bound
-// by its bytes and by silu's arithmetic: both kernels together, 8,192 rows of 3,072 channels 70 -> 58 us (3.5 TB/s), of 6,144 channels
-// 123 -> 103 (3.9), 1,024 rows of 6,144 channels 22 -> 21 (the kernel above: 111, 210, 117).  Eight blocks an SM (64 registers): five
-// (94, as it comes) 64 and 116, seven 73 and 133, nine 63 and 109; four rows a thread 60 and 109, six 82 and 158.
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+
+// out[r] of two rows of four channels, the newest input last; a row that is not `here` is left out.
 template <typename OutT, int TAPS>
-__global__ void __launch_bounds__(128, 8) causal_conv_rows4_kernel(ConvParams p) {
+__device__ __forceinline__ void conv_two_rows(const ConvParams& p, int r, int c, const float4* vals, const float4 (&w)[TAPS], float4 bias, bool here0,
+                                              bool here1) {
+    float acc[8];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        float* a = acc + 4 * q;
+        a[0] = bias.x; a[1] = bias.y; a[2] = bias.z; a[3] = bias.w;
+#pragma unroll
+        for (int k = 0; k < TAPS; ++k) {
+            a[0] = fmaf(w[k].x, vals[q + k].x, a[0]);
+            a[1] = fmaf(w[k].y, vals[q + k].y, a[1]);
+            a[2] = fmaf(w[k].z, vals[q + k].z, a[2]);
+            a[3] = fmaf(w[k].w, vals[q + k].w, a[3]);
+        }
+    }
+    if (p.activation == 1) silu_of(acc);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        if (!(q ? here1 : here0)) continue;
+        const size_t at = (size_t)(r + q) * p.channels + c;
+        *(float4*)(p.out32 + at) = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+        if (p.out_typed) {
+            OutT* typed = (OutT*)p.out_typed + at;
+            typed[0] = from_f32<OutT>(acc[4 * q]);
+            typed[1] = from_f32<OutT>(acc[4 * q + 1]);
+            typed[2] = from_f32<OutT>(acc[4 * q + 2]);
+            typed[3] = from_f32<OutT>(acc[4 * q + 3]);
+        }
+    }
+}
+
+// The same for prompts of the usual few taps, and in the same launch what causal_conv_heads_kernel does: the first num_seqs blocks have a
+// sequence's first TAPS - 1 rows and its state, the others runs of rows.  A thread takes rows_per_thread rows of four neighbouring channels,
+// 16 bytes and CONV_FOURS_BATCH rows at a time, and has registers and multiply-adds for TAPS taps, not for the most there can be.  The taps reach
+// the threads through shared memory: read in place, a warp's lanes lie a channel's taps apart and touch 16 lines a load, half of the
+// kernel's time in the load unit.  Bound by its bytes: 8,192 rows of 3,072 channels 45 us (4.5 TB/s), of 6,144 channels 84 (4.8); with eight
+// rows a thread, a division's own branch in each silu and the sequences' first rows in a launch of their own 66 and 105.  Six blocks an SM
+// (80 registers, nothing in local memory): eight (64) 76 and 141; batches of eight rows 61 and 115; the next batch asked for ahead (five
+// blocks, 93 registers) 49 and 91; batches of two rows, eight blocks 51 and 93.
+template <typename OutT, int TAPS>
+__global__ void __launch_bounds__(128, 6) causal_conv_fours_kernel(ConvParams p, int num_seqs) {
     __shared__ __align__(16) float s_taps[TAPS][512 + 8];      // 8: a warp's lanes write four taps of eight channels to 32 banks
     after_previous_kernel();
     const int c0 = 512 * blockIdx.y, c = c0 + 4 * threadIdx.x;
     const bool inside = c < p.channels;
-    const int r_begin = blockIdx.x * CONV_ROWS, r_end = min(p.num_rows, r_begin + CONV_ROWS);
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 in_bias = p.in_bias && inside ? *(const float4*)(p.in_bias + c) : zero, bias = p.bias && inside ? *(const float4*)(p.bias + c) : zero;
     const float* in = p.in + p.in_offset + c;
-    float4 vals[CONV_ROWS + TAPS - 1];         // the input of row r_begin - (TAPS - 1) + m
-#pragma unroll
-    for (int m = 0; m < CONV_ROWS + TAPS - 1; ++m) {
-        const int r = r_begin - (TAPS - 1) + m;
-        vals[m] = r >= 0 && r < r_end && inside ? *(const float4*)(in + (size_t)r * p.in_stride) : zero;
-    }
     const int entries = min(512, p.channels - c0) * TAPS;
 #pragma unroll
     for (int u = 0; u < 4 * TAPS; ++u) {
@@ -158,41 +189,66 @@ __global__ void __launch_bounds__(128, 8) causal_conv_rows4_kernel(ConvParams p)
     float4 w[TAPS];
 #pragma unroll
     for (int k = 0; k < TAPS; ++k) w[k] = *(const float4*)&s_taps[k][4 * threadIdx.x];
-    OutT* typed = (OutT*)p.out_typed;
+
+    if ((int)blockIdx.x < num_seqs) {
+        const int b = blockIdx.x, row0 = p.seq.cu_q_len[b], n = p.seq.cu_q_len[b + 1] - row0;
+        const int start = p.seq.seq_start[b], slot = p.seq.seq_slot[b];
+        const float* old_tail = state_at(p.state, slot, start & 1) + c;
+        float* new_tail = state_at(p.state, slot, (start + n) & 1) + c;
+        // vals[m]: for m < TAPS - 1 the inputs before the step (which may lie at any offset), then the step's first
+        float4 vals[2 * TAPS - 2 + 1];
+#pragma unroll
+        for (int m = 0; m < TAPS - 1; ++m) {
+            const float* from = old_tail + (size_t)m * p.channels;
+            vals[m] = make_float4(from[0], from[1], from[2], from[3]);
+        }
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j)
+            vals[TAPS - 1 + j] = j < min(n, TAPS - 1) ? add4(*(const float4*)(in + (size_t)(row0 + j) * p.in_stride), in_bias) : zero;
+#pragma unroll
+        for (int j = 0; j < TAPS - 1; j += 2)
+            if (j < n) conv_two_rows<OutT, TAPS>(p, row0 + j, c, vals + j, w, bias, true, j + 1 < min(n, TAPS - 1));
+#pragma unroll
+        for (int m = 0; m < TAPS - 1; ++m) {
+            // the step's input that becomes entry m of the new state, or an older one, from a place that is not yet written
+            const int at = n - (TAPS - 1) + m;
+            const float* from = old_tail + (size_t)max(n + m, 0) * p.channels;
+            float4 v;
+            if (at >= 0) v = add4(*(const float4*)(in + (size_t)(row0 + at) * p.in_stride), in_bias);
+            else v = make_float4(from[0], from[1], from[2], from[3]);
+            float* to = new_tail + (size_t)m * p.channels;
+            to[0] = v.x; to[1] = v.y; to[2] = v.z; to[3] = v.w;
+        }
+        return;
+    }
+    const int r_begin = ((int)blockIdx.x - num_seqs) * p.rows_per_thread, r_end = min(p.num_rows, r_begin + p.rows_per_thread);
     const int b_first = p.tok_seq[r_begin], b_last = p.tok_seq[r_end - 1];
     const int row0_first = p.seq.cu_q_len[b_first];
     const bool one_sequence = b_first == b_last;
+    float4 vals[TAPS - 1 + CONV_FOURS_BATCH];         // the input of row r - (TAPS - 1) + m
 #pragma unroll
-    for (int m = 0; m < CONV_ROWS + TAPS - 1; ++m) {
-        vals[m].x += in_bias.x;
-        vals[m].y += in_bias.y;
-        vals[m].z += in_bias.z;
-        vals[m].w += in_bias.w;
+    for (int m = 0; m < TAPS - 1; ++m) {
+        const int row = r_begin - (TAPS - 1) + m;
+        vals[m] = row >= 0 ? add4(*(const float4*)(in + (size_t)row * p.in_stride), in_bias) : zero;
     }
+#pragma unroll 1
+    for (int r = r_begin; r < r_end; r += CONV_FOURS_BATCH) {
 #pragma unroll
-    for (int q = 0; q < CONV_ROWS; ++q) {
-        const int r = r_begin + q;
-        if (r >= r_end) break;
-        const int row0 = one_sequence ? row0_first : p.seq.cu_q_len[p.tok_seq[r]];
-        if (r - row0 < TAPS - 1) continue;
-        float4 acc = bias;
+        for (int q = 0; q < CONV_FOURS_BATCH; ++q)
+            vals[TAPS - 1 + q] = r + q < r_end ? *(const float4*)(in + (size_t)(r + q) * p.in_stride) : zero;
 #pragma unroll
-        for (int k = 0; k < TAPS; ++k) {
-            acc.x = fmaf(w[k].x, vals[q + k].x, acc.x);
-            acc.y = fmaf(w[k].y, vals[q + k].y, acc.y);
-            acc.z = fmaf(w[k].z, vals[q + k].z, acc.z);
-            acc.w = fmaf(w[k].w, vals[q + k].w, acc.w);
+        for (int q = 0; q < CONV_FOURS_BATCH; ++q) vals[TAPS - 1 + q] = add4(vals[TAPS - 1 + q], in_bias);
+#pragma unroll
+        for (int q = 0; q < CONV_FOURS_BATCH; q += 2) {
+            if (r + q >= r_end) break;
+            const auto own = [&](int row) {
+                return row < r_end && row - (one_sequence ? row0_first : p.seq.cu_q_len[p.tok_seq[row]]) >= TAPS - 1;
+            };
+            const bool here0 = own(r + q), here1 = own(r + q + 1);
+            if (here0 || here1) conv_two_rows<OutT, TAPS>(p, r + q, c, vals + q, w, bias, here0, here1);
         }
-        acc = make_float4(conv_activation(acc.x, p.activation), conv_activation(acc.y, p.activation), conv_activation(acc.z, p.activation),
-                          conv_activation(acc.w, p.activation));
-        *(float4*)(p.out32 + (size_t)r * p.channels + c) = acc;
-        if (typed) {
-            OutT* to = typed + (size_t)r * p.channels + c;
-            to[0] = from_f32<OutT>(acc.x);
-            to[1] = from_f32<OutT>(acc.y);
-            to[2] = from_f32<OutT>(acc.z);
-            to[3] = from_f32<OutT>(acc.w);
-        }
+#pragma unroll
+        for (int m = 0; m < TAPS - 1; ++m) vals[m] = vals[CONV_FOURS_BATCH + m];
     }
 }
 
@@ -266,11 +322,20 @@ FRB_API int frb_causal_conv(const float* in, int in_stride, int in_offset, const
     FRB_DISPATCH_DTYPE(typed_dtype, OutT, {
         // one token a sequence: no row sees only its own step (unless there is one tap, and then no state)
         if (fours && num_rows > num_seqs) {
-            const dim3 grid4((num_rows + CONV_ROWS - 1) / CONV_ROWS, (channels / 4 + 127) / 128);
-            if (taps_count == 4) launch_dependent(causal_conv_rows4_kernel<OutT, 4>, grid4, dim3(128), 0, stream, p);
-            else if (taps_count == 3) launch_dependent(causal_conv_rows4_kernel<OutT, 3>, grid4, dim3(128), 0, stream, p);
-            else launch_dependent(causal_conv_rows4_kernel<OutT, 2>, grid4, dim3(128), 0, stream, p);
-        } else if (taps_count == 1 || num_rows > num_seqs) launch_dependent(causal_conv_rows_kernel<OutT>, grid, dim3(128), 0, stream, p);
+            // as many rows a thread as leave every SM its six blocks, up to 32 (8,192 rows of 6,144 channels: 32 rows 84 us, 16 85, 8 97), so
+            // that a run's first inputs, which the run before has read as well, are few
+            int device = 0, sms = 0;
+            cudaGetDevice(&device);
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+            p.rows_per_thread = 32;
+            while (p.rows_per_thread > 8 && (long long)(num_rows / p.rows_per_thread) * ((channels / 4 + 127) / 128) < 6ll * sms) p.rows_per_thread /= 2;
+            const dim3 fours_grid(num_seqs + (num_rows + p.rows_per_thread - 1) / p.rows_per_thread, (channels / 4 + 127) / 128);
+            if (taps_count == 4) launch_dependent(causal_conv_fours_kernel<OutT, 4>, fours_grid, dim3(128), 0, stream, p, num_seqs);
+            else if (taps_count == 3) launch_dependent(causal_conv_fours_kernel<OutT, 3>, fours_grid, dim3(128), 0, stream, p, num_seqs);
+            else launch_dependent(causal_conv_fours_kernel<OutT, 2>, fours_grid, dim3(128), 0, stream, p, num_seqs);
+            FRB_RETURN_LAUNCH("causal_conv");
+        }
+        if (taps_count == 1 || num_rows > num_seqs) launch_dependent(causal_conv_rows_kernel<OutT>, grid, dim3(128), 0, stream, p);
         if (taps_count > 1) launch_dependent(causal_conv_heads_kernel<OutT>, heads, dim3(128), 0, stream, p);
     });
     FRB_RETURN_LAUNCH("causal_conv");

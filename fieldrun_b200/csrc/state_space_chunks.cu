@@ -18,6 +18,7 @@
 // digits), against 676 us of four launches on mma.sync with a state written and read for every chunk of 128 tokens (states 189, chain
 // 65, outputs 382, pairs 40), and 1,210 token by token.
 #include "f16_parts.cuh"
+#include "silu.cuh"
 #include "tf32_parts.cuh"
 
 #define SC_CHUNK 128          // tokens of the callers' chunks: two of this file's
@@ -58,30 +59,6 @@ struct StateSpaceChunks {
 };
 
 __device__ __forceinline__ float sc_softplus(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
-
-// z / (1 + exp(-z)), of sixteen z.  Below 80 the divisor and its reciprocal are far from the ends of float32: there an approximate reciprocal
-// serves, and the quotient's residual, which fma() has exactly, corrects it (Markstein, IBM Journal of Research and Development 34,
-// 1990).  That alone does not promise the division's bits; a test has them at a million z of each of nine sizes and both signs.  (The
-// residual's sign is that way round so that minus zero stays what it is.)  A division's own branch lets no other work in between: with one
-// for each z launch 3 was bound by these, at 196 us.
-__device__ __forceinline__ void sc_silu(float (&z)[16]) {
-    float top = 0.f;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) top = fmaxf(top, fabsf(z[i]));
-    if (top < 80.f) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const float d = 1.0f + expf(-z[i]);
-            float r;
-            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-            const float q = z[i] * r;
-            z[i] = fmaf(-fmaf(q, d, -z[i]), r, q);
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) z[i] = z[i] / (1.0f + expf(-z[i]));
-    }
-}
 
 // Launch 1.  grid (chunk, group).  A warp takes a row tile of 16 and every other eight columns of the blocks up to it.
 template <int N>
@@ -644,13 +621,13 @@ __global__ void __launch_bounds__(ST_THREADS, 1) state_space_chain_kernel(const 
                     if (t0 + t < count) *(float2*)(out + (size_t)t * p.heads * p.vdim) = y;
                 }
             };
-            sc_silu(gates[0]);
+            silu_of(gates[0]);
             load(c, 1);
             if (!bar_wait(&o_stored, c & 1, failed)) { if (lane == 0) atomicExch(status, 93); }
             __syncwarp();
             write(0);
             if (c + 1 < chunks) load(c + 1, 0);
-            sc_silu(gates[1]);
+            silu_of(gates[1]);
             write(1);
             __syncwarp();
             if (lane == 0) bar_arrive(&o_free[c & 1]);

@@ -107,6 +107,27 @@ def test_convolution_of_four_channels_a_thread_equals_one_channel_a_thread(taps,
         assert a is None or torch.equal(a, b)
 
 
+@pytest.mark.parametrize("lengths", [[2900, 1, 33, 3, 300], [1000, 2, 900, 31]])
+def test_convolution_of_long_runs_of_rows(lengths):
+    """Runs of 32 rows a thread and of 16, sequences that begin and end inside them, sums beyond 80 in size (another form of silu), a state
+    at any offset: the same bits as one channel a thread."""
+    channels, taps, starts, slots = 6144, 4, [3, 0, 6, 1, 8][:len(lengths)], [4, 0, 2, 1, 3][:len(lengths)]
+    gen = torch.Generator(device=DEV).manual_seed(len(lengths))
+    tokens = sum(lengths)
+    rows = torch.randn(tokens, channels, device=DEV, generator=gen)
+    rows[::50] *= 100.0
+    weights, bias = torch.randn(channels, taps, device=DEV, generator=gen), torch.randn(channels, device=DEV, generator=gen)
+    before = torch.randn(5, 2, 3 + (taps - 1) * channels, device=DEV, generator=gen)
+    results = []
+    for offset in (4, 3):
+        shifted = torch.zeros(tokens, channels + 8, device=DEV)
+        shifted[:, offset:offset + channels] = rows
+        state, out32 = before.clone(), torch.full((tokens, channels), float("nan"), device=DEV)
+        ops().causal_conv(shifted, offset, channels, weights, bias, Tables(lengths, starts, slots), state, 3, out32, activation="silu")
+        results.append((out32, state))
+    assert torch.isfinite(results[0][0]).all() and torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
 @pytest.mark.parametrize("decay", ["mild", "strong", "extreme", "mixed"])
 @pytest.mark.parametrize("heads,groups,n,vdim", [(4, 2, 128, 64), (2, 1, 64, 64), (2, 2, 128, 128), (3, 1, 64, 128)])
 def test_state_space_in_chunks(heads, groups, n, vdim, decay):
