@@ -51,6 +51,7 @@ _SIGNATURES = {
     "frb_expert_combine": "pppiiip",
     "frb_expert_gemm_generic": "ppipppppipiiiif",
     "frb_rows_f32": "pppppppipiiif",
+    "frb_dense_rows_f32": "pppiii",
     "frb_weight_scales": "ppli",
     "frb_split_rows": "pppplii" "f",
     "frb_products_f32": "ppippl" "ppif" "ppppip" "iipp",
@@ -111,7 +112,7 @@ _ENTRY_GROUPS = {
     "attention": ("frb_attention_decode_mma", "frb_attention_prefill_mma", "frb_attention_decode_tma", "frb_attention_prefill_tc",
                   "frb_attention_pair_tc"),
     "attention32": ("frb_attention_f32_tiles", "frb_attention_f32_tc", "frb_attention_f32_token"),
-    "streams": ("frb_weight_stream", "frb_expert_gemm_mma", "frb_rows_f32"),
+    "streams": ("frb_weight_stream", "frb_expert_gemm_mma", "frb_rows_f32", "frb_dense_rows_f32"),
     "experts": ("frb_router_topk", "frb_expert_plan", "frb_expert_combine", "frb_expert_gemm_generic", "frb_route_plan_small",
                 "frb_router_small", "frb_router_logits", "frb_scaled_rows"),
     "products": ("frb_expert_gemm_tc", "frb_gather_rows_bf16"),
@@ -1066,6 +1067,16 @@ def rows_f32(w: torch.Tensor, x: torch.Tensor, x_rows: Optional[torch.Tensor], t
         raise KernelError(f"{list(w.shape)} weights with rows {list(x.shape)} into {list(out.shape)}")
     _call("frb_rows_f32", _ptr(w), _ptr(x), _ptr(x_rows), _ptr(tile_expert), _ptr(tile_row0), _ptr(num_tiles), _ptr(offsets), max_tiles,
           _ptr(out), feats, w.shape[2], int(paired), float(gate_limit))
+
+
+def dense_rows_f32(w: torch.Tensor, x: torch.Tensor, out: torch.Tensor) -> None:
+    """out [n, F] = x [n, K] w[F, K]^T in float32 for up to ``ROWS_F32_TILE`` rows, as a stream over the weights (rows_f32.cu); inner
+    sizes in steps of 4."""
+    for t, what in ((w, "weights"), (x, "their input"), (out, "their output")):
+        _want(t, torch.float32, what)
+    if w.dim() != 2 or x.dim() != 2 or x.shape[1] != w.shape[1] or out.shape != (x.shape[0], w.shape[0]):
+        raise KernelError(f"{list(w.shape)} weights with rows {list(x.shape)} into {list(out.shape)}")
+    _call("frb_dense_rows_f32", _ptr(w), _ptr(x), _ptr(out), x.shape[0], w.shape[0], w.shape[1])
 
 
 PRODUCTS_F32_TILE = 160    # rows of a tile of products_f32

@@ -38,6 +38,32 @@ __device__ __forceinline__ float rf_dot4(float4 a, float4 b, float c) {
     return fmaf(a.w, b.w, c);
 }
 
+// The sums of a warp's lanes, added by halves: value i of N ends in to[i].
+template <int N>
+__device__ __forceinline__ void rf_join(float (&acc)[N], int lane, float* to) {
+    __syncwarp();
+    int n = N;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (n > 1) {
+            n /= 2;
+            const bool upper = (lane & o) != 0;
+#pragma unroll
+            for (int i = 0; i < N / 2; ++i) {
+                if (i >= n) break;
+                const float keep = upper ? acc[i + n] : acc[i], send = upper ? acc[i] : acc[i + n];
+                acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+        } else {
+            acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+        }
+    }
+    constexpr int LEFT = N > 32 ? N / 32 : 1, SHARE = N < 32 ? 32 / N : 1;
+#pragma unroll
+    for (int j = 0; j < LEFT; ++j)
+        if (lane % SHARE == 0) to[lane / SHARE * LEFT + j] = acc[j];
+}
+
 // One warp: eight weight rows (`w`, their addresses) with R rows of x over the 16-byte units [begin, end) of the inner size.
 // Value f * R + r, weight row f with row r, ends in to[f * R + r]: the lanes' sums meet by halves.
 template <int R>
@@ -74,27 +100,7 @@ __device__ __forceinline__ void rf_products(float4* ring, const float* const (&w
         stage = (stage + 1) % RF_STAGES;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncwarp();
-    int n = N;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        if (n > 1) {
-            n /= 2;
-            const bool upper = (lane & o) != 0;
-#pragma unroll
-            for (int i = 0; i < N / 2; ++i) {
-                if (i >= n) break;
-                const float keep = upper ? acc[i + n] : acc[i], send = upper ? acc[i] : acc[i + n];
-                acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-            }
-        } else {
-            acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
-        }
-    }
-    constexpr int LEFT = N > 32 ? N / 32 : 1, SHARE = N < 32 ? 32 / N : 1;
-#pragma unroll
-    for (int j = 0; j < LEFT; ++j)
-        if (lane % SHARE == 0) to[lane / SHARE * LEFT + j] = acc[j];
+    rf_join<N>(acc, lane, to);
 }
 
 // PARTS: warps that share eight weight rows, each with its part of the inner size.
@@ -141,6 +147,194 @@ __global__ void __launch_bounds__(32 * RF_WARPS, 3) rows_f32_kernel(RowsParams p
         }
         if (f < p.F && r < rows) p.out[(size_t)(row0 + r) * p.F + f] = PAIRED ? paired_gate(sum, up, p.gate_limit) : sum;
     }
+}
+
+__device__ __forceinline__ uint64_t rf_pair(float lo, float hi) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+
+__device__ __forceinline__ void rf_fma_pair(uint64_t a, uint64_t b, uint64_t& c) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b)); }
+
+// Four entries of R rows of x; PAIRS: two rows at a time, for the same multiply-adds in half the instructions.
+template <int R, bool PAIRS>
+struct RowsOfX {
+    float4 one[PAIRS ? 1 : R];
+    uint64_t two[PAIRS ? R / 2 : 1][4];
+};
+
+template <int R, bool PAIRS>
+__device__ __forceinline__ void rf_load_x(RowsOfX<R, PAIRS>& to, const float* const (&x)[R], int u, int end) {
+#pragma unroll
+    for (int r = 0; r < R; r += PAIRS ? 2 : 1) {
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), a = u < end ? *(const float4*)(x[r] + 4 * u) : zero;
+        if (PAIRS) {
+            const float4 b = u < end ? *(const float4*)(x[r + PAIRS] + 4 * u) : zero;
+            to.two[r / 2][0] = rf_pair(a.x, b.x);
+            to.two[r / 2][1] = rf_pair(a.y, b.y);
+            to.two[r / 2][2] = rf_pair(a.z, b.z);
+            to.two[r / 2][3] = rf_pair(a.w, b.w);
+        } else {
+            to.one[r] = a;
+        }
+    }
+}
+
+// A dense product of up to eight rows: one matrix, no lists.  A block an SM for the whole launch takes its share of the weight rows (their
+// number over the blocks, to the row), eight at a time; its warps have a part of the inner size each, always the same one, and add theirs
+// in their order.  A warp's ring runs on from eight rows to the next and begins ahead of the wait for the kernel before: weights are no
+// kernel's result.  The rows of x stay in registers where a warp's part has at most HELD runs of them, else the next run's are asked for
+// ahead.  `tiles`: two where five to eight rows would not fit so; neighbouring blocks then have four rows each and the same weights.
+//
+// Bound by the weights' bytes up to four rows, beyond by the multiply-adds and the joins.  The kernel above, whose blocks begin and end
+// once for 32 KB to 96 KB of weights, and this one in a stream of launches, microseconds for 1, 4 and 8 rows: 8192 x 3072 weights 19.9 25.0
+// 29.4 | 15.8 16.3 20.7 (15.4 at the memory's rate), 3072 x 6144 15.5 17.5 19.8 | 12.3 13.3 19.3, 1024 x 1024 3.3 3.8 4.6 | 1.9 2.1 2.5,
+// 144 x 96 2.0 2.1 2.3 | 1.2 1.3 1.7.  Only with very many weight rows do a single row's joins cost more than that: 65536 x 3072 113 | 118,
+// 200064 x 3072 336 | 352; with two rows 362 | 358, with eight 419 | 377.  Rows two by two (fma.rn.f32x2) pay where the work is large enough
+// for eight rows' multiply-adds to bound it: 200064 x 3072 414 -> 377, 8192 x 3072 21.8 -> 20.7, but 1024 x 1024 2.5 -> 3.2.
+#define RD_WARPS 12
+
+template <int R, int HELD>
+__global__ void __launch_bounds__(32 * RD_WARPS, 1) dense_rows_f32_kernel(const float* __restrict__ W, const float* X, float* __restrict__ out,
+                                                                          int all_rows, int tiles, int F, int K) {
+    extern __shared__ float4 rf_smem[];
+    __shared__ float sums[2][RD_WARPS][RF_FEATS * R];
+    let_next_kernel_start();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int share = blockIdx.x / tiles, shares = gridDim.x / tiles, tile = blockIdx.x - share * tiles;
+    const int row0 = tile * R, rows = min(all_rows - row0, R);
+    X += (size_t)row0 * K;
+    out += (size_t)row0 * F;
+    const int f_begin = (int)((long long)F * share / shares), f_end = (int)((long long)F * (share + 1) / shares);
+    const int units = K >> 2, part = (units + 8 * warps - 1) / (8 * warps) * 8;               // whole lines of 128 bytes
+    const int begin = min(warp * part, units), end = min(begin + part, units), with_work = (units + part - 1) / part;
+    const int runs = (end - begin + 31) / 32, groups = (f_end - f_begin + RF_FEATS - 1) / RF_FEATS, all = groups * runs;
+    float4* ring = rf_smem + warp * RF_STAGES * RF_FEATS * 32 + lane;
+    // the place of the next run to be copied
+    const float* from = W + (size_t)f_begin * K;
+    int copy_run = 0, copy_left = f_end - f_begin, copied = 0;
+    auto copy = [&](int stage) {
+        if (copied < all) {
+            const int u = begin + 32 * copy_run + lane;
+            if (u < end)
+#pragma unroll
+                for (int f = 0; f < RF_FEATS; ++f)
+                    if (f < copy_left) rf_copy16(ring + (stage * RF_FEATS + f) * 32, from + (size_t)f * K + 4 * u);
+            ++copied;
+            if (++copy_run == runs) { copy_run = 0; copy_left -= RF_FEATS; from += (size_t)RF_FEATS * K; }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int s = 0; s < RF_STAGES - 1; ++s) copy(s);
+    wait_for_previous_kernel();
+    const float* x[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) x[r] = X + (size_t)min(r, rows - 1) * K;
+    constexpr bool PAIRS = R == 8 && HELD == 2;
+    RowsOfX<R, PAIRS> held[HELD ? HELD : 1];
+    auto load_x = [&](RowsOfX<R, PAIRS>& to, int run) { rf_load_x<R, PAIRS>(to, x, begin + 32 * run + lane, end); };
+#pragma unroll
+    for (int h = 0; h < (HELD ? HELD : 1); ++h) load_x(held[h], h);
+    float acc[PAIRS ? 1 : RF_FEATS * R];
+    uint64_t acc2[PAIRS ? RF_FEATS * R / 2 : 1];
+    int stage = 0;
+    auto multiply = [&](const RowsOfX<R, PAIRS>& xv, int run) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(RF_STAGES - 1) : "memory");
+        if (begin + 32 * run + lane < end)
+#pragma unroll
+            for (int f = 0; f < RF_FEATS; ++f) {
+                const float4 wv = ring[(stage * RF_FEATS + f) * 32];
+                if (PAIRS) {
+                    const uint64_t w2[4] = {rf_pair(wv.x, wv.x), rf_pair(wv.y, wv.y), rf_pair(wv.z, wv.z), rf_pair(wv.w, wv.w)};
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+#pragma unroll
+                        for (int r = 0; r < R / 2; ++r) rf_fma_pair(w2[k], xv.two[r][k], acc2[f * (R / 2) + r]);
+                } else {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) acc[f * R + r] = rf_dot4(wv, xv.one[r], acc[f * R + r]);
+                }
+            }
+        stage = (stage + 1) % RF_STAGES;
+    };
+#pragma unroll 1
+    for (int g = 0; g < groups; ++g) {
+        if (PAIRS) {
+#pragma unroll
+            for (int i = 0; i < RF_FEATS * R / 2; ++i) acc2[i] = 0;
+        } else {
+#pragma unroll
+            for (int i = 0; i < RF_FEATS * R; ++i) acc[i] = 0.f;
+        }
+        if (HELD) {
+#pragma unroll
+            for (int h = 0; h < HELD; ++h)
+                if (h < runs) {
+                    copy((stage + RF_STAGES - 1) % RF_STAGES);
+                    multiply(held[h], h);
+                }
+        } else {
+#pragma unroll 1
+            for (int run = 0; run < runs; ++run) {
+                RowsOfX<R, PAIRS> next;
+                copy((stage + RF_STAGES - 1) % RF_STAGES);
+                load_x(next, run + 1 < runs ? run + 1 : 0);
+                multiply(held[0], run);
+                held[0] = next;
+            }
+        }
+        float each[RF_FEATS * R];
+#pragma unroll
+        for (int i = 0; i < RF_FEATS * R; ++i) {
+            if (!PAIRS) each[i] = acc[i];
+            else if (i % 2 == 0) asm("mov.b64 {%0, %1}, %2;" : "=f"(each[i]), "=f"(each[i + 1]) : "l"(acc2[i / 2]));
+        }
+        rf_join<RF_FEATS * R>(each, lane, sums[g & 1][warp]);
+        __syncthreads();                                                 // the sums of two groups back are read by then
+        for (int v = threadIdx.x; v < RF_FEATS * R; v += blockDim.x) {
+            const int r = v % R, f = f_begin + g * RF_FEATS + v / R;
+            float sum = 0.f;
+            for (int k = 0; k < with_work; ++k) sum += sums[g & 1][k][v];
+            if (f < f_end && r < rows) out[(size_t)r * F + f] = sum;
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// out [rows, F] = X [rows, K] W^T, W [F][K], all float32; up to eight rows.
+FRB_API int frb_dense_rows_f32(const float* W, const float* X, float* out, int rows, int F, int K, cudaStream_t stream) {
+    if (rows == 0 || F == 0) return 0;
+    FRB_CHECK_ARG(rows > 0 && rows <= RF_ROWS, "dense float32 rows: %d rows are outside 1..%d", rows, RF_ROWS);
+    FRB_CHECK_ARG(K > 0 && K % 4 == 0, "dense float32 rows: an inner size of %d is not a multiple of 4", K);
+    FRB_CHECK_ARG((((uintptr_t)W | (uintptr_t)X) & 15) == 0, "dense float32 rows: operands must be 16-byte aligned");
+    int device = 0, sms = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const int units = K / 4, warps = units >= 32 * RD_WARPS ? RD_WARPS : (units + 31) / 32;
+    const int part = (units + 8 * warps - 1) / (8 * warps) * 8, runs = (part + 31) / 32;
+    // (with two tiles everywhere: 8192 x 3072 24.9 instead of 20.7, 2048 x 8192 23.6 instead of 19.9; with one 3072 x 6144 20.9 instead of 19.3)
+    const int tiles = rows > 4 && runs > 2 && runs <= 4 ? 2 : 1, groups = (F + RF_FEATS - 1) / RF_FEATS;
+    const int shares = groups < sms / tiles ? groups : sms / tiles, blocks = shares * tiles;
+    const size_t smem = (size_t)warps * RF_STAGES * RF_FEATS * 32 * sizeof(float4);
+#define FRB_DENSE(R, HELD)                                                                                                            do {                                                                                                                                  if (smem > 40 * 1024)                                                                                                                 cudaFuncSetAttribute(dense_rows_f32_kernel<R, HELD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                 launch_dependent(dense_rows_f32_kernel<R, HELD>, dim3(blocks), dim3(32 * warps), smem, stream, W, X, out, rows, tiles, F, K);        } while (0)
+#define FRB_DENSE_ROWS(R)                                                                                                         \
+    do {                                                                                                                          \
+        if (runs == 1) FRB_DENSE(R, 1);                                                                                           \
+        else if (runs == 2) FRB_DENSE(R, 2);                                                                                      \
+        else if (runs <= 4) FRB_DENSE(R, 4);                                                                                      \
+        else FRB_DENSE(R, 0);                                                                                                     \
+    } while (0)
+    if (rows == 1) FRB_DENSE_ROWS(1);
+    else if (rows == 2) FRB_DENSE_ROWS(2);
+    else if (rows <= 4 || tiles == 2) FRB_DENSE_ROWS(4);
+    else if (runs == 1) FRB_DENSE(8, 1);
+    else if (runs == 2) FRB_DENSE(8, 2);
+    else FRB_DENSE(8, 0);
+#undef FRB_DENSE_ROWS
+#undef FRB_DENSE
+    FRB_RETURN_LAUNCH("dense_rows_f32");
 }
 
 // W [E][(paired ? 2 : 1) * F][K]; X rows of K; out [N, F], all float32.  x_rows (nullable) maps a sorted row to its X row.

@@ -20,6 +20,8 @@ _ONE_TILE: dict[tuple[str, int], tuple[torch.Tensor, torch.Tensor, torch.Tensor,
 STREAM_ROWS = 8           # up to this many rows a dense product is a stream over the weight (experts_stream.cu); beyond, each
                           # item's rows of x are as many bytes as its weights and the library's product is faster (measured at
                           # 12 to 32 rows on a B200: 14 to 25 us against 11 for MiniMax-M2's projections)
+ONE_ROW_FEATURES = 65536  # from this many output features on a single float32 row's product is faster by the experts' kernel (rows_f32.cu;
+                          # 3,072 inputs, 32,768 features 60.6 us against 60.0, 65,536 113 against 118)
 STREAM_FEATURES = 65536   # beyond this many output features the library product is at the memory roofline anyway
 
 
@@ -107,8 +109,11 @@ def linear(rows: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor]
                 and (ops.rows_f32_takes(rows.shape[1]) if few else ops.products_f32_take(rows.shape[1])):
             result = out if out is not None else torch.empty((rows.shape[0], weight.shape[0]), dtype=torch.float32, device=rows.device)
             if few:
-                tile_expert, tile_row0, num_tiles, offsets = one_tile(rows.device, rows.shape[0])
-                ops.rows_f32(weight.unsqueeze(0), rows, None, tile_expert, tile_row0, num_tiles, offsets, 1, result, paired=False)
+                if rows.shape[0] == 1 and weight.shape[0] >= ONE_ROW_FEATURES:
+                    tile_expert, tile_row0, num_tiles, offsets = one_tile(rows.device, 1)
+                    ops.rows_f32(weight.unsqueeze(0), rows, None, tile_expert, tile_row0, num_tiles, offsets, 1, result, paired=False)
+                else:
+                    ops.dense_rows_f32(weight, rows, result)
             else:
                 parts = torch.empty((2, *rows.shape), dtype=torch.float16, device=rows.device)
                 scale = torch.empty(rows.shape[0], dtype=torch.float32, device=rows.device)

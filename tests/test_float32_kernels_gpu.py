@@ -123,6 +123,22 @@ def test_rows_equal_the_general_kernel(features, inner, paired, limit):
     assert (got - want).abs().max() < 4 * max(inner, 16) * 2.0 ** -24 * max(want.abs().max().item(), 1.0)
 
 
+@pytest.mark.parametrize("features,inner", [(1, 4), (7, 96), (130, 132), (2500, 1024), (1185, 2048), (601, 3072), (300, 4100), (149, 6144), (74, 6200), (33, 12300)])
+def test_dense_rows_of_every_number(features, inner):
+    """Parts of the inner size that fill no run, one to more than four of them, shares of a block that end inside eight weight rows; inputs and
+    results behind the last row stay as they are.  Sums of `inner` terms of size one: off by less than inner roundings of the largest."""
+    gen = torch.Generator(device=DEV).manual_seed(features + inner)
+    w = torch.randn(features, inner, device=DEV, generator=gen) * inner ** -0.5
+    for rows in range(1, 9):
+        x = torch.full((rows + 1, inner), float("nan"), device=DEV)
+        x[:rows] = torch.randn(rows, inner, device=DEV, generator=gen)
+        got = torch.full((rows + 1, features), 7.0, device=DEV)
+        ops().dense_rows_f32(w, x[:rows], got[:rows])
+        want = x[:rows].double() @ w.double().T
+        assert (got[:rows] - want).abs().max() < 2 * max(inner, 16) * 2.0 ** -24 * max(want.abs().max().item(), 1.0)
+        assert (got[rows] == 7.0).all()
+
+
 def split_product(w, x, lists=None, max_tiles=0, source=None, gated=False, limit=0.0):
     """w [E, F, K] times the rows of x (of ``source``) by the tensor cores' float32 products."""
     count = len(source) if source is not None else x.shape[0]

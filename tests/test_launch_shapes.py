@@ -63,6 +63,8 @@ def test_float32_rows_are_checked_against_the_weights_before_a_launch():
     for x, out in ((torch.zeros(2, 8), torch.zeros(2, 16)), (torch.zeros(2, 12), torch.zeros(2, 8)), (torch.zeros(3, 12), torch.zeros(2, 16))):
         with pytest.raises(ops.KernelError, match="with rows"):
             ops.rows_f32(torch.zeros(1, 16, 12), x, None, *lists, tile, out, paired=False)
+        with pytest.raises(ops.KernelError, match="with rows"):
+            ops.dense_rows_f32(torch.zeros(16, 12), x, out)
 
 
 @pytest.mark.parametrize("hidden,heads,dim,experts,width,vocab,expected", [
