@@ -170,17 +170,34 @@ class _Group:
 
     def sync(self) -> None:
         if self.table_dev is not None:
-            for slot, lo, hi in self.dirty:
-                self.table_dev[slot, lo:hi].copy_(torch.from_numpy(self.table[slot, lo:hi]))
-            if len(self.fresh) == 1:
-                self.keys[:, self.fresh[0]].zero_()
-                self.values[:, self.fresh[0]].zero_()
-            elif self.fresh:
-                pages = torch.tensor(self.fresh, dtype=torch.int64).to(self.keys.device)
-                self.keys.index_fill_(1, pages, 0)
-                self.values.index_fill_(1, pages, 0)
+            if len(self.dirty) + len(self.fresh) > 2:
+                self.sync_many()
+            else:
+                for slot, lo, hi in self.dirty:
+                    self.table_dev[slot, lo:hi].copy_(torch.from_numpy(self.table[slot, lo:hi]))
+                for page in self.fresh:
+                    self.keys[:, page].zero_()
+                    self.values[:, page].zero_()
         self.dirty.clear()
         self.fresh.clear()
+
+
+    def sync_many(self) -> None:
+        """The same with one copy to the device for all of it: the changed places of the table, the pages to be cleared, and the
+        places' entries, two in each of the copy's integers.  (A copy for each sequence was a fifth of a short prompt step's time
+        on the host, with four sequences 200 us of 1,100.)"""
+        width = self.table.shape[1]
+        places = np.concatenate([np.arange(slot * width + lo, slot * width + hi) for slot, lo, hi in self.dirty] or [np.zeros(0, np.int64)])
+        n, pages = len(places), len(self.fresh)
+        sent = np.zeros(n + pages + (n + 1) // 2, dtype=np.int64)
+        sent[:n], sent[n:n + pages] = places, self.fresh
+        sent[n + pages:].view(np.int32)[:n] = self.table.reshape(-1)[places]
+        dev = torch.from_numpy(sent).to(self.table_dev.device)
+        if n:
+            self.table_dev.view(-1).index_copy_(0, dev[:n], dev[n + pages:].view(torch.int32)[:n])
+        if pages:
+            self.keys.index_fill_(1, dev[n:n + pages], 0)
+            self.values.index_fill_(1, dev[n:n + pages], 0)
 
 
 class SequenceCache:

@@ -14,6 +14,7 @@ import torch
 from . import build as _build
 
 _LIBS: dict[str, ctypes.CDLL] = {}
+_FUNCTIONS: dict = {}          # entry points of the libraries loaded so far, by name
 _LIB_PATHS: dict[str, str] = {}
 
 _P, _I, _F, _L = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_longlong
@@ -143,6 +144,7 @@ def prepare(groups) -> None:
             fn = getattr(lib, name)
             fn.restype = _I
             fn.argtypes = [_CTYPE[c] for c in _SIGNATURES[name]] + [_P]
+            _FUNCTIONS[name] = fn
         _LIBS[group], _LIB_PATHS[group] = lib, paths[group]
 
 
@@ -171,6 +173,7 @@ def register(name: str, spec: str, group: str = "extras") -> None:
         fn = getattr(_LIBS[group], name)
         fn.restype = _I
         fn.argtypes = [_CTYPE[c] for c in spec] + [_P]
+        _FUNCTIONS[name] = fn
 
 
 def _code(dtype: torch.dtype) -> int:
@@ -184,21 +187,22 @@ def _code(dtype: torch.dtype) -> int:
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     if t is None:
         return None
+    if t.is_cuda and t.is_contiguous():
+        return t.data_ptr()
     if not t.is_cuda:
         raise KernelError("a CPU tensor was given to a CUDA kernel; fieldrun_b200 has no CPU path")
-    if not t.is_contiguous():
-        raise KernelError("a kernel was given a tensor that is not contiguous")
-    return t.data_ptr()
+    raise KernelError("a kernel was given a tensor that is not contiguous")
 
 
 _RAW_STREAM = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_DEVICE = getattr(torch._C, "_cuda_getDevice", None)
 
 
 def _stream() -> int:
     """The current stream's handle.  The direct call costs a fraction of a microsecond; building a
     ``torch.cuda.Stream`` object for every kernel of a step was a tenth of a short prompt's time on the host."""
-    if _RAW_STREAM is not None:
-        return _RAW_STREAM(torch.cuda.current_device())
+    if _RAW_STREAM is not None and _DEVICE is not None:
+        return _RAW_STREAM(_DEVICE())                      # a tensor of the device is among the arguments: it is set up
     return torch.cuda.current_stream().cuda_stream
 
 
@@ -262,14 +266,17 @@ class timed:
 
 def _call(name: str, *args) -> None:
     global _LAUNCHES
-    lib = library(_GROUP_OF[name])
+    fn = _FUNCTIONS.get(name)
+    if fn is None:
+        fn = getattr(library(_GROUP_OF[name]), name)
     if _TIMINGS is not None:
         with timed(name[4:]):
-            status = getattr(lib, name)(*args, _stream())
+            status = fn(*args, _stream())
     else:
-        status = getattr(lib, name)(*args, _stream())
+        status = fn(*args, _stream())
     _LAUNCHES += _KERNELS_PER_CALL.get(name, 1)
     if status != 0:
+        lib = library(_GROUP_OF[name])
         raise KernelError(f"{name}: {lib.frb_last_error().decode(errors='replace')} (status {status})")
 
 

@@ -1,5 +1,6 @@
 import random
 
+import numpy as np
 import pytest
 
 from fieldrun_b200.cache import CacheFull, CacheNeed, IndexPool, PAGE_TOKENS, SequenceCache, pages_for
@@ -139,3 +140,27 @@ def test_random_traffic_loses_nothing():
         cache.free(s)
     cache.check()
     assert all(g.pool.num_held == 0 for g in cache.groups)
+
+
+def test_the_tables_of_many_sequences_reach_the_device_whole():
+    """Steps of several sequences, with pages given back by a window between them and handed out again: the device's table is the host's, and
+    the pages that a step hands out in part are cleared, no others."""
+    import torch
+    rng = np.random.default_rng(5)
+    cache = SequenceCache([CacheNeed(1, 4, 70)], max_tokens=64 * 40, num_slots=6, dtype=torch.float32, device="cpu")
+    group = cache.groups[0]
+    held = [cache.alloc() for _ in range(5)]
+    for step in range(12):
+        if step % 5 == 4:
+            cache.free(held.pop(0))
+            held.append(cache.alloc())
+        new = [int(n) for n in rng.integers(1, 130, size=len(held))]
+        group.keys.fill_(3.0)
+        group.values.fill_(4.0)
+        before = group.end_page.copy()
+        cache.begin_step(held, new)
+        partial = {int(group.table[s, group.end_page[s] - 1]) for s, n in zip(held, new) if group.end_page[s] > before[s] and (cache.length(s) + n) % 64}
+        cleared = {p for p in range(group.num_pages) if (group.keys[:, p] == 0).all() and (group.values[:, p] == 0).all()}
+        assert cleared == partial and ((group.keys == 0) | (group.keys == 3.0)).all()
+        assert np.array_equal(group.table_dev.numpy(), group.table)
+        cache.end_step(held, new)
