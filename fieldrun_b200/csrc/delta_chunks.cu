@@ -8,7 +8,7 @@
 //     o_i = w(i) S^T q_i + sum_(j <= i) w(j, i) (q_i . k_j) u_j,   S <- w(end) S + sum_j w(j, end) k_j u_j^T.
 //   1. every chunk and key head side by side: the products of the unit keys with one another and with the unit queries;
 //   2. every chunk and head side by side: the weights, M and the pairs' weights for o; then (I + M) X = [beta w k | beta v] by
-//      substitution, a thread a column, in float32: W and U' with u = U' - W S.  (The entries of (I + M)^(-1) are at most one: each is
+//      substitution, two threads for two columns, in float32: W and U' with u = U' - W S.  (The entries of (I + M)^(-1) are at most one: each is
 //      what is left of a unit of v_j under steps that shorten, times beta k_i.)
 //   3. along the chunks of a sequence, a block that keeps the state in registers: u = U' - W S, o, and the new state.  Heads of 128 value
 //      columns: on tcgen05, a block a (sequence, head); of 64: on mma.sync.
@@ -18,11 +18,11 @@
 // tokens inside a block and up to 48 between blocks: a rounding of their logarithms, which are large only where the weight is small.
 //
 // Everything is float32; the products run on tensor cores with each operand as two parts (tf32_parts.cuh: sums of 16 entries, added in
-// float32 registers; f16_parts.cuh: of at most 128).  Four prompts of 2,048 tokens, 16 heads of 128 x 128 over 4 key heads: 345 us (34 +
-// 153 + 129 + 35 for the launches in turn; 34 + 151 + 129 + 35 without the pairs' scales of single rows and the look at the outputs that
-// they are for; delta_rule.cu token by token 1,367).  With launch 1's products made by launch 2 for every head, and
-// launch 3 on mma.sync, 589 (189 + 368 + 34).  Launch 2 is bound by the instructions of its substitution, two entries each (one
-// each: 168 us), and by the latencies before it, two blocks an SM; launch 3 by the chain of its phases.
+// float32 registers; f16_parts.cuh: of at most 128).  Four prompts of 2,048 tokens, 16 heads of 128 x 128 over 4 key heads: 320 us (34 +
+// 128 + 129 + 34 for the launches in turn; the pairs' scales of single rows and the look at the outputs that they are for cost launch 2 two
+// of its microseconds; delta_rule.cu token by token 1,367).  With launch 1's products made by launch 2 for every head, and
+// launch 3 on mma.sync, 589 (189 + 368 + 34).  Launch 2 is bound by its substitution's reads of M from shared memory and by the
+// latencies before it, two blocks an SM; launch 3 by the chain of its phases.
 #include "f16_parts.cuh"
 #include "tf32_parts.cuh"
 
@@ -193,13 +193,27 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
     const size_t row0 = (size_t)p.cu_q_len[b] + p.chunk_begin[item], at = (size_t)item * p.heads + h, kv_at = (size_t)item * p.kv_heads + kvh;
     const float* rows = p.conv + row0 * p.conv_stride;
 
-    // the substitution's right-hand side, a column of [k | v] a thread, on its way meanwhile
-    float x[DC_TOKENS];
-    const bool key = tid < DIM;
+    // the substitution's right-hand side, two columns of [k | v] for two neighbouring threads, on its way meanwhile: thread r of the two has
+    // the rows 8 g + 4 r .. + 3
+    float x[2][DC_TOKENS / 2];
+    const int column = tid & ~1, r = tid & 1;
+    const bool key = column < DIM;
+    const auto row_of = [&](int i) { return 2 * (i & ~3) + 4 * r + (i & 3); };
     if (tid < DIM + VDIM) {
-        const float* column = rows + (key ? p.k_off + kvh * DIM + tid : p.v_off + h * VDIM + tid - DIM);
+        const float* from = rows + (key ? p.k_off + kvh * DIM + column : p.v_off + h * VDIM + column - DIM);
+        const bool pairs_of_columns = key || (p.v_off & 1) == 0;         // the keys' rows are in steps of 16 bytes
 #pragma unroll
-        for (int i = 0; i < DC_TOKENS; ++i) x[i] = column[(size_t)min(i, count - 1) * p.conv_stride];
+        for (int i = 0; i < DC_TOKENS / 2; ++i) {
+            const float* at_row = from + (size_t)min(row_of(i), count - 1) * p.conv_stride;
+            if (pairs_of_columns) {
+                const float2 v = *(const float2*)at_row;
+                x[0][i] = v.x;
+                x[1][i] = v.y;
+            } else {
+                x[0][i] = at_row[0];
+                x[1][i] = at_row[1];
+            }
+        }
     }
     // a token a thread: beta; the logarithms of the decays from its block's start (with its own) and to its block's end
     if (tid < DC_TOKENS) {
@@ -320,43 +334,67 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_solve_kernel(DeltaChunks p
     }
     __syncthreads();
 
-    // substitution: a thread a column of [beta w k | beta v], its 64 entries in registers
-    if (tid < DIM + VDIM) {
-        if (key) {
+    // substitution: two threads for two columns of [beta w k | beta v], each with half of the rows of both.  It is bound by the reads of M, one
+    // entry a cycle for a whole warp: with two columns a thread they are half as many as with one (launch 2: 128 us instead of 153; with
+    // four columns and four threads, whose exchanges are twice as many, 144; with two threads a column, 64 registers each, 178).
+    if (tid >= DIM + VDIM) return;
 #pragma unroll
-            for (int i = 0; i < DC_TOKENS; ++i) x[i] = i < count ? beta_s[i] * start_s[i] * k_inv[i] * x[i] : 0.f;
-        } else {
+    for (int i = 0; i < DC_TOKENS / 2; ++i) {
+        const int row = row_of(i);
+        const float factor = key ? beta_s[row] * start_s[row] * k_inv[row] : beta_s[row];
 #pragma unroll
-            for (int i = 0; i < DC_TOKENS; ++i) x[i] = i < count ? x[i] * beta_s[i] : 0.f;
+        for (int c = 0; c < 2; ++c) x[c][i] = row < count ? factor * x[c][i] : 0.f;
+    }
+    const int lane = tid & 31, width = key ? DIM : VDIM;
+    float* to = key ? p.w + at * DC_TOKENS * DIM + column : p.u + at * DC_TOKENS * VDIM + column - DIM;
+    uint16_t* w_parts = p.w_parts + at * 2 * DC_TOKENS * DIM;
+    // four rows at a time, which one of the two threads has: it settles them among themselves, both learn them, and they leave every later row
+#pragma unroll
+    for (int g = 0; g < DC_TOKENS / 4; ++g) {
+        const int own_group = g >> 1, owner = g & 1;
+        const float* m = m_s + 4 * g * LS;
+        const float4 m0 = *(const float4*)(m + 4 * g), m1 = *(const float4*)(m + LS + 4 * g), m2 = *(const float4*)(m + 2 * LS + 4 * g);
+        float d[2][4];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const float* from = x[c] + 4 * own_group;
+            d[c][0] = from[0];
+            d[c][1] = fmaf(m0.y, -d[c][0], from[1]);
+            d[c][2] = fmaf(m1.z, -d[c][1], fmaf(m0.z, -d[c][0], from[2]));
+            d[c][3] = fmaf(m2.w, -d[c][2], fmaf(m1.w, -d[c][1], fmaf(m0.w, -d[c][0], from[3])));
+#pragma unroll
+            for (int e = 0; e < 4; ++e) d[c][e] = __shfl_sync(0xffffffffu, d[c][e], (lane & ~1) | owner);
         }
-        float* to = key ? p.w + at * DC_TOKENS * DIM + tid : p.u + at * DC_TOKENS * VDIM + tid - DIM;
-        uint16_t* w_parts = p.w_parts + at * 2 * DC_TOKENS * DIM;
-        const int width = key ? DIM : VDIM;
-        // an entry once it is final leaves every later one: those do not depend on one another
 #pragma unroll
-        for (int i = 0; i < DC_TOKENS; ++i) {
-            const float* m = m_s + i * LS;
-            const float done = x[i];
-            if (!PARTS || !key) to[(size_t)i * width] = done;
-            else if (i & 1) {                        // two columns' entries of two rows: a lane of the two has one row's
-                const bool odd_column = tid & 1;
-                const float theirs = __shfl_xor_sync(0xffffffffu, odd_column ? x[i - 1] : done, 1);
-                const int r = odd_column ? i : i - 1;
-                const float scale = w_scale[r];
+        for (int e = 0; e < 2; ++e) {                // a thread writes two of the four rows
+            const int row = 4 * g + 2 * r + e;
+            const float first = r ? d[0][2 + e] : d[0][e], second = r ? d[1][2 + e] : d[1][e];
+            if (!PARTS || !key) {
+                *(float2*)(to + (size_t)row * width) = make_float2(first, second);
+            } else {
+                const float scale = w_scale[row];
                 uint32_t hi, lo;
-                split_two(mul_pairs(odd_column ? pair_of(theirs, done) : pair_of(x[i - 1], theirs), pair_of(scale, scale)), hi, lo);
-                uint16_t* parts = w_parts + piece_place(r, tid & ~1);
+                split_two(mul_pairs(pair_of(first, second), pair_of(scale, scale)), hi, lo);
+                uint16_t* parts = w_parts + piece_place(row, column);
                 *(uint32_t*)parts = hi;
                 *(uint32_t*)(parts + DC_TOKENS * DIM) = lo;
             }
-            const uint64_t leaves = pair_of(-done, -done);
-#pragma unroll
-            for (int j = (i + 1) & ~3; j < DC_TOKENS; j += 4) {      // two entries at a time; M is zero up to its diagonal
-                const ulonglong2 w = *(const ulonglong2*)(m + j);
-                if (j + 1 > i) halves_of(fma_pairs(w.x, leaves, pair_of(x[j], x[j + 1])), x[j], x[j + 1]);
-                halves_of(fma_pairs(w.y, leaves, pair_of(x[j + 2], x[j + 3])), x[j + 2], x[j + 3]);
-            }
         }
+        const float* later = m + 4 * r;
+#pragma unroll
+        for (int l = own_group + owner; l < DC_TOKENS / 8; ++l)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {                                // two rows at a time
+                ulonglong2 w = *(const ulonglong2*)(later + e * LS + 8 * l);
+                if (l == own_group && r == 0) w = make_ulonglong2(0, 0); // the rows themselves
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const uint64_t leaves = pair_of(-d[c][e], -d[c][e]);
+                    float* y = x[c] + 4 * l;
+                    halves_of(fma_pairs(w.x, leaves, pair_of(y[0], y[1])), y[0], y[1]);
+                    halves_of(fma_pairs(w.y, leaves, pair_of(y[2], y[3])), y[2], y[3]);
+                }
+            }
     }
 }
 

@@ -165,6 +165,30 @@ def test_state_space_in_chunks(heads, groups, n, vdim, decay):
     assert torch.equal(results[1][1], state)                     # nothing else was written
 
 
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(2, 1, 128, 128), (2, 1, 64, 64), (2, 2, 128, 64), (1, 1, 64, 128)])
+def test_values_of_the_delta_rule_at_any_offset(heads, kv_heads, dim, vdim):
+    """Values that begin on 16 bytes, on 8, and on 4 alone (read two columns at a time or one): the same bits."""
+    gen = torch.Generator(device=DEV).manual_seed(dim + vdim)
+    lengths, starts, slots = [130, 1, 63, 64], [0, 3, 10, 6], [3, 0, 2, 1]
+    tokens, qk, inner = sum(lengths), kv_heads * dim, heads * vdim
+    rows, proj = torch.randn(tokens, 2 * qk + inner, device=DEV, generator=gen), torch.randn(tokens, 2 * heads + inner, device=DEV, generator=gen)
+    a_log, dt_bias, norm = (torch.randn(n, device=DEV, generator=gen) * 0.2 + 1.0 for n in (heads, heads, vdim))
+    state = torch.randn(4, 2, heads * dim * vdim, device=DEV, generator=gen)
+    chunks = tables(lengths, 64)
+    results = []
+    for shift in (0, 2, 1):
+        conv = torch.full((tokens, 2 * qk + inner + 4), float("nan"), device=DEV)
+        conv[:, :2 * qk], conv[:, 2 * qk + shift:2 * qk + shift + inner] = rows[:, :2 * qk], rows[:, 2 * qk:]
+        kept, out, raw = state.clone(), torch.full((tokens, inner), float("nan"), device=DEV), torch.full((tokens, inner), float("nan"), device=DEV)
+        scratch = torch.full((ops().delta_chunks_scratch_floats(chunks[0].numel(), heads, dim, vdim),), float("nan"), device=DEV)
+        ops().delta_chunks(conv, 0, qk, 2 * qk + shift, proj, 0, heads, 2 * heads, a_log, dt_bias, norm, Tables(lengths, starts, slots), kept, 0, out,
+                           raw=raw, chunks=chunks, scratch=scratch, heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, eps=1e-6)
+        results.append((out, kept))
+    assert torch.isfinite(results[0][0]).all()
+    for out, kept in results[1:]:
+        assert torch.equal(out, results[0][0]) and torch.equal(kept, results[0][1])
+
+
 @pytest.mark.parametrize("decay", ["mild", "strong", "extreme", "mixed"])
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim,dtype", [(4, 2, 128, 128, "float32"), (2, 1, 64, 64, "float32"), (2, 2, 128, 64, "float32"),
                                                            (1, 1, 64, 128, "float32"), (4, 1, 128, 128, "bfloat16")])
