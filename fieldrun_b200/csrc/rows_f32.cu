@@ -184,15 +184,17 @@ __device__ __forceinline__ void rf_load_x(RowsOfX<R, PAIRS>& to, const float* co
 // A dense product of up to eight rows: one matrix, no lists.  A block an SM for the whole launch takes its share of the weight rows (their
 // number over the blocks, to the row), eight at a time; its warps have a part of the inner size each, always the same one, and add theirs
 // in their order.  A warp's ring runs on from eight rows to the next and begins ahead of the wait for the kernel before: weights are no
-// kernel's result.  The rows of x stay in registers where a warp's part has at most HELD runs of them, else the next run's are asked for
-// ahead.  `tiles`: two where five to eight rows would not fit so; neighbouring blocks then have four rows each and the same weights.
+// kernel's result.  A run's place in the ring is filled again as soon as its lane has read it, ahead of the join.  The rows of x stay in
+// registers where a warp's part has at most HELD runs of them, else the next run's are asked for ahead.  `tiles`: two where seven or eight
+// rows would not fit so; neighbouring blocks then have four rows each and the same weights.
 //
 // Bound by the weights' bytes up to four rows, beyond by the multiply-adds and the joins.  The kernel above, whose blocks begin and end
-// once for 32 KB to 96 KB of weights, and this one in a stream of launches, microseconds for 1, 4 and 8 rows: 8192 x 3072 weights 19.9 25.0
-// 29.4 | 15.8 16.3 20.7 (15.4 at the memory's rate), 3072 x 6144 15.5 17.5 19.8 | 12.3 13.3 19.3, 1024 x 1024 3.3 3.8 4.6 | 1.9 2.1 2.5,
-// 144 x 96 2.0 2.1 2.3 | 1.2 1.3 1.7.  Only with very many weight rows do a single row's joins cost more than that: 65536 x 3072 113 | 118,
-// 200064 x 3072 336 | 352; with two rows 362 | 358, with eight 419 | 377.  Rows two by two (fma.rn.f32x2) pay where the work is large enough
-// for eight rows' multiply-adds to bound it: 200064 x 3072 414 -> 377, 8192 x 3072 21.8 -> 20.7, but 1024 x 1024 2.5 -> 3.2.
+// once for 32 KB to 96 KB of weights, and this one in a stream of launches, microseconds for 1, 4, 6 and 8 rows: 8192 x 3072 weights 19.9 25.0
+// 29.2 29.4 | 16.0 16.5 18.9 21.1 (15.4 at the memory's rate), 3072 x 6144 15.5 17.5 19.7 19.8 | 12.5 13.3 17.2 18.8, 1024 x 1024 3.3 3.8 4.5 4.6
+// | 2.0 2.2 2.5 2.6, 144 x 96 2.0 2.1 2.3 2.3 | 1.2 1.3 1.8 1.6.  Only with very many weight rows do a single row's joins cost more than that: 65536 x
+// 3072 113 | 120, 200064 x 3072 336 | 360; with two rows 362 | 365, with eight 419 | 377.  Rows two by two (fma.rn.f32x2) pay where the work is
+// large enough for six or eight rows' multiply-adds to bound it: 200064 x 3072 414 -> 377 with eight, 8192 x 3072 21.8 -> 20.7, but 1024 x 1024
+// 2.5 -> 3.2.  Six rows as eight: 8192 x 3072 20.6 instead of 18.9, 2048 x 8192 19.9 instead of 15.7.
 #define RD_WARPS 12
 
 template <int R, int HELD>
@@ -227,12 +229,12 @@ __global__ void __launch_bounds__(32 * RD_WARPS, 1) dense_rows_f32_kernel(const 
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
 #pragma unroll
-    for (int s = 0; s < RF_STAGES - 1; ++s) copy(s);
+    for (int s = 0; s < RF_STAGES; ++s) copy(s);
     wait_for_previous_kernel();
     const float* x[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) x[r] = X + (size_t)min(r, rows - 1) * K;
-    constexpr bool PAIRS = R == 8 && HELD == 2;
+    constexpr bool PAIRS = R >= 6 && HELD == 2;
     RowsOfX<R, PAIRS> held[HELD ? HELD : 1];
     auto load_x = [&](RowsOfX<R, PAIRS>& to, int run) { rf_load_x<R, PAIRS>(to, x, begin + 32 * run + lane, end); };
 #pragma unroll
@@ -257,6 +259,7 @@ __global__ void __launch_bounds__(32 * RD_WARPS, 1) dense_rows_f32_kernel(const 
                     for (int r = 0; r < R; ++r) acc[f * R + r] = rf_dot4(wv, xv.one[r], acc[f * R + r]);
                 }
             }
+        copy(stage);                                                     // what this lane copied there it has read
         stage = (stage + 1) % RF_STAGES;
     };
 #pragma unroll 1
@@ -271,15 +274,11 @@ __global__ void __launch_bounds__(32 * RD_WARPS, 1) dense_rows_f32_kernel(const 
         if (HELD) {
 #pragma unroll
             for (int h = 0; h < HELD; ++h)
-                if (h < runs) {
-                    copy((stage + RF_STAGES - 1) % RF_STAGES);
-                    multiply(held[h], h);
-                }
+                if (h < runs) multiply(held[h], h);
         } else {
 #pragma unroll 1
             for (int run = 0; run < runs; ++run) {
                 RowsOfX<R, PAIRS> next;
-                copy((stage + RF_STAGES - 1) % RF_STAGES);
                 load_x(next, run + 1 < runs ? run + 1 : 0);
                 multiply(held[0], run);
                 held[0] = next;
@@ -291,10 +290,23 @@ __global__ void __launch_bounds__(32 * RD_WARPS, 1) dense_rows_f32_kernel(const 
             if (!PAIRS) each[i] = acc[i];
             else if (i % 2 == 0) asm("mov.b64 {%0, %1}, %2;" : "=f"(each[i]), "=f"(each[i + 1]) : "l"(acc2[i / 2]));
         }
-        rf_join<RF_FEATS * R>(each, lane, sums[g & 1][warp]);
+        // (six rows as four and two: the lanes' sums meet by halves)
+        constexpr int HALVES = R == 6 ? 4 : R;
+        float first[RF_FEATS * HALVES], second[R == 6 ? RF_FEATS * 2 : 1];
+#pragma unroll
+        for (int f = 0; f < RF_FEATS; ++f)
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                if (r < HALVES) first[f * HALVES + r] = each[f * R + r];
+                else second[f * 2 + r - HALVES] = each[f * R + r];
+            }
+        rf_join<RF_FEATS * HALVES>(first, lane, sums[g & 1][warp]);
+        if constexpr (R == 6) rf_join<RF_FEATS * 2>(second, lane, sums[g & 1][warp] + RF_FEATS * HALVES);
         __syncthreads();                                                 // the sums of two groups back are read by then
         for (int v = threadIdx.x; v < RF_FEATS * R; v += blockDim.x) {
-            const int r = v % R, f = f_begin + g * RF_FEATS + v / R;
+            const bool last_two = v >= RF_FEATS * HALVES;
+            const int at = last_two ? v - RF_FEATS * HALVES : v, each_row = last_two ? 2 : HALVES;
+            const int r = at % each_row + (last_two ? HALVES : 0), f = f_begin + g * RF_FEATS + at / each_row;
             float sum = 0.f;
             for (int k = 0; k < with_work; ++k) sum += sums[g & 1][k][v];
             if (f < f_end && r < rows) out[(size_t)r * F + f] = sum;
@@ -314,8 +326,9 @@ FRB_API int frb_dense_rows_f32(const float* W, const float* X, float* out, int r
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const int units = K / 4, warps = units >= 32 * RD_WARPS ? RD_WARPS : (units + 31) / 32;
     const int part = (units + 8 * warps - 1) / (8 * warps) * 8, runs = (part + 31) / 32;
-    // (with two tiles everywhere: 8192 x 3072 24.9 instead of 20.7, 2048 x 8192 23.6 instead of 19.9; with one 3072 x 6144 20.9 instead of 19.3)
-    const int tiles = rows > 4 && runs > 2 && runs <= 4 ? 2 : 1, groups = (F + RF_FEATS - 1) / RF_FEATS;
+    // (with two tiles everywhere eight rows of 8192 x 3072 take 24.9 us instead of 20.7, of 2048 x 8192 23.6 instead of 20.8; with one, of 3072 x
+    // 6144 20.9 instead of 18.8, and six rows 18.6 with two instead of 17.2, 20.0 with their four runs in registers)
+    const int tiles = rows > 6 && runs > 2 && runs <= 4 ? 2 : 1, groups = (F + RF_FEATS - 1) / RF_FEATS;
     const int shares = groups < sms / tiles ? groups : sms / tiles, blocks = shares * tiles;
     const size_t smem = (size_t)warps * RF_STAGES * RF_FEATS * 32 * sizeof(float4);
 #define FRB_DENSE(R, HELD)                                                                                                            do {                                                                                                                                  if (smem > 40 * 1024)                                                                                                                 cudaFuncSetAttribute(dense_rows_f32_kernel<R, HELD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                 launch_dependent(dense_rows_f32_kernel<R, HELD>, dim3(blocks), dim3(32 * warps), smem, stream, W, X, out, rows, tiles, F, K);        } while (0)
@@ -329,6 +342,9 @@ FRB_API int frb_dense_rows_f32(const float* W, const float* X, float* out, int r
     if (rows == 1) FRB_DENSE_ROWS(1);
     else if (rows == 2) FRB_DENSE_ROWS(2);
     else if (rows <= 4 || tiles == 2) FRB_DENSE_ROWS(4);
+    else if (rows <= 6 && runs == 1) FRB_DENSE(6, 1);
+    else if (rows <= 6 && runs == 2) FRB_DENSE(6, 2);
+    else if (rows <= 6) FRB_DENSE(6, 0);
     else if (runs == 1) FRB_DENSE(8, 1);
     else if (runs == 2) FRB_DENSE(8, 2);
     else FRB_DENSE(8, 0);

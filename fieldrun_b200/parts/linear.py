@@ -21,7 +21,7 @@ STREAM_ROWS = 8           # up to this many rows a dense product is a stream ove
                           # item's rows of x are as many bytes as its weights and the library's product is faster (measured at
                           # 12 to 32 rows on a B200: 14 to 25 us against 11 for MiniMax-M2's projections)
 ONE_ROW_FEATURES = 65536  # from this many output features on a single float32 row's product is faster by the experts' kernel (rows_f32.cu;
-                          # 3,072 inputs, 32,768 features 60.6 us against 60.0, 65,536 113 against 118)
+                          # 3,072 inputs, 32,768 features 60.6 us against 61.4, 65,536 113 against 120, 200,064 336 against 360)
 STREAM_FEATURES = 65536   # beyond this many output features the library product is at the memory roofline anyway
 
 
