@@ -11,16 +11,18 @@
 // at most one each; within a block the 136 pairs run as the recurrence does, w k_j multiplied by one decay after the other.
 //
 // Everything is float32; the products run on tensor cores with each operand as two TF32 parts (tf32_parts.cuh), over inner
-// sizes of at most 192 entries, added in float32 registers every 16.  Four prompts of 2,048 tokens, 16 heads of 128 x 128: 0.50 ms
-// (about 0.20 + 0.04 + 0.26 for the launches in turn; gla.cu 1.66 ms in segments of 128, whose 500 instructions a warp and token run
-// one after the other).  What bounds them: the instructions around
-// the products (58 and 48 % of the issue slots; a decay's two exponentials and a logarithm, the parts, the block's own pairs),
-// with two blocks an SM to hide the rows' way in; with q, k and v loaded where they are used 0.68 ms.
+// sizes of at most 192 entries, added in float32 registers every 16.  Four prompts of 2,048 tokens, 16 heads of 128 x 128: 0.48 ms
+// (181 + 42 + 254 us for the launches in turn; with the rank's products one token at a time and a division's own branch in each gate 191
+// and 262; gla.cu 1.66 ms in segments of 128, whose 500 instructions a warp and token run one after the other).  What bounds them: the
+// instructions around the products (58 and 48 % of the issue slots; a decay's two exponentials and a logarithm, the parts, the block's own
+// pairs), with two blocks an SM to hide the rows' way in; with q, k and v loaded where they are used 0.68 ms.
+#include "silu.cuh"
 #include "tf32_parts.cuh"
 
 #define GC_TOKENS 64
 #define GC_BLOCK 16
 #define GC_THREADS 256
+#define GC_LA1 (GC_TOKENS + 4)      // tokens of one of the rank's entries in shared memory
 
 struct GlaChunks {
     const float* proj;       // [T, P]: q | k | v | g | a1 at the offsets below
@@ -49,6 +51,14 @@ __device__ __forceinline__ void gc_copy_rows(float* to, int ld, const float* fro
     }
 }
 
+__device__ __forceinline__ uint64_t gc_pair(float lo, float hi) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+
+__device__ __forceinline__ void gc_fma_pair(uint64_t a, uint64_t b, uint64_t& c) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b)); }
+
 __device__ __forceinline__ float gc_log_sigmoid(float z) { return fminf(z, 0.f) - log1pf(expf(-fabsf(z))); }
 
 // Launch 1.  grid (chunk, head).  A thread has one key channel and 64 DIM / 256 neighbouring tokens for what is made channel by
@@ -61,8 +71,8 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_states_kernel(GlaChun
     const int rank = p.rank, la2 = rank + 4;
     float* k_s = (float*)gc_smem;                   // [GC_TOKENS][LK]
     float* v_s = k_s + GC_TOKENS * LK;              // [GC_TOKENS][LV]
-    float* a1_s = v_s + GC_TOKENS * LV;             // [GC_TOKENS][rank]
-    float* a2_s = a1_s + GC_TOKENS * rank;          // [DIM][la2]
+    float* a1_s = v_s + GC_TOKENS * LV;             // [rank][GC_LA1]
+    float* a2_s = a1_s + GC_LA1 * rank;             // [DIM][la2]
     const int item = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int b = p.chunk_seq[item], count = p.chunk_end[item] - p.chunk_begin[item];
     const size_t row0 = (size_t)p.cu_q_len[b] + p.chunk_begin[item];
@@ -70,7 +80,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_states_kernel(GlaChun
 
     const WT* a2 = (const WT*)p.a2 + (size_t)h * DIM * rank;
     for (int r = lane; r < rank; r += 32) {
-        for (int t = warp; t < GC_TOKENS; t += GC_THREADS / 32) a1_s[t * rank + r] = t < count ? rows[(size_t)t * p.P + p.off_a + r] : 0.f;
+        for (int t = warp; t < GC_TOKENS; t += GC_THREADS / 32) a1_s[r * GC_LA1 + t] = t < count ? rows[(size_t)t * p.P + p.off_a + r] : 0.f;
 #pragma unroll 8
         for (int c = warp; c < DIM; c += GC_THREADS / 32) a2_s[c * la2 + r] = to_f32<WT>(a2[c * rank + r]);
     }
@@ -85,21 +95,28 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_states_kernel(GlaChun
     float* alpha = p.alpha + (row0 * p.heads + h) * DIM + d;
 #pragma unroll
     for (int tg = 0; tg < TOKENS; tg += 8) {
-        float z[8];
+        // two tokens at a time (the same multiply-adds, half the instructions)
+        uint64_t pairs[4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) z[i] = bias;
+        for (int i = 0; i < 4; ++i) pairs[i] = gc_pair(bias, bias);
 #pragma unroll 1
         for (int r = 0; r < rank; r += 4) {
             const float4 w = *(const float4*)(a2_s + d * la2 + r);
+            const float each[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float4 x = *(const float4*)(a1_s + (t0 + tg + i) * rank + r);
-                z[i] = fmaf(w.x, x.x, z[i]);
-                z[i] = fmaf(w.y, x.y, z[i]);
-                z[i] = fmaf(w.z, x.z, z[i]);
-                z[i] = fmaf(w.w, x.w, z[i]);
+            for (int q = 0; q < 4; ++q) {
+                const ulonglong2* x = (const ulonglong2*)(a1_s + (r + q) * GC_LA1 + t0 + tg);
+                const ulonglong2 x0 = x[0], x1 = x[1];
+                const uint64_t ww = gc_pair(each[q], each[q]);
+                gc_fma_pair(ww, x0.x, pairs[0]);
+                gc_fma_pair(ww, x0.y, pairs[1]);
+                gc_fma_pair(ww, x1.x, pairs[2]);
+                gc_fma_pair(ww, x1.y, pairs[3]);
             }
         }
+        float z[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) asm("mov.b64 {%0, %1}, %2;" : "=f"(z[2 * i]), "=f"(z[2 * i + 1]) : "l"(pairs[i]));
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int t = t0 + tg + i;
@@ -445,12 +462,19 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_outputs_kernel(GlaChu
                 const float rinv = 1.0f / sqrtf(ss / (float)VDIM + p.eps);
                 const float* gate = rows + (size_t)t * p.P + p.off_g + h * VDIM;
                 OutT* out = (OutT*)p.out + ((row0 + t) * p.heads + h) * VDIM;
+                float gates[8];
+#pragma unroll
+                for (int n = 0; n < 4; ++n) {
+                    const float2 g = *(const float2*)(gate + v0 + 8 * n + 2 * (lane & 3));
+                    gates[2 * n] = g.x;
+                    gates[2 * n + 1] = g.y;
+                }
+                silu_of(gates);
 #pragma unroll
                 for (int n = 0; n < 4; ++n) {
                     const int v = v0 + 8 * n + 2 * (lane & 3);
-                    const float2 g = *(const float2*)(gate + v);
-                    out[v] = from_f32<OutT>(acc[m][n][2 * half] * rinv * p.norm_w[v] * (g.x / (1.0f + expf(-g.x))));
-                    out[v + 1] = from_f32<OutT>(acc[m][n][2 * half + 1] * rinv * p.norm_w[v + 1] * (g.y / (1.0f + expf(-g.y))));
+                    out[v] = from_f32<OutT>(acc[m][n][2 * half] * rinv * p.norm_w[v] * gates[2 * n]);
+                    out[v + 1] = from_f32<OutT>(acc[m][n][2 * half + 1] * rinv * p.norm_w[v + 1] * gates[2 * n + 1]);
                 }
             }
 }
@@ -480,7 +504,7 @@ FRB_API int frb_gla_chunks(const float* proj, int P, int off_q, int off_k, int o
     p.off_q = off_q; p.off_k = off_k; p.off_v = off_v; p.off_g = off_g; p.off_a = off_a; p.heads = heads; p.rank = rank;
 #define FRB_GLA_CHUNKS(DIM, VDIM)                                                                                                    \
     do {                                                                                                                             \
-        const size_t one = (size_t)(GC_TOKENS * (DIM + 4 + VDIM + 4 + rank) + DIM * (rank + 4)) * sizeof(float);                     \
+        const size_t one = (size_t)(GC_TOKENS * (DIM + 4 + VDIM + 4) + GC_LA1 * rank + DIM * (rank + 4)) * sizeof(float);                     \
         const size_t slabs = 2 * 32 * (VDIM + 4), rows_q = GC_TOKENS * (DIM + 8);                                                    \
         const size_t three = (rows_q + (rows_q > slabs ? rows_q : slabs) + slabs) * sizeof(float);                                   \
         cudaFuncSetAttribute(gla_chunk_states_kernel<DIM, VDIM, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)one);          \
