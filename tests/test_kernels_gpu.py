@@ -183,6 +183,12 @@ def test_attention_over_scrambled_pages(dtype, heads, kv_heads, head_dim, window
     close(f64(out), ref, TOL[dtype], "attention")
 
 
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(4, 1, 1), (3, 3, 31), (4, 2, 33), (2, 1, 64), (2, 2, 65), (2, 1, 129), (1, 1, 256)])
+def test_attention_of_value_heads_of_any_size(heads, kv_heads, head_dim):
+    """The fewest and most entries of the output that a lane has in each form of the kernel."""
+    test_attention_over_scrambled_pages("float32", heads, kv_heads, head_dim, None)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_attention_finds_one_far_key_and_respects_the_windows_edge(dtype):
     """All keys are tiny except one far back whose score stands out: the output must be that key's value.
