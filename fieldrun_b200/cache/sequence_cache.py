@@ -181,11 +181,14 @@ class _Group:
         self.dirty.clear()
         self.fresh.clear()
 
-
     def sync_many(self) -> None:
         """The same with one copy to the device for all of it: the changed places of the table, the pages to be cleared, and the
         places' entries, two in each of the copy's integers.  (A copy for each sequence was a fifth of a short prompt step's time
-        on the host, with four sequences 200 us of 1,100.)"""
+        on the host, with four sequences 200 us of 1,100.)
+
+        A kernel writes the table here, and the kernels of a step read it ahead of their wait for the kernel before them.  So another
+        operation of the ordinary kind follows, which begins when the table is complete: the clearing of the pages, or a copy of
+        eight bytes."""
         width = self.table.shape[1]
         places = np.concatenate([np.arange(slot * width + lo, slot * width + hi) for slot, lo, hi in self.dirty] or [np.zeros(0, np.int64)])
         n, pages = len(places), len(self.fresh)
@@ -198,6 +201,8 @@ class _Group:
         if pages:
             self.keys.index_fill_(1, dev[n:n + pages], 0)
             self.values.index_fill_(1, dev[n:n + pages], 0)
+        else:
+            dev[:1].copy_(dev[1:2])
 
 
 class SequenceCache:

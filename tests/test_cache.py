@@ -164,3 +164,25 @@ def test_the_tables_of_many_sequences_reach_the_device_whole():
         assert cleared == partial and ((group.keys == 0) | (group.keys == 3.0)).all()
         assert np.array_equal(group.table_dev.numpy(), group.table)
         cache.end_step(held, new)
+
+
+def test_the_table_is_complete_when_a_step_begins():
+    """A step's kernels may read the page table while the operation before them still runs: the last one that a change of many places leaves
+    on the stream is not the one that writes the table."""
+    import torch
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Writes(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            if func._schema.name.endswith("_"):
+                written.append(args[0].untyped_storage().data_ptr())
+            return func(*args, **(kwargs or {}))
+
+    for lengths in ([64, 128, 192], [65, 128, 192], [10, 20, 30, 40]):
+        cache = SequenceCache([CacheNeed(1, 4, None)], max_tokens=64 * 40, num_slots=6, dtype=torch.float32, device="cpu")
+        slots, written = [cache.alloc() for _ in lengths], []
+        with Writes():
+            cache.begin_step(slots, lengths)
+        table = cache.groups[0].table_dev
+        assert table.untyped_storage().data_ptr() in written[:-1] and written[-1] != table.untyped_storage().data_ptr()
+        assert np.array_equal(table.numpy(), cache.groups[0].table)
