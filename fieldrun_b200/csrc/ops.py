@@ -52,7 +52,7 @@ _SIGNATURES = {
     "frb_expert_combine": "pppiiip",
     "frb_expert_gemm_generic": "ppipppppipiiiif",
     "frb_rows_f32": "pppppppipiiif",
-    "frb_dense_rows_f32": "pppiii",
+    "frb_dense_rows_f32": "pppiiii",
     "frb_weight_scales": "ppli",
     "frb_split_rows": "pppplii" "f",
     "frb_products_f32": "ppippl" "ppif" "ppppip" "iipp",
@@ -1076,14 +1076,15 @@ def rows_f32(w: torch.Tensor, x: torch.Tensor, x_rows: Optional[torch.Tensor], t
           _ptr(out), feats, w.shape[2], int(paired), float(gate_limit))
 
 
-def dense_rows_f32(w: torch.Tensor, x: torch.Tensor, out: torch.Tensor) -> None:
+def dense_rows_f32(w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, *, weights_final: bool = False) -> None:
     """out [n, F] = x [n, K] w[F, K]^T in float32 for up to ``ROWS_F32_TILE`` rows, as a stream over the weights (rows_f32.cu); inner
-    sizes in steps of 4."""
+    sizes in steps of 4.  ``weights_final``: ``w`` was complete before the kernel before this one in the stream began, so it may be read
+    while that one still runs."""
     for t, what in ((w, "weights"), (x, "their input"), (out, "their output")):
         _want(t, torch.float32, what)
     if w.dim() != 2 or x.dim() != 2 or x.shape[1] != w.shape[1] or out.shape != (x.shape[0], w.shape[0]):
         raise KernelError(f"{list(w.shape)} weights with rows {list(x.shape)} into {list(out.shape)}")
-    _call("frb_dense_rows_f32", _ptr(w), _ptr(x), _ptr(out), x.shape[0], w.shape[0], w.shape[1])
+    _call("frb_dense_rows_f32", _ptr(w), _ptr(x), _ptr(out), x.shape[0], w.shape[0], w.shape[1], int(weights_final))
 
 
 PRODUCTS_F32_TILE = 160    # rows of a tile of products_f32
@@ -1462,7 +1463,7 @@ def weight_stream(w: torch.Tensor, x: torch.Tensor, x_rows: Optional[torch.Tenso
                   tile_rows: int, out: torch.Tensor, *, paired: bool, lists_final: bool = False,
                   blocks: Optional[int] = None, ring_kb: Optional[int] = None, pieces: int = 0, gate_limit: float = 0.0) -> None:
     """Products of a few rows with bfloat16 weights [E, F or 2F, K] as one stream over the weights per SM: TMA into
-    a ring of stages, ``mma.sync`` from shared memory (tiles of 8, 16 or 32 rows).  ``lists_final``: the lists of
+    a ring of stages, ``mma.sync`` from shared memory (tiles of 8, 16 or 32 rows).  ``lists_final``: weights and lists of
     tiles were complete before the kernel before this one in the stream began (a dense layer's fixed lists; the
     experts' second product), so the weights may be asked for before that kernel has ended."""
     _want(w, torch.bfloat16, "streamed weights")

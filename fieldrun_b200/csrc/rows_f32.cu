@@ -183,8 +183,8 @@ __device__ __forceinline__ void rf_load_x(RowsOfX<R, PAIRS>& to, const float* co
 
 // A dense product of up to eight rows: one matrix, no lists.  A block an SM for the whole launch takes its share of the weight rows (their
 // number over the blocks, to the row), eight at a time; its warps have a part of the inner size each, always the same one, and add theirs
-// in their order.  A warp's ring runs on from eight rows to the next and begins ahead of the wait for the kernel before: weights are no
-// kernel's result.  A run's place in the ring is filled again as soon as its lane has read it, ahead of the join.  The rows of x stay in
+// in their order.  A warp's ring runs on from eight rows to the next and, where the weights are complete, begins ahead of the wait for the
+// kernel before.  A run's place in the ring is filled again as soon as its lane has read it, ahead of the join.  The rows of x stay in
 // registers where a warp's part has at most HELD runs of them, else the next run's are asked for ahead.  `tiles`: two where seven or eight
 // rows would not fit so; neighbouring blocks then have four rows each and the same weights.
 //
@@ -198,11 +198,10 @@ __device__ __forceinline__ void rf_load_x(RowsOfX<R, PAIRS>& to, const float* co
 #define RD_WARPS 12
 
 template <int R, int HELD>
-__global__ void __launch_bounds__(32 * RD_WARPS, 1) dense_rows_f32_kernel(const float* __restrict__ W, const float* X, float* __restrict__ out,
-                                                                          int all_rows, int tiles, int F, int K) {
+__global__ void __launch_bounds__(32 * RD_WARPS, 1) dense_rows_f32_kernel(const float* W, const float* X, float* __restrict__ out, int all_rows,
+                                                                          int tiles, int F, int K, int weights_final) {
     extern __shared__ float4 rf_smem[];
     __shared__ float sums[2][RD_WARPS][RF_FEATS * R];
-    let_next_kernel_start();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int share = blockIdx.x / tiles, shares = gridDim.x / tiles, tile = blockIdx.x - share * tiles;
     const int row0 = tile * R, rows = min(all_rows - row0, R);
@@ -228,9 +227,11 @@ __global__ void __launch_bounds__(32 * RD_WARPS, 1) dense_rows_f32_kernel(const 
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    if (!weights_final) wait_for_previous_kernel();
 #pragma unroll
     for (int s = 0; s < RF_STAGES; ++s) copy(s);
     wait_for_previous_kernel();
+    let_next_kernel_start();                          // not before: the next kernel may read, ahead of its wait, what is complete by now
     const float* x[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) x[r] = X + (size_t)min(r, rows - 1) * K;
@@ -315,8 +316,9 @@ __global__ void __launch_bounds__(32 * RD_WARPS, 1) dense_rows_f32_kernel(const 
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-// out [rows, F] = X [rows, K] W^T, W [F][K], all float32; up to eight rows.
-FRB_API int frb_dense_rows_f32(const float* W, const float* X, float* out, int rows, int F, int K, cudaStream_t stream) {
+// out [rows, F] = X [rows, K] W^T, W [F][K], all float32; up to eight rows.  weights_final: W was complete before the kernel before this one
+// began, and may be read while that one still runs.
+FRB_API int frb_dense_rows_f32(const float* W, const float* X, float* out, int rows, int F, int K, int weights_final, cudaStream_t stream) {
     if (rows == 0 || F == 0) return 0;
     FRB_CHECK_ARG(rows > 0 && rows <= RF_ROWS, "dense float32 rows: %d rows are outside 1..%d", rows, RF_ROWS);
     FRB_CHECK_ARG(K > 0 && K % 4 == 0, "dense float32 rows: an inner size of %d is not a multiple of 4", K);
@@ -331,7 +333,7 @@ FRB_API int frb_dense_rows_f32(const float* W, const float* X, float* out, int r
     const int tiles = rows > 6 && runs > 2 && runs <= 4 ? 2 : 1, groups = (F + RF_FEATS - 1) / RF_FEATS;
     const int shares = groups < sms / tiles ? groups : sms / tiles, blocks = shares * tiles;
     const size_t smem = (size_t)warps * RF_STAGES * RF_FEATS * 32 * sizeof(float4);
-#define FRB_DENSE(R, HELD)                                                                                                            do {                                                                                                                                  if (smem > 40 * 1024)                                                                                                                 cudaFuncSetAttribute(dense_rows_f32_kernel<R, HELD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                 launch_dependent(dense_rows_f32_kernel<R, HELD>, dim3(blocks), dim3(32 * warps), smem, stream, W, X, out, rows, tiles, F, K);        } while (0)
+#define FRB_DENSE(R, HELD)                                                                                                            do {                                                                                                                                  if (smem > 40 * 1024)                                                                                                                 cudaFuncSetAttribute(dense_rows_f32_kernel<R, HELD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                 launch_dependent(dense_rows_f32_kernel<R, HELD>, dim3(blocks), dim3(32 * warps), smem, stream, W, X, out, rows, tiles, F, K, weights_final); } while (0)
 #define FRB_DENSE_ROWS(R)                                                                                                         \
     do {                                                                                                                          \
         if (runs == 1) FRB_DENSE(R, 1);                                                                                           \

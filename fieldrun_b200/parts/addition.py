@@ -16,7 +16,7 @@ import torch
 from ..csrc import ops
 from ..weights.loader import MATRIX, VECTOR, TensorNeed, TensorSource
 from .base import Addition, as_tensor, register_part, shared_fetch
-from .linear import linear
+from .linear import part_linear
 
 
 class TokenSideInput(Addition):
@@ -66,8 +66,8 @@ class TokenSideInput(Addition):
             act = ctx.buffer("side.act", (rows, self.width), self.dtype)
             ops.add_typed_copy(x, delta, act)                      # the block's update is added on the way
         gated = ctx.buffer("side.gated", (rows, self.dim), self.dtype)
-        ops.token_side_gate(linear(act, self.w_gate), ctx.step_tokens, self.table, self.index * self.dim, gated)
-        ops.add_rms_normed(x, linear(gated, self.w_proj), self.norm, self.eps)
+        ops.token_side_gate(part_linear(act, self.w_gate), ctx.step_tokens, self.table, self.index * self.dim, gated)
+        ops.add_rms_normed(x, part_linear(gated, self.w_proj), self.norm, self.eps)
         return x, None
 
 

@@ -46,7 +46,7 @@ from ..cache import CacheNeed, LineView
 from ..csrc import ops
 from ..weights.loader import MATRIX, VECTOR, TensorNeed, TensorSource
 from .base import BiasedRows, Mixer, build_position, register_part
-from .linear import linear
+from .linear import part_linear
 
 
 TC_ATTENTION_MIN_QUERIES = 64       # a step whose longest run of new tokens is shorter uses tiles of 16 queries
@@ -235,7 +235,7 @@ class GQAAttention(Mixer):
         tokens = act.shape[0]
         if self.shares_kv and writes_cache:
             raise ValueError("an attention layer without keys and values of its own was asked to write a cache line")
-        qkv = linear(act, self.w_qkv)                                        # float32 [T, q + k + v] (or [T, q + k], [T, q])
+        qkv = part_linear(act, self.w_qkv)                                   # float32 [T, q + k + v] (or [T, q + k], [T, q])
         q = ctx.buffer("attention.q", (tokens, self.q_width), self.dtype)
         rotary_dim = self.position.rotary_dim if self.position is not None else 0
         ops.qkv_prepare(qkv, self.q_norm, self.k_norm, self.qk_norm_eps, self.cos, self.sin, ctx.tok_pos, ctx.tok_slot,
@@ -249,9 +249,9 @@ class GQAAttention(Mixer):
                         bias=self.b_qkv, v_dim=self.value_dim, q_temp=self.q_temp,
                         values_from_keys=self.values_from_keys and not self.shares_kv)
         out = ctx.buffer("attention.out", (tokens, self.out_width), self.dtype)
-        gate = linear(act, self.w_gate) if self.has_head_gate else None          # float32 [T, heads], before the sigmoid
+        gate = part_linear(act, self.w_gate) if self.has_head_gate else None     # float32 [T, heads], before the sigmoid
         self.attend(ctx, q, line, out, gate)
-        update = linear(out, self.w_o)
+        update = part_linear(out, self.w_o)
         return BiasedRows(update, self.b_o) if self.b_o is not None else update
 
     def attend(self, ctx, q: torch.Tensor, line: LineView, out: torch.Tensor, gate: Optional[torch.Tensor] = None) -> None:

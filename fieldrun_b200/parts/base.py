@@ -70,7 +70,9 @@ class Part:
         return self.tensor_needs()
 
     def load(self, source: TensorSource) -> None:
-        pass
+        """Fetch the part's tensors.  A step's kernels read them ahead of their wait for the kernel before, so the last kernel that
+        writes them is not the one right before a ``forward``: the copy that every new :class:`StepContext` makes to the device
+        comes between."""
 
     def children(self) -> list["Part"]:
         """Parts that this part is put together from (a mixer made of two mixers); the model counts their tensors,

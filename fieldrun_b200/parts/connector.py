@@ -14,7 +14,7 @@ import torch
 from ..csrc import ops
 from ..weights.loader import MATRIX, VECTOR, TensorNeed, TensorSource
 from .base import BiasedRows, Connector, UpdateSum, as_tensor, register_part
-from .linear import linear
+from .linear import part_linear
 
 
 class StreamReentry(Connector):
@@ -39,7 +39,7 @@ class StreamReentry(Connector):
             raise ValueError(f"pass {index} of {self.passes}")
         both = ctx.buffer("reentry.rows", (x.shape[0], 2 * self.width), self.dtype)
         ops.concat_rows(x, first, both, delta=as_tensor(ctx, pending))      # the update a block left is added on the way
-        ops.add_row_vector(linear(both, self.weight), self.step[index], x)
+        ops.add_row_vector(part_linear(both, self.weight), self.step[index], x)
         return x
 
 

@@ -18,7 +18,7 @@ from ..cache import CacheNeed
 from ..csrc import ops
 from ..weights.loader import MATRIX, TensorNeed, TensorSource
 from .base import Part, register_part
-from .linear import linear
+from .linear import part_linear
 from .norm import LayerNorm
 
 
@@ -93,7 +93,7 @@ class VocabHead(Part):
         self.weight = shared if shared is not None else source.fetch(self.tensor_needs()[0])
 
     def forward(self, ctx, rows: torch.Tensor) -> torch.Tensor:
-        logits = linear(rows, self.weight)
+        logits = part_linear(rows, self.weight)
         if self.softcap is not None or self.scale != 1.0:
             ops.softcap(logits, self.softcap, self.scale)
         return logits

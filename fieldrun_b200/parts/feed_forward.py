@@ -29,7 +29,7 @@ import torch
 from ..csrc import ops
 from ..weights.loader import MATRIX, VECTOR, TensorNeed, TensorSource
 from .base import FeedForward, UpdateSum, WeightedRows, register_part
-from .linear import STREAM_ROWS, linear, one_tile
+from .linear import STREAM_ROWS, one_tile, part_linear
 
 TILE_ROWS = 32        # rows of one expert that a block of the expert kernels takes
 # Above this many rows per expert (on average) a step's expert products run on tcgen05: tiles of 32 rows and more
@@ -206,14 +206,14 @@ class RoutedExperts(FeedForward):
             if self.shared_tc and rows >= FUSED_ACTIVATION_ROWS and not ctx.is_decode:
                 tile_expert, tile_row0, num_tiles, offsets, count, tile_rows = self.tiles.of(ctx, rows)
                 ops.expert_gemm_tc(pair, act, tile_expert, tile_row0, num_tiles, offsets, count, tile_rows, hidden, paired=True)
-                return linear(hidden, self.w_shared_down)
+                return part_linear(hidden, self.w_shared_down)
             if rows <= STREAM_ROWS and ops.weight_stream_takes(self.shared_width, self.hidden_size, paired=True):
                 tile_expert, tile_row0, num_tiles, offsets = one_tile(act.device, rows)
                 ops.weight_stream(pair, act, None, tile_expert, tile_row0, num_tiles, offsets, 1, 8, hidden, paired=True, lists_final=True)
-                return linear(hidden, self.w_shared_down)
-        both = linear(act, self.w_shared_in)
+                return part_linear(hidden, self.w_shared_down)
+        both = part_linear(act, self.w_shared_in)
         ops.gated_unit(both, hidden, "silu", row_gate=2 * self.shared_width if self.shared_gate else None)
-        return linear(hidden, self.w_shared_down)
+        return part_linear(hidden, self.w_shared_down)
 
     # -- one step --------------------------------------------------------------------------------------
     def logits(self, ctx, act32: torch.Tensor) -> torch.Tensor:
@@ -226,7 +226,7 @@ class RoutedExperts(FeedForward):
             return out
         # a model in bfloat16 keeps the library's product: a router has few features, so the split product's tiles leave most of the
         # device idle (2,048 rows of 256 features: 94 us, 110 split)
-        return linear(act32, self.router, split=self.dtype == torch.float32)
+        return part_linear(act32, self.router, split=self.dtype == torch.float32)
 
     def route(self, ctx, act32: torch.Tensor):
         tokens = act32.shape[0]
@@ -444,10 +444,10 @@ class DenseGatedUnit(FeedForward):
         self.w_down = down
 
     def forward(self, ctx, act, act32):
-        both = linear(act, self.w_gate_up)                         # float32 [T, 2I]
+        both = part_linear(act, self.w_gate_up)                    # float32 [T, 2I]
         hidden = ctx.buffer("dense.hidden", (act.shape[0], self.width), self.dtype)
         ops.gated_unit(both, hidden, self.activation)
-        return linear(hidden, self.w_down)
+        return part_linear(hidden, self.w_down)
 
 
 class DenseUnit(FeedForward):
@@ -498,7 +498,7 @@ class DenseUnit(FeedForward):
         rows = act.shape[0]
         hidden = ctx.buffer("dense.hidden", (rows, self.width), self.dtype)
         if self.normed_powers:
-            ops.poly_norm(linear(act, self.w_up), self.coefficients, self.norm_eps, hidden)
+            ops.poly_norm(part_linear(act, self.w_up), self.coefficients, self.norm_eps, hidden)
         elif (self.dtype == torch.bfloat16 and rows >= FUSED_ACTIVATION_ROWS and not ctx.is_decode and self.width % 128 == 0
                 and self.hidden_size % 64 == 0):
             # a prompt's rows: product and activation in one kernel on tcgen05, the result rounded once to bfloat16
@@ -506,9 +506,9 @@ class DenseUnit(FeedForward):
             ops.expert_gemm_tc(self.w_up.view(1, self.width, self.hidden_size), act, tile_expert, tile_row0, num_tiles, offsets,
                                count, tile_rows, hidden, paired=False, activation=self.activation)
         else:
-            up = linear(act, self.w_up)                            # float32 [T, I]
+            up = part_linear(act, self.w_up)                       # float32 [T, I]
             ops.unary_unit(up, hidden, self.activation)
-        return linear(hidden, self.w_down)
+        return part_linear(hidden, self.w_down)
 
 
 register_part("feed_forward", "routed_experts", RoutedExperts, replace=True)

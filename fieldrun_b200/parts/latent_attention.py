@@ -28,7 +28,7 @@ from ..cache import CacheNeed, LineView
 from ..csrc import ops
 from ..weights.loader import MATRIX, VECTOR, TensorNeed, TensorSource
 from .base import Mixer, build_position, register_part
-from .linear import linear
+from .linear import part_linear
 
 
 def batched_product(a: torch.Tensor, b: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
@@ -138,12 +138,12 @@ class LatentAttention(Mixer):
         if not self.shares_kv and not writes_cache:
             raise ValueError("a layer with latents of its own must write its cache line")
         interleaved = bool(self.position.interleaved) if self.position is not None else False
-        down = linear(act, self.w_down)                  # float32 [T, q_rank (+ kv_rank + rot_dim) (+ gate)]
+        down = part_linear(act, self.w_down)             # float32 [T, q_rank (+ kv_rank + rot_dim) (+ gate)]
         latent_q = ctx.buffer("latent.cq", (tokens, self.q_rank), self.dtype)
         ops.latent_prepare(down, self.q_norm, self.kv_norm, self.norm_eps, self.cos, self.sin, ctx.tok_pos, ctx.tok_slot,
                            line.page_table, latent_q, line.keys if writes_cache else None, q_rank=self.q_rank,
                            kv_rank=self.kv_rank, rot_dim=self.rot_dim, rotary_dims=self.rotary_dims, interleaved=interleaved)
-        q = linear(latent_q, self.w_uq)                  # float32 [T, heads * (head_dim + rot_dim)]
+        q = part_linear(latent_q, self.w_uq)             # float32 [T, heads * (head_dim + rot_dim)]
         q_plain = ctx.buffer("latent.q_plain", (self.num_heads, tokens, self.head_dim), self.dtype)
         q_rot = ctx.buffer("latent.q_rot", (tokens, self.num_heads, self.rot_dim), self.dtype)
         ops.latent_queries(q, q_plain, q_rot, self.cos, self.sin, ctx.tok_pos, heads=self.num_heads, dim=self.head_dim,
@@ -161,7 +161,7 @@ class LatentAttention(Mixer):
         else:
             gate_column = self.q_rank + (0 if self.shares_kv else self.key_width)
             ops.latent_gate(o, down, gate_column, self.gate == "head", out, heads=self.num_heads, vdim=self.value_dim)
-        return linear(out, self.w_o)
+        return part_linear(out, self.w_o)
 
     def attend(self, ctx, q_lat: torch.Tensor, q_rot: torch.Tensor, line: LineView, o_lat: torch.Tensor) -> None:
         """bfloat16: prompts over key rows in pieces of 64 entries go to the tcgen05 kernel; other key rows that the

@@ -10,6 +10,7 @@ is checked at every call.
 """
 from __future__ import annotations
 
+from functools import partial
 from typing import Optional
 
 import torch
@@ -87,10 +88,11 @@ def float32_kernels_read(rows: torch.Tensor, weight: torch.Tensor, out: Optional
 
 
 def linear(rows: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None, rounded: bool = False,
-           split: bool = True) -> torch.Tensor:
+           split: bool = True, weight_final: bool = False) -> torch.Tensor:
     """rows [T, in] @ weight[out, in]^T -> float32 [T, out]; ``split``: whether a large float32 product may run as split products
     on the tensor cores; with ``rounded`` (bfloat16 rows only) the float32 sums rounded once
-    to bfloat16, for a reader that takes its operands in that type anyway."""
+    to bfloat16, for a reader that takes its operands in that type anyway.  ``weight_final``: the weight was complete before the
+    kernel before this product in the stream began, so that a product of few rows may read it while that one still runs."""
     if rounded:
         if rows.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16 or not rows.is_cuda or out is not None:
             raise RuntimeError(f"a rounded matrix product of {rows.dtype} rows with a {weight.dtype} weight on {rows.device}")
@@ -113,7 +115,7 @@ def linear(rows: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor]
                     tile_expert, tile_row0, num_tiles, offsets = one_tile(rows.device, 1)
                     ops.rows_f32(weight.unsqueeze(0), rows, None, tile_expert, tile_row0, num_tiles, offsets, 1, result, paired=False)
                 else:
-                    ops.dense_rows_f32(weight, rows, result)
+                    ops.dense_rows_f32(weight, rows, result, weights_final=weight_final)
             else:
                 parts = torch.empty((2, *rows.shape), dtype=torch.float16, device=rows.device)
                 scale = torch.empty(rows.shape[0], dtype=torch.float32, device=rows.device)
@@ -133,9 +135,9 @@ def linear(rows: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor]
         tile_expert, tile_row0, num_tiles, offsets = one_tile(rows.device, count)
         result = out if out is not None else torch.empty((count, features), dtype=torch.float32, device=rows.device)
         if ops.weight_stream_takes(features, inner, paired=False):
-            # the lists of this one tile never change, so the weights may be on their way before the rows are ready
+            # the lists of this one tile never change, so a weight that does not either may be on its way before the rows are ready
             ops.weight_stream(weight.view(1, features, inner), rows, None, tile_expert, tile_row0, num_tiles, offsets, 1,
-                              tile_rows, result, paired=False, lists_final=True)
+                              tile_rows, result, paired=False, lists_final=weight_final)
         else:
             ops.expert_gemm_mma(weight.view(1, features, inner), rows, None, tile_expert, tile_row0, num_tiles, offsets, 1,
                                 tile_rows, result, paired=False, **ops.stream_shape(1, features, inner, tile_rows))
@@ -146,3 +148,7 @@ def linear(rows: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor]
         return result
     out.copy_(result)
     return out
+
+
+# The product with a part's own weight, which a step finds as it was loaded (see Part.load).
+part_linear = partial(linear, weight_final=True)

@@ -23,7 +23,7 @@ from ..cache import CacheNeed, LineView
 from ..csrc import ops
 from ..weights.loader import MATRIX, VECTOR, TensorNeed, TensorSource
 from .base import Mixer, register_part
-from .linear import linear
+from .linear import part_linear
 
 
 # From this many tokens of the longest prompt on a step may run in chunks as matrix products (gla_chunks.cu).  Measured on a B200, the
@@ -108,7 +108,7 @@ class GatedLinearAttention(Mixer):
     def forward(self, ctx, act: torch.Tensor, line: LineView, writes_cache: bool) -> torch.Tensor:
         if not writes_cache:
             raise ValueError("a recurrent layer cannot read another layer's state: it has to write its own")
-        proj = linear(act, self.w_in)                                       # float32 [T, 2 qk + 2 v + rank]
+        proj = part_linear(act, self.w_in)                                  # float32 [T, 2 qk + 2 v + rank]
         out = ctx.buffer("linear_attention.out", (act.shape[0], self.v_width), self.dtype)
         sizes = dict(heads=self.num_heads, dim=self.head_dim, vdim=self.value_dim, tau=self.tau, q_scale=self.q_scale, eps=self.norm_eps)
         args = (proj, self.offsets, self.w_decay, self.decay_bias, self.norm_weight, line.state, ctx.seq_slot, ctx.seq_start, ctx.cu_q_len, out)
@@ -116,7 +116,7 @@ class GatedLinearAttention(Mixer):
             chunks = ctx.token_chunks(ops.GLA_CHUNK_TOKENS)
             floats = ops.gla_chunks_scratch_floats(chunks[0].numel(), act.shape[0], self.num_heads, self.head_dim, self.value_dim)
             ops.gla_chunks(*args, chunks=chunks, scratch=ctx.buffer("linear_attention.segments", (floats,), torch.float32), **sizes)
-            return linear(out, self.w_o)
+            return part_linear(out, self.w_o)
         segments = scratch = None
         # a long prompt whose heads give the device fewer than two blocks an SM
         if (not ctx.is_decode and ctx.max_q_len >= 2 * SEGMENT_TOKENS
@@ -125,7 +125,7 @@ class GatedLinearAttention(Mixer):
             floats = ops.gla_scratch_floats(segments[0].numel(), self.num_heads, self.head_dim, self.value_dim)
             scratch = ctx.buffer("linear_attention.segments", (floats,), torch.float32)
         ops.gla_scan(*args, segments=segments, scratch=scratch, **sizes)
-        return linear(out, self.w_o)
+        return part_linear(out, self.w_o)
 
 
 register_part("mixer", "gated_linear_attention", GatedLinearAttention, replace=True)

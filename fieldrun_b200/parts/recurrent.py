@@ -32,7 +32,7 @@ from ..cache import CacheNeed, LineView
 from ..csrc import ops
 from ..weights.loader import MATRIX, VECTOR, TensorNeed, TensorSource
 from .base import Mixer, register_part
-from .linear import linear
+from .linear import part_linear
 
 
 # From this many tokens of the longest prompt on a step's recurrence may run in chunks as matrix products (state_space_chunks.cu,
@@ -106,16 +106,16 @@ class SelectiveScan(_StateMixer):
     def forward(self, ctx, act: torch.Tensor, line: LineView, writes_cache: bool) -> torch.Tensor:
         self._check(writes_cache)
         w, rows, c, n, r = self.w, act.shape[0], self.inner, self.state, self.dt_rank
-        xz = linear(act, w["in_proj"])                                           # float32 [T, 2 inner]: x | z
+        xz = part_linear(act, w["in_proj"])                                      # float32 [T, 2 inner]: x | z
         x32 = ctx.buffer("selective_scan.x32", (rows, c), torch.float32)
         x = self._typed(ctx, "selective_scan.x", (rows, c))
         ops.causal_conv(xz, 0, c, w["conv"], w["conv_bias"], ctx, line.state, self.state_floats, x32, x, activation="silu")
-        low = linear(x if x is not None else x32, w["x_proj"])                   # float32 [T, dt_rank + 2 state]: dt | B | C
+        low = part_linear(x if x is not None else x32, w["x_proj"])              # float32 [T, dt_rank + 2 state]: dt | B | C
         step_in = low[:, :r] if self.dtype == torch.float32 else low[:, :r].to(self.dtype)
-        dt = linear(step_in, w["dt_proj"])                                       # float32 [T, inner], before bias and softplus
+        dt = part_linear(step_in, w["dt_proj"])                                  # float32 [T, inner], before bias and softplus
         out = ctx.buffer("selective_scan.y", (rows, c), self.dtype)
         ops.selective_scan(xz, c, x32, low, r, r + n, dt, w["dt_bias"], w["a_log"], w["d"], ctx, line.state, 0, out)
-        return linear(out, w["o_proj"])
+        return part_linear(out, w["o_proj"])
 
 
 class GatedLinearRecurrence(_StateMixer):
@@ -164,7 +164,7 @@ class GatedLinearRecurrence(_StateMixer):
     def forward(self, ctx, act: torch.Tensor, line: LineView, writes_cache: bool) -> torch.Tensor:
         self._check(writes_cache)
         w, rows, c = self.w, act.shape[0], self.width
-        yx = linear(act, self.w_yx)                                              # float32 [T, 2 width]: gate branch | recurrent branch
+        yx = part_linear(act, self.w_yx)                                         # float32 [T, 2 width]: gate branch | recurrent branch
         u32 = ctx.buffer("gated_recurrence.u32", (rows, c), torch.float32)
         u = self._typed(ctx, "gated_recurrence.u", (rows, c))
         ops.causal_conv(yx, c, c, w["conv"], w["conv_bias"], ctx, line.state, self.state_floats, u32, u, in_bias=w["x_bias"])
@@ -179,7 +179,7 @@ class GatedLinearRecurrence(_StateMixer):
         prepared = ctx.buffer("gated_recurrence.prepared", (3, rows, c), torch.float32)
         ops.gated_recurrence(yx, 0, w["y_bias"], u32, gates, w["a_gate_bias"], w["i_gate_bias"], w["lam"], ctx, line.state, 0,
                              out, block_width=self.block_width, gate_constant=self.gate_constant, prepared=prepared)
-        return linear(out, w["o_proj"])
+        return part_linear(out, w["o_proj"])
 
 
 class ScalarDecayStateSpace(_StateMixer):
@@ -236,7 +236,7 @@ class ScalarDecayStateSpace(_StateMixer):
         self._check(writes_cache)
         w, rows, c = self.w, act.shape[0], self.inner
         gn = self.groups * self.state
-        proj = linear(act, w["in_proj"])                                         # float32 [T, ...]: z | x | B | C | dt
+        proj = part_linear(act, w["in_proj"])                                    # float32 [T, ...]: z | x | B | C | dt
         xbc = ctx.buffer("state_space.xbc", (rows, self.conv_channels), torch.float32)
         ops.causal_conv(proj, c, self.conv_channels, w["conv"], w["conv_bias"], ctx, line.state, self.state_floats, xbc,
                         activation="silu")
@@ -253,7 +253,7 @@ class ScalarDecayStateSpace(_StateMixer):
             ops.state_space_scan(*args, **sizes)
         out = ctx.buffer("state_space.out", (rows, c), self.dtype)
         ops.group_rms_norm(y, w["norm"], out, self.norm_groups, self.norm_eps)
-        return linear(out, w["o_proj"])
+        return part_linear(out, w["o_proj"])
 
 
 class GatedDeltaRule(_StateMixer):
@@ -329,7 +329,7 @@ class GatedDeltaRule(_StateMixer):
     def forward(self, ctx, act: torch.Tensor, line: LineView, writes_cache: bool) -> torch.Tensor:
         self._check(writes_cache)
         w, rows = self.w, act.shape[0]
-        proj = linear(act, self.w_in)                                            # float32 [T, in_rows]: q | k | v | beta | decay | gate
+        proj = part_linear(act, self.w_in)                                       # float32 [T, in_rows]: q | k | v | beta | decay | gate
         qkv = ctx.buffer("delta_rule.qkv", (rows, self.conv_channels), torch.float32)
         ops.causal_conv(proj, 0, self.conv_channels, w["conv"], None, ctx, line.state, self.state_floats, qkv, activation="silu")
         out = ctx.buffer("delta_rule.out", (rows, self.v_width), self.dtype)
@@ -344,7 +344,7 @@ class GatedDeltaRule(_StateMixer):
             ops.delta_chunks(*args, chunks=chunks, scratch=ctx.buffer("delta_rule.chunks", (floats,), torch.float32), **sizes)
         else:
             ops.gated_delta_rule(*args, **sizes)
-        return linear(out, w["o_proj"])
+        return part_linear(out, w["o_proj"])
 
 
 class MinGru(_StateMixer):
@@ -381,10 +381,10 @@ class MinGru(_StateMixer):
     def forward(self, ctx, act: torch.Tensor, line: LineView, writes_cache: bool) -> torch.Tensor:
         self._check(writes_cache)
         w, rows, c = self.w, act.shape[0], self.width
-        proj = linear(act, self.w_in)                                            # float32 [T, in_rows]: z | x | gate, before biases
+        proj = part_linear(act, self.w_in)                                       # float32 [T, in_rows]: z | x | gate, before biases
         out = ctx.buffer("min_gru.y", (rows, c), self.dtype)
         ops.min_gru(proj, 0, c, 2 * c, w["z_bias"], w["x_bias"], ctx, line.state, 0, out)
-        return linear(out, w["o_proj"])
+        return part_linear(out, w["o_proj"])
 
 
 register_part("mixer", "min_gru", MinGru, replace=True)

@@ -23,7 +23,7 @@ from ..cache import CacheNeed, LineView
 from ..csrc import ops
 from ..weights.loader import MATRIX, TensorNeed, TensorSource
 from .base import Mixer, register_part
-from .linear import linear
+from .linear import part_linear
 
 CHUNK_MIN_TOKENS = 8           # steps whose longest run of new tokens is shorter go token by token
 
@@ -89,12 +89,12 @@ class Retention(Mixer):
         rows = act.shape[0]
         # q | k | v | gate: float32 for the recurrence token by token; a bfloat16 prompt's chunks take them in bfloat16
         chunks = self.dtype == torch.bfloat16 and ctx.max_q_len >= CHUNK_MIN_TOKENS and ops.retention_chunks_take(self.head_dim, self.value_dim)
-        proj = linear(act, self.w_in, rounded=chunks)                       # [T, in_rows]
+        proj = part_linear(act, self.w_in, rounded=chunks)                  # [T, in_rows]
         out = ctx.buffer("retention.out", (rows, self.v_width), self.dtype)
         raw = ctx.buffer("retention.raw", (rows, self.v_width), torch.float32)      # for steps that cut the heads over blocks
         ops.retention(proj, self.offsets, self.decay, ctx, line.state, 0, out, raw, heads=self.num_heads, dim=self.head_dim,
                       vdim=self.value_dim, k_scale=self.k_scale, eps=self.norm_eps)
-        return linear(out, self.w_o)
+        return part_linear(out, self.w_o)
 
 
 register_part("mixer", "retention", Retention, replace=True)

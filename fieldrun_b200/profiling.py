@@ -563,12 +563,12 @@ def float32_products(kind: str, launches: int) -> dict:
             ops.products_f32(w2, scales[1], both, parts[:2 * n * WIDTH].view(2, n, WIDTH), scale, y, gated=True, **how)
         flops, weights = 6.0 * n * HIDDEN * WIDTH, (w13.numel() + w2.numel()) * 4
     else:
-        from .parts.linear import linear, require_true_float32
+        from .parts.linear import part_linear, require_true_float32
         require_true_float32()
         w, x = torch.randn(8192, HIDDEN, device=DEV) * 0.02, torch.randn(6 if kind == "rows" else 3704, HIDDEN, device=DEV)
 
         def launch():
-            linear(x, w)
+            part_linear(x, w)
         flops, weights = 2.0 * x.shape[0] * w.numel(), w.numel() * 4
     ms = _time(launch, launches)
     ops.tc_status_check(torch.device(DEV))

@@ -139,6 +139,19 @@ def test_dense_rows_of_every_number(features, inner):
         assert (got[rows] == 7.0).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_products_of_a_weight_that_the_kernel_before_wrote(dtype):
+    from fieldrun_b200.parts.linear import linear, require_true_float32
+    require_true_float32()
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    drawn, x = torch.randn(8192, 3072, device=DEV, generator=gen).to(dtype), torch.randn(4, 3072, device=DEV, generator=gen).to(dtype)
+    w, once = drawn.clone(), linear(x, drawn)
+    torch.cuda.synchronize()
+    for power in range(12):
+        torch.mul(drawn, 2.0 ** power, out=w)
+        assert torch.equal(linear(x, w), once * 2.0 ** power)
+
+
 def split_product(w, x, lists=None, max_tiles=0, source=None, gated=False, limit=0.0):
     """w [E, F, K] times the rows of x (of ``source``) by the tensor cores' float32 products."""
     count = len(source) if source is not None else x.shape[0]

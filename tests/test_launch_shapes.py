@@ -67,6 +67,24 @@ def test_float32_rows_are_checked_against_the_weights_before_a_launch():
             ops.dense_rows_f32(torch.zeros(16, 12), x, out)
 
 
+def test_only_a_parts_product_may_read_its_weight_early(monkeypatch):
+    """A product of any other weight, which may be the result of the kernel before it, waits for that one."""
+    import inspect
+
+    import torch
+    from fieldrun_b200.csrc import ops
+    from fieldrun_b200.parts import linear as products
+    calls = []
+    monkeypatch.setattr(ops, "_call", lambda name, *args: calls.append(args))
+    monkeypatch.setattr(ops, "_ptr", lambda t: 0)
+    weight, x, out = torch.zeros(16, 12), torch.zeros(2, 12), torch.zeros(2, 16)
+    ops.dense_rows_f32(weight, x, out)
+    ops.dense_rows_f32(weight, x, out, weights_final=True)
+    assert [c[-1] for c in calls] == [0, 1]
+    parameters = inspect.signature(products.linear).parameters
+    assert parameters["weight_final"].default is False and products.part_linear.keywords == {"weight_final": True}
+
+
 @pytest.mark.parametrize("hidden,heads,dim,experts,width,vocab,expected", [
     (3072, 48, 128, 256, 1536, 200064, {"attention32", "products32"}),       # MiniMax-M2's layer
     (96, 8, 12, 8, 48, 384, {"attention32", "products32"}),                  # small: attention in tiles; experts on the tensor cores
