@@ -55,6 +55,17 @@ __device__ __forceinline__ void after_previous_kernel() {
     wait_for_previous_kernel();
 }
 
+// The device's SMs (every device of a process is of the one kind that this library is built for).
+inline int frb_sm_count() {
+    static const int count = [] {
+        int device = 0, sms = 0;
+        cudaGetDevice(&device);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        return sms;
+    }();
+    return count;
+}
+
 // The largest grid that is started early: the number of SMs, or FIELDRUN_B200_PDL from the environment
 // (0 starts every kernel in the ordinary way).  Blocks that start early settle on whichever SMs have room at
 // that moment; a kernel of many blocks that is bound by memory bandwidth then runs from an uneven placement
@@ -62,11 +73,7 @@ __device__ __forceinline__ void after_previous_kernel() {
 inline long frb_dependent_launch_blocks() {
     static const long most = [] {
         const char* v = getenv("FIELDRUN_B200_PDL");
-        if (v && v[0]) return atol(v);
-        int device = 0, sms = 0;
-        cudaGetDevice(&device);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        return (long)sms;
+        return v && v[0] ? atol(v) : (long)frb_sm_count();
     }();
     return most;
 }

@@ -181,28 +181,30 @@ __device__ __forceinline__ void rf_load_x(RowsOfX<R, PAIRS>& to, const float* co
     }
 }
 
-// A dense product of up to eight rows: one matrix, no lists.  A block an SM for the whole launch takes its share of the weight rows (their
-// number over the blocks, to the row), eight at a time; its warps have a part of the inner size each, always the same one, and add theirs
-// in their order.  A warp's ring runs on from eight rows to the next and, where the weights are complete, begins ahead of the wait for the
-// kernel before.  A run's place in the ring is filled again as soon as its lane has read it, ahead of the join.  The rows of x stay in
-// registers where a warp's part has at most HELD runs of them, else the next run's are asked for ahead.  `tiles`: two where seven or eight
-// rows would not fit so; neighbouring blocks then have four rows each and the same weights.
+// A dense product of up to eight rows: one matrix, no lists.  As many blocks as are resident at once take a share of the weight rows each (their
+// number over the blocks, to the row), eight at a time, for the whole launch; a block's warps have a part of the inner size each, always the same
+// one, and add theirs in their order, so that a row's sums do not depend on the other rows.  A warp's ring runs on from eight rows to the next and,
+// where the weights are complete, begins ahead of the wait for the kernel before.  A run's place in the ring is filled again as soon as its lane
+// has read it, ahead of the join.  The rows of x stay in registers where a warp's part has at most HELD runs of them, else the next run's are asked
+// for ahead.  `tiles`: two where seven or eight rows would not fit so; neighbouring blocks then have four rows each and the same weights.
 //
 // Bound by the weights' bytes up to four rows, beyond by the multiply-adds and the joins.  The kernel above, whose blocks begin and end
-// once for 32 KB to 96 KB of weights, and this one in a stream of launches, microseconds for 1, 4, 6 and 8 rows: 8192 x 3072 weights 19.9 25.0
-// 29.2 29.4 | 16.0 16.5 18.9 21.1 (15.4 at the memory's rate), 3072 x 6144 15.5 17.5 19.7 19.8 | 12.5 13.3 17.2 18.8, 1024 x 1024 3.3 3.8 4.5 4.6
-// | 2.0 2.2 2.5 2.6, 144 x 96 2.0 2.1 2.3 2.3 | 1.2 1.3 1.8 1.6.  Only with very many weight rows do a single row's joins cost more than that: 65536 x
-// 3072 113 | 120, 200064 x 3072 336 | 360; with two rows 362 | 365, with eight 419 | 377.  Rows two by two (fma.rn.f32x2) pay where the work is
-// large enough for six or eight rows' multiply-adds to bound it: 200064 x 3072 414 -> 377 with eight, 8192 x 3072 21.8 -> 20.7, but 1024 x 1024
-// 2.5 -> 3.2.  Six rows as eight: 8192 x 3072 20.6 instead of 18.9, 2048 x 8192 19.9 instead of 15.7.
+// once for 32 KB to 96 KB of weights, and this one in a stream of launches, microseconds for 1, 4, 6 and 8 rows: 8192 x 3072 weights 19.6 24.6
+// 28.8 29.1 | 15.2 15.8 18.1 19.8 (15.4 at the memory's rate), 3072 x 6144 15.4 17.1 19.0 19.3 | 12.3 12.9 16.7 18.4, 8192 x 8192 49.6 55.9 60.9 62.3
+// | 40.0 44.6 49.3 60.4, 1024 x 1024 2.9 3.4 4.0 4.1 | 1.9 2.1 2.4 2.5, 144 x 96 2.2 2.4 2.5 2.6 | 1.5 1.7 2.0 1.9.  Twelve warps an SM: with one block
+// an SM whatever the inner size 65536 x 128 takes 28 us with one row and 51 with eight instead of 7 and 12 (28 and 38 by the kernel above).  Only with
+// very many weight rows do a single row's joins cost more than that kernel's ends: 65536 x 3072 113 | 120, 200064 x 3072 338 | 362; with eight
+// rows 163 | 126 and 469 | 419, but 131072 x 2048 194 | 232.  Rows two by two (fma.rn.f32x2) pay where the work is large enough for six or eight rows'
+// multiply-adds to bound it: 200064 x 3072 414 -> 377 with eight, 8192 x 3072 21.8 -> 20.7, but 1024 x 1024 2.5 -> 3.2.  Six rows as eight: 8192 x 3072
+// 20.6 instead of 18.9, 2048 x 8192 19.9 instead of 15.7.
 #define RD_WARPS 12
 
 template <int R, int HELD>
 __global__ void __launch_bounds__(32 * RD_WARPS, 1) dense_rows_f32_kernel(const float* W, const float* X, float* __restrict__ out, int all_rows,
                                                                           int tiles, int F, int K, int weights_final) {
     extern __shared__ float4 rf_smem[];
-    __shared__ float sums[2][RD_WARPS][RF_FEATS * R];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    float* sums = (float*)(rf_smem + warps * RF_STAGES * RF_FEATS * 32);                       // [2][warps][RF_FEATS * R]
     const int share = blockIdx.x / tiles, shares = gridDim.x / tiles, tile = blockIdx.x - share * tiles;
     const int row0 = tile * R, rows = min(all_rows - row0, R);
     X += (size_t)row0 * K;
@@ -301,19 +303,31 @@ __global__ void __launch_bounds__(32 * RD_WARPS, 1) dense_rows_f32_kernel(const 
                 if (r < HALVES) first[f * HALVES + r] = each[f * R + r];
                 else second[f * 2 + r - HALVES] = each[f * R + r];
             }
-        rf_join<RF_FEATS * HALVES>(first, lane, sums[g & 1][warp]);
-        if constexpr (R == 6) rf_join<RF_FEATS * 2>(second, lane, sums[g & 1][warp] + RF_FEATS * HALVES);
+        float* group_sums = sums + (g & 1) * warps * (RF_FEATS * R);
+        rf_join<RF_FEATS * HALVES>(first, lane, group_sums + warp * (RF_FEATS * R));
+        if constexpr (R == 6) rf_join<RF_FEATS * 2>(second, lane, group_sums + warp * (RF_FEATS * R) + RF_FEATS * HALVES);
         __syncthreads();                                                 // the sums of two groups back are read by then
         for (int v = threadIdx.x; v < RF_FEATS * R; v += blockDim.x) {
             const bool last_two = v >= RF_FEATS * HALVES;
             const int at = last_two ? v - RF_FEATS * HALVES : v, each_row = last_two ? 2 : HALVES;
             const int r = at % each_row + (last_two ? HALVES : 0), f = f_begin + g * RF_FEATS + at / each_row;
             float sum = 0.f;
-            for (int k = 0; k < with_work; ++k) sum += sums[g & 1][k][v];
+            for (int k = 0; k < with_work; ++k) sum += group_sums[k * (RF_FEATS * R) + v];
             if (f < f_end && r < rows) out[(size_t)r * F + f] = sum;
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// Warps of a block: twelve, or a run of the inner size each where that has fewer.  Beyond four runs a warp the rows of x do not stay in
+// registers, and twelve warps that meet after every eight weight rows wait for one another: where there are more than eight weight rows for
+// every SM six or four do, whichever leave fewer of their blocks' places empty (eight rows of 4096 x 8192 32 us instead of 38, of 8192 x 8192 60
+// instead of 64, of 3072 x 12288 32 instead of 38; the kernel above 41, 62 and 35.  It stays ahead by up to a tenth where seven or eight
+// rows meet some 640 groups of weight rows, 5120 x 8192, and neither count of blocks comes out even).
+static int dense_rows_warps(int units, int groups, int sms) {
+    if (units < 32 * RD_WARPS) return (units + 31) / 32;
+    if (units <= 4 * 32 * RD_WARPS || groups <= sms) return RD_WARPS;
+    return 2 * ((groups + 2 * sms - 1) / (2 * sms)) <= 3 * ((groups + 3 * sms - 1) / (3 * sms)) ? 6 : 4;
 }
 
 // out [rows, F] = X [rows, K] W^T, W [F][K], all float32; up to eight rows.  weights_final: W was complete before the kernel before this one
@@ -323,17 +337,20 @@ FRB_API int frb_dense_rows_f32(const float* W, const float* X, float* out, int r
     FRB_CHECK_ARG(rows > 0 && rows <= RF_ROWS, "dense float32 rows: %d rows are outside 1..%d", rows, RF_ROWS);
     FRB_CHECK_ARG(K > 0 && K % 4 == 0, "dense float32 rows: an inner size of %d is not a multiple of 4", K);
     FRB_CHECK_ARG((((uintptr_t)W | (uintptr_t)X) & 15) == 0, "dense float32 rows: operands must be 16-byte aligned");
-    int device = 0, sms = 0;
-    cudaGetDevice(&device);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const int units = K / 4, warps = units >= 32 * RD_WARPS ? RD_WARPS : (units + 31) / 32;
+    const int sms = frb_sm_count(), units = K / 4, groups = (F + RF_FEATS - 1) / RF_FEATS, warps = dense_rows_warps(units, groups, sms);
     const int part = (units + 8 * warps - 1) / (8 * warps) * 8, runs = (part + 31) / 32;
-    // (with two tiles everywhere eight rows of 8192 x 3072 take 24.9 us instead of 20.7, of 2048 x 8192 23.6 instead of 20.8; with one, of 3072 x
-    // 6144 20.9 instead of 18.8, and six rows 18.6 with two instead of 17.2, 20.0 with their four runs in registers)
-    const int tiles = rows > 6 && runs > 2 && runs <= 4 ? 2 : 1, groups = (F + RF_FEATS - 1) / RF_FEATS;
-    const int shares = groups < sms / tiles ? groups : sms / tiles, blocks = shares * tiles;
-    const size_t smem = (size_t)warps * RF_STAGES * RF_FEATS * 32 * sizeof(float4);
-#define FRB_DENSE(R, HELD)                                                                                                            do {                                                                                                                                  if (smem > 40 * 1024)                                                                                                                 cudaFuncSetAttribute(dense_rows_f32_kernel<R, HELD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                 launch_dependent(dense_rows_f32_kernel<R, HELD>, dim3(blocks), dim3(32 * warps), smem, stream, W, X, out, rows, tiles, F, K, weights_final); } while (0)
+    // (with two tiles everywhere eight rows of 8192 x 3072 take 24.9 us instead of 20.7; with one, of 3072 x 6144 20.9 instead of 18.8, and six
+    // rows 18.6 with two instead of 17.2, 20.0 with their four runs in registers)
+    const int tiles = rows > 6 && runs > 2 && runs <= 4 ? 2 : 1;
+    const int per_sm = RD_WARPS / warps, most = per_sm * sms / tiles, shares = groups < most ? groups : most, blocks = shares * tiles;
+#define FRB_DENSE(R, HELD)                                                                                                        \
+    do {                                                                                                                          \
+        const size_t smem = (size_t)warps * (RF_STAGES * RF_FEATS * 32 * sizeof(float4) + 2 * RF_FEATS * R * sizeof(float));      \
+        if (smem > 48 * 1024)                                                                                                     \
+            cudaFuncSetAttribute(dense_rows_f32_kernel<R, HELD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);         \
+        launch_dependent_resident(per_sm, dense_rows_f32_kernel<R, HELD>, dim3(blocks), dim3(32 * warps), smem, stream, W, X,     \
+                                  out, rows, tiles, F, K, weights_final);                                                         \
+    } while (0)
 #define FRB_DENSE_ROWS(R)                                                                                                         \
     do {                                                                                                                          \
         if (runs == 1) FRB_DENSE(R, 1);                                                                                           \
@@ -367,9 +384,9 @@ FRB_API int frb_rows_f32(const float* W, const float* X, const int* x_rows, cons
     const RowsParams p = {W, X, x_rows, tile_expert, tile_row0, num_tiles, offsets, out, F, K, gate_limit};
     const int outs = paired ? RF_FEATS / 2 : RF_FEATS, groups = (F + outs - 1) / outs;      // runs of eight weight rows of a tile
     // A single tile's blocks of four runs are one or two a SM and end unevenly: there four warps share a run of weight rows.
-    // (Six rows with 8192 x 3072 and 3072 x 6144 weights, an event pair around each launch, which itself is about 6 us: 33 us on
-    // average, 52 and 57 with other splits of the same sizes into blocks of four and two runs.)  With many tiles a warp to a run has
-    // the fewer joins.
+    // (Six rows with 8192 x 3072 and 3072 x 6144 weights, which the kernel above has by now, an event pair around each launch, which
+    // itself is about 6 us: 33 us on average, 52 and 57 with other splits of the same sizes into blocks of four and two runs.)  With many
+    // tiles, or the weight rows of a vocabulary, a warp to a run has the fewer joins.
     const bool parts = (long long)groups * max_tiles < 16384;
     const dim3 grid(parts ? groups : (groups + RF_WARPS - 1) / RF_WARPS, max_tiles);
     const size_t smem = (size_t)RF_WARPS * RF_STAGES * RF_FEATS * 32 * sizeof(float4);

@@ -123,19 +123,29 @@ def test_rows_equal_the_general_kernel(features, inner, paired, limit):
     assert (got - want).abs().max() < 4 * max(inner, 16) * 2.0 ** -24 * max(want.abs().max().item(), 1.0)
 
 
-@pytest.mark.parametrize("features,inner", [(1, 4), (7, 96), (130, 132), (2500, 1024), (1185, 2048), (601, 3072), (300, 4100), (149, 6144), (74, 6200), (33, 12300)])
+# Groups of eight weight rows a block, runs of the inner size a warp: one run of several warps and blocks an SM (three groups), of eight warps
+# and one block; two, three and four runs (three groups; five for seven and eight rows, whose blocks come in pairs); five runs and more (one
+# block an SM; six and four warps of several, three groups and more).  The last block's last group is never whole.
+@pytest.mark.parametrize("features,inner", [(1, 4), (7, 96), (130, 132), (43013, 100), (14501, 132), (7205, 516), (3077, 1024), (3077, 1536), (3077, 3072),
+                                            (3077, 4100), (3077, 6144), (74, 6200), (7205, 6200), (9597, 6200), (3077, 12300)])
 def test_dense_rows_of_every_number(features, inner):
-    """Parts of the inner size that fill no run, one to more than four of them, shares of a block that end inside eight weight rows; inputs and
-    results behind the last row stay as they are.  Sums of `inner` terms of size one: off by less than inner roundings of the largest."""
+    """Parts of the inner size that fill no run, one to many of them, shares of a block that end inside eight weight rows; inputs and results
+    behind the last row stay as they are.  Sums of `inner` terms of size one: off by less than inner roundings of the largest.  A row's bits
+    do not depend on the other rows."""
     gen = torch.Generator(device=DEV).manual_seed(features + inner)
     w = torch.randn(features, inner, device=DEV, generator=gen) * inner ** -0.5
+    all_rows = torch.randn(8, inner, device=DEV, generator=gen)
+    want = all_rows.double() @ w.double().T
+    alone = torch.empty(8, features, device=DEV)
+    for row in range(8):
+        ops().dense_rows_f32(w, all_rows[row:row + 1], alone[row:row + 1])
     for rows in range(1, 9):
         x = torch.full((rows + 1, inner), float("nan"), device=DEV)
-        x[:rows] = torch.randn(rows, inner, device=DEV, generator=gen)
+        x[:rows] = all_rows[:rows]
         got = torch.full((rows + 1, features), 7.0, device=DEV)
-        ops().dense_rows_f32(w, x[:rows], got[:rows])
-        want = x[:rows].double() @ w.double().T
-        assert (got[:rows] - want).abs().max() < 2 * max(inner, 16) * 2.0 ** -24 * max(want.abs().max().item(), 1.0)
+        ops().dense_rows_f32(w, x[:rows], got[:rows], weights_final=rows % 2 == 0)
+        assert (got[:rows] - want[:rows]).abs().max() < 2 * max(inner, 16) * 2.0 ** -24 * max(want.abs().max().item(), 1.0)
+        assert torch.equal(got[:rows], alone[:rows])
         assert (got[rows] == 7.0).all()
 
 
