@@ -18,11 +18,15 @@ import torch
 from ..csrc import ops
 
 _ONE_TILE: dict[tuple[str, int], tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]] = {}
-STREAM_ROWS = 8           # up to this many rows a dense product is a stream over the weight (experts_stream.cu); beyond, each
-                          # item's rows of x are as many bytes as its weights and the library's product is faster (measured at
+STREAM_ROWS = 8           # up to this many rows a dense product is a stream over the weight (experts_stream.cu; float32: rows_f32.cu); beyond,
+                          # each item's rows of x are as many bytes as its weights and the library's product is faster (measured at
                           # 12 to 32 rows on a B200: 14 to 25 us against 11 for MiniMax-M2's projections)
-ONE_ROW_FEATURES = 65536  # from this many output features on a single float32 row's product is faster by the experts' kernel (rows_f32.cu;
-                          # 3,072 inputs, 32,768 features 60.6 us against 61.4, 65,536 113 against 120, 200,064 336 against 360)
+# A float32 weight of up to this many entries is streamed by the dense products' kernel, a larger one by the experts' (both in rows_f32.cu).
+# The number of rows has no say: the two add a row's products in different orders, and a sequence's results shall not depend on how many
+# others are in its step.  The line lies where no number of rows is slower by the first than by the second; microseconds for 1, 4 and 8
+# rows by the second | the first: 65536 x 1024 weights 42 54 77 | 41 44 60, 21845 x 3072 43 56 63 | 41 43 45; beyond, 65536 x 3072
+# 113 141 163 | 120 125 126, 131072 x 2048 157 183 194 | 158 188 232, 200064 x 3072 338 417 469 | 362 383 419.
+DENSE_ROWS_ENTRIES = 1 << 26
 STREAM_FEATURES = 65536   # beyond this many output features the library product is at the memory roofline anyway
 
 
@@ -111,8 +115,8 @@ def linear(rows: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor]
                 and (ops.rows_f32_takes(rows.shape[1]) if few else ops.products_f32_take(rows.shape[1])):
             result = out if out is not None else torch.empty((rows.shape[0], weight.shape[0]), dtype=torch.float32, device=rows.device)
             if few:
-                if rows.shape[0] == 1 and weight.shape[0] >= ONE_ROW_FEATURES:
-                    tile_expert, tile_row0, num_tiles, offsets = one_tile(rows.device, 1)
+                if weight.numel() > DENSE_ROWS_ENTRIES:
+                    tile_expert, tile_row0, num_tiles, offsets = one_tile(rows.device, rows.shape[0])
                     ops.rows_f32(weight.unsqueeze(0), rows, None, tile_expert, tile_row0, num_tiles, offsets, 1, result, paired=False)
                 else:
                     ops.dense_rows_f32(weight, rows, result, weights_final=weight_final)

@@ -149,6 +149,20 @@ def test_dense_rows_of_every_number(features, inner):
         assert (got[rows] == 7.0).all()
 
 
+@pytest.mark.parametrize("features,inner", [(65536, 1024), (65544, 1024), (131073, 516)])
+def test_a_row_of_a_float32_product_is_the_same_in_any_company(features, inner):
+    """The largest weight that the dense products' kernel takes, and larger ones."""
+    from fieldrun_b200.parts.linear import DENSE_ROWS_ENTRIES, linear, require_true_float32
+    require_true_float32()
+    assert (features * inner <= DENSE_ROWS_ENTRIES) == (features == 65536)
+    gen = torch.Generator(device=DEV).manual_seed(features)
+    w, x = torch.randn(features, inner, device=DEV, generator=gen) * inner ** -0.5, torch.randn(8, inner, device=DEV, generator=gen)
+    together, want = linear(x, w), x.double() @ w.double().T
+    assert (together - want).abs().max() < 2 * inner * 2.0 ** -24 * want.abs().max()
+    for first, rows in ((0, 1), (7, 1), (3, 2), (0, 5), (1, 7)):
+        assert torch.equal(linear(x[first:first + rows], w), together[first:first + rows])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_products_of_a_weight_that_the_kernel_before_wrote(dtype):
     from fieldrun_b200.parts.linear import linear, require_true_float32
