@@ -1,8 +1,9 @@
 // Recurrences over a float32 state per sequence, and the short causal convolution that stands in front of them.
 //
 //   causal_conv      out[t, c] = act(bias[c] + sum_k taps[c, k] * in[t - (K-1) + k, c]), the inputs before a step's first
-//                    token coming from the state (the last K-1 inputs of the sequence; zeros for a new sequence); two
-//                    kernels: the rows that see only their own step, and each sequence's first rows with the state
+//                    token coming from the state (the last K-1 inputs of the sequence; zeros for a new sequence); the rows
+//                    that see only their own step, and each sequence's first rows with the state, in two kernels or (two to four
+//                    taps, 16-byte rows, 128 rows and more) in one
 //   selective_scan   S[c, n] <- exp(dt_c A[c, n]) S[c, n] + dt_c x_c B_n;  y_c = sum_n S[c, n] C_n + D_c x_c;  y silu(z)
 //   gated_recurrence a = exp(-g r softplus(lam)),  S <- a S + sqrt(1 - a^2) i u,  out = S * act(y)    (per channel)
 //   state_space_scan per head: S <- exp(-exp(A_log) dt) S + dt B x^T (S is [N, vdim]);  y = S^T C + D x;  y silu(z)
@@ -71,7 +72,7 @@ struct ConvParams {
     float* out32;            // [T, C]
     void* out_typed;         // null, or [T, C] in the model dtype
     int in_stride, in_offset, channels, taps_count, activation, num_rows;
-    int rows_per_thread;     // CONV_ROWS for a step of many rows, 1 for a step of few (one token a sequence)
+    int rows_per_thread;     // one channel a thread: CONV_ROWS, or 1 for a step of few rows; four channels a thread: conv_fours_rows()
 };
 
 __device__ __forceinline__ float conv_activation(float v, int activation) { return activation == 1 ? silu_f(v) : v; }
@@ -297,6 +298,16 @@ __global__ void __launch_bounds__(128) causal_conv_heads_kernel(ConvParams p) {
     }
 }
 
+// Rows a thread of causal_conv_fours_kernel: eight where all blocks are resident at once, else as many as make them so, up to 32, since a run's
+// first inputs, which the run before has read as well, are then few (8,192 rows of 6,144 channels: 32 rows 84 us, 16 85, 8 97).  Not 32 where
+// these leave a last wave of few blocks: two taps, 8,192 rows of 2,048 channels 42 us in 1.15 waves, with 16 rows 34 in 2.3.
+static int conv_fours_rows(int num_rows, int blocks_of_channels) {
+    const long long resident = 6ll * frb_sm_count();
+    const auto blocks = [&](int rows) { return (long long)((num_rows + rows - 1) / rows) * blocks_of_channels; };
+    if (blocks(8) <= resident) return 8;
+    return blocks(16) <= resident || (blocks(32) > resident && 2 * blocks(32) < 3 * resident) ? 16 : 32;
+}
+
 FRB_API int frb_causal_conv(const float* in, int in_stride, int in_offset, const float* in_bias, const float* taps,
                             const float* bias, const int* tok_seq, const int* seq_slot, const int* seq_start,
                             const int* cu_q_len, float* state, long long copy_floats, long long state_offset, float* out32,
@@ -322,13 +333,7 @@ FRB_API int frb_causal_conv(const float* in, int in_stride, int in_offset, const
     FRB_DISPATCH_DTYPE(typed_dtype, OutT, {
         // one token a sequence: no row sees only its own step (unless there is one tap, and then no state)
         if (fours && num_rows > num_seqs) {
-            // as many rows a thread as leave every SM its six blocks, up to 32 (8,192 rows of 6,144 channels: 32 rows 84 us, 16 85, 8 97), so
-            // that a run's first inputs, which the run before has read as well, are few
-            int device = 0, sms = 0;
-            cudaGetDevice(&device);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-            p.rows_per_thread = 32;
-            while (p.rows_per_thread > 8 && (long long)(num_rows / p.rows_per_thread) * ((channels / 4 + 127) / 128) < 6ll * sms) p.rows_per_thread /= 2;
+            p.rows_per_thread = conv_fours_rows(num_rows, (channels / 4 + 127) / 128);
             const dim3 fours_grid(num_seqs + (num_rows + p.rows_per_thread - 1) / p.rows_per_thread, (channels / 4 + 127) / 128);
             if (taps_count == 4) launch_dependent(causal_conv_fours_kernel<OutT, 4>, fours_grid, dim3(128), 0, stream, p, num_seqs);
             else if (taps_count == 3) launch_dependent(causal_conv_fours_kernel<OutT, 3>, fours_grid, dim3(128), 0, stream, p, num_seqs);
