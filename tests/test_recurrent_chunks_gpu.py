@@ -667,19 +667,32 @@ GATES = {"subnormal": (1e-45, 1e-38), "tiny": (1e-38, 1e-8), "small": (1e-8, 0.1
          "up to 80": (60.0, 79.9999), "around 80": (79.5, 80.5), "beyond": (80.0, 200.0)}
 
 
+def gates_of(size, sign, tokens, width):
+    """A million of that size and sign for 4,096 x 256, zeros, infinities and NaNs among them."""
+    gen = torch.Generator(device=DEV).manual_seed(7)
+    low, high = GATES[size]
+    spread = torch.rand(tokens, width, device=DEV, generator=gen, dtype=torch.float64)
+    gates = (sign * torch.exp(spread * np.log(high / low)) * low).float()
+    for row, odd in ((70, INF), (200, -INF), (330, NAN), (460, 0.0), (590, -0.0), (720, 500.0), (850, -500.0)):
+        gates[row, ::7] = odd
+    return gates
+
+
+def same_bits(plain, got, gates):
+    assert torch.equal(plain.isnan(), got.isnan()) and plain.isnan().any()
+    differ = (plain.view(torch.int32) != got.view(torch.int32)) & ~plain.isnan()
+    assert not differ.any(), (differ.sum().item(), gates[differ][:5].tolist(), plain[differ][:5].tolist(), got[differ][:5].tolist())
+
+
 @pytest.mark.parametrize("sign", [1.0, -1.0])
 @pytest.mark.parametrize("size", GATES)
 def test_gates_have_the_bits_of_the_division(size, sign):
     """x and D of one and a B of zeros: the outputs are z / (1 + exp(-z)), in chunks by a reciprocal and one correction below 80, token by
-    token by a division.  A million z of every size, and zeros, infinities and NaNs among them."""
+    token by a division."""
     heads, groups, n, vdim, tokens = 4, 1, 64, 64, 4096
-    inner, gen = heads * vdim, torch.Generator(device=DEV).manual_seed(7)
-    low, high = GATES[size]
+    inner = heads * vdim
     proj = torch.zeros(tokens, inner + heads, device=DEV)
-    spread = torch.rand(tokens, inner, device=DEV, generator=gen, dtype=torch.float64)
-    proj[:, :inner] = (sign * torch.exp(spread * np.log(high / low)) * low).float()
-    for row, odd in ((70, INF), (200, -INF), (330, NAN), (460, 0.0), (590, -0.0), (720, 500.0), (850, -500.0)):
-        proj[row, ::7] = odd
+    proj[:, :inner] = gates_of(size, sign, tokens, inner)
     xbc = torch.ones(tokens, inner + 2 * groups * n, device=DEV)
     xbc[:, inner:] = 0.0
     zeros, ones = torch.zeros(heads, device=DEV), torch.ones(heads, device=DEV)
@@ -694,7 +707,31 @@ def test_gates_have_the_bits_of_the_division(size, sign):
         else:
             ops().state_space_scan(*args, **sizes)
         results.append(out)
-    plain, got = results
-    assert torch.equal(plain.isnan(), got.isnan()) and plain.isnan().any()
-    differ = (plain.view(torch.int32) != got.view(torch.int32)) & ~plain.isnan()
-    assert not differ.any(), (differ.sum().item(), proj[:, :inner][differ][:5].tolist(), plain[differ][:5].tolist(), got[differ][:5].tolist())
+    same_bits(*results, proj[:, :inner])
+
+
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+@pytest.mark.parametrize("size", GATES)
+def test_gates_of_linear_attention_have_the_bits_of_the_division(size, sign):
+    """Decays of zero, one entry of q and k, values of one and no epsilon: every normed output is one, and the results are the gates."""
+    heads, dim, vdim, rank, tokens = 4, 64, 64, 4, 4096
+    qk, inner = heads * dim, heads * vdim
+    offsets = (0, qk, 2 * qk, 2 * qk + inner, 2 * qk + 2 * inner)
+    proj = torch.zeros(tokens, offsets[4] + rank, device=DEV)
+    proj[:, 0:2 * qk:dim] = 1.0
+    proj[:, offsets[2]:offsets[3]] = 1.0
+    gates = proj[:, offsets[3]:offsets[4]]
+    gates[:] = gates_of(size, sign, tokens, inner)
+    a2, bias, norm = torch.zeros(qk, rank, device=DEV), torch.full((qk,), -1000.0, device=DEV), torch.ones(vdim, device=DEV)
+    sizes, results = dict(heads=heads, dim=dim, vdim=vdim, tau=1.0, q_scale=1.0, eps=0.0), []
+    for chunked in (False, True):
+        state, out = torch.zeros(1, 2, heads, dim, vdim, device=DEV), torch.full((tokens, inner), NAN, device=DEV)
+        args = (proj, offsets, a2, bias, norm, state, i32([0]), i32([0]), i32([0, tokens]), out)
+        if chunked:
+            chunks = tables([tokens], 64)
+            scratch = torch.full((ops().gla_chunks_scratch_floats(chunks[0].numel(), tokens, heads, dim, vdim),), NAN, device=DEV)
+            ops().gla_chunks(*args, chunks=chunks, scratch=scratch, **sizes)
+        else:
+            ops().gla_scan(*args, **sizes)
+        results.append(out)
+    same_bits(*results, gates)
