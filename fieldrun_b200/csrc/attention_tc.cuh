@@ -1,7 +1,8 @@
-// What the tcgen05 prompt attention kernels share: arithmetic on pairs of float32, the hardware's exponential, capped scores.
+// What the tcgen05 prompt attention kernels share: the hardware's exponential, capped scores.
 #pragma once
 
 #include "common.cuh"
+#include "pairs.cuh"
 #include "tcgen05.cuh"
 
 #define AT_QUERIES 128
@@ -20,33 +21,6 @@ __device__ __forceinline__ float exp2_fast(float x) {
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
-
-// the hardware's instructions on two float32 values in one 64-bit register
-__device__ __forceinline__ uint64_t pair_of(float lo, float hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void halves_of(uint64_t v, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma_pairs(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ uint64_t add_pairs(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-
-
-__device__ __forceinline__ uint64_t mul_pairs(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
 

@@ -96,7 +96,7 @@ inline void launch_dependent_resident(int per_sm, void (*kernel)(Params...), dim
     cudaLaunchKernelEx(&config, kernel, Params(args)...);
 }
 
-// Starts `kernel`, whose first statement is after_previous_kernel(), early if its grid has at most a block per SM.
+// The same for grids of at most a block per SM.
 template <typename... Params, typename... Args>
 inline void launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
     launch_dependent_resident(1, kernel, grid, block, smem, stream, args...);

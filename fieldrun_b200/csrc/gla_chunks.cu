@@ -16,6 +16,7 @@
 // and 262; gla.cu 1.66 ms in segments of 128, whose 500 instructions a warp and token run one after the other).  What bounds them: the
 // instructions around the products (58 and 48 % of the issue slots; a decay's two exponentials and a logarithm, the parts, the block's own
 // pairs), with two blocks an SM to hide the rows' way in; with q, k and v loaded where they are used 0.68 ms.
+#include "pairs.cuh"
 #include "silu.cuh"
 #include "tf32_parts.cuh"
 
@@ -50,14 +51,6 @@ __device__ __forceinline__ void gc_copy_rows(float* to, int ld, const float* fro
         else *(float4*)(to + t * ld + 4 * u) = make_float4(0.f, 0.f, 0.f, 0.f);
     }
 }
-
-__device__ __forceinline__ uint64_t gc_pair(float lo, float hi) {
-    uint64_t v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-    return v;
-}
-
-__device__ __forceinline__ void gc_fma_pair(uint64_t a, uint64_t b, uint64_t& c) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b)); }
 
 __device__ __forceinline__ float gc_log_sigmoid(float z) { return fminf(z, 0.f) - log1pf(expf(-fabsf(z))); }
 
@@ -98,7 +91,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_states_kernel(GlaChun
         // two tokens at a time (the same multiply-adds, half the instructions)
         uint64_t pairs[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) pairs[i] = gc_pair(bias, bias);
+        for (int i = 0; i < 4; ++i) pairs[i] = pair_of(bias, bias);
 #pragma unroll 1
         for (int r = 0; r < rank; r += 4) {
             const float4 w = *(const float4*)(a2_s + d * la2 + r);
@@ -107,16 +100,16 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gla_chunk_states_kernel(GlaChun
             for (int q = 0; q < 4; ++q) {
                 const ulonglong2* x = (const ulonglong2*)(a1_s + (r + q) * GC_LA1 + t0 + tg);
                 const ulonglong2 x0 = x[0], x1 = x[1];
-                const uint64_t ww = gc_pair(each[q], each[q]);
-                gc_fma_pair(ww, x0.x, pairs[0]);
-                gc_fma_pair(ww, x0.y, pairs[1]);
-                gc_fma_pair(ww, x1.x, pairs[2]);
-                gc_fma_pair(ww, x1.y, pairs[3]);
+                const uint64_t ww = pair_of(each[q], each[q]);
+                pairs[0] = fma_pairs(ww, x0.x, pairs[0]);
+                pairs[1] = fma_pairs(ww, x0.y, pairs[1]);
+                pairs[2] = fma_pairs(ww, x1.x, pairs[2]);
+                pairs[3] = fma_pairs(ww, x1.y, pairs[3]);
             }
         }
         float z[8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) asm("mov.b64 {%0, %1}, %2;" : "=f"(z[2 * i]), "=f"(z[2 * i + 1]) : "l"(pairs[i]));
+        for (int i = 0; i < 4; ++i) halves_of(pairs[i], z[2 * i], z[2 * i + 1]);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int t = t0 + tg + i;
@@ -504,7 +497,7 @@ FRB_API int frb_gla_chunks(const float* proj, int P, int off_q, int off_k, int o
     p.off_q = off_q; p.off_k = off_k; p.off_v = off_v; p.off_g = off_g; p.off_a = off_a; p.heads = heads; p.rank = rank;
 #define FRB_GLA_CHUNKS(DIM, VDIM)                                                                                                    \
     do {                                                                                                                             \
-        const size_t one = (size_t)(GC_TOKENS * (DIM + 4 + VDIM + 4) + GC_LA1 * rank + DIM * (rank + 4)) * sizeof(float);                     \
+        const size_t one = (size_t)(GC_TOKENS * (DIM + 4 + VDIM + 4) + GC_LA1 * rank + DIM * (rank + 4)) * sizeof(float);            \
         const size_t slabs = 2 * 32 * (VDIM + 4), rows_q = GC_TOKENS * (DIM + 8);                                                    \
         const size_t three = (rows_q + (rows_q > slabs ? rows_q : slabs) + slabs) * sizeof(float);                                   \
         cudaFuncSetAttribute(gla_chunk_states_kernel<DIM, VDIM, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)one);          \

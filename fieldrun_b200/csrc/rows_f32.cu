@@ -11,6 +11,7 @@
 // products on the tensor cores (products_f32.cu) do not take them, run here in tiles of eight rows that read an expert's weights
 // again from L2.
 #include "common.cuh"
+#include "pairs.cuh"
 
 #define RF_WARPS 4
 #define RF_FEATS 8            // weight rows a warp takes
@@ -149,14 +150,6 @@ __global__ void __launch_bounds__(32 * RF_WARPS, 3) rows_f32_kernel(RowsParams p
     }
 }
 
-__device__ __forceinline__ uint64_t rf_pair(float lo, float hi) {
-    uint64_t v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-    return v;
-}
-
-__device__ __forceinline__ void rf_fma_pair(uint64_t a, uint64_t b, uint64_t& c) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b)); }
-
 // Four entries of R rows of x; PAIRS: two rows at a time, for the same multiply-adds in half the instructions.
 template <int R, bool PAIRS>
 struct RowsOfX {
@@ -171,10 +164,10 @@ __device__ __forceinline__ void rf_load_x(RowsOfX<R, PAIRS>& to, const float* co
         const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), a = u < end ? *(const float4*)(x[r] + 4 * u) : zero;
         if (PAIRS) {
             const float4 b = u < end ? *(const float4*)(x[r + PAIRS] + 4 * u) : zero;
-            to.two[r / 2][0] = rf_pair(a.x, b.x);
-            to.two[r / 2][1] = rf_pair(a.y, b.y);
-            to.two[r / 2][2] = rf_pair(a.z, b.z);
-            to.two[r / 2][3] = rf_pair(a.w, b.w);
+            to.two[r / 2][0] = pair_of(a.x, b.x);
+            to.two[r / 2][1] = pair_of(a.y, b.y);
+            to.two[r / 2][2] = pair_of(a.z, b.z);
+            to.two[r / 2][3] = pair_of(a.w, b.w);
         } else {
             to.one[r] = a;
         }
@@ -252,11 +245,14 @@ __global__ void __launch_bounds__(32 * RD_WARPS, 1) dense_rows_f32_kernel(const 
             for (int f = 0; f < RF_FEATS; ++f) {
                 const float4 wv = ring[(stage * RF_FEATS + f) * 32];
                 if (PAIRS) {
-                    const uint64_t w2[4] = {rf_pair(wv.x, wv.x), rf_pair(wv.y, wv.y), rf_pair(wv.z, wv.z), rf_pair(wv.w, wv.w)};
+                    const uint64_t w2[4] = {pair_of(wv.x, wv.x), pair_of(wv.y, wv.y), pair_of(wv.z, wv.z), pair_of(wv.w, wv.w)};
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
 #pragma unroll
-                        for (int r = 0; r < R / 2; ++r) rf_fma_pair(w2[k], xv.two[r][k], acc2[f * (R / 2) + r]);
+                        for (int r = 0; r < R / 2; ++r) {
+                            uint64_t& sum = acc2[f * (R / 2) + r];
+                            sum = fma_pairs(w2[k], xv.two[r][k], sum);
+                        }
                 } else {
 #pragma unroll
                     for (int r = 0; r < R; ++r) acc[f * R + r] = rf_dot4(wv, xv.one[r], acc[f * R + r]);
@@ -291,7 +287,7 @@ __global__ void __launch_bounds__(32 * RD_WARPS, 1) dense_rows_f32_kernel(const 
 #pragma unroll
         for (int i = 0; i < RF_FEATS * R; ++i) {
             if (!PAIRS) each[i] = acc[i];
-            else if (i % 2 == 0) asm("mov.b64 {%0, %1}, %2;" : "=f"(each[i]), "=f"(each[i + 1]) : "l"(acc2[i / 2]));
+            else if (i % 2 == 0) halves_of(acc2[i / 2], each[i], each[i + 1]);
         }
         // (six rows as four and two: the lanes' sums meet by halves)
         constexpr int HALVES = R == 6 ? 4 : R;
